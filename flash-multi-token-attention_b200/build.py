@@ -4,8 +4,8 @@
 
 Every translation unit under csrc/ is compiled with
 ``-gencode arch=compute_100a,code=sm_100a -lineinfo`` (cross-compiles without a GPU) and
-linked into ``fmta_b200/libfmta_b200.so`` next to the Python host layer, so the library
-travels with the source tree.  A unit is rebuilt when it or any header is newer than its
+linked into ``fmta_b200/libfmta_b200.so`` next to the Python layer, so the library
+travels with the source tree; ``csrc_torch/`` (the operators' host side, C++ against torch) becomes ``fmta_b200/_native.so``.  A unit is rebuilt when it or any header is newer than its
 object file.
 """
 import argparse
@@ -20,6 +20,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "fmta_b200", "libfmta_b200.so")
+NATIVE = os.path.join(HERE, "fmta_b200", "_native.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -71,7 +72,34 @@ def build(force=False, verbose=False):
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError("link failed:\n" + r.stdout + r.stderr)
+    _build_host_layer(force, verbose)
     return LIB
+
+
+def _build_host_layer(force=False, verbose=False):
+    """fmta_b200/_native.so: the operators' host side in C++ (csrc_torch/), linked against torch and LIB."""
+    import sysconfig
+    import torch
+    src = os.path.join(HERE, "csrc_torch", "fmta_torch.cpp")
+    hdr = os.path.join(HERE, "..", "include", "fmta_b200.h")
+    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) > max(os.path.getmtime(src), os.path.getmtime(hdr)):
+        return NATIVE
+    tdir = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    inc = [os.path.join(tdir, "include"), os.path.join(tdir, "include", "torch", "csrc", "api", "include"),
+           sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    cmd = [os.environ.get("CXX", "g++"), "-shared", "-fPIC", "-O2", "-std=c++17", src, "-o", NATIVE, "-DTORCH_EXTENSION_NAME=_native",
+           "-DTORCH_API_INCLUDE_EXTENSION_H", "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)]
+    for i in inc:
+        cmd += ["-isystem", i]
+    cmd += ["-L" + os.path.join(tdir, "lib"), "-L" + os.path.dirname(LIB), "-l:libfmta_b200.so", "-lc10", "-lc10_cuda", "-ltorch",
+            "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("host layer failed:\n%s" % (r.stdout + r.stderr)[-4000:])
+    if verbose:
+        print(r.stdout + r.stderr)
+    return NATIVE
 
 
 if __name__ == "__main__":

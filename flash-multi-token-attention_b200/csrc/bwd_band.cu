@@ -13,8 +13,8 @@
 //   dQ_i += sum_e dSb[i,e] k_{i-e};  dK_j += sum_e dSb[j+e,e] q_{j+e};  dV_j += sum_d P[j+d,d] dO_{j+d}
 // One CTA owns R consecutive positions (as query rows for dQ, as keys for dK/dV, as rows for
 // dTheta) and recomputes the halo of dC rows above them, so that no two CTAs add into the same
-// output element: the result is deterministic.  dQ/dK/dV are ADDED to what the tensor-core
-// kernels wrote before.
+// output element: the result is deterministic.  The kernel runs first and WRITES its part of dQ/dK/dV (fp32); the
+// tensor-core kernels behind it add theirs in their epilogues and store the sum.
 #include "fmta_common.cuh"
 #include "fmta_params.h"
 #include "launch_util.cuh"
@@ -97,8 +97,10 @@ __global__ void __launch_bounds__(bandcfg::NT, bandcfg::Layout<D>::kCtasPerSm) b
   const size_t bh = (size_t)b * H + h;
   const int t0 = win_lo(p) + blockIdx.x * Rt;
   const int R = p.row_hi > 0 ? min(Rt, p.row_hi - t0) : Rt;   // a call with a window owns no position past its end
+  // wait first, trigger second: once every CTA here has triggered, the pre-pass and D are known to be complete, and the
+  // dQ kernel behind this one starts on that
+  pdl_wait();
   pdl_trigger();
-  pdl_wait();                                          // launched with programmatic stream serialization
   const bf16* Qg = p.Q + bh * (size_t)N * D;
   const bf16* Kg = p.K + bh * (size_t)N * D;
   const bf16* Vg = p.V + bh * (size_t)N * D;
@@ -403,7 +405,7 @@ __global__ void __launch_bounds__(bandcfg::NT, bandcfg::Layout<D>::kCtasPerSm) b
   }
 
   if (mma_out) {
-    // ---- dQ, dK, dV on mma.sync: 16 positions x 32 head dims per job, accumulating onto the values in memory ----
+    // ---- dQ, dK, dV on mma.sync: 16 positions x 32 head dims per job ----
     const int ntile = (R + 15) / 16;
     constexpr int NCH = D / 32;                                          // 32-column chunks of the head dim
     for (int job = warp; job < ntile * 3 * NCH; job += NT / 32) {
@@ -413,14 +415,7 @@ __global__ void __launch_bounds__(bandcfg::NT, bandcfg::Layout<D>::kCtasPerSm) b
       float* gout = (which == 0) ? p.dQ : (which == 1) ? p.dK : p.dV;
       float* g0 = gout + (bh * N + t0 + x0) * D + ch * 32 + (lane & 3) * 2;
       float* g1 = gout + (bh * N + t0 + x1) * D + ch * 32 + (lane & 3) * 2;
-      float acc[4][4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float2 v0 = make_float2(0.f, 0.f), v1 = v0;
-        if (ok0) v0 = *reinterpret_cast<const float2*>(g0 + j * 8);
-        if (ok1) v1 = *reinterpret_cast<const float2*>(g1 + j * 8);
-        acc[j][0] = v0.x; acc[j][1] = v0.y; acc[j][2] = v1.x; acc[j][3] = v1.y;
-      }
+      float acc[4][4] = {};
       const int kd = (m == RC / 16 - 1 && which != 0) ? 16 : 32;        // the last tile must not read past the Q / dO rows
       const bf16* A = (which == 0) ? sAQ : (which == 1) ? sAK : sAV;
       const bf16* Bm = (which == 0) ? sK + (16 * m + 32) * LD : (which == 1) ? sQ + (16 * m + 16) * LD : sdO + (16 * m) * LD;
@@ -444,8 +439,7 @@ __global__ void __launch_bounds__(bandcfg::NT, bandcfg::Layout<D>::kCtasPerSm) b
       float* ga = p.dQ + (bh * N + ta) * D + col;
       float* gb = p.dQ + (bh * N + t0 + xb) * D + col;
       const ptrdiff_t kofs = p.dK - p.dQ, vofs = p.dV - p.dQ;  // element offsets between the three outputs
-      float2 aq0 = *reinterpret_cast<const float2*>(ga), ak0 = *reinterpret_cast<const float2*>(ga + kofs), av0 = *reinterpret_cast<const float2*>(ga + vofs);
-      float2 aq1 = *reinterpret_cast<const float2*>(gb), ak1 = *reinterpret_cast<const float2*>(gb + kofs), av1 = *reinterpret_cast<const float2*>(gb + vofs);
+      float2 aq0 = make_float2(0.f, 0.f), ak0 = aq0, av0 = aq0, aq1 = aq0, ak1 = aq0, av1 = aq0;
 #pragma unroll 3
       for (int e = 0; e < W; ++e) {
         const float s10 = sdS[xr0 * DS_LD + e], s11 = sdS[xb * DS_LD + e];
@@ -480,7 +474,7 @@ int bwd_band_theta_slots(int B, int N, int cq, int ck) {
   return B * ((N + R - 1) / R);
 }
 
-// Adds the band part of dQ/dK/dV and writes one dTheta partial per CTA into p.dTheta_part
+// Writes the band part of dQ/dK/dV and one dTheta partial per CTA into p.dTheta_part
 // ([slots][H][cq*ck]).  Nothing to do when the filter has no band (pad_q + pad_k == 0).
 template <int D>
 static cudaError_t launch_bwd_band_d(const TrainParams& p, dim3 grid, cudaStream_t stream) {

@@ -53,9 +53,11 @@ __global__ void rowdot_kernel(const bf16* __restrict__ dO, const void* __restric
 
 // The same with TPR = d / 8 threads per row, 16 bytes of dO (and 16 or 32 of O) per thread: one load
 // instruction per operand and thread, 256 / TPR rows per block.
-template <bool O_BF16, int TPR>
-__global__ void __launch_bounds__(256) rowdot_vec_kernel(const bf16* __restrict__ dO, const void* __restrict__ O,
-                                                         float* __restrict__ Dv, size_t rows) {
+// With DO_F32 the gradient arrives in fp32: it is rounded to bf16 on the way, stored for the tensor-core kernels and D is
+// taken from the rounded values, as if it had been converted by a pass of its own.
+template <bool O_BF16, bool DO_F32, int TPR>
+__global__ void __launch_bounds__(256) rowdot_vec_kernel(const void* __restrict__ dO_, const void* __restrict__ O,
+                                                         bf16* __restrict__ dOb, float* __restrict__ Dv, size_t rows) {
   constexpr int D = TPR * 8;
   const size_t row = (size_t)blockIdx.x * (256 / TPR) + threadIdx.x / TPR;
   const int c = (threadIdx.x % TPR) * 8;
@@ -63,7 +65,15 @@ __global__ void __launch_bounds__(256) rowdot_vec_kernel(const bf16* __restrict_
   pdl_trigger();
   pdl_wait();                                          // launched with programmatic stream serialization
   if (row < rows) {
-    const uint4 g = *reinterpret_cast<const uint4*>(dO + row * D + c);
+    uint4 g;
+    if (DO_F32) {
+      const float4 g0 = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(dO_) + row * D + c);
+      const float4 g1 = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(dO_) + row * D + c + 4);
+      g = make_uint4(pack_bf16(g0.x, g0.y), pack_bf16(g0.z, g0.w), pack_bf16(g1.x, g1.y), pack_bf16(g1.z, g1.w));
+      *reinterpret_cast<uint4*>(dOb + row * D + c) = g;
+    } else {
+      g = *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(dO_) + row * D + c);
+    }
     const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
     float o[8];
     if (O_BF16) {
@@ -120,17 +130,19 @@ cudaError_t launch_reduce_partials(const float* part, float* out, int n_slots, i
   return launch_pdl(reduce_partials_kernel, dim3((n + 31) / 32), dim3(256), 0, stream, part, out, n_slots, n);
 }
 
-cudaError_t launch_rowdot(const void* dO, const void* O, int o_bf16, float* Dv, size_t rows, int d, cudaStream_t stream) {
-  const bf16* g = reinterpret_cast<const bf16*>(dO);
+// dOb: where the bf16 rounding of an fp32 dO goes (nullptr: dO is bf16); d = 32, 64 or 128 and aligned pointers then.
+cudaError_t launch_rowdot(const void* dO, const void* O, int o_bf16, __nv_bfloat16* dOb, float* Dv, size_t rows, int d, cudaStream_t stream) {
 #define FMTA_ROWDOT(TPR)                                                                                   \
   { const unsigned nb = (unsigned)((rows + 256 / TPR - 1) / (256 / TPR));                                  \
-    if (o_bf16) return launch_pdl(rowdot_vec_kernel<true, TPR>, dim3(nb), dim3(256), 0, stream, g, O, Dv, rows);      \
-    return launch_pdl(rowdot_vec_kernel<false, TPR>, dim3(nb), dim3(256), 0, stream, g, O, Dv, rows); }
+    auto kern = dOb ? (o_bf16 ? rowdot_vec_kernel<true, true, TPR> : rowdot_vec_kernel<false, true, TPR>)     \
+                    : (o_bf16 ? rowdot_vec_kernel<true, false, TPR> : rowdot_vec_kernel<false, false, TPR>);  \
+    return launch_pdl(kern, dim3(nb), dim3(256), 0, stream, dO, O, dOb, Dv, rows); }
   const bool al = (reinterpret_cast<uintptr_t>(dO) % 16 == 0) && (reinterpret_cast<uintptr_t>(O) % 16 == 0);
   if (al && d == 64) FMTA_ROWDOT(8)
   if (al && d == 128) FMTA_ROWDOT(16)
   if (al && d == 32) FMTA_ROWDOT(4)
 #undef FMTA_ROWDOT
+  if (dOb) return cudaErrorInvalidValue;
   const unsigned blocks = (unsigned)((rows + 7) / 8);
   if (o_bf16) rowdot_kernel<true><<<blocks, 256, 0, stream>>>(reinterpret_cast<const bf16*>(dO), O, Dv, rows, d);
   else rowdot_kernel<false><<<blocks, 256, 0, stream>>>(reinterpret_cast<const bf16*>(dO), O, Dv, rows, d);

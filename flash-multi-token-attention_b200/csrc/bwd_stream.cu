@@ -188,11 +188,7 @@ bwd_dkdv_stream_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         for (int i = 0; i < 32; ++i) o[i] = 0.f;
       }
       if (acc == 0) {
-        if (store) {
-          float* dst = p.dV + ((size_t)bh * N + krow) * D + half * 32;
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
-        }
+        if (store) store_grad32(p.dV, p.out_bf16, p.dVadd, ((size_t)bh * N + krow) * D + half * 32, o, 1.f);
       } else {
         // dKt_a leaves as bf16 through shared memory (the stages are free once every MMA has completed):
         // [128 keys][128 B] with the 128-byte swizzle, then one TMA tile store per tap
@@ -255,8 +251,8 @@ cudaError_t launch_bwd_dkdv_stream(const TrainParams& p, const __nv_bfloat16* Pb
   if (!make_tensor_map_bf16(&tmP, Pbuf, 64, 64, n_tiles, 64, 64, false)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmdC, dCbuf, 64, 64, n_tiles, 64, 64, false)) return cudaErrorInvalidValue;
   BwdTcParams bp = {};
-  bp.dV = p.dV; bp.dKt = dKt; bp.status = status;
-  bp.H = p.H; bp.N = p.N; bp.cq = p.cq; bp.ck = p.ck; bp.causal = p.causal; bp.ldp = ldp;
+  bp.dV = p.dVo; bp.dVadd = p.causal ? p.dV : nullptr; bp.out_bf16 = p.grad_bf16; bp.dKt = dKt; bp.status = status;
+  bp.B = p.B; bp.H = p.H; bp.N = p.N; bp.cq = p.cq; bp.ck = p.ck; bp.causal = p.causal; bp.ldp = ldp;
   bp.selftest_expire = take_selftest_expire(kKernBwdDkdvTc);
   auto kern = bwd_dkdv_stream_kernel;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);

@@ -149,9 +149,12 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   for (int i = tid; i < NT * Cfg::DC_BYTES / 4; i += Cfg::kThreads) reinterpret_cast<uint32_t*>(sdC)[i] = 0u;
   tc::fence_proxy_async_smem();
   tc::tc_fence_before();
-  pdl_trigger();   // the next kernel's CTAs may be scheduled once every CTA here has got this far
+  // Behind the band kernel (p.early) everything but its part of dQ is complete already: the kernel starts under the
+  // band kernel's tail and waits in its epilogue.  Otherwise it waits here.  The dK/dV kernel behind it starts as soon as
+  // every CTA here has triggered and reads what was complete by then (all but this kernel's dQ), hence the order.
   __syncthreads();
-  pdl_wait();      // nothing before this line touches global memory
+  if (!p.early) pdl_wait();
+  pdl_trigger();
   tc::tc_fence_after();
   const uint32_t tmem = *s_tmem;
 
@@ -394,7 +397,8 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     tc::tc_fence_after();
     const bool have = (my_nkb > 0) && ok;
     const bool store = row_ok && (m < OWN) && (gi >= p.row_base) && (gi < p.row_end);
-    float* orow = p.dQ + ((size_t)bh * N + (row_ok ? gi : 0)) * D;
+    const size_t orow = ((size_t)bh * N + (row_ok ? gi : 0)) * D;
+    if (p.early) pdl_wait();                            // the band kernel's part of dQ
 #pragma unroll
     for (int c = 0; c < D / 32; ++c) {
       float o[32];
@@ -404,11 +408,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
         for (int i = 0; i < 32; ++i) o[i] = 0.f;
       }
-      if (store) {
-#pragma unroll
-        for (int i = 0; i < 32; i += 4)
-          *reinterpret_cast<float4*>(orow + c * 32 + i) = make_float4(o[i] * kLn2, o[i + 1] * kLn2, o[i + 2] * kLn2, o[i + 3] * kLn2);
-      }
+      if (store) store_grad32(p.dQ, p.out_bf16, p.dQadd, orow + c * 32, o, kLn2);
     }
   }
   __syncwarp();
@@ -505,9 +505,13 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   // (batch, head)-major block order: the key tiles of one (batch, head) run side by side and share its
   // Q / dO stream in L2 (the length-major order of the dQ kernel was 7 % slower here)
   // block order: see dkdv_block_order
+  // (with more taps than the tensor memory holds accumulators for, the batch index also counts the passes over them)
   int h, b, j0;
   dkdv_block_order(BK, h, b, j0);
   j0 += p.key_base;
+  const int pass = b / p.B;
+  b -= pass * p.B;
+  const int tap0 = pass ? p.ntap : 0, ntap = pass ? cq - p.ntap : p.ntap, with_dv = pass ? 0 : p.with_dv;
   const int bh = b * p.H + h;
   const int nQB = (N + BR - 1) / BR;
   const int qb_begin = p.causal ? min(nQB, (j0 + band) / BR) : 0;
@@ -531,7 +535,9 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc::tc_fence_before();
   pdl_trigger();
   __syncthreads();
-  pdl_wait();      // nothing before this line touches global memory
+  // no pdl_wait() here: the dQ kernel before this one let it start only when every CTA of it had seen its own inputs --
+  // which are this kernel's inputs too -- complete; the wait in the epilogue is for the band kernel's part of dV and for
+  // what 'this kernel has completed' has to imply
   tc::tc_fence_after();
   const uint32_t tmem = *s_tmem;
   const uint32_t tX = tmem + Cfg::colX;
@@ -635,7 +641,7 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       // this launch accumulates taps [tap0, tap0 + ntap) (accumulator i at column 64 * (with_dv + i)) and
       // dV (column 0) when with_dv; A0 takes dV and the first half of the tap groups, A1 the rest.  With
       // PAIR a group is two adjacent taps in one 128-wide MMA (an odd last tap goes alone).
-      const int ntap = p.ntap, tap0 = p.tap0, accb = p.with_dv ? 1 : 0;
+      const int accb = with_dv ? 1 : 0;
       const int pairs = PAIR ? ntap / 2 : 0, singles = ntap - 2 * pairs;     // groups: `pairs` pairs, then `singles` single taps
       const int ngrp = pairs + singles, g_half = ngrp / 2;
       const int g_begin = ai == 0 ? 0 : g_half, g_end = ai == 0 ? g_half : ngrp;
@@ -657,7 +663,7 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (!tc::mbar_wait_warp(&full[st], ph, s_abort)) { ok = false; break; }
         if (!tc::mbar_wait_warp(pdc_full, it & 1, s_abort)) { ok = false; break; }
         tc::tc_fence_after();
-        if (ai == 0 && p.with_dv) {
+        if (ai == 0 && with_dv) {
           tc::mma_ss2pe(tmem, pt_lo, pt_hi, o_lo, o_hi, idescA, acc_on);
 #pragma unroll
           for (int k = 1; k < BR / 16; ++k)
@@ -765,7 +771,8 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     if (nblk > 0 && ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(all_done, 0, s_abort));
     tc::tc_fence_after();
     const bool have = (nblk > 0) && ok;
-    const int nacc = (p.with_dv ? 1 : 0) + p.ntap;
+    const int nacc = (with_dv ? 1 : 0) + ntap;
+    pdl_wait();
     // Everything leaves through shared memory and TMA tile stores, as whole lines: dKt_a as bf16 (its adjoint
     // kernel feeds it to mma.sync as it is) through the Kt tiles, dV as fp32 through the first query-block
     // stage -- neither is read by an MMA any more.  Tiles are [128 keys][128 B] with the 128-byte swizzle, so
@@ -786,13 +793,29 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
           for (int i = 0; i < 32; ++i) o[i] = 0.f;
         }
-        if (p.with_dv && acc == 0) {
-          unsigned char* tile = sdV + half * Cfg::KT_BYTES + row * 128;
+        if (with_dv && acc == 0) {
+          if (p.dVadd && key < N) {                    // the band kernel's part
+            const float4* add = reinterpret_cast<const float4*>(p.dVadd + ((size_t)bh * N + key) * D + half * 32);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float4 t = add[i];
+              o[4 * i] += t.x; o[4 * i + 1] += t.y; o[4 * i + 2] += t.z; o[4 * i + 3] += t.w;
+            }
+          }
+          unsigned char* tile = sdV + (p.out_bf16 ? 0 : half * Cfg::KT_BYTES) + row * 128;
+          if (p.out_bf16) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              *reinterpret_cast<uint4*>(tile + (((half * 4 + i) ^ (row & 7)) << 4)) =
+                  make_uint4(pack_bf16(o[8 * i], o[8 * i + 1]), pack_bf16(o[8 * i + 2], o[8 * i + 3]),
+                             pack_bf16(o[8 * i + 4], o[8 * i + 5]), pack_bf16(o[8 * i + 6], o[8 * i + 7]));
+          } else {
 #pragma unroll
           for (int i = 0; i < 8; ++i)
             *reinterpret_cast<float4*>(tile + ((i ^ (row & 7)) << 4)) = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+          }
         } else {
-          unsigned char* tile = sKt + (acc - (p.with_dv ? 1 : 0)) * Cfg::KT_BYTES + row * 128;
+          unsigned char* tile = sKt + (acc - (with_dv ? 1 : 0)) * Cfg::KT_BYTES + row * 128;
 #pragma unroll
           for (int i = 0; i < 4; ++i)
             *reinterpret_cast<uint4*>(tile + (((half * 4 + i) ^ (row & 7)) << 4)) =
@@ -804,12 +827,12 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tc::named_bar_sync(1, Cfg::kEwWarps * 32);
       if (tid == 0) {                                  // one thread owns the bulk group of every round
         for (int acc = 2 * r; acc < min(2 * r + 2, nacc); ++acc) {
-          if (p.with_dv && acc == 0) {
+          if (with_dv && acc == 0) {
             tc::tma_store_3d(&tmdV, sdV, 0, j0, bh);
-            tc::tma_store_3d(&tmdV, sdV + Cfg::KT_BYTES, 32, j0, bh);
+            if (!p.out_bf16) tc::tma_store_3d(&tmdV, sdV + Cfg::KT_BYTES, 32, j0, bh);
           } else {
-            const int t = acc - (p.with_dv ? 1 : 0);
-            tc::tma_store_3d(&tmdKt, sKt + t * Cfg::KT_BYTES, 0, j0, bh * cq + p.tap0 + t);
+            const int t = acc - (with_dv ? 1 : 0);
+            tc::tma_store_3d(&tmdKt, sKt + t * Cfg::KT_BYTES, 0, j0, bh * cq + tap0 + t);
           }
         }
         tc::tma_store_commit();
@@ -854,7 +877,7 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 //       A[b, (j, d)] = k_{j + b - pad_k}[d],  B[(j, d), a] = dKt_a[j, d]  -- for a fixed key the 16
 //       contraction steps are 16 consecutive columns, so every fragment row is 16 contiguous bytes
 //       of shared memory and the products land in the accumulator already summed per (a, b).
-// The rows are staged by TMA (two mbarrier batches, bounded waits), the Toeplitz tiles by one bulk copy.
+// The rows are staged by TMA (two mbarrier batches, bounded waits); every CTA builds its Toeplitz tiles from the filter.
 // One CTA per (64 keys, batch*head); dTheta leaves as one partial per CTA.
 #ifndef FMTA_DKPOST_THETA_LO
 #define FMTA_DKPOST_THETA_LO 1
@@ -876,28 +899,9 @@ struct DkPostCfg {
   }
 };
 
-// The Toeplitz tiles of every head, [H][c_q][hi, lo][16][T_LD] bf16: T[x, r] = scale * theta[a, x + pad_k + 8 - r].
-__global__ void dk_post_toeplitz_kernel(const float* __restrict__ theta, bf16* __restrict__ Tg, int cq, int ck, float scale) {
-  constexpr int T_LD = DkPostCfg::T_LD, T_ELEMS = DkPostCfg::T_ELEMS, HALO = DkPostCfg::HALO;
-  const int h = blockIdx.x, pk = (ck - 1) / 2;
-  pdl_trigger();
-  for (int i = threadIdx.x; i < cq * 16 * T_LD; i += blockDim.x) {
-    const int a = i / (16 * T_LD), x = (i / T_LD) % 16, r = i % T_LD;
-    const int bb = x + pk + HALO - r;
-    const float w = (r < 32 && bb >= 0 && bb < ck) ? theta[((size_t)h * cq + a) * ck + bb] * scale : 0.f;
-    const bf16 hi = __float2bfloat16_rn(w);
-    bf16* dst = Tg + ((size_t)h * cq + a) * 2 * T_ELEMS + x * T_LD + r;
-    dst[0] = hi;
-    dst[T_ELEMS] = __float2bfloat16_rn(w - __bfloat162float(hi));
-  }
-  // the tiles depend on the filter only, so they are built while the kernel before this one still runs; waiting
-  // here keeps "this kernel has completed" implying that one has, which the adjoint kernel behind it relies on
-  pdl_wait();
-}
-
 __global__ void __launch_bounds__(DkPostCfg::NT, 2)
 dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmX,
-                   const bf16* __restrict__ Tg, float* __restrict__ dK, float* __restrict__ dTheta_part, int* status,
+                   const float* __restrict__ theta, void* dK, const float* dKadd, int out_bf16, float* __restrict__ dTheta_part, int* status,
                    int H, int N, int cq, int ck, float scale, int n_jblocks, int dfull, int j_base) {
   using Cfg = DkPostCfg;
   constexpr int D = Cfg::D, NT = Cfg::NT, KEYS = Cfg::KEYS, HALO = Cfg::HALO;
@@ -930,12 +934,20 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     tc::mbar_fence_init();
   }
   pdl_trigger();
+  // the Toeplitz tiles depend on the filter only: they are built under the tail of the dK/dV kernel
+  for (int i = tid; i < cq * 16 * 32; i += NT) {
+    const int a = i >> 9, x = (i >> 5) & 15, r = i & 31, bb = x + pk + HALO - r;
+    const float w = (bb >= 0 && bb < ck) ? theta[((size_t)h * cq + a) * ck + bb] * scale : 0.f;
+    const bf16 hi = __float2bfloat16_rn(w);
+    bf16* dst = sT + 2 * a * T_ELEMS + x * T_LD + r;
+    dst[0] = hi;
+    dst[T_ELEMS] = __float2bfloat16_rn(w - __bfloat162float(hi));
+  }
   __syncthreads();
-  pdl_wait();      // nothing before this line touches global memory
+  pdl_wait();      // nothing before this line reads what a kernel of the same call writes
   if (tid == 0) {
-    tc::mbar_expect_tx(&bars[0], (1 + half) * Cfg::TILE_BYTES + Cfg::t_bytes(cq));
+    tc::mbar_expect_tx(&bars[0], (1 + half) * Cfg::TILE_BYTES);
     tc::tma_load_3d(smem, &tmK, &bars[0], col0, J0 - HALO, bh);
-    tc::bulk_load(sTb, Tg + (size_t)h * cq * 2 * T_ELEMS, Cfg::t_bytes(cq), &bars[0]);
     for (int a = 0; a < half; ++a) tc::tma_load_3d(smem + (a + 1) * Cfg::TILE_STRIDE, &tmX, &bars[0], col0, J0 - HALO, bh * cq + a);
     if (cq > half) {
       tc::mbar_expect_tx(&bars[1], (cq - half) * Cfg::TILE_BYTES);
@@ -994,8 +1006,13 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
           const int key = J0 + 32 * kh + 16 * m + g + 8 * hh;
-          if (key < N)
-            *reinterpret_cast<float2*>(dK + ((size_t)bh * N + key) * dfull + col0 + 16 * cgp + 8 * j + 2 * t4) = make_float2(acc[m][j][2 * hh], acc[m][j][2 * hh + 1]);
+          if (key < N) {
+            const size_t at_ = ((size_t)bh * N + key) * dfull + col0 + 16 * cgp + 8 * j + 2 * t4;
+            float2 v = make_float2(acc[m][j][2 * hh], acc[m][j][2 * hh + 1]);
+            if (dKadd) { const float2 t = *reinterpret_cast<const float2*>(dKadd + at_); v.x += t.x; v.y += t.y; }
+            if (out_bf16) *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(dK) + at_) = pack_bf16(v.x, v.y);
+            else *reinterpret_cast<float2*>(reinterpret_cast<float*>(dK) + at_) = v;
+          }
         }
   }
 
@@ -1068,8 +1085,7 @@ bool bwd_tc_supported(const TrainParams& p) {
 size_t bwd_tc_workspace_bytes(int B, int H, int N, int d, int cq) {
   const size_t rows = (size_t)B * H * N;
   auto up = [](size_t x) { return (x + 1023) / 1024 * 1024; };
-  // Kt (bf16) + dKt (bf16) + status + the Toeplitz tiles of the dKt adjoint
-  return up(rows * cq * d * 2) + up(rows * cq * d * 2) + 2048 + up((size_t)H * DkPostCfg::t_bytes(cq));
+  return up(rows * cq * d * 2) + up(rows * cq * d * 2) + 2048;      // Kt (bf16) + dKt (bf16) + status
 }
 
 size_t bwd_tc_stream_workspace_bytes(int B, int H, int N, int d, int cq) {
@@ -1096,6 +1112,13 @@ __global__ void zero_tail_rows_kernel(bf16* __restrict__ P, bf16* __restrict__ d
   for (int i = threadIdx.x; i < (64 - r0) * 8; i += blockDim.x) { p4[i] = make_uint4(0u, 0u, 0u, 0u); c4[i] = make_uint4(0u, 0u, 0u, 0u); }
 }
 
+// The stacked key operand of the backward: the caller's, or made here in the workspace.
+cudaError_t launch_bwd_ktilde(const TrainParams& p, void* workspace, cudaStream_t stream) {
+  if (p.Kt_ext && p.kt_valid) return cudaSuccess;
+  unsigned char* w = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(workspace) + 1023) & ~uintptr_t(1023));
+  return launch_ktilde(p, p.Kt_ext ? p.Kt_ext : reinterpret_cast<__nv_bfloat16*>(w), stream);
+}
+
 cudaError_t launch_bwd_dq_tc(const TrainParams& p, void* workspace, bool keep_pdc, cudaStream_t stream) {
   constexpr int D = 64;
   using Cfg = DqCfg<D, false>;
@@ -1108,10 +1131,6 @@ cudaError_t launch_bwd_dq_tc(const TrainParams& p, void* workspace, bool keep_pd
   int* status = nullptr;
   cudaError_t e = status_word_of(reinterpret_cast<int*>(w), stream, &status);
   if (e != cudaSuccess) return e;
-  if (!(p.Kt_ext && p.kt_valid)) {
-    e = launch_ktilde(p, Kt, stream);
-    if (e != cudaSuccess) return e;
-  }
   if (p.d == 128) return launch_bwd_dq_tc128(p, Kt, status, stream);
   alignas(64) CUtensorMap tmQ, tmdO, tmKt, tmV;
   if (!make_tensor_map_bf16(&tmQ, p.Q, D, p.N, BH, 8, Cfg::QR / 2, false)) return cudaErrorInvalidValue;
@@ -1119,8 +1138,9 @@ cudaError_t launch_bwd_dq_tc(const TrainParams& p, void* workspace, bool keep_pd
   if (!make_tensor_map_bf16(&tmKt, Kt, D, p.N, BH * p.cq, 64, Cfg::BC, true)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmV, p.V, D, p.N, BH, 64, Cfg::BC, true)) return cudaErrorInvalidValue;
   BwdTcParams bp = {};
-  bp.LSE = p.LSE; bp.Dvec = p.Dvec; bp.dQ = p.dQ; bp.status = status;
-  bp.H = p.H; bp.N = p.N; bp.cq = p.cq; bp.ck = p.ck; bp.causal = p.causal;
+  bp.LSE = p.LSE; bp.Dvec = p.Dvec; bp.dQ = p.dQo; bp.dQadd = p.causal ? p.dQ : nullptr; bp.out_bf16 = p.grad_bf16; bp.status = status;
+  bp.early = p.causal && !keep_pdc;
+  bp.B = p.B; bp.H = p.H; bp.N = p.N; bp.cq = p.cq; bp.ck = p.ck; bp.causal = p.causal;
   bp.selftest_expire = take_selftest_expire(kKernBwdDqTc);
   bp.row_base = win_lo(p); bp.row_end = win_hi(p);
   bp.row_anchor = keep_pdc ? (bp.row_end + 7) / 8 * 8 : bp.row_end;
@@ -1147,30 +1167,33 @@ cudaError_t launch_bwd_dq_tc(const TrainParams& p, void* workspace, bool keep_pd
 }
 
 
-// One launch of the dK/dV kernel for the taps [tap0, tap0 + ntap) (and dV).
+// One launch of the dK/dV kernel: dV and the first `ntap` taps, and the rest of the taps as a second pass (its CTAs side by
+// side with the first one's).
 template <int CQMAX, bool PAIR>
-static cudaError_t launch_dkdv_pass(const TrainParams& p, const __nv_bfloat16* Kt, __nv_bfloat16* dKt, int* status, int tap0,
+static cudaError_t launch_dkdv_pass(const TrainParams& p, const __nv_bfloat16* Kt, __nv_bfloat16* dKt, int* status,
                                     int ntap, int with_dv, int key_lo, int key_hi, cudaStream_t stream) {
   constexpr int D = 64;
   using Cfg = DkvCfg<D, CQMAX, PAIR>;
   const size_t BH = (size_t)p.B * p.H;
   alignas(64) CUtensorMap tmQ, tmdO, tmKt, tmV, tmdKt, tmdV;
   if (!make_tensor_map_bf16(&tmdKt, dKt, D, p.N, BH * p.cq, 64, Cfg::BK, true)) return cudaErrorInvalidValue;
-  if (!make_tensor_map_f32(&tmdV, p.dV, D, p.N, BH, 32, Cfg::BK, true)) return cudaErrorInvalidValue;
+  if (!(p.grad_bf16 ? make_tensor_map_bf16(&tmdV, p.dVo, D, p.N, BH, 64, Cfg::BK, true)
+                    : make_tensor_map_f32(&tmdV, p.dVo, D, p.N, BH, 32, Cfg::BK, true))) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmQ, p.Q, D, p.N, BH, 64, Cfg::QR, true)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmdO, p.dO, D, p.N, BH, 64, Cfg::BR, true)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmKt, Kt, D, p.N, BH * p.cq, 64, Cfg::BK, true)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmV, p.V, D, p.N, BH, 64, Cfg::BK, true)) return cudaErrorInvalidValue;
   BwdTcParams bp = {};
-  bp.LSE = p.LSE; bp.Dvec = p.Dvec; bp.dV = p.dV; bp.dKt = dKt; bp.status = status;
-  bp.H = p.H; bp.N = p.N; bp.cq = p.cq; bp.ck = p.ck; bp.causal = p.causal;
-  bp.tap0 = tap0; bp.ntap = ntap; bp.with_dv = with_dv;
+  bp.LSE = p.LSE; bp.Dvec = p.Dvec; bp.dV = p.dVo; bp.dVadd = p.causal ? p.dV : nullptr; bp.out_bf16 = p.grad_bf16; bp.dKt = dKt; bp.status = status;
+  bp.B = p.B; bp.H = p.H; bp.N = p.N; bp.cq = p.cq; bp.ck = p.ck; bp.causal = p.causal;
+  bp.ntap = ntap; bp.with_dv = with_dv;
   bp.key_base = key_lo;
   bp.selftest_expire = take_selftest_expire(kKernBwdDkdvTc);
   auto kern = bwd_dkdv_tc_kernel<D, CQMAX, PAIR>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
-  dim3 grid((key_hi - key_lo + Cfg::BK - 1) / Cfg::BK, p.H, p.B);
+  const int passes = ntap < p.cq ? 2 : 1;
+  dim3 grid((key_hi - key_lo + Cfg::BK - 1) / Cfg::BK, p.H, p.B * passes);
   return launch_pdl(kern, grid, dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, tmQ, tmdO, tmKt, tmV, tmdKt, tmdV, bp);
 }
 
@@ -1203,12 +1226,11 @@ cudaError_t launch_bwd_dkdv_tc(const TrainParams& p, void* workspace, float* dTh
         if (D == 128) {
           e = launch_bwd_dkdv_tc128(p, Kt, dKt, status, dv, klo, khi, stream);
         } else if (p.cq <= 6) {
-          e = launch_dkdv_pass<6, true>(p, Kt, dKt, status, 0, p.cq, dv, klo, khi, stream);
+          e = launch_dkdv_pass<6, true>(p, Kt, dKt, status, p.cq, dv, klo, khi, stream);
         } else {
           // seven taps: dV + 7 accumulators + the scratch columns exceed the tensor memory, so the taps are
-          // split over two launches (each recomputes S^T and dP^T)
-          e = launch_dkdv_pass<7, false>(p, Kt, dKt, status, 0, 4, dv, klo, khi, stream);
-          if (e == cudaSuccess) e = launch_dkdv_pass<7, false>(p, Kt, dKt, status, 4, p.cq - 4, 0, klo, khi, stream);
+          // split over two passes (each recomputes S^T and dP^T)
+          e = launch_dkdv_pass<7, false>(p, Kt, dKt, status, 4, dv, klo, khi, stream);
         }
       }
     } }
@@ -1220,15 +1242,12 @@ cudaError_t launch_bwd_dkdv_tc(const TrainParams& p, void* workspace, float* dTh
   auto kern = dk_post_mma_kernel;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  __nv_bfloat16* Tg = reinterpret_cast<__nv_bfloat16*>(w + 1024);   // status word first
   alignas(64) CUtensorMap tmK, tmX;
   if (!make_tensor_map_bf16(&tmK, p.K, D, p.N, BH, 64, DkPostCfg::ROWS, true)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmX, dKt, D, p.N, BH * p.cq, 64, DkPostCfg::ROWS, true)) return cudaErrorInvalidValue;
   // (the maps span the full head dim; each CTA fetches its 64-column slab)
   ScopedKernelTimer timer2_(kKernDkPost, stream);
-  e = launch_pdl(dk_post_toeplitz_kernel, dim3(p.H), dim3(256), 0, stream, p.theta, Tg, p.cq, p.ck, p.scale);
-  if (e != cudaSuccess) return e;
-  return launch_pdl(kern, g2, dim3(DkPostCfg::NT), (size_t)smem, stream, tmK, tmX, Tg, p.dK, dTheta_part_tc, status, p.H, p.N, p.cq,
+  return launch_pdl(kern, g2, dim3(DkPostCfg::NT), (size_t)smem, stream, tmK, tmX, p.theta, p.dKo, p.causal ? p.dK : (const float*)nullptr, p.grad_bf16, dTheta_part_tc, status, p.H, p.N, p.cq,
                     p.ck, p.scale, njb, D, j_base);
 }
 

@@ -15,14 +15,21 @@ constexpr float kLn2 = 0.6931471805599453f;
 struct BwdTcParams {
   const float* LSE;   // [B,H,N] natural log
   const float* Dvec;  // [B,H,N]
-  float* dQ;          // [B,H,N,D]   (dq kernel: overwritten)
-  float* dV;          // [B,H,N,D]   (dkdv kernel: overwritten)
+  // [B,H,N,D] gradients, fp32 or bf16 (out_bf16): this kernel's part plus, with a causal mask, the fp32 band part that
+  // the band kernel left in dQadd / dVadd (which may be the output itself)
+  void* dQ;
+  void* dV;
+  const float* dQadd;
+  const float* dVadd;
+  int out_bf16;
+  int early;          // dQ kernel: the kernel before it in the stream is the band kernel, whose part is first needed in the
+                      // epilogue (everything else was complete before the band kernel's CTAs let this one start)
   bf16* dKt;          // [B,H,cq,N,D] bf16 (dkdv kernel: overwritten)
   int* status;
-  int H, N, cq, ck, causal;
-  // dK/dV kernel: the filter taps whose dKt this launch accumulates ([tap0, tap0 + ntap)) and whether it
-  // accumulates dV as well; seven taps do not fit the tensor memory at once and take two launches
-  int tap0, ntap, with_dv;
+  int B, H, N, cq, ck, causal;
+  // dK/dV kernel: the filter taps whose dKt the first pass accumulates ([0, ntap)) and whether it accumulates dV as
+  // well; seven taps do not fit the tensor memory at once and take two passes (two sets of CTAs of one launch)
+  int ntap, with_dv;
   // window of the call: the dQ kernel tiles the rows [row_base, row_end) and writes no other row; the dK/dV
   // kernel's key tile 0 starts at key_base (whole sequence: 0, N, 0)
   int row_base, row_end, key_base;
@@ -58,6 +65,26 @@ cudaError_t launch_bwd_dkdv_tc128(const TrainParams& p, const __nv_bfloat16* Kt,
 // are walked key-tile-major instead, so that the grid ends on the shortest CTAs of several pairs and not on
 // one whole pair (before, the SMs idled 7 % of the kernel at its end).
 #ifdef __CUDACC__
+// 32 consecutive columns of one gradient row: acc * mul (+ add), stored as fp32 or bf16.
+__device__ __forceinline__ void store_grad32(void* out, int out_bf16, const float* add, size_t off, const float (&o)[32], float mul) {
+  float v[32];
+#pragma unroll
+  for (int i = 0; i < 32; i += 4) {
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (add) t = *reinterpret_cast<const float4*>(add + off + i);
+    v[i] = fmaf(o[i], mul, t.x); v[i + 1] = fmaf(o[i + 1], mul, t.y); v[i + 2] = fmaf(o[i + 2], mul, t.z); v[i + 3] = fmaf(o[i + 3], mul, t.w);
+  }
+  if (out_bf16) {
+    bf16* dst = reinterpret_cast<bf16*>(out) + off;
+#pragma unroll
+    for (int i = 0; i < 32; i += 8)
+      *reinterpret_cast<uint4*>(dst + i) = make_uint4(pack_bf16(v[i], v[i + 1]), pack_bf16(v[i + 2], v[i + 3]), pack_bf16(v[i + 4], v[i + 5]), pack_bf16(v[i + 6], v[i + 7]));
+  } else {
+    float* dst = reinterpret_cast<float*>(out) + off;
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+  }
+}
 __device__ __forceinline__ void dkdv_block_order(int BK, int& h, int& b, int& j0) {
   const int nKT = gridDim.x, nBH = gridDim.y * gridDim.z;
   const int lin = blockIdx.x + nKT * (blockIdx.y + gridDim.y * blockIdx.z);

@@ -124,9 +124,9 @@ bwd_dq_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   for (int i = tid; i < (BC / 8) * DR * 4; i += Cfg::kThreads) reinterpret_cast<uint32_t*>(sdC)[i] = 0u;
   tc::fence_proxy_async_smem();
   tc::tc_fence_before();
-  pdl_trigger();
   __syncthreads();
-  pdl_wait();      // nothing before this line touches global memory that a kernel of this library writes or reads back
+  if (!p.early) pdl_wait();   // behind the band kernel: in the epilogue (see the d = 64 kernel)
+  pdl_trigger();
   tc::tc_fence_after();
   const uint32_t tmem = *s_tmem;
   const int per_kb = cq + 1;   // ring tiles per key block
@@ -313,7 +313,8 @@ bwd_dq_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tc::tc_fence_after();
     const bool have = (nkb > 0) && ok;
     const bool store = row_ok && (m < OWN) && (gi >= p.row_base) && (gi < p.row_end);
-    float* orow = p.dQ + ((size_t)bh * N + (row_ok ? gi : 0)) * D + 64 * cg;
+    const size_t orow = ((size_t)bh * N + (row_ok ? gi : 0)) * D + 64 * cg;
+    if (p.early) pdl_wait();                            // the band kernel's part of dQ
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       float o[32];
@@ -323,11 +324,7 @@ bwd_dq_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
         for (int i = 0; i < 32; ++i) o[i] = 0.f;
       }
-      if (store) {
-#pragma unroll
-        for (int i = 0; i < 32; i += 4)
-          *reinterpret_cast<float4*>(orow + c * 32 + i) = make_float4(o[i] * kLn2, o[i + 1] * kLn2, o[i + 2] * kLn2, o[i + 3] * kLn2);
-      }
+      if (store) store_grad32(p.dQ, p.out_bf16, p.dQadd, orow + c * 32, o, kLn2);
     }
   }
   __syncwarp();
@@ -446,8 +443,7 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   }
   tc::tc_fence_before();
   pdl_trigger();
-  __syncthreads();
-  pdl_wait();      // nothing before this line touches global memory that a kernel of this library writes or reads back
+  __syncthreads();   // no pdl_wait() here: see the d = 64 kernel
   tc::tc_fence_after();
   const uint32_t tmem = *s_tmem;
   const uint32_t tX = tmem + Cfg::colX;
@@ -549,7 +545,7 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     if (nblk > 0) {   // all lanes run the loop; one elected lane issues (see tc::elect_one)
       constexpr uint32_t idescA = tc::make_idesc(D, BK, 1, 1);     // 128 (head dim) x 64 (keys), both operands MN-major
       // A0 takes dV^T and the first half of the taps, A1 the rest
-      const int ntap = p.ntap, tap0 = p.tap0, accb = p.with_dv ? 1 : 0;
+      const int ntap = p.ntap, accb = p.with_dv ? 1 : 0;
       const int t_half = ntap / 2;
       const int t_begin = ai == 0 ? 0 : t_half, t_end = ai == 0 ? t_half : ntap;
       // dO read MN-major (M = head dim across the two slabs, K = rows): 16 rows = 2048 bytes per step
@@ -580,7 +576,7 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
         for (int i = t_begin; i < t_end; ++i) {
           const uint32_t dacc = tmem + 64 * (accb + i);
-          const uint32_t a_lo = qm_lo + (uint32_t)((tap0 + i) * (128 >> 4));     // K (row) shift = +128 B per row
+          const uint32_t a_lo = qm_lo + (uint32_t)(i * (128 >> 4));     // K (row) shift = +128 B per row
           tc::mma_ss2pe(dacc, a_lo, qm_hi, cb_lo, pb_hi, idescA, acc_on);
 #pragma unroll
           for (int k = 1; k < BR / 16; ++k)
@@ -684,6 +680,7 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     tc::tc_fence_after();
     const bool have = (nblk > 0) && ok;
     const int nacc = (p.with_dv ? 1 : 0) + p.ntap;
+    pdl_wait();                                         // the band kernel's part of dV
     const int dcol = qtr * 32 + lane;                   // head-dim index of this lane
     for (int ch = cg; ch < 2 * nacc; ch += NCG) {
       const int acc = ch >> 1, half = ch & 1;
@@ -696,13 +693,24 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
       const int key0 = j0 + half * 32;
       if (p.with_dv && acc == 0) {
-        float* dst = p.dV + ((size_t)bh * N + key0) * D + dcol;      // a warp writes 32 consecutive floats per key
+        const size_t at = ((size_t)bh * N + key0) * D + dcol;        // a warp touches 32 consecutive elements per key
+        if (p.dVadd) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (key0 + i < N) dst[(size_t)i * D] = o[i];
+          for (int i = 0; i < 32; ++i)
+            if (key0 + i < N) o[i] += p.dVadd[at + (size_t)i * D];
+        }
+        if (p.out_bf16) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (key0 + i < N) reinterpret_cast<bf16*>(p.dV)[at + (size_t)i * D] = __float2bfloat16(o[i]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (key0 + i < N) reinterpret_cast<float*>(p.dV)[at + (size_t)i * D] = o[i];
+        }
       } else {
         // dKt_a leaves as bf16 [key][d]: neighbouring lanes pair up so that every lane stores one 4-byte word
-        const int tap = p.tap0 + acc - (p.with_dv ? 1 : 0);
+        const int tap = acc - (p.with_dv ? 1 : 0);
         bf16* dst = p.dKt + (((size_t)bh * cq + tap) * N + key0) * D + (dcol & ~1);
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
@@ -756,8 +764,9 @@ cudaError_t launch_bwd_dq_tc128(const TrainParams& p, const __nv_bfloat16* Kt, i
   if (!make_tensor_map_bf16(&tmKt, Kt, D, p.N, BH * p.cq, 64, Cfg::BC, true)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmV, p.V, D, p.N, BH, 64, Cfg::BC, true)) return cudaErrorInvalidValue;
   BwdTcParams bp = {};
-  bp.LSE = p.LSE; bp.Dvec = p.Dvec; bp.dQ = p.dQ; bp.status = status;
-  bp.H = p.H; bp.N = p.N; bp.cq = p.cq; bp.ck = p.ck; bp.causal = p.causal;
+  bp.LSE = p.LSE; bp.Dvec = p.Dvec; bp.dQ = p.dQo; bp.dQadd = p.causal ? p.dQ : nullptr; bp.out_bf16 = p.grad_bf16; bp.status = status;
+  bp.early = p.causal;
+  bp.B = p.B; bp.H = p.H; bp.N = p.N; bp.cq = p.cq; bp.ck = p.ck; bp.causal = p.causal;
   bp.selftest_expire = take_selftest_expire(kKernBwdDqTc);
   bp.row_base = win_lo(p); bp.row_end = win_hi(p); bp.row_anchor = bp.row_end;
   bp.own = Cfg::BM - (p.cq - 1);
@@ -781,9 +790,9 @@ cudaError_t launch_bwd_dkdv_tc128(const TrainParams& p, const __nv_bfloat16* Kt,
   if (!make_tensor_map_bf16(&tmKt, Kt, D, p.N, BH * p.cq, 64, Cfg::BK, true)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmV, p.V, D, p.N, BH, 64, Cfg::BK, true)) return cudaErrorInvalidValue;
   BwdTcParams bp = {};
-  bp.LSE = p.LSE; bp.Dvec = p.Dvec; bp.dV = p.dV; bp.dKt = dKt; bp.status = status;
-  bp.H = p.H; bp.N = p.N; bp.cq = p.cq; bp.ck = p.ck; bp.causal = p.causal;
-  bp.tap0 = 0; bp.ntap = p.cq; bp.with_dv = with_dv;
+  bp.LSE = p.LSE; bp.Dvec = p.Dvec; bp.dV = p.dVo; bp.dVadd = p.causal ? p.dV : nullptr; bp.out_bf16 = p.grad_bf16; bp.dKt = dKt; bp.status = status;
+  bp.B = p.B; bp.H = p.H; bp.N = p.N; bp.cq = p.cq; bp.ck = p.ck; bp.causal = p.causal;
+  bp.ntap = p.cq; bp.with_dv = with_dv;
   bp.key_base = key_lo;
   bp.selftest_expire = take_selftest_expire(kKernBwdDkdvTc);
   auto kern = bwd_dkdv_tc128_kernel;

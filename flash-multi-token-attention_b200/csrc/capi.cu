@@ -121,6 +121,8 @@ int fmta_selftest_expire_next(int kernel_id) {
   return FMTA_OK;
 }
 
+static size_t up1k(size_t x) { return (x + 1023) / 1024 * 1024; }
+
 size_t fmta_workspace_bytes(int op, int B, int H, int N, int d, int cq, int ck, int G) {
   (void)d;
   if (op == FMTA_OP_BWD_DQ) {
@@ -139,6 +141,11 @@ size_t fmta_workspace_bytes(int op, int B, int H, int N, int d, int cq, int ck, 
     const size_t part = (slots * H * (size_t)(cq * ck) * sizeof(float) + 1023) / 1024 * 1024;
     return part + (op == FMTA_OP_BWD_TC_STREAM && d == 64 ? bwd_tc_stream_workspace_bytes(B, H, N, d, cq)
                                                           : bwd_tc_workspace_bytes(B, H, N, d, cq));
+  }
+  if (op == FMTA_OP_BWD_FUSED) {
+    // FMTA_OP_BWD_TC, then D, the bf16 dO and the band kernel's fp32 part of dQ, dK, dV
+    const size_t rows = (size_t)B * H * N;
+    return up1k(fmta_workspace_bytes(FMTA_OP_BWD_TC, B, H, N, d, cq, ck, G)) + up1k(rows * 4) + up1k(rows * d * 2) + 3 * up1k(rows * d * 4);
   }
   if (op == FMTA_OP_MIX_EXCHANGE) {
     // optional scratch of the conv + mix cluster kernels: two sets (alternate tiles) of two fp32 tiles per CTA
@@ -233,7 +240,7 @@ int fmta_bwd_prep_D(const void* dO, const void* O, int o_dtype, float* D, size_t
   if (!dO || !O || !D) return FMTA_ERR_NULL;
   if (rows == 0 || d < 2 || (d % 2) != 0) return FMTA_ERR_SHAPE;
   if (o_dtype != FMTA_DTYPE_F32 && o_dtype != FMTA_DTYPE_BF16) return FMTA_ERR_UNSUPPORTED;
-  return check_cuda(launch_rowdot(dO, O, o_dtype == FMTA_DTYPE_BF16, D, rows, d, (cudaStream_t)stream));
+  return check_cuda(launch_rowdot(dO, O, o_dtype == FMTA_DTYPE_BF16, nullptr, D, rows, d, (cudaStream_t)stream));
 }
 
 // conv + mix backward: the exchange scratch, when the workspace has room for it behind the partial sums
@@ -305,7 +312,7 @@ static int bwd_impl(const void* Q, const void* K, const void* V, const void* dO,
                     const float* LSE, const float* theta, const float* wmix, float* dQ, float* dK, float* dV,
                     float* dTheta, float* dW, int B, int H, int N, int d, int cq, int ck, int G, float scale,
                     int causal, int path, void* workspace, size_t workspace_bytes, void* stream, const void* ktilde,
-                    int row_lo = 0, int row_hi = 0) {
+                    int row_lo = 0, int row_hi = 0, void* const* grads_bf16 = nullptr) {
   TrainParams p = {};
   if (ktilde && !aligned16(ktilde)) return FMTA_ERR_ALIGN;
   if (int s = fill_bwd(p, Q, K, V, dO, D, LSE, theta, wmix, B, H, N, d, cq, ck, G, scale, causal)) return s;
@@ -322,7 +329,9 @@ static int bwd_impl(const void* Q, const void* K, const void* V, const void* dO,
     if (path == 1) return FMTA_ERR_WORKSPACE;
     use_tc = false;
   }
-  p.dQ = dQ; p.dK = dK; p.dV = dV;
+  p.dQ = dQ; p.dK = dK; p.dV = dV;                              // (the band kernel's part when grads_bf16 is given)
+  p.dQo = grads_bf16 ? grads_bf16[0] : dQ; p.dKo = grads_bf16 ? grads_bf16[1] : dK; p.dVo = grads_bf16 ? grads_bf16[2] : dV;
+  p.grad_bf16 = grads_bf16 != nullptr;
   int slots_ex = (!use_tc && hm_dense_supported(p)) ? hm_dq_slots(B, N, p.G) : B * ((N + 63) / 64);
   const size_t n_theta = (size_t)H * p.cq * p.ck;
   if (ktilde && !use_tc) return FMTA_ERR_UNSUPPORTED;   // only the tensor-core path uses the stacked key operand
@@ -342,7 +351,7 @@ static int bwd_impl(const void* Q, const void* K, const void* V, const void* dO,
       if (int s = check_cuda(launch_reduce_partials(p.dW_part, dW, slots_ex, H * G, st))) return s;
     return FMTA_OK;
   }
-  // tensor-core kernels for the entries off the causal band, then the band kernel adds its part
+  // the pre-pass, the band kernel (causal), then the tensor-core kernels for the entries off the band, which add to its part
   p.Kt_ext = reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(ktilde));   // the forward's stacked key operand, kept by the caller
   p.kt_valid = ktilde != nullptr;
   int Nw = N;                                                   // positions this call owns
@@ -350,7 +359,7 @@ static int bwd_impl(const void* Q, const void* K, const void* V, const void* dO,
     if (int s = check_window(row_lo, row_hi, N)) return s;
     p.row_lo = row_lo; p.row_hi = row_hi; Nw = row_hi - row_lo;
   }
-  slots_ex = bwd_band_theta_slots(B, Nw, p.cq, p.ck);           // one dTheta partial per band CTA
+  slots_ex = causal ? bwd_band_theta_slots(B, Nw, p.cq, p.ck) : 0;   // one dTheta partial per band CTA; no causal mask: no band
   const int slots_tc = bwd_tc_theta_slots(B, Nw, d);
   float* part = reinterpret_cast<float*>(workspace);
   const size_t part_bytes = ((size_t)(slots_ex + slots_tc) * n_theta * sizeof(float) + 1023) / 1024 * 1024;
@@ -359,15 +368,13 @@ static int bwd_impl(const void* Q, const void* K, const void* V, const void* dO,
   // memory and the dK/dV kernel streams them instead of recomputing them
   const bool keep_pdc = (d == 64) && row_hi == 0 &&
       workspace_bytes >= fmta_workspace_bytes(FMTA_OP_BWD_TC_STREAM, B, H, N, d, p.cq, p.ck, p.G);
-  if (int s = check_cuda(launch_bwd_dq_tc(p, tcw, keep_pdc, st))) return s;
-  if (int s = check_cuda(launch_bwd_dkdv_tc(p, tcw, part + (size_t)slots_ex * n_theta, keep_pdc, st))) return s;
+  if (int s = check_cuda(launch_bwd_ktilde(p, tcw, st))) return s;
   p.n_slots = slots_ex;
   p.dTheta_part = part;
-  if (causal) {
+  if (causal)
     if (int s = check_cuda(launch_bwd_band(p, st))) return s;
-  } else {   // no causal mask: no band
-    if (int s = check_cuda(cudaMemsetAsync(part, 0, (size_t)slots_ex * n_theta * sizeof(float), st))) return s;
-  }
+  if (int s = check_cuda(launch_bwd_dq_tc(p, tcw, keep_pdc, st))) return s;
+  if (int s = check_cuda(launch_bwd_dkdv_tc(p, tcw, part + (size_t)slots_ex * n_theta, keep_pdc, st))) return s;
   return check_cuda(launch_reduce_partials(part, dTheta, slots_ex + slots_tc, (int)n_theta, st));
 }
 
@@ -386,6 +393,35 @@ int fmta_bwd_with_ktilde(const void* Q, const void* K, const void* V, const void
   if (!ktilde || !theta) return FMTA_ERR_NULL;
   return bwd_impl(Q, K, V, dO, D, LSE, theta, nullptr, dQ, dK, dV, dTheta, nullptr, B, H, N, d, cq, ck, 1, scale, causal, 1,
                   workspace, workspace_bytes, stream, ktilde);
+}
+
+int fmta_bwd_fused(const void* Q, const void* K, const void* V, const void* dO, int do_dtype, const void* O, int o_dtype,
+                   const float* LSE, const float* theta, void* dQ, void* dK, void* dV, int grad_dtype, float* dTheta,
+                   int B, int H, int N, int d, int cq, int ck, float scale, int causal, void* workspace,
+                   size_t workspace_bytes, const void* ktilde, void* stream) {
+  if (!O || !dO || !theta || !dQ || !dK || !dV) return FMTA_ERR_NULL;
+  for (int t : {do_dtype, o_dtype, grad_dtype})
+    if (t != FMTA_DTYPE_F32 && t != FMTA_DTYPE_BF16) return FMTA_ERR_UNSUPPORTED;
+  if (int s = check_train_dims(B, H, N, d, cq, ck, 1, true, false)) return s;
+  if (!aligned16(dO) || !aligned16(O) || !aligned16(dQ) || !aligned16(dK) || !aligned16(dV)) return FMTA_ERR_ALIGN;
+  TrainParams q = {};
+  q.theta = theta; q.d = d; q.cq = cq; q.ck = ck;
+  if (!bwd_tc_supported(q)) return FMTA_ERR_UNSUPPORTED;
+  const size_t base = up1k(fmta_workspace_bytes(FMTA_OP_BWD_TC, B, H, N, d, cq, ck, 1));
+  if (!workspace || workspace_bytes < fmta_workspace_bytes(FMTA_OP_BWD_FUSED, B, H, N, d, cq, ck, 1)) return FMTA_ERR_WORKSPACE;
+  if (!aligned16(workspace)) return FMTA_ERR_ALIGN;
+  const size_t rows = (size_t)B * H * N;
+  unsigned char* w = reinterpret_cast<unsigned char*>(workspace) + base;
+  float* D = reinterpret_cast<float*>(w); w += up1k(rows * 4);
+  __nv_bfloat16* dOb = reinterpret_cast<__nv_bfloat16*>(w); w += up1k(rows * d * 2);
+  float* part[3];
+  for (int i = 0; i < 3; ++i) { part[i] = reinterpret_cast<float*>(w); w += up1k(rows * d * 4); }
+  void* outs[3] = {dQ, dK, dV};
+  const bool g16 = grad_dtype == FMTA_DTYPE_BF16, d32 = do_dtype == FMTA_DTYPE_F32;
+  if (!g16) for (int i = 0; i < 3; ++i) part[i] = reinterpret_cast<float*>(outs[i]);
+  if (int s = check_cuda(launch_rowdot(dO, O, o_dtype == FMTA_DTYPE_BF16, d32 ? dOb : nullptr, D, rows, d, (cudaStream_t)stream))) return s;
+  return bwd_impl(Q, K, V, d32 ? dOb : dO, D, LSE, theta, nullptr, part[0], part[1], part[2], dTheta, nullptr, B, H, N, d, cq,
+                  ck, 1, scale, causal, 1, workspace, base, stream, ktilde, 0, 0, g16 ? outs : nullptr);
 }
 
 int fmta_stacked_keys(const void* K, const float* theta, void* ktilde, int B, int H, int N, int d, int cq, int ck,

@@ -22,9 +22,12 @@ struct TrainParams {
   const float* Opart;        // forward band kernel: un-normalised partial (O, m, l) left by the tensor-core kernel
   const float* Mpart;
   const float* Lpart;
-  float* dQ;                 // backward outputs, fp32
+  float* dQ;                 // backward outputs, fp32.  Tensor-core path: the band kernel's part, written first
   float* dK;
   float* dV;
+  void* dQo;                 // tensor-core path: the final gradients, fp32 (may be dQ / dK / dV) or bf16 (grad_bf16)
+  void* dKo;
+  void* dVo;
   float* dTheta_part;        // [n_slots, H, cq*ck] per-CTA-slot partial sums (reduced later)
   float* dW_part;            // [n_slots, H/G, G*G]
   __nv_bfloat16* Kt_ext;     // tensor-core path: caller-owned stacked key operand [B,H,cq,N,d] instead of the workspace's (nullptr: none)
@@ -36,6 +39,7 @@ struct TrainParams {
   float scale;
   int causal;
   int o_bf16;
+  int grad_bf16;             // tensor-core backward: dQo, dKo, dVo are bf16
   int n_slots;
 };
 

@@ -65,7 +65,6 @@ __global__ void __launch_bounds__(FwdBandCfg<D>::NT, 2) fwd_band_kernel(const Tr
   const int t0 = win_lo(p) + blockIdx.x * R;          // a window starts on a multiple of R
   const int koff = (band > 16) ? 32 : 16;             // the P tile of 16 rows starts koff keys before them
   pdl_trigger();
-  pdl_wait();                                         // launched with programmatic stream serialization
 
   if (band > 0) {
     load_rows_async<D, NT>(sQ, LD, p.Q + bh * (size_t)N * D, t0 - 16, RS, N, tid);
@@ -161,6 +160,9 @@ __global__ void __launch_bounds__(FwdBandCfg<D>::NT, 2) fwd_band_kernel(const Tr
     __syncthreads();
   }
 
+  // Up to here only inputs of the call were read, which were complete before any CTA of the tensor-core kernel let this
+  // one start; its partial is needed from here on
+  pdl_wait();
   // ---- merge with the partial softmax state: one thread per row ----
   if (tid < R) {
     const int gi = t0 + tid;

@@ -241,9 +241,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     tc::tmem_relinquish();
   }
   tc::tc_fence_before();
-  pdl_trigger();
   __syncthreads();
   pdl_wait();      // nothing before this line touches global memory that a kernel of this library writes or reads back
+  pdl_trigger();   // after the wait: the band kernel behind this one reads Q, K, V before it waits for this kernel
   tc::tc_fence_after();
   const uint32_t tmem = *s_tmem;
 

@@ -1,0 +1,339 @@
+// Native host layer: the operators' argument checks, allocations, autograd nodes and calls of the C ABI, without the
+// interpreter in between.  The small problems are bound by the host: a training step of B=1, H=4, N=256 took 230 us in
+// Python (ctypes calls, one torch.empty per buffer, a Python autograd node) against about 50 us of work on the GPU.
+// Only this file sees torch; libfmta_b200.so stays a plain C library.
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/extension.h>
+
+#include <atomic>
+#include <cmath>
+#include <tuple>
+
+#include "../../include/fmta_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+// ---------------------------------------------------------------- checks
+#define FMTA_REQUIRE(cond, ...)                               \
+  do {                                                        \
+    if (!(cond)) throw std::runtime_error(c10::str(__VA_ARGS__)); \
+  } while (0)
+
+void check_status(int st, const char* what) {
+  if (st == 0) return;
+  if (st == FMTA_ERR_CUDA)
+    throw std::runtime_error(c10::str(what, ": ", fmta_strerror(st), " (cudaError ", fmta_last_cuda_error(), ")"));
+  throw std::runtime_error(c10::str(what, ": ", fmta_strerror(st)));
+}
+
+void require_cuda_bf16(const Tensor& t, const char* name) {
+  FMTA_REQUIRE(t.is_cuda(), name, " must be a CUDA tensor");
+  FMTA_REQUIRE(t.is_contiguous(), name, " must be contiguous");
+  FMTA_REQUIRE(t.scalar_type() == at::kBFloat16, name, " must be bfloat16");
+}
+
+void require_on(const Tensor& ref, const Tensor& t, const char* name) {
+  FMTA_REQUIRE(t.is_cuda() && t.device() == ref.device(), name, " must be a CUDA tensor on ", ref.device().str(), " (got ",
+               t.device().str(), ")");
+}
+void require_on(const Tensor& ref, const Tensor& t, const char* name, at::IntArrayRef shape) {
+  require_on(ref, t, name);
+  FMTA_REQUIRE(t.sizes() == shape, name, " must have shape ", shape, " (got ", t.sizes(), ")");
+}
+
+// The status word of a device is created and registered by the Python module on first use.
+std::atomic<bool> g_armed[64];
+void arm_status(const Tensor& t) {
+  const int dev = t.get_device();
+  if (dev >= 0 && dev < 64 && g_armed[dev].load(std::memory_order_acquire)) return;
+  pybind11::gil_scoped_acquire gil;
+  pybind11::module_::import("fmta_b200._lib").attr("arm_status")(t.device());
+  if (dev >= 0 && dev < 64) g_armed[dev].store(true, std::memory_order_release);
+}
+
+void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
+void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+float* fptr(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; }
+
+Tensor f32(const Tensor& t) { return t.scalar_type() == at::kFloat && t.is_contiguous() ? t : t.to(at::kFloat).contiguous(); }
+Tensor bf16c(const Tensor& t) { return t.scalar_type() == at::kBFloat16 && t.is_contiguous() ? t : t.to(at::kBFloat16).contiguous(); }
+Tensor new_f32(const Tensor& like, at::IntArrayRef shape) { return at::empty(shape, like.options().dtype(at::kFloat)); }
+Tensor new_bytes(const Tensor& like, size_t n) { return at::empty({(int64_t)(n < 16 ? 16 : n)}, like.options().dtype(at::kByte)); }
+int dtype_code(at::ScalarType t) { return t == at::kBFloat16 ? FMTA_DTYPE_BF16 : FMTA_DTYPE_F32; }
+bool exact_only() { return fmta_set_path(99) == 0; }
+
+// ---------------------------------------------------------------- conv attention
+struct Dims { int B, H, N, d, cq, ck; };
+Dims conv_dims(const Tensor& Q, const Tensor& theta, int64_t pad_q, int64_t pad_k) {
+  FMTA_REQUIRE(Q.dim() == 4, "Q must have shape [batch, heads, seq, d_head]");
+  Dims s{(int)Q.size(0), (int)Q.size(1), (int)Q.size(2), (int)Q.size(3), 0, 0};
+  FMTA_REQUIRE(theta.dim() == 3 && theta.size(0) == s.H, "conv_kernel must have shape [heads, kx, ky]");
+  s.cq = (int)theta.size(1); s.ck = (int)theta.size(2);
+  FMTA_REQUIRE(pad_q == s.cq - 1 && pad_k == (s.ck - 1) / 2, "pad_q/pad_k must be (kx-1, (ky-1)//2) for a [heads,kx,ky] kernel");
+  return s;
+}
+bool bwd_tc_shape(const Dims& s) { return (s.d == 64 && s.cq <= 7) || (s.d == 128 && s.cq <= 6); }
+
+// O (and LSE, M, L where defined); kt: buffer for the stacked key operand, or undefined.
+void conv_forward_raw(const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& theta, const Tensor& O, const Tensor& M,
+                      const Tensor& L, const Tensor& LSE, const Dims& s, double scale, bool causal, int path, const Tensor& kt) {
+  arm_status(Q);
+  const size_t n = path != 0 ? fmta_workspace_bytes(FMTA_OP_FWD_TC, s.B, s.H, s.N, s.d, s.cq, s.ck, 1) : 0;
+  const Tensor ws = n ? new_bytes(Q, n) : Tensor();
+  if (kt.defined())
+    check_status(fmta_fwd_keep_ktilde(ptr(Q), ptr(K), ptr(V), fptr(theta), ptr(O), fptr(M), fptr(L), fptr(LSE), s.B, s.H, s.N, s.d,
+                                      s.cq, s.ck, (float)scale, causal, dtype_code(O.scalar_type()), ptr(ws), n, ptr(kt), stream_of(Q)),
+                 "fmta_fwd_keep_ktilde");
+  else
+    check_status(fmta_fwd(ptr(Q), ptr(K), ptr(V), fptr(theta), nullptr, ptr(O), fptr(M), fptr(L), fptr(LSE), s.B, s.H, s.N, s.d, s.cq,
+                          s.ck, 1, (float)scale, causal, dtype_code(O.scalar_type()), path, ptr(ws), n, stream_of(Q)),
+                 "fmta_fwd");
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor> conv_forward(const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& theta_, double scale,
+                                                       int64_t pad_q, int64_t pad_k, bool causal, bool out_bf16, bool want_lse,
+                                                       int64_t path, const std::optional<Tensor>& kt) {
+  require_cuda_bf16(Q, "Q"); require_cuda_bf16(K, "K"); require_cuda_bf16(V, "V");
+  const Dims s = conv_dims(Q, theta_, pad_q, pad_k);
+  FMTA_REQUIRE(K.sizes() == Q.sizes() && V.sizes() == Q.sizes(), "Q, K, V must have the same shape [batch, heads, seq, d_head]");
+  require_on(Q, K, "K"); require_on(Q, V, "V"); require_on(Q, theta_, "conv_kernel");
+  c10::cuda::CUDAGuard guard(Q.device());
+  const Tensor theta = f32(theta_);
+  const Tensor O = at::empty(Q.sizes(), Q.options().dtype(out_bf16 ? at::kBFloat16 : at::kFloat));
+  const Tensor M = new_f32(Q, {s.B, s.H, s.N}), L = at::empty_like(M), LSE = want_lse ? at::empty_like(M) : Tensor();
+  conv_forward_raw(Q, K, V, theta, O, M, L, LSE, s, scale, causal, (int)path, kt ? *kt : Tensor());
+  return {O, M, L, LSE};
+}
+
+Tensor rowdot(const Tensor& dO, const Tensor& O) {
+  require_cuda_bf16(dO, "dO");
+  FMTA_REQUIRE((O.scalar_type() == at::kFloat || O.scalar_type() == at::kBFloat16) && O.is_contiguous(), "O must be contiguous fp32 or bf16");
+  require_on(dO, O, "O", dO.sizes());
+  c10::cuda::CUDAGuard guard(dO.device());
+  const Tensor D = new_f32(dO, dO.sizes().slice(0, dO.dim() - 1));
+  check_status(fmta_bwd_prep_D(ptr(dO), ptr(O), dtype_code(O.scalar_type()), fptr(D), D.numel(), (int)dO.size(-1), stream_of(dO)),
+               "fmta_bwd_prep_D");
+  return D;
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor> conv_backward_raw(const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& dO, const Tensor& D,
+                                                            const Tensor& LSE, const Tensor& theta, const Dims& s, double scale, bool causal,
+                                                            int path, int op, const Tensor& kt) {
+  arm_status(Q);
+  const Tensor dQ = new_f32(Q, Q.sizes()), dK = at::empty_like(dQ), dV = at::empty_like(dQ), dT = new_f32(Q, {s.H, s.cq, s.ck});
+  const size_t n = fmta_workspace_bytes(op, s.B, s.H, s.N, s.d, s.cq, s.ck, 1);
+  const Tensor ws = new_bytes(Q, n);
+  if (kt.defined())
+    check_status(fmta_bwd_with_ktilde(ptr(Q), ptr(K), ptr(V), ptr(dO), fptr(D), fptr(LSE), fptr(theta), fptr(dQ), fptr(dK), fptr(dV), fptr(dT),
+                                      s.B, s.H, s.N, s.d, s.cq, s.ck, (float)scale, causal, ptr(ws), n, ptr(kt), stream_of(Q)),
+                 "fmta_bwd_with_ktilde");
+  else
+    check_status(fmta_bwd(ptr(Q), ptr(K), ptr(V), ptr(dO), fptr(D), fptr(LSE), fptr(theta), nullptr, fptr(dQ), fptr(dK), fptr(dV), fptr(dT),
+                          nullptr, s.B, s.H, s.N, s.d, s.cq, s.ck, 1, (float)scale, causal, path, ptr(ws), n, stream_of(Q)),
+                 "fmta_bwd");
+  return {dQ, dK, dV, dT};
+}
+
+// stream: -1 where the P / dC tensors of the streaming dK/dV kernel fit `stream_limit` bytes, 0 never, 1 always
+int conv_backward_op(const Dims& s, int path, int stream, int64_t stream_limit) {
+  if (path == 0) return FMTA_OP_BWD_DQ;
+  if (s.d == 64 && (stream > 0 || (stream < 0 && stream_limit > 0))) {
+    const size_t big = fmta_workspace_bytes(FMTA_OP_BWD_TC_STREAM, s.B, s.H, s.N, s.d, s.cq, s.ck, 1);
+    const size_t base = fmta_workspace_bytes(FMTA_OP_BWD_TC, s.B, s.H, s.N, s.d, s.cq, s.ck, 1);
+    if (stream > 0 || big - base <= (size_t)stream_limit) return FMTA_OP_BWD_TC_STREAM;
+  }
+  return FMTA_OP_BWD_TC;
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor> conv_backward(const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& dO, const Tensor& D,
+                                                        const Tensor& L, const Tensor& theta_, double scale, int64_t pad_q, int64_t pad_k,
+                                                        bool causal, int64_t path, int64_t stream, int64_t stream_limit,
+                                                        const std::optional<Tensor>& kt) {
+  require_cuda_bf16(Q, "Q"); require_cuda_bf16(K, "K"); require_cuda_bf16(V, "V"); require_cuda_bf16(dO, "dO");
+  const Dims s = conv_dims(Q, theta_, pad_q, pad_k);
+  require_on(Q, K, "K", Q.sizes()); require_on(Q, V, "V", Q.sizes()); require_on(Q, dO, "dO", Q.sizes());
+  require_on(Q, D, "D", {s.B, s.H, s.N}); require_on(Q, L, "L (log-sum-exp)", {s.B, s.H, s.N}); require_on(Q, theta_, "conv_kernel");
+  c10::cuda::CUDAGuard guard(Q.device());
+  return conv_backward_raw(Q, K, V, dO, f32(D), f32(L), f32(theta_), s, scale, causal, (int)path,
+                           conv_backward_op(s, (int)path, (int)stream, stream_limit), kt ? *kt : Tensor());
+}
+
+Tensor pad64(const Tensor& t) { return at::constant_pad_nd(t, {0, 32}); }
+Tensor cut32(const Tensor& t) { return t.slice(3, 0, 32).contiguous(); }
+
+// The operator: forward saves what the backward needs, the backward is one call of the library (fmta_bwd_fused) that takes
+// the gradient in the dtype it arrives in and returns the gradients in the inputs' dtypes.
+struct ConvOp {
+  double scale; bool causal, pad; int64_t keep_limit, stream_limit;
+};
+bool wants_pad(const Tensor& Q, const Tensor& theta, bool pad_d32) {
+  return pad_d32 && Q.size(3) == 32 && theta.size(1) <= 7 && !exact_only();
+}
+Tensor conv_run(const ConvOp& op, const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& theta, const Dims& s, const Tensor& LSE,
+                const Tensor& kt) {
+  const Tensor O = new_f32(Q, Q.sizes());
+  conv_forward_raw(Q, K, V, theta, O, Tensor(), Tensor(), LSE, s, op.scale, op.causal, -1, kt);
+  return O;
+}
+
+struct ConvAttnFn : public torch::autograd::Function<ConvAttnFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& theta_, double scale, int64_t pad_q,
+                        int64_t pad_k, bool causal, int64_t keep_limit, int64_t stream_limit, bool pad_d32) {
+    const bool pad = wants_pad(Q, theta_, pad_d32);
+    Tensor q = bf16c(Q), k = bf16c(K), v = bf16c(V);
+    const Tensor theta = f32(theta_);
+    if (pad) { q = pad64(q); k = pad64(k); v = pad64(v); }
+    const Dims s = conv_dims(q, theta, pad_q, pad_k);
+    // The stacked key operand is kept for the backward up to keep_limit bytes (c_q times K): one launch less
+    Tensor kt;
+    if (bwd_tc_shape(s) && !exact_only() && (int64_t)s.B * s.H * s.N * s.d * s.cq * 2 <= keep_limit)
+      kt = at::empty({s.B, s.H, s.cq, s.N, s.d}, q.options());
+    const Tensor LSE = new_f32(q, {s.B, s.H, s.N});
+    const Tensor O = conv_run({scale, causal, pad, keep_limit, stream_limit}, q, k, v, theta, s, LSE, kt);
+    const Tensor out = pad ? cut32(O) : O;
+    ctx->save_for_backward({q, k, v, theta_, LSE, out, kt});
+    ctx->saved_data["scale"] = scale;
+    ctx->saved_data["causal"] = causal;
+    ctx->saved_data["pad"] = pad;
+    ctx->saved_data["stream_limit"] = stream_limit;
+    ctx->saved_data["tq"] = (int64_t)Q.scalar_type(); ctx->saved_data["tk"] = (int64_t)K.scalar_type(); ctx->saved_data["tv"] = (int64_t)V.scalar_type();
+    return out;
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    at::AutoGradMode no_grad(false);
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &theta_ = saved[3], &LSE = saved[4], &kt = saved[6];
+    Tensor O = saved[5], dO = grads[0];
+    const double scale = ctx->saved_data["scale"].toDouble();
+    const bool causal = ctx->saved_data["causal"].toBool(), pad = ctx->saved_data["pad"].toBool();
+    const int64_t stream_limit = ctx->saved_data["stream_limit"].toInt();
+    const at::ScalarType ty[3] = {(at::ScalarType)ctx->saved_data["tq"].toInt(), (at::ScalarType)ctx->saved_data["tk"].toInt(),
+                                  (at::ScalarType)ctx->saved_data["tv"].toInt()};
+    if (!dO.defined()) dO = at::zeros_like(O);
+    c10::cuda::CUDAGuard guard(q.device());
+    const Tensor theta = f32(theta_);
+    const Dims s{(int)q.size(0), (int)q.size(1), (int)q.size(2), (int)q.size(3), (int)theta.size(1), (int)theta.size(2)};
+    if (pad) { O = pad64(O); dO = pad64(dO); }
+    Tensor g[3], dT;
+    const int op = conv_backward_op(s, -1, -1, stream_limit);
+    if (bwd_tc_shape(s) && !exact_only() && op == FMTA_OP_BWD_TC) {
+      arm_status(q);
+      dO = dO.scalar_type() == at::kFloat && dO.is_contiguous() && reinterpret_cast<uintptr_t>(dO.data_ptr()) % 16 == 0 ? dO : bf16c(dO);
+      const bool g16 = ty[0] == at::kBFloat16 && ty[1] == at::kBFloat16 && ty[2] == at::kBFloat16;
+      for (auto& t : g) t = at::empty(q.sizes(), q.options().dtype(g16 ? at::kBFloat16 : at::kFloat));
+      dT = new_f32(q, {s.H, s.cq, s.ck});
+      const size_t n = fmta_workspace_bytes(FMTA_OP_BWD_FUSED, s.B, s.H, s.N, s.d, s.cq, s.ck, 1);
+      const Tensor ws = new_bytes(q, n);
+      check_status(fmta_bwd_fused(ptr(q), ptr(k), ptr(v), ptr(dO), dtype_code(dO.scalar_type()), ptr(O), FMTA_DTYPE_F32, fptr(LSE), fptr(theta),
+                                  ptr(g[0]), ptr(g[1]), ptr(g[2]), g16 ? FMTA_DTYPE_BF16 : FMTA_DTYPE_F32, fptr(dT), s.B, s.H, s.N, s.d, s.cq,
+                                  s.ck, (float)scale, causal, ptr(ws), n, kt.defined() ? ptr(kt) : nullptr, stream_of(q)),
+                   "fmta_bwd_fused");
+    } else {
+      dO = bf16c(dO);
+      std::tie(g[0], g[1], g[2], dT) =
+          conv_backward_raw(q, k, v, dO, rowdot(dO, O), LSE, theta, s, scale, causal, -1, op, kt);
+    }
+    for (int i = 0; i < 3; ++i) g[i] = (pad ? cut32(g[i]) : g[i]).to(ty[i]);
+    return {g[0], g[1], g[2], dT.to(theta_.scalar_type()), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor conv_attention(const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& theta_, double scale, int64_t pad_q, int64_t pad_k,
+                      bool causal, int64_t keep_limit, int64_t stream_limit, bool pad_d32) {
+  FMTA_REQUIRE(Q.is_cuda(), "Q must be a CUDA tensor");
+  conv_dims(Q, theta_, pad_q, pad_k);
+  FMTA_REQUIRE(K.sizes() == Q.sizes() && V.sizes() == Q.sizes(), "Q, K, V must have the same shape [batch, heads, seq, d_head]");
+  require_on(Q, K, "K"); require_on(Q, V, "V"); require_on(Q, theta_, "conv_kernel");
+  c10::cuda::CUDAGuard guard(Q.device());
+  if (at::GradMode::is_enabled() && (Q.requires_grad() || K.requires_grad() || V.requires_grad() || theta_.requires_grad()))
+    return ConvAttnFn::apply(Q, K, V, theta_, scale, pad_q, pad_k, causal, keep_limit, stream_limit, pad_d32);
+  at::AutoGradMode no_grad(false);
+  const bool pad = wants_pad(Q, theta_, pad_d32);
+  Tensor q = bf16c(Q), k = bf16c(K), v = bf16c(V);
+  if (pad) { q = pad64(q); k = pad64(k); v = pad64(v); }
+  const Tensor theta = f32(theta_);
+  const Tensor O = conv_run({scale, causal, pad, 0, 0}, q, k, v, theta, conv_dims(q, theta, pad_q, pad_k), Tensor(), Tensor());
+  return pad ? cut32(O) : O;
+}
+
+// ---------------------------------------------------------------- decode
+struct Splits { Tensor O, M, L; };
+Splits split_outputs(const Tensor& Q, int64_t B, int64_t H, int64_t ks, int64_t d) {   // carved out of one allocation
+  const int64_t n = B * H * ks;
+  const Tensor buf = new_f32(Q, {n * (d + 2)});
+  return {buf.as_strided({B, H, ks, d}, {H * ks * d, ks * d, d, 1}), buf.as_strided({B, H, ks}, {H * ks, ks, 1}, n * d),
+          buf.as_strided({B, H, ks}, {H * ks, ks, 1}, n * (d + 1))};
+}
+
+std::tuple<Tensor, Tensor, Tensor> decode(const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& theta_, int64_t ks, double scale,
+                                          int64_t pad_q, int64_t pad_k, bool offset_causal, bool merged_only) {
+  at::AutoGradMode no_grad(false);
+  require_cuda_bf16(Q, "Q"); require_cuda_bf16(K, "K"); require_cuda_bf16(V, "V");
+  FMTA_REQUIRE(Q.dim() == 4 && K.dim() == 4, "Q and K/V must be [batch, heads, seq, d_head]");
+  const int64_t B = Q.size(0), H = Q.size(1), q_len = Q.size(2), d = Q.size(3);
+  FMTA_REQUIRE(q_len >= 1 && q_len <= 16, "Q sequence length must be between 1 and 16 for inference");
+  FMTA_REQUIRE(K.size(0) == B && K.size(1) == H && K.size(3) == d && V.sizes() == K.sizes(), "K/V must be [batch, heads, seq_len, d_head] matching Q");
+  const int64_t Nk = K.size(2), cq = theta_.size(1), ck = theta_.size(2);
+  FMTA_REQUIRE(pad_q == cq - 1 && pad_k == (ck - 1) / 2, "pad_q/pad_k must be (kx-1, (ky-1)//2)");
+  FMTA_REQUIRE(ks > 0, "k_splits must be positive");
+  FMTA_REQUIRE(ks <= Nk, "k_splits cannot be larger than seq_len_k");
+  c10::cuda::CUDAGuard guard(Q.device());
+  const Tensor theta = f32(theta_);
+  Splits o = split_outputs(Q, B, H, ks, d);
+  check_status((offset_causal ? fmta_decode_offset_causal : fmta_decode)(ptr(Q), ptr(K), ptr(V), fptr(theta), fptr(o.O), fptr(o.M), fptr(o.L), B, H,
+                                                                          q_len, Nk, d, cq, ck, ks, (float)scale, stream_of(Q)),
+               "fmta_decode");
+  if (!merged_only) return {o.O, o.M, o.L};
+  return {o.O.as_strided({B, H, 1, d}, {H * ks * d, ks * d, d, 1}), o.M.as_strided({B, H, 1}, {H * ks, ks, 1}), o.L.as_strided({B, H, 1}, {H * ks, ks, 1})};
+}
+
+std::tuple<Tensor, Tensor, Tensor> decode_paged(const Tensor& Q, const Tensor& Kp, const Tensor& Vp, const Tensor& table, const Tensor& theta_,
+                                                int64_t ks, double scale, int64_t pad_q, int64_t pad_k, const std::optional<Tensor>& lens,
+                                                const std::optional<int64_t>& max_len, bool offset_causal) {
+  at::AutoGradMode no_grad(false);
+  require_cuda_bf16(Q, "Q"); require_cuda_bf16(Kp, "K_pool"); require_cuda_bf16(Vp, "V_pool");
+  FMTA_REQUIRE(Q.dim() == 4, "Q must be [batch, heads, seq, d_head]");
+  const int64_t B = Q.size(0), H = Q.size(1), q_len = Q.size(2), d = Q.size(3);
+  FMTA_REQUIRE(q_len >= 1 && q_len <= 16, "Q sequence length must be between 1 and 16 for inference");
+  FMTA_REQUIRE(Kp.dim() == 4 && Kp.size(1) == H && Kp.size(3) == d && Vp.sizes() == Kp.sizes(), "K_pool/V_pool must be [n_pages, heads, page_size, d_head] matching Q");
+  FMTA_REQUIRE(table.scalar_type() == at::kInt && table.is_cuda() && table.is_contiguous() && table.dim() == 2 && table.size(0) == B,
+               "block_table must be a contiguous CUDA int32 tensor [batch, max_pages]");
+  FMTA_REQUIRE(!lens || (lens->scalar_type() == at::kInt && lens->is_cuda() && lens->numel() == B), "seq_lens must be a CUDA int32 tensor [batch]");
+  const int64_t page = Kp.size(2), max_pages = table.size(1), cq = theta_.size(1), ck = theta_.size(2);
+  const int64_t Nk = max_len ? *max_len : max_pages * page;
+  FMTA_REQUIRE(pad_q == cq - 1 && pad_k == (ck - 1) / 2, "pad_q/pad_k must be (kx-1, (ky-1)//2)");
+  c10::cuda::CUDAGuard guard(Q.device());
+  const Tensor theta = f32(theta_);
+  Splits o = split_outputs(Q, B, H, ks, d);
+  check_status(fmta_decode_paged(ptr(Q), ptr(Kp), ptr(Vp), table.data_ptr<int>(), lens ? lens->data_ptr<int>() : nullptr, fptr(theta), fptr(o.O),
+                                 fptr(o.M), fptr(o.L), B, H, q_len, Nk, d, cq, ck, ks, (float)scale, page, max_pages, offset_causal, stream_of(Q)),
+               "fmta_decode_paged");
+  return {o.O, o.M, o.L};
+}
+
+void kv_append_paged(const Tensor& Kp, const Tensor& Vp, const Tensor& table, const Tensor& lens, const Tensor& Kn, const Tensor& Vn) {
+  require_cuda_bf16(Kp, "K_pool"); require_cuda_bf16(Vp, "V_pool"); require_cuda_bf16(Kn, "K_new"); require_cuda_bf16(Vn, "V_new");
+  FMTA_REQUIRE(Kn.dim() == 4, "K_new must be [batch, heads, n_new, d_head]");
+  c10::cuda::CUDAGuard guard(Kp.device());
+  check_status(fmta_kv_append_paged(ptr(Kp), ptr(Vp), table.data_ptr<int>(), lens.data_ptr<int>(), ptr(Kn), ptr(Vn), Kn.size(0), Kn.size(1),
+                                    Kn.size(2), Kn.size(3), Kp.size(2), table.size(1), stream_of(Kp)),
+               "fmta_kv_append_paged");
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_native, m) {
+  m.def("conv_forward", &conv_forward);
+  m.def("conv_backward", &conv_backward);
+  m.def("conv_attention", &conv_attention);
+  m.def("rowdot", &rowdot);
+  m.def("decode", &decode);
+  m.def("decode_paged", &decode_paged);
+  m.def("kv_append_paged", &kv_append_paged);
+}

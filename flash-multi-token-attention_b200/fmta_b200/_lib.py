@@ -26,6 +26,9 @@ if not os.path.exists(LIB_PATH):
 
 lib = ctypes.CDLL(LIB_PATH)
 
+if not os.path.exists(os.path.join(_HERE, "_native.so")):
+    raise ImportError("fmta_b200: _native.so is missing beside %s; build it with the same command." % LIB_PATH)
+
 _vp, _fp, _i, _f, _sz = ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_size_t
 
 lib.fmta_version.restype = _i
@@ -83,7 +86,11 @@ lib.fmta_set_status_word.argtypes = [_vp]
 lib.fmta_selftest_expire_next.restype = _i
 lib.fmta_selftest_expire_next.argtypes = [_i]
 
-EXPORTS = ["fmta_set_status_word", "fmta_selftest_expire_next", "fmta_version", "fmta_strerror", "fmta_last_cuda_error", "fmta_workspace_bytes", "fmta_fwd",
+lib.fmta_bwd_fused.restype = _i
+lib.fmta_bwd_fused.argtypes = [_vp, _vp, _vp, _vp, _i, _vp, _i, _fp, _fp, _vp, _vp, _vp, _i, _fp, _i, _i, _i, _i, _i, _i, _f, _i,
+                               _vp, _sz, _vp, _vp]
+
+EXPORTS = ["fmta_bwd_fused", "fmta_set_status_word", "fmta_selftest_expire_next", "fmta_version", "fmta_strerror", "fmta_last_cuda_error", "fmta_workspace_bytes", "fmta_fwd",
            "fmta_bwd_prep_D", "fmta_bwd", "fmta_fwd_keep_ktilde", "fmta_bwd_with_ktilde", "fmta_fwd_window", "fmta_bwd_window", "fmta_stacked_keys", "fmta_set_path", "fmta_profile_kernel", "fmta_bwd_dq_dw", "fmta_bwd_dq_dw_static", "fmta_bwd_dkdv", "fmta_decode", "fmta_decode_offset_causal", "fmta_decode_paged", "fmta_kv_append_paged"]
 
 

@@ -15,7 +15,7 @@ import os
 import torch
 import torch.nn as nn
 
-from . import _lib
+from . import _lib, _native
 from ._lib import lib, check, ptr, stream_ptr, require_cuda_bf16, as_f32, require_on, arm_status
 
 
@@ -53,7 +53,10 @@ def _pad64(t):
 # writes; forward and backward each run it.  A training step can keep the forward's copy for the backward
 # (c_q times the size of K for as long as the graph lives; about 2 % of a step at B=4, H=16, N=4096, d=64):
 # `ktilde_buffer` + the ``ktilde`` argument of `forward` / `backward`, or FMTA_KEEP_KTILDE=1 for the autograd Function.
+# The Function keeps it by itself up to KEEP_KTILDE_BYTES: there the pre-pass costs what its launch costs, and a layer holds
+# no more than that much longer.
 KEEP_KTILDE = os.environ.get("FMTA_KEEP_KTILDE", "0") != "0"
+KEEP_KTILDE_BYTES = 16 << 20
 
 
 def ktilde_buffer(Q, conv_kernel):
@@ -81,51 +84,21 @@ def forward(Q, K, V, conv_kernel, scale, pad_q, pad_k, causal, out_dtype=torch.f
     """(O, M, L) -- `forward` of conv_attn/bindings.cpp:46-48.  O is fp32 as in
     fwd_wrapper.cu:44-46 unless ``out_dtype=torch.bfloat16``; ``return_lse`` appends M+log L.
     ``ktilde`` (from `ktilde_buffer`): the stacked key operand is left there for `backward`."""
-    for t, n in ((Q, "Q"), (K, "K"), (V, "V")):
-        require_cuda_bf16(t, n)
-    B, H, N, d, cq, ck = _dims(Q, conv_kernel, pad_q, pad_k)
-    if K.shape != Q.shape or V.shape != Q.shape:
-        raise RuntimeError("Q, K, V must have the same shape [batch, heads, seq, d_head]")
     if ktilde is not None:
-        _check_ktilde(ktilde, Q, cq, path)
-    elif _pads_to_64(d, cq, path):
+        _check_ktilde(ktilde, Q, conv_kernel.shape[1], path)
+    elif Q.dim() == 4 and _pads_to_64(Q.shape[3], conv_kernel.shape[1], path):
+        for t, n in ((Q, "Q"), (K, "K"), (V, "V")):
+            require_cuda_bf16(t, n)
         out = forward(_pad64(Q), _pad64(K), _pad64(V), conv_kernel, scale, pad_q, pad_k, causal, out_dtype, return_lse, path)
         return (out[0][..., :32].contiguous(),) + tuple(out[1:])
-    require_on(Q, K, "K"); require_on(Q, V, "V"); require_on(Q, conv_kernel, "conv_kernel")
-    arm_status(Q.device)
-    theta = as_f32(conv_kernel)
-    O = torch.empty((B, H, N, d), dtype=out_dtype, device=Q.device)
-    M = torch.empty((B, H, N), dtype=torch.float32, device=Q.device)
-    L = torch.empty_like(M)
-    LSE = torch.empty_like(M) if return_lse else None
-    ws_bytes = lib.fmta_workspace_bytes(_lib.FMTA_OP_FWD_TC, B, H, N, d, cq, ck, 1) if path != 0 else 0
-    ws = _workspace(ws_bytes, Q.device) if ws_bytes else None
-    odt = _lib.FMTA_DTYPE_BF16 if out_dtype == torch.bfloat16 else _lib.FMTA_DTYPE_F32
-    if ktilde is not None:
-        st = lib.fmta_fwd_keep_ktilde(ptr(Q), ptr(K), ptr(V), ptr(theta), ptr(O), ptr(M), ptr(L), ptr(LSE), B, H, N, d,
-                                      cq, ck, float(scale), int(bool(causal)), odt, ptr(ws), ws_bytes, ptr(ktilde),
-                                      stream_ptr())
-        check(st, "fmta_fwd_keep_ktilde")
-        return (O, M, L, LSE) if return_lse else (O, M, L)
-    st = lib.fmta_fwd(ptr(Q), ptr(K), ptr(V), ptr(theta), None, ptr(O), ptr(M), ptr(L), ptr(LSE), B, H, N, d,
-                      cq, ck, 1, float(scale), int(bool(causal)),
-                      _lib.FMTA_DTYPE_BF16 if out_dtype == torch.bfloat16 else _lib.FMTA_DTYPE_F32,
-                      int(path), ptr(ws), ws_bytes, stream_ptr())
-    check(st, "fmta_fwd")
-    return (O, M, L, LSE) if return_lse else (O, M, L)
+    out = _native.conv_forward(Q, K, V, conv_kernel, scale, pad_q, pad_k, bool(causal), out_dtype == torch.bfloat16,
+                               bool(return_lse), path, ktilde)
+    return out if return_lse else out[:3]
 
 
 def rowdot(dO, O):
     """D = rowsum(dO * O) in fp32 (conv_attention_cuda.py:144 without the bf16 rounding)."""
-    require_cuda_bf16(dO, "dO")
-    if O.dtype not in (torch.float32, torch.bfloat16) or not O.is_contiguous():
-        raise RuntimeError("O must be contiguous fp32 or bf16")
-    require_on(dO, O, "O", dO.shape)
-    D = torch.empty(dO.shape[:-1], dtype=torch.float32, device=dO.device)
-    st = lib.fmta_bwd_prep_D(ptr(dO), ptr(O), 1 if O.dtype == torch.bfloat16 else 0, ptr(D),
-                             D.numel(), dO.shape[-1], stream_ptr())
-    check(st, "fmta_bwd_prep_D")
-    return D
+    return _native.rowdot(dO, O)
 
 
 def _check_bwd_args(Q, K, V, dO, D, L, conv_kernel):
@@ -186,66 +159,26 @@ def backward(Q, K, V, dO, D, L, conv_kernel, scale, pad_q, pad_k, causal, path=-
     0 exact kernels, 1 tensor-core kernels + band kernel, -1 library default.  ``stream_pdc``: let the dQ
     kernel keep P and dC for a streaming dK/dV kernel (None: whenever they fit STREAM_LIMIT_BYTES).
     ``ktilde``: the buffer `forward` filled for the same K, conv_kernel and scale; its pre-pass is then skipped."""
-    for t, n in ((Q, "Q"), (K, "K"), (V, "V"), (dO, "dO")):
-        require_cuda_bf16(t, n)
-    B, H, N, d, cq, ck = _dims(Q, conv_kernel, pad_q, pad_k)
-    _check_bwd_args(Q, K, V, dO, D, L, conv_kernel)
     if ktilde is not None:
-        _check_ktilde(ktilde, Q, cq, path)
-    elif _pads_to_64(d, cq, path):
+        _check_ktilde(ktilde, Q, conv_kernel.shape[1], path)
+    elif Q.dim() == 4 and _pads_to_64(Q.shape[3], conv_kernel.shape[1], path):
+        for t, n in ((Q, "Q"), (K, "K"), (V, "V"), (dO, "dO")):
+            require_cuda_bf16(t, n)
         dQ, dK, dV, dTheta = backward(_pad64(Q), _pad64(K), _pad64(V), _pad64(dO), D, L, conv_kernel, scale, pad_q, pad_k,
                                       causal, path, stream_pdc)
         return dQ[..., :32].contiguous(), dK[..., :32].contiguous(), dV[..., :32].contiguous(), dTheta
-    theta, Dv, LSE = as_f32(conv_kernel), as_f32(D), as_f32(L)
-    dQ = torch.empty((B, H, N, d), dtype=torch.float32, device=Q.device)
-    dK = torch.empty_like(dQ)
-    dV = torch.empty_like(dQ)
-    dTheta = torch.empty((H, cq, ck), dtype=torch.float32, device=Q.device)
-    op = _lib.FMTA_OP_BWD_DQ if path == 0 else _lib.FMTA_OP_BWD_TC
-    if path != 0 and d == 64 and stream_pdc is not False:
-        big = lib.fmta_workspace_bytes(_lib.FMTA_OP_BWD_TC_STREAM, B, H, N, d, cq, ck, 1)
-        base = lib.fmta_workspace_bytes(_lib.FMTA_OP_BWD_TC, B, H, N, d, cq, ck, 1)
-        if stream_pdc or big - base <= STREAM_LIMIT_BYTES:
-            op = _lib.FMTA_OP_BWD_TC_STREAM
-    ws_bytes = lib.fmta_workspace_bytes(op, B, H, N, d, cq, ck, 1)
-    ws = _workspace(ws_bytes, Q.device)
-    if ktilde is not None:
-        st = lib.fmta_bwd_with_ktilde(ptr(Q), ptr(K), ptr(V), ptr(dO), ptr(Dv), ptr(LSE), ptr(theta), ptr(dQ), ptr(dK),
-                                      ptr(dV), ptr(dTheta), B, H, N, d, cq, ck, float(scale), int(bool(causal)), ptr(ws),
-                                      ws_bytes, ptr(ktilde), stream_ptr())
-        check(st, "fmta_bwd_with_ktilde")
-        return dQ, dK, dV, dTheta
-    st = lib.fmta_bwd(ptr(Q), ptr(K), ptr(V), ptr(dO), ptr(Dv), ptr(LSE), ptr(theta), None, ptr(dQ), ptr(dK), ptr(dV),
-                      ptr(dTheta), None, B, H, N, d, cq, ck, 1, float(scale), int(bool(causal)), int(path), ptr(ws),
-                      ws_bytes, stream_ptr())
-    check(st, "fmta_bwd")
-    return dQ, dK, dV, dTheta
+    return _native.conv_backward(Q, K, V, dO, D, L, conv_kernel, scale, pad_q, pad_k, bool(causal), path,
+                                 -1 if stream_pdc is None else int(bool(stream_pdc)), STREAM_LIMIT_BYTES, ktilde)
 
 
 class FlashConvAttentionCUDAFunction(torch.autograd.Function):
-    """autograd.Function with the argument list of conv_attention_cuda.py:96-163."""
+    """The operator of conv_attention_cuda.py:96-163: same argument list of ``apply``.  Its autograd node is native
+    (csrc_torch/fmta_torch.cpp), so ``apply`` goes there directly."""
 
     @staticmethod
-    def forward(ctx, Q, K, V, conv_kernel, scale, pad_q, pad_k, causal):
-        Qb, Kb, Vb = (t.to(torch.bfloat16).contiguous() for t in (Q, K, V))
-        needs_grad = any(t.requires_grad for t in (Q, K, V, conv_kernel))
-        ctx.ktilde = ktilde_buffer(Qb, conv_kernel) if (KEEP_KTILDE and needs_grad) else None
-        O, M, L, LSE = forward(Qb, Kb, Vb, conv_kernel, scale, pad_q, pad_k, causal, return_lse=True, ktilde=ctx.ktilde)
-        ctx.save_for_backward(Qb, Kb, Vb, conv_kernel, LSE, O)
-        ctx.scale, ctx.pad_q, ctx.pad_k, ctx.causal = scale, pad_q, pad_k, causal
-        ctx.in_dtypes = (Q.dtype, K.dtype, V.dtype)
-        return O
-
-    @staticmethod
-    def backward(ctx, dO):
-        Q, K, V, conv_kernel, LSE, O = ctx.saved_tensors
-        dOb = dO.to(torch.bfloat16).contiguous()
-        D = rowdot(dOb, O)
-        dQ, dK, dV, dTheta = backward(Q, K, V, dOb, D, LSE, conv_kernel, ctx.scale, ctx.pad_q, ctx.pad_k, ctx.causal,
-                                      ktilde=ctx.ktilde)
-        ctx.ktilde = None
-        tq, tk, tv = ctx.in_dtypes
-        return dQ.to(tq), dK.to(tk), dV.to(tv), dTheta.to(conv_kernel.dtype), None, None, None, None
+    def apply(Q, K, V, conv_kernel, scale, pad_q, pad_k, causal):
+        return _native.conv_attention(Q, K, V, conv_kernel, scale, pad_q, pad_k, bool(causal),
+                                      1 << 62 if KEEP_KTILDE else KEEP_KTILDE_BYTES, STREAM_LIMIT_BYTES, PAD_D32)
 
 
 class ConvAttentionCUDA(nn.Module):

@@ -60,6 +60,7 @@ extern "C" {
  * shared memory.  fmta_fwd: a workspace of this size; fmta_bwd_dq_dw and fmta_bwd (path 0): this size behind the
  * FMTA_OP_BWD_DQ bytes rounded up to 256.  A smaller workspace is not an error. */
 #define FMTA_OP_MIX_EXCHANGE 5
+#define FMTA_OP_BWD_FUSED 6      /* fmta_bwd_fused */
 
 /* Library version (major*10000 + minor*100 + patch). */
 int fmta_version(void);
@@ -195,6 +196,19 @@ int fmta_bwd_with_ktilde(const void* Q, const void* K, const void* V, const void
                          const float* LSE, const float* theta, float* dQ, float* dK, float* dV, float* dTheta,
                          int B, int H, int N, int d, int cq, int ck, float scale, int causal, void* workspace,
                          size_t workspace_bytes, const void* ktilde, void* stream);
+
+/*
+ * The backward of the autograd operator in one call: D = rowsum(dO * O) and the rounding of an fp32 dO to bf16 in one pass,
+ * then fmta_bwd (path 1) with the gradients stored in `grad_dtype` by the kernels that finish them.  Replaces
+ * `FlashConvAttentionCUDAFunction.backward` (conv_attn/conv_attention_cuda.py:132-163) as a whole.
+ *   dO, O: do_dtype / o_dtype (FMTA_DTYPE_F32 or FMTA_DTYPE_BF16)     dQ, dK, dV: grad_dtype
+ *   ktilde: NULL, or the operand fmta_fwd_keep_ktilde left for these K, theta and scale
+ * Tensor-core shapes only (those of fmta_bwd with path = 1); workspace: FMTA_OP_BWD_FUSED.
+ */
+int fmta_bwd_fused(const void* Q, const void* K, const void* V, const void* dO, int do_dtype, const void* O, int o_dtype,
+                   const float* LSE, const float* theta, void* dQ, void* dK, void* dV, int grad_dtype, float* dTheta,
+                   int B, int H, int N, int d, int cq, int ck, float scale, int causal, void* workspace,
+                   size_t workspace_bytes, const void* ktilde, void* stream);
 
 /*
  * One window of sequence positions of a forward / backward (no counterpart in the reference, which has no
