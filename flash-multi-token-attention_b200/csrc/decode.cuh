@@ -1,26 +1,36 @@
 // Decode (fwd_inference) kernel: last-query-row conv attention over a KV cache, split-K.
 //
-// Memory-bound: K and V are each read once from HBM with 16-byte loads straight into
-// registers (no shared-memory staging, no block-level barrier in the key loop).  Every warp
-// owns a contiguous key range of its split and keeps its own online-softmax state:
-//   per 16-key step   S_a[j] = scale * q_a . k_j   for the <=16 most recent query rows   (mma.sync)
-//                     -> fp32 ring buffer in shared memory (per warp, 64 keys deep)
-//   one step later    C[j]  = sum_{a,b} theta[a,b] S_a[j+b-pad_k]   (needs +-pad_k neighbours)
-//                     p = exp(C - m), O += p V                                        (FP32 pipe)
-// The MMA contraction index is permuted so that each lane's B fragment is one contiguous
-// 16-byte piece of a K row (A = Q is laid out to match once, in registers).
-// Warps are merged in shared memory, splits by combine_splits_kernel on the same stream
-// (result normalised into split 0, as the reference leaves it).  With `offset_causal` the score of
-// a key later than a query row's own position is zeroed before the conv, as in the training
-// forward, so that the result equals the last row of the training forward over the same sequence.
+// Memory-bound: K and V are each read once from HBM with 16-byte loads straight into registers (no shared-memory
+// staging, no block-level barrier in the key loop).  Every warp owns a contiguous key range of its split and keeps its own
+// online-softmax state; a step is 32 keys:
+//   S_a[j] = scale * q_a . k_j for the <= 16 most recent query rows                                   (mma.sync)
+//            -> fp32 ring buffer in shared memory (per warp, 64 keys deep)
+//   C[j]  = sum_{a,b} theta[a,b] S_a[j+b-pad_k] of the step before, once the first half of this step's scores is there
+//            (FP32 pipe; lane = 4 keys x 2 or 4 rows: a window of float4 loads and the filter in registers)
+//   p = exp(C - m), O += p V                                                                          (mma.sync)
+// The GPU runs this at its power limit (B=32, H=32, Nk=32768, d=128: 990 W, 1.69 GHz), where every instruction costs
+// bandwidth: with the conv as one load pair per FMA and P V as FMAs on widened values (~1000 instructions per 32 keys) the
+// kernel sustained 5.56 TB/s; a plain read sustains 7.2.
+// Both products take K and V as the 16-row A operand, as they lie in global memory.  K: rows are keys and the contraction
+// index is permuted, so that a lane's fragment is one contiguous 16-byte piece of a K row (Q, the 8-column B operand, is laid
+// out to match once, in registers).  V: rows are head dims; a lane holds 16 bytes (8 dims) of 4 keys per MMA step, and a
+// fragment register is two halfwords of neighbouring keys (one PRMT).  p stays fp32: columns 0, 1, 2 of the B operand are its
+// bf16 parts hi, mid, lo (24 bits), whose products with V are exact; the three accumulator columns are added at the end.
+// Warps are merged in shared memory, sub-splits (and, for small problems, the splits) inside a thread-block cluster, splits
+// otherwise by combine_splits_kernel (result normalised into split 0, as the reference leaves it).  With `offset_causal` the
+// score of a key later than a query row's own position is zeroed before the conv, as in the training forward, so that the
+// result equals the last row of the training forward over the same sequence.
 #pragma once
+#include <cooperative_groups.h>
+
 #include "fmta_common.cuh"
 #include "fmta_params.h"
 
 namespace fmta {
 
 constexpr int kDecWarps = 4;
-constexpr int kDecRing = 64;   // keys kept per warp for the conv window
+constexpr int kDecRing = 64;         // keys kept per warp for the conv window
+constexpr int kDecRow = 68;          // ring row stride in floats: even rows 8 banks apart (no conflicts, stores or window loads)
 constexpr int kDecMaxPages = 2048;   // block-table entries of one sequence kept in shared memory (paged cache)
 
 FMTA_DEVINL uint4 ldg_nc_v4(const void* p) {
@@ -30,200 +40,245 @@ FMTA_DEVINL uint4 ldg_nc_v4(const void* p) {
                : "l"(p));
   return v;
 }
-FMTA_DEVINL float bf_lo(uint32_t x) { return __uint_as_float(x << 16); }
-FMTA_DEVINL float bf_hi(uint32_t x) { return __uint_as_float(x & 0xffff0000u); }
-
 // keys handled by one split, a multiple of 16 * kDecWarps
 __host__ __device__ inline int decode_keys_per_split(int Nk, int k_splits) {
   const int per = (Nk + k_splits - 1) / k_splits;
   return ((per + 16 * kDecWarps - 1) / (16 * kDecWarps)) * (16 * kDecWarps);
 }
 
-template <int D, bool R16, bool PAGED>
-__global__ void __launch_bounds__(kDecWarps * 32, 4) decode_kernel(const DecodeParams p) {
-  constexpr int KS = D / 16;       // k-steps of the MMA
-  constexpr int CH = D / 32;       // 32-element chunks per row (one 16-byte load per lane each)
-  constexpr int LPR = D / 8;       // lanes covering one V row with 16-byte loads
-  constexpr int KPL = 32 / LPR;    // V rows fetched by one warp-wide load
-  constexpr int VL = 16 / KPL;     // V loads per 16-key step
-  __shared__ float sRing[kDecWarps][16][kDecRing];
-  __shared__ float sTheta[16 * 20];
+// NR: query rows per lane in the conv (2t, 2t + 1 and, from 9 rows on, 8 + those): 2 or 4.  CKP: filter width the taps are padded
+// to with zeros (9: pad_k <= 4, 11: pad_k = 5, 17: any).
+template <int D, int NR, int CKP, bool PAGED>
+__global__ void __launch_bounds__(kDecWarps * 32, D == 128 ? 3 : 4) decode_kernel(const DecodeParams p) {
+  constexpr int KS = D / 16;               // k-steps of the QK MMA
+  constexpr int CH = D / 32;               // 32-element chunks per K row (one 16-byte load per lane each)
+  constexpr bool R16 = NR > 2;
+  constexpr int PKP = (CKP - 1) / 2, WC = (CKP <= 9) ? 3 : 5, W0 = 4 * ((WC - 1) / 2);   // conv window: WC float4 from 4g - W0 on
+  constexpr bool THREG = NR * CKP <= 24;   // the lane's filter rows fit registers
+  constexpr int VH = D >= 64 ? D / 64 : 1; // 64-column halves of a V row
+  __shared__ __align__(16) float sRing[kDecWarps][R16 ? 16 : 8][kDecRow];
+  __shared__ __align__(16) float sTheta[16][20];
+  __shared__ __align__(16) bf16 sPs[kDecWarps][4][32];     // hi, mid, lo of the step's probabilities, and a zero row
   __shared__ float sMergeO[kDecWarps][D];
   __shared__ float sMergeML[kDecWarps][2];
+  __shared__ float sPartO[D];              // the CTA's partial, read by the other CTAs of the cluster
+  __shared__ float sPartML[2];
   __shared__ int sTable[PAGED ? kDecMaxPages : 1];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int split = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int nsub = p.n_sub;
+  const int split = blockIdx.x / nsub, sub = blockIdx.x - split * nsub, h = blockIdx.y, b = blockIdx.z;
+  const int cq = p.cq, ck = p.ck, pk = (ck - 1) / 2;
+  const int rows = min(p.q_len, cq);          // query rows that the last output row sees
+  for (int i = tid; i < 16 * 20; i += kDecWarps * 32) (&sTheta[0][0])[i] = 0.f;
+  if (tid < kDecWarps * 32) reinterpret_cast<uint2*>(&sPs[0][0][0])[tid] = make_uint2(0u, 0u);
+  pdl_wait();
+  pdl_trigger();
   // a per-sequence length comes from device memory the caller may have left stale: clamp it to the range the
   // block table (and the shared-memory copy of its row) was sized for
   const int Nk = (PAGED && p.seq_lens) ? min(max(p.seq_lens[b], 1), p.Nk) : p.Nk;
-  const int cq = p.cq, ck = p.ck, pk = (ck - 1) / 2;
-  const int rows = min(p.q_len, cq);          // query rows that the last output row sees
   const size_t bh = (size_t)b * p.H + h;
-  const bf16* Kg = PAGED ? p.K : p.K + bh * (size_t)Nk * D;
-  const bf16* Vg = PAGED ? p.V : p.V + bh * (size_t)Nk * D;
-  // A 16-key step never straddles a page (pages hold a multiple of 16 keys), so the page lookup is
-  // done once per step: step_base(kb) is the element offset of key (kb rounded down to its page),
-  // and a key's row follows at (key - that) * D.
-  const int page_mask = PAGED ? p.page_size - 1 : 0;
-  auto step_base = [&](int kb) -> size_t {
+  // A 16-key tile never straddles a page (pages hold a multiple of 16 keys), so the page lookup is done once per tile:
+  // tile_base(kb) is the address of key kb (a multiple of 16, clamped to the cache).
+  auto tile_base = [&](const bf16* base, int kb) -> const bf16* {
     if (PAGED) {
-      const int pg = max(kb, 0) >> p.page_shift;
-      return ((size_t)sTable[pg] * p.H + h) * p.page_size * D;
+      const int k = min(max(kb, 0), (Nk - 1) & ~15);
+      return base + (((size_t)sTable[k >> p.page_shift] * p.H + h) * p.page_size + (k & (p.page_size - 1))) * D;
     }
-    return 0;
+    return base + (bh * (size_t)Nk + max(kb, 0)) * D;
   };
-  auto row_in = [&](int key) -> size_t { return PAGED ? (size_t)(key & page_mask) * D : (size_t)key * D; };
   if (PAGED) {
     const int npg = (Nk + p.page_size - 1) >> p.page_shift;
     for (int i = tid; i < npg; i += kDecWarps * 32) sTable[i] = p.block_table[(size_t)b * p.max_pages + i];
   }
   const bf16* Qg = p.Q + (bh * p.q_len + (p.q_len - rows)) * (size_t)D;
-
-  // theta rows that see a real query row: tap a = cq - rows + r  <->  ring row r
+  __syncthreads();
+  // theta rows that see a real query row: tap a = cq - rows + r  <->  ring row r; centred in CKP columns
   for (int i = tid; i < rows * ck; i += kDecWarps * 32)
-    sTheta[(i / ck) * 20 + (i % ck)] = p.theta[((size_t)h * cq + (cq - rows) + i / ck) * ck + (i % ck)];
-  for (int i = tid; i < kDecWarps * 16 * kDecRing; i += kDecWarps * 32) (&sRing[0][0][0])[i] = 0.f;
+    sTheta[i / ck][i % ck + PKP - pk] = p.theta[((size_t)h * cq + (cq - rows) + i / ck) * ck + (i % ck)];
 
-  // A fragments of Q in the permuted-k layout (rows >= `rows` are zero)
+  // B fragments of Q (column = query row) in the permuted-k layout (rows >= `rows` are zero)
   uint32_t qa[KS][R16 ? 4 : 2];
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
-    uint2 lo = make_uint2(0u, 0u), lo2 = lo, hi = lo, hi2 = lo;
-    if (g < rows) {
-      const uint4 v = *reinterpret_cast<const uint4*>(Qg + (size_t)g * D + c * 32 + t * 8);
-      lo = make_uint2(v.x, v.y); lo2 = make_uint2(v.z, v.w);
-    }
-    if (R16 && g + 8 < rows) {
-      const uint4 v = *reinterpret_cast<const uint4*>(Qg + (size_t)(g + 8) * D + c * 32 + t * 8);
-      hi = make_uint2(v.x, v.y); hi2 = make_uint2(v.z, v.w);
-    }
-    if (R16) {
-      qa[2 * c][0] = lo.x; qa[2 * c][1] = hi.x; qa[2 * c][2] = lo.y; qa[2 * c][3] = hi.y;
-      qa[2 * c + 1][0] = lo2.x; qa[2 * c + 1][1] = hi2.x; qa[2 * c + 1][2] = lo2.y; qa[2 * c + 1][3] = hi2.y;
-    } else {
-      qa[2 * c][0] = lo.x; qa[2 * c][1] = lo.y;
-      qa[2 * c + 1][0] = lo2.x; qa[2 * c + 1][1] = lo2.y;
+    uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
+    if (g < rows) lo = *reinterpret_cast<const uint4*>(Qg + (size_t)g * D + c * 32 + t * 8);
+    if (R16 && g + 8 < rows) hi = *reinterpret_cast<const uint4*>(Qg + (size_t)(g + 8) * D + c * 32 + t * 8);
+    qa[2 * c][0] = lo.x; qa[2 * c][1] = lo.y;
+    qa[2 * c + 1][0] = lo.z; qa[2 * c + 1][1] = lo.w;
+    if constexpr (R16) {
+      qa[2 * c][2] = hi.x; qa[2 * c][3] = hi.y;
+      qa[2 * c + 1][2] = hi.z; qa[2 * c + 1][3] = hi.w;
     }
   }
   __syncthreads();
-
-  const int keys_per_split = decode_keys_per_split(Nk, p.k_splits);   // (per sequence when lengths differ)
-  const int keys_per_warp = keys_per_split / kDecWarps;
-  const int k_lo = split * keys_per_split + warp * keys_per_warp;
-  const int k_hi = min(k_lo + keys_per_warp, ((Nk + 15) / 16) * 16);
-
-  float m_run = -INFINITY, l_run = 0.f;
-  float o[8];
+  auto row_of = [&](int r) { return 2 * t + (r & 1) + 8 * (r >> 1); };   // the lane's conv rows
+  float th[THREG ? NR : 1][THREG ? CKP : 1];
+  if constexpr (THREG) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) o[i] = 0.f;
+    for (int r = 0; r < NR; ++r)
+#pragma unroll
+      for (int i = 0; i < CKP; ++i) th[r][i] = sTheta[row_of(r)][i];
+  }
+
+  // ---- key range of this warp: 32-key blocks from k_lo (a multiple of 16) on ----
+  const int kps = decode_keys_per_split(Nk, p.k_splits);   // (per sequence when lengths differ)
+  const int kpc = ((kps + nsub - 1) / nsub + 63) / 64 * 64; // keys per CTA
+  const int kpw = (kpc / kDecWarps + 31) / 32 * 32;
+  const int c_lo = split * kps + sub * kpc, c_hi = min(min(c_lo + kpc, (split + 1) * kps), Nk);
+  const int k_lo = c_lo + warp * kpw, k_hi = min(k_lo + kpw, c_hi);
+  const int nblk = k_hi > k_lo ? (k_hi - k_lo + 31) / 32 : 0;
+
+  float m_run = -INFINITY, l_lane = 0.f;                     // l_lane: this lane's share of the sum
+  float o[VH][4][4];                                         // [64-dim half][dims 2w, 2w + 1 of the lane's 8][..]
+#pragma unroll
+  for (int i = 0; i < VH * 16; ++i) (&o[0][0][0])[i] = 0.f;
   float* ring = &sRing[warp][0][0];
-  const int vrow = lane / LPR, vcol = (lane % LPR) * 8;
-  const int ckey = lane & 15, chalf = lane >> 4;
-  const int ra = chalf ? (rows + 1) / 2 : 0, rb = chalf ? rows : (rows + 1) / 2;
+  bf16* ps = &sPs[warp][0][0];
+  uint4 kf[2][CH], vf[VH][4];
 
-  if (k_lo < k_hi) {
-    for (int kb = k_lo - 16; kb <= k_hi; kb += 16) {
-      // ---- issue loads: K block [kb, kb+16), V block [kb-16, kb) ----
-      uint4 kf[2][CH];
-      const bf16* Kst = Kg + step_base(kb);
+  auto load_k = [&](int kb) {                                // the 16-key tile at kb
+    const bf16* src = tile_base(p.K, kb) + g * D + t * 8;
+    const int lim = Nk - kb;                                 // rows of the tile inside the cache
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int key = kb + 8 * j + g;
-        const bool ok = key >= 0 && key < Nk;
+    for (int j = 0; j < 2; ++j) {
+      const bool ok = kb >= 0 && 8 * j + g < lim;
 #pragma unroll
-        for (int c = 0; c < CH; ++c)
-          kf[j][c] = ok ? ldg_nc_v4(Kst + row_in(key) + c * 32 + t * 8) : make_uint4(0u, 0u, 0u, 0u);
-      }
-      const bool do_pv = (kb - 16 >= k_lo);
-      uint4 vf[VL];
-      if (do_pv) {
-        const bf16* Vst = Vg + step_base(kb - 16);
-#pragma unroll
-        for (int i = 0; i < VL; ++i) {
-          const int key = kb - 16 + i * KPL + vrow;
-          vf[i] = (key < Nk) ? ldg_nc_v4(Vst + row_in(key) + vcol) : make_uint4(0u, 0u, 0u, 0u);
-        }
-      }
-      // ---- S for the K block -> ring ----
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int c = 0; c < CH; ++c) {
-          if (R16) {
-            const uint32_t a0[4] = {qa[2 * c][0], qa[2 * c][1], qa[2 * c][2], qa[2 * c][3]};
-            const uint32_t a1[4] = {qa[2 * c + 1][0], qa[2 * c + 1][1], qa[2 * c + 1][2], qa[2 * c + 1][3]};
-            mma_bf16(acc, a0, kf[j][c].x, kf[j][c].y);
-            mma_bf16(acc, a1, kf[j][c].z, kf[j][c].w);
-          } else {
-            const uint32_t a0[4] = {qa[2 * c][0], 0u, qa[2 * c][1], 0u};
-            const uint32_t a1[4] = {qa[2 * c + 1][0], 0u, qa[2 * c + 1][1], 0u};
-            mma_bf16(acc, a0, kf[j][c].x, kf[j][c].y);
-            mma_bf16(acc, a1, kf[j][c].z, kf[j][c].w);
-          }
-        }
-        const int kcol = (kb + 8 * j + 2 * t) & (kDecRing - 1);
-        float v0 = acc[0] * p.scale, v1 = acc[1] * p.scale, v2 = acc[2] * p.scale, v3 = acc[3] * p.scale;
-        if (p.offset_causal && kb + 16 > Nk - rows) {   // only the last keys of the cache can lie in a row's future
-          const int key0 = kb + 8 * j + 2 * t, lim = Nk - rows + g;
-          if (key0 > lim) v0 = 0.f;
-          if (key0 + 1 > lim) v1 = 0.f;
-          if (key0 > lim + 8) v2 = 0.f;
-          if (key0 + 1 > lim + 8) v3 = 0.f;
-        }
-        *reinterpret_cast<float2*>(ring + g * kDecRing + kcol) = make_float2(v0, v1);
-        if (R16) *reinterpret_cast<float2*>(ring + (g + 8) * kDecRing + kcol) = make_float2(v2, v3);
-      }
-      __syncwarp();
-      // ---- conv + softmax + PV for the previous block [kb-16, kb) ----
-      if (do_pv) {
-        const int key = kb - 16 + ckey;
-        float cpart = 0.f;
-        for (int a = ra; a < rb; ++a) {
-          const float* srow = ring + a * kDecRing;
-          const float* trow = sTheta + a * 20;
-          for (int bb = 0; bb < ck; ++bb)
-            cpart = fmaf(trow[bb], srow[(key + bb - pk) & (kDecRing - 1)], cpart);
-        }
-        float cval = cpart + __shfl_xor_sync(0xffffffffu, cpart, 16);
-        if (key >= Nk) cval = -INFINITY;
-        float mx = cval;
-#pragma unroll
-        for (int off = 8; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-        const float m_new = fmaxf(m_run, mx);      // finite: key kb-16 < Nk is always valid here
-        const float pj = exp2f((cval - m_new) * kLog2e);
-        float ps = pj;
-#pragma unroll
-        for (int off = 8; off > 0; off >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, off);
-        const float alpha = exp2f((m_run - m_new) * kLog2e);   // m_run = -inf -> 0
-        l_run = l_run * alpha + ps;
-        m_run = m_new;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] *= alpha;
-#pragma unroll
-        for (int i = 0; i < VL; ++i) {
-          const float pv = __shfl_sync(0xffffffffu, pj, i * KPL + vrow);
-          o[0] = fmaf(pv, bf_lo(vf[i].x), o[0]); o[1] = fmaf(pv, bf_hi(vf[i].x), o[1]);
-          o[2] = fmaf(pv, bf_lo(vf[i].y), o[2]); o[3] = fmaf(pv, bf_hi(vf[i].y), o[3]);
-          o[4] = fmaf(pv, bf_lo(vf[i].z), o[4]); o[5] = fmaf(pv, bf_hi(vf[i].z), o[5]);
-          o[6] = fmaf(pv, bf_lo(vf[i].w), o[6]); o[7] = fmaf(pv, bf_hi(vf[i].w), o[7]);
-        }
-      }
-      __syncwarp();
+      for (int c = 0; c < CH; ++c) kf[j][c] = ok ? ldg_nc_v4(src + 8 * j * D + c * 32) : make_uint4(0u, 0u, 0u, 0u);
     }
+  };
+  auto load_v = [&](int kb, int sb) {                        // keys kb + 8 t + 4 sb + {0..3}: half of the 32-key block at kb
+    const int k0 = kb + 8 * t + 4 * sb;
+    const bf16* src = tile_base(p.V, kb + 16 * (t >> 1)) + (8 * (t & 1) + 4 * sb) * D + g * 8;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const bool ok = k0 + e < Nk && (D >= 64 || g < 4);
+#pragma unroll
+      for (int hf = 0; hf < VH; ++hf) vf[hf][e] = ok ? ldg_nc_v4(src + e * D + hf * 64) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  };
+  auto scores = [&](int kb) {                                // S of the staged K tile -> ring
+#pragma unroll
+    for (int n = 0; n < (R16 ? 2 : 1); ++n) {                // query rows 8n ..
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};                   // (key g, rows 2t, 2t + 1), (key g + 8, the same)
+#pragma unroll
+      for (int c = 0; c < CH; ++c) {
+        const uint32_t a0[4] = {kf[0][c].x, kf[1][c].x, kf[0][c].y, kf[1][c].y};
+        const uint32_t a1[4] = {kf[0][c].z, kf[1][c].z, kf[0][c].w, kf[1][c].w};
+        mma_bf16(acc, a0, qa[2 * c][2 * n], qa[2 * c][2 * n + 1]);
+        mma_bf16(acc, a1, qa[2 * c + 1][2 * n], qa[2 * c + 1][2 * n + 1]);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[i] *= p.scale;
+      const int r0 = 8 * n + 2 * t;
+      if (p.offset_causal && kb + 16 > Nk - rows) {          // only the last keys of the cache can lie in a row's future
+        const int lim = Nk - rows + r0 - (kb + g);           // key offset from g of row r0's last key
+        if (0 > lim) acc[0] = 0.f;
+        if (0 > lim + 1) acc[1] = 0.f;
+        if (8 > lim) acc[2] = 0.f;
+        if (8 > lim + 1) acc[3] = 0.f;
+      }
+      const int col = (kb - k_lo + g) & (kDecRing - 1);      // col + 8 stays in the 16-key tile
+      float* dst = ring + r0 * kDecRow + col;
+      dst[0] = acc[0]; dst[kDecRow] = acc[1]; dst[8] = acc[2]; dst[kDecRow + 8] = acc[3];
+    }
+  };
+  auto pv = [&](int sb) {                                    // O += p V for the staged half of the block
+    const uint4 pa = *reinterpret_cast<const uint4*>(ps + min(g, 3) * 32 + 8 * t);
+    const uint32_t b0 = sb ? pa.z : pa.x, b1 = sb ? pa.w : pa.y;
+#pragma unroll
+    for (int hf = 0; hf < VH; ++hf) {
+      const uint32_t v0[4] = {vf[hf][0].x, vf[hf][0].y, vf[hf][0].z, vf[hf][0].w}, v1[4] = {vf[hf][1].x, vf[hf][1].y, vf[hf][1].z, vf[hf][1].w};
+      const uint32_t v2[4] = {vf[hf][2].x, vf[hf][2].y, vf[hf][2].z, vf[hf][2].w}, v3[4] = {vf[hf][3].x, vf[hf][3].y, vf[hf][3].z, vf[hf][3].w};
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const uint32_t a[4] = {__byte_perm(v0[w], v1[w], 0x5410), __byte_perm(v0[w], v1[w], 0x7632),
+                               __byte_perm(v2[w], v3[w], 0x5410), __byte_perm(v2[w], v3[w], 0x7632)};
+        mma_bf16(o[hf][w], a, b0, b1);
+      }
+    }
+  };
+
+  if (nblk > 0) {
+    load_k(k_lo - 16);
+    scores(k_lo - 16);
+    load_k(k_lo);
+    scores(k_lo);
+    load_k(k_lo + 16);
+#pragma unroll 1
+    for (int i = 0; i < nblk; ++i) {
+      // in flight here: the K tile at kb + 16 and the second V half of block i - 1
+      const int kb = k_lo + 32 * i;
+      scores(kb + 16);
+      load_k(kb + 32);
+      if (i > 0) pv(1);
+      load_v(kb, 0);
+      scores(kb + 32);
+      if (i + 1 < nblk) load_k(kb + 48);
+      __syncwarp();
+      // ---- conv of block i: lane = keys 4g .. 4g+3 and its rows; then lane = key ----
+      float c4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        const float* row = ring + row_of(r) * kDecRow;
+        float wv[4 * WC];
+#pragma unroll
+        for (int c = 0; c < WC; ++c) {
+          const float4 x = *reinterpret_cast<const float4*>(row + 4 * ((8 * i + g - W0 / 4 + c) & (kDecRing / 4 - 1)));
+          wv[4 * c] = x.x; wv[4 * c + 1] = x.y; wv[4 * c + 2] = x.z; wv[4 * c + 3] = x.w;
+        }
+#pragma unroll
+        for (int bb = 0; bb < CKP; ++bb) {
+          const float w = THREG ? th[THREG ? r : 0][THREG ? bb : 0] : sTheta[row_of(r)][bb];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) c4[e] = fmaf(w, wv[bb + e + W0 - PKP], c4[e]);
+        }
+      }
+      float cval;
+      {
+        const bool hi2 = t & 2, hi1 = t & 1;
+        const float k0 = (hi2 ? c4[2] : c4[0]) + __shfl_xor_sync(0xffffffffu, hi2 ? c4[0] : c4[2], 2);
+        const float k1 = (hi2 ? c4[3] : c4[1]) + __shfl_xor_sync(0xffffffffu, hi2 ? c4[1] : c4[3], 2);
+        cval = (hi1 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, hi1 ? k0 : k1, 1);
+      }
+      if (kb + lane >= k_hi) cval = -INFINITY;
+      float mx;
+      asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(mx) : "f"(cval));
+      if (mx > m_run) {                                      // warp-uniform
+        const float alpha = exp2f((m_run - mx) * kLog2e);    // m_run = -inf -> 0
+        m_run = mx;
+        l_lane *= alpha;
+#pragma unroll
+        for (int q = 0; q < VH * 16; ++q) (&o[0][0][0])[q] *= alpha;
+      }
+      const float pj = exp2f((cval - m_run) * kLog2e);
+      l_lane += pj;
+      const bf16 p_hi = __float2bfloat16_rn(pj);
+      const float r1 = pj - __bfloat162float(p_hi);
+      const bf16 p_mid = __float2bfloat16_rn(r1);
+      ps[lane] = p_hi; ps[32 + lane] = p_mid; ps[64 + lane] = __float2bfloat16_rn(r1 - __bfloat162float(p_mid));
+      __syncwarp();
+      pv(0);
+      load_v(kb, 1);
+    }
+    pv(1);
   }
-  // ---- merge the V-row parities inside the warp, then the warps of the CTA ----
+  // ---- columns hi + mid (lanes t = 0) + lo (t = 1), then the warps of the CTA ----
 #pragma unroll
-  for (int off = LPR; off < 32; off <<= 1)
+  for (int hf = 0; hf < VH; ++hf)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) o[i] += __shfl_xor_sync(0xffffffffu, o[i], off);
-  if (lane < LPR) {
+    for (int w = 0; w < 4; ++w)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) sMergeO[warp][vcol + i] = o[i];
+      for (int u = 0; u < 2; ++u) {
+        float v = o[hf][w][2 * u] + o[hf][w][2 * u + 1];
+        v += __shfl_down_sync(0xffffffffu, v, 1);
+        if (t == 0 && (D >= 64 || g < 4)) sMergeO[warp][hf * 64 + g * 8 + 2 * w + u] = v;
+      }
+  {
+    const float l = warp_sum(l_lane);
+    if (lane == 0) { sMergeML[warp][0] = m_run; sMergeML[warp][1] = l; }
   }
-  if (lane == 0) { sMergeML[warp][0] = m_run; sMergeML[warp][1] = l_run; }
   __syncthreads();
   float m = -INFINITY;
 #pragma unroll
@@ -234,38 +289,78 @@ __global__ void __launch_bounds__(kDecWarps * 32, 4) decode_kernel(const DecodeP
     wgt[w] = (sMergeML[w][0] == -INFINITY) ? 0.f : exp2f((sMergeML[w][0] - m) * kLog2e);
     l += sMergeML[w][1] * wgt[w];
   }
-  const size_t so = (bh * p.k_splits + split);
-  for (int dcol = tid; dcol < D; dcol += kDecWarps * 32) {
-    float acc = 0.f;
+  float acc = 0.f;                                           // D <= 128 = blockDim.x: one head dim per thread
+  if (tid < D)
 #pragma unroll
-    for (int w = 0; w < kDecWarps; ++w) acc += sMergeO[w][dcol] * wgt[w];
-    p.O_splits[so * D + dcol] = acc;   // un-normalised partial
+    for (int w = 0; w < kDecWarps; ++w) acc += sMergeO[w][tid] * wgt[w];
+  const size_t so = bh * p.k_splits + split;
+  if (nsub == 1 && !p.fused) {
+    if (tid < D) p.O_splits[so * D + tid] = acc;             // un-normalised partial
+    if (tid == 0) { p.M_splits[so] = m; p.L_splits[so] = l; }
+    return;
   }
-  if (tid == 0) { p.M_splits[so] = m; p.L_splits[so] = l; }
+  // ---- the CTAs of a split, and with `fused` all splits of the (batch, head), merge through distributed shared memory ----
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  if (tid < D) sPartO[tid] = acc;
+  if (tid == 0) { sPartML[0] = m; sPartML[1] = l; }
+  cl.sync();
+  if (sub == 0) {
+    const bool total = p.fused && split == 0;                // the merged, normalised result goes to split 0
+    const int r0 = p.fused ? split * nsub : 0, r1 = total ? (int)cl.num_blocks() : r0 + nsub;
+    float mm = -INFINITY, ll = 0.f, aa = 0.f;
+    for (int r = r0; r < r1; ++r) mm = fmaxf(mm, cl.map_shared_rank(sPartML, r)[0]);
+    for (int r = r0; r < r1; ++r) {
+      const float* ml = cl.map_shared_rank(sPartML, r);
+      const float w = (ml[0] == -INFINITY) ? 0.f : exp2f((ml[0] - mm) * kLog2e);
+      ll += ml[1] * w;
+      if (tid < D) aa += cl.map_shared_rank(sPartO, r)[tid] * w;
+    }
+    if (tid < D) p.O_splits[so * D + tid] = total ? aa / ll : aa;
+    if (tid == 0) { p.M_splits[so] = mm; p.L_splits[so] = ll; }
+  }
+  cl.sync();                                                 // remote reads are done before a CTA's shared memory goes
 }
 
 // Merge the split partials of one (batch, head) and leave the normalised result in split 0
-// (fwd_inference.cu:332-367 keeps the same convention).
-__global__ void combine_splits_kernel(float* __restrict__ O_splits, float* __restrict__ M_splits,
-                                      float* __restrict__ L_splits, int k_splits, int D) {
+// (fwd_inference.cu:332-367 keeps the same convention).  The weights of the splits are made once, a thread each.
+__global__ void __launch_bounds__(128) combine_splits_kernel(float* __restrict__ O_splits, float* __restrict__ M_splits,
+                                                             float* __restrict__ L_splits, int k_splits, int D) {
+  __shared__ float sW[128];
+  __shared__ float sRed[4];
   const size_t bh = blockIdx.x;
   float* Ms = M_splits + bh * k_splits;
   float* Ls = L_splits + bh * k_splits;
+  const int tid = threadIdx.x;
+  pdl_wait();
   float m = -INFINITY;
-  for (int s = 0; s < k_splits; ++s) m = fmaxf(m, Ms[s]);
-  float l = 0.f;
-  for (int s = 0; s < k_splits; ++s) l += (Ms[s] == -INFINITY) ? 0.f : Ls[s] * exp2f((Ms[s] - m) * kLog2e);
-  const float inv = 1.f / l;
-  for (int dcol = threadIdx.x; dcol < D; dcol += blockDim.x) {
-    float acc = 0.f;
-    for (int s = 0; s < k_splits; ++s) {
-      const float w = (Ms[s] == -INFINITY) ? 0.f : exp2f((Ms[s] - m) * kLog2e);
-      acc += O_splits[(bh * k_splits + s) * D + dcol] * w;
-    }
-    O_splits[(bh * k_splits) * D + dcol] = acc * inv;
-  }
+  for (int s = tid; s < k_splits; s += 128) m = fmaxf(m, Ms[s]);
+  m = warp_max(m);
+  if ((tid & 31) == 0) sRed[tid >> 5] = m;
   __syncthreads();
-  if (threadIdx.x == 0) { Ms[0] = m; Ls[0] = l; }
+  m = fmaxf(fmaxf(sRed[0], sRed[1]), fmaxf(sRed[2], sRed[3]));
+  float l = 0.f, acc = 0.f;
+  for (int s0 = 0; s0 < k_splits; s0 += 128) {
+    const int n = min(128, k_splits - s0);
+    __syncthreads();
+    if (tid < n) {
+      const float ms = Ms[s0 + tid], w = (ms == -INFINITY) ? 0.f : exp2f((ms - m) * kLog2e);
+      sW[tid] = w;
+      l += Ls[s0 + tid] * w;
+    }
+    __syncthreads();
+    const float* src = O_splits + (bh * k_splits + s0) * D + tid;
+    if (tid < D)
+#pragma unroll 8
+      for (int s = 0; s < n; ++s) acc += src[(size_t)s * D] * sW[s];
+  }
+  l = warp_sum(l);
+  __syncthreads();
+  if ((tid & 31) == 0) sRed[tid >> 5] = l;
+  __syncthreads();
+  l = (sRed[0] + sRed[1]) + (sRed[2] + sRed[3]);
+  if (tid < D) O_splits[(bh * k_splits) * D + tid] = acc / l;
+  if (tid == 0) { Ms[0] = m; Ls[0] = l; }
 }
 
 // Append n_new key/value rows per sequence to a paged cache: row r of sequence b goes to position
@@ -276,10 +371,12 @@ __global__ void kv_append_paged_kernel(bf16* __restrict__ Kpool, bf16* __restric
                                        const bf16* __restrict__ Knew, const bf16* __restrict__ Vnew, int H, int n_new,
                                        int page_size, int page_shift, int max_pages) {
   constexpr int CPR = D / 8;
-  const int b = blockIdx.z, h = blockIdx.y;
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= n_new * CPR) return;
-  const int r = idx / CPR, c = idx % CPR;
+  const int b = blockIdx.z;
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;     // (head, row, chunk)
+  pdl_wait();
+  pdl_trigger();
+  if (idx >= H * n_new * CPR) return;
+  const int c = idx % CPR, r = (idx / CPR) % n_new, h = idx / (CPR * n_new);
   const int pos = seq_lens[b] + r;
   if (pos < 0 || (pos >> page_shift) >= max_pages) return;   // past the block table: the row is dropped, nothing is written
   const int pg = block_table[(size_t)b * max_pages + (pos >> page_shift)], in = pos & (page_size - 1);

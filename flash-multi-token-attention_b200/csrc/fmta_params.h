@@ -70,6 +70,8 @@ struct DecodeParams {
   float* L_splits;
   int B, H, q_len, Nk, d, cq, ck, k_splits;
   float scale;
+  int n_sub;                 // CTAs per split (a thread-block cluster merges them)
+  int fused;                 // the cluster holds all splits of a (batch, head) and writes the merged result: no combine launch
   int offset_causal;         // zero the scores of keys later than each query row's position (row r sits at Nk - rows + r)
   // paged cache (block_table != nullptr): K and V point at pools [n_pages, H, page_size, d]; page p of
   // sequence b is pool page block_table[b * max_pages + p]; seq_lens (optional) gives Nk per sequence
