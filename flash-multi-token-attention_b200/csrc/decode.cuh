@@ -12,8 +12,8 @@
 // bandwidth: with the conv as one load pair per FMA and P V as FMAs on widened values (~1000 instructions per 32 keys) the
 // kernel sustained 5.56 TB/s; a plain read sustains 7.2.
 // Both products take K and V as the 16-row A operand, as they lie in global memory.  K: rows are keys and the contraction
-// index is permuted, so that a lane's fragment is one contiguous 16-byte piece of a K row (Q, the 8-column B operand, is laid
-// out to match once, in registers).  V: rows are head dims; a lane holds 16 bytes (8 dims) of 4 keys per MMA step, and a
+// index is permuted, so that a lane's fragment is contiguous pieces of a K row (Q, the 8-column B operand, is laid
+// out to match once, in registers).  V: rows are head dims; a lane holds 16 or 32 bytes of 4 keys per MMA step, and a
 // fragment register is two halfwords of neighbouring keys (one PRMT).  p stays fp32: columns 0, 1, 2 of the B operand are its
 // bf16 parts hi, mid, lo (24 bits), whose products with V are exact; the three accumulator columns are added at the end.
 // Warps are merged in shared memory, sub-splits (and, for small problems, the splits) inside a thread-block cluster, splits
@@ -33,13 +33,28 @@ constexpr int kDecRing = 64;         // keys kept per warp for the conv window
 constexpr int kDecRow = 68;          // ring row stride in floats: even rows 8 banks apart (no conflicts, stores or window loads)
 constexpr int kDecMaxPages = 2048;   // block-table entries of one sequence kept in shared memory (paged cache)
 
-FMTA_DEVINL uint4 ldg_nc_v4(const void* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.u32 {%0,%1,%2,%3}, [%4];\n"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+// 16 or 32 bytes per lane, read once.  The 32-byte form lets the four lanes that share a K row of an MMA fragment fetch a whole
+// 128-byte line with one instruction (with 16 bytes they fetch half of it, and the L2 sees twice the requests).
+FMTA_DEVINL void ldg_nc_v4(uint32_t* v, const void* p) {
+  asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.b32 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
                : "l"(p));
-  return v;
 }
+FMTA_DEVINL void ldg_nc_v8(uint32_t* v, const void* p) {
+  asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "l"(p));
+}
+template <int W>
+FMTA_DEVINL void ldg_nc(uint32_t* v, const void* p, bool ok) {   // W words, zeros when !ok
+  if (ok) {
+    if (W == 8) ldg_nc_v8(v, p); else ldg_nc_v4(v, p);
+  } else {
+#pragma unroll
+    for (int i = 0; i < W; ++i) v[i] = 0u;
+  }
+}
+
 // keys handled by one split, a multiple of 16 * kDecWarps
 __host__ __device__ inline int decode_keys_per_split(int Nk, int k_splits) {
   const int per = (Nk + k_splits - 1) / k_splits;
@@ -51,11 +66,12 @@ __host__ __device__ inline int decode_keys_per_split(int Nk, int k_splits) {
 template <int D, int NR, int CKP, bool PAGED>
 __global__ void __launch_bounds__(kDecWarps * 32, D == 128 ? 3 : 4) decode_kernel(const DecodeParams p) {
   constexpr int KS = D / 16;               // k-steps of the QK MMA
-  constexpr int CH = D / 32;               // 32-element chunks per K row (one 16-byte load per lane each)
+  constexpr int KW = D >= 64 ? 8 : 4;      // words of a K row per lane and load: 4 lanes cover 128 bytes (64 at d = 32)
+  constexpr int KL = D / 8 / KW;           // loads per K row and lane
   constexpr bool R16 = NR > 2;
   constexpr int PKP = (CKP - 1) / 2, WC = (CKP <= 9) ? 3 : 5, W0 = 4 * ((WC - 1) / 2);   // conv window: WC float4 from 4g - W0 on
   constexpr bool THREG = NR * CKP <= 24;   // the lane's filter rows fit registers
-  constexpr int VH = D >= 64 ? D / 64 : 1; // 64-column halves of a V row
+  constexpr int VW = D == 128 ? 8 : 4;     // words of a V row per lane: 8 lanes cover the row (half of them idle at d = 32)
   __shared__ __align__(16) float sRing[kDecWarps][R16 ? 16 : 8][kDecRow];
   __shared__ __align__(16) float sTheta[16][20];
   __shared__ __align__(16) bf16 sPs[kDecWarps][4][32];     // hi, mid, lo of the step's probabilities, and a zero row
@@ -99,19 +115,14 @@ __global__ void __launch_bounds__(kDecWarps * 32, D == 128 ? 3 : 4) decode_kerne
     sTheta[i / ck][i % ck + PKP - pk] = p.theta[((size_t)h * cq + (cq - rows) + i / ck) * ck + (i % ck)];
 
   // B fragments of Q (column = query row) in the permuted-k layout (rows >= `rows` are zero)
-  uint32_t qa[KS][R16 ? 4 : 2];
+  uint32_t qa[R16 ? 2 : 1][2 * KS];                         // word w: as the words of a K row
 #pragma unroll
-  for (int c = 0; c < CH; ++c) {
-    uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
-    if (g < rows) lo = *reinterpret_cast<const uint4*>(Qg + (size_t)g * D + c * 32 + t * 8);
-    if (R16 && g + 8 < rows) hi = *reinterpret_cast<const uint4*>(Qg + (size_t)(g + 8) * D + c * 32 + t * 8);
-    qa[2 * c][0] = lo.x; qa[2 * c][1] = lo.y;
-    qa[2 * c + 1][0] = lo.z; qa[2 * c + 1][1] = lo.w;
-    if constexpr (R16) {
-      qa[2 * c][2] = hi.x; qa[2 * c][3] = hi.y;
-      qa[2 * c + 1][2] = hi.z; qa[2 * c + 1][3] = hi.w;
-    }
-  }
+  for (int n = 0; n < (R16 ? 2 : 1); ++n)
+#pragma unroll
+    for (int c = 0; c < KL; ++c)
+#pragma unroll
+      for (int i = 0; i < KW; ++i)
+        qa[n][c * KW + i] = g + 8 * n < rows ? *reinterpret_cast<const uint32_t*>(Qg + (size_t)(g + 8 * n) * D + c * 8 * KW + t * 2 * KW + 2 * i) : 0u;
   __syncthreads();
   auto row_of = [&](int r) { return 2 * t + (r & 1) + 8 * (r >> 1); };   // the lane's conv rows
   float th[THREG ? NR : 1][THREG ? CKP : 1];
@@ -131,43 +142,37 @@ __global__ void __launch_bounds__(kDecWarps * 32, D == 128 ? 3 : 4) decode_kerne
   const int nblk = k_hi > k_lo ? (k_hi - k_lo + 31) / 32 : 0;
 
   float m_run = -INFINITY, l_lane = 0.f;                     // l_lane: this lane's share of the sum
-  float o[VH][4][4];                                         // [64-dim half][dims 2w, 2w + 1 of the lane's 8][..]
+  float o[VW][4];                                            // [dims 2w, 2w + 1 of the lane's 2 VW][..]
 #pragma unroll
-  for (int i = 0; i < VH * 16; ++i) (&o[0][0][0])[i] = 0.f;
+  for (int i = 0; i < VW * 4; ++i) (&o[0][0])[i] = 0.f;
   float* ring = &sRing[warp][0][0];
   bf16* ps = &sPs[warp][0][0];
-  uint4 kf[2][CH], vf[VH][4];
+  uint32_t kf[2][2 * KS], vf[4][VW];
 
   auto load_k = [&](int kb) {                                // the 16-key tile at kb
-    const bf16* src = tile_base(p.K, kb) + g * D + t * 8;
+    const bf16* src = tile_base(p.K, kb) + g * D + t * 2 * KW;
     const int lim = Nk - kb;                                 // rows of the tile inside the cache
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const bool ok = kb >= 0 && 8 * j + g < lim;
 #pragma unroll
-      for (int c = 0; c < CH; ++c) kf[j][c] = ok ? ldg_nc_v4(src + 8 * j * D + c * 32) : make_uint4(0u, 0u, 0u, 0u);
+      for (int c = 0; c < KL; ++c) ldg_nc<KW>(&kf[j][c * KW], src + 8 * j * D + c * 8 * KW, ok);
     }
   };
   auto load_v = [&](int kb, int sb) {                        // keys kb + 8 t + 4 sb + {0..3}: half of the 32-key block at kb
     const int k0 = kb + 8 * t + 4 * sb;
-    const bf16* src = tile_base(p.V, kb + 16 * (t >> 1)) + (8 * (t & 1) + 4 * sb) * D + g * 8;
+    const bf16* src = tile_base(p.V, kb + 16 * (t >> 1)) + (8 * (t & 1) + 4 * sb) * D + g * 2 * VW;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const bool ok = k0 + e < Nk && (D >= 64 || g < 4);
-#pragma unroll
-      for (int hf = 0; hf < VH; ++hf) vf[hf][e] = ok ? ldg_nc_v4(src + e * D + hf * 64) : make_uint4(0u, 0u, 0u, 0u);
-    }
+    for (int e = 0; e < 4; ++e) ldg_nc<VW>(vf[e], src + e * D, k0 + e < Nk && (D >= 64 || g < 4));
   };
   auto scores = [&](int kb) {                                // S of the staged K tile -> ring
 #pragma unroll
     for (int n = 0; n < (R16 ? 2 : 1); ++n) {                // query rows 8n ..
       float acc[4] = {0.f, 0.f, 0.f, 0.f};                   // (key g, rows 2t, 2t + 1), (key g + 8, the same)
 #pragma unroll
-      for (int c = 0; c < CH; ++c) {
-        const uint32_t a0[4] = {kf[0][c].x, kf[1][c].x, kf[0][c].y, kf[1][c].y};
-        const uint32_t a1[4] = {kf[0][c].z, kf[1][c].z, kf[0][c].w, kf[1][c].w};
-        mma_bf16(acc, a0, qa[2 * c][2 * n], qa[2 * c][2 * n + 1]);
-        mma_bf16(acc, a1, qa[2 * c + 1][2 * n], qa[2 * c + 1][2 * n + 1]);
+      for (int s = 0; s < KS; ++s) {
+        const uint32_t a[4] = {kf[0][2 * s], kf[1][2 * s], kf[0][2 * s + 1], kf[1][2 * s + 1]};
+        mma_bf16(acc, a, qa[n][2 * s], qa[n][2 * s + 1]);
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[i] *= p.scale;
@@ -188,15 +193,10 @@ __global__ void __launch_bounds__(kDecWarps * 32, D == 128 ? 3 : 4) decode_kerne
     const uint4 pa = *reinterpret_cast<const uint4*>(ps + min(g, 3) * 32 + 8 * t);
     const uint32_t b0 = sb ? pa.z : pa.x, b1 = sb ? pa.w : pa.y;
 #pragma unroll
-    for (int hf = 0; hf < VH; ++hf) {
-      const uint32_t v0[4] = {vf[hf][0].x, vf[hf][0].y, vf[hf][0].z, vf[hf][0].w}, v1[4] = {vf[hf][1].x, vf[hf][1].y, vf[hf][1].z, vf[hf][1].w};
-      const uint32_t v2[4] = {vf[hf][2].x, vf[hf][2].y, vf[hf][2].z, vf[hf][2].w}, v3[4] = {vf[hf][3].x, vf[hf][3].y, vf[hf][3].z, vf[hf][3].w};
-#pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        const uint32_t a[4] = {__byte_perm(v0[w], v1[w], 0x5410), __byte_perm(v0[w], v1[w], 0x7632),
-                               __byte_perm(v2[w], v3[w], 0x5410), __byte_perm(v2[w], v3[w], 0x7632)};
-        mma_bf16(o[hf][w], a, b0, b1);
-      }
+    for (int w = 0; w < VW; ++w) {
+      const uint32_t a[4] = {__byte_perm(vf[0][w], vf[1][w], 0x5410), __byte_perm(vf[0][w], vf[1][w], 0x7632),
+                             __byte_perm(vf[2][w], vf[3][w], 0x5410), __byte_perm(vf[2][w], vf[3][w], 0x7632)};
+      mma_bf16(o[w], a, b0, b1);
     }
   };
 
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, D == 128 ? 3 : 4) decode_kerne
         m_run = mx;
         l_lane *= alpha;
 #pragma unroll
-        for (int q = 0; q < VH * 16; ++q) (&o[0][0][0])[q] *= alpha;
+        for (int q = 0; q < VW * 4; ++q) (&o[0][0])[q] *= alpha;
       }
       const float pj = exp2f((cval - m_run) * kLog2e);
       l_lane += pj;
@@ -266,15 +266,13 @@ __global__ void __launch_bounds__(kDecWarps * 32, D == 128 ? 3 : 4) decode_kerne
   }
   // ---- columns hi + mid (lanes t = 0) + lo (t = 1), then the warps of the CTA ----
 #pragma unroll
-  for (int hf = 0; hf < VH; ++hf)
+  for (int w = 0; w < VW; ++w)
 #pragma unroll
-    for (int w = 0; w < 4; ++w)
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        float v = o[hf][w][2 * u] + o[hf][w][2 * u + 1];
-        v += __shfl_down_sync(0xffffffffu, v, 1);
-        if (t == 0 && (D >= 64 || g < 4)) sMergeO[warp][hf * 64 + g * 8 + 2 * w + u] = v;
-      }
+    for (int u = 0; u < 2; ++u) {
+      float v = o[w][2 * u] + o[w][2 * u + 1];
+      v += __shfl_down_sync(0xffffffffu, v, 1);
+      if (t == 0 && (D >= 64 || g < 4)) sMergeO[warp][g * 2 * VW + 2 * w + u] = v;
+    }
   {
     const float l = warp_sum(l_lane);
     if (lane == 0) { sMergeML[warp][0] = m_run; sMergeML[warp][1] = l; }
