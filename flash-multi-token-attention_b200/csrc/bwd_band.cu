@@ -63,7 +63,9 @@ inline int bwd_band_positions(int cq, int ck) {
 }
 
 
-template <int D, int CQ, int CK>   // head dim; filter shape at compile time, or (0, 0): read from the parameters
+// head dim; filter shape at compile time, or (0, 0): read from the parameters; GIVEN: dC of the band comes from p.dCband (head
+// mixing) and P dO is not the kernel's: dQ, dK and dTheta only
+template <int D, int CQ, int CK, bool GIVEN>
 __global__ void __launch_bounds__(bandcfg::NT, bandcfg::Layout<D>::kCtasPerSm) bwd_band_kernel(const TrainParams p) {
   using namespace bandcfg;
   using BL = Layout<D>;
@@ -93,8 +95,8 @@ __global__ void __launch_bounds__(bandcfg::NT, bandcfg::Layout<D>::kCtasPerSm) b
   const int pq = cq - 1, pk = (ck - 1) / 2, band = pq + pk, W = band + pk;
   const int Rt = min(RC, RC - (W - 1 + pq));           // positions per CTA
   const bool mma_out = (W <= 17);
-  const int h = blockIdx.y, b = blockIdx.z;
-  const size_t bh = (size_t)b * H + h;
+  const size_t bh = (size_t)p.bh_base + blockIdx.y + (size_t)gridDim.y * blockIdx.z;
+  const int h = (int)(bh % H), b = (int)(bh / H);
   const int t0 = win_lo(p) + blockIdx.x * Rt;
   const int R = p.row_hi > 0 ? min(Rt, p.row_hi - t0) : Rt;   // a call with a window owns no position past its end
   // wait first, trigger second: once every CTA here has triggered, the pre-pass and D are known to be complete, and the
@@ -108,13 +110,15 @@ __global__ void __launch_bounds__(bandcfg::NT, bandcfg::Layout<D>::kCtasPerSm) b
 
   load_rows_async<D, NT>(sQ, LD, Qg, t0 - 16, RS, N, tid);
   load_rows_async<D, NT>(sK, LD, Kg, t0 - 48, RK, N, tid);
-  load_rows_async<D, NT>(sV, LD, Vg, t0 - 16, RS, N, tid);
-  load_rows_async<D, NT>(sdO, LD, dOg, t0, RC, N, tid);
+  if (!GIVEN) {
+    load_rows_async<D, NT>(sV, LD, Vg, t0 - 16, RS, N, tid);
+    load_rows_async<D, NT>(sdO, LD, dOg, t0, RC, N, tid);
+  }
   cp_async_commit();
   for (int i = tid; i < cq * ck; i += NT) sTheta[(i / ck) * kThetaLdBand + (i % ck)] = p.theta[((size_t)h * cq) * ck + i];
   for (int i = tid; i < RS * SB_LD; i += NT) sSb[i] = 0.f;
   if (mma_out) for (int i = tid; i < RC * A_LD / 2; i += NT) reinterpret_cast<uint32_t*>(sAV)[i] = 0u;
-  if (tid < RC) {
+  if (!GIVEN && tid < RC) {
     const int gi = t0 + tid;
     sLse[tid] = gi < N ? p.LSE[bh * N + gi] * kLog2e : 0.f;
     sDv[tid] = gi < N ? p.Dvec[bh * N + gi] : 0.f;
@@ -125,7 +129,7 @@ __global__ void __launch_bounds__(bandcfg::NT, bandcfg::Layout<D>::kCtasPerSm) b
   // ---- Sb and dPb on 16 x 16 tiles along the diagonal ----
   {
     const int nkt = (W > 17) ? 3 : 2;
-    const int nS = (RS / 16) * nkt, nP = (RC / 16) * 2;
+    const int nS = (RS / 16) * nkt, nP = GIVEN ? 0 : (RC / 16) * 2;
     for (int job = warp; job < nS + nP; job += NT / 32) {
       float acc[2][4] = {};
       if (job < nS) {
@@ -167,7 +171,12 @@ __global__ void __launch_bounds__(bandcfg::NT, bandcfg::Layout<D>::kCtasPerSm) b
   __syncthreads();
 
   // ---- conv, P and dC ----
-  if constexpr (CQ > 0) {
+  if constexpr (GIVEN) {
+    for (int o = tid; o < RC * band; o += NT) {
+      const int x = o / band, dd = o - x * band, gi = t0 + x;
+      if (gi < N && gi - dd >= 0) sdC[x * DC_LD + pk + dd] = p.dCband[(bh * N + gi) * band + dd];
+    }
+  } else if constexpr (CQ > 0) {
     // compile-time filter: a thread owns half of the diagonals of one row and keeps the score
     // segment each filter row needs in registers (one shared-memory load per ~5 FMAs)
     constexpr int PQ = CQ - 1, PK = (CK - 1) / 2, BAND = PQ + PK, HB = (BAND + 1) / 2, SEG = HB + CK - 1;
@@ -408,8 +417,9 @@ __global__ void __launch_bounds__(bandcfg::NT, bandcfg::Layout<D>::kCtasPerSm) b
     // ---- dQ, dK, dV on mma.sync: 16 positions x 32 head dims per job ----
     const int ntile = (R + 15) / 16;
     constexpr int NCH = D / 32;                                          // 32-column chunks of the head dim
-    for (int job = warp; job < ntile * 3 * NCH; job += NT / 32) {
-      const int m = job / (3 * NCH), which = (job % (3 * NCH)) / NCH, ch = job % NCH;      // which: 0 dQ, 1 dK, 2 dV
+    constexpr int NO = GIVEN ? 2 : 3;
+    for (int job = warp; job < ntile * NO * NCH; job += NT / 32) {
+      const int m = job / (NO * NCH), which = (job % (NO * NCH)) / NCH, ch = job % NCH;      // which: 0 dQ, 1 dK, 2 dV
       const int x0 = 16 * m + (lane >> 2), x1 = x0 + 8;
       const bool ok0 = (x0 < R) && (t0 + x0 < N), ok1 = (x1 < R) && (t0 + x1 < N);
       float* gout = (which == 0) ? p.dQ : (which == 1) ? p.dK : p.dV;
@@ -454,15 +464,16 @@ __global__ void __launch_bounds__(bandcfg::NT, bandcfg::Layout<D>::kCtasPerSm) b
         ak1.x = fmaf(s21, __low2float(q1), ak1.x); ak1.y = fmaf(s21, __high2float(q1), ak1.y);
       }
 #pragma unroll 2
-      for (int dd = 0; dd < band; ++dd) {
+      for (int dd = 0; dd < (GIVEN ? 0 : band); ++dd) {
         const float p0 = sP[(xr0 + dd) * P_LD + dd], p1 = sP[(xb + dd) * P_LD + dd];
         const __nv_bfloat162 o0 = *reinterpret_cast<const __nv_bfloat162*>(sdO + (xr0 + dd) * LD + col);
         const __nv_bfloat162 o1 = *reinterpret_cast<const __nv_bfloat162*>(sdO + (xb + dd) * LD + col);
         av0.x = fmaf(p0, __low2float(o0), av0.x); av0.y = fmaf(p0, __high2float(o0), av0.y);
         av1.x = fmaf(p1, __low2float(o1), av1.x); av1.y = fmaf(p1, __high2float(o1), av1.y);
       }
-      *reinterpret_cast<float2*>(ga) = aq0; *reinterpret_cast<float2*>(ga + kofs) = ak0; *reinterpret_cast<float2*>(ga + vofs) = av0;
-      if (two) { *reinterpret_cast<float2*>(gb) = aq1; *reinterpret_cast<float2*>(gb + kofs) = ak1; *reinterpret_cast<float2*>(gb + vofs) = av1; }
+      *reinterpret_cast<float2*>(ga) = aq0; *reinterpret_cast<float2*>(ga + kofs) = ak0;
+      if (two) { *reinterpret_cast<float2*>(gb) = aq1; *reinterpret_cast<float2*>(gb + kofs) = ak1; }
+      if (!GIVEN) { *reinterpret_cast<float2*>(ga + vofs) = av0; if (two) *reinterpret_cast<float2*>(gb + vofs) = av1; }
      }
     }
   }
@@ -476,24 +487,33 @@ int bwd_band_theta_slots(int B, int N, int cq, int ck) {
 
 // Writes the band part of dQ/dK/dV and one dTheta partial per CTA into p.dTheta_part
 // ([slots][H][cq*ck]).  Nothing to do when the filter has no band (pad_q + pad_k == 0).
-template <int D>
+template <int D, bool GIVEN>
 static cudaError_t launch_bwd_band_d(const TrainParams& p, dim3 grid, cudaStream_t stream) {
   constexpr int smem = bandcfg::Layout<D>::kSmemBytes;
   if (p.cq == 6 && p.ck == 11)
-    return launch_kernel<TrainParams>(bwd_band_kernel<D, 6, 11>, grid, dim3(bandcfg::NT), smem, stream, -1, p);
+    return launch_kernel<TrainParams>(bwd_band_kernel<D, 6, 11, GIVEN>, grid, dim3(bandcfg::NT), smem, stream, -1, p);
   if (p.cq == 7 && p.ck == 7 && D == 64)
-    return launch_kernel<TrainParams>(bwd_band_kernel<D, 7, 7>, grid, dim3(bandcfg::NT), smem, stream, -1, p);
+    return launch_kernel<TrainParams>(bwd_band_kernel<D, 7, 7, GIVEN>, grid, dim3(bandcfg::NT), smem, stream, -1, p);
   if (p.cq == 3 && p.ck == 5)
-    return launch_kernel<TrainParams>(bwd_band_kernel<D, 3, 5>, grid, dim3(bandcfg::NT), smem, stream, -1, p);
-  return launch_kernel<TrainParams>(bwd_band_kernel<D, 0, 0>, grid, dim3(bandcfg::NT), smem, stream, -1, p);
+    return launch_kernel<TrainParams>(bwd_band_kernel<D, 3, 5, GIVEN>, grid, dim3(bandcfg::NT), smem, stream, -1, p);
+  return launch_kernel<TrainParams>(bwd_band_kernel<D, 0, 0, GIVEN>, grid, dim3(bandcfg::NT), smem, stream, -1, p);
 }
 
 cudaError_t launch_bwd_band(const TrainParams& p, cudaStream_t stream) {
   const int R = bwd_band_positions(p.cq, p.ck);
   dim3 grid((win_hi(p) - win_lo(p) + R - 1) / R, p.H, p.B);
   ScopedKernelTimer timer_(kKernBwdBand, stream);
-  if (p.d == 128) return launch_bwd_band_d<128>(p, grid, stream);
-  return launch_bwd_band_d<64>(p, grid, stream);
+  if (p.d == 128) return launch_bwd_band_d<128, false>(p, grid, stream);
+  return launch_bwd_band_d<64, false>(p, grid, stream);
+}
+
+// Head mixing: the (batch, head) pairs bh0 .. bh0 + nbh - 1, from p.dCband.
+cudaError_t launch_bwd_band_given(const TrainParams& p_, int bh0, int nbh, cudaStream_t stream) {
+  TrainParams p = p_;
+  p.bh_base = bh0;
+  const int R = bwd_band_positions(p.cq, p.ck);
+  dim3 grid((p.N + R - 1) / R, nbh);
+  return p.d == 128 ? launch_bwd_band_d<128, true>(p, grid, stream) : launch_bwd_band_d<64, true>(p, grid, stream);
 }
 
 }  // namespace fmta

@@ -894,12 +894,14 @@ struct DkPostCfg {
   static constexpr int T_LD = 40, T_ELEMS = 16 * T_LD;        // one 16 x 32 Toeplitz tile (bf16), rows 80 bytes apart
   static constexpr int RED_LD = 7 * 24;              // floats per warp in the dTheta reduction buffer
   __host__ __device__ static constexpr int t_bytes(int cq) { return 2 * cq * T_ELEMS * 2; }
-  static constexpr int smem_bytes(int cq) {           // alignment slack + key rows + c_q tap tiles + max(Toeplitz tiles, reduction buffer) + barriers
-    return 1024 + (cq + 1) * TILE_STRIDE + (t_bytes(cq) > 8 * RED_LD * 4 ? t_bytes(cq) : 8 * RED_LD * 4) + 64;
+  static constexpr int smem_bytes(int cq, bool lo) {           // alignment slack + key rows + c_q tap tiles + max(Toeplitz tiles, reduction buffer) + barriers
+    return 1024 + (cq * (lo ? 2 : 1) + 1) * TILE_STRIDE + (t_bytes(cq) > 8 * RED_LD * 4 ? t_bytes(cq) : 8 * RED_LD * 4) + 64;
   }
 };
 
-__global__ void __launch_bounds__(DkPostCfg::NT, 2)
+// LO: dKt_a is a (hi, lo) pair of tiles; the lo tiles follow the hi tiles in shared memory
+template <bool LO>
+__global__ void __launch_bounds__(DkPostCfg::NT, LO ? 1 : 2)
 dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmX,
                    const float* __restrict__ theta, void* dK, const float* dKadd, int out_bf16, float* __restrict__ dTheta_part, int* status,
                    int H, int N, int cq, int ck, float scale, int n_jblocks, int dfull, int j_base) {
@@ -909,7 +911,8 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   // tile 0: key rows, tile 1 + a: dKt_a rows; row r of a tile is key J0 - HALO + r
-  unsigned char* sTb = smem + (cq + 1) * Cfg::TILE_STRIDE;
+  constexpr int HL = LO ? 2 : 1;
+  unsigned char* sTb = smem + (cq * HL + 1) * Cfg::TILE_STRIDE;
   bf16* sT = reinterpret_cast<bf16*>(sTb);                  // [cq][hi, lo][16][T_LD]
   float* sRed = reinterpret_cast<float*>(sTb);               // takes the place of the Toeplitz tiles once the dK GEMMs are done
   const int t_or_red = Cfg::t_bytes(cq) > 8 * RED_LD * 4 ? Cfg::t_bytes(cq) : 8 * RED_LD * 4;
@@ -946,12 +949,16 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   __syncthreads();
   pdl_wait();      // nothing before this line reads what a kernel of the same call writes
   if (tid == 0) {
-    tc::mbar_expect_tx(&bars[0], (1 + half) * Cfg::TILE_BYTES);
+    tc::mbar_expect_tx(&bars[0], (1 + half * HL) * Cfg::TILE_BYTES);
     tc::tma_load_3d(smem, &tmK, &bars[0], col0, J0 - HALO, bh);
-    for (int a = 0; a < half; ++a) tc::tma_load_3d(smem + (a + 1) * Cfg::TILE_STRIDE, &tmX, &bars[0], col0, J0 - HALO, bh * cq + a);
+    auto load_tap = [&](int a, uint64_t* bar) {
+      for (int hl = 0; hl < HL; ++hl)
+        tc::tma_load_3d(smem + (1 + hl * cq + a) * Cfg::TILE_STRIDE, &tmX, bar, col0, J0 - HALO, (bh * cq + a) * HL + hl);
+    };
+    for (int a = 0; a < half; ++a) load_tap(a, &bars[0]);
     if (cq > half) {
-      tc::mbar_expect_tx(&bars[1], (cq - half) * Cfg::TILE_BYTES);
-      for (int a = half; a < cq; ++a) tc::tma_load_3d(smem + (a + 1) * Cfg::TILE_STRIDE, &tmX, &bars[1], col0, J0 - HALO, bh * cq + a);
+      tc::mbar_expect_tx(&bars[1], (cq - half) * HL * Cfg::TILE_BYTES);
+      for (int a = half; a < cq; ++a) load_tap(a, &bars[1]);
     }
   }
   bool ok = true;
@@ -978,9 +985,10 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
           ldsm_x4(al[1], sT + (2 * a + 1) * T_ELEMS + t_off + 16);
         }
 #pragma unroll
-        for (int st = 0; st < 3; ++st) {
+        for (int sh = 0; sh < 3 * HL; ++sh) {
+          const int st = sh % 3;
           uint32_t bfr[4];
-          ldsm_x4_t(bfr, at(a + 1, x_row + 16 * st, x_chunk));
+          ldsm_x4_t(bfr, at(a + 1 + (sh / 3) * cq, x_row + 16 * st, x_chunk));
 #pragma unroll
           for (int ks = 0; ks < 2; ++ks) {
             const int m = st - ks;                           // the tile whose step ks these rows are
@@ -1028,9 +1036,10 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     for (int kk = 0; kk < 8; ++kk) {
       const int row = HALO + 8 * warp + kk;                  // shared-memory row of this key
 #pragma unroll
-      for (int c0 = 0; c0 < D / 8; c0 += 4) {
+      for (int ch_ = 0; ch_ < D / 8 * HL; ch_ += 4) {
+        const int c0 = ch_ % (D / 8);
         uint32_t bfr[4], a0[4], a1[4];
-        ldsm_x4(bfr, at(bt, row, c0 + q));
+        ldsm_x4(bfr, at(bt + (ch_ / (D / 8)) * cq, row, c0 + q));
         ldsm_x4(a0, at(0, row + sA0, c0 + (q >> 1)));
         ldsm_x4(a1, at(0, row + sA0, c0 + 2 + (q >> 1)));
         const int ch = (c0 >> 1) & 2;                        // chains 0, 1 for columns 0..31, 2, 3 for columns 32..63
@@ -1073,8 +1082,6 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
 // ==========================================================================================
 // host side
 // ==========================================================================================
-cudaError_t launch_ktilde(const TrainParams& p, __nv_bfloat16* Kt, cudaStream_t stream);
-
 bool bwd_tc_supported(const TrainParams& p) {
   // head dim 64: up to seven query taps (two launches of the dK/dV kernel for the seventh); head dim 128:
   // up to six (the resident stacked key tiles of the dK/dV kernel fill its shared memory)
@@ -1199,7 +1206,7 @@ static cudaError_t launch_dkdv_pass(const TrainParams& p, const __nv_bfloat16* K
 
 cudaError_t launch_bwd_dkdv_tc(const TrainParams& p, void* workspace, float* dTheta_part_tc, bool keep_pdc, cudaStream_t stream) {
   const int D = p.d;
-  const size_t rows = (size_t)p.B * p.H * p.N, BH = (size_t)p.B * p.H;
+  const size_t rows = (size_t)p.B * p.H * p.N;
   auto up = [](size_t x) { return (x + 1023) / 1024 * 1024; };
   unsigned char* w = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(workspace) + 1023) & ~uintptr_t(1023));
   __nv_bfloat16* Kt = reinterpret_cast<__nv_bfloat16*>(w); w += up(rows * p.cq * D * 2);
@@ -1235,16 +1242,23 @@ cudaError_t launch_bwd_dkdv_tc(const TrainParams& p, void* workspace, float* dTh
       }
     } }
   if (e != cudaSuccess) return e;
+  return launch_dk_post(p, dKt, false, dTheta_part_tc, status, stream);
+}
+
+// The adjoint of the pre-pass over the call's window: dK (plus the band's part, causal) and the dTheta partials.
+cudaError_t launch_dk_post(const TrainParams& p, __nv_bfloat16* dKt, bool with_lo, float* dTheta_part_tc, int* status, cudaStream_t stream) {
+  const int D = p.d;
+  const size_t BH = (size_t)p.B * p.H;
   const int j_base = win_lo(p);
   const int njb = (win_hi(p) - j_base + DkPostCfg::KEYS - 1) / DkPostCfg::KEYS;
   dim3 g2(njb, (unsigned)BH, D / DkPostCfg::D);      // one CTA per 64 keys and 64 columns of the head dim
-  const int smem = DkPostCfg::smem_bytes(p.cq);
-  auto kern = dk_post_mma_kernel;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const int smem = DkPostCfg::smem_bytes(p.cq, with_lo);
+  auto kern = with_lo ? dk_post_mma_kernel<true> : dk_post_mma_kernel<false>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   alignas(64) CUtensorMap tmK, tmX;
   if (!make_tensor_map_bf16(&tmK, p.K, D, p.N, BH, 64, DkPostCfg::ROWS, true)) return cudaErrorInvalidValue;
-  if (!make_tensor_map_bf16(&tmX, dKt, D, p.N, BH * p.cq, 64, DkPostCfg::ROWS, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmX, dKt, D, p.N, BH * p.cq * (with_lo ? 2 : 1), 64, DkPostCfg::ROWS, true)) return cudaErrorInvalidValue;
   // (the maps span the full head dim; each CTA fetches its 64-column slab)
   ScopedKernelTimer timer2_(kKernDkPost, stream);
   return launch_pdl(kern, g2, dim3(DkPostCfg::NT), (size_t)smem, stream, tmK, tmX, p.theta, p.dKo, p.causal ? p.dK : (const float*)nullptr, p.grad_bf16, dTheta_part_tc, status, p.H, p.N, p.cq,

@@ -147,6 +147,7 @@ size_t fmta_workspace_bytes(int op, int B, int H, int N, int d, int cq, int ck, 
     const size_t rows = (size_t)B * H * N;
     return up1k(fmta_workspace_bytes(FMTA_OP_BWD_TC, B, H, N, d, cq, ck, G)) + up1k(rows * 4) + up1k(rows * d * 2) + 3 * up1k(rows * d * 4);
   }
+  if (op == FMTA_OP_MIX_FWD || op == FMTA_OP_MIX_BWD) return mix_tc_workspace_bytes(B, H, N, d, cq, ck, G, op == FMTA_OP_MIX_BWD);
   if (op == FMTA_OP_MIX_EXCHANGE) {
     // optional scratch of the conv + mix cluster kernels: two sets (alternate tiles) of two fp32 tiles per CTA
     // (one CTA per 64 rows / keys and head)
@@ -189,6 +190,9 @@ static int fwd_impl(const void* Q, const void* K, const void* V, const float* th
   // when W is absent -- with G == 1 and W given the scalar still applies:
   if (wmix && G == 1) return FMTA_ERR_UNSUPPORTED;
   if (path != 0 && path != 1 && path != -1) return FMTA_ERR_SHAPE;
+  if (path != 0 && g_path != 0 && row_hi == 0 && mix_tc_supported(p) && workspace && aligned16(workspace) &&
+      workspace_bytes >= fmta_workspace_bytes(FMTA_OP_MIX_FWD, B, H, N, d, p.cq, p.ck, p.G))
+    return check_cuda(launch_mix_fwd(p, workspace, (cudaStream_t)stream));
   bool use_tc = (path != 0) && fwd_tc_supported(p);
   if (path == 1 && !use_tc) return FMTA_ERR_UNSUPPORTED;
   if (use_tc) {
@@ -422,6 +426,27 @@ int fmta_bwd_fused(const void* Q, const void* K, const void* V, const void* dO, 
   if (int s = check_cuda(launch_rowdot(dO, O, o_dtype == FMTA_DTYPE_BF16, d32 ? dOb : nullptr, D, rows, d, (cudaStream_t)stream))) return s;
   return bwd_impl(Q, K, V, d32 ? dOb : dO, D, LSE, theta, nullptr, part[0], part[1], part[2], dTheta, nullptr, B, H, N, d, cq,
                   ck, 1, scale, causal, 1, workspace, base, stream, ktilde, 0, 0, g16 ? outs : nullptr);
+}
+
+int fmta_mix_bwd(const void* Q, const void* K, const void* V, const void* dO, int do_dtype, const void* O, int o_dtype,
+                 const float* LSE, const float* theta, const float* wmix, void* dQ, void* dK, void* dV, int grad_dtype,
+                 float* dTheta, float* dW, int B, int H, int N, int d, int cq, int ck, int G, float scale, int causal,
+                 void* workspace, size_t workspace_bytes, void* stream) {
+  TrainParams p = {};
+  if (int s = fill_bwd(p, Q, K, V, dO, /* D is made here */ LSE, LSE, theta, wmix, B, H, N, d, cq, ck, G, scale, causal)) return s;
+  if (!O || !wmix) return FMTA_ERR_NULL;
+  const int want = (dQ ? 1 : 0) | (dK ? 2 : 0);
+  if (!want || (!dK) != (!dV) || (theta && want != 3)) return FMTA_ERR_NULL;
+  if (dQ && (!dW || (theta && !dTheta))) return FMTA_ERR_NULL;
+  for (int t : {do_dtype, o_dtype, grad_dtype})
+    if (t != FMTA_DTYPE_F32 && t != FMTA_DTYPE_BF16) return FMTA_ERR_UNSUPPORTED;
+  for (const void* x : {O, (const void*)dQ, (const void*)dK, (const void*)dV, (const void*)workspace})
+    if (!aligned16(x)) return FMTA_ERR_ALIGN;
+  if (!mix_tc_supported(p)) return FMTA_ERR_UNSUPPORTED;
+  if (!workspace || workspace_bytes < fmta_workspace_bytes(FMTA_OP_MIX_BWD, B, H, N, d, p.cq, p.ck, G)) return FMTA_ERR_WORKSPACE;
+  p.dQo = dQ; p.dKo = dK; p.dVo = dV; p.grad_bf16 = grad_dtype == FMTA_DTYPE_BF16;
+  return check_cuda(launch_mix_bwd(p, dO, do_dtype == FMTA_DTYPE_F32, O, o_dtype == FMTA_DTYPE_BF16, dTheta, dW, want, workspace,
+                                   (cudaStream_t)stream));
 }
 
 int fmta_stacked_keys(const void* K, const float* theta, void* ktilde, int B, int H, int N, int d, int cq, int ck,

@@ -34,6 +34,9 @@ struct TrainParams {
   int kt_valid;              //   ... which already holds the operand of these K / theta / scale: the pre-pass is skipped
   int row_lo, row_hi;        // tensor-core path: the window of sequence positions this call computes (output rows of the
                              //   forward; dQ rows, dK / dV keys and the dTheta terms of the backward); 0, 0 = the whole sequence
+  float* Cband;              // head mix on the tensor cores: scores of the causal band after the filter [B*H, N, band], natural units
+  float* dCband;             //   ... and their gradient
+  int bh_base;               // bwd_band_kernel: first (batch, head) of the launch
   float* xchg;               // conv + mix cluster kernels: optional global scratch, 2 sets x 2 * kMixXchFloats floats per CTA (nullptr: exchange through distributed shared memory)
   int B, H, N, d, cq, ck, G;
   float scale;

@@ -39,7 +39,9 @@ struct FwdBandCfg {
   static constexpr int kSmemBytes = oTheta + 16 * kThLd * 4;
 };
 
-template <int D, int CQ, int CK>   // filter shape at compile time, or (0, 0): read from the parameters
+// filter shape at compile time, or (0, 0): read from the parameters; SCORES: only Cb, to p.Cband (head mixing, which needs all
+// heads' scores before the softmax)
+template <int D, int CQ, int CK, bool SCORES>
 __global__ void __launch_bounds__(FwdBandCfg<D>::NT, 2) fwd_band_kernel(const TrainParams p) {
   using Cfg = FwdBandCfg<D>;
   constexpr int NT = Cfg::NT, R = Cfg::R, RS = Cfg::RS, RK = Cfg::RK, RV = Cfg::RV, LD = Cfg::LD;
@@ -64,12 +66,13 @@ __global__ void __launch_bounds__(FwdBandCfg<D>::NT, 2) fwd_band_kernel(const Tr
   const size_t bh = (size_t)b * H + h;
   const int t0 = win_lo(p) + blockIdx.x * R;          // a window starts on a multiple of R
   const int koff = (band > 16) ? 32 : 16;             // the P tile of 16 rows starts koff keys before them
+  if (SCORES) pdl_wait();
   pdl_trigger();
 
   if (band > 0) {
     load_rows_async<D, NT>(sQ, LD, p.Q + bh * (size_t)N * D, t0 - 16, RS, N, tid);
     load_rows_async<D, NT>(sK, LD, p.K + bh * (size_t)N * D, t0 - 48, RK, N, tid);
-    load_rows_async<D, NT>(sV, LD, p.V + bh * (size_t)N * D, t0 - 32, RV, N, tid);
+    if (!SCORES) load_rows_async<D, NT>(sV, LD, p.V + bh * (size_t)N * D, t0 - 32, RV, N, tid);
     cp_async_commit();
     for (int i = tid; i < cq * ck; i += NT) sTheta[(i / ck) * kThLd + (i % ck)] = p.theta[((size_t)h * cq) * ck + i];
     for (int i = tid; i < RS * SB_LD; i += NT) sSb[i] = 0.f;
@@ -159,6 +162,13 @@ __global__ void __launch_bounds__(FwdBandCfg<D>::NT, 2) fwd_band_kernel(const Tr
     }
     __syncthreads();
   }
+  if constexpr (SCORES) {
+    for (int o = tid; o < R * band; o += NT) {
+      const int x = o / band, gi = t0 + x;
+      if (gi < N) p.Cband[(bh * N + gi) * band + (o - x * band)] = sC[x * C_LD + (o - x * band)];
+    }
+    return;
+  }
 
   // Up to here only inputs of the call were read, which were complete before any CTA of the tensor-core kernel let this
   // one start; its partial is needed from here on
@@ -230,24 +240,28 @@ __global__ void __launch_bounds__(FwdBandCfg<D>::NT, 2) fwd_band_kernel(const Tr
   }
 }
 
-template <int D>
+template <int D, bool SCORES>
 static cudaError_t launch_fwd_band_t(const TrainParams& p, cudaStream_t stream) {
   using Cfg = FwdBandCfg<D>;
   dim3 grid((win_hi(p) - win_lo(p) + Cfg::R - 1) / Cfg::R, p.H, p.B);
   if (p.cq == 6 && p.ck == 11)
-    return launch_kernel<TrainParams>(fwd_band_kernel<D, 6, 11>, grid, dim3(Cfg::NT), Cfg::kSmemBytes, stream, -1, p);
+    return launch_kernel<TrainParams>(fwd_band_kernel<D, 6, 11, SCORES>, grid, dim3(Cfg::NT), Cfg::kSmemBytes, stream, -1, p);
   if (p.cq == 7 && p.ck == 7)
-    return launch_kernel<TrainParams>(fwd_band_kernel<D, 7, 7>, grid, dim3(Cfg::NT), Cfg::kSmemBytes, stream, -1, p);
+    return launch_kernel<TrainParams>(fwd_band_kernel<D, 7, 7, SCORES>, grid, dim3(Cfg::NT), Cfg::kSmemBytes, stream, -1, p);
   if (p.cq == 3 && p.ck == 5)
-    return launch_kernel<TrainParams>(fwd_band_kernel<D, 3, 5>, grid, dim3(Cfg::NT), Cfg::kSmemBytes, stream, -1, p);
-  return launch_kernel<TrainParams>(fwd_band_kernel<D, 0, 0>, grid, dim3(Cfg::NT), Cfg::kSmemBytes, stream, -1, p);
+    return launch_kernel<TrainParams>(fwd_band_kernel<D, 3, 5, SCORES>, grid, dim3(Cfg::NT), Cfg::kSmemBytes, stream, -1, p);
+  return launch_kernel<TrainParams>(fwd_band_kernel<D, 0, 0, SCORES>, grid, dim3(Cfg::NT), Cfg::kSmemBytes, stream, -1, p);
 }
 
 // Finishes the forward started by the stacked tensor-core kernel: band entries + normalisation.
 cudaError_t launch_fwd_band(const TrainParams& p, cudaStream_t stream) {
   ScopedKernelTimer timer_(kKernFwdExact, stream);
-  if (p.d == 64) return launch_fwd_band_t<64>(p, stream);
-  return launch_fwd_band_t<128>(p, stream);
+  if (p.d == 64) return launch_fwd_band_t<64, false>(p, stream);
+  return launch_fwd_band_t<128, false>(p, stream);
+}
+
+cudaError_t launch_band_scores(const TrainParams& p, cudaStream_t stream) {
+  return p.d == 64 ? launch_fwd_band_t<64, true>(p, stream) : launch_fwd_band_t<128, true>(p, stream);
 }
 
 }  // namespace fmta

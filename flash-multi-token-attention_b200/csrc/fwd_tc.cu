@@ -33,9 +33,18 @@
 namespace fmta {
 
 
+// what eight bf16 roundings leave over, as bf16
+FMTA_DEVINL uint4 bf16_rest(const float (&v)[8], const uint4& o) {
+  const uint32_t h[4] = {o.x, o.y, o.z, o.w};
+  uint32_t r[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) r[e] = pack_bf16(v[2 * e] - __uint_as_float(h[e] << 16), v[2 * e + 1] - __uint_as_float(h[e] & 0xffff0000u));
+  return make_uint4(r[0], r[1], r[2], r[3]);
+}
+
 // ------------------------------------------------------------------------------------------
 // Kt[bh, a, j, :] = scale * sum_b theta[h, a, b] * K[bh, j + b - pad_k, :]   (bf16, zero beyond ends)
-template <int D>
+template <int D, bool LO>   // LO: a (hi, lo) bf16 pair per tap
 __global__ void __launch_bounds__(256) ktilde_kernel(const bf16* __restrict__ K, const float* __restrict__ theta,
                                                      bf16* __restrict__ Kt, int H, int N, int cq, int ck,
                                                      float scale) {
@@ -71,13 +80,15 @@ __global__ void __launch_bounds__(256) ktilde_kernel(const bf16* __restrict__ K,
   uint4 o;
   o.x = pack_bf16(acc[0], acc[1]); o.y = pack_bf16(acc[2], acc[3]);
   o.z = pack_bf16(acc[4], acc[5]); o.w = pack_bf16(acc[6], acc[7]);
-  *reinterpret_cast<uint4*>(Kt + (((size_t)bh * cq + a) * N + j) * D + c * 8) = o;
+  bf16* dst = Kt + ((((size_t)bh * cq + a) * (LO ? 2 : 1)) * N + j) * D + c * 8;
+  *reinterpret_cast<uint4*>(dst) = o;
+  if (LO) *reinterpret_cast<uint4*>(dst + (size_t)N * D) = bf16_rest(acc, o);
 }
 
 // Same pre-pass with the filter width known at compile time: one thread owns one 16-byte column
 // chunk of RR consecutive rows and produces all c_q taps from a register window of RR + CK - 1
 // key rows, so every key row is loaded once per RR outputs instead of once per output and tap.
-template <int D, int CK, int RR>
+template <int D, int CK, int RR, bool LO>
 __global__ void __launch_bounds__(256) ktilde_window_kernel(const bf16* __restrict__ K, const float* __restrict__ theta,
                                                             bf16* __restrict__ Kt, int H, int N, int cq, float scale) {
   constexpr int CPR = D / 8, RUNS = 256 / CPR, PK = (CK - 1) / 2, WIN = RR + CK - 1;
@@ -100,7 +111,7 @@ __global__ void __launch_bounds__(256) ktilde_window_kernel(const bf16* __restri
     float w[CK];
 #pragma unroll
     for (int b = 0; b < CK; ++b) w[b] = sTh[a * CK + b];
-    bf16* out = Kt + (((size_t)bh * cq + a) * N + j0) * D + c * 8;
+    bf16* out = Kt + ((((size_t)bh * cq + a) * (LO ? 2 : 1)) * N + j0) * D + c * 8;
 #pragma unroll
     for (int r = 0; r < RR; ++r) {
       float acc[8];
@@ -121,6 +132,7 @@ __global__ void __launch_bounds__(256) ktilde_window_kernel(const bf16* __restri
         o.x = pack_bf16(acc[0], acc[1]); o.y = pack_bf16(acc[2], acc[3]);
         o.z = pack_bf16(acc[4], acc[5]); o.w = pack_bf16(acc[6], acc[7]);
         *reinterpret_cast<uint4*>(out + (size_t)r * D) = o;
+        if (LO) *reinterpret_cast<uint4*>(out + (size_t)(N + r) * D) = bf16_rest(acc, o);
       }
     }
   }
@@ -539,7 +551,7 @@ bool make_tensor_map_f32(CUtensorMap* map, const void* base, int D, int rows, si
 }
 
 // Pre-pass: Kt = scale * log2(e) * (theta applied along the key axis of K), c_q bf16 copies.
-cudaError_t launch_ktilde(const TrainParams& p, __nv_bfloat16* Kt, cudaStream_t stream) {
+cudaError_t launch_ktilde(const TrainParams& p, __nv_bfloat16* Kt, cudaStream_t stream, bool with_lo) {
   ScopedKernelTimer timer_(kKernKtilde, stream);
   const size_t BH = (size_t)p.B * p.H;
   const float sc = p.scale * kLog2e;
@@ -548,7 +560,8 @@ cudaError_t launch_ktilde(const TrainParams& p, __nv_bfloat16* Kt, cudaStream_t 
 #define FMTA_KT_WIN(DD, CKK)                                                                                      \
     { constexpr int RUNS = 256 / (DD / 8);                                                                        \
       dim3 grid((p.N + RUNS * RR - 1) / (RUNS * RR), (unsigned)BH);                                               \
-      (void)launch_pdl(ktilde_window_kernel<DD, CKK, RR>, grid, dim3(256), 0, stream, p.K, p.theta, Kt, p.H, p.N, p.cq, sc); }
+      auto kern = with_lo ? ktilde_window_kernel<DD, CKK, RR, true> : ktilde_window_kernel<DD, CKK, RR, false>;          \
+      (void)launch_pdl(kern, grid, dim3(256), 0, stream, p.K, p.theta, Kt, p.H, p.N, p.cq, sc); }
     if (p.d == 64) {
       if (p.ck == 11) FMTA_KT_WIN(64, 11) else if (p.ck == 7) FMTA_KT_WIN(64, 7) else if (p.ck == 5) FMTA_KT_WIN(64, 5) else FMTA_KT_WIN(64, 3)
     } else {
@@ -560,11 +573,11 @@ cudaError_t launch_ktilde(const TrainParams& p, __nv_bfloat16* Kt, cudaStream_t 
   if (p.d == 64) {
     constexpr int RPB = 256 / (64 / 8);
     dim3 grid((p.N + RPB - 1) / RPB, (unsigned)BH, p.cq);
-    ktilde_kernel<64><<<grid, 256, 0, stream>>>(p.K, p.theta, Kt, p.H, p.N, p.cq, p.ck, sc);
+    return launch_pdl(with_lo ? ktilde_kernel<64, true> : ktilde_kernel<64, false>, grid, dim3(256), 0, stream, p.K, p.theta, Kt, p.H, p.N, p.cq, p.ck, sc);
   } else {
     constexpr int RPB = 256 / (128 / 8);
     dim3 grid((p.N + RPB - 1) / RPB, (unsigned)BH, p.cq);
-    ktilde_kernel<128><<<grid, 256, 0, stream>>>(p.K, p.theta, Kt, p.H, p.N, p.cq, p.ck, sc);
+    return launch_pdl(with_lo ? ktilde_kernel<128, true> : ktilde_kernel<128, false>, grid, dim3(256), 0, stream, p.K, p.theta, Kt, p.H, p.N, p.cq, p.ck, sc);
   }
   return cudaGetLastError();
 }

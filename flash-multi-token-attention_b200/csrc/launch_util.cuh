@@ -112,7 +112,18 @@ cudaError_t launch_kv_append_paged(void* Kpool, void* Vpool, const int* block_ta
                                    int page_shift, int max_pages, cudaStream_t stream);
 bool fwd_tc_supported(const TrainParams& p);
 // pre-pass of the tensor-core kernels: Kt[b,h,t,j,:] = scale * log2(e) * sum_u theta[h,t,u] * K[b,h,j + pad_k - u,:]
-cudaError_t launch_ktilde(const TrainParams& p, __nv_bfloat16* Kt, cudaStream_t stream);
+// with_lo: a (hi, lo) bf16 pair per tap, [B,H,cq,2,N,d]
+cudaError_t launch_ktilde(const TrainParams& p, __nv_bfloat16* Kt, cudaStream_t stream, bool with_lo = false);
+cudaError_t launch_band_scores(const TrainParams& p, cudaStream_t stream);            // p.Cband
+cudaError_t launch_bwd_band_given(const TrainParams& p, int bh0, int nbh, cudaStream_t stream);   // from p.dCband: dQ, dK, dTheta parts
+// with_lo: dKt is [B,H,cq,2,N,d], a (hi, lo) pair per tap
+cudaError_t launch_dk_post(const TrainParams& p, __nv_bfloat16* dKt, bool with_lo, float* dTheta_part, int* status, cudaStream_t stream);
+// head mix on the tensor cores (mix_tc.cu)
+bool mix_tc_supported(const TrainParams& p);
+size_t mix_tc_workspace_bytes(int B, int H, int N, int d, int cq, int ck, int G, bool bwd);
+cudaError_t launch_mix_fwd(const TrainParams& p, void* workspace, cudaStream_t stream);
+cudaError_t launch_mix_bwd(const TrainParams& p, const void* dO, bool do_f32, const void* O, bool o_bf16, float* dTheta, float* dW, int want,
+                           void* workspace, cudaStream_t stream);
 size_t fwd_tc_workspace_bytes(int B, int H, int N, int d, int cq);
 bool bwd_tc_supported(const TrainParams& p);
 size_t bwd_tc_workspace_bytes(int B, int H, int N, int d, int cq);

@@ -1,0 +1,556 @@
+// The per-head products behind the mixed scores (mix_score.cu), as GEMM pipelines on tcgen05: P and dC come from global memory
+// in the X8 layout (mix_tc.cuh), so there is no element-wise phase in the loops.
+//   mix_pv_kernel   : O = P V.  CTA = 128 rows of a head; P is relative to one reference per row and key chunk, so the
+//                     accumulator is taken out of tensor memory and rescaled once per chunk.  Writes O, M, L, LSE.
+//   mix_dq_kernel   : dQ[i'] = sum_a dC[i' + pad_q - a] Kt_a.  CTA = two tiles of 128 rows that share every key tile; the row
+//                     shift is 16 bytes per row of the no-swizzle dC operand (136 rows are staged).
+//   mix_dkdv_kernel : dV = P^T dO, dKt_a = dC^T Q^(a).  CTA = 128 keys x 64 columns of the head dim (two CTAs at d = 128);
+//                     P and dC are read MN-major, so nothing is transposed.
+// All are bound by the stream of P / dC (2 bytes per score entry and tensor) or by the MMAs at c_q = 6.
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include "mix_tc.cuh"
+
+namespace fmta {
+
+// ==========================================================================================
+template <int D>
+struct PvCfg {
+  static constexpr int BM = 128, BC = 64, SL = D / 64;
+  static constexpr int P_BYTES = BM * BC * 2, V_SLAB = BC * 128;
+  static constexpr int STAGE = P_BYTES + SL * V_SLAB, NSTG = D == 64 ? 4 : 3;
+  static constexpr int oBar = NSTG * STAGE;
+  static constexpr int kSmemBytes = oBar + 256 + 1024;        // two CTAs per SM
+  static constexpr int kTmemCols = 2 * D;                     // two accumulators: a chunk's product runs while the last one is taken out
+  static constexpr int kThreads = 192;
+};
+
+template <int D>
+__global__ void __launch_bounds__(192, 2)
+mix_pv_kernel(const __grid_constant__ CUtensorMap tmV, const MixParams p, void* O, int o_bf16, float* Mo, float* Lo, float* LSEo) {
+  using Cfg = PvCfg<D>;
+  constexpr int BM = Cfg::BM, BC = Cfg::BC, NSTG = Cfg::NSTG, SL = Cfg::SL;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::oBar);
+  uint64_t* full = bars;
+  uint64_t* empty = full + NSTG;
+  uint64_t* o_full = empty + NSTG;       // [2] the accumulator of a chunk is complete
+  uint64_t* o_free = o_full + 2;         // [2] it is in registers
+  uint64_t* mma_drain = o_free + 2;
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(mma_drain + 1);
+  volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
+  volatile int* s_issued = s_abort + 1;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int lh = blockIdx.y, rt = p.nRT - 1 - blockIdx.x;
+  const int u = p.u0 + lh / p.G, HG = p.H / p.G, b = u / HG, bh = b * p.H + (u - b * HG) * p.G + lh % p.G;
+  const int N = p.N, R0 = rt * BM;
+  const int k_end = p.causal ? min(R0 + BM, p.N8) : p.N8;     // as the score kernel's
+  const int nblk = k_end / BC, bpc = p.kch / BC;              // blocks, blocks per chunk
+  const int nch = (nblk + bpc - 1) / bpc;
+
+  if (tid == 0) {
+    for (int i = 0; i < NSTG; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { tc::mbar_init(&o_full[i], 1); tc::mbar_init(&o_free[i], 4); }
+    tc::mbar_init(mma_drain, 1);
+    *s_abort = 0; *s_issued = 0;
+    tc::mbar_fence_init();
+  }
+  if (warp == 5) {
+    tc::tmem_alloc(s_tmem, Cfg::kTmemCols);
+    tc::tmem_relinquish();
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  pdl_wait();
+  pdl_trigger();
+  tc::tc_fence_after();
+  const uint32_t tmem = *s_tmem;
+
+  if (warp == 4) {
+    if (lane == 0) {
+      const bf16* src = p.P8 + ((size_t)lh * (p.N8 / 8) * p.RP + R0) * 8;
+      for (int kb = 0; kb < nblk; ++kb) {
+        const int st = kb % NSTG, ph = (kb / NSTG) & 1;
+        if (!tc::mbar_wait(&empty[st], ph ^ 1, s_abort)) break;
+        unsigned char* sg = smem + st * Cfg::STAGE;
+        tc::mbar_expect_tx(&full[st], Cfg::STAGE);
+        for (int c = 0; c < BC / 8; ++c) tc::bulk_load(sg + c * (BM * 16), src + (size_t)(kb * (BC / 8) + c) * p.RP * 8, BM * 16, &full[st]);
+        for (int sl = 0; sl < SL; ++sl) tc::tma_load_3d(sg + Cfg::P_BYTES + sl * Cfg::V_SLAB, &tmV, &full[st], sl * 64, kb * BC, bh);
+        *s_issued = kb + 1;
+      }
+    }
+  } else if (warp == 5) {
+    constexpr uint32_t idesc = tc::make_idesc(BM, D, 0, 1);
+    const uint64_t dA = tc::make_sdesc(smem_u32(smem), BM * 16, 128, tc::kLayoutNone);
+    const uint64_t dB = tc::make_sdesc(smem_u32(smem) + Cfg::P_BYTES, SL > 1 ? Cfg::V_SLAB : 16, 1024, tc::kLayoutSW128);
+    const uint32_t a_hi = (uint32_t)(dA >> 32), a0 = (uint32_t)dA, b_hi = (uint32_t)(dB >> 32), b0 = (uint32_t)dB;
+    bool ok = true;
+    for (int ch = 0; ch < nch && ok; ++ch) {
+      const int bf = ch & 1;
+      if (ch > 1) { ok = tc::mbar_wait_warp(&o_free[bf], ((ch >> 1) - 1) & 1, s_abort); tc::tc_fence_after(); }
+      for (int kb = ch * bpc; kb < min(nblk, (ch + 1) * bpc) && ok; ++kb) {
+        const int st = kb % NSTG, ph = (kb / NSTG) & 1;
+        ok = tc::mbar_wait_warp(&full[st], ph, s_abort);
+        if (!ok) break;
+        tc::tc_fence_after();
+        const uint32_t a = a0 + (uint32_t)(st * (Cfg::STAGE >> 4)), bb = b0 + (uint32_t)(st * (Cfg::STAGE >> 4));
+        tc::mma_ss2pe(tmem + bf * D, a, a_hi, bb, b_hi, idesc, kb != ch * bpc);
+#pragma unroll
+        for (int k = 1; k < BC / 16; ++k) tc::mma_ss2e<1>(tmem + bf * D, a + (uint32_t)(2 * k * BM), a_hi, bb + (uint32_t)(k * (2048 / 16)), b_hi, idesc);
+        tc::mma_commit_e(&empty[st]);
+      }
+      if (ok) tc::mma_commit_e(&o_full[bf]);
+    }
+  } else {
+    const int r = warp * 32 + lane, gi = R0 + r;
+    const uint32_t tO = tmem + ((uint32_t)(warp * 32) << 16);
+    // the row's statistics over the chunks and halves
+    const float* st = p.stat + (size_t)lh * 2 * p.nKC * 3 * p.RP + gi;
+    float m = -INFINITY;
+    for (int i = 0; i < 2 * nch; ++i) m = fmaxf(m, st[(size_t)i * 3 * p.RP]);
+    float l = 0.f;
+    for (int i = 0; i < 2 * nch; ++i) {
+      const float ref = st[((size_t)i * 3 + 1) * p.RP];
+      if (ref != -INFINITY) l += st[((size_t)i * 3 + 2) * p.RP] * exp2f(ref - m);
+    }
+    float o[D];
+#pragma unroll
+    for (int i = 0; i < D; ++i) o[i] = 0.f;
+    bool ok = true;
+    for (int ch = 0; ch < nch; ++ch) {
+      const int bf = ch & 1;
+      const float ref = st[((size_t)(2 * ch) * 3 + 1) * p.RP], sc = ref == -INFINITY ? 0.f : exp2f(ref - m);
+      ok = __all_sync(0xffffffffu, tc::mbar_wait(&o_full[bf], (ch >> 1) & 1, s_abort));
+      if (!ok) break;
+      tc::tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < D / 32; ++c) {
+        float v[32];
+        tc::tmem_ld32(tO + bf * D + c * 32, v);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[c * 32 + i] = fmaf(v[i], sc, o[c * 32 + i]);
+      }
+      tc::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&o_free[bf]);
+    }
+    if (gi < N) {
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      const size_t row = (size_t)bh * N + gi;
+#pragma unroll
+      for (int c = 0; c < D / 32; ++c) store_grad32(O, o_bf16, nullptr, row * D + c * 32, reinterpret_cast<const float (&)[32]>(o[c * 32]), inv);
+      const float mn = m * kLn2;
+      if (Mo) Mo[row] = mn;
+      if (Lo) Lo[row] = l;
+      if (LSEo) LSEo[row] = mn + logf(l);
+    }
+  }
+  __syncwarp();
+  tc::tc_fence_before();
+  __syncthreads();
+  if (*s_abort) {
+    if (tid == 0) atomicExch(p.status, 1);
+    if (warp == 5) tc::mma_commit_e(mma_drain);
+    if (tid == 128) {
+      volatile int never = 0;
+      const int issued = *s_issued;
+      for (int it = max(0, issued - NSTG); it < issued; ++it) tc::mbar_wait(&full[it % NSTG], (it / NSTG) & 1, &never);
+      tc::mbar_wait(mma_drain, 0, &never);
+    }
+    __syncthreads();
+  }
+  if (warp == 5) {
+    tc::tc_fence_after();
+    tc::tmem_dealloc(tmem, Cfg::kTmemCols);
+  }
+}
+
+// ==========================================================================================
+template <int D>
+struct MixDqCfg {
+  static constexpr int BM = 128, AR = BM + 8, BC = 64, SL = D / 64, NT = 2;
+  static constexpr int A_BYTES = AR * 128;                    // one dC tile: 136 rows x 64 keys
+  static constexpr int SLAB = BC * 128, B_BYTES = SL * SLAB;  // one key tile: 64 x D
+  static constexpr int NA = 2;                                // dC stages (both tiles), held for all key tiles of their block
+  static constexpr int NB = D == 64 ? 16 : 9;                 // key tiles in flight
+  static constexpr int oB = NA * NT * A_BYTES;
+  static constexpr int oBar = oB + NB * B_BYTES;
+  static constexpr int kSmemBytes = oBar + 512 + 1024;
+  static constexpr int kThreads = (NT * 4 + 1 + NT) * 32;
+  static_assert(kSmemBytes <= 227 * 1024 && oB % 1024 == 0, "shared memory");
+};
+
+struct MixGradOut {
+  void* out;              // [B,H,N,D] fp32 or bf16
+  const float* add;       // fp32 part to add (the band kernel's), or nullptr
+  int bf16_out;
+  float mul;
+};
+
+template <int D>
+__global__ void __launch_bounds__(MixDqCfg<D>::kThreads, 1)
+mix_dq_kernel(const __grid_constant__ CUtensorMap tmB, const MixParams p, int ntap, int nhl, MixGradOut out) {
+  using Cfg = MixDqCfg<D>;
+  constexpr int BM = Cfg::BM, AR = Cfg::AR, BC = Cfg::BC, SL = Cfg::SL, NT = Cfg::NT, NA = Cfg::NA, NB = Cfg::NB;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::oBar);
+  uint64_t* a_full = bars;               // [NA]
+  uint64_t* a_empty = a_full + NA;       // both issuers release every stage and key tile
+  uint64_t* full = a_empty + NA;         // [NB]
+  uint64_t* empty = full + NB;
+  uint64_t* done = empty + NB;           // [NT]
+  uint64_t* mma_drain = done + NT;
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(mma_drain + 1);
+  volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
+  volatile int* s_issued = s_abort + 1;  // key tiles and dC stages the producer has issued
+  volatile int* s_aissued = s_abort + 2;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int lh = blockIdx.y, nQ = (p.nRT + 1) / 2, q = nQ - 1 - blockIdx.x;
+  const int u = p.u0 + lh / p.G, HG = p.H / p.G, b = u / HG, bh = b * p.H + (u - b * HG) * p.G + lh % p.G;
+  const int N = p.N, pq = ntap - 1;
+  int nkb_t[NT];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    const int rt = 2 * q + t;
+    nkb_t[t] = rt >= p.nRT ? 0 : (p.causal ? min(rt * BM + BM, p.N8) : p.N8) / BC;
+  }
+  const int nB = ntap * nhl;             // key tiles per block: taps, as (hi, lo) pairs with a filter
+  const int nkb = max(nkb_t[0], nkb_t[1]);
+
+  if (tid == 0) {
+    for (int i = 0; i < NA; ++i) { tc::mbar_init(&a_full[i], 1); tc::mbar_init(&a_empty[i], NT); }
+    for (int i = 0; i < NB; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], NT); }
+    for (int i = 0; i < NT; ++i) tc::mbar_init(&done[i], 1);
+    tc::mbar_init(mma_drain, NT);
+    *s_abort = 0; *s_issued = 0; *s_aissued = 0;
+    tc::mbar_fence_init();
+  }
+  if (warp == NT * 4 + 1) {
+    tc::tmem_alloc(s_tmem, NT * D);
+    tc::tmem_relinquish();
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  pdl_wait();
+  pdl_trigger();
+  tc::tc_fence_after();
+  const uint32_t tmem = *s_tmem;
+
+  if (warp == NT * 4) {
+    if (lane == 0) {
+      const bf16* src = p.C8 + (size_t)lh * (p.N8 / 8) * p.RP * 8;
+      int id = 0;
+      bool ok = true;
+      for (int kb = 0; kb < nkb && ok; ++kb) {
+        const int st = kb % NA;
+        ok = tc::mbar_wait(&a_empty[st], ((kb / NA) & 1) ^ 1, s_abort);
+        if (!ok) break;
+        tc::mbar_expect_tx(&a_full[st], NT * Cfg::A_BYTES);
+        for (int t = 0; t < NT; ++t) {
+          // a tile past its last block (or past the last row tile) gets an earlier valid block's data
+          const int rt = min(2 * q + t, p.nRT - 1), kk = min(kb, max(nkb_t[t], 1) - 1);
+          for (int c = 0; c < BC / 8; ++c)
+            tc::bulk_load(smem + (st * NT + t) * Cfg::A_BYTES + c * (AR * 16), src + ((size_t)(kk * (BC / 8) + c) * p.RP + rt * BM) * 8, AR * 16, &a_full[st]);
+        }
+        *s_aissued = kb + 1;
+        for (int a = 0; a < nB; ++a, ++id) {
+          const int s = id % NB;
+          ok = tc::mbar_wait(&empty[s], ((id / NB) & 1) ^ 1, s_abort);
+          if (!ok) break;
+          tc::mbar_expect_tx(&full[s], Cfg::B_BYTES);
+          for (int sl = 0; sl < SL; ++sl) tc::tma_load_3d(smem + Cfg::oB + s * Cfg::B_BYTES + sl * Cfg::SLAB, &tmB, &full[s], sl * 64, kb * BC, bh * nB + a);
+          *s_issued = id + 1;
+        }
+      }
+    }
+  } else if (warp > NT * 4) {
+    const int t = warp - (NT * 4 + 1);
+    constexpr uint32_t idesc = tc::make_idesc(BM, D, 0, 1);
+    const uint64_t dA = tc::make_sdesc(smem_u32(smem), AR * 16, 128, tc::kLayoutNone);
+    const uint64_t dB = tc::make_sdesc(smem_u32(smem) + Cfg::oB, SL > 1 ? Cfg::SLAB : 16, 1024, tc::kLayoutSW128);
+    const uint32_t a_hi = (uint32_t)(dA >> 32), a0 = (uint32_t)dA, b_hi = (uint32_t)(dB >> 32), b0 = (uint32_t)dB;
+    const uint32_t dst = tmem + t * D;
+    bool ok = true;
+    int id = 0;
+    for (int kb = 0; kb < nkb && ok; ++kb) {
+      const bool active = kb < nkb_t[t];
+      const int st = kb % NA;
+      ok = tc::mbar_wait_warp(&a_full[st], (kb / NA) & 1, s_abort);
+      if (!ok) break;
+      for (int a = 0; a < nB; ++a, ++id) {
+        const int s = id % NB;
+        ok = tc::mbar_wait_warp(&full[s], (id / NB) & 1, s_abort);
+        if (!ok) break;
+        if (active) {
+          tc::tc_fence_after();
+          const uint32_t al = a0 + (uint32_t)((st * NT + t) * (Cfg::A_BYTES >> 4) + (pq - a / nhl));                 // dC rows i' + pad_q - a
+          const uint32_t bl = b0 + (uint32_t)(s * (Cfg::B_BYTES >> 4));
+          tc::mma_ss2pe(dst, al, a_hi, bl, b_hi, idesc, (kb != 0) || (a != 0));
+#pragma unroll
+          for (int k = 1; k < BC / 16; ++k) tc::mma_ss2e<1>(dst, al + (uint32_t)(2 * k * AR), a_hi, bl + (uint32_t)(k * (2048 / 16)), b_hi, idesc);
+        }
+        tc::mma_commit_e(&empty[s]);
+      }
+      if (ok) tc::mma_commit_e(&a_empty[st]);
+    }
+    if (ok) tc::mma_commit_e(&done[t]);
+  } else {
+    const int t = warp >> 2, r = tid & (BM - 1), gi = (2 * q + t) * BM + r;
+    const uint32_t tQ = tmem + ((uint32_t)((warp & 3) * 32) << 16) + t * D;
+    const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&done[t], 0, s_abort));
+    tc::tc_fence_after();
+#pragma unroll
+    for (int c = 0; c < D / 32; ++c) {
+      float o[32];
+      if (ok && nkb_t[t] > 0) {
+        tc::tmem_ld32(tQ + c * 32, o);
+        if (gi < N) store_grad32(out.out, out.bf16_out, out.add, ((size_t)bh * N + gi) * D + c * 32, o, out.mul);
+      }
+    }
+  }
+  __syncwarp();
+  tc::tc_fence_before();
+  __syncthreads();
+  if (*s_abort) {
+    if (tid == 0) atomicExch(p.status, 1);
+    if (warp > NT * 4) tc::mma_commit_e(mma_drain);
+    if (tid == NT * 4 * 32) {
+      volatile int never = 0;
+      const int issued = *s_issued, ai = *s_aissued;
+      for (int id = max(0, issued - NB); id < issued; ++id) tc::mbar_wait(&full[id % NB], (id / NB) & 1, &never);
+      for (int kb = max(0, ai - NA); kb < ai; ++kb) tc::mbar_wait(&a_full[kb % NA], (kb / NA) & 1, &never);
+      tc::mbar_wait(mma_drain, 0, &never);
+    }
+    __syncthreads();
+  }
+  if (warp == NT * 4 + 1) {
+    tc::tc_fence_after();
+    tc::tmem_dealloc(tmem, NT * D);
+  }
+}
+
+// ==========================================================================================
+struct MixDkvCfg {
+  static constexpr int BK = 128, BR = 64, HALO = 8, QR = BR + HALO, NSTG = 4;
+  static constexpr int X_BYTES = BK * BR * 2;                 // P or dC: [BK / 8][BR][16 B]
+  static constexpr int sgP = 0, sgC = X_BYTES, sgdO = 2 * X_BYTES, sgQ = sgdO + BR * 128;
+  static constexpr int STAGE = sgQ + QR * 128;                // 50176 bytes
+  static constexpr int KT_BYTES = BK * 128;                   // one dKt tile on its way out
+  static constexpr int oBar = NSTG * STAGE;
+  static constexpr int kSmemBytes = oBar + 256 + 1024;
+  static constexpr int kEpWarps = 8, kThreads = (kEpWarps + 3) * 32;
+  static_assert(STAGE % 1024 == 0 && 7 * KT_BYTES <= NSTG * STAGE && kSmemBytes <= 227 * 1024, "shared memory");
+};
+
+__global__ void __launch_bounds__(MixDkvCfg::kThreads, 1)
+mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO, const __grid_constant__ CUtensorMap tmdKt,
+                const MixParams p, int cq, int d, MixGradOut dV, MixGradOut dK) {
+  using Cfg = MixDkvCfg;
+  constexpr int BK = Cfg::BK, BR = Cfg::BR, HALO = Cfg::HALO, NSTG = Cfg::NSTG;
+  constexpr int W_TMA = Cfg::kEpWarps, W_A0 = Cfg::kEpWarps + 1;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::oBar);
+  uint64_t* full = bars;
+  uint64_t* empty = full + NSTG;         // both issuers release a stage
+  uint64_t* all_done = empty + NSTG;
+  uint64_t* mma_drain = all_done + 1;
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(mma_drain + 1);
+  volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
+  volatile int* s_issued = s_abort + 1;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nh = d / 64, lh = blockIdx.y, kt = blockIdx.x / nh, col0 = (blockIdx.x % nh) * 64;
+  const int u = p.u0 + lh / p.G, HG = p.H / p.G, b = u / HG, bh = b * p.H + (u - b * HG) * p.G + lh % p.G;
+  const int N = p.N, pq = cq - 1, j0 = kt * BK;
+  const int nQB = (N + BR - 1) / BR, qb_begin = p.causal ? min(nQB, j0 / BR) : 0, nblk = nQB - qb_begin;
+
+  if (tid == 0) {
+    for (int i = 0; i < NSTG; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 2); }
+    tc::mbar_init(all_done, 2); tc::mbar_init(mma_drain, 2);
+    *s_abort = 0; *s_issued = 0;
+    tc::mbar_fence_init();
+  }
+  if (warp == W_A0) {
+    tc::tmem_alloc(s_tmem, 512);
+    tc::tmem_relinquish();
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  pdl_wait();
+  pdl_trigger();
+  tc::tc_fence_after();
+  const uint32_t tmem = *s_tmem;
+
+  if (warp == W_TMA) {
+    if (lane == 0) {
+      const size_t base = ((size_t)lh * (p.N8 / 8) + j0 / 8) * p.RP * 8;
+      for (int it = 0; it < nblk; ++it) {
+        const int st = it % NSTG, ph = (it / NSTG) & 1, i0 = (qb_begin + it) * BR;
+        if (!tc::mbar_wait(&empty[st], ph ^ 1, s_abort)) break;
+        unsigned char* sg = smem + st * Cfg::STAGE;
+        tc::mbar_expect_tx(&full[st], Cfg::STAGE);
+        tc::tma_load_3d(sg + Cfg::sgdO, &tmdO, &full[st], col0, i0, bh);
+        tc::tma_load_3d(sg + Cfg::sgQ, &tmQ, &full[st], col0, i0 - HALO, bh);
+        for (int c = 0; c < BK / 8; ++c) tc::bulk_load(sg + Cfg::sgP + c * (BR * 16), p.P8 + base + ((size_t)c * p.RP + i0) * 8, BR * 16, &full[st]);
+        for (int c = 0; c < BK / 8; ++c) tc::bulk_load(sg + Cfg::sgC + c * (BR * 16), p.C8 + base + ((size_t)c * p.RP + i0) * 8, BR * 16, &full[st]);
+        *s_issued = it + 1;
+      }
+    }
+  } else if (warp > W_TMA) {
+    // ===================== MMA issuers: A0 takes dV and the first half of the tap groups, A1 the rest =====================
+    const int ai = warp - W_A0;
+    constexpr uint32_t idescV = tc::make_idesc(BK, 64, 1, 1);        // both operands MN-major
+    constexpr uint32_t idescK2 = tc::make_idesc(BK, 128, 1, 1);      // two adjacent taps (see bwd_stream.cu)
+    const int pairs = cq / 2, ngrp = pairs + (cq & 1), g_half = ngrp / 2;
+    const int g_begin = ai == 0 ? 0 : g_half, g_end = ai == 0 ? g_half : ngrp;
+    bool ok = true;
+    for (int it = 0; it < nblk && ok; ++it) {
+      const int st = it % NSTG, ph = (it / NSTG) & 1;
+      const uint32_t sg = smem_u32(smem + st * Cfg::STAGE);
+      // P / dC: M = keys in chunks of 8, BR * 16 bytes apart; K = rows, 16 bytes apart
+      const uint64_t dPa = tc::make_sdesc(sg + Cfg::sgP, 128, BR * 16, tc::kLayoutNone);
+      const uint64_t dCa = tc::make_sdesc(sg + Cfg::sgC, 128, BR * 16, tc::kLayoutNone);
+      const uint64_t dOb = tc::make_sdesc(sg + Cfg::sgdO, 16, 1024, tc::kLayoutSW128);
+      const uint64_t dQb = tc::make_sdesc(sg + Cfg::sgQ + (HALO - pq) * 128, 128, 1024, tc::kLayoutSW128);
+      const uint32_t pa_hi = (uint32_t)(dPa >> 32), pa_lo = (uint32_t)dPa, ca_lo = (uint32_t)dCa;
+      const uint32_t ob_hi = (uint32_t)(dOb >> 32), ob_lo = (uint32_t)dOb, qb_hi = (uint32_t)(dQb >> 32), qb_lo = (uint32_t)dQb;
+      ok = tc::mbar_wait_warp(&full[st], ph, s_abort);
+      if (!ok) break;
+      tc::tc_fence_after();
+      if (ai == 0) {
+        tc::mma_ss2pe(tmem, pa_lo, pa_hi, ob_lo, ob_hi, idescV, it != 0);
+#pragma unroll
+        for (int k = 1; k < BR / 16; ++k) tc::mma_ss2e<1>(tmem, pa_lo + (uint32_t)(k * 16), pa_hi, ob_lo + (uint32_t)(k * (2048 / 16)), ob_hi, idescV);
+      }
+      for (int gi = g_begin; gi < g_end; ++gi) {
+        const bool pair = gi < pairs;
+        const uint32_t dacc = tmem + 64 * (1 + 2 * gi), idg = pair ? idescK2 : idescV;
+        const uint32_t bl = qb_lo + (uint32_t)(2 * gi * (128 >> 4));
+        tc::mma_ss2pe(dacc, ca_lo, pa_hi, bl, qb_hi, idg, it != 0);
+#pragma unroll
+        for (int k = 1; k < BR / 16; ++k) tc::mma_ss2e<1>(dacc, ca_lo + (uint32_t)(k * 16), pa_hi, bl + (uint32_t)(k * (2048 / 16)), qb_hi, idg);
+      }
+      tc::mma_commit_e(&empty[st]);
+    }
+    if (ok) tc::mma_commit_e(all_done);
+  } else {
+    constexpr int NCG = Cfg::kEpWarps / 4;
+    const int qtr = warp & 3, cg = warp >> 2, row = qtr * 32 + lane, key = j0 + row;
+    const uint32_t tA = tmem + ((uint32_t)(qtr * 32) << 16);
+    bool ok = true;
+    if (nblk > 0) ok = __all_sync(0xffffffffu, tc::mbar_wait(all_done, 0, s_abort));
+    tc::tc_fence_after();
+    const bool have = nblk > 0 && ok;
+    // dKt leaves as (hi, lo) bf16 pairs (its adjoint takes bf16 operands; one rounding would be one more than dS K has): the hi
+    // tiles of all taps go through the stages (read by no MMA any more), then the lo tiles
+    for (int hl = 0; hl < (dK.out == nullptr ? 2 : 1); ++hl) {
+    for (int ch = cg + (hl ? 2 : 0); ch < 2 * (1 + cq); ch += NCG) {
+      const int acc = ch >> 1, half = ch & 1;
+      float o[32];
+      if (have) {
+        tc::tmem_ld32(tA + ch * 32, o);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = 0.f;
+      }
+      if (acc == 0 || dK.out != nullptr) {
+        const MixGradOut& t = acc == 0 ? dV : dK;
+        if (key < N) store_grad32(t.out, t.bf16_out, t.add, ((size_t)bh * N + key) * d + col0 + half * 32, o, t.mul);
+      } else {
+        unsigned char* tile = smem + (acc - 1) * Cfg::KT_BYTES + row * 128;
+        if (hl) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] -= __bfloat162float(__float2bfloat16_rn(o[i]));
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<uint4*>(tile + (((half * 4 + i) ^ (row & 7)) << 4)) =
+              make_uint4(pack_bf16(o[8 * i], o[8 * i + 1]), pack_bf16(o[8 * i + 2], o[8 * i + 3]), pack_bf16(o[8 * i + 4], o[8 * i + 5]), pack_bf16(o[8 * i + 6], o[8 * i + 7]));
+      }
+    }
+    if (dK.out == nullptr) {
+      tc::fence_proxy_async_smem();
+      tc::named_bar_sync(1, Cfg::kEpWarps * 32);
+      if (warp == 0 && tc::elect_one()) {
+        for (int t = 0; t < cq; ++t) tc::tma_store_3d(&tmdKt, smem + t * Cfg::KT_BYTES, col0, j0, (bh * cq + t) * 2 + hl);
+        tc::tma_store_commit();
+        tc::tma_store_wait_read();
+      }
+      tc::named_bar_sync(1, Cfg::kEpWarps * 32);
+    }
+    }
+  }
+  __syncwarp();
+  tc::tc_fence_before();
+  __syncthreads();
+  if (*s_abort) {
+    if (tid == 0) atomicExch(p.status, 1);
+    if (warp > W_TMA) tc::mma_commit_e(mma_drain);
+    if (tid == W_TMA * 32) {
+      volatile int never = 0;
+      const int issued = *s_issued;
+      for (int it = max(0, issued - NSTG); it < issued; ++it) tc::mbar_wait(&full[it % NSTG], (it / NSTG) & 1, &never);
+      tc::mbar_wait(mma_drain, 0, &never);
+    }
+    __syncthreads();
+  }
+  if (warp == W_A0) {
+    tc::tc_fence_after();
+    tc::tmem_dealloc(tmem, 512);
+  }
+}
+
+// ==========================================================================================
+namespace {
+template <int D>
+cudaError_t launch_pv_t(const TrainParams& p, const MixParams& mp, cudaStream_t stream) {
+  using Cfg = PvCfg<D>;
+  alignas(64) CUtensorMap tmV;
+  if (!make_tensor_map_bf16(&tmV, p.V, D, p.N, (size_t)p.B * p.H, 64, Cfg::BC, true)) return cudaErrorInvalidValue;
+  auto kern = mix_pv_kernel<D>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+  if (e != cudaSuccess) return e;
+  return launch_pdl(kern, dim3(mp.nRT, mp.nU * mp.G), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmV, mp, p.O, p.o_bf16, p.M, p.L, p.LSEout);
+}
+template <int D>
+cudaError_t launch_dq_t(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, cudaStream_t stream) {
+  using Cfg = MixDqCfg<D>;
+  const size_t BH = (size_t)p.B * p.H;
+  const bool conv = p.theta != nullptr;
+  alignas(64) CUtensorMap tmB;
+  if (!make_tensor_map_bf16(&tmB, conv ? Kt : p.K, D, p.N, conv ? BH * p.cq * 2 : BH, 64, Cfg::BC, true)) return cudaErrorInvalidValue;
+  auto kern = mix_dq_kernel<D>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+  if (e != cudaSuccess) return e;
+  const MixGradOut out = {p.dQo, conv && p.causal ? p.dQ : nullptr, p.grad_bf16, conv ? kLn2 : p.scale};
+  return launch_pdl(kern, dim3((mp.nRT + 1) / 2, mp.nU * mp.G), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmB, mp, conv ? p.cq : 1,
+                    conv ? 2 : 1, out);
+}
+}  // namespace
+
+cudaError_t launch_mix_pv(const TrainParams& p, const MixParams& mp, cudaStream_t stream) {
+  return p.d == 64 ? launch_pv_t<64>(p, mp, stream) : launch_pv_t<128>(p, mp, stream);
+}
+cudaError_t launch_mix_dq(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, cudaStream_t stream) {
+  return p.d == 64 ? launch_dq_t<64>(p, mp, Kt, stream) : launch_dq_t<128>(p, mp, Kt, stream);
+}
+cudaError_t launch_mix_dkdv(const TrainParams& p, const MixParams& mp, __nv_bfloat16* dKt, cudaStream_t stream) {
+  using Cfg = MixDkvCfg;
+  const size_t BH = (size_t)p.B * p.H;
+  const bool conv = p.theta != nullptr;
+  const int cq = conv ? p.cq : 1;
+  alignas(64) CUtensorMap tmQ, tmdO, tmdKt;
+  if (!make_tensor_map_bf16(&tmQ, p.Q, p.d, p.N, BH, 64, Cfg::QR, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmdO, p.dO, p.d, p.N, BH, 64, Cfg::BR, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmdKt, conv ? dKt : p.Q, p.d, p.N, conv ? BH * cq * 2 : BH, 64, Cfg::BK, true)) return cudaErrorInvalidValue;
+  cudaError_t e = cudaFuncSetAttribute(mix_dkdv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+  if (e != cudaSuccess) return e;
+  const MixGradOut dV = {p.dVo, nullptr, p.grad_bf16, 1.f}, dK = {conv ? nullptr : p.dKo, nullptr, p.grad_bf16, p.scale};
+  return launch_pdl(mix_dkdv_kernel, dim3(mp.N8 / 128 * (p.d / 64), mp.nU * mp.G), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmQ, tmdO,
+                    tmdKt, mp, cq, p.d, dV, dK);
+}
+
+}  // namespace fmta

@@ -1,0 +1,689 @@
+// Scores, mix and softmax terms of head-mixing attention (see mix_tc.cuh): one kernel for forward and backward, with and
+// without a key-query filter.
+//
+// CTA = 128 query rows x one chunk of keys x all G heads of a group.  Warp roles: 8 element-wise warps (row = TMEM lane, two
+// warps per lane quarter split the keys of a block), a TMA warp, an MMA warp.  Per block of KB keys the G score tiles
+// 128 x KB lie side by side in tensor memory; an element-wise thread reads KT keys of every head, mixes them in registers
+// (packed fp32 FMAs, weights broadcast from shared memory) and goes on to
+//   forward : P = exp2(C' - ref) as bf16 (ref: one value per row, head and key chunk), row max and sum
+//   backward: P = exp2(C' - LSE), dC' = P (dP - D), the transposed mix dC, dW; P and dC as bf16
+// Bound: without a filter the FP32 pipe (G FMAs per score entry and pass over the heads: 1 forward, 2 backward, dW aside);
+// with one the stacked score MMAs (2 c_q d / 16 per tile).  With a filter the stacked key operand is a bf16 pair (hi, lo), so
+// that the logits keep 16 mantissa bits as the unstacked products followed by an fp32 filter did.
+//
+// Without a filter neither Q nor dO of 16 heads fits shared memory, so their tiles stream through the ring once per block
+// beside K and V (18 bytes per score entry from L2); with a filter Q stays resident where it fits and the stacked keys stream.
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include "mix_tc.cuh"
+
+namespace fmta {
+
+template <int G, int D, bool CONV, bool BWD>
+struct MixCfg {
+  static constexpr int BM = 128, SL = D / 64, HALO = 8, QR = BM + HALO;
+  // keys per block: S and dP (backward) or two buffers of S (forward with a filter, where the MMAs are the bound) take 256
+  // columns each; otherwise one buffer of up to 512
+  static constexpr int KB = (BWD || (CONV && G <= 8)) ? 256 / G : (512 / G < 128 ? 512 / G : 128);
+  static constexpr int NBUF = BWD ? 1 : 512 / (G * KB);
+  static constexpr int KT = G >= 8 ? 4 : 8;                    // keys per thread and pass
+  static constexpr int GC = G < 4 ? G : 4;                     // output heads per register pass
+  static constexpr int NPASS = KB / 2 / KT;
+  static constexpr bool RES = CONV && G * SL * QR * 128 <= 140 * 1024;   // Q resident
+  static constexpr int SLOT = CONV ? QR * 128 : BM * 128;      // ring slot: one A slab tile, or B slab tiles
+  static constexpr int TB = KB * 128, TPS = 16384 / TB;        // B slab tile (KB keys x 64 columns), tiles per slot
+  static constexpr bool DW_MMA = BWD && G == 16;               // dW by mma.sync from transposed bf16 pairs; else in registers
+  static constexpr int oQ = 0;
+  static constexpr int oW = oQ + (RES ? G * SL * QR * 128 : 0);
+  static constexpr int W_BYTES = G * G * 8;                    // (w, w) pairs
+  static constexpr int oRow = oW + (BWD ? 2 : 1) * ((W_BYTES + 127) / 128 * 128);   // backward: LSE, D; forward: ref, exchange
+  static constexpr int oDW = oRow + 2 * G * BM * 4;
+  static constexpr int DW_BYTES = DW_MMA ? 8 * 4096 : (BWD ? 8 * G * G * 4 : 0);
+  static constexpr int oBar = oDW + DW_BYTES;
+  static constexpr int oRing = (oBar + 512 + 1023) / 1024 * 1024;
+  static constexpr int NSLOT_ = (226 * 1024 - oRing) / SLOT;
+  static constexpr int NSLOT = NSLOT_ > 20 ? 20 : NSLOT_;
+  // a slot is held until the last tile that uses it: B tiles of several heads in one slot, with an A slot for each, and (Q not
+  // resident) the Q slots of a head while its stacked keys pass
+  static constexpr int TPP = TPS < NSLOT - 2 ? TPS : NSLOT - 2;
+  static constexpr int kSmemBytes = oRing + NSLOT * SLOT + 1024;
+  // 8 element-wise warps with 216 registers, a warpgroup with 72 for the TMA and the MMA warp: 256 * 216 + 128 * 72 = 384 * 168,
+  // the registers the block is launched with
+  static constexpr int kThreads = 384, kRegsEw = 216, kRegsOther = 72;
+  static_assert(NSLOT >= 4 && (RES || !CONV || NSLOT >= SL + (7 * 2 * SL + TPS - 1) / TPS), "ring");
+  static_assert(kSmemBytes <= 227 * 1024, "shared memory");
+  static_assert(SLOT % 1024 == 0 && TB % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
+};
+
+template <int G, int D, bool CONV, bool BWD>
+__global__ void __launch_bounds__(384, 1)
+mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmB,
+                 const __grid_constant__ CUtensorMap tmdO, const __grid_constant__ CUtensorMap tmV, const MixParams p) {
+  using Cfg = MixCfg<G, D, CONV, BWD>;
+  constexpr int BM = Cfg::BM, SL = Cfg::SL, HALO = Cfg::HALO, KB = Cfg::KB, KT = Cfg::KT, GC = Cfg::GC, NPASS = Cfg::NPASS;
+  constexpr int SLOT = Cfg::SLOT, NSLOT = Cfg::NSLOT, TB = Cfg::TB, TPS = Cfg::TPS, TPP = Cfg::TPP, NBUF = Cfg::NBUF;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* sQ = smem + Cfg::oQ;
+  unsigned char* sRing = smem + Cfg::oRing;
+  uint64_t* sWf = reinterpret_cast<uint64_t*>(smem + Cfg::oW);                 // [g'][g] (w, w): the mix
+  uint64_t* sWb = reinterpret_cast<uint64_t*>(smem + Cfg::oW + (Cfg::W_BYTES + 127) / 128 * 128);   // [g][g']: its transpose
+  float* sR0 = reinterpret_cast<float*>(smem + Cfg::oRow);                      // [G][128]: LSE (log2) / ref
+  float* sR1 = sR0 + G * BM;                                                    // [G][128]: D / exchange
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::oBar);
+  uint64_t* full = bars;                 // [NSLOT]
+  uint64_t* empty = full + NSLOT;        // [NSLOT]
+  uint64_t* q_full = empty + NSLOT;
+  uint64_t* s_full = q_full + 1;         // [2]
+  uint64_t* s_free = s_full + 2;         // [2]
+  uint64_t* d_full = s_free + 2;
+  uint64_t* d_free = d_full + 1;
+  uint64_t* x_bar = d_free + 1;          // the element-wise warps meet (bounded, unlike a named barrier)
+  uint64_t* mma_drain = x_bar + 1;
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(mma_drain + 1);
+  volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
+  volatile int* s_issued = s_abort + 1;
+  volatile int* s_redo = s_abort + 2;    // forward: a logit left the range of P around the row's reference
+  static_assert((2 * NSLOT + 9) * 8 + 16 <= 512, "barrier block");
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int N = p.N, cq = CONV ? p.cq : 1, pq = cq - 1, pk = CONV ? (p.ck - 1) / 2 : 0;
+  const int band = CONV && p.causal ? pq + pk : 0;
+  // row tiles from the last (most keys) on; the key chunks of a row tile side by side
+  const int kc = blockIdx.x % p.nKC, rt = p.nRT - 1 - blockIdx.x / p.nKC, ul = blockIdx.y;
+  const int u = p.u0 + ul, HG = p.H / G, b = u / HG, grp = u - b * HG;
+  const int bh0 = b * p.H + grp * G;                         // first head of the group
+  const int R0 = rt * BM;
+  const int k_lo = kc * p.kch;
+  const int k_hi = min(min(k_lo + p.kch, p.N8), p.causal ? R0 + BM : p.N8);     // multiples of 128
+  const int nblk = k_hi > k_lo ? (k_hi - k_lo) / KB : 0;
+
+  if (tid == 0) {
+    for (int i = 0; i < NSLOT; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 1); }
+    tc::mbar_init(q_full, 1); tc::mbar_init(d_full, 1); tc::mbar_init(d_free, 8); tc::mbar_init(x_bar, 8); tc::mbar_init(mma_drain, 1);
+    for (int i = 0; i < 2; ++i) { tc::mbar_init(&s_full[i], 1); tc::mbar_init(&s_free[i], 8); }
+    *s_abort = 0; *s_issued = 0; *s_redo = 0;
+    tc::mbar_fence_init();
+  }
+  if (warp == 9) {
+    tc::tmem_alloc(s_tmem, 512);
+    tc::tmem_relinquish();
+  }
+  tc::tc_fence_before();
+  pdl_wait();
+  pdl_trigger();
+  for (int i = tid; i < G * G; i += Cfg::kThreads) {
+    const float w = p.W[(size_t)grp * G * G + i];            // [g][g']
+    const int g = i / G, g2 = i % G;
+    sWf[g2 * G + g] = f2_pack(w * p.c2, w * p.c2);
+    if (BWD) sWb[g * G + g2] = f2_pack(w, w);
+  }
+  for (int i = tid; i < G * BM; i += Cfg::kThreads) {
+    const int g = i / BM, r = R0 + i % BM;
+    if (BWD) {
+      sR0[i] = r < N ? p.LSE[(size_t)(bh0 + g) * N + r] * kLog2e : 0.f;
+      sR1[i] = r < N ? p.Dvec[(size_t)(bh0 + g) * N + r] : 0.f;
+    } else {
+      sR0[i] = -INFINITY;
+    }
+  }
+  __syncthreads();
+  tc::tc_fence_after();
+  const uint32_t tmem = *s_tmem;
+  int ring = 0, meets = 0;               // ring position (warps 8 and 9) and meetings of the element-wise warps, over all attempts
+
+  // forward: a second attempt only when a logit exceeds its row's reference (the maximum of the first keys) by 2^100
+  const int attempts = nblk > 0 ? (BWD ? 1 : 2) : 0;
+  auto attempt_done = [&]() -> bool {                        // every warp, after each attempt
+    __syncwarp();
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    return BWD || !*s_redo || *s_abort;
+  };
+  if (warp >= 8) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::kRegsOther));
+  if (warp == 8) {
+    // ===================== TMA producer =====================
+    for (int attempt = 0; attempt < attempts; ++attempt) {
+    if (lane == 0) {
+      bool ok = true;
+      auto slot_of = [&](uint32_t bytes) -> int {            // waits for the slot, arms its barrier
+        const int slot = ring % NSLOT, ph = (ring / NSLOT) & 1;
+        if (!tc::mbar_wait(&empty[slot], ph ^ 1, s_abort)) { ok = false; return slot; }
+        tc::mbar_expect_tx(&full[slot], bytes);
+        ++ring;
+        *s_issued = ring;
+        return slot;
+      };
+      if (Cfg::RES && attempt == 0) {
+        tc::mbar_expect_tx(q_full, G * SL * Cfg::QR * 128);
+        for (int i = 0; i < G * SL; ++i) tc::tma_load_3d(sQ + i * (Cfg::QR * 128), &tmQ, q_full, (i % SL) * 64, R0 - HALO, bh0 + i / SL);
+      }
+      // the B tiles of one head pair up in slots; A and B in the order the MMA warp takes them
+      auto plain = [&](const CUtensorMap* ta, const CUtensorMap* tb, int key) {
+        for (int i = 0; i < G * SL && ok; ++i) {
+          if (i % TPP == 0) {
+            const int n = min(TPP, G * SL - i), s = slot_of(n * TB);
+            if (!ok) return;
+            for (int j = 0; j < n; ++j) tc::tma_load_3d(sRing + s * SLOT + j * TB, tb, &full[s], ((i + j) % SL) * 64, key, bh0 + (i + j) / SL);
+          }
+          const int s = slot_of(BM * 128);
+          if (!ok) return;
+          tc::tma_load_3d(sRing + s * SLOT, ta, &full[s], (i % SL) * 64, R0, bh0 + i / SL);
+        }
+      };
+      auto stacked = [&](int key) {
+        const int nt = cq * 2 * SL;                          // (tap, hi / lo, slab) tiles of a head
+        for (int g = 0; g < G && ok; ++g) {
+          if (!Cfg::RES)
+            for (int sl = 0; sl < SL && ok; ++sl) {
+              const int s = slot_of(Cfg::QR * 128);
+              if (ok) tc::tma_load_3d(sRing + s * SLOT, &tmQ, &full[s], sl * 64, R0 - HALO, bh0 + g);
+            }
+          for (int i = 0; i < nt && ok; i += TPS) {
+            const int n = min(TPS, nt - i), s = slot_of(n * TB);
+            if (!ok) return;
+            for (int j = 0; j < n; ++j)
+              tc::tma_load_3d(sRing + s * SLOT + j * TB, &tmB, &full[s], ((i + j) % SL) * 64, key, (bh0 + g) * cq * 2 + (i + j) / SL);
+          }
+        }
+      };
+      for (int kb = 0; kb < nblk && ok; ++kb) {
+        const int key = k_lo + kb * KB;
+        if constexpr (CONV) stacked(key); else plain(&tmQ, &tmB, key);
+        if constexpr (BWD) { if (ok) plain(&tmdO, &tmV, key); }
+      }
+    }
+    if (attempt_done()) break;
+    }
+  } else if (warp == 9) {
+    // ===================== MMA issuer: all lanes run the loop; one elected lane issues =====================
+    for (int attempt = 0; attempt < attempts; ++attempt) {
+    constexpr uint32_t idesc = tc::make_idesc(BM, KB, 0, 0);
+    const uint64_t d0 = tc::make_sdesc(smem_u32(sRing), 16, 1024, tc::kLayoutSW128);
+    const uint32_t hi = (uint32_t)(d0 >> 32), lo0 = (uint32_t)d0;
+    const uint32_t q_lo = (uint32_t)tc::make_sdesc(smem_u32(sQ), 16, 1024, tc::kLayoutSW128);
+    bool ok = true;
+    auto take = [&]() -> int {
+      const int slot = ring % NSLOT, ph = (ring / NSLOT) & 1;
+      if (!tc::mbar_wait_warp(&full[slot], ph, s_abort)) { ok = false; return slot; }
+      tc::tc_fence_after();
+      ++ring;
+      return slot;
+    };
+    auto mma4 = [&](uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t acc) {
+      tc::mma_ss2pe(d, a_lo, hi, b_lo, hi, idesc, acc);
+#pragma unroll
+      for (int k = 1; k < 4; ++k) tc::mma_ss2e<1>(d, a_lo + 2 * k, hi, b_lo + 2 * k, hi, idesc);
+    };
+    auto plain = [&](uint32_t dst) {
+      int bs = 0;
+      for (int i = 0; i < G * SL && ok; ++i) {
+        if (i % TPP == 0) bs = take();
+        if (!ok) return;
+        const int s = take();
+        if (!ok) return;
+        mma4(dst + (i / SL) * KB, lo0 + (uint32_t)(s * (SLOT >> 4)), lo0 + (uint32_t)(bs * (SLOT >> 4) + (i % TPP) * (TB >> 4)), i % SL != 0);
+        tc::mma_commit_e(&empty[s]);
+        if (i % TPP == TPP - 1 || i == G * SL - 1) tc::mma_commit_e(&empty[bs]);
+      }
+    };
+    auto stacked = [&](uint32_t dst) {
+      const int nt = cq * 2 * SL;
+      for (int g = 0; g < G && ok; ++g) {
+        uint32_t a0[SL];
+        int qs[SL];
+#pragma unroll
+        for (int sl = 0; sl < SL; ++sl) {
+          if (Cfg::RES) { a0[sl] = q_lo + (uint32_t)((g * SL + sl) * (Cfg::QR * 8)); qs[sl] = 0; }
+          else { qs[sl] = take(); if (!ok) return; a0[sl] = lo0 + (uint32_t)(qs[sl] * (SLOT >> 4)); }
+          a0[sl] += (uint32_t)((HALO - pq) * 8);             // row shift: 128 bytes per row
+        }
+        for (int i = 0; i < nt; i += TPS) {
+          const int s = take();
+          if (!ok) return;
+          const int n = min(TPS, nt - i);
+          for (int j = 0; j < n; ++j) {
+            const int a = (i + j) / (2 * SL), sl = (i + j) % SL;
+            mma4(dst + g * KB, (SL > 1 && sl ? a0[SL - 1] : a0[0]) + (uint32_t)(a * 8), lo0 + (uint32_t)(s * (SLOT >> 4) + j * (TB >> 4)), i + j != 0);
+          }
+          tc::mma_commit_e(&empty[s]);
+        }
+        if (!Cfg::RES)
+#pragma unroll
+          for (int sl = 0; sl < SL; ++sl) tc::mma_commit_e(&empty[qs[sl]]);
+      }
+    };
+    if (Cfg::RES && attempt == 0) ok = tc::mbar_wait_warp(q_full, 0, s_abort);
+    for (int kb = 0; kb < nblk && ok; ++kb) {
+      const int it = attempt * nblk + kb;                    // uses of the buffers over both attempts
+      const int bf = it % NBUF, ub = it / NBUF;
+      if (ub > 0) { ok = tc::mbar_wait_warp(&s_free[bf], (ub - 1) & 1, s_abort); tc::tc_fence_after(); }
+      if (!ok) break;
+      if constexpr (CONV) stacked(tmem + bf * (G * KB)); else plain(tmem + bf * (G * KB));
+      if (!ok) break;
+      tc::mma_commit_e(&s_full[bf]);
+      if constexpr (BWD) {
+        if (kb > 0) { ok = tc::mbar_wait_warp(d_free, (kb - 1) & 1, s_abort); tc::tc_fence_after(); }
+        if (!ok) break;
+        plain(tmem + 256);
+        if (ok) tc::mma_commit_e(d_full);
+      }
+    }
+    if (attempt_done()) break;
+    }
+  } else if (warp > 9) {
+    for (int attempt = 0; attempt < attempts; ++attempt)
+      if (attempt_done()) break;
+  } else {
+    // ===================== element-wise warps =====================
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::kRegsEw));
+    for (int attempt = 0; attempt < attempts; ++attempt) {
+    const int qtr = warp & 3, hf = warp >> 2;
+    const int r = qtr * 32 + lane, gi = R0 + r;              // row of the tile = TMEM lane; query index
+    const uint32_t tS0 = tmem + ((uint32_t)(qtr * 32) << 16) + hf * (KB / 2);
+    const int jlim = gi < N ? (p.causal ? min(gi, N - 1) : N - 1) : -1;        // last key of this row
+    const size_t lh0 = (size_t)ul * G;
+    const size_t kc8 = p.N8 / 8;
+    bool ok = true;
+    constexpr int KP = KT / 2;
+    auto meet = [&]() {                                      // false: a wait ran out somewhere
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(x_bar);
+      const bool good = __all_sync(0xffffffffu, tc::mbar_wait(x_bar, meets & 1, s_abort));
+      ++meets;
+      return good;
+    };
+    // S of this thread's keys of a pass, all heads, as key pairs; with a filter and a causal mask the entries of the band
+    // come from the band kernel (the stacked product does not hold there)
+    auto load_s = [&](uint64_t (&s)[G][KP], uint32_t base, int j0) {
+      float v[G][KT];
+#pragma unroll
+      for (int g = 0; g < G; ++g) tmem_ld_nowait<KT>(base + g * KB, v[g]);
+      tc::tmem_wait_ld();
+      if (CONV && band > 0 && gi < N && j0 + KT - 1 > gi - band && j0 <= gi) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          const float* cb = p.Cband + ((size_t)(bh0 + g) * N + gi) * band;
+#pragma unroll
+          for (int k = 0; k < KT; ++k) {
+            const int e = gi - (j0 + k);
+            if (e >= 0 && e < band) v[g][k] = cb[e] * kLog2e;
+          }
+        }
+      }
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int k = 0; k < KP; ++k) s[g][k] = f2_pack(v[g][2 * k], v[g][2 * k + 1]);
+    };
+    // acc[c] = sum_x tab[x][g0 + c] * in[x]
+    auto mix = [&](uint64_t (&acc)[GC][KP], const uint64_t (&in)[G][KP], const uint64_t* tab, int g0) {
+#pragma unroll
+      for (int x = 0; x < G; ++x) {
+        uint64_t w[GC];
+#pragma unroll
+        for (int c = 0; c < GC; c += 2) {
+          const ulonglong2 t2 = *reinterpret_cast<const ulonglong2*>(tab + x * G + g0 + c);
+          w[c] = t2.x; w[c + 1] = t2.y;
+        }
+#pragma unroll
+        for (int c = 0; c < GC; ++c)
+#pragma unroll
+          for (int k = 0; k < KP; ++k) acc[c][k] = x == 0 ? f2_mul(w[c], in[x][k]) : f2_fma(w[c], in[x][k], acc[c][k]);
+      }
+    };
+    auto store8 = [&](bf16* base, size_t lh, int key, const uint32_t (&w)[KP]) {   // KT keys of this row, X8 layout
+      bf16* dst = base + ((lh * kc8 + (key >> 3)) * p.RP + gi) * 8 + (key & 7);
+      if constexpr (KT == 8) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+      else *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+    };
+
+    if constexpr (!BWD) {
+      float mt[G], l[G];
+#pragma unroll
+      for (int g = 0; g < G; ++g) { mt[g] = attempt == 0 ? -INFINITY : sR1[g * BM + r]; l[g] = 0.f; }
+      // row maximum of this thread's valid keys of a block -> ref (both halves of a row agree on one value)
+      auto init_ref = [&](uint32_t base, int j0) {
+        const bool whole = k_lo + KB <= N && (!p.causal || j0 - hf * (KB / 2) + KB - 1 <= R0);   // every key valid for every row
+#pragma unroll 1
+        for (int ps = 0; ps < (whole ? 1 : NPASS); ++ps) {
+          const int j = j0 + ps * KT;
+          uint64_t s[G][KP];
+          load_s(s, base + ps * KT, j);
+#pragma unroll
+          for (int g0 = 0; g0 < G; g0 += GC) {
+            uint64_t acc[GC][KP];
+            mix(acc, s, sWf, g0);
+#pragma unroll
+            for (int c = 0; c < GC; ++c) {
+              float mx = -INFINITY;
+#pragma unroll
+              for (int k = 0; k < KP; ++k) {
+                float a, bb;
+                f2_unpack(acc[c][k], a, bb);
+                if (j + 2 * k <= jlim) mx = fmaxf(mx, a);
+                if (j + 2 * k + 1 <= jlim) mx = fmaxf(mx, bb);
+              }
+              float* x = sR1 + (g0 + c) * BM + r;
+              if (hf == 1) *x = ps == 0 ? mx : fmaxf(*x, mx);                  // one half leaves its maxima,
+              else mt[g0 + c] = fmaxf(mt[g0 + c], mx);
+            }
+          }
+        }
+        if (!meet()) return false;
+        if (hf == 0)
+#pragma unroll
+          for (int g = 0; g < G; ++g) {                                        // the other merges
+            const float m2 = fmaxf(mt[g], sR1[g * BM + r]);
+            if (sR0[g * BM + r] == -INFINITY) sR0[g * BM + r] = m2;
+          }
+        return meet();
+      };
+      bool redo = false;
+      for (int kb = 0; kb < nblk; ++kb) {
+        const int it = attempt * nblk + kb, bf = it % NBUF;
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(&s_full[bf], (it / NBUF) & 1, s_abort));
+        if (!ok) break;
+        tc::tc_fence_after();
+        const uint32_t base = tS0 + bf * (G * KB);
+        const int j0 = k_lo + kb * KB + hf * (KB / 2);
+        // rows whose first valid key is not in block 0 exist only on the diagonal
+        if (attempt == 0 && (kb == 0 || (p.causal && k_lo + kb * KB + KB - 1 > R0))) ok = init_ref(base, j0);
+        if (!ok) break;
+#pragma unroll 1
+        for (int ps = 0; ps < NPASS; ++ps) {
+          const int j = j0 + ps * KT;
+          uint64_t s[G][KP];
+          load_s(s, base + ps * KT, j);
+          if (ps == NPASS - 1) {
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&s_free[bf]);
+          }
+          const bool mask = !__all_sync(0xffffffffu, j + KT - 1 <= jlim);
+#pragma unroll
+          for (int g0 = 0; g0 < G; g0 += GC) {
+            uint64_t acc[GC][KP];
+            mix(acc, s, sWf, g0);
+#pragma unroll
+            for (int c = 0; c < GC; ++c) {
+              float v[KT];
+#pragma unroll
+              for (int k = 0; k < KP; ++k) f2_unpack(acc[c][k], v[2 * k], v[2 * k + 1]);
+              if (mask) {
+#pragma unroll
+                for (int k = 0; k < KT; ++k) if (j + k > jlim) v[k] = -INFINITY;
+              }
+              float mx = v[0];
+#pragma unroll
+              for (int k = 1; k < KT; ++k) mx = fmaxf(mx, v[k]);
+              const float rf = sR0[(g0 + c) * BM + r], ref = rf == -INFINITY ? 0.f : rf;
+              redo |= mx > ref + 100.f;
+              mt[g0 + c] = fmaxf(mt[g0 + c], mx);
+              float sum = 0.f;
+              uint32_t w[KP];
+#pragma unroll
+              for (int k = 0; k < KT; k += 2) {
+                const float p0 = exp2f(v[k] - ref), p1 = exp2f(v[k + 1] - ref);
+                sum += p0 + p1;
+                w[k / 2] = pack_bf16(p0, p1);
+              }
+              l[g0 + c] += sum;
+              store8(p.P8, lh0 + g0 + c, j, w);
+            }
+          }
+        }
+      }
+      if (ok) {
+        const size_t ns = 2 * (size_t)p.nKC;
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          float* st = p.stat + (((lh0 + g) * ns + 2 * kc + hf) * 3) * p.RP + gi;
+          st[0] = mt[g]; st[p.RP] = sR0[g * BM + r]; st[2 * (size_t)p.RP] = l[g];
+        }
+        if (attempt == 0 && redo) *s_redo = 1;
+      }
+      // for the second attempt: the true maxima of the row, both halves
+      ok = ok && meet();
+      if (ok && *s_redo && attempt == 0) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) if (hf == 1) sR1[g * BM + r] = mt[g];
+        ok = meet();
+        if (ok && hf == 0)
+#pragma unroll
+          for (int g = 0; g < G; ++g) sR0[g * BM + r] = sR1[g * BM + r] = fmaxf(mt[g], sR1[g * BM + r]);
+      }
+    } else {
+      // ---- backward ----
+      constexpr bool DWM = Cfg::DW_MMA;
+      float dw[DWM ? 8 : G * G];
+#pragma unroll
+      for (int i = 0; i < (DWM ? 8 : G * G); ++i) dw[i] = 0.f;
+      for (int kb = 0; kb < nblk; ++kb) {
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(s_full, kb & 1, s_abort) && tc::mbar_wait(d_full, kb & 1, s_abort));
+        if (!ok) break;
+        tc::tc_fence_after();
+        const int j0 = k_lo + kb * KB + hf * (KB / 2);
+#pragma unroll 1
+        for (int ps = 0; ps < NPASS; ++ps) {
+          const int j = j0 + ps * KT;
+          uint64_t s[G][KP], dc[G][KP];
+          load_s(s, tS0 + ps * KT, j);
+          const bool mask = !__all_sync(0xffffffffu, j + KT - 1 <= jlim);
+#pragma unroll
+          for (int g0 = 0; g0 < G; g0 += GC) {
+            float dp[GC][KT];
+#pragma unroll
+            for (int c = 0; c < GC; ++c) tmem_ld_nowait<KT>(tS0 + 256 + (g0 + c) * KB + ps * KT, dp[c]);
+            uint64_t acc[GC][KP];
+            mix(acc, s, sWf, g0);
+            tc::tmem_wait_ld();
+#pragma unroll
+            for (int c = 0; c < GC; ++c) {
+              const float lse = sR0[(g0 + c) * BM + r], dv = sR1[(g0 + c) * BM + r];
+              uint32_t w[KP];
+#pragma unroll
+              for (int k = 0; k < KP; ++k) {
+                float a, bb;
+                f2_unpack(acc[c][k], a, bb);
+                a = exp2f(a - lse); bb = exp2f(bb - lse);
+                if (mask) { if (j + 2 * k > jlim) a = 0.f; if (j + 2 * k + 1 > jlim) bb = 0.f; }
+                w[k] = pack_bf16(a, bb);
+                dc[g0 + c][k] = f2_pack(a * (dp[c][2 * k] - dv), bb * (dp[c][2 * k + 1] - dv));
+              }
+              store8(p.P8, lh0 + g0 + c, j, w);
+            }
+          }
+          if (ps == NPASS - 1) {                             // both tiles are in registers
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) { tc::mbar_arrive(s_free); tc::mbar_arrive(d_free); }
+          }
+          // ---- dC_x = sum_g W[g,x] dC'_g ----
+#pragma unroll
+          for (int x0 = 0; x0 < G; x0 += GC) {
+            uint64_t acc[GC][KP];
+            mix(acc, dc, sWb, x0);
+#pragma unroll
+            for (int c = 0; c < GC; ++c) {
+              float v[KT];
+#pragma unroll
+              for (int k = 0; k < KP; ++k) f2_unpack(acc[c][k], v[2 * k], v[2 * k + 1]);
+              if (CONV && band > 0 && gi < N && j + KT - 1 > gi - band && j <= gi) {   // the band's gradient goes its own way
+                float* cb = p.dCband + ((size_t)(bh0 + x0 + c) * N + gi) * band;
+#pragma unroll
+                for (int k = 0; k < KT; ++k) {
+                  const int e = gi - (j + k);
+                  if (e >= 0 && e < band) { cb[e] = v[k]; v[k] = 0.f; }
+                }
+              }
+              uint32_t w[KP];
+#pragma unroll
+              for (int k = 0; k < KP; ++k) w[k] = pack_bf16(v[2 * k], v[2 * k + 1]);
+              store8(p.C8, lh0 + x0 + c, j, w);
+            }
+          }
+          // ---- dW[g][x] += sum dC'_g S_x ----
+          // masked entries have dC' = 0; S is finite there
+          if constexpr (!DWM) {
+#pragma unroll
+            for (int g = 0; g < G; ++g)
+#pragma unroll
+              for (int x = 0; x < G; ++x) {
+                float t = dw[g * G + x];
+#pragma unroll
+                for (int k = 0; k < KP; ++k) {
+                  float a, bb, c, d;
+                  f2_unpack(dc[g][k], a, bb); f2_unpack(s[x][k], c, d);
+                  t = fmaf(a, c, t); t = fmaf(bb, d, t);
+                }
+                dw[g * G + x] = t;
+              }
+          } else {
+            // 16 x 16 heads over 32 rows x KT keys: the contraction runs over the lanes, so each key's 32 x 16 values go through
+            // shared memory as bf16 pairs (hi, lo: 16 mantissa bits) and come back as transposed fragments;
+            // hi hi + hi lo + lo hi.  Rows of 32 bytes, their two chunks swapped every four rows (no bank conflicts).
+            unsigned char* st = smem + Cfg::oDW + warp * 4096;
+            const int swz = (lane >> 2) & 1;
+            auto put = [&](int off, const uint64_t (&v)[G][KP], int k) {       // hi at off, lo at off + 1024
+              uint32_t h[8], lo[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                float a0, a1, b0, b1;
+                f2_unpack(v[2 * i][k >> 1], a0, a1); f2_unpack(v[2 * i + 1][k >> 1], b0, b1);
+                const float x = (k & 1) ? a1 : a0, y = (k & 1) ? b1 : b0;
+                h[i] = pack_bf16(x, y);
+                lo[i] = pack_bf16(x - __uint_as_float(h[i] << 16), y - __uint_as_float(h[i] & 0xffff0000u));
+              }
+              unsigned char* d = st + off + lane * 32;
+              *reinterpret_cast<uint4*>(d + 16 * swz) = make_uint4(h[0], h[1], h[2], h[3]);
+              *reinterpret_cast<uint4*>(d + 16 * (swz ^ 1)) = make_uint4(h[4], h[5], h[6], h[7]);
+              *reinterpret_cast<uint4*>(d + 1024 + 16 * swz) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+              *reinterpret_cast<uint4*>(d + 1024 + 16 * (swz ^ 1)) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+            };
+            const int l8 = lane & 7, q = lane >> 3;
+#pragma unroll
+            for (int k = 0; k < KT; ++k) {
+              __syncwarp();
+              put(0, dc, k);
+              put(2048, s, k);
+              __syncwarp();
+#pragma unroll
+              for (int ks = 0; ks < 2; ++ks) {               // 16 rows per step
+                // A: stored [row][head], chunk = head / 8; matrices (heads 0-7, rows 0-7) (8-15, 0-7) (0-7, 8-15) (8-15, 8-15)
+                const int ra = 16 * ks + l8 + (q >> 1) * 8, ca = (q & 1) ^ ((ra >> 2) & 1);
+                // B: matrices (rows 0-7, heads 0-7) (8-15, 0-7) (0-7, 8-15) (8-15, 8-15)
+                const int rb = 16 * ks + l8 + (q & 1) * 8, cb = (q >> 1) ^ ((rb >> 2) & 1);
+                uint32_t ah[4], al[4], bh[4], bl[4];
+                ldsm_x4_t(ah, st + ra * 32 + ca * 16);
+                ldsm_x4_t(al, st + 1024 + ra * 32 + ca * 16);
+                ldsm_x4_t(bh, st + 2048 + rb * 32 + cb * 16);
+                ldsm_x4_t(bl, st + 3072 + rb * 32 + cb * 16);
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+                  float (&acc)[4] = reinterpret_cast<float (&)[4]>(dw[4 * n]);
+                  mma_bf16(acc, ah, bh[2 * n], bh[2 * n + 1]);
+                  mma_bf16(acc, ah, bl[2 * n], bl[2 * n + 1]);
+                  mma_bf16(acc, al, bh[2 * n], bh[2 * n + 1]);
+                }
+              }
+            }
+          }
+        }
+      }
+      // ---- dW partial of the CTA ----
+      __syncwarp();
+      float* red = reinterpret_cast<float*>(smem + Cfg::oDW) + warp * (G * G);
+      if constexpr (DWM) {
+        red = reinterpret_cast<float*>(smem + Cfg::oDW + warp * 4096);
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) red[((lane >> 2) + 8 * (i >> 1)) * 16 + 8 * n + 2 * (lane & 3) + (i & 1)] = dw[4 * n + i];
+      } else {
+#pragma unroll
+        for (int i = 0; i < G * G; ++i) {
+          const float t = warp_sum(dw[i]);
+          if (lane == 0) red[i] = t;
+        }
+      }
+      // the rows past the padded tile that a shifted dC operand of the last row tile reads
+      if (rt == p.nRT - 1 && ok) {
+        const int nch = (k_hi - k_lo) / 8;
+        for (int i = tid; i < G * nch * 16; i += 256) {
+          const int g = i / (nch * 16), rem = i - g * nch * 16;
+          *reinterpret_cast<uint4*>(p.C8 + (((lh0 + g) * kc8 + (k_lo >> 3) + (rem >> 4)) * p.RP + p.nRT * BM + (rem & 15)) * 8) = make_uint4(0u, 0u, 0u, 0u);
+        }
+      }
+    }
+    if (attempt_done()) break;
+    }
+  }
+  __syncthreads();
+
+  if constexpr (BWD) {
+    const int slot = (b * p.nRT + rt) * p.nKC + kc;
+    float* out = p.dW_part + ((size_t)slot * HG + grp) * (G * G);
+    for (int i = tid; i < G * G; i += Cfg::kThreads) {
+      float t = 0.f;
+      if (nblk > 0)
+        for (int w = 0; w < 8; ++w) t += reinterpret_cast<const float*>(smem + Cfg::oDW + w * (Cfg::DW_MMA ? 4096 : G * G * 4))[i];
+      out[i] = t * p.cw;
+    }
+  }
+  if (*s_abort) {
+    if (tid == 0) atomicExch(p.status, 1);
+    // nothing of this CTA may still be in flight when its shared and tensor memory are given up
+    if (warp == 9) tc::mma_commit_e(mma_drain);
+    if (tid == 256) {
+      volatile int never = 0;
+      if (Cfg::RES && nblk > 0) tc::mbar_wait(q_full, 0, &never);
+      const int issued = *s_issued;
+      for (int id = max(0, issued - NSLOT); id < issued; ++id) tc::mbar_wait(&full[id % NSLOT], (id / NSLOT) & 1, &never);
+    }
+    if (tid == 256) { volatile int never = 0; tc::mbar_wait(mma_drain, 0, &never); }
+    __syncthreads();
+  }
+  if (warp == 9) {
+    tc::tc_fence_after();
+    tc::tmem_dealloc(tmem, 512);
+  }
+}
+
+// ------------------------------------------------------------------------------------------
+namespace {
+
+template <int G, int D, bool CONV, bool BWD>
+cudaError_t launch_score_t(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, cudaStream_t stream) {
+  using Cfg = MixCfg<G, D, CONV, BWD>;
+  const size_t BH = (size_t)p.B * p.H;
+  alignas(64) CUtensorMap tmQ, tmB, tmdO, tmV;
+  if (!make_tensor_map_bf16(&tmQ, p.Q, D, p.N, BH, 64, CONV ? Cfg::QR : Cfg::BM, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmB, CONV ? Kt : p.K, D, p.N, CONV ? BH * p.cq * 2 : BH, 64, Cfg::KB, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmdO, BWD ? p.dO : p.Q, D, p.N, BH, 64, Cfg::BM, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmV, p.V, D, p.N, BH, 64, Cfg::KB, true)) return cudaErrorInvalidValue;
+  auto kern = mix_score_kernel<G, D, CONV, BWD>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+  if (e != cudaSuccess) return e;
+  return launch_pdl(kern, dim3(mp.nRT * mp.nKC, mp.nU), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmQ, tmB, tmdO, tmV, mp);
+}
+
+template <int G, int D>
+cudaError_t launch_score_g(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, bool bwd, cudaStream_t stream) {
+  if (p.theta) return bwd ? launch_score_t<G, D, true, true>(p, mp, Kt, stream) : launch_score_t<G, D, true, false>(p, mp, Kt, stream);
+  return bwd ? launch_score_t<G, D, false, true>(p, mp, Kt, stream) : launch_score_t<G, D, false, false>(p, mp, Kt, stream);
+}
+
+}  // namespace
+
+cudaError_t launch_mix_score(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, bool bwd, cudaStream_t stream) {
+#define FMTA_MIX_G(GG) \
+  if (p.G == GG) return p.d == 64 ? launch_score_g<GG, 64>(p, mp, Kt, bwd, stream) : launch_score_g<GG, 128>(p, mp, Kt, bwd, stream);
+  FMTA_MIX_G(2) FMTA_MIX_G(4) FMTA_MIX_G(8) FMTA_MIX_G(16)
+#undef FMTA_MIX_G
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace fmta

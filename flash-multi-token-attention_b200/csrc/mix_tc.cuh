@@ -1,0 +1,75 @@
+// Head mixing on the tensor cores: parameter block and host-side declarations shared by the score kernel (mix_score.cu), the
+// products that follow it (mix_gemm.cu) and their driver (mix_tc.cu).
+//
+//   C_g[i,j]  = sum_a q_{i-(pad_q-a)} . Kt_a[j]  (with a key-query filter)   or   q_i . k_j  (without)
+//   C'_g      = sum_g' W[g,g'] C_g',  P = softmax(C'),  O = P V
+//   dP = dO V^T,  dC' = P (dP - D),  dC_g' = sum_g W[g,g'] dC'_g,  dW[g,g'] = sum dC'_g C_g'
+//
+// The mix needs all G heads of a group at one place, their output accumulators (G x d columns) do not fit beside the scores,
+// and nothing after the mix couples heads.  So the score kernel makes C (tcgen05, G tiles side by side in tensor memory),
+// mixes it in registers (one query row per thread, fp32) and leaves what the per-head products need in global memory as bf16
+// operands: P (forward: relative to a reference per row; backward: P and dC).  The products are plain GEMM pipelines.
+//
+// Operand tensors P / dC: "X8" = [head][key chunk of 8][row][8 keys], rows padded to X8 rows = roundup(N, 128) + 16.  A thread
+// of the score kernel owns a row, so its 16-byte stores of 8 keys are contiguous across a warp; and every consumer gets an
+// MMA operand with plain bulk copies of rows x 16 bytes: no-swizzle core matrices, K-major for O = P V and dQ (a row shift is
+// 16 bytes), MN-major for dV = P^T dO and dKt = dC^T Q.
+#pragma once
+#include <cuda.h>
+
+#include "bwd_tc.cuh"
+#include "fmta_common.cuh"
+#include "fmta_params.h"
+#include "fmta_tc.cuh"
+#include "launch_util.cuh"
+
+namespace fmta {
+
+struct MixParams {
+  const float* W;         // [H/G, G, G] fp32, row = output head
+  const float* LSE;       // backward
+  const float* Dvec;      // backward
+  const float* Cband;     // causal with a filter: [B*H, N, band] scores of the band after the filter, natural units (else nullptr)
+  float* dCband;          // backward: the gradient of those
+  bf16* P8;               // [heads of the launch][N8 / 8][RP][8]
+  bf16* C8;               // backward: dC
+  float* ref;             // forward: [heads of the launch][N8 / 16][RP] log2 reference of 16 keys of P
+  float* stat;            // forward: [heads of the launch][2 nKC][3][RP]: row max, reference, sum, per key chunk and half
+  float* dW_part;         // backward: [slots][H/G][G*G], slot = (b * nRT + row tile) * nKC + key chunk
+  int* status;
+  int B, H, N, G, cq, ck, causal;
+  int u0, nU;             // (batch, group) units of this launch: u0 .. u0 + nU - 1
+  int nRT, nKC, kch;      // row tiles of 128, key chunks of kch keys
+  int RP, N8;
+  float c2;               // factor on W for logits in log2 units (scale * log2e without a filter, 1 with one)
+  float cw;               // factor on dW (scale without a filter, ln2 with one)
+};
+
+// 128 rows x n columns of fp32 from tensor memory, no wait.
+template <int NC>
+FMTA_DEVINL void tmem_ld_nowait(uint32_t taddr, float* v) {
+  if constexpr (NC == 4) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(taddr) : "memory");
+  } else if constexpr (NC == 8) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "r"(taddr) : "memory");
+  } else {
+    static_assert(NC == 16, "");
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]),
+                   "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]) : "r"(taddr) : "memory");
+  }
+}
+
+// two fp32 FMAs on a register pair: same rate as two FMAs, half the issue slots
+FMTA_DEVINL uint64_t f2_pack(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+FMTA_DEVINL void f2_unpack(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+FMTA_DEVINL uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+FMTA_DEVINL uint64_t f2_mul(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+
+cudaError_t launch_mix_score(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, bool bwd, cudaStream_t stream);
+cudaError_t launch_mix_pv(const TrainParams& p, const MixParams& mp, cudaStream_t stream);
+cudaError_t launch_mix_dq(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, cudaStream_t stream);
+cudaError_t launch_mix_dkdv(const TrainParams& p, const MixParams& mp, __nv_bfloat16* dKt, cudaStream_t stream);
+
+}  // namespace fmta

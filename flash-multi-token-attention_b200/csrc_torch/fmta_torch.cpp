@@ -262,6 +262,207 @@ Tensor conv_attention(const Tensor& Q, const Tensor& K, const Tensor& V, const T
   return pad ? cut32(O) : O;
 }
 
+// ---------------------------------------------------------------- head mixing
+[[noreturn]] void not_implemented(const std::string& what) {
+  PyErr_SetString(PyExc_NotImplementedError, what.c_str());
+  throw pybind11::error_already_set();
+}
+
+struct Mix {
+  Dims s;
+  int G;
+  Tensor w, theta;        // fp32 [H/G, G, G]; fp32 [H, cq, ck] or undefined
+  bool tc(bool bwd, size_t* bytes) const {                 // the tensor-core kernels take this problem
+    if (exact_only() || (s.d != 64 && s.d != 128) || G > 16 || (theta.defined() && s.cq > 7)) return false;
+    const size_t n8 = ((size_t)s.N + 127) / 128 * 128;     // P and dC of one (batch, group) unit: see fmta_mix_bwd
+    if ((size_t)G * (n8 / 8) * (n8 + 16) * 32 > ((size_t)16 << 30)) return false;
+    *bytes = fmta_workspace_bytes(bwd ? FMTA_OP_MIX_BWD : FMTA_OP_MIX_FWD, s.B, s.H, s.N, s.d, s.cq, s.ck, G);
+    return true;
+  }
+  size_t exchange(int64_t limit) const {
+    if (!theta.defined()) return 0;
+    const size_t n = fmta_workspace_bytes(FMTA_OP_MIX_EXCHANGE, s.B, s.H, s.N, s.d, s.cq, s.ck, G);
+    return n <= (size_t)limit ? n : 0;
+  }
+};
+
+Mix mix_of(const Tensor& q, const Tensor& w, const Tensor& theta_) {
+  FMTA_REQUIRE(q.dim() == 4, "q must have shape [batch, heads, seq, d_head]");
+  Mix m{{(int)q.size(0), (int)q.size(1), (int)q.size(2), (int)q.size(3), 1, 1}, 0, {}, {}};
+  const int H = m.s.H;
+  if (w.dim() == 2) {
+    FMTA_REQUIRE(w.size(0) == H && w.size(1) == H, "w must be [heads, heads] or [heads/G, G, G]");
+    m.G = H;
+    m.w = f32(w).view({1, H, H});
+  } else {
+    FMTA_REQUIRE(w.dim() == 3, "w must be [heads, heads] or [heads/G, G, G]");
+    m.G = (int)w.size(1);
+    FMTA_REQUIRE(w.size(2) == m.G && w.size(0) * m.G == H, "grouped w must be [heads/G, G, G]");
+    m.w = f32(w);
+  }
+  if (m.G == 32 && (theta_.defined() || m.s.d > 64)) not_implemented("32 mixed heads are supported without a key-query conv and up to head dim 64");
+  if (m.G != 2 && m.G != 4 && m.G != 8 && m.G != 16 && m.G != 32)
+    not_implemented(c10::str("head mixing supports group sizes 2, 4, 8, 16, 32 (got ", m.G, ")"));
+  if (theta_.defined()) {
+    m.theta = f32(theta_);
+    m.s.cq = (int)m.theta.size(1); m.s.ck = (int)m.theta.size(2);
+  }
+  return m;
+}
+
+// O (preallocated, fp32 or bf16), L, M, LSE
+void mix_forward_raw(const Mix& m, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& O, const Tensor& M, const Tensor& L,
+                     const Tensor& LSE, double scale, bool causal, int64_t xlimit) {
+  const Dims& s = m.s;
+  arm_status(q);
+  size_t n = 0;
+  const bool tc = m.tc(false, &n);
+  if (!tc) n = m.exchange(xlimit);
+  const Tensor ws = n ? new_bytes(q, n) : Tensor();
+  check_status(fmta_fwd(ptr(q), ptr(k), ptr(v), fptr(m.theta), fptr(m.w), ptr(O), fptr(M), fptr(L), fptr(LSE), s.B, s.H, s.N, s.d, s.cq, s.ck, m.G,
+                        (float)scale, causal, dtype_code(O.scalar_type()), tc ? -1 : 0, ptr(ws), n, stream_of(q)),
+               "fmta_fwd(head mix)");
+}
+
+// {dQ, dK, dV, dW [H/G,G,G], dTheta}: gradients in grad_dtype on the tensor-core kernels, else fp32; want: 1 dQ (dW, dTheta), 2 dK and dV
+std::vector<Tensor> mix_backward_raw(const Mix& m, const Tensor& q, const Tensor& k, const Tensor& v, Tensor dO, const Tensor& O, const Tensor& LSE,
+                                     double scale, bool causal, int want, bool g16, int64_t xlimit) {
+  const Dims& s = m.s;
+  arm_status(q);
+  const bool conv = m.theta.defined();
+  const Tensor dW = want & 1 ? new_f32(q, {s.H / m.G, m.G, m.G}) : Tensor(), dT = conv ? new_f32(q, {s.H, s.cq, s.ck}) : Tensor();
+  size_t n = 0;
+  if (m.tc(true, &n)) {
+    dO = dO.scalar_type() == at::kFloat && dO.is_contiguous() && reinterpret_cast<uintptr_t>(dO.data_ptr()) % 16 == 0 ? dO : bf16c(dO);
+    Tensor g[3];
+    for (int i = 0; i < 3; ++i)
+      if (conv || (i == 0 ? want & 1 : want & 2)) g[i] = at::empty(q.sizes(), q.options().dtype(g16 ? at::kBFloat16 : at::kFloat));
+    const Tensor dWt = dW.defined() ? dW : (conv ? new_f32(q, {s.H / m.G, m.G, m.G}) : Tensor());
+    const Tensor ws = new_bytes(q, n);
+    check_status(fmta_mix_bwd(ptr(q), ptr(k), ptr(v), ptr(dO), dtype_code(dO.scalar_type()), ptr(O), dtype_code(O.scalar_type()), fptr(LSE), fptr(m.theta),
+                              fptr(m.w), ptr(g[0]), ptr(g[1]), ptr(g[2]), g16 ? FMTA_DTYPE_BF16 : FMTA_DTYPE_F32, fptr(dT), fptr(dWt), s.B, s.H, s.N, s.d,
+                              s.cq, s.ck, m.G, (float)scale, causal, ptr(ws), n, stream_of(q)),
+                 "fmta_mix_bwd");
+    return {g[0], g[1], g[2], dW, dT};
+  }
+  dO = bf16c(dO);
+  const Tensor D = rowdot(dO, O);
+  n = fmta_workspace_bytes(FMTA_OP_BWD_DQ, s.B, s.H, s.N, s.d, s.cq, s.ck, m.G);
+  if (const size_t x = m.exchange(xlimit)) n = (n + 255) / 256 * 256 + x;
+  const Tensor ws = new_bytes(q, n);
+  const Tensor dQ = want & 1 ? new_f32(q, q.sizes()) : Tensor(), dK = want & 2 ? new_f32(q, q.sizes()) : Tensor(), dV = want & 2 ? new_f32(q, q.sizes()) : Tensor();
+  if (want == 3)
+    check_status(fmta_bwd(ptr(q), ptr(k), ptr(v), ptr(dO), fptr(D), fptr(LSE), fptr(m.theta), fptr(m.w), fptr(dQ), fptr(dK), fptr(dV), fptr(dT), fptr(dW),
+                          s.B, s.H, s.N, s.d, s.cq, s.ck, m.G, (float)scale, causal, 0, ptr(ws), n, stream_of(q)),
+                 "fmta_bwd(head mix)");
+  else if (want == 1)
+    check_status(fmta_bwd_dq_dw(ptr(q), ptr(k), ptr(v), ptr(dO), fptr(D), fptr(LSE), fptr(m.theta), fptr(m.w), fptr(dQ), fptr(dT), fptr(dW), s.B, s.H, s.N,
+                                s.d, s.cq, s.ck, m.G, (float)scale, causal, ptr(ws), n, stream_of(q)),
+                 "fmta_bwd_dq_dw(head mix)");
+  else
+    check_status(fmta_bwd_dkdv(ptr(q), ptr(k), ptr(v), ptr(dO), fptr(D), fptr(LSE), fptr(m.theta), fptr(m.w), fptr(dK), fptr(dV), s.B, s.H, s.N, s.d, s.cq,
+                               s.ck, m.G, (float)scale, causal, stream_of(q)),
+                 "fmta_bwd_dkdv(head mix)");
+  return {dQ, dK, dV, dW, dT};
+}
+
+at::ScalarType mix_out_dtype(const Tensor& q, const std::optional<at::ScalarType>& out) {
+  if (out) return *out;
+  return q.scalar_type() == at::kFloat || q.scalar_type() == at::kBFloat16 ? q.scalar_type() : at::kFloat;
+}
+
+void mix_check(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& theta) {
+  FMTA_REQUIRE(q.is_cuda(), "q must be a CUDA tensor");
+  require_on(q, k, "k", q.sizes()); require_on(q, v, "v", q.sizes()); require_on(q, w, "w");
+  if (theta.defined()) require_on(q, theta, "conv_kernel");
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor> mix_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& w, const std::optional<Tensor>& theta_,
+                                                      double scale, bool causal, const std::optional<at::ScalarType>& out, int64_t xlimit) {
+  const Tensor theta = theta_ ? *theta_ : Tensor();
+  mix_check(q, k, v, w, theta);
+  at::AutoGradMode no_grad(false);
+  c10::cuda::CUDAGuard guard(q.device());
+  const Mix m = mix_of(q, w, theta);
+  const Tensor O = at::empty(q.sizes(), q.options().dtype(mix_out_dtype(q, out)));
+  const Tensor M = new_f32(q, {m.s.B, m.s.H, m.s.N}), L = at::empty_like(M), LSE = at::empty_like(M);
+  mix_forward_raw(m, bf16c(q), bf16c(k), bf16c(v), O, M, L, LSE, scale, causal, xlimit);
+  return {out ? O : O.to(q.scalar_type()), L, M, LSE};
+}
+
+std::vector<Tensor> mix_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& o, const Tensor& dO, const Tensor& l,
+                                 const Tensor& mx, const std::optional<Tensor>& theta_, bool causal, const std::optional<double>& scale,
+                                 const std::optional<Tensor>& lse_, int64_t want, int64_t xlimit) {
+  const Tensor theta = theta_ ? *theta_ : Tensor();
+  mix_check(q, k, v, w, theta);
+  require_on(q, dO, "do", q.sizes()); require_on(q, o, "o", q.sizes());
+  at::AutoGradMode no_grad(false);
+  c10::cuda::CUDAGuard guard(q.device());
+  const Mix m = mix_of(q, w, theta);
+  require_on(q, l, "l", {m.s.B, m.s.H, m.s.N}); require_on(q, mx, "m", {m.s.B, m.s.H, m.s.N});
+  const Tensor lse = lse_ ? f32(*lse_) : at::add(f32(mx), at::log(f32(l)));
+  const Tensor oc = o.scalar_type() == at::kBFloat16 ? o.contiguous() : f32(o);
+  auto g = mix_backward_raw(m, bf16c(q), bf16c(k), bf16c(v), bf16c(dO), oc, lse, scale ? *scale : 1.0 / std::sqrt((double)m.s.d), causal, (int)want, false, xlimit);
+  if (g[3].defined()) g[3] = g[3].reshape(w.sizes());
+  return g;
+}
+
+struct MixFn : public torch::autograd::Function<MixFn> {
+  // no theta: mix only.  out32: fp32 output whatever q's dtype (the filter + mix operator)
+  static Tensor forward(AutogradContext* ctx, const Tensor& Q, const Tensor& K, const Tensor& V, const std::optional<Tensor>& theta_o, const Tensor& w,
+                        double scale, bool causal, bool out32, int64_t xlimit) {
+    const Tensor theta_ = theta_o ? *theta_o : Tensor();
+    const Mix m = mix_of(Q, w, theta_);
+    const Tensor q = bf16c(Q), k = bf16c(K), v = bf16c(V);
+    const Tensor O = at::empty(q.sizes(), q.options().dtype(out32 ? at::kFloat : mix_out_dtype(Q, std::nullopt)));
+    const Tensor LSE = new_f32(q, {m.s.B, m.s.H, m.s.N});
+    mix_forward_raw(m, q, k, v, O, Tensor(), Tensor(), LSE, scale, causal, xlimit);
+    const Tensor out = out32 ? O : O.to(Q.scalar_type());
+    ctx->save_for_backward({q, k, v, theta_, w, out, LSE});
+    ctx->saved_data["scale"] = scale; ctx->saved_data["causal"] = causal; ctx->saved_data["xlimit"] = xlimit;
+    ctx->saved_data["tq"] = (int64_t)Q.scalar_type(); ctx->saved_data["tk"] = (int64_t)K.scalar_type(); ctx->saved_data["tv"] = (int64_t)V.scalar_type();
+    ctx->saved_data["has_theta"] = theta_.defined();
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    at::AutoGradMode no_grad(false);
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &theta = saved[3], &w = saved[4], &out = saved[5], &LSE = saved[6];
+    const at::ScalarType ty[3] = {(at::ScalarType)ctx->saved_data["tq"].toInt(), (at::ScalarType)ctx->saved_data["tk"].toInt(),
+                                  (at::ScalarType)ctx->saved_data["tv"].toInt()};
+    c10::cuda::CUDAGuard guard(q.device());
+    const Tensor dO = grads[0].defined() ? grads[0] : at::zeros_like(out);
+    const Tensor O = out.scalar_type() == at::kBFloat16 ? out.contiguous() : f32(out);
+    const bool g16 = ty[0] == at::kBFloat16 && ty[1] == at::kBFloat16 && ty[2] == at::kBFloat16;
+    // without a filter each half of the gradients is a set of kernels of its own
+    const bool has_theta = ctx->saved_data["has_theta"].toBool();
+    const int base = 0, iw = has_theta ? 4 : 3;
+    int want = 3;
+    if (!has_theta) want = (ctx->needs_input_grad(base) || ctx->needs_input_grad(iw) ? 1 : 0) | (ctx->needs_input_grad(1) || ctx->needs_input_grad(2) ? 2 : 0);
+    if (want == 0) return variable_list(9);
+    auto g = mix_backward_raw(mix_of(q, w, theta), q, k, v, dO, O, LSE, ctx->saved_data["scale"].toDouble(), ctx->saved_data["causal"].toBool(), want, g16,
+                              ctx->saved_data["xlimit"].toInt());
+    for (int i = 0; i < 3; ++i) if (g[i].defined()) g[i] = g[i].to(ty[i]);
+    const Tensor dT = has_theta ? g[4].to(theta.scalar_type()) : Tensor();
+    const Tensor dW = g[3].defined() ? g[3].reshape(w.sizes()).to(w.scalar_type()) : Tensor();
+    return {g[0], g[1], g[2], dT, dW, Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor mix_attention(const Tensor& q, const Tensor& k, const Tensor& v, const std::optional<Tensor>& theta_, const Tensor& w, double scale, bool causal,
+                     bool out32, int64_t xlimit) {
+  const Tensor theta = theta_ ? *theta_ : Tensor();
+  mix_check(q, k, v, w, theta);
+  c10::cuda::CUDAGuard guard(q.device());
+  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad() || w.requires_grad() || (theta.defined() && theta.requires_grad())))
+    return MixFn::apply(q, k, v, theta_, w, scale, causal, out32, xlimit);
+  at::AutoGradMode no_grad(false);
+  const Mix m = mix_of(q, w, theta);
+  const Tensor O = at::empty(q.sizes(), q.options().dtype(out32 ? at::kFloat : mix_out_dtype(q, std::nullopt)));
+  mix_forward_raw(m, bf16c(q), bf16c(k), bf16c(v), O, Tensor(), Tensor(), Tensor(), scale, causal, xlimit);
+  return out32 ? O : O.to(q.scalar_type());
+}
+
 // ---------------------------------------------------------------- decode
 struct Splits { Tensor O, M, L; };
 Splits split_outputs(const Tensor& Q, int64_t B, int64_t H, int64_t ks, int64_t d) {   // carved out of one allocation
@@ -333,6 +534,9 @@ PYBIND11_MODULE(_native, m) {
   m.def("conv_backward", &conv_backward);
   m.def("conv_attention", &conv_attention);
   m.def("rowdot", &rowdot);
+  m.def("mix_forward", &mix_forward);
+  m.def("mix_backward", &mix_backward);
+  m.def("mix_attention", &mix_attention);
   m.def("decode", &decode);
   m.def("decode_paged", &decode_paged);
   m.def("kv_append_paged", &kv_append_paged);

@@ -61,6 +61,11 @@ extern "C" {
  * FMTA_OP_BWD_DQ bytes rounded up to 256.  A smaller workspace is not an error. */
 #define FMTA_OP_MIX_EXCHANGE 5
 #define FMTA_OP_BWD_FUSED 6      /* fmta_bwd_fused */
+/* Head mixing on the tensor cores (d = 64 or 128, groups of 2, 4, 8 or 16 heads, c_q <= 7): fmta_fwd with path -1 or 1 and a
+ * workspace of FMTA_OP_MIX_FWD; fmta_mix_bwd with FMTA_OP_MIX_BWD.  P (and dC) of a few (batch, group) units at a time:
+ * at most 4.5 GiB, or one unit's. */
+#define FMTA_OP_MIX_FWD 7
+#define FMTA_OP_MIX_BWD 8
 
 /* Library version (major*10000 + minor*100 + patch). */
 int fmta_version(void);
@@ -209,6 +214,18 @@ int fmta_bwd_fused(const void* Q, const void* K, const void* V, const void* dO, 
                    const float* LSE, const float* theta, void* dQ, void* dK, void* dV, int grad_dtype, float* dTheta,
                    int B, int H, int N, int d, int cq, int ck, float scale, int causal, void* workspace,
                    size_t workspace_bytes, const void* ktilde, void* stream);
+
+/*
+ * Backward of head-mixing attention in one call, with or without a key-query filter (theta may be NULL): what
+ * fmta_bwd_prep_D and fmta_bwd with wmix compute, on the tensor-core kernels.  Replaces the host functions
+ * `head_conv_attention_bwd_dq_dw` / `_bwd_dkdv` (head_conv_attn/bwd_dq_dw.py:373, bwd_dk_dv.py:407).
+ *   dO, O: do_dtype / o_dtype     dQ, dK, dV: grad_dtype     dTheta fp32 (NULL without theta)   dW fp32 [H/G,G,G]
+ * Without theta either dQ (and dW) or dK and dV may be NULL.  Shapes and workspace: FMTA_OP_MIX_BWD.
+ */
+int fmta_mix_bwd(const void* Q, const void* K, const void* V, const void* dO, int do_dtype, const void* O, int o_dtype,
+                 const float* LSE, const float* theta, const float* wmix, void* dQ, void* dK, void* dV, int grad_dtype,
+                 float* dTheta, float* dW, int B, int H, int N, int d, int cq, int ck, int G, float scale, int causal,
+                 void* workspace, size_t workspace_bytes, void* stream);
 
 /*
  * One window of sequence positions of a forward / backward (no counterpart in the reference, which has no
