@@ -28,7 +28,7 @@ struct PvCfg {
 
 template <int D>
 __global__ void __launch_bounds__(192, 2)
-mix_pv_kernel(const __grid_constant__ CUtensorMap tmV, const MixParams p, void* O, int o_bf16, float* Mo, float* Lo, float* LSEo) {
+mix_pv_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmV, const MixParams p, void* O, int o_bf16, float* Mo, float* Lo, float* LSEo) {
   using Cfg = PvCfg<D>;
   constexpr int BM = Cfg::BM, BC = Cfg::BC, NSTG = Cfg::NSTG, SL = Cfg::SL;
   extern __shared__ unsigned char smem_raw[];
@@ -70,13 +70,12 @@ mix_pv_kernel(const __grid_constant__ CUtensorMap tmV, const MixParams p, void* 
 
   if (warp == 4) {
     if (lane == 0) {
-      const bf16* src = p.P8 + ((size_t)lh * (p.N8 / 8) * p.RP + R0) * 8;
       for (int kb = 0; kb < nblk; ++kb) {
         const int st = kb % NSTG, ph = (kb / NSTG) & 1;
         if (!tc::mbar_wait(&empty[st], ph ^ 1, s_abort)) break;
         unsigned char* sg = smem + st * Cfg::STAGE;
         tc::mbar_expect_tx(&full[st], Cfg::STAGE);
-        for (int c = 0; c < BC / 8; ++c) tc::bulk_load(sg + c * (BM * 16), src + (size_t)(kb * (BC / 8) + c) * p.RP * 8, BM * 16, &full[st]);
+        tc::tma_load_3d(sg, &tmP, &full[st], 0, R0 / 8, lh * (p.N8 / 8) + kb * (BC / 8));
         for (int sl = 0; sl < SL; ++sl) tc::tma_load_3d(sg + Cfg::P_BYTES + sl * Cfg::V_SLAB, &tmV, &full[st], sl * 64, kb * BC, bh);
         *s_issued = kb + 1;
       }
@@ -168,13 +167,15 @@ mix_pv_kernel(const __grid_constant__ CUtensorMap tmV, const MixParams p, void* 
 }
 
 // ==========================================================================================
-template <int D>
+template <int D, int NT_, bool CONV>
 struct MixDqCfg {
-  static constexpr int BM = 128, AR = BM + 8, BC = 64, SL = D / 64, NT = 2;
+  static constexpr int BM = 128, AR = BM + 8, BC = 64, SL = D / 64, NT = NT_;
   static constexpr int A_BYTES = AR * 128;                    // one dC tile: 136 rows x 64 keys
   static constexpr int SLAB = BC * 128, B_BYTES = SL * SLAB;  // one key tile: 64 x D
-  static constexpr int NA = 2;                                // dC stages (both tiles), held for all key tiles of their block
-  static constexpr int NB = D == 64 ? 16 : 9;                 // key tiles in flight
+  // dC stages (all tiles), held for the key tiles of their block, and key tiles in flight: with a filter a block has 2 c_q key
+  // tiles, without one a single one
+  static constexpr int NA = CONV ? 2 : (NT == 2 ? 3 : 6);
+  static constexpr int NB_ = (225 * 1024 - NA * NT * A_BYTES) / B_BYTES, NB = NB_ > 16 ? 16 : NB_;
   static constexpr int oB = NA * NT * A_BYTES;
   static constexpr int oBar = oB + NB * B_BYTES;
   static constexpr int kSmemBytes = oBar + 512 + 1024;
@@ -189,10 +190,11 @@ struct MixGradOut {
   float mul;
 };
 
-template <int D>
-__global__ void __launch_bounds__(MixDqCfg<D>::kThreads, 1)
-mix_dq_kernel(const __grid_constant__ CUtensorMap tmB, const MixParams p, int ntap, int nhl, MixGradOut out) {
-  using Cfg = MixDqCfg<D>;
+template <int D, int NT_, bool CONV>
+__global__ void __launch_bounds__(MixDqCfg<D, NT_, CONV>::kThreads, 1)
+mix_dq_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmB, const MixParams p, int ntap, MixGradOut out) {
+  constexpr int nhl = CONV ? 2 : 1;      // key tiles per tap: a (hi, lo) pair with a filter
+  using Cfg = MixDqCfg<D, NT_, CONV>;
   constexpr int BM = Cfg::BM, AR = Cfg::AR, BC = Cfg::BC, SL = Cfg::SL, NT = Cfg::NT, NA = Cfg::NA, NB = Cfg::NB;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -208,17 +210,17 @@ mix_dq_kernel(const __grid_constant__ CUtensorMap tmB, const MixParams p, int nt
   volatile int* s_issued = s_abort + 1;  // key tiles and dC stages the producer has issued
   volatile int* s_aissued = s_abort + 2;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int lh = blockIdx.y, nQ = (p.nRT + 1) / 2, q = nQ - 1 - blockIdx.x;
+  const int lh = blockIdx.y, nQ = (p.nRT + NT - 1) / NT, q = nQ - 1 - blockIdx.x;
   const int u = p.u0 + lh / p.G, HG = p.H / p.G, b = u / HG, bh = b * p.H + (u - b * HG) * p.G + lh % p.G;
   const int N = p.N, pq = ntap - 1;
   int nkb_t[NT];
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
-    const int rt = 2 * q + t;
+    const int rt = NT * q + t;
     nkb_t[t] = rt >= p.nRT ? 0 : (p.causal ? min(rt * BM + BM, p.N8) : p.N8) / BC;
   }
-  const int nB = ntap * nhl;             // key tiles per block: taps, as (hi, lo) pairs with a filter
-  const int nkb = max(nkb_t[0], nkb_t[1]);
+  const int nB = ntap * nhl;             // key tiles per block
+  const int nkb = max(nkb_t[0], nkb_t[NT - 1]);
 
   if (tid == 0) {
     for (int i = 0; i < NA; ++i) { tc::mbar_init(&a_full[i], 1); tc::mbar_init(&a_empty[i], NT); }
@@ -241,7 +243,6 @@ mix_dq_kernel(const __grid_constant__ CUtensorMap tmB, const MixParams p, int nt
 
   if (warp == NT * 4) {
     if (lane == 0) {
-      const bf16* src = p.C8 + (size_t)lh * (p.N8 / 8) * p.RP * 8;
       int id = 0;
       bool ok = true;
       for (int kb = 0; kb < nkb && ok; ++kb) {
@@ -251,9 +252,9 @@ mix_dq_kernel(const __grid_constant__ CUtensorMap tmB, const MixParams p, int nt
         tc::mbar_expect_tx(&a_full[st], NT * Cfg::A_BYTES);
         for (int t = 0; t < NT; ++t) {
           // a tile past its last block (or past the last row tile) gets an earlier valid block's data
-          const int rt = min(2 * q + t, p.nRT - 1), kk = min(kb, max(nkb_t[t], 1) - 1);
-          for (int c = 0; c < BC / 8; ++c)
-            tc::bulk_load(smem + (st * NT + t) * Cfg::A_BYTES + c * (AR * 16), src + ((size_t)(kk * (BC / 8) + c) * p.RP + rt * BM) * 8, AR * 16, &a_full[st]);
+          const int rt = min(NT * q + t, p.nRT - 1), kk = min(kb, max(nkb_t[t], 1) - 1);
+          if (CONV) tc::tma_load_3d(smem + (st * NT + t) * Cfg::A_BYTES, &tmC, &a_full[st], kk * BC, rt * BM, lh);
+          else tc::tma_load_3d(smem + (st * NT + t) * Cfg::A_BYTES, &tmC, &a_full[st], 0, rt * (BM / 8), lh * (p.N8 / 8) + kk * (BC / 8));
         }
         *s_aissued = kb + 1;
         for (int a = 0; a < nB; ++a, ++id) {
@@ -269,36 +270,40 @@ mix_dq_kernel(const __grid_constant__ CUtensorMap tmB, const MixParams p, int nt
   } else if (warp > NT * 4) {
     const int t = warp - (NT * 4 + 1);
     constexpr uint32_t idesc = tc::make_idesc(BM, D, 0, 1);
-    const uint64_t dA = tc::make_sdesc(smem_u32(smem), AR * 16, 128, tc::kLayoutNone);
+    const uint64_t dA = CONV ? tc::make_sdesc(smem_u32(smem), 16, 1024, tc::kLayoutSW128) : tc::make_sdesc(smem_u32(smem), AR * 16, 128, tc::kLayoutNone);
+    constexpr uint32_t row_step = CONV ? 8 : 1, k_step = CONV ? 2 : 2 * AR;     // 16-byte units per row and per 16 keys
     const uint64_t dB = tc::make_sdesc(smem_u32(smem) + Cfg::oB, SL > 1 ? Cfg::SLAB : 16, 1024, tc::kLayoutSW128);
     const uint32_t a_hi = (uint32_t)(dA >> 32), a0 = (uint32_t)dA, b_hi = (uint32_t)(dB >> 32), b0 = (uint32_t)dB;
     const uint32_t dst = tmem + t * D;
     bool ok = true;
-    int id = 0;
+    int s = 0, ph = 0;                                        // key-tile ring position
     for (int kb = 0; kb < nkb && ok; ++kb) {
       const bool active = kb < nkb_t[t];
       const int st = kb % NA;
       ok = tc::mbar_wait_warp(&a_full[st], (kb / NA) & 1, s_abort);
       if (!ok) break;
-      for (int a = 0; a < nB; ++a, ++id) {
-        const int s = id % NB;
-        ok = tc::mbar_wait_warp(&full[s], (id / NB) & 1, s_abort);
-        if (!ok) break;
-        if (active) {
-          tc::tc_fence_after();
-          const uint32_t al = a0 + (uint32_t)((st * NT + t) * (Cfg::A_BYTES >> 4) + (pq - a / nhl));                 // dC rows i' + pad_q - a
-          const uint32_t bl = b0 + (uint32_t)(s * (Cfg::B_BYTES >> 4));
-          tc::mma_ss2pe(dst, al, a_hi, bl, b_hi, idesc, (kb != 0) || (a != 0));
+      uint32_t al = a0 + (uint32_t)((st * NT + t) * (Cfg::A_BYTES >> 4) + pq * row_step);        // dC rows i' + pad_q - a
+      for (int a = 0; a < ntap && ok; ++a, al -= row_step) {
 #pragma unroll
-          for (int k = 1; k < BC / 16; ++k) tc::mma_ss2e<1>(dst, al + (uint32_t)(2 * k * AR), a_hi, bl + (uint32_t)(k * (2048 / 16)), b_hi, idesc);
+        for (int hl = 0; hl < nhl; ++hl) {
+          ok = tc::mbar_wait_warp(&full[s], ph, s_abort);
+          if (!ok) break;
+          if (active) {
+            tc::tc_fence_after();
+            const uint32_t bl = b0 + (uint32_t)(s * (Cfg::B_BYTES >> 4));
+            tc::mma_ss2pe(dst, al, a_hi, bl, b_hi, idesc, (kb | a | hl) != 0);
+#pragma unroll
+            for (int k = 1; k < BC / 16; ++k) tc::mma_ss2e<1>(dst, al + k * k_step, a_hi, bl + (uint32_t)(k * (2048 / 16)), b_hi, idesc);
+          }
+          tc::mma_commit_e(&empty[s]);
+          if (++s == NB) { s = 0; ph ^= 1; }
         }
-        tc::mma_commit_e(&empty[s]);
       }
       if (ok) tc::mma_commit_e(&a_empty[st]);
     }
     if (ok) tc::mma_commit_e(&done[t]);
   } else {
-    const int t = warp >> 2, r = tid & (BM - 1), gi = (2 * q + t) * BM + r;
+    const int t = warp >> 2, r = tid & (BM - 1), gi = (NT * q + t) * BM + r;
     const uint32_t tQ = tmem + ((uint32_t)((warp & 3) * 32) << 16) + t * D;
     const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(&done[t], 0, s_abort));
     tc::tc_fence_after();
@@ -345,9 +350,10 @@ struct MixDkvCfg {
   static_assert(STAGE % 1024 == 0 && 7 * KT_BYTES <= NSTG * STAGE && kSmemBytes <= 227 * 1024, "shared memory");
 };
 
+template <bool CONV>
 __global__ void __launch_bounds__(MixDkvCfg::kThreads, 1)
 mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO, const __grid_constant__ CUtensorMap tmdKt,
-                const MixParams p, int cq, int d, MixGradOut dV, MixGradOut dK) {
+                const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmC, const MixParams p, int cq, int d, MixGradOut dV, MixGradOut dK, int early) {
   using Cfg = MixDkvCfg;
   constexpr int BK = Cfg::BK, BR = Cfg::BR, HALO = Cfg::HALO, NSTG = Cfg::NSTG;
   constexpr int W_TMA = Cfg::kEpWarps, W_A0 = Cfg::kEpWarps + 1;
@@ -379,14 +385,15 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   }
   tc::tc_fence_before();
   __syncthreads();
-  pdl_wait();
+  // behind the dQ kernel (early) no wait here: it let this kernel start only after its own wait, when P and dC were complete;
+  // the wait below keeps "this kernel has completed" meaning "every earlier one has"
+  if (!early) pdl_wait();
   pdl_trigger();
   tc::tc_fence_after();
   const uint32_t tmem = *s_tmem;
 
   if (warp == W_TMA) {
     if (lane == 0) {
-      const size_t base = ((size_t)lh * (p.N8 / 8) + j0 / 8) * p.RP * 8;
       for (int it = 0; it < nblk; ++it) {
         const int st = it % NSTG, ph = (it / NSTG) & 1, i0 = (qb_begin + it) * BR;
         if (!tc::mbar_wait(&empty[st], ph ^ 1, s_abort)) break;
@@ -394,8 +401,13 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tc::mbar_expect_tx(&full[st], Cfg::STAGE);
         tc::tma_load_3d(sg + Cfg::sgdO, &tmdO, &full[st], col0, i0, bh);
         tc::tma_load_3d(sg + Cfg::sgQ, &tmQ, &full[st], col0, i0 - HALO, bh);
-        for (int c = 0; c < BK / 8; ++c) tc::bulk_load(sg + Cfg::sgP + c * (BR * 16), p.P8 + base + ((size_t)c * p.RP + i0) * 8, BR * 16, &full[st]);
-        for (int c = 0; c < BK / 8; ++c) tc::bulk_load(sg + Cfg::sgC + c * (BR * 16), p.C8 + base + ((size_t)c * p.RP + i0) * 8, BR * 16, &full[st]);
+        tc::tma_load_3d(sg + Cfg::sgP, &tmP, &full[st], 0, i0 / 8, (lh * p.N8 + j0) / 8);
+        if (CONV) {                                            // two slabs of 64 keys
+          tc::tma_load_3d(sg + Cfg::sgC, &tmC, &full[st], j0, i0, lh);
+          tc::tma_load_3d(sg + Cfg::sgC + BR * 128, &tmC, &full[st], j0 + 64, i0, lh);
+        } else {
+          tc::tma_load_3d(sg + Cfg::sgC, &tmC, &full[st], 0, i0 / 8, (lh * p.N8 + j0) / 8);
+        }
         *s_issued = it + 1;
       }
     }
@@ -412,10 +424,11 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint32_t sg = smem_u32(smem + st * Cfg::STAGE);
       // P / dC: M = keys in chunks of 8, BR * 16 bytes apart; K = rows, 16 bytes apart
       const uint64_t dPa = tc::make_sdesc(sg + Cfg::sgP, 128, BR * 16, tc::kLayoutNone);
-      const uint64_t dCa = tc::make_sdesc(sg + Cfg::sgC, 128, BR * 16, tc::kLayoutNone);
+      const uint64_t dCa = CONV ? tc::make_sdesc(sg + Cfg::sgC, BR * 128, 1024, tc::kLayoutSW128) : tc::make_sdesc(sg + Cfg::sgC, 128, BR * 16, tc::kLayoutNone);
+      constexpr uint32_t c_step = CONV ? 2048 / 16 : 16;       // 16 rows
       const uint64_t dOb = tc::make_sdesc(sg + Cfg::sgdO, 16, 1024, tc::kLayoutSW128);
       const uint64_t dQb = tc::make_sdesc(sg + Cfg::sgQ + (HALO - pq) * 128, 128, 1024, tc::kLayoutSW128);
-      const uint32_t pa_hi = (uint32_t)(dPa >> 32), pa_lo = (uint32_t)dPa, ca_lo = (uint32_t)dCa;
+      const uint32_t pa_hi = (uint32_t)(dPa >> 32), pa_lo = (uint32_t)dPa, ca_hi = (uint32_t)(dCa >> 32), ca_lo = (uint32_t)dCa;
       const uint32_t ob_hi = (uint32_t)(dOb >> 32), ob_lo = (uint32_t)dOb, qb_hi = (uint32_t)(dQb >> 32), qb_lo = (uint32_t)dQb;
       ok = tc::mbar_wait_warp(&full[st], ph, s_abort);
       if (!ok) break;
@@ -429,9 +442,9 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const bool pair = gi < pairs;
         const uint32_t dacc = tmem + 64 * (1 + 2 * gi), idg = pair ? idescK2 : idescV;
         const uint32_t bl = qb_lo + (uint32_t)(2 * gi * (128 >> 4));
-        tc::mma_ss2pe(dacc, ca_lo, pa_hi, bl, qb_hi, idg, it != 0);
+        tc::mma_ss2pe(dacc, ca_lo, ca_hi, bl, qb_hi, idg, it != 0);
 #pragma unroll
-        for (int k = 1; k < BR / 16; ++k) tc::mma_ss2e<1>(dacc, ca_lo + (uint32_t)(k * 16), pa_hi, bl + (uint32_t)(k * (2048 / 16)), qb_hi, idg);
+        for (int k = 1; k < BR / 16; ++k) tc::mma_ss2e<1>(dacc, ca_lo + k * c_step, ca_hi, bl + (uint32_t)(k * (2048 / 16)), qb_hi, idg);
       }
       tc::mma_commit_e(&empty[st]);
     }
@@ -444,6 +457,7 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (nblk > 0) ok = __all_sync(0xffffffffu, tc::mbar_wait(all_done, 0, s_abort));
     tc::tc_fence_after();
     const bool have = nblk > 0 && ok;
+    pdl_wait();
     // dKt leaves as (hi, lo) bf16 pairs (its adjoint takes bf16 operands; one rounding would be one more than dS K has): the hi
     // tiles of all taps go through the stages (read by no MMA any more), then the lo tiles
     for (int hl = 0; hl < (dK.out == nullptr ? 2 : 1); ++hl) {
@@ -505,29 +519,42 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
 // ==========================================================================================
 namespace {
+// An X8 tensor as rows of 128 bytes (8 query rows x 8 keys): box = `rows` query rows x `keys` keys, landing as [keys / 8][rows][16 B]
+// with one copy (as bulk copies of one key chunk each, 1 to 2 KB, the copy engine's cost per copy was what bound these kernels).
+bool make_x8_map(CUtensorMap* map, const bf16* base, const MixParams& mp, int rows, int keys) {
+  return make_tensor_map_bf16(map, base, 64, mp.RP / 8, (size_t)mp.nU * mp.G * (mp.N8 / 8), 64, rows / 8, false, keys / 8);
+}
+
+// dC with a filter: row-major, rows x 64 keys in a 128-byte-swizzled tile.
+bool make_dc_map(CUtensorMap* map, const MixParams& mp, int rows) {
+  return make_tensor_map_bf16(map, mp.C8, mp.N8, mp.RP, (size_t)mp.nU * mp.G, 64, rows, true);
+}
+
 template <int D>
 cudaError_t launch_pv_t(const TrainParams& p, const MixParams& mp, cudaStream_t stream) {
   using Cfg = PvCfg<D>;
-  alignas(64) CUtensorMap tmV;
+  alignas(64) CUtensorMap tmP, tmV;
+  if (!make_x8_map(&tmP, mp.P8, mp, Cfg::BM, Cfg::BC)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmV, p.V, D, p.N, (size_t)p.B * p.H, 64, Cfg::BC, true)) return cudaErrorInvalidValue;
   auto kern = mix_pv_kernel<D>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
-  return launch_pdl(kern, dim3(mp.nRT, mp.nU * mp.G), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmV, mp, p.O, p.o_bf16, p.M, p.L, p.LSEout);
+  return launch_pdl(kern, dim3(mp.nRT, mp.nU * mp.G), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmP, tmV, mp, p.O, p.o_bf16, p.M, p.L, p.LSEout);
 }
-template <int D>
+template <int D, int NT_, bool CONV>
 cudaError_t launch_dq_t(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, cudaStream_t stream) {
-  using Cfg = MixDqCfg<D>;
+  using Cfg = MixDqCfg<D, NT_, CONV>;
   const size_t BH = (size_t)p.B * p.H;
-  const bool conv = p.theta != nullptr;
-  alignas(64) CUtensorMap tmB;
+  constexpr bool conv = CONV;
+  alignas(64) CUtensorMap tmC, tmB;
+  if (!(CONV ? make_dc_map(&tmC, mp, Cfg::AR) : make_x8_map(&tmC, mp.C8, mp, Cfg::AR, Cfg::BC))) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmB, conv ? Kt : p.K, D, p.N, conv ? BH * p.cq * 2 : BH, 64, Cfg::BC, true)) return cudaErrorInvalidValue;
-  auto kern = mix_dq_kernel<D>;
+  auto kern = mix_dq_kernel<D, NT_, CONV>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
   const MixGradOut out = {p.dQo, conv && p.causal ? p.dQ : nullptr, p.grad_bf16, conv ? kLn2 : p.scale};
-  return launch_pdl(kern, dim3((mp.nRT + 1) / 2, mp.nU * mp.G), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmB, mp, conv ? p.cq : 1,
-                    conv ? 2 : 1, out);
+  return launch_pdl(kern, dim3((mp.nRT + NT_ - 1) / NT_, mp.nU * mp.G), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmC, tmB, mp, conv ? p.cq : 1,
+                    out);
 }
 }  // namespace
 
@@ -535,22 +562,29 @@ cudaError_t launch_mix_pv(const TrainParams& p, const MixParams& mp, cudaStream_
   return p.d == 64 ? launch_pv_t<64>(p, mp, stream) : launch_pv_t<128>(p, mp, stream);
 }
 cudaError_t launch_mix_dq(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, cudaStream_t stream) {
-  return p.d == 64 ? launch_dq_t<64>(p, mp, Kt, stream) : launch_dq_t<128>(p, mp, Kt, stream);
+  // two row tiles per CTA share the key tiles; with fewer than two such CTAs per SM one tile per CTA fills the GPU better
+  const bool one = (long)((mp.nRT + 1) / 2) * mp.nU * mp.G < 2 * 148;
+#define FMTA_MIX_DQ(DD, C) (one ? launch_dq_t<DD, 1, C>(p, mp, Kt, stream) : launch_dq_t<DD, 2, C>(p, mp, Kt, stream))
+  if (p.theta) return p.d == 64 ? FMTA_MIX_DQ(64, true) : FMTA_MIX_DQ(128, true);
+  return p.d == 64 ? FMTA_MIX_DQ(64, false) : FMTA_MIX_DQ(128, false);
+#undef FMTA_MIX_DQ
 }
-cudaError_t launch_mix_dkdv(const TrainParams& p, const MixParams& mp, __nv_bfloat16* dKt, cudaStream_t stream) {
+cudaError_t launch_mix_dkdv(const TrainParams& p, const MixParams& mp, __nv_bfloat16* dKt, bool early, cudaStream_t stream) {
   using Cfg = MixDkvCfg;
   const size_t BH = (size_t)p.B * p.H;
   const bool conv = p.theta != nullptr;
   const int cq = conv ? p.cq : 1;
-  alignas(64) CUtensorMap tmQ, tmdO, tmdKt;
+  alignas(64) CUtensorMap tmQ, tmdO, tmdKt, tmP, tmC;
+  if (!make_x8_map(&tmP, mp.P8, mp, Cfg::BR, Cfg::BK) || !(conv ? make_dc_map(&tmC, mp, Cfg::BR) : make_x8_map(&tmC, mp.C8, mp, Cfg::BR, Cfg::BK))) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmQ, p.Q, p.d, p.N, BH, 64, Cfg::QR, true)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmdO, p.dO, p.d, p.N, BH, 64, Cfg::BR, true)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmdKt, conv ? dKt : p.Q, p.d, p.N, conv ? BH * cq * 2 : BH, 64, Cfg::BK, true)) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(mix_dkdv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+  auto kern = conv ? mix_dkdv_kernel<true> : mix_dkdv_kernel<false>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
   const MixGradOut dV = {p.dVo, nullptr, p.grad_bf16, 1.f}, dK = {conv ? nullptr : p.dKo, nullptr, p.grad_bf16, p.scale};
-  return launch_pdl(mix_dkdv_kernel, dim3(mp.N8 / 128 * (p.d / 64), mp.nU * mp.G), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmQ, tmdO,
-                    tmdKt, mp, cq, p.d, dV, dK);
+  return launch_pdl(kern, dim3(mp.N8 / 128 * (p.d / 64), mp.nU * mp.G), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmQ, tmdO,
+                    tmdKt, tmP, tmC, mp, cq, p.d, dV, dK, (int)early);
 }
 
 }  // namespace fmta

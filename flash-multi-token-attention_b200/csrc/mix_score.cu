@@ -30,13 +30,14 @@ struct MixCfg {
   static constexpr int KT = G >= 8 ? 4 : 8;                    // keys per thread and pass
   static constexpr int GC = G < 4 ? G : 4;                     // output heads per register pass
   static constexpr int NPASS = KB / 2 / KT;
-  static constexpr bool RES = CONV && G * SL * QR * 128 <= 140 * 1024;   // Q resident
-  static constexpr int SLOT = CONV ? QR * 128 : BM * 128;      // ring slot: one A slab tile, or B slab tiles
+  static constexpr bool RES = CONV && G * SL * QR * 128 <= 100 * 1024;   // Q resident; else (with a filter) two stages of one head's Q
+  static constexpr int Q_HEAD = SL * QR * 128;
+  static constexpr int SLOT = BM * 128;                        // ring slot: one A slab tile, or B slab tiles
   static constexpr int TB = KB * 128, TPS = 16384 / TB;        // B slab tile (KB keys x 64 columns), tiles per slot
   static constexpr bool DW_MMA = BWD && G == 16;               // dW by mma.sync from transposed bf16 pairs; else in registers
   static constexpr int oQ = 0;
-  static constexpr int oW = oQ + (RES ? G * SL * QR * 128 : 0);
-  static constexpr int W_BYTES = G * G * 8;                    // (w, w) pairs
+  static constexpr int oW = oQ + (CONV ? (RES ? G : 2) * Q_HEAD : 0);
+  static constexpr int W_BYTES = G * G * 4;
   static constexpr int oRow = oW + (BWD ? 2 : 1) * ((W_BYTES + 127) / 128 * 128);   // backward: LSE, D; forward: ref, exchange
   static constexpr int oDW = oRow + 2 * G * BM * 4;
   static constexpr int DW_BYTES = DW_MMA ? 8 * 4096 : (BWD ? 8 * G * G * 4 : 0);
@@ -44,14 +45,13 @@ struct MixCfg {
   static constexpr int oRing = (oBar + 512 + 1023) / 1024 * 1024;
   static constexpr int NSLOT_ = (226 * 1024 - oRing) / SLOT;
   static constexpr int NSLOT = NSLOT_ > 20 ? 20 : NSLOT_;
-  // a slot is held until the last tile that uses it: B tiles of several heads in one slot, with an A slot for each, and (Q not
-  // resident) the Q slots of a head while its stacked keys pass
+  // a slot is held until the last tile that uses it: B tiles of several heads in one slot, with an A slot for each
   static constexpr int TPP = TPS < NSLOT - 2 ? TPS : NSLOT - 2;
   static constexpr int kSmemBytes = oRing + NSLOT * SLOT + 1024;
   // 8 element-wise warps with 216 registers, a warpgroup with 72 for the TMA and the MMA warp: 256 * 216 + 128 * 72 = 384 * 168,
   // the registers the block is launched with
   static constexpr int kThreads = 384, kRegsEw = 216, kRegsOther = 72;
-  static_assert(NSLOT >= 4 && (RES || !CONV || NSLOT >= SL + (7 * 2 * SL + TPS - 1) / TPS), "ring");
+  static_assert(NSLOT >= 4, "ring");
   static_assert(kSmemBytes <= 227 * 1024, "shared memory");
   static_assert(SLOT % 1024 == 0 && TB % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
 };
@@ -67,15 +67,16 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* sQ = smem + Cfg::oQ;
   unsigned char* sRing = smem + Cfg::oRing;
-  uint64_t* sWf = reinterpret_cast<uint64_t*>(smem + Cfg::oW);                 // [g'][g] (w, w): the mix
-  uint64_t* sWb = reinterpret_cast<uint64_t*>(smem + Cfg::oW + (Cfg::W_BYTES + 127) / 128 * 128);   // [g][g']: its transpose
+  float* sWf = reinterpret_cast<float*>(smem + Cfg::oW);                       // [g'][g]: the mix
+  float* sWb = reinterpret_cast<float*>(smem + Cfg::oW + (Cfg::W_BYTES + 127) / 128 * 128);   // [g][g']: its transpose
   float* sR0 = reinterpret_cast<float*>(smem + Cfg::oRow);                      // [G][128]: LSE (log2) / ref
   float* sR1 = sR0 + G * BM;                                                    // [G][128]: D / exchange
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::oBar);
   uint64_t* full = bars;                 // [NSLOT]
   uint64_t* empty = full + NSLOT;        // [NSLOT]
-  uint64_t* q_full = empty + NSLOT;
-  uint64_t* s_full = q_full + 1;         // [2]
+  uint64_t* q_full = empty + NSLOT;      // [2] resident Q, or the two stages
+  uint64_t* q_empty = q_full + 2;        // [2]
+  uint64_t* s_full = q_empty + 2;        // [2]
   uint64_t* s_free = s_full + 2;         // [2]
   uint64_t* d_full = s_free + 2;
   uint64_t* d_free = d_full + 1;
@@ -84,8 +85,9 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(mma_drain + 1);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
   volatile int* s_issued = s_abort + 1;
+  volatile int* s_qissued = s_abort + 3;
   volatile int* s_redo = s_abort + 2;    // forward: a logit left the range of P around the row's reference
-  static_assert((2 * NSLOT + 9) * 8 + 16 <= 512, "barrier block");
+  static_assert((2 * NSLOT + 12) * 8 + 16 <= 512, "barrier block");
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int N = p.N, cq = CONV ? p.cq : 1, pq = cq - 1, pk = CONV ? (p.ck - 1) / 2 : 0;
@@ -101,9 +103,9 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
   if (tid == 0) {
     for (int i = 0; i < NSLOT; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 1); }
-    tc::mbar_init(q_full, 1); tc::mbar_init(d_full, 1); tc::mbar_init(d_free, 8); tc::mbar_init(x_bar, 8); tc::mbar_init(mma_drain, 1);
-    for (int i = 0; i < 2; ++i) { tc::mbar_init(&s_full[i], 1); tc::mbar_init(&s_free[i], 8); }
-    *s_abort = 0; *s_issued = 0; *s_redo = 0;
+    tc::mbar_init(d_full, 1); tc::mbar_init(d_free, 8); tc::mbar_init(x_bar, 8); tc::mbar_init(mma_drain, 1);
+    for (int i = 0; i < 2; ++i) { tc::mbar_init(&q_full[i], 1); tc::mbar_init(&q_empty[i], 1); tc::mbar_init(&s_full[i], 1); tc::mbar_init(&s_free[i], 8); }
+    *s_abort = 0; *s_issued = 0; *s_redo = 0; *s_qissued = 0;
     tc::mbar_fence_init();
   }
   if (warp == 9) {
@@ -116,8 +118,8 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   for (int i = tid; i < G * G; i += Cfg::kThreads) {
     const float w = p.W[(size_t)grp * G * G + i];            // [g][g']
     const int g = i / G, g2 = i % G;
-    sWf[g2 * G + g] = f2_pack(w * p.c2, w * p.c2);
-    if (BWD) sWb[g * G + g2] = f2_pack(w, w);
+    sWf[g2 * G + g] = w * p.c2;
+    if (BWD) sWb[g * G + g2] = w;
   }
   for (int i = tid; i < G * BM; i += Cfg::kThreads) {
     const int g = i / BM, r = R0 + i % BM;
@@ -131,7 +133,7 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = *s_tmem;
-  int ring = 0, meets = 0;               // ring position (warps 8 and 9) and meetings of the element-wise warps, over all attempts
+  int ring = 0, ring_ph = 0, qring = 0, meets = 0;    // ring positions (warps 8 and 9) and meetings of the element-wise warps, over all attempts
 
   // forward: a second attempt only when a logit exceeds its row's reference (the maximum of the first keys) by 2^100
   const int attempts = nblk > 0 ? (BWD ? 1 : 2) : 0;
@@ -176,11 +178,14 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       auto stacked = [&](int key) {
         const int nt = cq * 2 * SL;                          // (tap, hi / lo, slab) tiles of a head
         for (int g = 0; g < G && ok; ++g) {
-          if (!Cfg::RES)
-            for (int sl = 0; sl < SL && ok; ++sl) {
-              const int s = slot_of(Cfg::QR * 128);
-              if (ok) tc::tma_load_3d(sRing + s * SLOT, &tmQ, &full[s], sl * 64, R0 - HALO, bh0 + g);
-            }
+          if (!Cfg::RES) {
+            const int st = qring & 1;
+            if (!tc::mbar_wait(&q_empty[st], ((qring >> 1) & 1) ^ 1, s_abort)) { ok = false; return; }
+            tc::mbar_expect_tx(&q_full[st], Cfg::Q_HEAD);
+            for (int sl = 0; sl < SL; ++sl) tc::tma_load_3d(sQ + st * Cfg::Q_HEAD + sl * (Cfg::QR * 128), &tmQ, &q_full[st], sl * 64, R0 - HALO, bh0 + g);
+            ++qring;
+            *s_qissued = qring;
+          }
           for (int i = 0; i < nt && ok; i += TPS) {
             const int n = min(TPS, nt - i), s = slot_of(n * TB);
             if (!ok) return;
@@ -206,10 +211,10 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint32_t q_lo = (uint32_t)tc::make_sdesc(smem_u32(sQ), 16, 1024, tc::kLayoutSW128);
     bool ok = true;
     auto take = [&]() -> int {
-      const int slot = ring % NSLOT, ph = (ring / NSLOT) & 1;
-      if (!tc::mbar_wait_warp(&full[slot], ph, s_abort)) { ok = false; return slot; }
+      const int slot = ring;
+      if (!tc::mbar_wait_warp(&full[slot], ring_ph, s_abort)) { ok = false; return slot; }
       tc::tc_fence_after();
-      ++ring;
+      if (++ring == NSLOT) { ring = 0; ring_ph ^= 1; }
       return slot;
     };
     auto mma4 = [&](uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t acc) {
@@ -232,27 +237,26 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     auto stacked = [&](uint32_t dst) {
       const int nt = cq * 2 * SL;
       for (int g = 0; g < G && ok; ++g) {
-        uint32_t a0[SL];
-        int qs[SL];
-#pragma unroll
-        for (int sl = 0; sl < SL; ++sl) {
-          if (Cfg::RES) { a0[sl] = q_lo + (uint32_t)((g * SL + sl) * (Cfg::QR * 8)); qs[sl] = 0; }
-          else { qs[sl] = take(); if (!ok) return; a0[sl] = lo0 + (uint32_t)(qs[sl] * (SLOT >> 4)); }
-          a0[sl] += (uint32_t)((HALO - pq) * 8);             // row shift: 128 bytes per row
+        const int st = qring & 1;
+        if (!Cfg::RES) {
+          ok = tc::mbar_wait_warp(&q_full[st], (qring >> 1) & 1, s_abort);
+          if (!ok) return;
+          ++qring;
         }
+        const uint32_t aq = q_lo + (uint32_t)((Cfg::RES ? g : st) * (Cfg::Q_HEAD >> 4) + (HALO - pq) * 8);   // row shift: 128 bytes per row
         for (int i = 0; i < nt; i += TPS) {
           const int s = take();
           if (!ok) return;
-          const int n = min(TPS, nt - i);
-          for (int j = 0; j < n; ++j) {
-            const int a = (i + j) / (2 * SL), sl = (i + j) % SL;
-            mma4(dst + g * KB, (SL > 1 && sl ? a0[SL - 1] : a0[0]) + (uint32_t)(a * 8), lo0 + (uint32_t)(s * (SLOT >> 4) + j * (TB >> 4)), i + j != 0);
-          }
+          const uint32_t bl = lo0 + (uint32_t)(s * (SLOT >> 4));
+#pragma unroll
+          for (int j = 0; j < TPS; ++j)
+            if (i + j < nt) {
+              const int a = (i + j) / (2 * SL), sl = (i + j) % SL;
+              mma4(dst + g * KB, aq + (uint32_t)(sl * (Cfg::QR * 8) + a * 8), bl + (uint32_t)(j * (TB >> 4)), i + j != 0);
+            }
           tc::mma_commit_e(&empty[s]);
         }
-        if (!Cfg::RES)
-#pragma unroll
-          for (int sl = 0; sl < SL; ++sl) tc::mma_commit_e(&empty[qs[sl]]);
+        if (!Cfg::RES) tc::mma_commit_e(&q_empty[st]);
       }
     };
     if (Cfg::RES && attempt == 0) ok = tc::mbar_wait_warp(q_full, 0, s_abort);
@@ -318,15 +322,18 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
         for (int k = 0; k < KP; ++k) s[g][k] = f2_pack(v[g][2 * k], v[g][2 * k + 1]);
     };
-    // acc[c] = sum_x tab[x][g0 + c] * in[x]
-    auto mix = [&](uint64_t (&acc)[GC][KP], const uint64_t (&in)[G][KP], const uint64_t* tab, int g0) {
+    // acc[c] = sum_x tab[x][g0 + c] * in[x].  A broadcast load returns its bytes to all 32 lanes (128 bytes per cycle), so the
+    // weights are loaded as single floats and doubled in registers: as (w, w) pairs they took twice the time of the FMAs.
+    auto mix = [&](uint64_t (&acc)[GC][KP], const uint64_t (&in)[G][KP], const float* tab, int g0) {
 #pragma unroll
       for (int x = 0; x < G; ++x) {
         uint64_t w[GC];
-#pragma unroll
-        for (int c = 0; c < GC; c += 2) {
-          const ulonglong2 t2 = *reinterpret_cast<const ulonglong2*>(tab + x * G + g0 + c);
-          w[c] = t2.x; w[c + 1] = t2.y;
+        if constexpr (GC == 4) {
+          const float4 t = *reinterpret_cast<const float4*>(tab + x * G + g0);
+          w[0] = f2_pack(t.x, t.x); w[1] = f2_pack(t.y, t.y); w[2] = f2_pack(t.z, t.z); w[3] = f2_pack(t.w, t.w);
+        } else {
+          const float2 t = *reinterpret_cast<const float2*>(tab + x * G + g0);
+          w[0] = f2_pack(t.x, t.x); w[1] = f2_pack(t.y, t.y);
         }
 #pragma unroll
         for (int c = 0; c < GC; ++c)
@@ -338,6 +345,15 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       bf16* dst = base + ((lh * kc8 + (key >> 3)) * p.RP + gi) * 8 + (key & 7);
       if constexpr (KT == 8) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
       else *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+    };
+    auto store_dc = [&](size_t lh, int key, const uint32_t (&w)[KP]) {
+      if constexpr (!CONV) {
+        store8(p.C8, lh, key, w);
+      } else {
+        bf16* dst = p.C8 + (lh * p.RP + gi) * p.N8 + key;
+        if constexpr (KT == 8) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+        else *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+      }
     };
 
     if constexpr (!BWD) {
@@ -471,6 +487,11 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           const int j = j0 + ps * KT;
           uint64_t s[G][KP], dc[G][KP];
           load_s(s, tS0 + ps * KT, j);
+          if (ps == NPASS - 1) {                             // the scores are in registers: the next block's MMAs may start
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(s_free);
+          }
           const bool mask = !__all_sync(0xffffffffu, j + KT - 1 <= jlim);
 #pragma unroll
           for (int g0 = 0; g0 < G; g0 += GC) {
@@ -496,10 +517,10 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
               store8(p.P8, lh0 + g0 + c, j, w);
             }
           }
-          if (ps == NPASS - 1) {                             // both tiles are in registers
+          if (ps == NPASS - 1) {
             tc::tc_fence_before();
             __syncwarp();
-            if (lane == 0) { tc::mbar_arrive(s_free); tc::mbar_arrive(d_free); }
+            if (lane == 0) tc::mbar_arrive(d_free);
           }
           // ---- dC_x = sum_g W[g,x] dC'_g ----
 #pragma unroll
@@ -522,7 +543,7 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
               uint32_t w[KP];
 #pragma unroll
               for (int k = 0; k < KP; ++k) w[k] = pack_bf16(v[2 * k], v[2 * k + 1]);
-              store8(p.C8, lh0 + x0 + c, j, w);
+              store_dc(lh0 + x0 + c, j, w);
             }
           }
           // ---- dW[g][x] += sum dC'_g S_x ----
@@ -614,7 +635,9 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const int nch = (k_hi - k_lo) / 8;
         for (int i = tid; i < G * nch * 16; i += 256) {
           const int g = i / (nch * 16), rem = i - g * nch * 16;
-          *reinterpret_cast<uint4*>(p.C8 + (((lh0 + g) * kc8 + (k_lo >> 3) + (rem >> 4)) * p.RP + p.nRT * BM + (rem & 15)) * 8) = make_uint4(0u, 0u, 0u, 0u);
+          const int row = p.nRT * BM + (rem & 15), ch = rem >> 4;
+          bf16* dst = CONV ? p.C8 + ((lh0 + g) * p.RP + row) * p.N8 + k_lo + 8 * ch : p.C8 + (((lh0 + g) * kc8 + (k_lo >> 3) + ch) * p.RP + row) * 8;
+          *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
         }
       }
     }
@@ -640,7 +663,8 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (tid == 256) {
       volatile int never = 0;
       if (Cfg::RES && nblk > 0) tc::mbar_wait(q_full, 0, &never);
-      const int issued = *s_issued;
+      const int issued = *s_issued, qi = *s_qissued;
+      for (int id = max(0, qi - 2); id < qi; ++id) tc::mbar_wait(&q_full[id & 1], (id >> 1) & 1, &never);
       for (int id = max(0, issued - NSLOT); id < issued; ++id) tc::mbar_wait(&full[id % NSLOT], (id / NSLOT) & 1, &never);
     }
     if (tid == 256) { volatile int never = 0; tc::mbar_wait(mma_drain, 0, &never); }

@@ -31,7 +31,10 @@ MixPlan plan(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool 
   // keys per CTA: long chunks keep the row tile's operands and amortise the fixed cost of a CTA; about three CTAs per SM
   // (dead ones above the diagonal not counted) even out the load
   m.kch = 1024;
-  while (m.kch > 128 && (long)m.nRT * ((m.N8 + m.kch - 1) / m.kch) * m.nU / (causal ? 2 : 1) < 3 * 148) m.kch /= 2;
+  auto live = [&]() { return (long)m.nRT * ((m.N8 + m.kch - 1) / m.kch) * m.nU / (causal ? 2 : 1); };
+  while (m.kch > 128 && live() < 3 * 148) m.kch /= 2;
+  // a GPU that is not full: half as long CTAs (a block is at most 64 keys there; with a filter a CTA's fixed cost is larger)
+  if (live() < (conv ? 74 : 148) && G >= (conv ? 4 : 8)) m.kch = 64;
   m.nKC = (m.N8 + m.kch - 1) / m.kch;
   m.rows = (size_t)B * H * N;
   const int band = (cq - 1) + (ck - 1) / 2;
@@ -148,7 +151,7 @@ cudaError_t launch_mix_bwd(const TrainParams& p_, const void* dO, bool do_f32, c
     FMTA_TRY(launch_mix_score(p, q, Kt, true, stream));
     if (conv && p.causal) FMTA_TRY(launch_bwd_band_given(p, q.u0 * p.G, q.nU * p.G, stream));
     if (want & 1) FMTA_TRY(launch_mix_dq(p, q, Kt, stream));
-    if ((want & 2) || conv) FMTA_TRY(launch_mix_dkdv(p, q, dKt, stream));      // dTheta comes out of dKt
+    if ((want & 2) || conv) FMTA_TRY(launch_mix_dkdv(p, q, dKt, want & 1, stream));      // dTheta comes out of dKt
   }
   if (conv) {
     FMTA_TRY(launch_dk_post(p, dKt, true, theta_part + (size_t)m.theta_band_slots * p.H * p.cq * p.ck, status, stream));

@@ -12,8 +12,10 @@
 //
 // Operand tensors P / dC: "X8" = [head][key chunk of 8][row][8 keys], rows padded to X8 rows = roundup(N, 128) + 16.  A thread
 // of the score kernel owns a row, so its 16-byte stores of 8 keys are contiguous across a warp; and every consumer gets an
-// MMA operand with plain bulk copies of rows x 16 bytes: no-swizzle core matrices, K-major for O = P V and dQ (a row shift is
-// 16 bytes), MN-major for dV = P^T dO and dKt = dC^T Q.
+// MMA operand with one tiled copy of 128-byte pieces: no-swizzle core matrices, K-major for O = P V and dQ (a row shift is
+// 16 bytes), MN-major for dV = P^T dO and dKt = dC^T Q.  With a filter dC is row-major instead: dQ reads it at c_q row shifts, and a
+// shift inside the no-swizzle layout misaligns every core matrix (117 cycles per 128x128x16 MMA instead of 80); in a swizzled
+// tile it moves whole rows.
 #pragma once
 #include <cuda.h>
 
@@ -32,7 +34,7 @@ struct MixParams {
   const float* Cband;     // causal with a filter: [B*H, N, band] scores of the band after the filter, natural units (else nullptr)
   float* dCband;          // backward: the gradient of those
   bf16* P8;               // [heads of the launch][N8 / 8][RP][8]
-  bf16* C8;               // backward: dC
+  bf16* C8;               // backward: dC, the same; with a filter row-major, [heads of the launch][RP][N8]
   float* ref;             // forward: [heads of the launch][N8 / 16][RP] log2 reference of 16 keys of P
   float* stat;            // forward: [heads of the launch][2 nKC][3][RP]: row max, reference, sum, per key chunk and half
   float* dW_part;         // backward: [slots][H/G][G*G], slot = (b * nRT + row tile) * nKC + key chunk
@@ -70,6 +72,6 @@ FMTA_DEVINL uint64_t f2_mul(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f3
 cudaError_t launch_mix_score(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, bool bwd, cudaStream_t stream);
 cudaError_t launch_mix_pv(const TrainParams& p, const MixParams& mp, cudaStream_t stream);
 cudaError_t launch_mix_dq(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, cudaStream_t stream);
-cudaError_t launch_mix_dkdv(const TrainParams& p, const MixParams& mp, __nv_bfloat16* dKt, cudaStream_t stream);
+cudaError_t launch_mix_dkdv(const TrainParams& p, const MixParams& mp, __nv_bfloat16* dKt, bool early, cudaStream_t stream);
 
 }  // namespace fmta
