@@ -276,20 +276,152 @@ FMTA_DEVINL bool elect_one() {
 FMTA_DEVINL bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
+// Elections and MMAs sit in one asm block, the MMAs PREDICATED on the elected lane.  Behind a branch (`if (elect_one())`
+// around each MMA) every operand goes through the reconvergence of the warp and back into uniform registers: back to back
+// that took 101-108 cycles per MMA whatever its size; predicated, 39 cycles at N = 16 and the tensor core's own rate above
+// (64 cycles for 128 x 128 x 16, 43 for a pair's 256 x 64 x 16).
 template <int ACC>
 FMTA_DEVINL void mma_ss2e(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc) {
-  if (elect_one()) mma_ss2<ACC>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc);
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "mov.b64 da, {%1, %2};\n\t"
+      "mov.b64 db, {%3, %4};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "n"(ACC)
+      : "memory");
 }
 FMTA_DEVINL void mma_ss2pe(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
                            uint32_t accumulate) {
-  if (elect_one()) mma_ss2p(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc, accumulate);
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "mov.b64 da, {%1, %2};\n\t"
+      "mov.b64 db, {%3, %4};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+      : "memory");
 }
 template <int ACC>
 FMTA_DEVINL void mma_ts2e(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc) {
-  if (elect_one()) mma_ts2<ACC>(d_tmem, a_tmem, b_lo, b_hi, idesc);
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "n"(ACC)
+      : "memory");
 }
 FMTA_DEVINL void mma_commit_e(uint64_t* bar) {
-  if (elect_one()) mma_commit(bar);
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
+      : "memory");
+}
+// Four MMAs of one chain: operands as_ and bs_ (descriptor units of 16 bytes; tensor-memory columns for a TMEM A) apart,
+// the first one overwriting unless `accumulate`.  G = 2: of a CTA pair.
+#define FMTA_MMA4_SS(CG)                                                                                          \
+  asm volatile(                                                                                                  \
+      "{\n\t.reg .pred p, q, t;\n\t.reg .b64 da, db;\n\t"                                                           \
+      "elect.sync _|q, 0xffffffff;\n\t"                                                                           \
+      "setp.ne.b32 p, %12, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"                                                           \
+      "mov.b64 da, {%1, %9};\n\tmov.b64 db, {%5, %10};\n\t"                                                          \
+      "@q tcgen05.mma.cta_group::" CG ".kind::f16 [%0], da, db, %11, p;\n\t"                                        \
+      "mov.b64 da, {%2, %9};\n\tmov.b64 db, {%6, %10};\n\t"                                                          \
+      "@q tcgen05.mma.cta_group::" CG ".kind::f16 [%0], da, db, %11, t;\n\t"                                        \
+      "mov.b64 da, {%3, %9};\n\tmov.b64 db, {%7, %10};\n\t"                                                          \
+      "@q tcgen05.mma.cta_group::" CG ".kind::f16 [%0], da, db, %11, t;\n\t"                                        \
+      "mov.b64 da, {%4, %9};\n\tmov.b64 db, {%8, %10};\n\t"                                                          \
+      "@q tcgen05.mma.cta_group::" CG ".kind::f16 [%0], da, db, %11, t;\n\t}"                                       \
+      ::"r"(d_tmem), "r"(a_lo), "r"(a_lo + as_), "r"(a_lo + 2 * as_), "r"(a_lo + 3 * as_), "r"(b_lo), "r"(b_lo + bs_), \
+      "r"(b_lo + 2 * bs_), "r"(b_lo + 3 * bs_), "r"(a_hi), "r"(b_hi), "r"(idesc), "r"(accumulate)                   \
+      : "memory")
+#define FMTA_MMA4_TS(CG)                                                                                          \
+  asm volatile(                                                                                                  \
+      "{\n\t.reg .pred p, q, t;\n\t.reg .b64 db;\n\t"                                                               \
+      "elect.sync _|q, 0xffffffff;\n\t"                                                                           \
+      "setp.ne.b32 p, %11, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"                                                           \
+      "mov.b64 db, {%5, %9};\n\t@q tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [%1], db, %10, p;\n\t"             \
+      "mov.b64 db, {%6, %9};\n\t@q tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [%2], db, %10, t;\n\t"             \
+      "mov.b64 db, {%7, %9};\n\t@q tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [%3], db, %10, t;\n\t"             \
+      "mov.b64 db, {%8, %9};\n\t@q tcgen05.mma.cta_group::" CG ".kind::f16 [%0], [%4], db, %10, t;\n\t}"            \
+      ::"r"(d_tmem), "r"(a_tmem), "r"(a_tmem + as_), "r"(a_tmem + 2 * as_), "r"(a_tmem + 3 * as_), "r"(b_lo),       \
+      "r"(b_lo + bs_), "r"(b_lo + 2 * bs_), "r"(b_lo + 3 * bs_), "r"(b_hi), "r"(idesc), "r"(accumulate)             \
+      : "memory")
+template <int G = 1>
+FMTA_DEVINL void mma4_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t as_, uint32_t b_lo, uint32_t b_hi, uint32_t bs_,
+                         uint32_t idesc, uint32_t accumulate) {
+  if constexpr (G == 1) FMTA_MMA4_SS("1"); else FMTA_MMA4_SS("2");
+}
+template <int G = 1>
+FMTA_DEVINL void mma4_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t as_, uint32_t b_lo, uint32_t b_hi, uint32_t bs_, uint32_t idesc,
+                         uint32_t accumulate) {
+  if constexpr (G == 1) FMTA_MMA4_TS("1"); else FMTA_MMA4_TS("2");
+}
+#undef FMTA_MMA4_SS
+#undef FMTA_MMA4_TS
+
+// ---- CTA pairs (cta_group::2) --------------------------------------------------------------
+// The two CTAs of a cluster of 2 work on one 256-row MMA: each holds its 128 rows of A and of the accumulator and
+// HALF of the B tile; the CTA of rank 0 issues for both.  Shared-memory operands sit at the same offsets in both CTAs,
+// barriers the issuer waits on live in rank 0's shared memory, commits arrive in both.
+FMTA_DEVINL uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+FMTA_DEVINL uint32_t cluster_addr(const void* smem, uint32_t rank) {      // shared::cluster address of the same variable in CTA `rank`
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(smem)), "r"(rank));
+  return a;
+}
+FMTA_DEVINL void cluster_sync_all() {     // every thread of both CTAs
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+FMTA_DEVINL void mbar_arrive_cluster(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+FMTA_DEVINL void st_cluster_u32(uint32_t cluster_dst, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_dst), "r"(v) : "memory");
+}
+// bounded wait whose arrivals may come from the other CTA
+FMTA_DEVINL bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t limit = kSpinLimit) {
+  for (uint32_t i = 0; i < limit; ++i) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    if (ok) return true;
+    if ((i & 1023u) == 1023u && *abort_flag) return false;
+  }
+  *abort_flag = 1;
+  return false;
+}
+FMTA_DEVINL bool mbar_wait_cluster_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag));
+}
+// tile into this CTA's shared memory, completing on a barrier of rank 0 (cluster_bar: shared::cluster address)
+FMTA_DEVINL void tma_load_3d_pair(void* smem_dst, const CUtensorMap* map, uint32_t cluster_bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(map), "r"(cluster_bar), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+FMTA_DEVINL void tmem_alloc_pair(uint32_t* smem_dst, uint32_t ncols) {    // one warp of each CTA
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+FMTA_DEVINL void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {      // one warp of each CTA
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+// arrive on the barrier at this offset in both CTAs once all MMAs issued so far by this thread have completed
+FMTA_DEVINL void mma_commit_pair(uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+      ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 
 // Instruction descriptor, kind::f16: bf16 x bf16 -> fp32, M x N tile.
@@ -303,8 +435,8 @@ __host__ __device__ constexpr uint32_t make_idesc(int M, int N, int a_mn_major, 
 // Shared-memory matrix descriptor.
 //   bits [0,14) start address >> 4; [16,30) leading byte offset >> 4; [32,46) stride byte offset >> 4;
 //   [46,48) version = 1; [61,64) layout: 0 = no swizzle ("interleaved" 8x16-byte core matrices),
-//   2 = 128-byte swizzle.
-constexpr uint64_t kLayoutNone = 0, kLayoutSW128 = 2;
+//   2 = 128-byte swizzle, 4 = 64-byte swizzle.
+constexpr uint64_t kLayoutNone = 0, kLayoutSW128 = 2, kLayoutSW64 = 4;
 FMTA_DEVINL uint64_t make_sdesc(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes, uint64_t layout) {
   return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16) |
          ((uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32) | (1ull << 46) | (layout << 61);
