@@ -6,21 +6,19 @@
 // so those tiles are FlashAttention with c_q accumulating MMAs per score tile and no work on the
 // FP32 pipe.  This file holds
 //   ktilde_kernel : the memory-bound pre-pass that writes the c_q bf16 operands Kt_a;
-//   fwd_tc_kernel : the warp-specialised main kernel (1 TMA warp, 1 MMA warp, 2 softmax warpgroups);
+//   fwd_tc_kernel : the warp-specialised main kernel, a cluster of two CTAs (1 TMA warp, 1 MMA warp, 8 softmax warps each);
 //   launch_fwd_tc : tensor maps + launches.
 // Ownership is per score entry: the stacked kernel takes every entry with query - key >= pad_q +
 // pad_k (masking the rest of a diagonal tile), the band kernel (fwd_band.cu) takes the band entries.  The
 // kernel leaves an UN-normalised partial (O, m, l) per query row; the band kernel continues the
 // online softmax from that state over the band and writes the final O, M, L.
 //
-// Row-shifted A operands without copies: Q is staged in the no-swizzle K-major core-matrix
-// layout [d/8][rows][8 elements]; the M-direction stride of that layout is 16 bytes, so the
-// operand "Q shifted by s rows" is the same buffer with the descriptor start address advanced
-// by 16*s bytes.  K-tilde / V tiles use the 128-byte swizzle that TMA writes natively.
+// Row-shifted A operands without copies: Q is staged as a 128-byte-swizzled tile; the tensor core applies the swizzle
+// to the absolute shared-memory address, so the operand "Q shifted by s rows" is the same buffer with the descriptor
+// start address advanced by 128*s bytes.
 //
-// Every wait on an mbarrier is bounded (tc::mbar_wait); on expiry the CTA raises an abort flag,
-// records it in the caller's status word, drains its outstanding copies, frees its TMEM and
-// returns.  No TMA multicast, no cluster, cta_group::1 only.
+// Every wait on an mbarrier is bounded (tc::mbar_wait); on expiry the CTA raises an abort flag, both CTAs of the pair
+// drain their outstanding copies, record it in the caller's status word, free their TMEM and return.  No TMA multicast.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -144,266 +142,263 @@ struct TcParams {
   float* Mpart;   // [B,H,N]  row max, natural-log units
   float* Lpart;
   int* status;    // device word: set non-zero when a bounded wait expired
-  int H, N, cq, ck, causal;
-  int qb_hi;      // the grid covers the row blocks [qb_hi - gridDim.x, qb_hi) (all of them unless the call has a window)
+  int B, H, N, cq, ck, causal;
+  int qb_lo, qb_hi;      // row blocks [qb_lo, qb_hi) of 256 rows (all of them unless the call has a window)
   int selftest_expire;   // failure-detection self-test: the softmax warps' first wait is on a barrier nothing arrives at
 };
 
-// One CTA owns two row tiles of 128 query rows (one softmax warpgroup and one TMEM lane per row).
-// Every Kt / V tile staged in shared memory feeds the MMAs of both row tiles.  Tensor memory per row
-// tile: S (BC columns, fp32), P (BC / 2 columns, bf16 pairs) and O (D columns, fp32); S is released to
-// the next block's MMAs as soon as the softmax threads have loaded it into registers.
-//   d = 64 : key blocks are 128 wide, so that every score MMA is 128 x 128 x 16 (a 64-wide MMA is bound
-//            by shared-memory operand fetch: 4 KB of A per 2 KB of B);
-//   d = 128: two row tiles only fit the tensor memory with 64-key blocks (2 x (64 + 32 + 128) = 448
-//            columns).  A single 128-row tile with 128-key blocks has the cheaper MMAs, but streams
-//            fourteen 16 KB tiles per block for 128 rows -- 62 bytes per cycle, more than eleven ring
-//            slots cover at the latency of a TMA copy (tensor pipe 42 % busy); sharing every tile between
-//            256 rows halves that.
-template <int D, int NT_ = 2>
+// Two CTAs own 256 query rows (128 each: one TMEM lane per row) and walk blocks of 128 keys.
+//   S = sum_a Q^(a) Kt_a^T : 256 x 128 x 16 MMAs, each CTA stages its own Q and HALF the keys of every Kt tile;
+//   O += P V               : 256 x d x 16 MMAs, P in tensor memory, each CTA stages half the columns of V.
+// A single CTA's 128 x 128 x 16 MMA reads 8 KB of operands in 64 cycles, all the shared memory can deliver; a pair's reads
+// 6 KB per CTA, which leaves room for the copies that fill the ring, and every key tile crosses from L2 once for 256 rows.
+//   d = 64 : 256 tensor-memory columns and 113 KB, so two pairs share two SMs: one's softmax under the other's MMAs;
+//   d = 128: S is double-buffered instead (2 x 128 + 64 + 128 columns).
+// Measured (B200, c_q 6, causal, N 4096, single CTAs with two row tiles before): d = 64, B 4, H 16: 415 -> 387 us; d = 128,
+// B 8, H 32: 4.33 -> 3.7 ms (1040 TFLOP/s); one sequence of N 1000, 8 heads, d = 128: 80 -> 45 us with the pre-pass and the
+// band kernel.  What bounds it is the supply of key tiles (31 bytes per cycle and SM at the tensor core's rate) and power.
+template <int D>
 struct TcCfg {
-  static constexpr int BM = 128;               // rows per tile (= TMEM lanes)
-  static constexpr int BC = (D == 64) ? 128 : 64;   // keys per block
-  static constexpr int NT = NT_;               // row tiles per CTA (TMEM: NT * (BC + BC / 2 + D) <= 512); 2, or 1 for
-                                               // grids that would leave SMs without a CTA (one long sequence, few heads)
+  static constexpr int BM = 128, BC = 128;
   static constexpr int HALO = 16;              // rows staged above the block (pad_q <= 15)
-  static constexpr int QR = NT * BM + HALO;    // rows of Q in shared memory
-  static constexpr int QBOX = QR / 2;          // Q is fetched as two boxes per 16-byte column slab
+  static constexpr int QR = BM + HALO;
   static constexpr int SLABS = D / 64;         // 64-element (128-byte) column slabs per row
-  static constexpr int TILE_BYTES = BC * 128;  // one ring tile: BC keys x 64 elements, 128B-swizzled
-  static constexpr int NSLOT = (D == 64) ? 11 : 19;
-  static constexpr int oQ = 0;
+  static constexpr int VW = D / 2;             // V columns staged by one CTA
+  static constexpr int VT = (BC * VW * 2) / 8192;   // ring tiles of one V half: 1 (d = 64: 128 keys x 32, 64-byte swizzle) or 2 (64 keys x 64)
+  static constexpr int TILE_BYTES = 8192;      // Kt: 64 keys x 64 elements, 128-byte swizzle
+  static constexpr int NS = (D == 64) ? 1 : 2; // S buffers
+  static constexpr int NSLOT = (D == 64) ? 11 : 23;   // d = 64: two CTAs share an SM
+  static constexpr int oQ = 0;                 // [d/64][QR][128 B], 128-byte swizzle
   static constexpr int oRing = ((oQ + QR * D * 2 + 1023) / 1024) * 1024;
-  static constexpr int oBar = oRing + NSLOT * TILE_BYTES;
-  static constexpr int kSmemBytes = oBar + 512 + 1024;   // + alignment slack
-  static constexpr int kTmemCols = 512;
-  static constexpr int colS = 0;               // S[t] at colS + t*BC
-  static constexpr int colP = NT * BC;         // P[t] at colP + t*BC/2
-  static constexpr int colO = NT * BC + NT * BC / 2;   // O[t] at colO + t*D
-  static constexpr int kThreads = (NT * 4 + 1 + NT) * 32;   // softmax warpgroups, TMA warp, one MMA warp per row tile
-  static_assert(NT * (BC + BC / 2 + D) <= kTmemCols, "TMEM budget");
-  static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
-  static_assert(QR <= 512 && QBOX <= 256, "TMA box limit");
+  static constexpr int oMax = oRing + NSLOT * TILE_BYTES;    // row maxima, exchanged between the two column halves: [2][2][128]
+  static constexpr int oBar = oMax + 2 * 2 * BM * 4;
+  static constexpr int kSmemBytes = oBar + 512 + 1024;       // + alignment slack
+  static constexpr int colS = 0, colP = NS * BC, colO = colP + BC / 2;
+  static constexpr int kTmemCols = (D == 64) ? 256 : 512;
+  static constexpr int kEw = 8;                // softmax warps: 4 lane quarters x 2 column halves
+  static constexpr int kThreads = (kEw + 2) * 32;
+  static_assert(colO + D <= kTmemCols, "TMEM budget");
+  static_assert(kSmemBytes <= (D == 64 ? 113 : 227) * 1024, "shared memory budget");
 };
 
 constexpr float kRescaleTau = 8.f;   // log2 units: P may reach 2^8 before O is rescaled
 
-template <int D, int NT_>
-__global__ void __launch_bounds__(TcCfg<D, NT_>::kThreads, 1)
+// CTAs are dispatched in linear block order.  The row blocks of a (batch, head) pair run side by side, longest first, and
+// share its K-tilde and V in L2; the last `X` pairs (a few waves of the GPU) are walked length-major, so that the greedy
+// hardware scheduler ends with the short CTAs.
+FMTA_DEVINL void pair_block_order(int lin, int nqb, int nBH, int& bh, int& r) {
+  const int X = min(nBH, max(1, (256 + nqb / 2) / nqb));
+  const int head = (nBH - X) * nqb;
+  if (lin < head) { bh = lin / nqb; r = lin - bh * nqb; }
+  else { lin -= head; r = lin / X; bh = nBH - X + (lin - r * X); }
+}
+
+template <int D>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TcCfg<D>::kThreads, D == 64 ? 2 : 1)
 fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKt,
-              const __grid_constant__ CUtensorMap tmV, const TcParams p) {
-  using Cfg = TcCfg<D, NT_>;
-  constexpr int BM = Cfg::BM, BC = Cfg::BC, HALO = Cfg::HALO, QR = Cfg::QR, NSLOT = Cfg::NSLOT, NT = Cfg::NT;
-  constexpr int SLABS = Cfg::SLABS;
+                const __grid_constant__ CUtensorMap tmV, const TcParams p) {
+  using Cfg = TcCfg<D>;
+  constexpr int BM = Cfg::BM, BC = Cfg::BC, HALO = Cfg::HALO, QR = Cfg::QR, NSLOT = Cfg::NSLOT, NS = Cfg::NS;
+  constexpr int SLABS = Cfg::SLABS, EW = Cfg::kEw;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* sQ = smem + Cfg::oQ;
   unsigned char* sRing = smem + Cfg::oRing;
+  float* sMax = reinterpret_cast<float*>(smem + Cfg::oMax);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::oBar);
-  uint64_t* full = bars;                 // [NSLOT]  TMA -> MMA
+  // (rank 0): only the copy in rank 0's shared memory is used
+  uint64_t* full = bars;                 // [NSLOT]  TMA of both CTAs -> MMA (rank 0)
   uint64_t* empty = bars + NSLOT;        // [NSLOT]  MMA -> TMA
-  uint64_t* q_full = bars + 2 * NSLOT;
-  uint64_t* s_full = q_full + 1;         // [NT]  S[t] ready (one commit per key block)
-  uint64_t* s_free = s_full + 2;         // [NT]  S[t] loaded into registers (128 arrivals)
-  uint64_t* p_full = s_free + 2;         // [NT]  P[t] written to tensor memory (128 arrivals)
-  uint64_t* o_full = p_full + 2;         // [NT]  PV(t, kb) completed
-  uint64_t* never_bar = o_full + 2;      // nothing arrives here (expiry self-test)
-  uint64_t* mma_drain = never_bar + 1;   // abort path: every issuer's MMAs have completed (NT arrivals)
+  uint64_t* q_full = bars + 2 * NSLOT;   // (rank 0)
+  uint64_t* s_full = q_full + 1;         // [NS]  S ready
+  uint64_t* s_free = s_full + NS;        // [NS]  S loaded into registers by all warps of both CTAs (rank 0)
+  uint64_t* p_full = s_free + NS;        // P written to tensor memory (rank 0)
+  uint64_t* o_full = p_full + 1;         // PV(kb) completed
+  uint64_t* xch = o_full + 1;            // [4]  both warps of 32 rows have left their maxima in shared memory
+  uint64_t* never_bar = xch + 4;         // nothing arrives here (expiry self-test)
+  uint64_t* mma_drain = never_bar + 1;   // abort path: the issued MMAs have completed
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(mma_drain + 1);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
   volatile int* s_issued = s_abort + 1;
-  volatile int* s_consumed = s_abort + 2;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = tc::cluster_rank();
   const int N = p.N, cq = p.cq, pq = cq - 1, pk = (p.ck - 1) / 2;
   const int band = pq + pk;              // entries with query - key < band belong to the band kernel
-  const int nQB = (N + NT * BM - 1) / (NT * BM);
-  // CTAs are dispatched in linear block order; walk it length-major (all (batch, head) pairs of the
-  // longest row block first) so that the greedy hardware scheduler ends with the short CTAs
-  const int lin = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-  const int nBH = gridDim.y * gridDim.z;
-  const int qb = p.qb_hi - 1 - lin / nBH;
-  const int h = (lin % nBH) % (int)gridDim.y, b = (lin % nBH) / (int)gridDim.y;
-  const int bh = b * p.H + h;
-  const int i0 = qb * NT * BM;
-  const int nKB = (N + BC - 1) / BC;
-  int nkb_t[2] = {0, 0};
-#pragma unroll
-  for (int t = 0; t < NT; ++t) {
-    const int r0 = i0 + t * BM;
-    if (r0 >= N) nkb_t[t] = 0;
-    else if (p.causal) {
-      // key blocks that hold at least one key j <= (last row) - band
-      const int last = min(N - 1, r0 + BM - 1) - band;
-      nkb_t[t] = last >= 0 ? min(nKB, last / BC + 1) : 0;
-    } else nkb_t[t] = nKB;
+  int bh, qb;
+  pair_block_order(blockIdx.x >> 1, p.qb_hi - p.qb_lo, p.B * p.H, bh, qb);
+  qb = p.qb_hi - 1 - qb;
+  const int P0 = qb * 2 * BM, i0 = P0 + (int)rank * BM;     // first row of the pair, of this CTA
+  int nkb = (N + BC - 1) / BC;
+  if (p.causal) {                        // key blocks that hold at least one key j <= (last row) - band
+    const int last = min(N - 1, P0 + 2 * BM - 1) - band;
+    nkb = last >= 0 ? min(nkb, last / BC + 1) : 0;
   }
-  const int nkb = max(nkb_t[0], nkb_t[1]);
 
   if (tid == 0) {
-    for (int i = 0; i < NSLOT; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], NT); }   // every MMA warp releases a slot
+    for (int i = 0; i < NSLOT; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 1); }
     tc::mbar_init(q_full, 1);
-    tc::mbar_init(never_bar, 1); tc::mbar_init(mma_drain, NT);
-    for (int i = 0; i < 2; ++i) { tc::mbar_init(&s_full[i], 1); tc::mbar_init(&s_free[i], BM); tc::mbar_init(&p_full[i], BM); tc::mbar_init(&o_full[i], 1); }
-    *s_abort = 0; *s_issued = 0; *s_consumed = 0;
+    for (int i = 0; i < NS; ++i) { tc::mbar_init(&s_full[i], 1); tc::mbar_init(&s_free[i], 2 * EW); }
+    tc::mbar_init(p_full, 2 * EW); tc::mbar_init(o_full, 1);
+    for (int i = 0; i < 4; ++i) tc::mbar_init(&xch[i], 2);
+    tc::mbar_init(never_bar, 1); tc::mbar_init(mma_drain, 1);
+    *s_abort = 0; *s_issued = 0;
     tc::mbar_fence_init();
   }
-  if (warp == NT * 4 + 1) {   // the first MMA warp owns the tensor-memory allocation
-    tc::tmem_alloc(s_tmem, Cfg::kTmemCols);
-    tc::tmem_relinquish();
-  }
+  if (warp == EW + 1) tc::tmem_alloc_pair(s_tmem, Cfg::kTmemCols);
   tc::tc_fence_before();
-  __syncthreads();
+  tc::cluster_sync_all();
   pdl_wait();      // nothing before this line touches global memory that a kernel of this library writes or reads back
   pdl_trigger();   // after the wait: the band kernel behind this one reads Q, K, V before it waits for this kernel
   tc::tc_fence_after();
   const uint32_t tmem = *s_tmem;
 
-  if (warp == NT * 4) {
-    // ===================== TMA producer =====================
+  if (warp == EW) {
+    // ===================== TMA producer: this CTA's Q, its half of every Kt and V tile =====================
     if (lane == 0 && nkb > 0) {
       tc::tma_prefetch_desc(&tmQ); tc::tma_prefetch_desc(&tmKt); tc::tma_prefetch_desc(&tmV);
-      tc::mbar_expect_tx(q_full, QR * D * 2);
-      for (int kc = 0; kc < D / 8; ++kc) {   // 16-byte-wide column slabs -> [kc][row][8 elements]
-        tc::tma_load_3d(sQ + kc * (QR * 16), &tmQ, q_full, kc * 8, i0 - HALO, bh);
-        tc::tma_load_3d(sQ + kc * (QR * 16) + Cfg::QBOX * 16, &tmQ, q_full, kc * 8, i0 - HALO + Cfg::QBOX, bh);
-      }
-      int id = 0;
+      const uint32_t full0 = tc::cluster_addr(full, 0);
+      if (rank == 0) tc::mbar_expect_tx(q_full, 2 * QR * D * 2);
+      const uint32_t qf = tc::cluster_addr(q_full, 0);
+      for (int sl = 0; sl < SLABS; ++sl) tc::tma_load_3d_pair(sQ + sl * (QR * 128), &tmQ, qf, sl * 64, i0 - HALO, bh);
+      int slot = 0, ph = 1, id = 0;
       bool ok = true;
       auto put = [&](const CUtensorMap* map, int x, int y, int z) {
-        const int slot = id % NSLOT, ph = (id / NSLOT) & 1;
-        if (!tc::mbar_wait(&empty[slot], ph ^ 1, s_abort)) { ok = false; return; }
-        tc::mbar_expect_tx(&full[slot], Cfg::TILE_BYTES);
-        tc::tma_load_3d(sRing + slot * Cfg::TILE_BYTES, map, &full[slot], x, y, z);
-        ++id;
-        *s_issued = id;
+        if (!tc::mbar_wait(&empty[slot], ph, s_abort)) { ok = false; return; }
+        if (rank == 0) tc::mbar_expect_tx(&full[slot], 2 * Cfg::TILE_BYTES);
+        tc::tma_load_3d_pair(sRing + slot * Cfg::TILE_BYTES, map, full0 + slot * 8, x, y, z);
+        if (++slot == NSLOT) { slot = 0; ph ^= 1; }
+        *s_issued = ++id;
+      };
+      auto put_K = [&](int kb) {
+        for (int a = 0; a < cq && ok; ++a)
+          for (int sl = 0; sl < SLABS && ok; ++sl) put(&tmKt, sl * 64, kb * BC + (int)rank * (BC / 2), bh * cq + a);
       };
       // same order as the MMA warp consumes: S(0); then S(kb+1), V(kb)
-      for (int a = 0; a < cq && ok; ++a)
-        for (int sl = 0; sl < SLABS && ok; ++sl) put(&tmKt, sl * 64, 0, bh * cq + a);
+      put_K(0);
       for (int kb = 0; kb < nkb && ok; ++kb) {
-        if (kb + 1 < nkb)
-          for (int a = 0; a < cq && ok; ++a)
-            for (int sl = 0; sl < SLABS && ok; ++sl) put(&tmKt, sl * 64, (kb + 1) * BC, bh * cq + a);
-        for (int sl = 0; sl < SLABS && ok; ++sl) put(&tmV, sl * 64, kb * BC, bh);
+        if (kb + 1 < nkb) put_K(kb + 1);
+        for (int v = 0; v < Cfg::VT && ok; ++v) put(&tmV, (int)rank * Cfg::VW, kb * BC + v * 64, bh);
+      }
+      // the last arrivals on this CTA's `empty` barriers have landed before it leaves
+      for (int i = 0; i < NSLOT && i < id && ok; ++i) {
+        if (--slot < 0) { slot = NSLOT - 1; ph ^= 1; }
+        ok = tc::mbar_wait(&empty[slot], ph ^ 1, s_abort);
       }
     }
-  } else if (warp > NT * 4) {
-    // ===================== MMA issuers: one warp (one elected thread) per row tile =====================
-    // Both walk the same tile stream; a ring slot is released when every issuer has committed
-    // its MMAs on it.  Two issuers keep the tensor pipe fed while one of them sits in a barrier
-    // wait or a commit.
-    const int t = warp - (NT * 4 + 1);
-    if (nkb > 0) {   // all lanes run the loop; one elected lane issues (see tc::elect_one)
-      constexpr uint32_t idescS = tc::make_idesc(BM, BC, 0, 0);
-      constexpr uint32_t idescPV = tc::make_idesc(BM, 64, 0, 1);
+  } else if (warp == EW + 1) {
+    // ===================== MMA issuer (rank 0) =====================
+    if (nkb > 0 && rank == 0) {   // all lanes run the loop; one elected lane issues (see tc::elect_one)
+      constexpr uint32_t idescS = tc::make_idesc(2 * BM, BC, 0, 0);
+      constexpr uint32_t idescPV = tc::make_idesc(2 * BM, D, 0, 1);
       // descriptors split into a constant high word and a low word that carries the start address
-      const uint64_t dQ0 = tc::make_sdesc(smem_u32(sQ) + (t * BM + HALO - pq) * 16, QR * 16, 128, tc::kLayoutNone);
+      // row shift: the same tile with the start address moved by 128 bytes per row (the tensor core applies the
+      // swizzle to the absolute shared-memory address, as TMA did)
+      const uint64_t dQ0 = tc::make_sdesc(smem_u32(sQ) + (HALO - pq) * 128, 16, 1024, tc::kLayoutSW128);
       const uint64_t dK0 = tc::make_sdesc(smem_u32(sRing), 16, 1024, tc::kLayoutSW128);
-      const uint32_t aS_hi = (uint32_t)(dQ0 >> 32), aS_lo = (uint32_t)dQ0;
-      const uint32_t b_hi = (uint32_t)(dK0 >> 32), b_lo0 = (uint32_t)dK0;
-      const uint32_t dS = tmem + Cfg::colS + t * BC;
-      const uint32_t aP = tmem + Cfg::colP + t * (BC / 2);      // bf16 pairs: 8 columns per 16 keys
-      const int my_nkb = nkb_t[t];
-      int id = 0;
-      bool ok = tc::mbar_wait_warp(q_full, 0, s_abort);
+      const uint64_t dV0 = D == 64 ? tc::make_sdesc(smem_u32(sRing), 16, 512, tc::kLayoutSW64) : dK0;
+      const uint32_t a_hi = (uint32_t)(dQ0 >> 32), a_lo0 = (uint32_t)dQ0;
+      const uint32_t k_hi = (uint32_t)(dK0 >> 32), v_hi = (uint32_t)(dV0 >> 32), b_lo0 = (uint32_t)dK0;
+      int slot = 0, ph = 0;
+      bool ok = tc::mbar_wait_cluster_warp(q_full, 0, s_abort);
       auto issue_S = [&](int kb) {
-        const bool active = kb < my_nkb;
-        // S[t] is single-buffered: wait until the softmax threads have taken block kb-1 out of it
-        if (active && kb > 0) {
-          ok = tc::mbar_wait_warp(&s_free[t], (kb - 1) & 1, s_abort);
+        const int buf = kb % NS;
+        const uint32_t dS = tmem + Cfg::colS + buf * BC;
+        if (kb >= NS) {      // the softmax threads have taken block kb - NS out of this buffer
+          ok = tc::mbar_wait_cluster_warp(&s_free[buf], (kb / NS - 1) & 1, s_abort);
+          if (!ok) return;
           tc::tc_fence_after();
         }
-        for (int a = 0; a < cq && ok; ++a) {
+        uint32_t a_lo = a_lo0;
+        for (int a = 0; a < cq; ++a, a_lo += 128 >> 4) {
 #pragma unroll
           for (int sl = 0; sl < SLABS; ++sl) {
-            const int slot = id % NSLOT, ph = (id / NSLOT) & 1;
-            if (!tc::mbar_wait_warp(&full[slot], ph, s_abort)) { ok = false; return; }
-            if (active) {
-              tc::tc_fence_after();
-              const uint32_t b_lo = b_lo0 + (uint32_t)(slot * (Cfg::TILE_BYTES >> 4));
-              const uint32_t a_lo = aS_lo + (uint32_t)(a + sl * 8 * QR);   // row shift = +16 B per row
-              if (a == 0 && sl == 0) tc::mma_ss2e<0>(dS, a_lo, aS_hi, b_lo, b_hi, idescS);
-              else tc::mma_ss2e<1>(dS, a_lo, aS_hi, b_lo, b_hi, idescS);
-#pragma unroll
-              for (int k = 1; k < 4; ++k)
-                tc::mma_ss2e<1>(dS, a_lo + (uint32_t)(2 * k * QR), aS_hi, b_lo + (uint32_t)(k * 2), b_hi, idescS);
-            }
-            tc::mma_commit_e(&empty[slot]);
-            ++id;
-          }
-        }
-        if (ok && active) tc::mma_commit_e(&s_full[t]);
-      };
-      auto issue_PV = [&](int kb) {
-        const bool active = kb < my_nkb;
-#pragma unroll
-        for (int sl = 0; sl < SLABS; ++sl) {
-          const int slot = id % NSLOT, ph = (id / NSLOT) & 1;
-          if (!tc::mbar_wait_warp(&full[slot], ph, s_abort)) { ok = false; return; }
-          if (active) {
-            if (sl == 0 && !tc::mbar_wait_warp(&p_full[t], kb & 1, s_abort)) { ok = false; return; }
+            ok = tc::mbar_wait_cluster_warp(&full[slot], ph, s_abort);
+            if (!ok) return;
             tc::tc_fence_after();
             const uint32_t b_lo = b_lo0 + (uint32_t)(slot * (Cfg::TILE_BYTES >> 4));
-            const uint32_t dO = tmem + Cfg::colO + t * D + sl * 64;
-            if (kb == 0) tc::mma_ts2e<0>(dO, aP, b_lo, b_hi, idescPV);
-            else tc::mma_ts2e<1>(dO, aP, b_lo, b_hi, idescPV);
-#pragma unroll
-            for (int k = 1; k < BC / 16; ++k)
-              tc::mma_ts2e<1>(dO, aP + 8 * k, b_lo + (uint32_t)(k * (2048 / 16)), b_hi, idescPV);
-            if (sl == SLABS - 1) tc::mma_commit_e(&o_full[t]);
+            tc::mma4_ss<2>(dS, a_lo + (uint32_t)(sl * (QR * 128 >> 4)), a_hi, 2, b_lo, k_hi, 2, idescS, (a | sl) != 0);
+            tc::mma_commit_pair(&empty[slot]);
+            if (++slot == NSLOT) { slot = 0; ph ^= 1; }
           }
-          tc::mma_commit_e(&empty[slot]);
-          ++id;
         }
+        tc::mma_commit_pair(&s_full[buf]);
+      };
+      auto issue_PV = [&](int kb) {
+        ok = tc::mbar_wait_cluster_warp(p_full, kb & 1, s_abort);
+        if (!ok) return;
+#pragma unroll
+        for (int v = 0; v < Cfg::VT; ++v) {
+          ok = tc::mbar_wait_cluster_warp(&full[slot], ph, s_abort);
+          if (!ok) return;
+          tc::tc_fence_after();
+          const uint32_t b_lo = b_lo0 + (uint32_t)(slot * (Cfg::TILE_BYTES >> 4));
+#pragma unroll
+          for (int k = 0; k < BC / 16 / Cfg::VT; k += 4)       // 16 keys: 16 rows of V, 8 columns of P
+            tc::mma4_ts<2>(tmem + Cfg::colO, tmem + Cfg::colP + 8 * (v * 4 + k), 8, b_lo + (uint32_t)(k * (16 * Cfg::VW * 2 / 16)), v_hi,
+                           16 * Cfg::VW * 2 / 16, idescPV, (kb | v | k) != 0);
+          tc::mma_commit_pair(&empty[slot]);
+          if (++slot == NSLOT) { slot = 0; ph ^= 1; }
+        }
+        tc::mma_commit_pair(o_full);
       };
       if (ok) issue_S(0);
       for (int kb = 0; kb < nkb && ok; ++kb) {
         if (kb + 1 < nkb) issue_S(kb + 1);
         if (ok) issue_PV(kb);
       }
-      if (t == 0) *s_consumed = id;
     }
   } else {
-    // ===================== softmax warpgroups: one query row per thread =====================
-    const int t = warp >> 2;                            // row tile of this warpgroup
-    const int m = tid & (BM - 1);                       // row within the tile = TMEM lane
-    const int gi = i0 + t * BM + m;                     // query index
+    // ===================== softmax warps: one query row and 64 of the 128 keys per thread =====================
+    const int c = warp >> 2;                            // column half
+    const int m = (warp & 3) * 32 + lane;               // row within the tile = TMEM lane
+    const int gi = i0 + m;                              // query index
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t tS = tmem + Cfg::colS + t * BC + lane_base;
-    const uint32_t tP = tmem + Cfg::colP + t * (BC / 2) + lane_base;
-    const uint32_t tO = tmem + Cfg::colO + t * D + lane_base;
-    const int my_nkb = nkb_t[t];
+    const uint32_t tS = tmem + Cfg::colS + c * (BC / 2) + lane_base;
+    const uint32_t tP = tmem + Cfg::colP + c * (BC / 4) + lane_base;
+    const uint32_t tO = tmem + Cfg::colO + c * (D / 2) + lane_base;
+    const uint32_t r_sfree = tc::cluster_addr(s_free, 0), r_pfull = tc::cluster_addr(p_full, 0);
+    const int jlim = p.causal ? min(N - 1, gi - band) : N - 1;   // last key this row may see here
     float m_run = -INFINITY, l_run = 0.f;               // log2 units (Kt carries scale * log2(e))
     float m_true = -INFINITY;                           // true row max (m_run lags it by up to tau)
     bool ok = true;
-    for (int kb = 0; kb < my_nkb && ok; ++kb) {
+    for (int kb = 0; kb < nkb && ok; ++kb) {
+      const int buf = kb % NS;
       ok = __all_sync(0xffffffffu, (p.selftest_expire && kb == 0)
                                        ? tc::mbar_wait(never_bar, 0, s_abort, tc::kSelfTestSpinLimit)
-                                       : tc::mbar_wait(&s_full[t], kb & 1, s_abort));
+                                       : tc::mbar_wait(&s_full[buf], (kb / NS) & 1, s_abort));
       if (!ok) break;   // warp-uniform: the TMEM accesses below are warp-collective
       tc::tc_fence_after();
-      float s[BC];
-#pragma unroll
-      for (int c = 0; c < BC / 32; ++c) tc::tmem_ld32_nowait(tS + 32 * c, reinterpret_cast<float(&)[32]>(s[32 * c]));
+      float s[64];
+      tc::tmem_ld32_nowait(tS + buf * BC, reinterpret_cast<float(&)[32]>(s[0]));
+      tc::tmem_ld32_nowait(tS + buf * BC + 32, reinterpret_cast<float(&)[32]>(s[32]));
       tc::tmem_wait_ld();
-      // S[t] is in registers: let the MMA warp overwrite it with the next key block
+      // S is in registers: the MMA warp may overwrite it
       tc::tc_fence_before();
-      tc::mbar_arrive(&s_free[t]);
-      const int j0 = kb * BC;
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive_cluster(r_sfree + buf * 8);
+      const int j0 = kb * BC + c * 64;
       // mask: keys past N, and (causal) entries on or above the band, which the band kernel owns
-      const int jlim = p.causal ? min(N - 1, gi - band) : N - 1;   // last key this row may see here
-      if (j0 + BC - 1 > jlim) {
+      if (j0 + 63 > jlim) {
 #pragma unroll
-        for (int i = 0; i < BC; ++i) if (j0 + i > jlim) s[i] = -INFINITY;
+        for (int i = 0; i < 64; ++i) if (j0 + i > jlim) s[i] = -INFINITY;
       }
       float mx0 = fmaxf(s[0], s[1]), mx1 = fmaxf(s[2], s[3]), mx2 = fmaxf(s[4], s[5]), mx3 = fmaxf(s[6], s[7]);
 #pragma unroll
-      for (int i = 8; i < BC; i += 8) {
+      for (int i = 8; i < 64; i += 8) {
         mx0 = fmaxf(mx0, fmaxf(s[i], s[i + 1])); mx1 = fmaxf(mx1, fmaxf(s[i + 2], s[i + 3]));
         mx2 = fmaxf(mx2, fmaxf(s[i + 4], s[i + 5])); mx3 = fmaxf(mx3, fmaxf(s[i + 6], s[i + 7]));
       }
-      const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
+      float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
+      // both halves of a row use one reference: exchange the maxima (double-buffered: a buffer is rewritten two blocks
+      // later, behind the barrier of the block between)
+      float* mrow = sMax + (kb & 1) * (2 * BM) + m;
+      mrow[c * BM] = mx;
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&xch[warp & 3]);
+      ok = __all_sync(0xffffffffu, tc::mbar_wait(&xch[warp & 3], kb & 1, s_abort));
+      if (!ok) break;
+      mx = fmaxf(mx, mrow[(c ^ 1) * BM]);
       m_true = fmaxf(m_true, mx);
       // lazy rescale: keep the reference max until a block exceeds it by more than tau
       float alpha = 1.f;
@@ -417,9 +412,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       }
       const float mref = (m_run == -INFINITY) ? 0.f : m_run;
       float sum0 = 0.f, sum1 = 0.f;
-      uint32_t pk32[BC / 2];
+      uint32_t pk32[32];
 #pragma unroll
-      for (int i = 0; i < BC; i += 4) {
+      for (int i = 0; i < 64; i += 4) {
         const float p0 = exp2f(s[i] - mref), p1 = exp2f(s[i + 1] - mref);
         const float p2 = exp2f(s[i + 2] - mref), p3 = exp2f(s[i + 3] - mref);
         sum0 += p0 + p1; sum1 += p2 + p3;
@@ -427,50 +422,58 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       }
       l_run = l_run * alpha + (sum0 + sum1);
       if (kb > 0) {
-        // PV(kb-1) complete: P[t] may be overwritten and O touched.  Waited for on every block
+        // PV(kb-1) complete: P may be overwritten and O touched.  Waited for on every block
         // (not only when O is rescaled) so that the parity wait never aliases an older phase.
-        ok = __all_sync(0xffffffffu, tc::mbar_wait(&o_full[t], (kb - 1) & 1, s_abort));
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(o_full, (kb - 1) & 1, s_abort));
         if (!ok) break;
         tc::tc_fence_after();
       }
       if (__any_sync(0xffffffffu, need)) {   // O *= alpha (need is false on the first block)
 #pragma unroll
-        for (int c = 0; c < D / 32; ++c) {
+        for (int q = 0; q < D / 64; ++q) {
           float o[32];
-          tc::tmem_ld32(tO + c * 32, o);
+          tc::tmem_ld32(tO + q * 32, o);
 #pragma unroll
           for (int i = 0; i < 32; ++i) o[i] *= alpha;
-          tc::tmem_st32(tO + c * 32, o);
+          tc::tmem_st32(tO + q * 32, o);
         }
       }
-#pragma unroll
-      for (int c = 0; c < BC / 64; ++c) tc::tmem_st32u(tP + 32 * c, reinterpret_cast<const uint32_t(&)[32]>(pk32[32 * c]));
+      tc::tmem_st32u(tP, pk32);
       tc::tmem_wait_st();
       tc::tc_fence_before();
-      tc::mbar_arrive(&p_full[t]);
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive_cluster(r_pfull);
     }
     // ---- epilogue: un-normalised partial row ----
-    if (my_nkb > 0 && ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(&o_full[t], (my_nkb - 1) & 1, s_abort));
+    if (nkb > 0 && ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(o_full, (nkb - 1) & 1, s_abort));
     tc::tc_fence_after();
-    const bool have = (my_nkb > 0) && ok;               // warp-uniform
+    if (ok) {                                           // row sum: the two halves together
+      float* lrow = sMax + (nkb & 1) * (2 * BM) + m;
+      lrow[c * BM] = l_run;
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&xch[warp & 3]);
+      ok = __all_sync(0xffffffffu, tc::mbar_wait(&xch[warp & 3], nkb & 1, s_abort));
+      if (ok) l_run += lrow[(c ^ 1) * BM];
+    }
+    const bool have = (nkb > 0) && ok;                  // warp-uniform
     // re-reference the partial to the true row max (what the reference reports as M)
     const float fix = (m_true == -INFINITY) ? 0.f : exp2f(m_run - m_true);
-    float* orow = p.Opart + ((size_t)bh * N + (gi < N ? gi : 0)) * D;
+    float* orow = p.Opart + ((size_t)bh * N + (gi < N ? gi : 0)) * D + c * (D / 2);
 #pragma unroll
-    for (int c = 0; c < D / 32; ++c) {
+    for (int q = 0; q < D / 64; ++q) {
       float o[32];
       if (have) {
-        tc::tmem_ld32(tO + c * 32, o);                  // warp-collective: every lane takes part
+        tc::tmem_ld32(tO + q * 32, o);                  // warp-collective: every lane takes part
       } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i) o[i] = 0.f;
       }
       if (gi < N) {
 #pragma unroll
-        for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(orow + c * 32 + i) = make_float4(o[i] * fix, o[i + 1] * fix, o[i + 2] * fix, o[i + 3] * fix);
+        for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(orow + q * 32 + i) = make_float4(o[i] * fix, o[i + 1] * fix, o[i + 2] * fix, o[i + 3] * fix);
       }
     }
-    if (gi < N) {
+    if (gi < N && c == 0) {
       const bool any = have && (m_run != -INFINITY);
       p.Mpart[(size_t)bh * N + gi] = any ? m_true * 0.6931471805599453f : -INFINITY;
       p.Lpart[(size_t)bh * N + gi] = any ? l_run * fix : 0.f;
@@ -479,24 +482,27 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   __syncwarp();
 
   // ===================== teardown =====================
+  if (tid == 0 && *s_abort) tc::st_cluster_u32(tc::cluster_addr((const void*)s_abort, rank ^ 1), 1);
   tc::tc_fence_before();
-  __syncthreads();
-  if (*s_abort) {
+  tc::cluster_sync_all();
+  if (*s_abort) {        // of either CTA
     if (tid == 0) atomicExch(p.status, 1);
-    // nothing of this CTA may still be in flight when its shared and tensor memory are given up: every
-    // issuer commits behind its last MMA, one thread waits (bounded) for those commits and for the
-    // copies that were issued but never consumed
-    if (warp > NT * 4) tc::mma_commit_e(mma_drain);
-    if (tid == NT * 4 * 32) {
+    // nothing of the pair may still be in flight when its shared and tensor memory are given up: the issuer commits
+    // behind its last MMA, one thread waits (bounded) for that commit and for the copies issued last into each slot
+    if (rank == 0 && warp == EW + 1) tc::mma_commit_pair(mma_drain);
+    if (rank == 0 && tid == EW * 32 && nkb > 0) {
       volatile int never = 0;
-      for (int id = *s_consumed; id < *s_issued; ++id) tc::mbar_wait(&full[id % NSLOT], (id / NSLOT) & 1, &never);
-      tc::mbar_wait(mma_drain, 0, &never);
+      constexpr uint32_t kDrain = 1u << 14;
+      tc::mbar_wait(q_full, 0, &never, kDrain);
+      const int issued = *s_issued;
+      for (int id = max(0, issued - NSLOT); id < issued; ++id) tc::mbar_wait(&full[id % NSLOT], (id / NSLOT) & 1, &never, kDrain);
     }
-    __syncthreads();
+    if (tid == EW * 32) { volatile int never = 0; tc::mbar_wait(mma_drain, 0, &never); }
+    tc::cluster_sync_all();
   }
-  if (warp == NT * 4 + 1) {
+  if (warp == EW + 1) {
     tc::tc_fence_after();
-    tc::tmem_dealloc(tmem, Cfg::kTmemCols);
+    tc::tmem_dealloc_pair(tmem, Cfg::kTmemCols);
   }
 }
 
@@ -533,7 +539,7 @@ bool make_tensor_map_bf16(CUtensorMap* map, const void* base, int D, int rows, s
   cuuint32_t box[3] = {(cuuint32_t)box_x, (cuuint32_t)box_rows, (cuuint32_t)box_outer};
   cuuint32_t es[3] = {1, 1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, es,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, sw128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, !sw128 ? CU_TENSOR_MAP_SWIZZLE_NONE : box_x == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -584,36 +590,26 @@ cudaError_t launch_ktilde(const TrainParams& p, __nv_bfloat16* Kt, cudaStream_t 
 
 namespace {
 
-template <int D, int NT_>
-cudaError_t launch_tc_t(const TrainParams& p, bf16* Kt, float* Opart, float* Mpart, float* Lpart, int* status,
-                        cudaStream_t stream) {
-  using Cfg = TcCfg<D, NT_>;
+template <int D>
+cudaError_t launch_tc(const TrainParams& p, bf16* Kt, float* Opart, float* Mpart, float* Lpart, int* status, cudaStream_t stream) {
+  using Cfg = TcCfg<D>;
   const size_t BH = (size_t)p.B * p.H;
   alignas(64) CUtensorMap tmQ, tmKt, tmV;
-  if (!make_tensor_map_bf16(&tmQ, p.Q, D, p.N, BH, 8, Cfg::QBOX, false)) return cudaErrorInvalidValue;
-  if (!make_tensor_map_bf16(&tmKt, Kt, D, p.N, BH * p.cq, 64, Cfg::BC, true)) return cudaErrorInvalidValue;
-  if (!make_tensor_map_bf16(&tmV, p.V, D, p.N, BH, 64, Cfg::BC, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmQ, p.Q, D, p.N, BH, 64, Cfg::QR, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmKt, Kt, D, p.N, BH * p.cq, 64, 64, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmV, p.V, D, p.N, BH, Cfg::VW, D == 64 ? 128 : 64, true)) return cudaErrorInvalidValue;
   TcParams tp;
   tp.Opart = Opart; tp.Mpart = Mpart; tp.Lpart = Lpart; tp.status = status;
-  tp.H = p.H; tp.N = p.N; tp.cq = p.cq; tp.ck = p.ck; tp.causal = p.causal;
+  tp.B = p.B; tp.H = p.H; tp.N = p.N; tp.cq = p.cq; tp.ck = p.ck; tp.causal = p.causal;
   tp.selftest_expire = take_selftest_expire(kKernFwdTc);
-  auto kern = fwd_tc_kernel<D, NT_>;
+  auto kern = fwd_tc_kernel<D>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
-  constexpr int RB = Cfg::NT * Cfg::BM;                           // rows per CTA; a window starts on a multiple of it
-  tp.qb_hi = (win_hi(p) + RB - 1) / RB;
-  dim3 grid(tp.qb_hi - win_lo(p) / RB, p.H, p.B);
-  { ScopedKernelTimer timer_(kKernFwdTc, stream);
-    e = launch_pdl(kern, grid, dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, tmQ, tmKt, tmV, tp); }
-  return e;
-}
-
-int sm_count() {
-  static int n[16] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return 148;
-  if (n[dev] == 0 && cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n[dev] = 148;
-  return n[dev];
+  constexpr int RB = 2 * Cfg::BM;                                 // rows per pair; a window starts on a multiple of it
+  tp.qb_hi = (win_hi(p) + RB - 1) / RB; tp.qb_lo = win_lo(p) / RB;
+  dim3 grid(2 * (tp.qb_hi - tp.qb_lo) * (unsigned)BH);
+  ScopedKernelTimer timer_(kKernFwdTc, stream);
+  return launch_pdl(kern, grid, dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, tmQ, tmKt, tmV, tp);
 }
 
 }  // namespace
@@ -648,12 +644,7 @@ cudaError_t launch_fwd_tc(const TrainParams& p, void* workspace, const float** O
     e = launch_ktilde(p, Kt, stream);
     if (e != cudaSuccess) return e;
   }
-  // Two row tiles per CTA share every key tile they stage; when that leaves SMs without a CTA (fewer CTAs than SMs:
-  // a window of one long sequence with few heads) one tile per CTA doubles the CTAs instead.
-  const long ctas2 = (long)((win_hi(p) - win_lo(p) + 255) / 256) * p.B * p.H;
-  const bool one_tile = ctas2 < sm_count();
-  if (p.d == 64) e = one_tile ? launch_tc_t<64, 1>(p, Kt, Op, Mp, Lp, status, stream) : launch_tc_t<64, 2>(p, Kt, Op, Mp, Lp, status, stream);
-  else e = one_tile ? launch_tc_t<128, 1>(p, Kt, Op, Mp, Lp, status, stream) : launch_tc_t<128, 2>(p, Kt, Op, Mp, Lp, status, stream);
+  e = p.d == 64 ? launch_tc<64>(p, Kt, Op, Mp, Lp, status, stream) : launch_tc<128>(p, Kt, Op, Mp, Lp, status, stream);
   *Opart = Op; *Mpart = Mp; *Lpart = Lp;
   return e;
 }
