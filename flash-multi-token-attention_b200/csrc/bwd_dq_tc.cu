@@ -1,0 +1,401 @@
+// dQ of the stacked-GEMM backward on CTA pairs (the math of bwd_tc.cu; entries off the causal band):
+//     C = sum_a Q^(a) Kt_a^T,  P = exp2(C - LSE*log2e),  dC = P * (dO V^T - D),  dQ[i'] = ln2 * sum_a sum_j dC[i' + pad_q - a, j] Kt_a[j]
+//
+// A pair of CTAs walks blocks of 128 keys for 256 * NT rows of dC (a tile of 128 per CTA and t, one TMEM lane per row).  A
+// tile computes 128 dC rows but owns only the first 128 - pad_q as dQ rows: dQ row i' needs dC rows i'..i'+pad_q, so tiles
+// overlap by pad_q rows (recomputed) and no dQ row is shared.  The row shifts of Q and dC are free: both are staged as
+// 128-byte-swizzled tiles and the tensor core applies the swizzle to the absolute shared-memory address, so a view shifted
+// by s rows starts 128 s bytes further.
+//   S, dP : 256 x 128 x 16 MMAs, each CTA stages half the KEYS of every Kt and V tile;
+//   dQ    : 256 x d x 16 MMAs, each CTA stages half the COLUMNS of every Kt tile (a second copy, fetched just in time
+//           instead of being held from S to dQ).
+// One warp issues everything, in an order that has independent MMAs in every wait for the element-wise warps:
+//   NT = 1: S(kb) dP(kb) | dQ(kb-1) | S(kb+1) ...                     S and dP in columns of their own
+//   NT = 2: S(kb) | dQ(kb-1) first taps | dP(kb) | dQ(kb-1) last taps | S(kb+1) ...     S and dP share 128 columns
+// Every mbarrier wait is bounded; on expiry the status word is set and the pair drains and leaves.  No TMA multicast.
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include "bwd_tc.cuh"
+#include "fmta_tc.cuh"
+#include "launch_util.cuh"
+
+namespace fmta {
+
+template <int D, int NT_>
+struct DqCfg {
+  static constexpr int BM = 128, BC = 128, NT = NT_;
+  static constexpr int HALO = 8;                                // rows of Q staged above a tile (pad_q <= 8)
+  static constexpr int SLABS = D / 64;                          // 64-element (128-byte) column slabs per row
+  static constexpr int Q_SLAB = (BM + HALO) * 128, Q_TILE = SLABS * Q_SLAB;
+  static constexpr int O_SLAB = BM * 128, O_TILE = SLABS * O_SLAB;
+  // dC: 64-key slabs of [136 rows][128 B]; the 8 rows below the tile are read by the shifted views of rows that are not owned
+  static constexpr int C_SLAB = (BM + 8) * 128, C_TILE = 2 * C_SLAB;
+  static constexpr int TILE_BYTES = 8192;                       // ring tile: 64 keys x 64 elements, or 128 keys x 32 (dQ, d = 64)
+  static constexpr int DT = D / 64;                             // ring tiles of one tap's dQ half
+  static constexpr int oQ = 0, oO = oQ + NT * Q_TILE, oC = oO + NT * O_TILE, oRing = oC + NT * C_TILE;
+  static_assert(Q_SLAB % 1024 == 0 && C_SLAB % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
+  static constexpr int NSLOT = (227 * 1024 - 1024 - 512 - oRing) / TILE_BYTES;
+  static constexpr int oBar = oRing + NSLOT * TILE_BYTES;
+  static constexpr int kSmemBytes = oBar + 512 + 1024;
+  static constexpr bool SEP = NT == 1;                          // S and dP in columns of their own
+  static constexpr int colX = 0, colP = SEP ? 128 : 0, TCOLS = (SEP ? 256 : 128) + D, colQ = TCOLS - D;   // per tile
+  static constexpr int kTmemCols = 512;
+  static constexpr int EWT = 8, kEw = NT * EWT;                 // element-wise warps: 4 lane quarters x 2 key halves per tile
+  static constexpr int kThreads = (kEw + 2) * 32;
+  static_assert(NT * TCOLS <= kTmemCols, "TMEM budget");
+  static_assert(NSLOT >= 8 && kSmemBytes <= 227 * 1024, "shared memory budget");
+  static_assert((2 * NSLOT + 1 + 6 * NT + 2) * 8 + 16 <= 512, "barriers");
+};
+
+template <int D, int NT_>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DqCfg<D, NT_>::kThreads, 1)
+bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO, const __grid_constant__ CUtensorMap tmKt,
+                 const __grid_constant__ CUtensorMap tmKd, const __grid_constant__ CUtensorMap tmV, const BwdTcParams p) {
+  using Cfg = DqCfg<D, NT_>;
+  constexpr int BM = Cfg::BM, BC = Cfg::BC, NT = Cfg::NT, HALO = Cfg::HALO, SLABS = Cfg::SLABS, NSLOT = Cfg::NSLOT, EW = Cfg::kEw, EWT = Cfg::EWT;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* sRing = smem + Cfg::oRing;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::oBar);
+  // (rank 0): only the copy in rank 0's shared memory is used
+  uint64_t* full = bars;                 // [NSLOT]  TMA of both CTAs -> MMA (rank 0)
+  uint64_t* empty = bars + NSLOT;        // [NSLOT]  MMA -> TMA
+  uint64_t* q_full = bars + 2 * NSLOT;   // Q and dO staged (rank 0)
+  uint64_t* s_full = q_full + 1;         // [NT] S ready
+  uint64_t* s_free = s_full + NT;        // [NT] S taken into registers (rank 0)
+  uint64_t* p_full = s_free + NT;        // [NT] dP ready
+  uint64_t* p_free = p_full + NT;        // [NT] dP taken into registers (rank 0)
+  uint64_t* dc_full = p_free + NT;       // [NT] dC written to shared memory (rank 0)
+  uint64_t* dq_done = dc_full + NT;      // [NT] dQ MMAs of the block complete (dC buffer reusable)
+  uint64_t* never_bar = dq_done + NT;    // nothing arrives here (expiry self-test)
+  uint64_t* mma_drain = never_bar + 1;   // abort path: the issued MMAs have completed
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(mma_drain + 1);
+  volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
+  volatile int* s_issued = s_abort + 1;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = tc::cluster_rank();
+  const int N = p.N, cq = p.cq, pq = cq - 1, pk = (p.ck - 1) / 2;
+  const int band = pq + pk;
+  const int OWN = p.own, rows_per_pair = OWN * 2 * NT;
+  const int nQB = (p.row_end - p.row_base + rows_per_pair - 1) / rows_per_pair;
+  int bh, qb;
+  tc::pair_block_order(blockIdx.x >> 1, nQB, p.B * p.H, bh, qb);
+  // Row blocks are laid out from the END of the rows: when their number is not a multiple of the block, the partly filled
+  // block is the first one, which sees the fewest keys.  Its rows before row_base are computed (negative rows as zero
+  // rows) and not stored.  Tile t of the pair: rows R0 + 2 t OWN (rank 0), R0 + (2 t + 1) OWN (rank 1).
+  const int R0 = p.row_end - (qb + 1) * rows_per_pair;
+  const int nKB = (N + BC - 1) / BC;
+  int nkb_t[NT];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    const int r1 = R0 + (2 * t + 1) * OWN;               // the later of the two tiles
+    if (r1 + OWN <= p.row_base) nkb_t[t] = 0;
+    else if (p.causal) {
+      const int last = min(N - 1, r1 + BM - 1) - band;
+      nkb_t[t] = last >= 0 ? min(nKB, last / BC + 1) : 0;
+    } else nkb_t[t] = nKB;
+  }
+  const int nkb = nkb_t[NT - 1];                         // tiles of later rows see no fewer keys
+
+  if (tid == 0) {
+    for (int i = 0; i < NSLOT; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 1); }
+    tc::mbar_init(q_full, 1);
+    for (int t = 0; t < NT; ++t) {
+      tc::mbar_init(&s_full[t], 1); tc::mbar_init(&s_free[t], 2 * EWT);
+      tc::mbar_init(&p_full[t], 1); tc::mbar_init(&p_free[t], 2 * EWT);
+      tc::mbar_init(&dc_full[t], 2 * EWT); tc::mbar_init(&dq_done[t], 1);
+    }
+    tc::mbar_init(never_bar, 1); tc::mbar_init(mma_drain, 1);
+    *s_abort = 0; *s_issued = 0;
+    tc::mbar_fence_init();
+  }
+  if (warp == EW + 1) tc::tmem_alloc_pair(s_tmem, Cfg::kTmemCols);
+  tc::tc_fence_before();
+  tc::cluster_sync_all();
+  // Behind the band kernel (p.early) everything but its part of dQ is complete already: the kernel starts under the
+  // band kernel's tail and waits in its epilogue.  Otherwise it waits here.  The dK/dV kernel behind it starts as soon as
+  // every CTA here has triggered and reads what was complete by then (all but this kernel's dQ), hence the order.
+  if (!p.early) pdl_wait();
+  pdl_trigger();
+  tc::tc_fence_after();
+  const uint32_t tmem = *s_tmem;
+  const int h1 = NT == 2 ? cq / 2 : cq;      // taps in the first part of dQ
+
+  if (warp == EW) {
+    // ===================== TMA producer: this CTA's Q and dO, its half of every Kt and V tile =====================
+    if (lane == 0 && nkb > 0) {
+      tc::tma_prefetch_desc(&tmQ); tc::tma_prefetch_desc(&tmdO); tc::tma_prefetch_desc(&tmKt); tc::tma_prefetch_desc(&tmKd); tc::tma_prefetch_desc(&tmV);
+      const uint32_t full0 = tc::cluster_addr(full, 0), qf = tc::cluster_addr(q_full, 0);
+      if (rank == 0) tc::mbar_expect_tx(q_full, 2 * NT * (Cfg::Q_TILE + Cfg::O_TILE));
+      for (int t = 0; t < NT; ++t)
+        for (int sl = 0; sl < SLABS; ++sl) {
+          const int r = R0 + (2 * t + (int)rank) * OWN;
+          tc::tma_load_3d_pair(smem + Cfg::oQ + t * Cfg::Q_TILE + sl * Cfg::Q_SLAB, &tmQ, qf, sl * 64, r - HALO, bh);
+          tc::tma_load_3d_pair(smem + Cfg::oO + t * Cfg::O_TILE + sl * Cfg::O_SLAB, &tmdO, qf, sl * 64, r, bh);
+        }
+      int slot = 0, ph = 1, id = 0;
+      bool ok = true;
+      auto put = [&](const CUtensorMap* map, int x, int y, int z) {
+        if (!tc::mbar_wait(&empty[slot], ph, s_abort)) { ok = false; return; }
+        if (rank == 0) tc::mbar_expect_tx(&full[slot], 2 * Cfg::TILE_BYTES);
+        tc::tma_load_3d_pair(sRing + slot * Cfg::TILE_BYTES, map, full0 + slot * 8, x, y, z);
+        if (++slot == NSLOT) { slot = 0; ph ^= 1; }
+        *s_issued = ++id;
+      };
+      auto put_S = [&](int kb) {
+        for (int a = 0; a < cq && ok; ++a)
+          for (int sl = 0; sl < SLABS && ok; ++sl) put(&tmKt, sl * 64, kb * BC + (int)rank * 64, bh * cq + a);
+      };
+      auto put_V = [&](int kb) {
+        for (int sl = 0; sl < SLABS && ok; ++sl) put(&tmV, sl * 64, kb * BC + (int)rank * 64, bh);
+      };
+      auto put_dQ = [&](int kb, int a0, int a1) {
+        for (int a = a0; a < a1 && ok; ++a)
+          for (int v = 0; v < Cfg::DT && ok; ++v) put(&tmKd, (int)rank * (D / 2), kb * BC + v * 64, bh * cq + a);
+      };
+      for (int kb = 0; kb <= nkb && ok; ++kb) {      // the order of the issuer
+        if (kb < nkb) put_S(kb);
+        if (NT == 1 && kb < nkb) put_V(kb);
+        if (kb > 0) put_dQ(kb - 1, 0, h1);
+        if (NT == 2 && kb < nkb) put_V(kb);
+        if (kb > 0) put_dQ(kb - 1, h1, cq);
+      }
+      // the last arrivals on this CTA's `empty` barriers have landed before it leaves
+      for (int i = 0; i < NSLOT && i < id && ok; ++i) {
+        if (--slot < 0) { slot = NSLOT - 1; ph ^= 1; }
+        ok = tc::mbar_wait(&empty[slot], ph ^ 1, s_abort);
+      }
+    }
+  } else if (warp == EW + 1) {
+    // ===================== MMA issuer (rank 0) =====================
+    if (nkb > 0 && rank == 0) {   // all lanes run the loop; one elected lane issues
+      constexpr uint32_t idescS = tc::make_idesc(2 * BM, BC, 0, 0);    // S, dP: both operands K-major
+      constexpr uint32_t idescQ = tc::make_idesc(2 * BM, D, 0, 1);     // dQ: B (Kt) MN-major
+      const uint64_t d128 = tc::make_sdesc(smem_u32(sRing), 16, 1024, tc::kLayoutSW128);
+      const uint64_t d64 = tc::make_sdesc(smem_u32(sRing), 16, 512, tc::kLayoutSW64);
+      const uint32_t hi = (uint32_t)(d128 >> 32), r_lo = (uint32_t)d128, d_hi = D == 64 ? (uint32_t)(d64 >> 32) : hi;
+      const uint32_t s_lo = r_lo - (uint32_t)(Cfg::oRing >> 4);        // descriptor of shared-memory offset 0
+      const uint32_t q_lo = s_lo + (uint32_t)((Cfg::oQ + (HALO - pq) * 128) >> 4), o_lo = s_lo + (uint32_t)(Cfg::oO >> 4), c_lo = s_lo + (uint32_t)(Cfg::oC >> 4);
+      int slot = 0, ph = 0;
+      bool ok = tc::mbar_wait_cluster_warp(q_full, 0, s_abort);
+      auto take = [&]() -> bool { ok = tc::mbar_wait_cluster_warp(&full[slot], ph, s_abort); tc::tc_fence_after(); return ok; };
+      auto give = [&]() { tc::mma_commit_pair(&empty[slot]); if (++slot == NSLOT) { slot = 0; ph ^= 1; } };
+      auto wait_all = [&](uint64_t* bar, int kb, int n) {              // completion n of bar[t] for every tile that has block kb
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+          if (ok && kb < nkb_t[t]) ok = tc::mbar_wait_cluster_warp(&bar[t], n & 1, s_abort);
+        tc::tc_fence_after();
+      };
+      auto issue_S = [&](int kb) {
+        if (kb > 0) wait_all(Cfg::SEP ? s_free : p_free, kb, kb - 1);  // what block kb-1 left in these columns has been taken
+        for (int a = 0; a < cq && ok; ++a)
+#pragma unroll
+          for (int sl = 0; sl < SLABS; ++sl) {
+            if (!take()) return;
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+              if (kb < nkb_t[t])
+                tc::mma4_ss<2>(tmem + t * Cfg::TCOLS + Cfg::colX, q_lo + (uint32_t)((t * Cfg::Q_TILE + sl * Cfg::Q_SLAB + a * 128) >> 4), hi, 2,
+                               r_lo + (uint32_t)(slot * (Cfg::TILE_BYTES >> 4)), hi, 2, idescS, (a | sl) != 0);
+            give();
+          }
+#pragma unroll
+        for (int t = 0; t < NT; ++t) if (ok && kb < nkb_t[t]) tc::mma_commit_pair(&s_full[t]);
+      };
+      auto issue_dP = [&](int kb) {
+        if (!Cfg::SEP) wait_all(s_free, kb, kb);                       // S of this block has been taken
+        else if (kb > 0) wait_all(p_free, kb, kb - 1);
+#pragma unroll
+        for (int sl = 0; sl < SLABS; ++sl) {
+          if (!ok || !take()) return;
+#pragma unroll
+          for (int t = 0; t < NT; ++t)
+            if (kb < nkb_t[t])
+              tc::mma4_ss<2>(tmem + t * Cfg::TCOLS + Cfg::colP, o_lo + (uint32_t)((t * Cfg::O_TILE + sl * Cfg::O_SLAB) >> 4), hi, 2,
+                             r_lo + (uint32_t)(slot * (Cfg::TILE_BYTES >> 4)), hi, 2, idescS, sl != 0);
+          give();
+        }
+#pragma unroll
+        for (int t = 0; t < NT; ++t) if (kb < nkb_t[t]) tc::mma_commit_pair(&p_full[t]);
+      };
+      auto issue_dQ = [&](int kb, int a0, int a1) {
+        if (a0 == 0) wait_all(dc_full, kb, kb);
+        for (int a = a0; a < a1 && ok; ++a)
+#pragma unroll
+          for (int v = 0; v < Cfg::DT; ++v) {
+            if (!take()) return;
+            const uint32_t b_lo = r_lo + (uint32_t)(slot * (Cfg::TILE_BYTES >> 4));
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+              if (kb < nkb_t[t]) {                                     // dC rows i' + pad_q - a
+                const uint32_t a_lo = c_lo + (uint32_t)((t * Cfg::C_TILE + (pq - a) * 128) >> 4), dst = tmem + t * Cfg::TCOLS + Cfg::colQ;
+                if constexpr (D == 64) {                               // 128 keys x 32 columns, 64-byte swizzle
+                  tc::mma4_ss<2>(dst, a_lo, hi, 2, b_lo, d_hi, 64, idescQ, (kb | a) != 0);
+                  tc::mma4_ss<2>(dst, a_lo + (uint32_t)(Cfg::C_SLAB >> 4), hi, 2, b_lo + 256, d_hi, 64, idescQ, 1);
+                } else {
+                  tc::mma4_ss<2>(dst, a_lo + (uint32_t)(v * (Cfg::C_SLAB >> 4)), hi, 2, b_lo, d_hi, 128, idescQ, (kb | a | v) != 0);
+                }
+              }
+            give();
+          }
+        if (ok && a1 == cq) {
+#pragma unroll
+          for (int t = 0; t < NT; ++t) if (kb < nkb_t[t]) tc::mma_commit_pair(&dq_done[t]);
+        }
+      };
+      for (int kb = 0; kb <= nkb && ok; ++kb) {
+        if (kb < nkb) issue_S(kb);
+        if (NT == 1 && ok && kb < nkb) issue_dP(kb);
+        if (ok && kb > 0) issue_dQ(kb - 1, 0, h1);
+        if (NT == 2 && ok && kb < nkb) issue_dP(kb);
+        if (NT == 2 && ok && kb > 0) issue_dQ(kb - 1, h1, cq);
+      }
+    }
+  } else {
+    // ===================== element-wise warps: one dC row and 64 of the 128 keys per thread =====================
+    const int t = warp / EWT, c = (warp >> 2) & 1;
+    const int m = (warp & 3) * 32 + lane;               // row within the tile = TMEM lane
+    const int gi = R0 + (2 * t + (int)rank) * OWN + m;  // query index of this dC row
+    const uint32_t tT = tmem + t * Cfg::TCOLS + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t tS = tT + Cfg::colX + c * 64, tP = tT + Cfg::colP + c * 64, tQ = tT + Cfg::colQ + c * (D / 2);
+    const uint32_t r_sfree = tc::cluster_addr(&s_free[t], 0), r_pfree = tc::cluster_addr(&p_free[t], 0), r_dc = tc::cluster_addr(&dc_full[t], 0);
+    const int my_nkb = nkb_t[t];
+    const bool row_ok = gi >= 0 && gi < N;
+    const float lse2 = row_ok ? p.LSE[(size_t)bh * N + gi] * kLog2e : 0.f;
+    const float dvec = row_ok ? p.Dvec[(size_t)bh * N + gi] : 0.f;
+    const int jlim = row_ok ? (p.causal ? min(N - 1, gi - band) : N - 1) : -1;   // last key owned here
+    unsigned char* cbuf = smem + Cfg::oC + t * Cfg::C_TILE + c * Cfg::C_SLAB + m * 128;   // 16-byte chunk k of the row at chunk k ^ (row & 7)
+    bool ok = true;
+    for (int kb = 0; kb < my_nkb && ok; ++kb) {
+      ok = __all_sync(0xffffffffu, (p.selftest_expire && kb == 0)
+                                       ? tc::mbar_wait(never_bar, 0, s_abort, tc::kSelfTestSpinLimit)
+                                       : tc::mbar_wait(&s_full[t], kb & 1, s_abort));
+      if (!ok) break;   // warp-uniform: the TMEM accesses below are warp-collective
+      tc::tc_fence_after();
+      float s[64];
+      tc::tmem_ld32_nowait(tS, reinterpret_cast<float(&)[32]>(s[0]));
+      tc::tmem_ld32_nowait(tS + 32, reinterpret_cast<float(&)[32]>(s[32]));
+      tc::tmem_wait_ld();
+      tc::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive_cluster(r_sfree);
+#pragma unroll
+      for (int i = 0; i < 64; ++i) s[i] = exp2f(s[i] - lse2);
+      const int j0 = kb * BC + c * 64;
+      if (j0 + 63 > jlim) {
+#pragma unroll
+        for (int i = 0; i < 64; ++i) if (j0 + i > jlim) s[i] = 0.f;
+      }
+      ok = __all_sync(0xffffffffu, tc::mbar_wait(&p_full[t], kb & 1, s_abort));
+      if (!ok) break;
+      tc::tc_fence_after();
+      uint32_t pk32[32];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float dp[16];
+        tc::tmem_ld16(tP + 16 * q, dp);
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+          const float c0 = s[16 * q + i], c1 = s[16 * q + i + 1];       // 0 where masked, whatever dP is there
+          pk32[8 * q + i / 2] = pack_bf16(c0 * (dp[i] - dvec), c1 * (dp[i + 1] - dvec));
+        }
+      }
+      tc::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive_cluster(r_pfree);
+      if (kb > 0) {   // dQ(kb-1) has finished reading the dC buffer
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(&dq_done[t], (kb - 1) & 1, s_abort));
+        if (!ok) break;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        *reinterpret_cast<uint4*>(cbuf + ((k ^ (m & 7)) << 4)) = make_uint4(pk32[4 * k], pk32[4 * k + 1], pk32[4 * k + 2], pk32[4 * k + 3]);
+      tc::fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive_cluster(r_dc);
+    }
+    // ---- epilogue: the owned dQ rows of this tile, half the columns per thread ----
+    if (my_nkb > 0 && ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(&dq_done[t], (my_nkb - 1) & 1, s_abort));
+    tc::tc_fence_after();
+    const bool have = (my_nkb > 0) && ok;
+    const bool store = row_ok && (m < OWN) && (gi >= p.row_base) && (gi < p.row_end);
+    const size_t orow = ((size_t)bh * N + (row_ok ? gi : 0)) * D + c * (D / 2);
+    if (p.early) pdl_wait();                            // the band kernel's part of dQ
+#pragma unroll
+    for (int q = 0; q < D / 64; ++q) {
+      float o[32];
+      if (have) {
+        tc::tmem_ld32(tQ + q * 32, o);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = 0.f;
+      }
+      if (store) store_grad32(p.dQ, p.out_bf16, p.dQadd, orow + q * 32, o, kLn2);
+    }
+  }
+  __syncwarp();
+
+  // ===================== teardown =====================
+  if (tid == 0 && *s_abort) tc::st_cluster_u32(tc::cluster_addr((const void*)s_abort, rank ^ 1), 1);
+  tc::tc_fence_before();
+  tc::cluster_sync_all();
+  if (*s_abort) {        // of either CTA
+    if (tid == 0) atomicExch(p.status, 1);
+    // nothing of the pair may still be in flight when its shared and tensor memory are given up: the issuer commits
+    // behind its last MMA, one thread waits (bounded) for that commit and for the copies issued last into each slot
+    if (rank == 0 && warp == EW + 1) tc::mma_commit_pair(mma_drain);
+    if (rank == 0 && tid == EW * 32 && nkb > 0) {
+      volatile int never = 0;
+      constexpr uint32_t kDrain = 1u << 14;
+      tc::mbar_wait(q_full, 0, &never, kDrain);
+      const int issued = *s_issued;
+      for (int id = max(0, issued - NSLOT); id < issued; ++id) tc::mbar_wait(&full[id % NSLOT], (id / NSLOT) & 1, &never, kDrain);
+    }
+    if (tid == EW * 32) { volatile int never = 0; tc::mbar_wait(mma_drain, 0, &never); }
+    tc::cluster_sync_all();
+  }
+  if (warp == EW + 1) {
+    tc::tc_fence_after();
+    tc::tmem_dealloc_pair(tmem, Cfg::kTmemCols);
+  }
+}
+
+namespace {
+
+template <int D, int NT>
+cudaError_t launch_t(const TrainParams& p, __nv_bfloat16* Kt, int* status, cudaStream_t stream) {
+  using Cfg = DqCfg<D, NT>;
+  const size_t BH = (size_t)p.B * p.H;
+  alignas(64) CUtensorMap tmQ, tmdO, tmKt, tmKd, tmV;
+  if (!make_tensor_map_bf16(&tmQ, p.Q, D, p.N, BH, 64, Cfg::BM + Cfg::HALO, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmdO, p.dO, D, p.N, BH, 64, Cfg::BM, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmKt, Kt, D, p.N, BH * p.cq, 64, 64, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmKd, Kt, D, p.N, BH * p.cq, D / 2, D == 64 ? 128 : 64, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmV, p.V, D, p.N, BH, 64, 64, true)) return cudaErrorInvalidValue;
+  BwdTcParams bp = {};
+  bp.LSE = p.LSE; bp.Dvec = p.Dvec; bp.dQ = p.dQo; bp.dQadd = p.causal ? p.dQ : nullptr; bp.out_bf16 = p.grad_bf16; bp.status = status;
+  bp.early = p.causal;
+  bp.B = p.B; bp.H = p.H; bp.N = p.N; bp.cq = p.cq; bp.ck = p.ck; bp.causal = p.causal;
+  bp.selftest_expire = take_selftest_expire(kKernBwdDqTc);
+  bp.row_base = win_lo(p); bp.row_end = win_hi(p);
+  bp.own = Cfg::BM - (p.cq - 1);
+  const int rows = bp.own * 2 * NT;
+  auto kern = bwd_dq_tc_kernel<D, NT>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+  if (e != cudaSuccess) return e;
+  dim3 grid(2u * (unsigned)((bp.row_end - bp.row_base + rows - 1) / rows) * (unsigned)BH);
+  ScopedKernelTimer timer_(kKernBwdDqTc, stream);
+  return launch_pdl(kern, grid, dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, tmQ, tmdO, tmKt, tmKd, tmV, bp);
+}
+
+}  // namespace
+
+cudaError_t launch_bwd_dq_pair(const TrainParams& p, __nv_bfloat16* Kt, int* status, cudaStream_t stream) {
+  if (p.d == 128) return launch_t<128, 1>(p, Kt, status, stream);
+  static const char* f = getenv("FMTA_DQ_NT");
+  return f && f[0] == '2' ? launch_t<64, 2>(p, Kt, status, stream) : launch_t<64, 1>(p, Kt, status, stream);
+}
+
+}  // namespace fmta

@@ -54,8 +54,9 @@ size_t bwd_stream_extra_bytes(int B, int H, int N);
 cudaError_t launch_bwd_dkdv_stream(const TrainParams& p, const __nv_bfloat16* Pbuf, const __nv_bfloat16* dCbuf, int ldp,
                                    __nv_bfloat16* dKt, int* status, cudaStream_t stream);
 
+// dQ on CTA pairs, head dims 64 and 128 (bwd_dq_tc.cu)
+cudaError_t launch_bwd_dq_pair(const TrainParams& p, __nv_bfloat16* Kt, int* status, cudaStream_t stream);
 // head dim 128 (bwd_tc128.cu)
-cudaError_t launch_bwd_dq_tc128(const TrainParams& p, const __nv_bfloat16* Kt, int* status, cudaStream_t stream);
 cudaError_t launch_bwd_dkdv_tc128(const TrainParams& p, const __nv_bfloat16* Kt, __nv_bfloat16* dKt, int* status, int with_dv,
                                   int key_lo, int key_hi, cudaStream_t stream);
 

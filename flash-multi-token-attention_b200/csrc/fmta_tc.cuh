@@ -424,6 +424,16 @@ FMTA_DEVINL void mma_commit_pair(uint64_t* bar) {
       ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 
+// CTAs are dispatched in linear block order.  The row blocks of a (batch, head) pair run side by side, longest first, and
+// share its K-tilde and V in L2; the last `X` pairs (a few waves of the GPU) are walked length-major, so that the greedy
+// hardware scheduler ends with the short CTAs.
+FMTA_DEVINL void pair_block_order(int lin, int nqb, int nBH, int& bh, int& r) {
+  const int X = min(nBH, max(1, (256 + nqb / 2) / nqb));
+  const int head = (nBH - X) * nqb;
+  if (lin < head) { bh = lin / nqb; r = lin - bh * nqb; }
+  else { lin -= head; r = lin / X; bh = nBH - X + (lin - r * X); }
+}
+
 // Instruction descriptor, kind::f16: bf16 x bf16 -> fp32, M x N tile.
 //   bits [4,6) D format (1 = F32); [7,10) A format (1 = BF16); [10,13) B format (1 = BF16);
 //   bit 15 A major (0 = K, 1 = MN); bit 16 B major; [17,23) N >> 3; [24,29) M >> 4.

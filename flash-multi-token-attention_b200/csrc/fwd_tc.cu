@@ -183,16 +183,6 @@ struct TcCfg {
 
 constexpr float kRescaleTau = 8.f;   // log2 units: P may reach 2^8 before O is rescaled
 
-// CTAs are dispatched in linear block order.  The row blocks of a (batch, head) pair run side by side, longest first, and
-// share its K-tilde and V in L2; the last `X` pairs (a few waves of the GPU) are walked length-major, so that the greedy
-// hardware scheduler ends with the short CTAs.
-FMTA_DEVINL void pair_block_order(int lin, int nqb, int nBH, int& bh, int& r) {
-  const int X = min(nBH, max(1, (256 + nqb / 2) / nqb));
-  const int head = (nBH - X) * nqb;
-  if (lin < head) { bh = lin / nqb; r = lin - bh * nqb; }
-  else { lin -= head; r = lin / X; bh = nBH - X + (lin - r * X); }
-}
-
 template <int D>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TcCfg<D>::kThreads, D == 64 ? 2 : 1)
 fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKt,
@@ -226,7 +216,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   const int N = p.N, cq = p.cq, pq = cq - 1, pk = (p.ck - 1) / 2;
   const int band = pq + pk;              // entries with query - key < band belong to the band kernel
   int bh, qb;
-  pair_block_order(blockIdx.x >> 1, p.qb_hi - p.qb_lo, p.B * p.H, bh, qb);
+  tc::pair_block_order(blockIdx.x >> 1, p.qb_hi - p.qb_lo, p.B * p.H, bh, qb);
   qb = p.qb_hi - 1 - qb;
   const int P0 = qb * 2 * BM, i0 = P0 + (int)rank * BM;     // first row of the pair, of this CTA
   int nkb = (N + BC - 1) / BC;
