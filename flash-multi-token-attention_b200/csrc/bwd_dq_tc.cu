@@ -9,9 +9,9 @@
 //   S, dP : 256 x 128 x 16 MMAs, each CTA stages half the KEYS of every Kt and V tile;
 //   dQ    : 256 x d x 16 MMAs, each CTA stages half the COLUMNS of every Kt tile (a second copy, fetched just in time
 //           instead of being held from S to dQ).
-// One warp issues everything, in an order that has independent MMAs in every wait for the element-wise warps:
-//   NT = 1: S(kb) dP(kb) | dQ(kb-1) | S(kb+1) ...                     S and dP in columns of their own
-//   NT = 2: S(kb) | dQ(kb-1) first taps | dP(kb) | dQ(kb-1) last taps | S(kb+1) ...     S and dP share 128 columns
+// Scores (S, dP) and dQ are two streams with an issuing warp, a TMA warp and a ring of tiles each: the tensor core takes an
+// MMA only when the one before it is under way, so what one issuer does between two tiles (190 cycles) leaves it idle unless
+// the other has MMAs waiting.  NT = 1: S and dP have 128 columns each; NT = 2: they take turns in 128 columns.
 // Every mbarrier wait is bounded; on expiry the status word is set and the pair drains and leaves.  No TMA multicast.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -31,20 +31,21 @@ struct DqCfg {
   static constexpr int O_SLAB = BM * 128, O_TILE = SLABS * O_SLAB;
   // dC: 64-key slabs of [136 rows][128 B]; the 8 rows below the tile are read by the shifted views of rows that are not owned
   static constexpr int C_SLAB = (BM + 8) * 128, C_TILE = 2 * C_SLAB;
-  static constexpr int TILE_BYTES = 8192;                       // ring tile: 64 keys x 64 elements, or 128 keys x 32 (dQ, d = 64)
-  static constexpr int DT = D / 64;                             // ring tiles of one tap's dQ half
+  // ring tile: SLABS x [64 keys][64 elements] of Kt or V for S / dP; [128 keys][32] (d = 64) or 2 x [64 keys][64] (d = 128)
+  // of Kt for dQ
+  static constexpr int TILE_BYTES = D * 128;
   static constexpr int oQ = 0, oO = oQ + NT * Q_TILE, oC = oO + NT * O_TILE, oRing = oC + NT * C_TILE;
   static_assert(Q_SLAB % 1024 == 0 && C_SLAB % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
-  static constexpr int NSLOT = (227 * 1024 - 1024 - 512 - oRing) / TILE_BYTES;
+  static constexpr int NSLOT = (227 * 1024 - 1024 - 512 - oRing) / TILE_BYTES, NSS = (NSLOT + 1) / 2, NSD = NSLOT - NSS;
   static constexpr int oBar = oRing + NSLOT * TILE_BYTES;
   static constexpr int kSmemBytes = oBar + 512 + 1024;
   static constexpr bool SEP = NT == 1;                          // S and dP in columns of their own
   static constexpr int colX = 0, colP = SEP ? 128 : 0, TCOLS = (SEP ? 256 : 128) + D, colQ = TCOLS - D;   // per tile
   static constexpr int kTmemCols = 512;
   static constexpr int EWT = 8, kEw = NT * EWT;                 // element-wise warps: 4 lane quarters x 2 key halves per tile
-  static constexpr int kThreads = (kEw + 2) * 32;
+  static constexpr int kThreads = (kEw + 4) * 32;               // + TMA and MMA warp of the scores, of dQ
   static_assert(NT * TCOLS <= kTmemCols, "TMEM budget");
-  static_assert(NSLOT >= 8 && kSmemBytes <= 227 * 1024, "shared memory budget");
+  static_assert(NSD >= 3 && kSmemBytes <= 227 * 1024, "shared memory budget");
   static_assert((2 * NSLOT + 1 + 6 * NT + 2) * 8 + 16 <= 512, "barriers");
 };
 
@@ -53,13 +54,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DqCfg<D, NT_>::kThre
 bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO, const __grid_constant__ CUtensorMap tmKt,
                  const __grid_constant__ CUtensorMap tmKd, const __grid_constant__ CUtensorMap tmV, const BwdTcParams p) {
   using Cfg = DqCfg<D, NT_>;
-  constexpr int BM = Cfg::BM, BC = Cfg::BC, NT = Cfg::NT, HALO = Cfg::HALO, SLABS = Cfg::SLABS, NSLOT = Cfg::NSLOT, EW = Cfg::kEw, EWT = Cfg::EWT;
+  constexpr int BM = Cfg::BM, BC = Cfg::BC, NT = Cfg::NT, HALO = Cfg::HALO, SLABS = Cfg::SLABS, NSLOT = Cfg::NSLOT, NSS = Cfg::NSS, EW = Cfg::kEw, EWT = Cfg::EWT;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* sRing = smem + Cfg::oRing;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::oBar);
   // (rank 0): only the copy in rank 0's shared memory is used
-  uint64_t* full = bars;                 // [NSLOT]  TMA of both CTAs -> MMA (rank 0)
+  uint64_t* full = bars;                 // [NSLOT]  TMA of both CTAs -> MMA (rank 0); the first NSS are the scores' ring
   uint64_t* empty = bars + NSLOT;        // [NSLOT]  MMA -> TMA
   uint64_t* q_full = bars + 2 * NSLOT;   // Q and dO staged (rank 0)
   uint64_t* s_full = q_full + 1;         // [NT] S ready
@@ -69,7 +70,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint64_t* dc_full = p_free + NT;       // [NT] dC written to shared memory (rank 0)
   uint64_t* dq_done = dc_full + NT;      // [NT] dQ MMAs of the block complete (dC buffer reusable)
   uint64_t* never_bar = dq_done + NT;    // nothing arrives here (expiry self-test)
-  uint64_t* mma_drain = never_bar + 1;   // abort path: the issued MMAs have completed
+  uint64_t* mma_drain = never_bar + 1;   // abort path: the issued MMAs have completed (both issuers)
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(mma_drain + 1);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
   volatile int* s_issued = s_abort + 1;
@@ -107,8 +108,8 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tc::mbar_init(&p_full[t], 1); tc::mbar_init(&p_free[t], 2 * EWT);
       tc::mbar_init(&dc_full[t], 2 * EWT); tc::mbar_init(&dq_done[t], 1);
     }
-    tc::mbar_init(never_bar, 1); tc::mbar_init(mma_drain, 1);
-    *s_abort = 0; *s_issued = 0;
+    tc::mbar_init(never_bar, 1); tc::mbar_init(mma_drain, 2);
+    *s_abort = 0; s_issued[0] = 0; s_issued[1] = 0;
     tc::mbar_fence_init();
   }
   if (warp == EW + 1) tc::tmem_alloc_pair(s_tmem, Cfg::kTmemCols);
@@ -121,55 +122,52 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   pdl_trigger();
   tc::tc_fence_after();
   const uint32_t tmem = *s_tmem;
-  const int h1 = NT == 2 ? cq / 2 : cq;      // taps in the first part of dQ
+  const int role = warp - EW;                // 0, 1: TMA and MMA of the scores, 2, 3: of dQ
 
-  if (warp == EW) {
-    // ===================== TMA producer: this CTA's Q and dO, its half of every Kt and V tile =====================
+  if (role == 0 || role == 2) {
+    // ===================== TMA producers: this CTA's Q and dO, its half of every Kt and V tile =====================
     if (lane == 0 && nkb > 0) {
-      tc::tma_prefetch_desc(&tmQ); tc::tma_prefetch_desc(&tmdO); tc::tma_prefetch_desc(&tmKt); tc::tma_prefetch_desc(&tmKd); tc::tma_prefetch_desc(&tmV);
-      const uint32_t full0 = tc::cluster_addr(full, 0), qf = tc::cluster_addr(q_full, 0);
-      if (rank == 0) tc::mbar_expect_tx(q_full, 2 * NT * (Cfg::Q_TILE + Cfg::O_TILE));
-      for (int t = 0; t < NT; ++t)
-        for (int sl = 0; sl < SLABS; ++sl) {
-          const int r = R0 + (2 * t + (int)rank) * OWN;
-          tc::tma_load_3d_pair(smem + Cfg::oQ + t * Cfg::Q_TILE + sl * Cfg::Q_SLAB, &tmQ, qf, sl * 64, r - HALO, bh);
-          tc::tma_load_3d_pair(smem + Cfg::oO + t * Cfg::O_TILE + sl * Cfg::O_SLAB, &tmdO, qf, sl * 64, r, bh);
-        }
-      int slot = 0, ph = 1, id = 0;
+      const bool is_s = role == 0;
+      const int base = is_s ? 0 : NSS, n = is_s ? NSS : NSLOT - NSS;
+      const uint32_t full0 = tc::cluster_addr(full, 0);
+      if (is_s) {
+        tc::tma_prefetch_desc(&tmQ); tc::tma_prefetch_desc(&tmdO); tc::tma_prefetch_desc(&tmKt); tc::tma_prefetch_desc(&tmV);
+        const uint32_t qf = tc::cluster_addr(q_full, 0);
+        if (rank == 0) tc::mbar_expect_tx(q_full, 2 * NT * (Cfg::Q_TILE + Cfg::O_TILE));
+        for (int t = 0; t < NT; ++t)
+          for (int sl = 0; sl < SLABS; ++sl) {
+            const int r = R0 + (2 * t + (int)rank) * OWN;
+            tc::tma_load_3d_pair(smem + Cfg::oQ + t * Cfg::Q_TILE + sl * Cfg::Q_SLAB, &tmQ, qf, sl * 64, r - HALO, bh);
+            tc::tma_load_3d_pair(smem + Cfg::oO + t * Cfg::O_TILE + sl * Cfg::O_SLAB, &tmdO, qf, sl * 64, r, bh);
+          }
+      } else tc::tma_prefetch_desc(&tmKd);
+      int slot = base, ph = 1, id = 0;
       bool ok = true;
-      auto put = [&](const CUtensorMap* map, int x, int y, int z) {
+      auto put = [&](const CUtensorMap* map, int x0, int dx, int y0, int dy, int z) {      // SLABS boxes of 8 KB
         if (!tc::mbar_wait(&empty[slot], ph, s_abort)) { ok = false; return; }
         if (rank == 0) tc::mbar_expect_tx(&full[slot], 2 * Cfg::TILE_BYTES);
-        tc::tma_load_3d_pair(sRing + slot * Cfg::TILE_BYTES, map, full0 + slot * 8, x, y, z);
-        if (++slot == NSLOT) { slot = 0; ph ^= 1; }
-        *s_issued = ++id;
+#pragma unroll
+        for (int i = 0; i < SLABS; ++i)
+          tc::tma_load_3d_pair(sRing + slot * Cfg::TILE_BYTES + i * 8192, map, full0 + slot * 8, x0 + i * dx, y0 + i * dy, z);
+        if (++slot == base + n) { slot = base; ph ^= 1; }
+        s_issued[is_s ? 0 : 1] = ++id;
       };
-      auto put_S = [&](int kb) {
-        for (int a = 0; a < cq && ok; ++a)
-          for (int sl = 0; sl < SLABS && ok; ++sl) put(&tmKt, sl * 64, kb * BC + (int)rank * 64, bh * cq + a);
-      };
-      auto put_V = [&](int kb) {
-        for (int sl = 0; sl < SLABS && ok; ++sl) put(&tmV, sl * 64, kb * BC + (int)rank * 64, bh);
-      };
-      auto put_dQ = [&](int kb, int a0, int a1) {
-        for (int a = a0; a < a1 && ok; ++a)
-          for (int v = 0; v < Cfg::DT && ok; ++v) put(&tmKd, (int)rank * (D / 2), kb * BC + v * 64, bh * cq + a);
-      };
-      for (int kb = 0; kb <= nkb && ok; ++kb) {      // the order of the issuer
-        if (kb < nkb) put_S(kb);
-        if (NT == 1 && kb < nkb) put_V(kb);
-        if (kb > 0) put_dQ(kb - 1, 0, h1);
-        if (NT == 2 && kb < nkb) put_V(kb);
-        if (kb > 0) put_dQ(kb - 1, h1, cq);
+      for (int kb = 0; kb < nkb && ok; ++kb) {
+        if (is_s) {
+          for (int a = 0; a < cq && ok; ++a) put(&tmKt, 0, 64, kb * BC + (int)rank * 64, 0, bh * cq + a);
+          if (ok) put(&tmV, 0, 64, kb * BC + (int)rank * 64, 0, bh);
+        } else {
+          for (int a = 0; a < cq && ok; ++a) put(&tmKd, (int)rank * (D / 2), 0, kb * BC, 64, bh * cq + a);
+        }
       }
       // the last arrivals on this CTA's `empty` barriers have landed before it leaves
-      for (int i = 0; i < NSLOT && i < id && ok; ++i) {
-        if (--slot < 0) { slot = NSLOT - 1; ph ^= 1; }
+      for (int i = 0; i < n && i < id && ok; ++i) {
+        if (--slot < base) { slot = base + n - 1; ph ^= 1; }
         ok = tc::mbar_wait(&empty[slot], ph ^ 1, s_abort);
       }
     }
-  } else if (warp == EW + 1) {
-    // ===================== MMA issuer (rank 0) =====================
+  } else if (role == 1 || role == 3) {
+    // ===================== MMA issuers (rank 0) =====================
     if (nkb > 0 && rank == 0) {   // all lanes run the loop; one elected lane issues
       constexpr uint32_t idescS = tc::make_idesc(2 * BM, BC, 0, 0);    // S, dP: both operands K-major
       constexpr uint32_t idescQ = tc::make_idesc(2 * BM, D, 0, 1);     // dQ: B (Kt) MN-major
@@ -177,80 +175,69 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const uint64_t d64 = tc::make_sdesc(smem_u32(sRing), 16, 512, tc::kLayoutSW64);
       const uint32_t hi = (uint32_t)(d128 >> 32), r_lo = (uint32_t)d128, d_hi = D == 64 ? (uint32_t)(d64 >> 32) : hi;
       const uint32_t s_lo = r_lo - (uint32_t)(Cfg::oRing >> 4);        // descriptor of shared-memory offset 0
-      const uint32_t q_lo = s_lo + (uint32_t)((Cfg::oQ + (HALO - pq) * 128) >> 4), o_lo = s_lo + (uint32_t)(Cfg::oO >> 4), c_lo = s_lo + (uint32_t)(Cfg::oC >> 4);
-      int slot = 0, ph = 0;
-      bool ok = tc::mbar_wait_cluster_warp(q_full, 0, s_abort);
-      auto take = [&]() -> bool { ok = tc::mbar_wait_cluster_warp(&full[slot], ph, s_abort); tc::tc_fence_after(); return ok; };
-      auto give = [&]() { tc::mma_commit_pair(&empty[slot]); if (++slot == NSLOT) { slot = 0; ph ^= 1; } };
+      bool ok = true;
       auto wait_all = [&](uint64_t* bar, int kb, int n) {              // completion n of bar[t] for every tile that has block kb
 #pragma unroll
         for (int t = 0; t < NT; ++t)
           if (ok && kb < nkb_t[t]) ok = tc::mbar_wait_cluster_warp(&bar[t], n & 1, s_abort);
         tc::tc_fence_after();
       };
-      auto issue_S = [&](int kb) {
-        if (kb > 0) wait_all(Cfg::SEP ? s_free : p_free, kb, kb - 1);  // what block kb-1 left in these columns has been taken
-        for (int a = 0; a < cq && ok; ++a)
+      if (role == 1) {
+        const uint32_t q_lo = s_lo + (uint32_t)((Cfg::oQ + (HALO - pq) * 128) >> 4), o_lo = s_lo + (uint32_t)(Cfg::oO >> 4);
+        tc::PairRing<NSS> ring(full, empty, s_abort);
+        ok = tc::mbar_wait_cluster_warp(q_full, 0, s_abort);
+        for (int kb = 0; kb < nkb && ok; ++kb) {
+          if (kb > 0) wait_all(Cfg::SEP ? s_free : p_free, kb, kb - 1);  // what block kb-1 left in these columns has been taken
+          for (int a = 0; a < cq && ok; ++a) {
+            if (!(ok = ring.take())) break;
 #pragma unroll
-          for (int sl = 0; sl < SLABS; ++sl) {
-            if (!take()) return;
+            for (int sl = 0; sl < SLABS; ++sl)
+#pragma unroll
+              for (int t = 0; t < NT; ++t)
+                if (kb < nkb_t[t])
+                  tc::mma4_ss<2>(tmem + t * Cfg::TCOLS + Cfg::colX, q_lo + (uint32_t)((t * Cfg::Q_TILE + sl * Cfg::Q_SLAB + a * 128) >> 4), hi, 2,
+                                 r_lo + (uint32_t)((ring.slot * Cfg::TILE_BYTES + sl * 8192) >> 4), hi, 2, idescS, (a | sl) != 0);
+            ring.give();
+          }
+          if (!ok) break;
+#pragma unroll
+          for (int t = 0; t < NT; ++t) if (kb < nkb_t[t]) tc::mma_commit_pair(&s_full[t]);
+          if (!Cfg::SEP) wait_all(s_free, kb, kb);                       // S of this block has been taken
+          else if (kb > 0) wait_all(p_free, kb, kb - 1);
+          if (!ok || !(ok = ring.take())) break;
+#pragma unroll
+          for (int sl = 0; sl < SLABS; ++sl)
 #pragma unroll
             for (int t = 0; t < NT; ++t)
               if (kb < nkb_t[t])
-                tc::mma4_ss<2>(tmem + t * Cfg::TCOLS + Cfg::colX, q_lo + (uint32_t)((t * Cfg::Q_TILE + sl * Cfg::Q_SLAB + a * 128) >> 4), hi, 2,
-                               r_lo + (uint32_t)(slot * (Cfg::TILE_BYTES >> 4)), hi, 2, idescS, (a | sl) != 0);
-            give();
-          }
+                tc::mma4_ss<2>(tmem + t * Cfg::TCOLS + Cfg::colP, o_lo + (uint32_t)((t * Cfg::O_TILE + sl * Cfg::O_SLAB) >> 4), hi, 2,
+                               r_lo + (uint32_t)((ring.slot * Cfg::TILE_BYTES + sl * 8192) >> 4), hi, 2, idescS, sl != 0);
+          ring.give();
 #pragma unroll
-        for (int t = 0; t < NT; ++t) if (ok && kb < nkb_t[t]) tc::mma_commit_pair(&s_full[t]);
-      };
-      auto issue_dP = [&](int kb) {
-        if (!Cfg::SEP) wait_all(s_free, kb, kb);                       // S of this block has been taken
-        else if (kb > 0) wait_all(p_free, kb, kb - 1);
-#pragma unroll
-        for (int sl = 0; sl < SLABS; ++sl) {
-          if (!ok || !take()) return;
-#pragma unroll
-          for (int t = 0; t < NT; ++t)
-            if (kb < nkb_t[t])
-              tc::mma4_ss<2>(tmem + t * Cfg::TCOLS + Cfg::colP, o_lo + (uint32_t)((t * Cfg::O_TILE + sl * Cfg::O_SLAB) >> 4), hi, 2,
-                             r_lo + (uint32_t)(slot * (Cfg::TILE_BYTES >> 4)), hi, 2, idescS, sl != 0);
-          give();
+          for (int t = 0; t < NT; ++t) if (kb < nkb_t[t]) tc::mma_commit_pair(&p_full[t]);
         }
-#pragma unroll
-        for (int t = 0; t < NT; ++t) if (kb < nkb_t[t]) tc::mma_commit_pair(&p_full[t]);
-      };
-      auto issue_dQ = [&](int kb, int a0, int a1) {
-        if (a0 == 0) wait_all(dc_full, kb, kb);
-        for (int a = a0; a < a1 && ok; ++a)
-#pragma unroll
-          for (int v = 0; v < Cfg::DT; ++v) {
-            if (!take()) return;
-            const uint32_t b_lo = r_lo + (uint32_t)(slot * (Cfg::TILE_BYTES >> 4));
+      } else {
+        const uint32_t c_lo = s_lo + (uint32_t)(Cfg::oC >> 4), rd_lo = r_lo + (uint32_t)(NSS * (Cfg::TILE_BYTES >> 4));
+        tc::PairRing<NSLOT - NSS> ring(full + NSS, empty + NSS, s_abort);
+        for (int kb = 0; kb < nkb && ok; ++kb) {
+          wait_all(dc_full, kb, kb);
+          for (int a = 0; a < cq && ok; ++a) {
+            if (!(ok = ring.take())) break;
+            const uint32_t b_lo = rd_lo + (uint32_t)(ring.slot * (Cfg::TILE_BYTES >> 4));
 #pragma unroll
             for (int t = 0; t < NT; ++t)
               if (kb < nkb_t[t]) {                                     // dC rows i' + pad_q - a
                 const uint32_t a_lo = c_lo + (uint32_t)((t * Cfg::C_TILE + (pq - a) * 128) >> 4), dst = tmem + t * Cfg::TCOLS + Cfg::colQ;
-                if constexpr (D == 64) {                               // 128 keys x 32 columns, 64-byte swizzle
-                  tc::mma4_ss<2>(dst, a_lo, hi, 2, b_lo, d_hi, 64, idescQ, (kb | a) != 0);
-                  tc::mma4_ss<2>(dst, a_lo + (uint32_t)(Cfg::C_SLAB >> 4), hi, 2, b_lo + 256, d_hi, 64, idescQ, 1);
-                } else {
-                  tc::mma4_ss<2>(dst, a_lo + (uint32_t)(v * (Cfg::C_SLAB >> 4)), hi, 2, b_lo, d_hi, 128, idescQ, (kb | a | v) != 0);
-                }
+                constexpr uint32_t step = D == 64 ? 64 : 128;          // 16 keys
+                tc::mma4_ss<2>(dst, a_lo, hi, 2, b_lo, d_hi, step, idescQ, (kb | a) != 0);
+                tc::mma4_ss<2>(dst, a_lo + (uint32_t)(Cfg::C_SLAB >> 4), hi, 2, b_lo + 4 * step, d_hi, step, idescQ, 1);
               }
-            give();
+            ring.give();
           }
-        if (ok && a1 == cq) {
+          if (!ok) break;
 #pragma unroll
           for (int t = 0; t < NT; ++t) if (kb < nkb_t[t]) tc::mma_commit_pair(&dq_done[t]);
         }
-      };
-      for (int kb = 0; kb <= nkb && ok; ++kb) {
-        if (kb < nkb) issue_S(kb);
-        if (NT == 1 && ok && kb < nkb) issue_dP(kb);
-        if (ok && kb > 0) issue_dQ(kb - 1, 0, h1);
-        if (NT == 2 && ok && kb < nkb) issue_dP(kb);
-        if (NT == 2 && ok && kb > 0) issue_dQ(kb - 1, h1, cq);
       }
     }
   } else {
@@ -345,13 +332,15 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (tid == 0) atomicExch(p.status, 1);
     // nothing of the pair may still be in flight when its shared and tensor memory are given up: the issuer commits
     // behind its last MMA, one thread waits (bounded) for that commit and for the copies issued last into each slot
-    if (rank == 0 && warp == EW + 1) tc::mma_commit_pair(mma_drain);
+    if (rank == 0 && (role == 1 || role == 3)) tc::mma_commit_pair(mma_drain);
     if (rank == 0 && tid == EW * 32 && nkb > 0) {
       volatile int never = 0;
       constexpr uint32_t kDrain = 1u << 14;
       tc::mbar_wait(q_full, 0, &never, kDrain);
-      const int issued = *s_issued;
-      for (int id = max(0, issued - NSLOT); id < issued; ++id) tc::mbar_wait(&full[id % NSLOT], (id / NSLOT) & 1, &never, kDrain);
+      for (int r = 0; r < 2; ++r) {
+        const int issued = s_issued[r], base = r ? NSS : 0, n = r ? NSLOT - NSS : NSS;
+        for (int id = max(0, issued - n); id < issued; ++id) tc::mbar_wait(&full[base + id % n], (id / n) & 1, &never, kDrain);
+      }
     }
     if (tid == EW * 32) { volatile int never = 0; tc::mbar_wait(mma_drain, 0, &never); }
     tc::cluster_sync_all();

@@ -1141,7 +1141,7 @@ cudaError_t launch_bwd_dq_tc(const TrainParams& p, void* workspace, bool keep_pd
   // d = 64: two row tiles of one CTA share every key tile and keep it from S to dQ; the pair kernel has half the rows per
   // SM and wins where that leaves no SM without work
   const long ctas = (long)BH * ((win_hi(p) - win_lo(p) + 2 * (Cfg::BM - p.cq)) / (2 * (Cfg::BM - p.cq + 1)));
-  if (p.d == 128 || (!keep_pdc && ctas <= 148)) return launch_bwd_dq_pair(p, Kt, status, stream);
+  if (p.d == 128 || (!keep_pdc && ctas <= 74)) return launch_bwd_dq_pair(p, Kt, status, stream);
   alignas(64) CUtensorMap tmQ, tmdO, tmKt, tmV;
   if (!make_tensor_map_bf16(&tmQ, p.Q, D, p.N, BH, 8, Cfg::QR / 2, false)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmdO, p.dO, D, p.N, BH, 64, Cfg::BM, true)) return cudaErrorInvalidValue;

@@ -402,6 +402,34 @@ FMTA_DEVINL bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int*
 FMTA_DEVINL bool mbar_wait_cluster_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag));
 }
+// One look at a barrier, no waiting.
+FMTA_DEVINL uint32_t mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return ok;
+}
+// The issuer's end of a ring of tiles.  The tensor core takes an MMA only when the one before it is under way, so whatever
+// the issuer does between two tiles leaves it idle: a wait that is over already still costs 200 cycles.  take() therefore
+// looks at the NEXT tile's barrier before the MMAs of this one are issued and give() picks the answer up behind them.
+template <int NSLOT>
+struct PairRing {
+  uint64_t *full, *empty;
+  volatile int* abort_flag;
+  int slot = 0, ph = 0, nslot = 0, nph = 0;
+  uint32_t seen = 0;
+  bool ready = false;
+  FMTA_DEVINL PairRing(uint64_t* f, uint64_t* e, volatile int* a) : full(f), empty(e), abort_flag(a) {}
+  FMTA_DEVINL bool take() {
+    if (!ready && !mbar_wait_cluster_warp(&full[slot], ph, abort_flag)) return false;
+    tc_fence_after();
+    nslot = slot + 1 == NSLOT ? 0 : slot + 1;
+    nph = nslot == 0 ? ph ^ 1 : ph;
+    seen = mbar_test(&full[nslot], nph);
+    return true;
+  }
+  FMTA_DEVINL void give();
+};
 // tile into this CTA's shared memory, completing on a barrier of rank 0 (cluster_bar: shared::cluster address)
 FMTA_DEVINL void tma_load_3d_pair(void* smem_dst, const CUtensorMap* map, uint32_t cluster_bar, int c0, int c1, int c2) {
   asm volatile(
@@ -422,6 +450,13 @@ FMTA_DEVINL void mma_commit_pair(uint64_t* bar) {
       "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
       "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
       ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
+
+template <int NSLOT>
+FMTA_DEVINL void PairRing<NSLOT>::give() {
+  mma_commit_pair(&empty[slot]);
+  slot = nslot; ph = nph;
+  ready = __all_sync(0xffffffffu, seen);
 }
 
 // CTAs are dispatched in linear block order.  The row blocks of a (batch, head) pair run side by side, longest first, and

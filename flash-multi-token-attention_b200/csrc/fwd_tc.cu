@@ -289,7 +289,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       const uint64_t dV0 = D == 64 ? tc::make_sdesc(smem_u32(sRing), 16, 512, tc::kLayoutSW64) : dK0;
       const uint32_t a_hi = (uint32_t)(dQ0 >> 32), a_lo0 = (uint32_t)dQ0;
       const uint32_t k_hi = (uint32_t)(dK0 >> 32), v_hi = (uint32_t)(dV0 >> 32), b_lo0 = (uint32_t)dK0;
-      int slot = 0, ph = 0;
+      tc::PairRing<NSLOT> ring(full, empty, s_abort);
       bool ok = tc::mbar_wait_cluster_warp(q_full, 0, s_abort);
       auto issue_S = [&](int kb) {
         const int buf = kb % NS;
@@ -303,13 +303,10 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         for (int a = 0; a < cq; ++a, a_lo += 128 >> 4) {
 #pragma unroll
           for (int sl = 0; sl < SLABS; ++sl) {
-            ok = tc::mbar_wait_cluster_warp(&full[slot], ph, s_abort);
-            if (!ok) return;
-            tc::tc_fence_after();
-            const uint32_t b_lo = b_lo0 + (uint32_t)(slot * (Cfg::TILE_BYTES >> 4));
+            if (!(ok = ring.take())) return;
+            const uint32_t b_lo = b_lo0 + (uint32_t)(ring.slot * (Cfg::TILE_BYTES >> 4));
             tc::mma4_ss<2>(dS, a_lo + (uint32_t)(sl * (QR * 128 >> 4)), a_hi, 2, b_lo, k_hi, 2, idescS, (a | sl) != 0);
-            tc::mma_commit_pair(&empty[slot]);
-            if (++slot == NSLOT) { slot = 0; ph ^= 1; }
+            ring.give();
           }
         }
         tc::mma_commit_pair(&s_full[buf]);
@@ -319,16 +316,13 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         if (!ok) return;
 #pragma unroll
         for (int v = 0; v < Cfg::VT; ++v) {
-          ok = tc::mbar_wait_cluster_warp(&full[slot], ph, s_abort);
-          if (!ok) return;
-          tc::tc_fence_after();
-          const uint32_t b_lo = b_lo0 + (uint32_t)(slot * (Cfg::TILE_BYTES >> 4));
+          if (!(ok = ring.take())) return;
+          const uint32_t b_lo = b_lo0 + (uint32_t)(ring.slot * (Cfg::TILE_BYTES >> 4));
 #pragma unroll
           for (int k = 0; k < BC / 16 / Cfg::VT; k += 4)       // 16 keys: 16 rows of V, 8 columns of P
             tc::mma4_ts<2>(tmem + Cfg::colO, tmem + Cfg::colP + 8 * (v * 4 + k), 8, b_lo + (uint32_t)(k * (16 * Cfg::VW * 2 / 16)), v_hi,
                            16 * Cfg::VW * 2 / 16, idescPV, (kb | v | k) != 0);
-          tc::mma_commit_pair(&empty[slot]);
-          if (++slot == NSLOT) { slot = 0; ph ^= 1; }
+          ring.give();
         }
         tc::mma_commit_pair(o_full);
       };
