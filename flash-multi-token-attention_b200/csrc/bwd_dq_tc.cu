@@ -1,7 +1,7 @@
 // dQ of the stacked-GEMM backward on CTA pairs (the math of bwd_tc.cu; entries off the causal band):
 //     C = sum_a Q^(a) Kt_a^T,  P = exp2(C - LSE*log2e),  dC = P * (dO V^T - D),  dQ[i'] = ln2 * sum_a sum_j dC[i' + pad_q - a, j] Kt_a[j]
 //
-// A pair of CTAs walks blocks of 128 keys for 256 * NT rows of dC (a tile of 128 per CTA and t, one TMEM lane per row).  A
+// A pair of CTAs walks blocks of 128 keys for 256 rows of dC (a tile of 128 per CTA, one TMEM lane per row).  A
 // tile computes 128 dC rows but owns only the first 128 - pad_q as dQ rows: dQ row i' needs dC rows i'..i'+pad_q, so tiles
 // overlap by pad_q rows (recomputed) and no dQ row is shared.  The row shifts of Q and dC are free: both are staged as
 // 128-byte-swizzled tiles and the tensor core applies the swizzle to the absolute shared-memory address, so a view shifted
@@ -11,7 +11,10 @@
 //           instead of being held from S to dQ).
 // Scores (S, dP) and dQ are two streams with an issuing warp, a TMA warp and a ring of tiles each: the tensor core takes an
 // MMA only when the one before it is under way, so what one issuer does between two tiles (190 cycles) leaves it idle unless
-// the other has MMAs waiting.  NT = 1: S and dP have 128 columns each; NT = 2: they take turns in 128 columns.
+// the other has MMAs waiting.
+// Measured (B200, c_q 6, causal, N 4096; single CTAs before): d = 128, B 8, H 32: 7.8 -> 5.1 ms; d = 64, B 4, H 16: 831 ->
+// 793 us; d = 64, N 1024, 8 heads, c_q 7: 63 -> 33 us.  Two row tiles per CTA (d = 64, S and dP taking turns in one set of
+// columns) move half the key tiles but took 864 us.  Bound by shared-memory operand reads: 5 KB per 43-cycle dQ MMA at d = 64.
 // Every mbarrier wait is bounded; on expiry the status word is set and the pair drains and leaves.  No TMA multicast.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -22,9 +25,9 @@
 
 namespace fmta {
 
-template <int D, int NT_>
+template <int D>
 struct DqCfg {
-  static constexpr int BM = 128, BC = 128, NT = NT_;
+  static constexpr int BM = 128, BC = 128;
   static constexpr int HALO = 8;                                // rows of Q staged above a tile (pad_q <= 8)
   static constexpr int SLABS = D / 64;                          // 64-element (128-byte) column slabs per row
   static constexpr int Q_SLAB = (BM + HALO) * 128, Q_TILE = SLABS * Q_SLAB;
@@ -34,27 +37,25 @@ struct DqCfg {
   // ring tile: SLABS x [64 keys][64 elements] of Kt or V for S / dP; [128 keys][32] (d = 64) or 2 x [64 keys][64] (d = 128)
   // of Kt for dQ
   static constexpr int TILE_BYTES = D * 128;
-  static constexpr int oQ = 0, oO = oQ + NT * Q_TILE, oC = oO + NT * O_TILE, oRing = oC + NT * C_TILE;
+  static constexpr int oQ = 0, oO = oQ + Q_TILE, oC = oO + O_TILE, oRing = oC + C_TILE;
   static_assert(Q_SLAB % 1024 == 0 && C_SLAB % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
   static constexpr int NSLOT = (227 * 1024 - 1024 - 512 - oRing) / TILE_BYTES, NSS = (NSLOT + 1) / 2, NSD = NSLOT - NSS;
   static constexpr int oBar = oRing + NSLOT * TILE_BYTES;
   static constexpr int kSmemBytes = oBar + 512 + 1024;
-  static constexpr bool SEP = NT == 1;                          // S and dP in columns of their own
-  static constexpr int colX = 0, colP = SEP ? 128 : 0, TCOLS = (SEP ? 256 : 128) + D, colQ = TCOLS - D;   // per tile
+  static constexpr int colS = 0, colP = 128, colQ = 256;
   static constexpr int kTmemCols = 512;
-  static constexpr int EWT = 8, kEw = NT * EWT;                 // element-wise warps: 4 lane quarters x 2 key halves per tile
+  static constexpr int kEw = 8;                                 // element-wise warps: 4 lane quarters x 2 key halves
   static constexpr int kThreads = (kEw + 4) * 32;               // + TMA and MMA warp of the scores, of dQ
-  static_assert(NT * TCOLS <= kTmemCols, "TMEM budget");
   static_assert(NSD >= 3 && kSmemBytes <= 227 * 1024, "shared memory budget");
-  static_assert((2 * NSLOT + 1 + 6 * NT + 2) * 8 + 16 <= 512, "barriers");
+  static_assert((2 * NSLOT + 9) * 8 + 16 <= 512, "barriers");
 };
 
-template <int D, int NT_>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DqCfg<D, NT_>::kThreads, 1)
+template <int D>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DqCfg<D>::kThreads, 1)
 bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO, const __grid_constant__ CUtensorMap tmKt,
                  const __grid_constant__ CUtensorMap tmKd, const __grid_constant__ CUtensorMap tmV, const BwdTcParams p) {
-  using Cfg = DqCfg<D, NT_>;
-  constexpr int BM = Cfg::BM, BC = Cfg::BC, NT = Cfg::NT, HALO = Cfg::HALO, SLABS = Cfg::SLABS, NSLOT = Cfg::NSLOT, NSS = Cfg::NSS, EW = Cfg::kEw, EWT = Cfg::EWT;
+  using Cfg = DqCfg<D>;
+  constexpr int BM = Cfg::BM, BC = Cfg::BC, HALO = Cfg::HALO, SLABS = Cfg::SLABS, NSLOT = Cfg::NSLOT, NSS = Cfg::NSS, EW = Cfg::kEw;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* sRing = smem + Cfg::oRing;
@@ -63,13 +64,13 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint64_t* full = bars;                 // [NSLOT]  TMA of both CTAs -> MMA (rank 0); the first NSS are the scores' ring
   uint64_t* empty = bars + NSLOT;        // [NSLOT]  MMA -> TMA
   uint64_t* q_full = bars + 2 * NSLOT;   // Q and dO staged (rank 0)
-  uint64_t* s_full = q_full + 1;         // [NT] S ready
-  uint64_t* s_free = s_full + NT;        // [NT] S taken into registers (rank 0)
-  uint64_t* p_full = s_free + NT;        // [NT] dP ready
-  uint64_t* p_free = p_full + NT;        // [NT] dP taken into registers (rank 0)
-  uint64_t* dc_full = p_free + NT;       // [NT] dC written to shared memory (rank 0)
-  uint64_t* dq_done = dc_full + NT;      // [NT] dQ MMAs of the block complete (dC buffer reusable)
-  uint64_t* never_bar = dq_done + NT;    // nothing arrives here (expiry self-test)
+  uint64_t* s_full = q_full + 1;         // S ready
+  uint64_t* s_free = s_full + 1;        // S taken into registers (rank 0)
+  uint64_t* p_full = s_free + 1;        // dP ready
+  uint64_t* p_free = p_full + 1;        // dP taken into registers (rank 0)
+  uint64_t* dc_full = p_free + 1;       // dC written to shared memory (rank 0)
+  uint64_t* dq_done = dc_full + 1;      // dQ MMAs of the block complete (dC buffer reusable)
+  uint64_t* never_bar = dq_done + 1;    // nothing arrives here (expiry self-test)
   uint64_t* mma_drain = never_bar + 1;   // abort path: the issued MMAs have completed (both issuers)
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(mma_drain + 1);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
@@ -79,35 +80,27 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const uint32_t rank = tc::cluster_rank();
   const int N = p.N, cq = p.cq, pq = cq - 1, pk = (p.ck - 1) / 2;
   const int band = pq + pk;
-  const int OWN = p.own, rows_per_pair = OWN * 2 * NT;
+  const int OWN = p.own, rows_per_pair = OWN * 2;
   const int nQB = (p.row_end - p.row_base + rows_per_pair - 1) / rows_per_pair;
   int bh, qb;
   tc::pair_block_order(blockIdx.x >> 1, nQB, p.B * p.H, bh, qb);
   // Row blocks are laid out from the END of the rows: when their number is not a multiple of the block, the partly filled
   // block is the first one, which sees the fewest keys.  Its rows before row_base are computed (negative rows as zero
-  // rows) and not stored.  Tile t of the pair: rows R0 + 2 t OWN (rank 0), R0 + (2 t + 1) OWN (rank 1).
+  // rows) and not stored.  CTA r's tile starts at row R0 + r OWN.
   const int R0 = p.row_end - (qb + 1) * rows_per_pair;
   const int nKB = (N + BC - 1) / BC;
-  int nkb_t[NT];
-#pragma unroll
-  for (int t = 0; t < NT; ++t) {
-    const int r1 = R0 + (2 * t + 1) * OWN;               // the later of the two tiles
-    if (r1 + OWN <= p.row_base) nkb_t[t] = 0;
-    else if (p.causal) {
-      const int last = min(N - 1, r1 + BM - 1) - band;
-      nkb_t[t] = last >= 0 ? min(nKB, last / BC + 1) : 0;
-    } else nkb_t[t] = nKB;
+  int nkb = nKB;
+  if (p.causal) {                                        // key blocks with at least one key j <= (last row) - band
+    const int last = min(N - 1, R0 + OWN + BM - 1) - band;
+    nkb = last >= 0 ? min(nKB, last / BC + 1) : 0;
   }
-  const int nkb = nkb_t[NT - 1];                         // tiles of later rows see no fewer keys
 
   if (tid == 0) {
     for (int i = 0; i < NSLOT; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 1); }
     tc::mbar_init(q_full, 1);
-    for (int t = 0; t < NT; ++t) {
-      tc::mbar_init(&s_full[t], 1); tc::mbar_init(&s_free[t], 2 * EWT);
-      tc::mbar_init(&p_full[t], 1); tc::mbar_init(&p_free[t], 2 * EWT);
-      tc::mbar_init(&dc_full[t], 2 * EWT); tc::mbar_init(&dq_done[t], 1);
-    }
+    tc::mbar_init(s_full, 1); tc::mbar_init(s_free, 2 * EW);
+    tc::mbar_init(p_full, 1); tc::mbar_init(p_free, 2 * EW);
+    tc::mbar_init(dc_full, 2 * EW); tc::mbar_init(dq_done, 1);
     tc::mbar_init(never_bar, 1); tc::mbar_init(mma_drain, 2);
     *s_abort = 0; s_issued[0] = 0; s_issued[1] = 0;
     tc::mbar_fence_init();
@@ -133,13 +126,11 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (is_s) {
         tc::tma_prefetch_desc(&tmQ); tc::tma_prefetch_desc(&tmdO); tc::tma_prefetch_desc(&tmKt); tc::tma_prefetch_desc(&tmV);
         const uint32_t qf = tc::cluster_addr(q_full, 0);
-        if (rank == 0) tc::mbar_expect_tx(q_full, 2 * NT * (Cfg::Q_TILE + Cfg::O_TILE));
-        for (int t = 0; t < NT; ++t)
-          for (int sl = 0; sl < SLABS; ++sl) {
-            const int r = R0 + (2 * t + (int)rank) * OWN;
-            tc::tma_load_3d_pair(smem + Cfg::oQ + t * Cfg::Q_TILE + sl * Cfg::Q_SLAB, &tmQ, qf, sl * 64, r - HALO, bh);
-            tc::tma_load_3d_pair(smem + Cfg::oO + t * Cfg::O_TILE + sl * Cfg::O_SLAB, &tmdO, qf, sl * 64, r, bh);
-          }
+        if (rank == 0) tc::mbar_expect_tx(q_full, 2 * (Cfg::Q_TILE + Cfg::O_TILE));
+        for (int sl = 0; sl < SLABS; ++sl) {
+          tc::tma_load_3d_pair(smem + Cfg::oQ + sl * Cfg::Q_SLAB, &tmQ, qf, sl * 64, R0 + (int)rank * OWN - HALO, bh);
+          tc::tma_load_3d_pair(smem + Cfg::oO + sl * Cfg::O_SLAB, &tmdO, qf, sl * 64, R0 + (int)rank * OWN, bh);
+        }
       } else tc::tma_prefetch_desc(&tmKd);
       int slot = base, ph = 1, id = 0;
       bool ok = true;
@@ -176,10 +167,8 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const uint32_t hi = (uint32_t)(d128 >> 32), r_lo = (uint32_t)d128, d_hi = D == 64 ? (uint32_t)(d64 >> 32) : hi;
       const uint32_t s_lo = r_lo - (uint32_t)(Cfg::oRing >> 4);        // descriptor of shared-memory offset 0
       bool ok = true;
-      auto wait_all = [&](uint64_t* bar, int kb, int n) {              // completion n of bar[t] for every tile that has block kb
-#pragma unroll
-        for (int t = 0; t < NT; ++t)
-          if (ok && kb < nkb_t[t]) ok = tc::mbar_wait_cluster_warp(&bar[t], n & 1, s_abort);
+      auto wait = [&](uint64_t* bar, int n) {                          // completion n of the barrier
+        ok = tc::mbar_wait_cluster_warp(bar, n & 1, s_abort);
         tc::tc_fence_after();
       };
       if (role == 1) {
@@ -187,78 +176,63 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         tc::PairRing<NSS> ring(full, empty, s_abort);
         ok = tc::mbar_wait_cluster_warp(q_full, 0, s_abort);
         for (int kb = 0; kb < nkb && ok; ++kb) {
-          if (kb > 0) wait_all(Cfg::SEP ? s_free : p_free, kb, kb - 1);  // what block kb-1 left in these columns has been taken
+          if (kb > 0) wait(s_free, kb - 1);                              // S(kb-1) has been taken
           for (int a = 0; a < cq && ok; ++a) {
             if (!(ok = ring.take())) break;
 #pragma unroll
             for (int sl = 0; sl < SLABS; ++sl)
-#pragma unroll
-              for (int t = 0; t < NT; ++t)
-                if (kb < nkb_t[t])
-                  tc::mma4_ss<2>(tmem + t * Cfg::TCOLS + Cfg::colX, q_lo + (uint32_t)((t * Cfg::Q_TILE + sl * Cfg::Q_SLAB + a * 128) >> 4), hi, 2,
-                                 r_lo + (uint32_t)((ring.slot * Cfg::TILE_BYTES + sl * 8192) >> 4), hi, 2, idescS, (a | sl) != 0);
+              tc::mma4_ss<2>(tmem + Cfg::colS, q_lo + (uint32_t)((sl * Cfg::Q_SLAB + a * 128) >> 4), hi, 2,
+                             r_lo + (uint32_t)((ring.slot * Cfg::TILE_BYTES + sl * 8192) >> 4), hi, 2, idescS, (a | sl) != 0);
             ring.give();
           }
           if (!ok) break;
-#pragma unroll
-          for (int t = 0; t < NT; ++t) if (kb < nkb_t[t]) tc::mma_commit_pair(&s_full[t]);
-          if (!Cfg::SEP) wait_all(s_free, kb, kb);                       // S of this block has been taken
-          else if (kb > 0) wait_all(p_free, kb, kb - 1);
+          tc::mma_commit_pair(s_full);
+          if (kb > 0) wait(p_free, kb - 1);
           if (!ok || !(ok = ring.take())) break;
 #pragma unroll
           for (int sl = 0; sl < SLABS; ++sl)
-#pragma unroll
-            for (int t = 0; t < NT; ++t)
-              if (kb < nkb_t[t])
-                tc::mma4_ss<2>(tmem + t * Cfg::TCOLS + Cfg::colP, o_lo + (uint32_t)((t * Cfg::O_TILE + sl * Cfg::O_SLAB) >> 4), hi, 2,
-                               r_lo + (uint32_t)((ring.slot * Cfg::TILE_BYTES + sl * 8192) >> 4), hi, 2, idescS, sl != 0);
+            tc::mma4_ss<2>(tmem + Cfg::colP, o_lo + (uint32_t)((sl * Cfg::O_SLAB) >> 4), hi, 2,
+                           r_lo + (uint32_t)((ring.slot * Cfg::TILE_BYTES + sl * 8192) >> 4), hi, 2, idescS, sl != 0);
           ring.give();
-#pragma unroll
-          for (int t = 0; t < NT; ++t) if (kb < nkb_t[t]) tc::mma_commit_pair(&p_full[t]);
+          tc::mma_commit_pair(p_full);
         }
       } else {
         const uint32_t c_lo = s_lo + (uint32_t)(Cfg::oC >> 4), rd_lo = r_lo + (uint32_t)(NSS * (Cfg::TILE_BYTES >> 4));
         tc::PairRing<NSLOT - NSS> ring(full + NSS, empty + NSS, s_abort);
         for (int kb = 0; kb < nkb && ok; ++kb) {
-          wait_all(dc_full, kb, kb);
+          wait(dc_full, kb);
           for (int a = 0; a < cq && ok; ++a) {
             if (!(ok = ring.take())) break;
             const uint32_t b_lo = rd_lo + (uint32_t)(ring.slot * (Cfg::TILE_BYTES >> 4));
-#pragma unroll
-            for (int t = 0; t < NT; ++t)
-              if (kb < nkb_t[t]) {                                     // dC rows i' + pad_q - a
-                const uint32_t a_lo = c_lo + (uint32_t)((t * Cfg::C_TILE + (pq - a) * 128) >> 4), dst = tmem + t * Cfg::TCOLS + Cfg::colQ;
-                constexpr uint32_t step = D == 64 ? 64 : 128;          // 16 keys
-                tc::mma4_ss<2>(dst, a_lo, hi, 2, b_lo, d_hi, step, idescQ, (kb | a) != 0);
-                tc::mma4_ss<2>(dst, a_lo + (uint32_t)(Cfg::C_SLAB >> 4), hi, 2, b_lo + 4 * step, d_hi, step, idescQ, 1);
-              }
+            const uint32_t a_lo = c_lo + (uint32_t)(((pq - a) * 128) >> 4);      // dC rows i' + pad_q - a
+            constexpr uint32_t step = D == 64 ? 64 : 128;                        // 16 keys
+            tc::mma4_ss<2>(tmem + Cfg::colQ, a_lo, hi, 2, b_lo, d_hi, step, idescQ, (kb | a) != 0);
+            tc::mma4_ss<2>(tmem + Cfg::colQ, a_lo + (uint32_t)(Cfg::C_SLAB >> 4), hi, 2, b_lo + 4 * step, d_hi, step, idescQ, 1);
             ring.give();
           }
           if (!ok) break;
-#pragma unroll
-          for (int t = 0; t < NT; ++t) if (kb < nkb_t[t]) tc::mma_commit_pair(&dq_done[t]);
+          tc::mma_commit_pair(dq_done);
         }
       }
     }
   } else {
     // ===================== element-wise warps: one dC row and 64 of the 128 keys per thread =====================
-    const int t = warp / EWT, c = (warp >> 2) & 1;
+    const int c = warp >> 2;                            // key half
     const int m = (warp & 3) * 32 + lane;               // row within the tile = TMEM lane
-    const int gi = R0 + (2 * t + (int)rank) * OWN + m;  // query index of this dC row
-    const uint32_t tT = tmem + t * Cfg::TCOLS + ((uint32_t)((warp & 3) * 32) << 16);
-    const uint32_t tS = tT + Cfg::colX + c * 64, tP = tT + Cfg::colP + c * 64, tQ = tT + Cfg::colQ + c * (D / 2);
-    const uint32_t r_sfree = tc::cluster_addr(&s_free[t], 0), r_pfree = tc::cluster_addr(&p_free[t], 0), r_dc = tc::cluster_addr(&dc_full[t], 0);
-    const int my_nkb = nkb_t[t];
+    const int gi = R0 + (int)rank * OWN + m;  // query index of this dC row
+    const uint32_t tT = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t tS = tT + Cfg::colS + c * 64, tP = tT + Cfg::colP + c * 64, tQ = tT + Cfg::colQ + c * (D / 2);
+    const uint32_t r_sfree = tc::cluster_addr(s_free, 0), r_pfree = tc::cluster_addr(p_free, 0), r_dc = tc::cluster_addr(dc_full, 0);
     const bool row_ok = gi >= 0 && gi < N;
     const float lse2 = row_ok ? p.LSE[(size_t)bh * N + gi] * kLog2e : 0.f;
     const float dvec = row_ok ? p.Dvec[(size_t)bh * N + gi] : 0.f;
     const int jlim = row_ok ? (p.causal ? min(N - 1, gi - band) : N - 1) : -1;   // last key owned here
-    unsigned char* cbuf = smem + Cfg::oC + t * Cfg::C_TILE + c * Cfg::C_SLAB + m * 128;   // 16-byte chunk k of the row at chunk k ^ (row & 7)
+    unsigned char* cbuf = smem + Cfg::oC + c * Cfg::C_SLAB + m * 128;   // 16-byte chunk k of the row at chunk k ^ (row & 7)
     bool ok = true;
-    for (int kb = 0; kb < my_nkb && ok; ++kb) {
+    for (int kb = 0; kb < nkb && ok; ++kb) {
       ok = __all_sync(0xffffffffu, (p.selftest_expire && kb == 0)
                                        ? tc::mbar_wait(never_bar, 0, s_abort, tc::kSelfTestSpinLimit)
-                                       : tc::mbar_wait(&s_full[t], kb & 1, s_abort));
+                                       : tc::mbar_wait(s_full, kb & 1, s_abort));
       if (!ok) break;   // warp-uniform: the TMEM accesses below are warp-collective
       tc::tc_fence_after();
       float s[64];
@@ -275,7 +249,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
         for (int i = 0; i < 64; ++i) if (j0 + i > jlim) s[i] = 0.f;
       }
-      ok = __all_sync(0xffffffffu, tc::mbar_wait(&p_full[t], kb & 1, s_abort));
+      ok = __all_sync(0xffffffffu, tc::mbar_wait(p_full, kb & 1, s_abort));
       if (!ok) break;
       tc::tc_fence_after();
       uint32_t pk32[32];
@@ -293,7 +267,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       __syncwarp();
       if (lane == 0) tc::mbar_arrive_cluster(r_pfree);
       if (kb > 0) {   // dQ(kb-1) has finished reading the dC buffer
-        ok = __all_sync(0xffffffffu, tc::mbar_wait(&dq_done[t], (kb - 1) & 1, s_abort));
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(dq_done, (kb - 1) & 1, s_abort));
         if (!ok) break;
       }
 #pragma unroll
@@ -304,9 +278,9 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (lane == 0) tc::mbar_arrive_cluster(r_dc);
     }
     // ---- epilogue: the owned dQ rows of this tile, half the columns per thread ----
-    if (my_nkb > 0 && ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(&dq_done[t], (my_nkb - 1) & 1, s_abort));
+    if (nkb > 0 && ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(dq_done, (nkb - 1) & 1, s_abort));
     tc::tc_fence_after();
-    const bool have = (my_nkb > 0) && ok;
+    const bool have = (nkb > 0) && ok;
     const bool store = row_ok && (m < OWN) && (gi >= p.row_base) && (gi < p.row_end);
     const size_t orow = ((size_t)bh * N + (row_ok ? gi : 0)) * D + c * (D / 2);
     if (p.early) pdl_wait();                            // the band kernel's part of dQ
@@ -353,9 +327,9 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
 namespace {
 
-template <int D, int NT>
+template <int D>
 cudaError_t launch_t(const TrainParams& p, __nv_bfloat16* Kt, int* status, cudaStream_t stream) {
-  using Cfg = DqCfg<D, NT>;
+  using Cfg = DqCfg<D>;
   const size_t BH = (size_t)p.B * p.H;
   alignas(64) CUtensorMap tmQ, tmdO, tmKt, tmKd, tmV;
   if (!make_tensor_map_bf16(&tmQ, p.Q, D, p.N, BH, 64, Cfg::BM + Cfg::HALO, true)) return cudaErrorInvalidValue;
@@ -370,8 +344,8 @@ cudaError_t launch_t(const TrainParams& p, __nv_bfloat16* Kt, int* status, cudaS
   bp.selftest_expire = take_selftest_expire(kKernBwdDqTc);
   bp.row_base = win_lo(p); bp.row_end = win_hi(p);
   bp.own = Cfg::BM - (p.cq - 1);
-  const int rows = bp.own * 2 * NT;
-  auto kern = bwd_dq_tc_kernel<D, NT>;
+  const int rows = bp.own * 2;
+  auto kern = bwd_dq_tc_kernel<D>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
   dim3 grid(2u * (unsigned)((bp.row_end - bp.row_base + rows - 1) / rows) * (unsigned)BH);
@@ -382,9 +356,7 @@ cudaError_t launch_t(const TrainParams& p, __nv_bfloat16* Kt, int* status, cudaS
 }  // namespace
 
 cudaError_t launch_bwd_dq_pair(const TrainParams& p, __nv_bfloat16* Kt, int* status, cudaStream_t stream) {
-  if (p.d == 128) return launch_t<128, 1>(p, Kt, status, stream);
-  static const char* f = getenv("FMTA_DQ_NT");
-  return f && f[0] == '2' ? launch_t<64, 2>(p, Kt, status, stream) : launch_t<64, 1>(p, Kt, status, stream);
+  return p.d == 128 ? launch_t<128>(p, Kt, status, stream) : launch_t<64>(p, Kt, status, stream);
 }
 
 }  // namespace fmta

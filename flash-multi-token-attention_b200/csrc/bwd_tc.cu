@@ -9,7 +9,9 @@
 // The band entries are handled by bwd_band_kernel (bwd_band.cu), which adds its part to the same
 // outputs afterwards.
 //
-//   bwd_dq_tc_kernel   : CTA = NT query-row tiles, loops key blocks.  A tile computes dC for
+//   bwd_dq_tc_kernel (bwd_dq_tc.cu): dQ on CTA pairs.
+//   bwd_dq_stream_kernel : dQ for the calls that stream P and dC to the dK/dV kernel (bwd_stream.cu): it also leaves
+//                        them in global memory.  CTA = NT query-row tiles, loops key blocks.  A tile computes dC for
 //                        128 rows but owns only the first 120 of them as dQ rows: dQ row i'
 //                        needs dC rows i'..i'+pad_q, so consecutive tiles overlap by 8 rows
 //                        (recomputed, like the halo of the exact kernels) and no dQ row is
@@ -17,7 +19,6 @@
 //                        in shared memory as a 128-byte-swizzled [rows][64 keys] tile, and the tensor
 //                        core applies the swizzle to the absolute address, so a view shifted by s
 //                        rows is the same tile with the descriptor start address moved by 128 s bytes.
-//                        With STREAM the kernel also leaves P and dC in global memory (bwd_stream.cu).
 //   bwd_dkdv_tc_kernel : CTA = 128 keys (= TMEM lanes), loops 64-row query blocks; transposed
 //                        scores S^T = Kt_a Q^(a)T so that P^T and dC^T are produced with keys on the
 //                        lanes (rows of the dV / dKt accumulators).  Q is staged once per block as a
@@ -37,11 +38,10 @@ namespace fmta {
 // ==========================================================================================
 // dQ
 // ==========================================================================================
-template <int D, bool STREAM = false>   // STREAM: the kernel also leaves P and dC in global memory (see bwd_stream.cu)
-struct DqCfg {
-  static_assert(D == 64, "the dQ tensor-core kernel is instantiated for d = 64");
+struct DqStreamCfg {
+  static constexpr int D = 64;
   static constexpr int BM = 128;               // dC rows per tile (= TMEM lanes)
-  static constexpr int OWN = 120;              // dQ rows a tile owns at most when its rows must start on a multiple of 8 (STREAM); else 128 - pad_q (dQ row i needs dC rows i .. i + pad_q)
+  static constexpr int OWN = 120;              // dQ rows a tile owns (its rows start on a multiple of 8; dQ row i needs dC rows i .. i + pad_q)
   static constexpr int OWN_MAX = 128;
   static constexpr int BC = 64;                // keys per block
   static constexpr int NT = 2;                 // row tiles per CTA
@@ -52,31 +52,29 @@ struct DqCfg {
   static_assert((QR / 2 * 16) % 128 == 0, "TMA destination alignment");
   static constexpr int DR = BM + 16;           // rows of a dC buffer (16 zero rows below)
   static constexpr int TILE_BYTES = BC * 128;  // Kt / V ring tile: 64 keys x 64 elements
-  static constexpr int NSLOT = STREAM ? 11 : 15;   // the Kt tiles of one key block held for its dQ MMAs (cq <= 7) while
-                                               // the next block's cq + 1 tiles stream in: 2 cq + 1 slots (four of them
-                                               // make room for the P tiles when P and dC are streamed out)
+  static constexpr int NSLOT = 11;             // the Kt tiles of one key block held for its dQ MMAs (cq <= 7) while
+                                               // the next block's tiles stream in
   static constexpr int oQ = 0;                                  // [D/8][QR][16 B]
   static constexpr int odO = oQ + QR * D * 2;                   // NT x [128 rows][128 B], 128B swizzle
   static constexpr int DC_BYTES = DR * 128;                     // one dC buffer: [DR rows][128 B], 128B swizzle
   static constexpr int odC = odO + NT * BM * 128;               // NT buffers
   static_assert(odC % 1024 == 0 && DC_BYTES % 1024 == 0, "swizzled dC buffers start on 1024-byte boundaries");
-  static constexpr int P_BYTES = BM * 128;                      // STREAM: one P tile, [128 rows][128 B], 128B swizzle
+  static constexpr int P_BYTES = BM * 128;                      // one P tile, [128 rows][128 B], 128B swizzle
   static constexpr int oP = odC + NT * DC_BYTES;
-  static constexpr int oRing = ((oP + (STREAM ? NT * P_BYTES : 0) + 1023) / 1024) * 1024;
+  static constexpr int oRing = ((oP + NT * P_BYTES + 1023) / 1024) * 1024;
   static constexpr int oBar = oRing + NSLOT * TILE_BYTES;
   static constexpr int kSmemBytes = oBar + 512 + 1024;
   static constexpr int kTmemCols = 512;        // per tile t: S (two buffers) at 256t and 256t+64, dP at 256t+128, dQ at 256t+192
   static constexpr int kThreads = (NT * 4 + 1 + 2 * NT) * 32;   // element-wise warps, TMA warp, two MMA issuer warps per tile
 };
 
-template <int D, bool STREAM>
-__global__ void __launch_bounds__(DqCfg<D, STREAM>::kThreads, 1)
-bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
+__global__ void __launch_bounds__(DqStreamCfg::kThreads, 1)
+bwd_dq_stream_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
                  const __grid_constant__ CUtensorMap tmKt, const __grid_constant__ CUtensorMap tmV,
                  const BwdTcParams p) {
-  using Cfg = DqCfg<D, STREAM>;
-  constexpr int BM = Cfg::BM, BC = Cfg::BC, NT = Cfg::NT, HALO = Cfg::HALO, QR = Cfg::QR;
-  const int OWN = STREAM ? Cfg::OWN : p.own;
+  using Cfg = DqStreamCfg;
+  constexpr int D = Cfg::D, BM = Cfg::BM, BC = Cfg::BC, NT = Cfg::NT, HALO = Cfg::HALO, QR = Cfg::QR;
+  constexpr int OWN = Cfg::OWN;
   constexpr int DR = Cfg::DR, NSLOT = Cfg::NSLOT;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -149,12 +147,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   for (int i = tid; i < NT * Cfg::DC_BYTES / 4; i += Cfg::kThreads) reinterpret_cast<uint32_t*>(sdC)[i] = 0u;
   tc::fence_proxy_async_smem();
   tc::tc_fence_before();
-  // Behind the band kernel (p.early) everything but its part of dQ is complete already: the kernel starts under the
-  // band kernel's tail and waits in its epilogue.  Otherwise it waits here.  The dK/dV kernel behind it starts as soon as
-  // every CTA here has triggered and reads what was complete by then (all but this kernel's dQ), hence the order.
   __syncthreads();
-  if (!p.early) pdl_wait();
-  pdl_trigger();
   tc::tc_fence_after();
   const uint32_t tmem = *s_tmem;
 
@@ -252,7 +245,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           if (active) {
             ok = tc::mbar_wait_warp(&dc_full[t], kb & 1, s_abort);
             tc::tc_fence_after();
-            if constexpr (STREAM) {
+            {
               // P and dC of the tile's owned rows leave as they lie in shared memory (the swizzled image): the
               // global tensors are tile-major [B*H][row block of 64][key block of 64][64 rows x 128 bytes], a
               // tile's rows start at a multiple of 8, so a row keeps its swizzle phase and the streaming kernel
@@ -292,13 +285,13 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             if (!tc::mbar_wait_warp(&full[slot], ph, s_abort)) { ok = false; break; }
             if (tc::elect_one()) tc::mbar_arrive(&empty[slot]);
           }
-          if constexpr (STREAM) {   // the bulk copies have read their tiles before the buffers are handed back
+          {   // the bulk copies have read their tiles before the buffers are handed back
             if (active && tc::elect_one()) tc::tma_store_wait_read();
             __syncwarp();
           }
           if (active) tc::mma_commit_e(&dq_done[t]);
         }
-        if constexpr (STREAM) {
+        {
           if (tc::elect_one()) tc::tma_store_wait_all();
           __syncwarp();
         }
@@ -317,7 +310,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const float dvec = row_ok ? p.Dvec[(size_t)bh * N + gi] : 0.f;
     unsigned char* ctile = sdC + t * Cfg::DC_BYTES;     // this tile's dC buffer; chunk c of row r at r*128 + ((c ^ (r & 7)) << 4)
     unsigned char* cbuf = ctile + m * 128;
-    // STREAM: P goes to a second swizzled tile beside dC; the dQ issuer of the tile sends both out with bulk copies
+    // P goes to a second swizzled tile beside dC; the dQ issuer of the tile sends both out with bulk copies
     unsigned char* pbuf = smem + Cfg::oP + t * Cfg::P_BYTES + m * 128;
     bool ok = true;
     for (int kb = 0; kb < my_nkb && ok; ++kb) {
@@ -340,37 +333,23 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tc::mbar_arrive(&s_free[2 * t + (kb & 1)]);
       const int j0 = kb * BC;
       const int jlim = row_ok ? (p.causal ? min(N - 1, gi - band) : N - 1) : -1;   // last key owned here
-      uint32_t pk32[BC / 2], pp32[STREAM ? BC / 2 : 1];
-      if constexpr (!STREAM) {
-        // one loop with the ownership mask always applied: two predicated selects per pair cost less than the
-        // registers a separate unmasked copy of the loop takes (this kernel is capped at 128 registers)
+      uint32_t pk32[BC / 2], pp32[BC / 2];
 #pragma unroll
-        for (int i = 0; i < BC; i += 2) {
-          float c0 = exp2f(s[i] - lse2) * (dp[i] - dvec);
-          float c1 = exp2f(s[i + 1] - lse2) * (dp[i + 1] - dvec);
-          if (j0 + i > jlim) c0 = 0.f;
-          if (j0 + i + 1 > jlim) c1 = 0.f;
-          pk32[i / 2] = pack_bf16(c0, c1);
-        }
-      } else {   // same arithmetic, keeping P as well
-#pragma unroll
-        for (int i = 0; i < BC; i += 2) {
-          float p0 = exp2f(s[i] - lse2), p1 = exp2f(s[i + 1] - lse2);
-          if (j0 + i > jlim) p0 = 0.f;
-          if (j0 + i + 1 > jlim) p1 = 0.f;
-          pp32[i / 2] = pack_bf16(p0, p1);
-          pk32[i / 2] = pack_bf16(p0 * (dp[i] - dvec), p1 * (dp[i + 1] - dvec));
-        }
+      for (int i = 0; i < BC; i += 2) {
+        float p0 = exp2f(s[i] - lse2), p1 = exp2f(s[i + 1] - lse2);
+        if (j0 + i > jlim) p0 = 0.f;
+        if (j0 + i + 1 > jlim) p1 = 0.f;
+        pp32[i / 2] = pack_bf16(p0, p1);
+        pk32[i / 2] = pack_bf16(p0 * (dp[i] - dvec), p1 * (dp[i + 1] - dvec));
       }
-      if (kb > 0) {   // dQ(kb-1) has finished reading the dC buffer (STREAM: and the bulk copies of block kb-1 both tiles)
+      if (kb > 0) {   // dQ(kb-1) has finished reading the dC buffer and the bulk copies of block kb-1 both tiles
         ok = __all_sync(0xffffffffu, tc::mbar_wait(&dq_done[t], (kb - 1) & 1, s_abort));
         if (!ok) break;
       }
 #pragma unroll
       for (int kc = 0; kc < BC / 8; ++kc) {
         *reinterpret_cast<uint4*>(cbuf + ((kc ^ (m & 7)) << 4)) = make_uint4(pk32[4 * kc], pk32[4 * kc + 1], pk32[4 * kc + 2], pk32[4 * kc + 3]);
-        if constexpr (STREAM)
-          *reinterpret_cast<uint4*>(pbuf + ((kc ^ (m & 7)) << 4)) = make_uint4(pp32[4 * kc], pp32[4 * kc + 1], pp32[4 * kc + 2], pp32[4 * kc + 3]);
+        *reinterpret_cast<uint4*>(pbuf + ((kc ^ (m & 7)) << 4)) = make_uint4(pp32[4 * kc], pp32[4 * kc + 1], pp32[4 * kc + 2], pp32[4 * kc + 3]);
       }
       tc::fence_proxy_async_smem();
       tc::mbar_arrive(&dc_full[t]);
@@ -378,7 +357,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // ---- streaming outputs: zero the key blocks this tile did not visit but a 64-row x 128-key tile of the
     // dK/dV kernel that holds one of its rows may read: up to the end of the 128-key tile of key
     // (last row + 63 - band); without a causal mask, up to ldp ----
-    if (STREAM && row_ok && m < OWN) {
+    if (row_ok && m < OWN) {
       const int nkb64 = p.ldp >> 6;
       const size_t tile_row = ((size_t)bh * ((N + 63) >> 6) + (gi >> 6)) * nkb64 * 4096 + (size_t)(gi & 63) * 64;
       bf16* prow = p.Pout + tile_row;     // key block kz of this row: + kz * 4096
@@ -398,7 +377,6 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const bool have = (my_nkb > 0) && ok;
     const bool store = row_ok && (m < OWN) && (gi >= p.row_base) && (gi < p.row_end);
     const size_t orow = ((size_t)bh * N + (row_ok ? gi : 0)) * D;
-    if (p.early) pdl_wait();                            // the band kernel's part of dQ
 #pragma unroll
     for (int c = 0; c < D / 32; ++c) {
       float o[32];
@@ -1127,8 +1105,8 @@ cudaError_t launch_bwd_ktilde(const TrainParams& p, void* workspace, cudaStream_
 }
 
 cudaError_t launch_bwd_dq_tc(const TrainParams& p, void* workspace, bool keep_pdc, cudaStream_t stream) {
-  constexpr int D = 64;
-  using Cfg = DqCfg<D, false>;
+  using Cfg = DqStreamCfg;
+  constexpr int D = Cfg::D;
   const size_t rows = (size_t)p.B * p.H * p.N, BH = (size_t)p.B * p.H;
   auto up = [](size_t x) { return (x + 1023) / 1024 * 1024; };
   unsigned char* w = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(workspace) + 1023) & ~uintptr_t(1023));
@@ -1138,10 +1116,7 @@ cudaError_t launch_bwd_dq_tc(const TrainParams& p, void* workspace, bool keep_pd
   int* status = nullptr;
   cudaError_t e = status_word_of(reinterpret_cast<int*>(w), stream, &status);
   if (e != cudaSuccess) return e;
-  // d = 64: two row tiles of one CTA share every key tile and keep it from S to dQ; the pair kernel has half the rows per
-  // SM and wins where that leaves no SM without work
-  const long ctas = (long)BH * ((win_hi(p) - win_lo(p) + 2 * (Cfg::BM - p.cq)) / (2 * (Cfg::BM - p.cq + 1)));
-  if (p.d == 128 || (!keep_pdc && ctas <= 74)) return launch_bwd_dq_pair(p, Kt, status, stream);
+  if (p.d == 128 || !keep_pdc) return launch_bwd_dq_pair(p, Kt, status, stream);
   alignas(64) CUtensorMap tmQ, tmdO, tmKt, tmV;
   if (!make_tensor_map_bf16(&tmQ, p.Q, D, p.N, BH, 8, Cfg::QR / 2, false)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmdO, p.dO, D, p.N, BH, 64, Cfg::BM, true)) return cudaErrorInvalidValue;
@@ -1149,31 +1124,19 @@ cudaError_t launch_bwd_dq_tc(const TrainParams& p, void* workspace, bool keep_pd
   if (!make_tensor_map_bf16(&tmV, p.V, D, p.N, BH, 64, Cfg::BC, true)) return cudaErrorInvalidValue;
   BwdTcParams bp = {};
   bp.LSE = p.LSE; bp.Dvec = p.Dvec; bp.dQ = p.dQo; bp.dQadd = p.causal ? p.dQ : nullptr; bp.out_bf16 = p.grad_bf16; bp.status = status;
-  bp.early = p.causal && !keep_pdc;
   bp.B = p.B; bp.H = p.H; bp.N = p.N; bp.cq = p.cq; bp.ck = p.ck; bp.causal = p.causal;
   bp.selftest_expire = take_selftest_expire(kKernBwdDqTc);
   bp.row_base = win_lo(p); bp.row_end = win_hi(p);
-  bp.row_anchor = keep_pdc ? (bp.row_end + 7) / 8 * 8 : bp.row_end;
-  bp.own = keep_pdc ? Cfg::OWN : Cfg::BM - (p.cq - 1);
-  const int rows_per_cta = bp.own * Cfg::NT;
+  bp.row_anchor = (bp.row_end + 7) / 8 * 8;
+  constexpr int rows_per_cta = Cfg::OWN * Cfg::NT;
   dim3 grid((bp.row_anchor - bp.row_base + rows_per_cta - 1) / rows_per_cta, p.H, p.B);
-  if (keep_pdc) {
-    stream_buffers(p, workspace, &bp.Pout, &bp.dCout, &bp.ldp);
-    if (p.N % 64 != 0) zero_tail_rows_kernel<<<dim3(bp.ldp / 64, (unsigned)BH), 128, 0, stream>>>(bp.Pout, bp.dCout, p.N, bp.ldp / 64);
-    using CfgS = DqCfg<D, true>;
-    auto kern = bwd_dq_tc_kernel<D, true>;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CfgS::kSmemBytes);
-    if (e != cudaSuccess) return e;
-    ScopedKernelTimer timer_(kKernBwdDqTc, stream);
-    kern<<<grid, CfgS::kThreads, CfgS::kSmemBytes, stream>>>(tmQ, tmdO, tmKt, tmV, bp);
-    return cudaGetLastError();
-  }
-  auto kern = bwd_dq_tc_kernel<D, false>;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+  stream_buffers(p, workspace, &bp.Pout, &bp.dCout, &bp.ldp);
+  if (p.N % 64 != 0) zero_tail_rows_kernel<<<dim3(bp.ldp / 64, (unsigned)BH), 128, 0, stream>>>(bp.Pout, bp.dCout, p.N, bp.ldp / 64);
+  e = cudaFuncSetAttribute(bwd_dq_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
-  { ScopedKernelTimer timer_(kKernBwdDqTc, stream);
-    e = launch_pdl(kern, grid, dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, tmQ, tmdO, tmKt, tmV, bp); }
-  return e;
+  ScopedKernelTimer timer_(kKernBwdDqTc, stream);
+  bwd_dq_stream_kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(tmQ, tmdO, tmKt, tmV, bp);
+  return cudaGetLastError();
 }
 
 
