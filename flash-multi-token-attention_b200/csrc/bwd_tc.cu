@@ -432,11 +432,16 @@ struct DkvCfg {
   static constexpr int oStage = oV + KT_BYTES;
   static constexpr int sgdO = 0;                                  // [64 rows][128 B], 128B swizzle
   static constexpr int sgQ = BR * 128;                            // [QR rows][128 B], 128B swizzle (one TMA copy)
-  static constexpr int sgLD = sgQ + QR * 128;                     // LSE*log2e [64], D [64]
-  static constexpr int STAGE_BYTES = ((sgLD + 2 * BR * 4 + 1023) / 1024) * 1024;
+  static constexpr int sgLD = sgQ + QR * 128;                     // -LSE*log2e [64 rows][16 B], then -D: B operands, see oOnes
+  static constexpr int STAGE_BYTES = ((sgLD + 2 * BR * 16 + 1023) / 1024) * 1024;
   static constexpr int oPT = oStage + NSTG * STAGE_BYTES;         // P^T : [BR/8][128 keys][16 B] (K-major A operand)
   static constexpr int oDCT = oPT + (BR / 8) * BK * 16;           // dC^T: same layout
-  static constexpr int oBar = oDCT + (BR / 8) * BK * 16;
+  // The row statistics enter through the tensor core: S^T - LSE and dP^T - D are one more contraction step each, with
+  // A = [1 1 1 0 ...] for every key and B = the statistic of a row as three bf16 pieces (24 bits: exact).  As values the
+  // element-wise warps load, they are 16 floats per thread and statistic, the same for all lanes: 512 of the 990
+  // shared-memory cycles that those warps took per block, while the MMAs' operands alone take 2300 of 3700.
+  static constexpr int oOnes = oDCT + (BR / 8) * BK * 16;         // [2][128 keys][16 B]
+  static constexpr int oBar = oOnes + 2 * BK * 16;
   static constexpr int kSmemBytes = oBar + 512 + 1024;
   static_assert(kSmemBytes <= 227 * 1024, "dK/dV kernel: shared memory budget");
   static constexpr int kTmemCols = 512;        // dV at 0, dKt_a at 64*(1+a), scratch X at 448
@@ -510,6 +515,9 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tc::tmem_alloc(s_tmem, Cfg::kTmemCols);
     tc::tmem_relinquish();
   }
+  for (int i = tid; i < 2 * BK; i += Cfg::kThreads)      // bf16 1, 1, 1, 0 ... | 0 ...
+    reinterpret_cast<uint4*>(smem + Cfg::oOnes)[i] = i < BK ? make_uint4(0x3f803f80u, 0x00003f80u, 0u, 0u) : make_uint4(0u, 0u, 0u, 0u);
+  tc::fence_proxy_async_smem();
   tc::tc_fence_before();
   pdl_trigger();
   __syncthreads();
@@ -537,14 +545,21 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         unsigned char* sg = sStage + st * Cfg::STAGE_BYTES;
         ok = __all_sync(0xffffffffu, tc::mbar_wait(&empty[st], ph ^ 1, s_abort));
         if (!ok) break;
-        // LSE * log2(e) and D of the 64 rows: two rows per lane, plain loads and stores
-        float* ld = reinterpret_cast<float*>(sg + Cfg::sgLD);
+        // -LSE * log2(e) and -D of the 64 rows, two rows per lane, in three bf16 pieces each
+        uint4* ld = reinterpret_cast<uint4*>(sg + Cfg::sgLD);
+        auto pieces = [](float v) {
+          const bf16 a = __float2bfloat16_rn(v);
+          const float r1 = v - __bfloat162float(a);
+          const bf16 b2 = __float2bfloat16_rn(r1), c = __float2bfloat16_rn(r1 - __bfloat162float(b2));
+          return make_uint4((uint32_t)__bfloat16_as_ushort(a) | ((uint32_t)__bfloat16_as_ushort(b2) << 16), (uint32_t)__bfloat16_as_ushort(c), 0u, 0u);
+        };
 #pragma unroll
         for (int r = lane; r < BR; r += 32) {
           const int gi = i0 + r;
-          ld[r] = gi < N ? p.LSE[(size_t)bh * N + gi] * kLog2e : 0.f;
-          ld[BR + r] = gi < N ? p.Dvec[(size_t)bh * N + gi] : 0.f;
+          ld[r] = pieces(gi < N ? -p.LSE[(size_t)bh * N + gi] * kLog2e : 0.f);
+          ld[BR + r] = pieces(gi < N ? -p.Dvec[(size_t)bh * N + gi] : 0.f);
         }
+        tc::fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
           tc::mbar_expect_tx(&full[st], BR * 128 + QR * 128);
@@ -568,6 +583,10 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const uint64_t dKtA = tc::make_sdesc(smem_u32(sKt), 16, 1024, tc::kLayoutSW128);
       const uint32_t kt_hi = (uint32_t)(dKtA >> 32), kt_lo = (uint32_t)dKtA;
       const uint32_t v_lo = kt_lo + (uint32_t)((Cfg::oV - Cfg::oKt) >> 4);
+      const uint64_t dOn = tc::make_sdesc(smem_u32(smem + Cfg::oOnes), BK * 16, 128, tc::kLayoutNone);
+      // a statistic's rows, 16 bytes each; the second 8 contraction columns meet zeros of A, so they may be the same bytes
+      const uint64_t dSt = tc::make_sdesc(smem_u32(sStage) + Cfg::sgLD, 0, 128, tc::kLayoutNone);
+      const uint32_t ones_hi = (uint32_t)(dOn >> 32), ones_lo = (uint32_t)dOn, st_hi = (uint32_t)(dSt >> 32), st_lo = (uint32_t)dSt;
       bool ok = tc::mbar_wait_warp(v_full, 0, s_abort);
       // X holds dP^T(it) first (taken by the element-wise warps one block ahead), then S^T(it):
       //   dP^T(0) | S^T(0) dP^T(1) | S^T(1) dP^T(2) | ...
@@ -577,10 +596,8 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const uint32_t o_hi = (uint32_t)(dOk >> 32), o_lo = (uint32_t)dOk;
         if (!tc::mbar_wait_warp(&full[st], ph, s_abort)) { ok = false; return; }
         tc::tc_fence_after();
-        tc::mma_ss2e<0>(tX, v_lo, kt_hi, o_lo, o_hi, idescT);               // dP^T = V dO^T
-#pragma unroll
-        for (int k = 1; k < D / 16; ++k)
-          tc::mma_ss2e<1>(tX, v_lo + (uint32_t)(2 * k), kt_hi, o_lo + (uint32_t)(2 * k), o_hi, idescT);
+        tc::mma4_ss(tX, v_lo, kt_hi, 2, o_lo, o_hi, 2, idescT, 0);           // dP^T - D = V dO^T - D
+        tc::mma_ss2e<1>(tX, ones_lo, ones_hi, st_lo + (uint32_t)((st * Cfg::STAGE_BYTES + BR * 16) >> 4), st_hi, idescT);
         tc::mma_commit_e(dpt_full);
       };
       if (ok) issue_dPT(0);
@@ -594,15 +611,11 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (it == 0 && !tc::mbar_wait_warp(kv_full, 0, s_abort)) { ok = false; break; }   // the Kt tiles
         if (!tc::mbar_wait_warp(xd_free, it & 1, s_abort)) { ok = false; break; }   // dP^T(it) has left X
         tc::tc_fence_after();
-        // S^T = sum_a Kt_a Q^(a)T
-        for (int a = 0; a < cq; ++a) {
-          const uint32_t a_lo = kt_lo + (uint32_t)(a * (Cfg::KT_BYTES >> 4));
-          const uint32_t b_lo = qk_lo + (uint32_t)(a * (128 >> 4));
-          tc::mma_ss2pe(tX, a_lo, kt_hi, b_lo, qk_hi, idescT, a != 0);
-#pragma unroll
-          for (int k = 1; k < D / 16; ++k)
-            tc::mma_ss2e<1>(tX, a_lo + (uint32_t)(2 * k), kt_hi, b_lo + (uint32_t)(2 * k), qk_hi, idescT);
-        }
+        // S^T - LSE = sum_a Kt_a Q^(a)T - LSE
+        for (int a = 0; a < cq; ++a)
+          tc::mma4_ss(tX, kt_lo + (uint32_t)(a * (Cfg::KT_BYTES >> 4)), kt_hi, 2, qk_lo + (uint32_t)(a * (128 >> 4)), qk_hi, 2, idescT, a != 0);
+        // last, so that the sum is rounded at the size of S - LSE once, as a subtraction in a register would
+        tc::mma_ss2e<1>(tX, ones_lo, ones_hi, st_lo + (uint32_t)((st * Cfg::STAGE_BYTES) >> 4), st_hi, idescT);
         tc::mma_commit_e(st_full);
         tc::mma_commit_e(&empty[st]);        // this issuer's reads of the stage (dO for dP^T, Q for S^T) are done then
         if (!tc::mbar_wait_warp(xs_free, it & 1, s_abort)) { ok = false; break; }   // S^T(it) has left X
@@ -642,10 +655,7 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (!tc::mbar_wait_warp(pdc_full, it & 1, s_abort)) { ok = false; break; }
         tc::tc_fence_after();
         if (ai == 0 && with_dv) {
-          tc::mma_ss2pe(tmem, pt_lo, pt_hi, o_lo, o_hi, idescA, acc_on);
-#pragma unroll
-          for (int k = 1; k < BR / 16; ++k)
-            tc::mma_ss2e<1>(tmem, pt_lo + (uint32_t)(2 * k * BK), pt_hi, o_lo + (uint32_t)(k * (2048 / 16)), o_hi, idescA);
+          tc::mma4_ss(tmem, pt_lo, pt_hi, 2 * BK, o_lo, o_hi, 2048 / 16, idescA, acc_on);
         }
         for (int gi = g_begin; gi < g_end; ++gi) {
           const bool pair = gi < pairs;
@@ -653,10 +663,7 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           const uint32_t dacc = tmem + 64 * (accb + i);
           const uint32_t b_lo = qm_lo + (uint32_t)((tap0 + i) * (128 >> 4));
           const uint32_t idg = pair ? idescA2 : idescA;
-          tc::mma_ss2pe(dacc, dc_lo, pt_hi, b_lo, qm_hi, idg, acc_on);
-#pragma unroll
-          for (int k = 1; k < BR / 16; ++k)
-            tc::mma_ss2e<1>(dacc, dc_lo + (uint32_t)(2 * k * BK), pt_hi, b_lo + (uint32_t)(k * (2048 / 16)), qm_hi, idg);
+          tc::mma4_ss(dacc, dc_lo, pt_hi, 2 * BK, b_lo, qm_hi, 2048 / 16, idg, acc_on);
         }
         tc::mma_commit_e(&empty[st]);
         tc::mma_commit_e(pdc_free);
@@ -683,11 +690,7 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     }
     for (int it = 0; it < nblk && ok; ++it) {
-      const int st = it % NSTG, ph = (it / NSTG) & 1;
       const int i0 = (qb_begin + it) * BR;
-      const float* ld = reinterpret_cast<const float*>(sStage + st * Cfg::STAGE_BYTES + Cfg::sgLD) + CW * cg;
-      ok = __all_sync(0xffffffffu, tc::mbar_wait(&full[st], ph, s_abort));
-      if (!ok) break;
       ok = __all_sync(0xffffffffu, tc::mbar_wait(st_full, it & 1, s_abort));
       if (!ok) break;
       tc::tc_fence_after();
@@ -706,14 +709,15 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tc::tc_fence_before();
         tc::mbar_arrive(xd_free);
       }
-      // P^T[key, i] = exp2(S^T - LSE_i), kept only where this kernel owns the entry; dC^T = P^T (dP^T - D_i)
+      // P^T[key, i] = exp2(S^T - LSE_i), kept only where this kernel owns the entry; dC^T = P^T (dP^T - D_i); the statistics
+      // are in S^T and dP^T already
       uint32_t pp[CW / 2], cc[CW / 2];
       if ((j0 + BK <= N) && (i0 + BR <= N) && (!p.causal || j0 + BK - 1 + band <= i0)) {   // block owned entirely
 #pragma unroll
         for (int c = 0; c < CW; c += 2) {
-          const float p0 = exp2f(s[c] - ld[c]), p1 = exp2f(s[c + 1] - ld[c + 1]);
+          const float p0 = exp2f(s[c]), p1 = exp2f(s[c + 1]);
           pp[c / 2] = pack_bf16(p0, p1);
-          cc[c / 2] = pack_bf16(p0 * (dpc[c] - ld[BR + c]), p1 * (dpc[c + 1] - ld[BR + c + 1]));
+          cc[c / 2] = pack_bf16(p0 * dpc[c], p1 * dpc[c + 1]);
         }
       } else {
 #pragma unroll
@@ -721,10 +725,10 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           const int gi = i0 + CW * cg + c;
           const bool own0 = (key < N) && (gi < N) && (!p.causal || key <= gi - band);
           const bool own1 = (key < N) && (gi + 1 < N) && (!p.causal || key <= gi + 1 - band);
-          const float p0 = own0 ? exp2f(s[c] - ld[c]) : 0.f;
-          const float p1 = own1 ? exp2f(s[c + 1] - ld[c + 1]) : 0.f;
+          const float p0 = own0 ? exp2f(s[c]) : 0.f;
+          const float p1 = own1 ? exp2f(s[c + 1]) : 0.f;
           pp[c / 2] = pack_bf16(p0, p1);
-          cc[c / 2] = pack_bf16(p0 * (dpc[c] - ld[BR + c]), p1 * (dpc[c + 1] - ld[BR + c + 1]));
+          cc[c / 2] = pack_bf16(p0 * dpc[c], p1 * dpc[c + 1]);
         }
       }
 #pragma unroll
