@@ -6,16 +6,18 @@
 // here keeps the query rows on the TMEM lanes for the scores (S = sum_a Q^(a) Kt_a^T, M = 128 rows, N = 64
 // keys):
 //
-//   bwd_dkdv_tc128_kernel : CTA = 64 keys, loops 128-row query blocks.  The c_q stacked key tiles and V
-//                           stay resident (112 KB).  The accumulators are kept TRANSPOSED, with the head
+//   bwd_dkdv_tc128_kernel : CTA = 64 keys, loops 128-row query blocks.  The accumulators are kept TRANSPOSED, with the head
 //                           dim on the lanes: dV^T[d, key] += dO^T P and dKt_a^T[d, key] += Q^(a)T dC are
 //                           M = 128 MMAs whose A operand is the staged dO / Q tile read MN-major (for Q
 //                           with the tap's row shift as a start-address offset of 128 bytes per row into
 //                           the 128-byte-swizzled tile) and whose B operand is the
 //                           bf16 P / dC tile exactly as the element-wise warps write it (one row per
 //                           thread).  dV^T + 6 dKt^T take 448 columns; S and dP share the last 64
-//                           (dP(0) | S(0) dP(1) | S(1) dP(2) ...), as in the d = 64 kernel.  Scores and dP
-//                           are computed once per entry: no second pass over the head dim.
+//                           (S(0) dP(0) | S(1) dP(1) | ...).  Scores and dP are computed once per entry.
+//   Four of the stacked key tiles stay resident; the others and V come again for every block through a ring of three 8 KB
+//   slabs, interleaved with the resident ones.  That is 48 KB per 128 x 64 block more from L2, and makes room for a second
+//   Q tile, so that S of the next block runs under the dKt MMAs of this one: with everything resident and one Q tile the
+//   block's load, S, element-wise part and dKt were one chain (tensor core 35 % busy, B 8, H 32, N 4096: 10.4 ms; now 9.4).
 // Every mbarrier wait is bounded; no TMA multicast, no cluster, cta_group::1 only.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -33,27 +35,28 @@ struct Dkv128Cfg {
   static constexpr int D = 128;
   static constexpr int BK = 64;                // keys per CTA (= columns of the transposed accumulators)
   static constexpr int BR = 128;               // query rows per block (= TMEM lanes of S and dP)
-  static constexpr int HALO = 16;
-  static constexpr int QR = BR + HALO;         // 144 rows of Q per block
-  static constexpr int MAXCQ = 6;              // resident Kt tiles
+  static constexpr int HALO = 8;               // pad_q <= 5
+  static constexpr int QR = BR + HALO;         // rows of Q per block
+  static constexpr int RES = 4;                // resident Kt tiles
+  static constexpr int NST = 3;                // slabs of the ring for the other Kt tiles and V
   static constexpr int SLAB_BYTES = BK * 128;  // 64 keys x 64 elements, 128-byte swizzle
   static constexpr int KT_BYTES = 2 * SLAB_BYTES;
   static constexpr int DO_SLAB = BR * 128;     // 128 rows x 64 elements, 128-byte swizzle
   static constexpr int oKt = 0;
-  static constexpr int oV = oKt + MAXCQ * KT_BYTES;
-  static constexpr int Q_SLAB = QR * 128;      // 144 rows x 64 elements, 128-byte swizzle
-  static constexpr int oQ = oV + KT_BYTES;                      // two slabs
-  static constexpr int odO = oQ + QR * D * 2;                   // two slabs
+  static constexpr int oSt = oKt + RES * KT_BYTES;
+  static constexpr int Q_SLAB = QR * 128;      // 136 rows x 64 elements, 128-byte swizzle
+  static constexpr int oQ = oSt + NST * SLAB_BYTES;             // two buffers of two slabs
+  static constexpr int odO = oQ + 4 * Q_SLAB;                   // two slabs
   static constexpr int oP = odO + 2 * DO_SLAB;                  // P  : [BK/8][BR][16 B]  (MN-major B operand)
   static constexpr int oDC = oP + (BK / 8) * BR * 16;           // dC : same layout
   static constexpr int oBar = oDC + (BK / 8) * BR * 16;
   static constexpr int kSmemBytes = oBar + 512 + 1024;
-  static_assert(odO % 1024 == 0 && oV % 1024 == 0 && oQ % 1024 == 0 && Q_SLAB % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
+  static_assert(odO % 1024 == 0 && oSt % 1024 == 0 && oQ % 1024 == 0 && Q_SLAB % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
   static_assert(kSmemBytes <= 227 * 1024, "dK/dV kernel (d = 128): shared memory budget");
   static constexpr int kTmemCols = 512;        // dV^T at 0, dKt_a^T at 64 (1 + a), scratch X (S / dP) at 448
   static constexpr int colX = 448;
   static constexpr int kEwWarps = 8;
-  static constexpr int kThreads = (kEwWarps + 4) * 32;   // + producer, issuer S, issuers A0 and A1
+  static constexpr int kThreads = (kEwWarps + 5) * 32;   // + issuer S, issuers A0 and A1, two producers
 };
 
 __global__ void __launch_bounds__(Dkv128Cfg::kThreads, 1)
@@ -65,28 +68,34 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* sKt = smem + Cfg::oKt;
-  unsigned char* sV = smem + Cfg::oV;
+  unsigned char* sSt = smem + Cfg::oSt;
   unsigned char* sQ = smem + Cfg::oQ;
   unsigned char* sdO = smem + Cfg::odO;
+  constexpr int NST = Cfg::NST;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::oBar);
-  uint64_t* kv_full = bars;
-  uint64_t* q_full = kv_full + 1;        // Q of the block staged
-  uint64_t* q_free = q_full + 1;         // the three issuers are done with it (3 commits)
-  uint64_t* do_full = q_free + 1;        // dO of the block staged
+  uint64_t* st_full = bars;              // [NST] slab of the ring staged
+  uint64_t* st_empty = st_full + NST;    // [NST] slab read
+  uint64_t* kt_full = st_empty + NST;    // resident Kt tiles staged
+  uint64_t* q_full = kt_full + 1;        // [2] Q of the block staged
+  uint64_t* q_free = q_full + 2;         // [2] the three issuers are done with it (3 commits)
+  uint64_t* do_full = q_free + 2;        // dO of the block staged
   uint64_t* do_free = do_full + 1;       // dP and dV^T of the block have read it (2 commits)
-  uint64_t* st_full = do_free + 1;       // S in X
-  uint64_t* xs_free = st_full + 1;       // S taken into registers (256 arrivals): X free for the next dP
-  uint64_t* dpt_full = xs_free + 1;      // dP in X
-  uint64_t* xd_free = dpt_full + 1;      // dP taken into registers (256 arrivals): X free for S
-  uint64_t* pdc_full = xd_free + 1;      // P and dC (bf16) written to shared memory (256 arrivals)
-  uint64_t* pdc_free = pdc_full + 1;     // the dV^T / dKt^T MMAs that read them have completed (2 commits)
-  uint64_t* all_done = pdc_free + 1;
+  uint64_t* s_full = do_free + 1;        // S in X
+  uint64_t* xs_free = s_full + 1;        // S taken into registers (256 arrivals): X free for dP
+  uint64_t* dp_full = xs_free + 1;       // dP in X
+  uint64_t* xd_free = dp_full + 1;       // dP taken into registers (256 arrivals): X free for the next S
+  uint64_t* p_full = xd_free + 1;        // P (bf16) written to shared memory (256 arrivals)
+  uint64_t* p_free = p_full + 1;         // the dV^T MMAs that read it have completed
+  uint64_t* dc_full = p_free + 1;        // dC (bf16) written to shared memory (256 arrivals)
+  uint64_t* dc_free = dc_full + 1;       // the dKt^T MMAs that read it have completed (2 commits)
+  uint64_t* all_done = dc_free + 1;
   uint64_t* never_bar = all_done + 1;
   uint64_t* mma_drain = never_bar + 1;
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(mma_drain + 1);
   volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
-  volatile int* s_q_issued = s_abort + 1;    // blocks whose Q / dO copies the producer has issued
+  volatile int* s_q_issued = s_abort + 1;    // blocks whose Q / dO copies, slabs whose copies the producers have issued
   volatile int* s_do_issued = s_abort + 2;
+  volatile int* s_st_issued = s_abort + 3;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int N = p.N, cq = p.cq, pq = cq - 1, pk = (p.ck - 1) / 2;
@@ -100,18 +109,20 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const int nblk = nQB - qb_begin;
 
   if (tid == 0) {
-    tc::mbar_init(kv_full, 1);
-    tc::mbar_init(q_full, 1); tc::mbar_init(q_free, 3);
+    for (int i = 0; i < NST; ++i) { tc::mbar_init(&st_full[i], 1); tc::mbar_init(&st_empty[i], 1); }
+    tc::mbar_init(kt_full, 1);
+    for (int i = 0; i < 2; ++i) { tc::mbar_init(&q_full[i], 1); tc::mbar_init(&q_free[i], 3); }
     tc::mbar_init(do_full, 1); tc::mbar_init(do_free, 2);
-    tc::mbar_init(st_full, 1); tc::mbar_init(xs_free, Cfg::kEwWarps * 32);
-    tc::mbar_init(dpt_full, 1); tc::mbar_init(xd_free, Cfg::kEwWarps * 32);
-    tc::mbar_init(pdc_full, Cfg::kEwWarps * 32); tc::mbar_init(pdc_free, 2);
+    tc::mbar_init(s_full, 1); tc::mbar_init(xs_free, Cfg::kEwWarps * 32);
+    tc::mbar_init(dp_full, 1); tc::mbar_init(xd_free, Cfg::kEwWarps * 32);
+    tc::mbar_init(p_full, Cfg::kEwWarps * 32); tc::mbar_init(p_free, 1);
+    tc::mbar_init(dc_full, Cfg::kEwWarps * 32); tc::mbar_init(dc_free, 2);
     tc::mbar_init(all_done, 2);
     tc::mbar_init(never_bar, 1); tc::mbar_init(mma_drain, 3);
-    *s_abort = 0; *s_q_issued = 0; *s_do_issued = 0;
+    *s_abort = 0; *s_q_issued = 0; *s_do_issued = 0; *s_st_issued = 0;
     tc::mbar_fence_init();
   }
-  if (warp == Cfg::kEwWarps + 1) {
+  if (warp == Cfg::kEwWarps) {
     tc::tmem_alloc(s_tmem, Cfg::kTmemCols);
     tc::tmem_relinquish();
   }
@@ -122,101 +133,119 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const uint32_t tmem = *s_tmem;
   const uint32_t tX = tmem + Cfg::colX;
 
-  if (warp == Cfg::kEwWarps) {
-    // ===================== producer warp (TMA) =====================
-    if (nblk > 0) {
-      if (lane == 0) {
-        tc::tma_prefetch_desc(&tmQ); tc::tma_prefetch_desc(&tmdO); tc::tma_prefetch_desc(&tmKt); tc::tma_prefetch_desc(&tmV);
-        tc::mbar_expect_tx(kv_full, (cq + 1) * Cfg::KT_BYTES);
-        for (int a = 0; a < cq; ++a) {
-          tc::tma_load_3d(sKt + a * Cfg::KT_BYTES, &tmKt, kv_full, 0, j0, bh * cq + a);
-          tc::tma_load_3d(sKt + a * Cfg::KT_BYTES + Cfg::SLAB_BYTES, &tmKt, kv_full, 64, j0, bh * cq + a);
-        }
-        tc::tma_load_3d(sV, &tmV, kv_full, 0, j0, bh);
-        tc::tma_load_3d(sV + Cfg::SLAB_BYTES, &tmV, kv_full, 64, j0, bh);
-      }
-      bool ok = true;
-      for (int it = 0; it < nblk && ok; ++it) {
+  const int role = warp - Cfg::kEwWarps;       // 0: issuer S, 1, 2: issuers A0, A1, 3: producer of Kt, Q and dO, 4: of the ring
+  const int nres = min(cq, Cfg::RES);
+
+  if (role == 3) {
+    if (nblk > 0 && lane == 0) {
+      tc::tma_prefetch_desc(&tmQ); tc::tma_prefetch_desc(&tmdO); tc::tma_prefetch_desc(&tmKt);
+      auto load_q = [&](int it) {
+        uint64_t* bar = &q_full[it & 1];
+        unsigned char* dst = sQ + (it & 1) * (2 * Cfg::Q_SLAB);
         const int i0 = (qb_begin + it) * BR;
-        // ---- dO of block `it` (its buffer is free once dP and dV^T of block it-1 are done) ----
-        if (it > 0) {
-          ok = __all_sync(0xffffffffu, tc::mbar_wait(do_free, (it - 1) & 1, s_abort));
-          if (!ok) break;
-        }
-        if (lane == 0) {
-          tc::mbar_expect_tx(do_full, 2 * Cfg::DO_SLAB);
-          tc::tma_load_3d(sdO, &tmdO, do_full, 0, i0, bh);
-          tc::tma_load_3d(sdO + Cfg::DO_SLAB, &tmdO, do_full, 64, i0, bh);
-          *s_do_issued = it + 1;
-        }
-        // ---- Q of block `it` (free once S and every dKt^T tap of block it-1 are done) ----
-        if (it > 0) {
-          ok = __all_sync(0xffffffffu, tc::mbar_wait(q_free, (it - 1) & 1, s_abort));
-          if (!ok) break;
-        }
-        if (lane == 0) {
-          tc::mbar_expect_tx(q_full, QR * D * 2);
-          tc::tma_load_3d(sQ, &tmQ, q_full, 0, i0 - HALO, bh);
-          tc::tma_load_3d(sQ + Cfg::Q_SLAB, &tmQ, q_full, 64, i0 - HALO, bh);
-          *s_q_issued = it + 1;
+        tc::mbar_expect_tx(bar, QR * D * 2);
+        tc::tma_load_3d(dst, &tmQ, bar, 0, i0 - HALO, bh);
+        tc::tma_load_3d(dst + Cfg::Q_SLAB, &tmQ, bar, 64, i0 - HALO, bh);
+        *s_q_issued = it + 1;
+      };
+      load_q(0);
+      tc::mbar_expect_tx(kt_full, nres * Cfg::KT_BYTES);
+      for (int a = 0; a < nres; ++a) {
+        tc::tma_load_3d(sKt + a * Cfg::KT_BYTES, &tmKt, kt_full, 0, j0, bh * cq + a);
+        tc::tma_load_3d(sKt + a * Cfg::KT_BYTES + Cfg::SLAB_BYTES, &tmKt, kt_full, 64, j0, bh * cq + a);
+      }
+      for (int it = 0; it < nblk; ++it) {
+        const int i0 = (qb_begin + it) * BR;
+        if (it > 0 && !tc::mbar_wait(do_free, (it - 1) & 1, s_abort)) break;                     // dP and dV of block it-1
+        tc::mbar_expect_tx(do_full, 2 * Cfg::DO_SLAB);
+        tc::tma_load_3d(sdO, &tmdO, do_full, 0, i0, bh);
+        tc::tma_load_3d(sdO + Cfg::DO_SLAB, &tmdO, do_full, 64, i0, bh);
+        *s_do_issued = it + 1;
+        if (it + 1 < nblk) {
+          if (it > 0 && !tc::mbar_wait(&q_free[(it + 1) & 1], ((it - 1) >> 1) & 1, s_abort)) break;   // everything of block it-1
+          load_q(it + 1);
         }
       }
     }
-  } else if (warp == Cfg::kEwWarps + 1) {
-    // ===================== MMA issuer S: dP and S of block `it` into the scratch columns X ==========
-    if (nblk > 0) {   // all lanes run the loop; one elected lane issues (see tc::elect_one)
+  } else if (role == 4) {
+    // the ring, in the order of the issuer: the slabs of the taps that are not resident, then V
+    if (nblk > 0 && lane == 0) {
+      tc::tma_prefetch_desc(&tmV);
+      const int per = 2 * (cq - nres) + 2;
+      int slot = 0, ph = 1, id = 0;
+      bool ok = true;
+      for (int it = 0; it < nblk && ok; ++it)
+        for (int i = 0; i < per; ++i) {
+          if (!(ok = tc::mbar_wait(&st_empty[slot], ph, s_abort))) break;
+          tc::mbar_expect_tx(&st_full[slot], Cfg::SLAB_BYTES);
+          const bool is_v = i >= per - 2;
+          tc::tma_load_3d(sSt + slot * Cfg::SLAB_BYTES, is_v ? &tmV : &tmKt, &st_full[slot], (i & 1) * 64, j0, is_v ? bh : bh * cq + nres + (i >> 1));
+          if (++slot == NST) { slot = 0; ph ^= 1; }
+          *s_st_issued = ++id;
+        }
+    }
+  } else if (role == 0) {
+    // ===================== MMA issuer S: S and dP of block `it` into the scratch columns X =====================
+    if (nblk > 0) {   // all lanes run the loop; one elected lane issues
       constexpr uint32_t idescT = tc::make_idesc(BR, BK, 0, 0);    // 128 x 64, K-major operands
       const uint64_t dKtB = tc::make_sdesc(smem_u32(sKt), 16, 1024, tc::kLayoutSW128);
-      const uint32_t kt_hi = (uint32_t)(dKtB >> 32), kt_lo = (uint32_t)dKtB;
-      const uint32_t v_lo = kt_lo + (uint32_t)((Cfg::oV - Cfg::oKt) >> 4);
-      const uint64_t dOk = tc::make_sdesc(smem_u32(sdO), 16, 1024, tc::kLayoutSW128);
-      const uint32_t o_lo = (uint32_t)dOk;                         // same high word as the Kt tiles
+      const uint32_t hi = (uint32_t)(dKtB >> 32), kt_lo = (uint32_t)dKtB;
+      const uint32_t ring_lo = kt_lo + (uint32_t)((Cfg::oSt - Cfg::oKt) >> 4), o_lo = kt_lo + (uint32_t)((Cfg::odO - Cfg::oKt) >> 4);
       // Q^(a), K-major: the same swizzled tile with the start address moved down by the tap's row shift.  The
       // tensor core applies the 128-byte swizzle to the absolute shared-memory address, exactly as TMA did when
       // it wrote the tile, so a start that is a multiple of 128 bytes (not of the 1024-byte pattern) reads the
       // shifted rows correctly.
-      const uint64_t dQk = tc::make_sdesc(smem_u32(sQ) + (HALO - pq) * 128, 16, 1024, tc::kLayoutSW128);
-      const uint32_t qk_lo = (uint32_t)dQk;                        // same high word as the Kt tiles
-      bool ok = tc::mbar_wait_warp(kv_full, 0, s_abort);
-      // X holds dP(it) first (taken into registers by the element-wise warps), then S(it):
-      //   dP(0) | S(0) dP(1) | S(1) dP(2) | ...
-      auto issue_dP = [&](int it) {
-        if (!tc::mbar_wait_warp(do_full, it & 1, s_abort)) { ok = false; return; }
+      const uint32_t q_lo0 = kt_lo + (uint32_t)((Cfg::oQ - Cfg::oKt + (HALO - pq) * 128) >> 4);
+      int slot = 0, ph = 0;
+      bool ok = tc::mbar_wait_warp(kt_full, 0, s_abort);
+      bool ready = false;                                          // the ring's next slab was seen staged (a wait that is
+                                                                   // over already costs 200 cycles)
+      auto slab = [&](uint32_t a_lo, uint32_t acc) {               // 64 contraction columns against the ring's next slab
+        if (!ready && !(ok = tc::mbar_wait_warp(&st_full[slot], ph, s_abort))) return;
         tc::tc_fence_after();
-        tc::mma_ss2e<0>(tX, o_lo, kt_hi, v_lo, kt_hi, idescT);               // dP = dO V^T
-#pragma unroll
-        for (int k = 1; k < D / 16; ++k)
-          tc::mma_ss2e<1>(tX, o_lo + (uint32_t)((k >> 2) * (Cfg::DO_SLAB >> 4) + (k & 3) * 2), kt_hi,
-                          v_lo + (uint32_t)((k >> 2) * (Cfg::SLAB_BYTES >> 4) + (k & 3) * 2), kt_hi, idescT);
-        tc::mma_commit_e(dpt_full);
-        tc::mma_commit_e(do_free);
+        const int ns = slot + 1 == NST ? 0 : slot + 1, nph = ns == 0 ? ph ^ 1 : ph;
+        const uint32_t seen = tc::mbar_test(&st_full[ns], nph);
+        tc::mma4_ss(tX, a_lo, hi, 2, ring_lo + (uint32_t)(slot * (Cfg::SLAB_BYTES >> 4)), hi, 2, idescT, acc);
+        tc::mma_commit_e(&st_empty[slot]);
+        slot = ns; ph = nph;
+        ready = __all_sync(0xffffffffu, seen);
       };
-      if (ok) issue_dP(0);
       for (int it = 0; it < nblk && ok; ++it) {
-        if (!tc::mbar_wait_warp(q_full, it & 1, s_abort)) { ok = false; break; }
-        if (!tc::mbar_wait_warp(xd_free, it & 1, s_abort)) { ok = false; break; }   // dP(it) has left X
+        ok = tc::mbar_wait_warp(&q_full[it & 1], (it >> 1) & 1, s_abort);
+        if (ok && it > 0) ok = tc::mbar_wait_warp(xd_free, (it - 1) & 1, s_abort);       // dP(it-1) has left X
+        if (!ok) break;
         tc::tc_fence_after();
-        // S = sum_a Q^(a) Kt_a^T
-        for (int a = 0; a < cq; ++a) {
-          const uint32_t b_lo = kt_lo + (uint32_t)(a * (Cfg::KT_BYTES >> 4));
-          const uint32_t a_lo = qk_lo + (uint32_t)(a * (128 >> 4));       // row shift = +128 B per row
-          tc::mma_ss2pe(tX, a_lo, kt_hi, b_lo, kt_hi, idescT, a != 0);
+        // S = sum_a Q^(a) Kt_a^T: one slab of the ring, two resident ones, ...
+        const uint32_t q_lo = q_lo0 + (uint32_t)((it & 1) * (2 * Cfg::Q_SLAB >> 4));
+        const int ns = 2 * (cq - nres), nr = 2 * nres;
+        for (int i = 0; i < max(ns, nres) && ok; ++i) {
+          if (i < ns) slab(q_lo + (uint32_t)((i & 1) * (Cfg::Q_SLAB >> 4) + (nres + (i >> 1)) * (128 >> 4)), i != 0);
+          if (!ok) break;
+          if (2 * i < nr) {
 #pragma unroll
-          for (int k = 1; k < D / 16; ++k)
-            tc::mma_ss2e<1>(tX, a_lo + (uint32_t)((k >> 2) * (Cfg::Q_SLAB >> 4) + (k & 3) * 2), kt_hi,
-                            b_lo + (uint32_t)((k >> 2) * (Cfg::SLAB_BYTES >> 4) + (k & 3) * 2), kt_hi, idescT);
+            for (int sl = 0; sl < 2; ++sl)
+              tc::mma4_ss(tX, q_lo + (uint32_t)(sl * (Cfg::Q_SLAB >> 4) + i * (128 >> 4)), hi, 2,
+                          kt_lo + (uint32_t)((i * Cfg::KT_BYTES + sl * Cfg::SLAB_BYTES) >> 4), hi, 2, idescT, ns > 0 || i + sl != 0);
+          }
         }
-        tc::mma_commit_e(st_full);
-        tc::mma_commit_e(q_free);
-        if (!tc::mbar_wait_warp(xs_free, it & 1, s_abort)) { ok = false; break; }   // S(it) has left X
+        if (!ok) break;
+        tc::mma_commit_e(s_full);
+        tc::mma_commit_e(&q_free[it & 1]);
+        ok = tc::mbar_wait_warp(xs_free, it & 1, s_abort);                               // S(it) has left X
+        if (ok) ok = tc::mbar_wait_warp(do_full, it & 1, s_abort);
+        if (!ok) break;
         tc::tc_fence_after();
-        if (it + 1 < nblk) issue_dP(it + 1);
+        slab(o_lo, 0);                                                                   // dP = dO V^T
+        if (ok) slab(o_lo + (uint32_t)(Cfg::DO_SLAB >> 4), 1);
+        if (!ok) break;
+        tc::mma_commit_e(dp_full);
+        tc::mma_commit_e(do_free);
       }
     }
-  } else if (warp >= Cfg::kEwWarps + 2) {
+  } else if (role > 0) {
     // ===================== MMA issuers A0 / A1: dV^T += dO^T P ; dKt_a^T += Q^(a)T dC =====================
-    const int ai = warp - (Cfg::kEwWarps + 2);
-    if (nblk > 0) {   // all lanes run the loop; one elected lane issues (see tc::elect_one)
+    const int ai = role - 1;
+    if (nblk > 0) {   // all lanes run the loop; one elected lane issues
       constexpr uint32_t idescA = tc::make_idesc(D, BK, 1, 1);     // 128 (head dim) x 64 (keys), both operands MN-major
       // A0 takes dV^T and the first half of the taps, A1 the rest
       const int ntap = p.ntap, accb = p.with_dv ? 1 : 0;
@@ -228,36 +257,35 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       const uint64_t dQm = tc::make_sdesc(smem_u32(sQ) + (HALO - pq) * 128, Cfg::Q_SLAB, 1024, tc::kLayoutSW128);
       // P / dC: N = keys in 8-key chunks BR * 16 bytes apart, K = rows 16 bytes apart
       const uint64_t dPb = tc::make_sdesc(smem_u32(smem + Cfg::oP), 128, BR * 16, tc::kLayoutNone);
-      const uint64_t dCb = tc::make_sdesc(smem_u32(smem + Cfg::oDC), 128, BR * 16, tc::kLayoutNone);
       const uint32_t om_hi = (uint32_t)(dOm >> 32), om_lo = (uint32_t)dOm;
-      const uint32_t qm_hi = (uint32_t)(dQm >> 32), qm_lo = (uint32_t)dQm;
-      const uint32_t pb_hi = (uint32_t)(dPb >> 32), pb_lo = (uint32_t)dPb, cb_lo = (uint32_t)dCb;
+      const uint32_t qm_hi = (uint32_t)(dQm >> 32), qm_lo0 = (uint32_t)dQm;
+      const uint32_t pb_hi = (uint32_t)(dPb >> 32), pb_lo = (uint32_t)dPb, cb_lo = pb_lo + (uint32_t)((Cfg::oDC - Cfg::oP) >> 4);
+      auto mma8 = [&](uint32_t dst, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t acc) {       // 128 rows
+        tc::mma4_ss(dst, a_lo, a_hi, 2048 / 16, b_lo, pb_hi, 16, idescA, acc);
+        tc::mma4_ss(dst, a_lo + 4 * (2048 / 16), a_hi, 2048 / 16, b_lo + 4 * 16, pb_hi, 16, idescA, 1);
+      };
       bool ok = true;
       for (int it = 0; it < nblk && ok; ++it) {
         const uint32_t acc_on = it != 0;
-        if (!tc::mbar_wait_warp(q_full, it & 1, s_abort)) { ok = false; break; }
-        if (ai == 0 && !tc::mbar_wait_warp(do_full, it & 1, s_abort)) { ok = false; break; }
-        if (!tc::mbar_wait_warp(pdc_full, it & 1, s_abort)) { ok = false; break; }
-        tc::tc_fence_after();
         if (ai == 0) {
-          if (p.with_dv) {
-            tc::mma_ss2pe(tmem, om_lo, om_hi, pb_lo, pb_hi, idescA, acc_on);
-#pragma unroll
-            for (int k = 1; k < BR / 16; ++k)
-              tc::mma_ss2e<1>(tmem, om_lo + (uint32_t)(k * (2048 / 16)), om_hi, pb_lo + (uint32_t)(k * 16), pb_hi, idescA);
-          }
+          ok = tc::mbar_wait_warp(do_full, it & 1, s_abort) && tc::mbar_wait_warp(p_full, it & 1, s_abort);
+          if (!ok) break;
+          tc::tc_fence_after();
+          if (p.with_dv) mma8(tmem, om_lo, om_hi, pb_lo, acc_on);
           tc::mma_commit_e(do_free);
+          tc::mma_commit_e(p_free);
         }
-        for (int i = t_begin; i < t_end; ++i) {
-          const uint32_t dacc = tmem + 64 * (accb + i);
-          const uint32_t a_lo = qm_lo + (uint32_t)(i * (128 >> 4));     // K (row) shift = +128 B per row
-          tc::mma_ss2pe(dacc, a_lo, qm_hi, cb_lo, pb_hi, idescA, acc_on);
-#pragma unroll
-          for (int k = 1; k < BR / 16; ++k)
-            tc::mma_ss2e<1>(dacc, a_lo + (uint32_t)(k * (2048 / 16)), qm_hi, cb_lo + (uint32_t)(k * 16), pb_hi, idescA);
-        }
-        tc::mma_commit_e(q_free);
-        tc::mma_commit_e(pdc_free);
+        ok = tc::mbar_wait_warp(&q_full[it & 1], (it >> 1) & 1, s_abort) && tc::mbar_wait_warp(dc_full, it & 1, s_abort);
+        if (!ok) break;
+        tc::tc_fence_after();
+        const uint32_t qm_lo = qm_lo0 + (uint32_t)((it & 1) * (2 * Cfg::Q_SLAB >> 4));
+        // A1's taps go behind S of the next block, which would otherwise share the tensor core with all of them from its
+        // first MMA on and end with nothing left to run while it is taken out of X
+        if (ai == 1 && it + 1 < nblk && !tc::mbar_wait_warp(s_full, (it + 1) & 1, s_abort)) { ok = false; break; }
+        for (int i = t_begin; i < t_end; ++i)
+          mma8(tmem + 64 * (accb + i), qm_lo + (uint32_t)(i * (128 >> 4)), qm_hi, cb_lo, acc_on);        // K (row) shift = +128 B per row
+        tc::mma_commit_e(&q_free[it & 1]);
+        tc::mma_commit_e(dc_free);
       }
       if (ok) tc::mma_commit_e(all_done);
     }
@@ -269,22 +297,11 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const uint32_t lane_base = (uint32_t)(qtr * 32) << 16;
     const uint32_t tXl = tX + lane_base + CW * cg;
     bool ok = true;
-    float dpc[CW];                                      // dP of the block about to be processed
     // every thread fetches the statistics of its own row (LSE in log2 units, D), one block ahead
     float lse2 = 0.f, dvec = 0.f;
     if (nblk > 0) {
       const int gi = qb_begin * BR + row;
       if (gi < N) { lse2 = p.LSE[(size_t)bh * N + gi] * kLog2e; dvec = p.Dvec[(size_t)bh * N + gi]; }
-    }
-    if (nblk > 0) {
-      ok = __all_sync(0xffffffffu, p.selftest_expire ? tc::mbar_wait(never_bar, 0, s_abort, tc::kSelfTestSpinLimit)
-                                                     : tc::mbar_wait(dpt_full, 0, s_abort));
-      if (ok) {
-        tc::tc_fence_after();
-        tc::tmem_ldn(tXl, dpc);
-        tc::tc_fence_before();
-        tc::mbar_arrive(xd_free);
-      }
     }
     for (int it = 0; it < nblk && ok; ++it) {
       const int i0 = (qb_begin + it) * BR;
@@ -294,7 +311,8 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         lse2_next = p.LSE[(size_t)bh * N + gi + BR] * kLog2e;
         dvec_next = p.Dvec[(size_t)bh * N + gi + BR];
       }
-      ok = __all_sync(0xffffffffu, tc::mbar_wait(st_full, it & 1, s_abort));
+      ok = __all_sync(0xffffffffu, (p.selftest_expire && it == 0) ? tc::mbar_wait(never_bar, 0, s_abort, tc::kSelfTestSpinLimit)
+                                                                  : tc::mbar_wait(s_full, it & 1, s_abort));
       if (!ok) break;
       tc::tc_fence_after();
       float s[CW];
@@ -302,50 +320,47 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       tc::tc_fence_before();
       tc::mbar_arrive(xs_free);
       // P[i, key] = exp2(S - LSE_i), kept only where this kernel owns the entry; dC = P (dP - D_i)
-      uint32_t pp[CW / 2], cc[CW / 2];
+      uint32_t pp[CW / 2];
       const int kbase = j0 + CW * cg;
       if ((j0 + BK <= N) && (i0 + BR <= N) && (!p.causal || j0 + BK - 1 + band <= i0)) {   // block owned entirely
 #pragma unroll
-        for (int c = 0; c < CW; c += 2) {
-          const float p0 = exp2f(s[c] - lse2), p1 = exp2f(s[c + 1] - lse2);
-          pp[c / 2] = pack_bf16(p0, p1);
-          cc[c / 2] = pack_bf16(p0 * (dpc[c] - dvec), p1 * (dpc[c + 1] - dvec));
-        }
+        for (int c = 0; c < CW; ++c) s[c] = exp2f(s[c] - lse2);
       } else {
         const int jlim = (gi < N) ? (p.causal ? min(N - 1, gi - band) : N - 1) : -1;   // last key this row owns here
 #pragma unroll
-        for (int c = 0; c < CW; c += 2) {
-          const float p0 = (kbase + c <= jlim) ? exp2f(s[c] - lse2) : 0.f;
-          const float p1 = (kbase + c + 1 <= jlim) ? exp2f(s[c + 1] - lse2) : 0.f;
-          pp[c / 2] = pack_bf16(p0, p1);
-          cc[c / 2] = pack_bf16(p0 * (dpc[c] - dvec), p1 * (dpc[c + 1] - dvec));
-        }
+        for (int c = 0; c < CW; ++c) s[c] = (kbase + c <= jlim) ? exp2f(s[c] - lse2) : 0.f;
       }
-      if (it > 0) {   // the MMAs of block it-1 have finished reading the P / dC buffers
-        ok = __all_sync(0xffffffffu, tc::mbar_wait(pdc_free, (it - 1) & 1, s_abort));
-        if (!ok) break;
-      }
-      {
-        unsigned char* pt = smem + Cfg::oP + row * 16;
-        unsigned char* dc = smem + Cfg::oDC + row * 16;
 #pragma unroll
-        for (int q4 = 0; q4 < CW / 8; ++q4) {          // 8 keys (16 bytes) per chunk
-          *reinterpret_cast<uint4*>(pt + ((CW / 8) * cg + q4) * (BR * 16)) = make_uint4(pp[4 * q4], pp[4 * q4 + 1], pp[4 * q4 + 2], pp[4 * q4 + 3]);
-          *reinterpret_cast<uint4*>(dc + ((CW / 8) * cg + q4) * (BR * 16)) = make_uint4(cc[4 * q4], cc[4 * q4 + 1], cc[4 * q4 + 2], cc[4 * q4 + 3]);
-        }
-      }
-      tc::fence_proxy_async_smem();
-      tc::mbar_arrive(pdc_full);
-      // dP of the next block: its dO is staged once dV^T of this block has read the buffer, which in turn
-      // waits for the P tile just written -- so it can only be taken out of X here, not earlier
-      if (it + 1 < nblk) {
-        ok = __all_sync(0xffffffffu, tc::mbar_wait(dpt_full, (it + 1) & 1, s_abort));
+      for (int c = 0; c < CW; c += 2) pp[c / 2] = pack_bf16(s[c], s[c + 1]);
+      if (it > 0) {   // dV^T of block it-1 has finished reading P
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(p_free, (it - 1) & 1, s_abort));
         if (!ok) break;
-        tc::tc_fence_after();
-        tc::tmem_ldn(tXl, dpc);
-        tc::tc_fence_before();
-        tc::mbar_arrive(xd_free);
       }
+      unsigned char* pt = smem + Cfg::oP + row * 16;
+      unsigned char* dc = smem + Cfg::oDC + row * 16;
+#pragma unroll
+      for (int q4 = 0; q4 < CW / 8; ++q4)            // 8 keys (16 bytes) per chunk
+        *reinterpret_cast<uint4*>(pt + ((CW / 8) * cg + q4) * (BR * 16)) = make_uint4(pp[4 * q4], pp[4 * q4 + 1], pp[4 * q4 + 2], pp[4 * q4 + 3]);
+      tc::fence_proxy_async_smem();
+      tc::mbar_arrive(p_full);
+      ok = __all_sync(0xffffffffu, tc::mbar_wait(dp_full, it & 1, s_abort));
+      if (!ok) break;
+      tc::tc_fence_after();
+      float dp[CW];
+      tc::tmem_ldn(tXl, dp);
+      tc::tc_fence_before();
+      tc::mbar_arrive(xd_free);
+#pragma unroll
+      for (int c = 0; c < CW; c += 2) pp[c / 2] = pack_bf16(s[c] * (dp[c] - dvec), s[c + 1] * (dp[c + 1] - dvec));
+      if (it > 0) {   // dKt^T of block it-1 has finished reading dC
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(dc_free, (it - 1) & 1, s_abort));
+        if (!ok) break;
+      }
+#pragma unroll
+      for (int q4 = 0; q4 < CW / 8; ++q4)
+        *reinterpret_cast<uint4*>(dc + ((CW / 8) * cg + q4) * (BR * 16)) = make_uint4(pp[4 * q4], pp[4 * q4 + 1], pp[4 * q4 + 2], pp[4 * q4 + 3]);
+      tc::fence_proxy_async_smem();
+      tc::mbar_arrive(dc_full);
       lse2 = lse2_next; dvec = dvec_next;
     }
     // ---- epilogue: the accumulators hold dV^T and dKt_a^T (lane = head dim, column = key); chunks of 32
@@ -407,20 +422,21 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   if (*s_abort) {
     if (tid == 0) atomicExch(p.status, 1);
     // MMAs and copies of this CTA are waited for (bounded) before its memories go
-    if (warp > Cfg::kEwWarps) tc::mma_commit_e(mma_drain);
-    if (tid == Cfg::kEwWarps * 32) {
+    if (role >= 0 && role < 3) tc::mma_commit_e(mma_drain);
+    if (role == 3 && lane == 0) {
       volatile int never = 0;
       if (nblk > 0) {
-        tc::mbar_wait(kv_full, 0, &never);
-        const int qi = *s_q_issued, di = *s_do_issued;
-        if (qi > 0) tc::mbar_wait(q_full, (qi - 1) & 1, &never);
+        const int qi = *s_q_issued, di = *s_do_issued, si = *s_st_issued;
+        tc::mbar_wait(kt_full, 0, &never);
+        for (int it = max(0, qi - 2); it < qi; ++it) tc::mbar_wait(&q_full[it & 1], (it >> 1) & 1, &never);
         if (di > 0) tc::mbar_wait(do_full, (di - 1) & 1, &never);
+        for (int id = max(0, si - NST); id < si; ++id) tc::mbar_wait(&st_full[id % NST], (id / NST) & 1, &never);
       }
       tc::mbar_wait(mma_drain, 0, &never);
     }
     __syncthreads();
   }
-  if (warp == Cfg::kEwWarps + 1) {
+  if (warp == Cfg::kEwWarps) {
     tc::tc_fence_after();
     tc::tmem_dealloc(tmem, Cfg::kTmemCols);
   }
