@@ -231,8 +231,8 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (!ok) break;
         tc::mma_commit_e(s_full);
         tc::mma_commit_e(&q_free[it & 1]);
-        ok = tc::mbar_wait_warp(xs_free, it & 1, s_abort);                               // S(it) has left X
-        if (ok) ok = tc::mbar_wait_warp(do_full, it & 1, s_abort);
+        ok = tc::mbar_wait_warp(do_full, it & 1, s_abort);
+        if (ok) ok = tc::mbar_wait_warp(xs_free, it & 1, s_abort);                       // S(it) has left X
         if (!ok) break;
         tc::tc_fence_after();
         slab(o_lo, 0);                                                                   // dP = dO V^T
