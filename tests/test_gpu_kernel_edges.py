@@ -4,7 +4,7 @@ import math
 import pytest
 import torch
 
-from helpers import TOL_BF16, maxabs
+from helpers import check_outputs, maxabs
 from oracle import conv_attn_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -42,3 +42,75 @@ def test_decode_blocks_splits_and_filters(B, H, q_len, Nk, d, cq, ck, k_splits, 
     Op, Mp, Lp = F.forward_inference_paged(q, pool[0], pool[1], table, theta.cuda(), k_splits, scale, cq - 1, (ck - 1) // 2,
                                            max_seq_len=Nk, offset_causal=offset_causal)
     assert torch.equal(Op[:, :, 0:1], O) and torch.equal(Mp[:, :, 0:1], M) and torch.equal(Lp[:, :, 0:1], L)
+
+
+@pytest.mark.parametrize("B,H,N,d,cq,ck,causal", [
+    (1, 2, 123, 64, 6, 11, True),      # one row tile of the dQ pair, exactly (128 - 5)
+    (1, 2, 247, 64, 6, 11, True),      # two tiles of it and one row
+    (1, 1, 256, 128, 6, 11, True),     # one pair of the forward, two key blocks
+    (1, 2, 257, 128, 5, 9, False),     # one row and one key past them; one tap streamed
+    (2, 1, 129, 128, 4, 5, True),      # every tap resident
+    (1, 1, 385, 128, 1, 3, True),      # one tap: no row shift, shortest contraction
+    (1, 2, 640, 64, 7, 7, True),       # seven taps: two passes of dK/dV
+    (1, 3, 500, 64, 2, 17, False),     # widest filter row, ragged key blocks
+    (1, 2, 383, 32, 3, 3, True),       # padded head dim
+])
+@pytest.mark.parametrize("fp32_inputs", [False, True])
+def test_training_tiles_and_taps(B, H, N, d, cq, ck, causal, fp32_inputs):
+    import fmta_b200 as F
+    Q, K, V, dO, theta = orc.make_inputs(B, H, N, d, cq, ck, seed=N + d + cq, theta_std=0.05, dtype=torch.bfloat16)
+    scale = 1.0 / math.sqrt(d)
+    O, _, _ = orc.conv_attn_fwd(Q, K, V, theta, scale, causal)
+    dQ, dK, dV, dTh = orc.conv_attn_bwd_autograd(Q, K, V, theta, dO, scale, causal)
+    layer = F.ConvAttentionCUDA(H, cq, ck, init_random=False).to("cuda")
+    with torch.no_grad():
+        layer.conv_weight.copy_(theta)
+    dt = torch.float32 if fp32_inputs else torch.bfloat16      # gradients come in the type of the inputs
+    q, k, v = (t.cuda().to(dt).requires_grad_() for t in (Q, K, V))
+    o = layer(q, k, v, causal=causal)
+    gq, gk, gv, gt = torch.autograd.grad(o, (q, k, v, layer.conv_weight), dO.cuda().to(o.dtype))
+    check_outputs(dict(O=o, dQ=gq, dK=gk, dV=gv, dTheta=gt), dict(O=O, dQ=dQ, dK=dK, dV=dV, dTheta=dTh),
+                  "edges B%d H%d N%d d%d theta(%d,%d) causal=%d fp32=%d" % (B, H, N, d, cq, ck, causal, fp32_inputs))
+
+
+@pytest.mark.parametrize("B,H,N,d,G,cq,ck,causal", [
+    (1, 4, 127, 64, 2, 3, 5, True),        # groups of 2; one key short of a block
+    (1, 4, 130, 128, 4, 6, 11, True),      # two keys past one
+    (1, 8, 65, 64, 8, 5, 5, False),        # groups of 8: 16-row tiles, 64-key blocks
+    (2, 2, 193, 64, 2, 7, 7, True),        # seven taps
+    (1, 16, 231, 64, 16, 0, 0, True),      # mix alone, past the rule for the one-CTA kernels
+    (1, 8, 300, 128, 8, 0, 0, False),
+])
+@pytest.mark.parametrize("spread", [1.0, 12.0])    # 12: logits in the hundreds, most probabilities vanish
+def test_mixing_tiles_and_groups(B, H, N, d, G, cq, ck, causal, spread):
+    import fmta_b200 as F
+    g = torch.Generator().manual_seed(N + d + G)
+    Q, K, V, dO, theta = orc.make_inputs(B, H, N, d, max(cq, 1), max(ck, 1), seed=N, dtype=torch.bfloat16)
+    Q = (Q * spread).to(torch.bfloat16).float()
+    wg = torch.eye(G).repeat(H // G, 1, 1) + 0.05 * torch.randn(H // G, G, G, generator=g)
+    scale = 1.0 / math.sqrt(d)
+    th = theta if cq else None
+    wfull = orc.block_diag_mix(wg)
+    Or, _, _ = orc.conv_headmix_fwd(Q, K, V, th, wfull, scale, causal)
+    dq, dk, dv, dth, dw = orc.conv_headmix_bwd_autograd(Q, K, V, th, wfull, dO, scale, causal)
+    dw = torch.stack([dw[G * i:G * i + G, G * i:G * i + G] for i in range(H // G)])
+    q, k, v = (t.cuda().to(torch.bfloat16).requires_grad_() for t in (Q, K, V))
+    w = wg.cuda().requires_grad_()
+    if cq:
+        t = theta.cuda().requires_grad_()
+        o = F.conv_headmix_attention(q, k, v, t, w, causal, scale)
+        gq, gk, gv, gt, gw = torch.autograd.grad(o, (q, k, v, t, w), dO.cuda().to(o.dtype))
+    else:
+        w1 = w if G < H else wg[0].cuda().requires_grad_()
+        o = F.head_conv_attention(q, k, v, w1, causal, scale)
+        gq, gk, gv, gw = torch.autograd.grad(o, (q, k, v, w1), dO.cuda().to(o.dtype))
+        gt, dth = None, None
+
+    def rel(a, b):
+        return float((a.detach().float().cpu().reshape(b.shape) - b).norm() / b.norm())
+
+    # sharp softmax: one rounding of a probability or of a gradient of the scores shows at its full relative size
+    tol = 1e-2 if spread == 1.0 else 2e-2
+    assert rel(o, Or) <= tol
+    for got, ref in ((gq, dq), (gk, dk), (gv, dv), (gw, dw)) + (((gt, dth),) if cq else ()):
+        assert torch.isfinite(got).all() and rel(got, ref) <= tol
