@@ -912,37 +912,40 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     return smem + t * Cfg::TILE_STRIDE + r * 128 + (((c ^ (r + t)) & 7) << 4);
   };
 
-  if (tid == 0) {
-    tc::tma_prefetch_desc(&tmK); tc::tma_prefetch_desc(&tmX);
-    tc::mbar_init(&bars[0], 1); tc::mbar_init(&bars[1], 1);
-    *s_abort = 0;
-    tc::mbar_fence_init();
-  }
   pdl_trigger();
-  // the Toeplitz tiles depend on the filter only: they are built under the tail of the dK/dV kernel
-  for (int i = tid; i < cq * 16 * 32; i += NT) {
-    const int a = i >> 9, x = (i >> 5) & 15, r = i & 31, bb = x + pk + HALO - r;
-    const float w = (bb >= 0 && bb < ck) ? theta[((size_t)h * cq + a) * ck + bb] * scale : 0.f;
-    const bf16 hi = __float2bfloat16_rn(w);
-    bf16* dst = sT + 2 * a * T_ELEMS + x * T_LD + r;
-    dst[0] = hi;
-    dst[T_ELEMS] = __float2bfloat16_rn(w - __bfloat162float(hi));
-  }
-  __syncthreads();
-  pdl_wait();      // nothing before this line reads what a kernel of the same call writes
-  if (tid == 0) {
-    tc::mbar_expect_tx(&bars[0], (1 + half * HL) * Cfg::TILE_BYTES);
-    tc::tma_load_3d(smem, &tmK, &bars[0], col0, J0 - HALO, bh);
-    auto load_tap = [&](int a, uint64_t* bar) {
-      for (int hl = 0; hl < HL; ++hl)
-        tc::tma_load_3d(smem + (1 + hl * cq + a) * Cfg::TILE_STRIDE, &tmX, bar, col0, J0 - HALO, (bh * cq + a) * HL + hl);
-    };
-    for (int a = 0; a < half; ++a) load_tap(a, &bars[0]);
-    if (cq > half) {
-      tc::mbar_expect_tx(&bars[1], (cq - half) * HL * Cfg::TILE_BYTES);
-      for (int a = half; a < cq; ++a) load_tap(a, &bars[1]);
+  // Warp 0 waits for the dK/dV kernel and fetches the rows; the others build the Toeplitz tiles, which depend on the filter
+  // only, meanwhile (fetched behind them, the rows came 1.5 us later in every CTA).
+  if (warp == 0) {
+    if (lane == 0) {
+      tc::tma_prefetch_desc(&tmK); tc::tma_prefetch_desc(&tmX);
+      tc::mbar_init(&bars[0], 1); tc::mbar_init(&bars[1], 1);
+      *s_abort = 0;
+      tc::mbar_fence_init();
+      pdl_wait();      // nothing before this line reads what a kernel of the same call writes
+      tc::mbar_expect_tx(&bars[0], (1 + half * HL) * Cfg::TILE_BYTES);
+      tc::tma_load_3d(smem, &tmK, &bars[0], col0, J0 - HALO, bh);
+      auto load_tap = [&](int a, uint64_t* bar) {
+        for (int hl = 0; hl < HL; ++hl)
+          tc::tma_load_3d(smem + (1 + hl * cq + a) * Cfg::TILE_STRIDE, &tmX, bar, col0, J0 - HALO, (bh * cq + a) * HL + hl);
+      };
+      for (int a = 0; a < half; ++a) load_tap(a, &bars[0]);
+      if (cq > half) {
+        tc::mbar_expect_tx(&bars[1], (cq - half) * HL * Cfg::TILE_BYTES);
+        for (int a = half; a < cq; ++a) load_tap(a, &bars[1]);
+      }
+    }
+  } else {
+#pragma unroll 4
+    for (int i = tid - 32; i < cq * 16 * 32; i += NT - 32) {
+      const int a = i >> 9, x = (i >> 5) & 15, r = i & 31, bb = x + pk + HALO - r;
+      const float w = (bb >= 0 && bb < ck) ? theta[((size_t)h * cq + a) * ck + bb] * scale : 0.f;
+      const bf16 hi = __float2bfloat16_rn(w);
+      bf16* dst = sT + 2 * a * T_ELEMS + x * T_LD + r;
+      dst[0] = hi;
+      dst[T_ELEMS] = __float2bfloat16_rn(w - __bfloat162float(hi));
     }
   }
+  __syncthreads();
   bool ok = true;
 
   // ---- dK: warp = (32 keys, 16 columns).  Its two 16-key tiles share the middle one of their three
@@ -987,6 +990,7 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
       }
     }
   }
+  pdl_wait();      // for the band kernel's part of dK (and what 'this kernel has completed' has to imply)
   {
     const int g = lane >> 2, t4 = lane & 3;
 #pragma unroll
