@@ -13,9 +13,8 @@
 // Operand tensors P / dC: "X8" = [head][key chunk of 8][row][8 keys], rows padded to X8 rows = roundup(N, 128) + 16.  A thread
 // of the score kernel owns a row, so its 16-byte stores of 8 keys are contiguous across a warp; and every consumer gets an
 // MMA operand with one tiled copy of 128-byte pieces: no-swizzle core matrices, K-major for O = P V and dQ (a row shift is
-// 16 bytes), MN-major for dV = P^T dO and dKt = dC^T Q.  With a filter dC is row-major instead: dQ reads it at c_q row shifts, and a
-// shift inside the no-swizzle layout misaligns every core matrix (117 cycles per 128x128x16 MMA instead of 80); in a swizzled
-// tile it moves whole rows.
+// 16 bytes), MN-major for dV = P^T dO and dKt = dC^T Q.  With a filter dC is row-major instead: dQ reads it at c_q row shifts,
+// which move whole rows of a swizzled tile.
 #pragma once
 #include <cuda.h>
 
