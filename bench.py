@@ -485,9 +485,9 @@ def main():
                             stacked_keys="built once per step (forward), kept for the backward" if kt is not None else "built by forward and by backward",
                             flops_attn_gflop=fl / 1e9, flops_conv_gflop=8 * cq * ck * E / 1e9),
                 # kernels of this library per step: forward = stacked-key pre-pass, fwd_tc, fwd_band;
-                # rowdot; backward = pre-pass (not when the forward's operand is kept), dq_tc, dkdv_tc, Toeplitz tiles + dKt adjoint, bwd_band,
+                # rowdot; backward = pre-pass (not when the forward's operand is kept), bwd_band, dq_tc, dkdv_tc, dKt adjoint,
                 # partial reduction
-                e2e=e2e, roofline=roof, clocks=clocks, gpu_launches=(11 if kt is None else 10) * args.steps * len(loops))
+                e2e=e2e, roofline=roof, clocks=clocks, gpu_launches=(10 if kt is None else 9) * args.steps * len(loops))
 
     # ---- decode (HBM-bound), rank-local, reported beside the headline ----
     if not args.no_decode:
