@@ -57,13 +57,14 @@ __global__ void rowdot_kernel(const bf16* __restrict__ dO, const void* __restric
 // taken from the rounded values, as if it had been converted by a pass of its own.
 template <bool O_BF16, bool DO_F32, int TPR>
 __global__ void __launch_bounds__(256) rowdot_vec_kernel(const void* __restrict__ dO_, const void* __restrict__ O,
-                                                         bf16* __restrict__ dOb, float* __restrict__ Dv, size_t rows) {
+                                                         bf16* __restrict__ dOb, float* __restrict__ Dv, size_t rows, unsigned* __restrict__ zero, int n_zero) {
   constexpr int D = TPR * 8;
   const size_t row = (size_t)blockIdx.x * (256 / TPR) + threadIdx.x / TPR;
   const int c = (threadIdx.x % TPR) * 8;
   float t = 0.f;
   pdl_trigger();
   pdl_wait();                                          // launched with programmatic stream serialization
+  if (blockIdx.x == 0) for (int i = threadIdx.x; i < n_zero; i += 256) zero[i] = 0u;   // counters of a later kernel of the call
   if (row < rows) {
     uint4 g;
     if (DO_F32) {
@@ -131,18 +132,18 @@ cudaError_t launch_reduce_partials(const float* part, float* out, int n_slots, i
 }
 
 // dOb: where the bf16 rounding of an fp32 dO goes (nullptr: dO is bf16); d = 32, 64 or 128 and aligned pointers then.
-cudaError_t launch_rowdot(const void* dO, const void* O, int o_bf16, __nv_bfloat16* dOb, float* Dv, size_t rows, int d, cudaStream_t stream) {
+cudaError_t launch_rowdot(const void* dO, const void* O, int o_bf16, __nv_bfloat16* dOb, float* Dv, size_t rows, int d, cudaStream_t stream, unsigned* zero, int n_zero) {
 #define FMTA_ROWDOT(TPR)                                                                                   \
   { const unsigned nb = (unsigned)((rows + 256 / TPR - 1) / (256 / TPR));                                  \
     auto kern = dOb ? (o_bf16 ? rowdot_vec_kernel<true, true, TPR> : rowdot_vec_kernel<false, true, TPR>)     \
                     : (o_bf16 ? rowdot_vec_kernel<true, false, TPR> : rowdot_vec_kernel<false, false, TPR>);  \
-    return launch_pdl(kern, dim3(nb), dim3(256), 0, stream, dO, O, dOb, Dv, rows); }
+    return launch_pdl(kern, dim3(nb), dim3(256), 0, stream, dO, O, dOb, Dv, rows, zero, n_zero); }
   const bool al = (reinterpret_cast<uintptr_t>(dO) % 16 == 0) && (reinterpret_cast<uintptr_t>(O) % 16 == 0);
   if (al && d == 64) FMTA_ROWDOT(8)
   if (al && d == 128) FMTA_ROWDOT(16)
   if (al && d == 32) FMTA_ROWDOT(4)
 #undef FMTA_ROWDOT
-  if (dOb) return cudaErrorInvalidValue;
+  if (dOb || zero) return cudaErrorInvalidValue;
   const unsigned blocks = (unsigned)((rows + 7) / 8);
   if (o_bf16) rowdot_kernel<true><<<blocks, 256, 0, stream>>>(reinterpret_cast<const bf16*>(dO), O, Dv, rows, d);
   else rowdot_kernel<false><<<blocks, 256, 0, stream>>>(reinterpret_cast<const bf16*>(dO), O, Dv, rows, d);

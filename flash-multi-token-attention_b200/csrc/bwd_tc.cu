@@ -886,7 +886,7 @@ template <bool LO>
 __global__ void __launch_bounds__(DkPostCfg::NT, LO ? 1 : 2)
 dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmX,
                    const float* __restrict__ theta, void* dK, const float* dKadd, int out_bf16, float* __restrict__ dTheta_part, int* status,
-                   int H, int N, int cq, int ck, float scale, int n_jblocks, int dfull, int j_base) {
+                   int H, int N, int cq, int ck, float scale, int n_jblocks, int dfull, int j_base, const ThetaFold fold) {
   using Cfg = DkPostCfg;
   constexpr int D = Cfg::D, NT = Cfg::NT, KEYS = Cfg::KEYS, HALO = Cfg::HALO;
   constexpr int T_LD = Cfg::T_LD, T_ELEMS = Cfg::T_ELEMS, RED_LD = Cfg::RED_LD;
@@ -1063,6 +1063,35 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     dTheta_part[((size_t)slot * H + h) * (cq * ck) + i] = t * scale;
   }
   if (!ok) atomicExch(status, 1);
+  if (fold.count) {
+    // few partials: the head's last CTA adds them, in the order of reduce_partials_kernel (a launch less: 2.4 us of the host)
+    __threadfence();
+    __syncthreads();
+    volatile int* last = s_abort;                            // free by now
+    if (tid == 0) {
+      const unsigned total = gridDim.x * gridDim.z * (gridDim.y / H);
+      *last = atomicAdd(&fold.count[h], 1u) == total - 1;
+    }
+    __syncthreads();
+    if (!*last) return;
+    __threadfence();
+    const int k = tid >> 5, n = cq * ck;
+    for (int i0 = 0; i0 < n; i0 += 32) {
+      const int i = i0 + lane;
+      float t = 0.f;
+      if (i < n)
+        for (int sl = k; sl < fold.slots; sl += 8) t += __ldcg(fold.part + ((size_t)sl * H + h) * n + i);
+      __syncthreads();                                       // sRed: the partials, then the sums of the 32 outputs before
+      sRed[k * 33 + lane] = t;
+      __syncthreads();
+      if (k == 0 && i < n) {
+        float r = 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) r += sRed[q * 33 + lane];
+        fold.out[(size_t)h * n + i] = r;
+      }
+    }
+  }
 }
 
 // ==========================================================================================
@@ -1236,7 +1265,7 @@ cudaError_t launch_dk_post(const TrainParams& p, __nv_bfloat16* dKt, bool with_l
   // (the maps span the full head dim; each CTA fetches its 64-column slab)
   ScopedKernelTimer timer2_(kKernDkPost, stream);
   return launch_pdl(kern, g2, dim3(DkPostCfg::NT), (size_t)smem, stream, tmK, tmX, p.theta, p.dKo, p.causal ? p.dK : (const float*)nullptr, p.grad_bf16, dTheta_part_tc, status, p.H, p.N, p.cq,
-                    p.ck, p.scale, njb, D, j_base);
+                    p.ck, p.scale, njb, D, j_base, p.fold);
 }
 
 // slots of dTheta partials written by the dKt adjoint kernel: one per CTA

@@ -143,9 +143,9 @@ size_t fmta_workspace_bytes(int op, int B, int H, int N, int d, int cq, int ck, 
                                                           : bwd_tc_workspace_bytes(B, H, N, d, cq));
   }
   if (op == FMTA_OP_BWD_FUSED) {
-    // FMTA_OP_BWD_TC, then D, the bf16 dO and the band kernel's fp32 part of dQ, dK, dV
+    // FMTA_OP_BWD_TC, then D, the bf16 dO, the adjoint kernel's counters and the band kernel's fp32 part of dQ, dK, dV
     const size_t rows = (size_t)B * H * N;
-    return up1k(fmta_workspace_bytes(FMTA_OP_BWD_TC, B, H, N, d, cq, ck, G)) + up1k(rows * 4) + up1k(rows * d * 2) + 3 * up1k(rows * d * 4);
+    return up1k(fmta_workspace_bytes(FMTA_OP_BWD_TC, B, H, N, d, cq, ck, G)) + up1k(rows * 4) + up1k(rows * d * 2) + up1k((size_t)H * 4) + 3 * up1k(rows * d * 4);
   }
   if (op == FMTA_OP_MIX_FWD || op == FMTA_OP_MIX_BWD) return mix_tc_workspace_bytes(B, H, N, d, cq, ck, G, op == FMTA_OP_MIX_BWD);
   if (op == FMTA_OP_MIX_EXCHANGE) {
@@ -312,11 +312,14 @@ int fmta_bwd_dkdv(const void* Q, const void* K, const void* V, const void* dO, c
   return check_cuda(launch_bwd_dkdv(p, (cudaStream_t)stream));
 }
 
+// partials a head's last CTA of the adjoint kernel adds itself; with more, the reduction's own launch is the faster one
+constexpr int kFoldSlots = 64;
+
 static int bwd_impl(const void* Q, const void* K, const void* V, const void* dO, const float* D,
                     const float* LSE, const float* theta, const float* wmix, float* dQ, float* dK, float* dV,
                     float* dTheta, float* dW, int B, int H, int N, int d, int cq, int ck, int G, float scale,
                     int causal, int path, void* workspace, size_t workspace_bytes, void* stream, const void* ktilde,
-                    int row_lo = 0, int row_hi = 0, void* const* grads_bf16 = nullptr) {
+                    int row_lo = 0, int row_hi = 0, void* const* grads_bf16 = nullptr, unsigned* theta_count = nullptr) {
   TrainParams p = {};
   if (ktilde && !aligned16(ktilde)) return FMTA_ERR_ALIGN;
   if (int s = fill_bwd(p, Q, K, V, dO, D, LSE, theta, wmix, B, H, N, d, cq, ck, G, scale, causal)) return s;
@@ -375,10 +378,12 @@ static int bwd_impl(const void* Q, const void* K, const void* V, const void* dO,
   if (int s = check_cuda(launch_bwd_ktilde(p, tcw, st))) return s;
   p.n_slots = slots_ex;
   p.dTheta_part = part;
+  if (theta_count && slots_ex + slots_tc <= kFoldSlots) p.fold = {part, dTheta, theta_count, slots_ex + slots_tc};
   if (causal)
     if (int s = check_cuda(launch_bwd_band(p, st))) return s;
   if (int s = check_cuda(launch_bwd_dq_tc(p, tcw, keep_pdc, st))) return s;
   if (int s = check_cuda(launch_bwd_dkdv_tc(p, tcw, part + (size_t)slots_ex * n_theta, keep_pdc, st))) return s;
+  if (p.fold.count) return FMTA_OK;
   return check_cuda(launch_reduce_partials(part, dTheta, slots_ex + slots_tc, (int)n_theta, st));
 }
 
@@ -418,14 +423,15 @@ int fmta_bwd_fused(const void* Q, const void* K, const void* V, const void* dO, 
   unsigned char* w = reinterpret_cast<unsigned char*>(workspace) + base;
   float* D = reinterpret_cast<float*>(w); w += up1k(rows * 4);
   __nv_bfloat16* dOb = reinterpret_cast<__nv_bfloat16*>(w); w += up1k(rows * d * 2);
+  unsigned* count = reinterpret_cast<unsigned*>(w); w += up1k((size_t)H * 4);
   float* part[3];
   for (int i = 0; i < 3; ++i) { part[i] = reinterpret_cast<float*>(w); w += up1k(rows * d * 4); }
   void* outs[3] = {dQ, dK, dV};
   const bool g16 = grad_dtype == FMTA_DTYPE_BF16, d32 = do_dtype == FMTA_DTYPE_F32;
   if (!g16) for (int i = 0; i < 3; ++i) part[i] = reinterpret_cast<float*>(outs[i]);
-  if (int s = check_cuda(launch_rowdot(dO, O, o_dtype == FMTA_DTYPE_BF16, d32 ? dOb : nullptr, D, rows, d, (cudaStream_t)stream))) return s;
+  if (int s = check_cuda(launch_rowdot(dO, O, o_dtype == FMTA_DTYPE_BF16, d32 ? dOb : nullptr, D, rows, d, (cudaStream_t)stream, count, H))) return s;
   return bwd_impl(Q, K, V, d32 ? dOb : dO, D, LSE, theta, nullptr, part[0], part[1], part[2], dTheta, nullptr, B, H, N, d, cq,
-                  ck, 1, scale, causal, 1, workspace, base, stream, ktilde, 0, 0, g16 ? outs : nullptr);
+                  ck, 1, scale, causal, 1, workspace, base, stream, ktilde, 0, 0, g16 ? outs : nullptr, count);
 }
 
 int fmta_mix_bwd(const void* Q, const void* K, const void* V, const void* dO, int do_dtype, const void* O, int o_dtype,

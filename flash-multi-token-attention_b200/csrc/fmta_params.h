@@ -6,6 +6,14 @@
 
 namespace fmta {
 
+// The dTheta reduction as the tail of the adjoint kernel: the CTA of a head that arrives last adds the head's partials
+struct ThetaFold {
+  const float* part;         // [slots, H, cq*ck], all of them
+  float* out;                // [H, cq*ck]
+  unsigned* count;           // [H], zero before the backward's first kernel has completed (nullptr: no fold, reduce_partials_kernel follows)
+  int slots;
+};
+
 struct TrainParams {
   const __nv_bfloat16* Q;
   const __nv_bfloat16* K;
@@ -44,6 +52,7 @@ struct TrainParams {
   int o_bf16;
   int grad_bf16;             // tensor-core backward: dQo, dKo, dVo are bf16
   int n_slots;
+  ThetaFold fold;
 };
 
 #ifdef __CUDACC__

@@ -105,7 +105,8 @@ cudaError_t launch_fwd_exact(const TrainParams& p, cudaStream_t stream);
 cudaError_t launch_bwd_dq(const TrainParams& p, cudaStream_t stream);
 cudaError_t launch_bwd_dkdv(const TrainParams& p, cudaStream_t stream);
 cudaError_t launch_reduce_partials(const float* part, float* out, int n_slots, int n, cudaStream_t stream);
-cudaError_t launch_rowdot(const void* dO, const void* O, int o_bf16, __nv_bfloat16* dOb, float* Dv, size_t rows, int d, cudaStream_t stream);
+cudaError_t launch_rowdot(const void* dO, const void* O, int o_bf16, __nv_bfloat16* dOb, float* Dv, size_t rows, int d, cudaStream_t stream,
+                          unsigned* zero = nullptr, int n_zero = 0);
 cudaError_t launch_decode(const DecodeParams& p, cudaStream_t stream);
 cudaError_t launch_kv_append_paged(void* Kpool, void* Vpool, const int* block_table, const int* seq_lens,
                                    const void* Knew, const void* Vnew, int B, int H, int n_new, int d, int page_size,

@@ -197,11 +197,10 @@ struct ConvAttnFn : public torch::autograd::Function<ConvAttnFn> {
     const Tensor O = conv_run({scale, causal, pad, keep_limit, stream_limit}, q, k, v, theta, s, LSE, kt);
     const Tensor out = pad ? cut32(O) : O;
     ctx->save_for_backward({q, k, v, theta_, LSE, out, kt});
-    ctx->saved_data["scale"] = scale;
-    ctx->saved_data["causal"] = causal;
-    ctx->saved_data["pad"] = pad;
-    ctx->saved_data["stream_limit"] = stream_limit;
-    ctx->saved_data["tq"] = (int64_t)Q.scalar_type(); ctx->saved_data["tk"] = (int64_t)K.scalar_type(); ctx->saved_data["tv"] = (int64_t)V.scalar_type();
+    // few entries: each is a string, a map node and a lookup
+    ctx->saved_data["s"] = scale;
+    ctx->saved_data["f"] = (int64_t)causal | (int64_t)pad << 1 | (int64_t)Q.scalar_type() << 8 | (int64_t)K.scalar_type() << 16 | (int64_t)V.scalar_type() << 24;
+    if (stream_limit) ctx->saved_data["l"] = stream_limit;
     return out;
   }
 
@@ -210,11 +209,12 @@ struct ConvAttnFn : public torch::autograd::Function<ConvAttnFn> {
     const auto saved = ctx->get_saved_variables();
     const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &theta_ = saved[3], &LSE = saved[4], &kt = saved[6];
     Tensor O = saved[5], dO = grads[0];
-    const double scale = ctx->saved_data["scale"].toDouble();
-    const bool causal = ctx->saved_data["causal"].toBool(), pad = ctx->saved_data["pad"].toBool();
-    const int64_t stream_limit = ctx->saved_data["stream_limit"].toInt();
-    const at::ScalarType ty[3] = {(at::ScalarType)ctx->saved_data["tq"].toInt(), (at::ScalarType)ctx->saved_data["tk"].toInt(),
-                                  (at::ScalarType)ctx->saved_data["tv"].toInt()};
+    const double scale = ctx->saved_data["s"].toDouble();
+    const int64_t flags = ctx->saved_data["f"].toInt();
+    const bool causal = flags & 1, pad = flags & 2;
+    const auto limit = ctx->saved_data.find("l");
+    const int64_t stream_limit = limit == ctx->saved_data.end() ? 0 : limit->second.toInt();
+    const at::ScalarType ty[3] = {(at::ScalarType)(flags >> 8 & 0xff), (at::ScalarType)(flags >> 16 & 0xff), (at::ScalarType)(flags >> 24 & 0xff)};
     if (!dO.defined()) dO = at::zeros_like(O);
     c10::cuda::CUDAGuard guard(q.device());
     const Tensor theta = f32(theta_);
