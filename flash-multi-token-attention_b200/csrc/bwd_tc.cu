@@ -1080,6 +1080,7 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
       const int i = i0 + lane;
       float t = 0.f;
       if (i < n)
+#pragma unroll 8
         for (int sl = k; sl < fold.slots; sl += 8) t += __ldcg(fold.part + ((size_t)sl * H + h) * n + i);
       __syncthreads();                                       // sRed: the partials, then the sums of the 32 outputs before
       sRed[k * 33 + lane] = t;

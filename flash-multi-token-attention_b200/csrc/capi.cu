@@ -312,8 +312,10 @@ int fmta_bwd_dkdv(const void* Q, const void* K, const void* V, const void* dO, c
   return check_cuda(launch_bwd_dkdv(p, (cudaStream_t)stream));
 }
 
-// partials a head's last CTA of the adjoint kernel adds itself; with more, the reduction's own launch is the faster one
-constexpr int kFoldSlots = 64;
+// A head's last CTA of the adjoint kernel adds the dTheta partials itself where the step is bound by the host's launches (no
+// more CTAs than SMs) and they are few; with more of either the fences and the serial sum cost the GPU more (2-15 us) than
+// the reduction's own launch.
+constexpr int kFoldSlots = 32, kFoldCtas = 148;
 
 static int bwd_impl(const void* Q, const void* K, const void* V, const void* dO, const float* D,
                     const float* LSE, const float* theta, const float* wmix, float* dQ, float* dK, float* dV,
@@ -378,7 +380,7 @@ static int bwd_impl(const void* Q, const void* K, const void* V, const void* dO,
   if (int s = check_cuda(launch_bwd_ktilde(p, tcw, st))) return s;
   p.n_slots = slots_ex;
   p.dTheta_part = part;
-  if (theta_count && slots_ex + slots_tc <= kFoldSlots) p.fold = {part, dTheta, theta_count, slots_ex + slots_tc};
+  if (theta_count && slots_ex + slots_tc <= kFoldSlots && slots_tc * H <= kFoldCtas) p.fold = {part, dTheta, theta_count, slots_ex + slots_tc};
   if (causal)
     if (int s = check_cuda(launch_bwd_band(p, st))) return s;
   if (int s = check_cuda(launch_bwd_dq_tc(p, tcw, keep_pdc, st))) return s;
