@@ -496,6 +496,12 @@ static cudaError_t launch_bwd_band_d(const TrainParams& p, dim3 grid, cudaStream
     return launch_kernel<TrainParams>(bwd_band_kernel<D, 7, 7, GIVEN>, grid, dim3(bandcfg::NT), smem, stream, -1, p);
   if (p.cq == 3 && p.ck == 5)
     return launch_kernel<TrainParams>(bwd_band_kernel<D, 3, 5, GIVEN>, grid, dim3(bandcfg::NT), smem, stream, -1, p);
+  if (p.cq == 3 && p.ck == 3)
+    return launch_kernel<TrainParams>(bwd_band_kernel<D, 3, 3, GIVEN>, grid, dim3(bandcfg::NT), smem, stream, -1, p);
+  if (p.cq == 5 && p.ck == 5)
+    return launch_kernel<TrainParams>(bwd_band_kernel<D, 5, 5, GIVEN>, grid, dim3(bandcfg::NT), smem, stream, -1, p);
+  if (p.cq == 5 && p.ck == 9)
+    return launch_kernel<TrainParams>(bwd_band_kernel<D, 5, 9, GIVEN>, grid, dim3(bandcfg::NT), smem, stream, -1, p);
   return launch_kernel<TrainParams>(bwd_band_kernel<D, 0, 0, GIVEN>, grid, dim3(bandcfg::NT), smem, stream, -1, p);
 }
 

@@ -881,8 +881,9 @@ struct DkPostCfg {
   }
 };
 
-// LO: dKt_a is a (hi, lo) pair of tiles; the lo tiles follow the hi tiles in shared memory
-template <bool LO>
+// LO: dKt_a is a (hi, lo) pair of tiles; the lo tiles follow the hi tiles in shared memory.  FOLD: see ThetaFold (an
+// instantiation of its own, because its registers cost the others their third CTA per SM)
+template <bool LO, bool FOLD>
 __global__ void __launch_bounds__(DkPostCfg::NT, LO ? 1 : 2)
 dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmX,
                    const float* __restrict__ theta, void* dK, const float* dKadd, int out_bf16, float* __restrict__ dTheta_part, int* status,
@@ -1063,7 +1064,7 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     dTheta_part[((size_t)slot * H + h) * (cq * ck) + i] = t * scale;
   }
   if (!ok) atomicExch(status, 1);
-  if (fold.count) {
+  if constexpr (FOLD) {
     // few partials: the head's last CTA adds them, in the order of reduce_partials_kernel (a launch less: 2.4 us of the host)
     __threadfence();
     __syncthreads();
@@ -1257,7 +1258,7 @@ cudaError_t launch_dk_post(const TrainParams& p, __nv_bfloat16* dKt, bool with_l
   const int njb = (win_hi(p) - j_base + DkPostCfg::KEYS - 1) / DkPostCfg::KEYS;
   dim3 g2(njb, (unsigned)BH, D / DkPostCfg::D);      // one CTA per 64 keys and 64 columns of the head dim
   const int smem = DkPostCfg::smem_bytes(p.cq, with_lo);
-  auto kern = with_lo ? dk_post_mma_kernel<true> : dk_post_mma_kernel<false>;
+  auto kern = with_lo ? dk_post_mma_kernel<true, false> : p.fold.count ? dk_post_mma_kernel<false, true> : dk_post_mma_kernel<false, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   alignas(64) CUtensorMap tmK, tmX;

@@ -250,6 +250,12 @@ static cudaError_t launch_fwd_band_t(const TrainParams& p, cudaStream_t stream) 
     return launch_kernel<TrainParams>(fwd_band_kernel<D, 7, 7, SCORES>, grid, dim3(Cfg::NT), Cfg::kSmemBytes, stream, -1, p);
   if (p.cq == 3 && p.ck == 5)
     return launch_kernel<TrainParams>(fwd_band_kernel<D, 3, 5, SCORES>, grid, dim3(Cfg::NT), Cfg::kSmemBytes, stream, -1, p);
+  if (p.cq == 3 && p.ck == 3)
+    return launch_kernel<TrainParams>(fwd_band_kernel<D, 3, 3, SCORES>, grid, dim3(Cfg::NT), Cfg::kSmemBytes, stream, -1, p);
+  if (p.cq == 5 && p.ck == 5)
+    return launch_kernel<TrainParams>(fwd_band_kernel<D, 5, 5, SCORES>, grid, dim3(Cfg::NT), Cfg::kSmemBytes, stream, -1, p);
+  if (p.cq == 5 && p.ck == 9)
+    return launch_kernel<TrainParams>(fwd_band_kernel<D, 5, 9, SCORES>, grid, dim3(Cfg::NT), Cfg::kSmemBytes, stream, -1, p);
   return launch_kernel<TrainParams>(fwd_band_kernel<D, 0, 0, SCORES>, grid, dim3(Cfg::NT), Cfg::kSmemBytes, stream, -1, p);
 }
 

@@ -53,10 +53,10 @@ def _pad64(t):
 # writes; forward and backward each run it.  A training step can keep the forward's copy for the backward
 # (c_q times the size of K for as long as the graph lives; about 2 % of a step at B=4, H=16, N=4096, d=64):
 # `ktilde_buffer` + the ``ktilde`` argument of `forward` / `backward`, or FMTA_KEEP_KTILDE=1 for the autograd Function.
-# The Function keeps it by itself up to KEEP_KTILDE_BYTES: there the pre-pass costs what its launch costs, and a layer holds
-# no more than that much longer.
+# The Function keeps it by itself up to KEEP_KTILDE_BYTES: there the pre-pass is 2 to 5 % of the step (19 MB: 172 -> 164 us),
+# and a layer holds no more than that much longer.
 KEEP_KTILDE = os.environ.get("FMTA_KEEP_KTILDE", "0") != "0"
-KEEP_KTILDE_BYTES = 16 << 20
+KEEP_KTILDE_BYTES = 64 << 20
 
 
 def ktilde_buffer(Q, conv_kernel):

@@ -54,6 +54,9 @@ def test_decode_blocks_splits_and_filters(B, H, q_len, Nk, d, cq, ck, k_splits, 
     (1, 2, 640, 64, 7, 7, True),       # seven taps: two passes of dK/dV
     (1, 3, 500, 64, 2, 17, False),     # widest filter row, ragged key blocks
     (1, 2, 383, 32, 3, 3, True),       # padded head dim
+    (1, 2, 300, 64, 5, 9, True),       # filter shapes with band kernels of their own
+    (1, 2, 301, 128, 5, 5, True),
+    (2, 1, 150, 128, 3, 3, True),
 ])
 @pytest.mark.parametrize("fp32_inputs", [False, True])
 def test_training_tiles_and_taps(B, H, N, d, cq, ck, causal, fp32_inputs):
