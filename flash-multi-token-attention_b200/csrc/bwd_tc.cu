@@ -527,6 +527,10 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc::tc_fence_after();
   const uint32_t tmem = *s_tmem;
   const uint32_t tX = tmem + Cfg::colX;
+  // Up to six accumulators leave 64 more columns: S^T and dP^T then have columns of their own, and each only waits for the
+  // element-wise warps to have taken its own last block.  With seven they take turns in X.
+  const bool sep = (with_dv ? 1 : 0) + ntap <= 6;
+  const uint32_t tXd = sep ? tX - 64 : tX;
 
   if (warp == Cfg::kEwWarps) {
     // ===================== producer warp (TMA + row statistics) =====================
@@ -596,8 +600,8 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const uint32_t o_hi = (uint32_t)(dOk >> 32), o_lo = (uint32_t)dOk;
         if (!tc::mbar_wait_warp(&full[st], ph, s_abort)) { ok = false; return; }
         tc::tc_fence_after();
-        tc::mma4_ss(tX, v_lo, kt_hi, 2, o_lo, o_hi, 2, idescT, 0);           // dP^T - D = V dO^T - D
-        tc::mma_ss2e<1>(tX, ones_lo, ones_hi, st_lo + (uint32_t)((st * Cfg::STAGE_BYTES + BR * 16) >> 4), st_hi, idescT);
+        tc::mma4_ss(tXd, v_lo, kt_hi, 2, o_lo, o_hi, 2, idescT, 0);           // dP^T - D = V dO^T - D
+        tc::mma_ss2e<1>(tXd, ones_lo, ones_hi, st_lo + (uint32_t)((st * Cfg::STAGE_BYTES + BR * 16) >> 4), st_hi, idescT);
         tc::mma_commit_e(dpt_full);
       };
       if (ok) issue_dPT(0);
@@ -609,7 +613,9 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const uint64_t dQk = tc::make_sdesc(sg + Cfg::sgQ + (HALO - pq) * 128, 16, 1024, tc::kLayoutSW128);
         const uint32_t qk_hi = (uint32_t)(dQk >> 32), qk_lo = (uint32_t)dQk;
         if (it == 0 && !tc::mbar_wait_warp(kv_full, 0, s_abort)) { ok = false; break; }   // the Kt tiles
-        if (!tc::mbar_wait_warp(xd_free, it & 1, s_abort)) { ok = false; break; }   // dP^T(it) has left X
+        // S's columns are free: dP^T(it) has left X, or (columns of its own) S^T(it-1) has
+        if (!sep && !tc::mbar_wait_warp(xd_free, it & 1, s_abort)) { ok = false; break; }
+        if (sep && it > 0 && !tc::mbar_wait_warp(xs_free, (it - 1) & 1, s_abort)) { ok = false; break; }
         tc::tc_fence_after();
         // S^T - LSE = sum_a Kt_a Q^(a)T - LSE
         for (int a = 0; a < cq; ++a)
@@ -618,9 +624,10 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tc::mma_ss2e<1>(tX, ones_lo, ones_hi, st_lo + (uint32_t)((st * Cfg::STAGE_BYTES) >> 4), st_hi, idescT);
         tc::mma_commit_e(st_full);
         tc::mma_commit_e(&empty[st]);        // this issuer's reads of the stage (dO for dP^T, Q for S^T) are done then
-        if (!tc::mbar_wait_warp(xs_free, it & 1, s_abort)) { ok = false; break; }   // S^T(it) has left X
+        if (it + 1 == nblk) break;
+        if (!tc::mbar_wait_warp(sep ? xd_free : xs_free, it & 1, s_abort)) { ok = false; break; }   // dP's: dP^T(it), or S^T(it), has left
         tc::tc_fence_after();
-        if (it + 1 < nblk) issue_dPT(it + 1);
+        issue_dPT(it + 1);
       }
     }
   } else if (warp >= Cfg::kEwWarps + 2) {
@@ -676,7 +683,7 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const int qtr = warp & 3, cg = warp >> 2;
     const int key = j0 + qtr * 32 + lane;
     const uint32_t lane_base = (uint32_t)(qtr * 32) << 16;
-    const uint32_t tXl = tX + lane_base + CW * cg;
+    const uint32_t tXl = tX + lane_base + CW * cg, tXdl = tXd + lane_base + CW * cg;
     bool ok = true;
     float dpc[CW];                                      // dP^T of the block about to be processed
     if (nblk > 0) {
@@ -684,7 +691,7 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                                                      : tc::mbar_wait(dpt_full, 0, s_abort));
       if (ok) {
         tc::tc_fence_after();
-        tc::tmem_ldn(tXl, dpc);
+        tc::tmem_ldn(tXdl, dpc);
         tc::tc_fence_before();
         tc::mbar_arrive(xd_free);
       }
@@ -705,7 +712,7 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         ok = __all_sync(0xffffffffu, tc::mbar_wait(dpt_full, (it + 1) & 1, s_abort));
         if (!ok) break;
         tc::tc_fence_after();
-        tc::tmem_ldn(tXl, dpn);
+        tc::tmem_ldn(tXdl, dpn);
         tc::tc_fence_before();
         tc::mbar_arrive(xd_free);
       }
@@ -1242,7 +1249,7 @@ cudaError_t launch_bwd_dkdv_tc(const TrainParams& p, void* workspace, float* dTh
         } else {
           // seven taps: dV + 7 accumulators + the scratch columns exceed the tensor memory, so the taps are
           // split over two passes (each recomputes S^T and dP^T)
-          e = launch_dkdv_pass<7, false>(p, Kt, dKt, status, 4, dv, klo, khi, stream);
+          e = launch_dkdv_pass<7, true>(p, Kt, dKt, status, 4, dv, klo, khi, stream);
         }
       }
     } }
