@@ -65,19 +65,6 @@ FMTA_DEVINL void tma_load_3d(void* smem_dst, const CUtensorMap* map, uint64_t* b
       ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
-FMTA_DEVINL void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2,
-                             int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-      ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-      : "memory");
-}
-// Contiguous copy global -> shared (both addresses and the size multiples of 16 bytes), completing on an mbarrier.
-FMTA_DEVINL void bulk_load(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(smem_dst)), "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
 // Tile store shared -> global (bulk async-group).  c0 = 0 and c1 >= 0 at every call: a store must not
 // start at a negative coordinate; rows past the tensor's extent are clipped.
 FMTA_DEVINL void tma_store_3d(const CUtensorMap* map, const void* smem_src, int c0, int c1, int c2) {
@@ -85,13 +72,8 @@ FMTA_DEVINL void tma_store_3d(const CUtensorMap* map, const void* smem_src, int 
                ::"l"(map), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
-// Contiguous copy shared -> global (bulk async-group); both addresses and the size multiples of 16 bytes.
-FMTA_DEVINL void bulk_store(void* gdst, const void* smem_src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
-               ::"l"(gdst), "r"(smem_u32(smem_src)), "r"(bytes)
-               : "memory");
-}
-// Same with an L2 eviction-priority hint: data that is written once and read much later should not push the
+// Contiguous copy shared -> global (bulk async-group; both addresses and the size multiples of 16 bytes) with an L2
+// eviction-priority hint: data that is written once and read much later should not push the
 // operands that are being re-read out of the cache.
 FMTA_DEVINL uint64_t l2_policy_evict_first() {
   uint64_t pol;
@@ -189,53 +171,6 @@ FMTA_DEVINL void tmem_st32(uint32_t taddr, const float (&v)[32]) {
 FMTA_DEVINL void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ---------------------------------------------------------------- tcgen05.mma
-// D[tmem] (+)= A[smem] * B[smem], kind::f16 (bf16 inputs, fp32 accumulate), issued by ONE thread.
-FMTA_DEVINL void mma_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)accumulate)
-      : "memory");
-}
-// Same with the descriptors given as (constant high word, low word): the low word holds the
-// start address, so stepping through an operand is a 32-bit add.  ACC selects accumulate (1) or
-// overwrite (0) at compile time.
-template <int ACC>
-FMTA_DEVINL void mma_ss2(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-      "setp.ne.b32 p, %6, 0;\n\t"
-      "mov.b64 da, {%1, %2};\n\t"
-      "mov.b64 db, {%3, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "n"(ACC)
-      : "memory");
-}
-// Same with the accumulate flag in a register (no branch around the first MMA of a chain).
-FMTA_DEVINL void mma_ss2p(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
-                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-      "setp.ne.b32 p, %6, 0;\n\t"
-      "mov.b64 da, {%1, %2};\n\t"
-      "mov.b64 db, {%3, %4};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// A operand in tensor memory (128 lanes = rows, each 32-bit column = 2 consecutive K elements),
-// B in shared memory.
-template <int ACC>
-FMTA_DEVINL void mma_ts2(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "mov.b64 db, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "n"(ACC)
-      : "memory");
-}
 FMTA_DEVINL void tmem_st32u(uint32_t taddr, const uint32_t (&v)[32]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -247,21 +182,9 @@ FMTA_DEVINL void tmem_st32u(uint32_t taddr, const uint32_t (&v)[32]) {
       "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
       : "memory");
 }
-FMTA_DEVINL void tmem_st16u(uint32_t taddr, const uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-      "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-      : "memory");
-}
 // Named barrier among `count` threads (ids 1..15; 0 is __syncthreads).
 FMTA_DEVINL void named_bar_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
-// Arrive on an mbarrier once all MMAs issued so far by this thread have completed.
-FMTA_DEVINL void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
 }
 
 // ---- warp-uniform issue ------------------------------------------------------------------
@@ -276,6 +199,9 @@ FMTA_DEVINL bool elect_one() {
 FMTA_DEVINL bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
+// D[tmem] (+)= A * B, kind::f16 (bf16 inputs, fp32 accumulate).  Descriptors come as (constant high word, low word): the low
+// word holds the start address, so stepping through an operand is a 32-bit add.  ss: both operands in shared memory; ts: A in
+// tensor memory (128 lanes = rows, each 32-bit column = 2 consecutive K elements).
 // Elections and MMAs sit in one asm block, the MMAs PREDICATED on the elected lane.  Behind a branch (`if (elect_one())`
 // around each MMA) every operand goes through the reconvergence of the warp and back into uniform registers: back to back
 // that took 101-108 cycles per MMA whatever its size; predicated, 39 cycles at N = 16 and the tensor core's own rate above
@@ -302,17 +228,6 @@ FMTA_DEVINL void mma_ss2pe(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32
       "mov.b64 db, {%3, %4};\n\t"
       "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}"
       ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-template <int ACC>
-FMTA_DEVINL void mma_ts2e(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\t"
-      "elect.sync _|q, 0xffffffff;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "mov.b64 db, {%2, %3};\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "n"(ACC)
       : "memory");
 }
 FMTA_DEVINL void mma_commit_e(uint64_t* bar) {
