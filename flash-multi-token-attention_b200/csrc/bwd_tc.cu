@@ -417,7 +417,7 @@ bwd_dq_stream_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // ==========================================================================================
 // dK-tilde / dV
 // ==========================================================================================
-template <int D, int CQMAX, bool PAIR>   // PAIR: two adjacent taps share one 128-wide MMA
+template <int D, int CQMAX>
 struct DkvCfg {
   static_assert(D == 64, "the dK/dV tensor-core kernel is instantiated for d = 64");
   static constexpr int BK = 128;               // keys per CTA (= TMEM lanes)
@@ -450,13 +450,13 @@ struct DkvCfg {
   static constexpr int kThreads = (kEwWarps + 4) * 32;   // + producer, issuer S, issuers A0 and A1
 };
 
-template <int D, int CQMAX, bool PAIR>
-__global__ void __launch_bounds__(DkvCfg<D, CQMAX, PAIR>::kThreads, 1)
+template <int D, int CQMAX, bool SEP>
+__global__ void __launch_bounds__(DkvCfg<D, CQMAX>::kThreads, 1)
 bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
                    const __grid_constant__ CUtensorMap tmKt, const __grid_constant__ CUtensorMap tmV,
                    const __grid_constant__ CUtensorMap tmdKt, const __grid_constant__ CUtensorMap tmdV,
                    const BwdTcParams p) {
-  using Cfg = DkvCfg<D, CQMAX, PAIR>;
+  using Cfg = DkvCfg<D, CQMAX>;
   constexpr int BK = Cfg::BK, BR = Cfg::BR, HALO = Cfg::HALO, QR = Cfg::QR, NSTG = Cfg::NSTG;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -527,10 +527,9 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc::tc_fence_after();
   const uint32_t tmem = *s_tmem;
   const uint32_t tX = tmem + Cfg::colX;
-  // Up to six accumulators leave 64 more columns: S^T and dP^T then have columns of their own, and each only waits for the
-  // element-wise warps to have taken its own last block.  With seven they take turns in X.
-  const bool sep = (with_dv ? 1 : 0) + ntap <= 6;
-  const uint32_t tXd = sep ? tX - 64 : tX;
+  // SEP: up to six accumulators leave 64 more columns; S^T and dP^T then have columns of their own, and each only waits for
+  // the element-wise warps to have taken its own last block.  With seven they take turns in X.
+  const uint32_t tXd = SEP ? tX - 64 : tX;
 
   if (warp == Cfg::kEwWarps) {
     // ===================== producer warp (TMA + row statistics) =====================
@@ -614,8 +613,8 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const uint32_t qk_hi = (uint32_t)(dQk >> 32), qk_lo = (uint32_t)dQk;
         if (it == 0 && !tc::mbar_wait_warp(kv_full, 0, s_abort)) { ok = false; break; }   // the Kt tiles
         // S's columns are free: dP^T(it) has left X, or (columns of its own) S^T(it-1) has
-        if (!sep && !tc::mbar_wait_warp(xd_free, it & 1, s_abort)) { ok = false; break; }
-        if (sep && it > 0 && !tc::mbar_wait_warp(xs_free, (it - 1) & 1, s_abort)) { ok = false; break; }
+        if (!SEP && !tc::mbar_wait_warp(xd_free, it & 1, s_abort)) { ok = false; break; }
+        if (SEP && it > 0 && !tc::mbar_wait_warp(xs_free, (it - 1) & 1, s_abort)) { ok = false; break; }
         tc::tc_fence_after();
         // S^T - LSE = sum_a Kt_a Q^(a)T - LSE
         for (int a = 0; a < cq; ++a)
@@ -625,7 +624,7 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tc::mma_commit_e(st_full);
         tc::mma_commit_e(&empty[st]);        // this issuer's reads of the stage (dO for dP^T, Q for S^T) are done then
         if (it + 1 == nblk) break;
-        if (!tc::mbar_wait_warp(sep ? xd_free : xs_free, it & 1, s_abort)) { ok = false; break; }   // dP's: dP^T(it), or S^T(it), has left
+        if (!tc::mbar_wait_warp(SEP ? xd_free : xs_free, it & 1, s_abort)) { ok = false; break; }   // dP's: dP^T(it), or S^T(it), has left
         tc::tc_fence_after();
         issue_dPT(it + 1);
       }
@@ -637,10 +636,10 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       constexpr uint32_t idescA = tc::make_idesc(BK, D, 0, 1);     // 128 x D, B MN-major
       constexpr uint32_t idescA2 = tc::make_idesc(BK, 2 * D, 0, 1); // 128 x 2D: two adjacent taps at once
       // this launch accumulates taps [tap0, tap0 + ntap) (accumulator i at column 64 * (with_dv + i)) and
-      // dV (column 0) when with_dv; A0 takes dV and the first half of the tap groups, A1 the rest.  With
-      // PAIR a group is two adjacent taps in one 128-wide MMA (an odd last tap goes alone).
+      // dV (column 0) when with_dv; A0 takes dV and the first half of the tap groups, A1 the rest.
+      // A group is two adjacent taps in one 128-wide MMA (an odd last tap goes alone).
       const int accb = with_dv ? 1 : 0;
-      const int pairs = PAIR ? ntap / 2 : 0, singles = ntap - 2 * pairs;     // groups: `pairs` pairs, then `singles` single taps
+      const int pairs = ntap / 2, singles = ntap - 2 * pairs;     // groups: `pairs` pairs, then `singles` single taps
       const int ngrp = pairs + singles, g_half = ngrp / 2;
       const int g_begin = ai == 0 ? 0 : g_half, g_end = ai == 0 ? g_half : ngrp;
       const uint64_t dPTa = tc::make_sdesc(smem_u32(smem + Cfg::oPT), BK * 16, 128, tc::kLayoutNone);
@@ -1188,11 +1187,11 @@ cudaError_t launch_bwd_dq_tc(const TrainParams& p, void* workspace, bool keep_pd
 
 // One launch of the dK/dV kernel: dV and the first `ntap` taps, and the rest of the taps as a second pass (its CTAs side by
 // side with the first one's).
-template <int CQMAX, bool PAIR>
+template <int CQMAX, bool SEP>
 static cudaError_t launch_dkdv_pass(const TrainParams& p, const __nv_bfloat16* Kt, __nv_bfloat16* dKt, int* status,
                                     int ntap, int with_dv, int key_lo, int key_hi, cudaStream_t stream) {
   constexpr int D = 64;
-  using Cfg = DkvCfg<D, CQMAX, PAIR>;
+  using Cfg = DkvCfg<D, CQMAX>;
   const size_t BH = (size_t)p.B * p.H;
   alignas(64) CUtensorMap tmQ, tmdO, tmKt, tmV, tmdKt, tmdV;
   if (!make_tensor_map_bf16(&tmdKt, dKt, D, p.N, BH * p.cq, 64, Cfg::BK, true)) return cudaErrorInvalidValue;
@@ -1208,7 +1207,7 @@ static cudaError_t launch_dkdv_pass(const TrainParams& p, const __nv_bfloat16* K
   bp.ntap = ntap; bp.with_dv = with_dv;
   bp.key_base = key_lo;
   bp.selftest_expire = take_selftest_expire(kKernBwdDkdvTc);
-  auto kern = bwd_dkdv_tc_kernel<D, CQMAX, PAIR>;
+  auto kern = bwd_dkdv_tc_kernel<D, CQMAX, SEP>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
   const int passes = ntap < p.cq ? 2 : 1;
@@ -1245,7 +1244,8 @@ cudaError_t launch_bwd_dkdv_tc(const TrainParams& p, void* workspace, float* dTh
         if (D == 128) {
           e = launch_bwd_dkdv_tc128(p, Kt, dKt, status, dv, klo, khi, stream);
         } else if (p.cq <= 6) {
-          e = launch_dkdv_pass<6, true>(p, Kt, dKt, status, p.cq, dv, klo, khi, stream);
+          e = p.cq <= 5 ? launch_dkdv_pass<6, true>(p, Kt, dKt, status, p.cq, dv, klo, khi, stream)
+                        : launch_dkdv_pass<6, false>(p, Kt, dKt, status, p.cq, dv, klo, khi, stream);
         } else {
           // seven taps: dV + 7 accumulators + the scratch columns exceed the tensor memory, so the taps are
           // split over two passes (each recomputes S^T and dP^T)
