@@ -122,9 +122,10 @@ cudaError_t launch_dk_post(const TrainParams& p, __nv_bfloat16* dKt, bool with_l
 // head mix on the tensor cores (mix_tc.cu)
 bool mix_tc_supported(const TrainParams& p);
 size_t mix_tc_workspace_bytes(int B, int H, int N, int d, int cq, int ck, int G, bool bwd);
-cudaError_t launch_mix_fwd(const TrainParams& p, void* workspace, cudaStream_t stream);
+size_t mix_tc_call_bytes(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool causal, bool bwd);
+cudaError_t launch_mix_fwd(const TrainParams& p, void* workspace, size_t workspace_bytes, cudaStream_t stream);
 cudaError_t launch_mix_bwd(const TrainParams& p, const void* dO, bool do_f32, const void* O, bool o_bf16, float* dTheta, float* dW, int want,
-                           void* workspace, cudaStream_t stream);
+                           void* workspace, size_t workspace_bytes, cudaStream_t stream);
 size_t fwd_tc_workspace_bytes(int B, int H, int N, int d, int cq);
 bool bwd_tc_supported(const TrainParams& p);
 size_t bwd_tc_workspace_bytes(int B, int H, int N, int d, int cq);

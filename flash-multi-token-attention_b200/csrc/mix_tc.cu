@@ -1,6 +1,8 @@
 // Driver of the tensor-core head-mix path (mix_tc.cuh): workspace layout, chunking over (batch, group) units, launches.
 #include "mix_tc.cuh"
 
+#include <type_traits>
+
 namespace fmta {
 
 namespace {
@@ -13,6 +15,8 @@ inline size_t up(size_t x) { return (x + 1023) / 1024 * 1024; }
 constexpr size_t kMixChunkBytes = (size_t)4500 << 20, kMixUnitMax = (size_t)16 << 30;
 
 struct MixPlan {
+  int d;
+  bool conv, causal, bwd;
   int nRT, N8, RP, U, nU, nKC, kch;
   size_t unit;            // bytes of one operand tensor (P or dC) of a unit
   size_t kt, cband, dkt, theta_part, dw_part, stat, x8;      // bytes of the workspace's parts (0: absent)
@@ -22,6 +26,7 @@ struct MixPlan {
 
 MixPlan plan(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool causal, bool bwd) {
   MixPlan m = {};
+  m.d = d; m.conv = conv; m.causal = causal; m.bwd = bwd;
   m.nRT = (N + 127) / 128; m.N8 = m.nRT * 128; m.RP = m.N8 + 16;
   m.U = B * (H / G);
   m.unit = (size_t)G * (m.N8 / 8) * m.RP * 16;
@@ -39,24 +44,60 @@ MixPlan plan(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool 
   m.rows = (size_t)B * H * N;
   const int band = (cq - 1) + (ck - 1) / 2;
   if (conv) {
-    m.kt = up(m.rows * cq * 2 * d * 2);
-    if (causal) m.cband = up(m.rows * (band > 0 ? band : 1) * 4);
+    m.kt = m.rows * cq * 2 * d * 2;
+    if (causal) m.cband = m.rows * (band > 0 ? band : 1) * 4;
     if (bwd) {
-      m.dkt = up(m.rows * cq * 2 * d * 2);
+      m.dkt = m.rows * cq * 2 * d * 2;
       m.theta_band_slots = causal ? bwd_band_theta_slots(B, N, cq, ck) : 0;
       m.theta_post_slots = bwd_tc_theta_slots(B, N, d);
-      m.theta_part = up((size_t)(m.theta_band_slots + m.theta_post_slots) * H * cq * ck * 4);
+      m.theta_part = (size_t)(m.theta_band_slots + m.theta_post_slots) * H * cq * ck * 4;
     }
   }
   if (bwd) {
     m.dw_slots = B * m.nRT * m.nKC;
-    m.dw_part = up((size_t)m.dw_slots * H * G * 4);
+    m.dw_part = (size_t)m.dw_slots * H * G * 4;
   } else {
-    m.stat = up((size_t)m.nU * G * 2 * m.nKC * 3 * m.RP * 4);
+    m.stat = (size_t)m.nU * G * 2 * m.nKC * 3 * m.RP * 4;
   }
-  m.x8 = up((size_t)m.nU * m.unit);
+  m.x8 = (size_t)m.nU * m.unit;
   return m;
 }
+
+struct MixBuffers {
+  int* status;
+  __nv_bfloat16 *Kt, *dKt, *dOb, *P8, *C8;
+  float *Cband, *dCband, *theta_part, *dw_part, *D, *dQ, *dK, *stat;
+};
+
+// The workspace's layout, for its size as for its use: the buffers of a call from `base` (any alignment; nullptr: sizes only).
+// Returns the bytes taken, the alignment of the base included.
+size_t carve(const MixPlan& m, void* base, MixBuffers& b) {
+  unsigned char* const w = base ? reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(base) + 1023) & ~uintptr_t(1023)) : nullptr;
+  size_t off = 0;
+  auto take = [&](auto*& p, size_t n) {
+    p = w && n ? reinterpret_cast<std::remove_reference_t<decltype(p)>>(w + off) : nullptr;
+    off += up(n);
+  };
+  b = MixBuffers{};
+  take(b.status, sizeof(int));
+  take(b.Kt, m.kt);
+  take(b.Cband, m.cband);
+  if (m.bwd) {
+    take(b.dCband, m.cband);
+    take(b.dKt, m.dkt);
+    take(b.theta_part, m.theta_part);
+    take(b.dw_part, m.dw_part);
+    take(b.D, m.rows * 4);
+    take(b.dOb, m.rows * m.d * 2);
+    if (m.conv && m.causal) { take(b.dQ, m.rows * m.d * 4); take(b.dK, m.rows * m.d * 4); }
+  }
+  take(b.stat, m.stat);
+  take(b.P8, m.x8);
+  if (m.bwd) take(b.C8, m.x8);
+  return off + 1024;
+}
+
+size_t bytes_of(const MixPlan& m) { MixBuffers b; return carve(m, nullptr, b); }
 
 }  // namespace
 
@@ -68,16 +109,21 @@ bool mix_tc_supported(const TrainParams& p) {
   return (size_t)p.G * (n8 / 8) * (n8 + 16) * 32 <= kMixUnitMax;
 }
 
-// Neither the causal flag nor the presence of a filter is an argument of fmta_workspace_bytes: the most of all.
+// What one call takes.
+size_t mix_tc_call_bytes(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool causal, bool bwd) {
+  return bytes_of(plan(B, H, N, d, conv ? cq : 1, conv ? ck : 1, G, conv, causal, bwd));
+}
+
+// Neither the causal flag nor, for a 1 x 1 filter, the presence of a filter is an argument of fmta_workspace_bytes: the most
+// of all.  (They are not ordered: without a filter a sequence may be cut into more chunks, with twice the statistics.)
 size_t mix_tc_workspace_bytes(int B, int H, int N, int d, int cq, int ck, int G, bool bwd) {
   if (G < 2 || H % G != 0) return 0;
   size_t most = 0;
-  for (int causal = 0; causal < 2; ++causal) {
-    const MixPlan m = plan(B, H, N, d, cq, ck, G, true, causal, bwd);
-    size_t n = 2048 + m.kt + m.cband * (bwd ? 2 : 1) + m.dkt + m.theta_part + m.dw_part + m.stat + m.x8 * (bwd ? 2 : 1);
-    if (bwd) n += up(m.rows * 4) + up(m.rows * d * 2) + (causal ? 2 * up(m.rows * d * 4) : 0);
-    if (n > most) most = n;
-  }
+  for (int causal = 0; causal < 2; ++causal)
+    for (int conv = cq * ck > 1; conv < 2; ++conv) {
+      const size_t n = bytes_of(plan(B, H, N, d, cq, ck, G, conv, causal, bwd));
+      if (n > most) most = n;
+    }
   return most;
 }
 
@@ -92,24 +138,24 @@ static void fill(MixParams& q, const TrainParams& p, const MixPlan& m, int* stat
 
 #define FMTA_TRY(x) do { const cudaError_t e_ = (x); if (e_ != cudaSuccess) return e_; } while (0)
 
-cudaError_t launch_mix_fwd(const TrainParams& p_, void* workspace, cudaStream_t stream) {
+cudaError_t launch_mix_fwd(const TrainParams& p_, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   TrainParams p = p_;
   const MixPlan m = plan(p.B, p.H, p.N, p.d, p.cq, p.ck, p.G, p.theta != nullptr, p.causal, false);
-  unsigned char* w = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(workspace) + 1023) & ~uintptr_t(1023));
+  MixBuffers b;
+  if (carve(m, workspace, b) > workspace_bytes) return cudaErrorInvalidValue;
   int* status = nullptr;
-  FMTA_TRY(status_word_of(reinterpret_cast<int*>(w), stream, &status)); w += 1024;
-  __nv_bfloat16* Kt = reinterpret_cast<__nv_bfloat16*>(w); w += m.kt;
+  FMTA_TRY(status_word_of(b.status, stream, &status));
   MixParams q;
   fill(q, p, m, status);
   if (p.theta) {
-    FMTA_TRY(launch_ktilde(p, Kt, stream, true));
-    if (p.causal) { p.Cband = reinterpret_cast<float*>(w); q.Cband = p.Cband; w += m.cband; FMTA_TRY(launch_band_scores(p, stream)); }
+    FMTA_TRY(launch_ktilde(p, b.Kt, stream, true));
+    if (p.causal) { p.Cband = b.Cband; q.Cband = b.Cband; FMTA_TRY(launch_band_scores(p, stream)); }
   }
-  q.stat = reinterpret_cast<float*>(w); w += m.stat;
-  q.P8 = reinterpret_cast<bf16*>(w);
+  q.stat = b.stat;
+  q.P8 = b.P8;
   for (q.u0 = 0; q.u0 < m.U; q.u0 += m.nU) {
     q.nU = m.U - q.u0 < m.nU ? m.U - q.u0 : m.nU;
-    FMTA_TRY(launch_mix_score(p, q, Kt, false, stream));
+    FMTA_TRY(launch_mix_score(p, q, b.Kt, false, stream));
     FMTA_TRY(launch_mix_pv(p, q, stream));
   }
   return cudaSuccess;
@@ -117,47 +163,40 @@ cudaError_t launch_mix_fwd(const TrainParams& p_, void* workspace, cudaStream_t 
 
 // dO / O in do_f32 / o_bf16; want: 1 = dQ (and dTheta, dW), 2 = dK, dV, 3 = all
 cudaError_t launch_mix_bwd(const TrainParams& p_, const void* dO, bool do_f32, const void* O, bool o_bf16, float* dTheta, float* dW, int want,
-                           void* workspace, cudaStream_t stream) {
+                           void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   TrainParams p = p_;
   const bool conv = p.theta != nullptr;
   const MixPlan m = plan(p.B, p.H, p.N, p.d, p.cq, p.ck, p.G, conv, p.causal, true);
-  unsigned char* w = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(workspace) + 1023) & ~uintptr_t(1023));
-  auto take = [&](size_t n) { unsigned char* r = w; w += n; return r; };
+  MixBuffers b;
+  if (carve(m, workspace, b) > workspace_bytes) return cudaErrorInvalidValue;
   int* status = nullptr;
-  FMTA_TRY(status_word_of(reinterpret_cast<int*>(take(1024)), stream, &status));
-  __nv_bfloat16* Kt = reinterpret_cast<__nv_bfloat16*>(take(m.kt));
-  if (conv && p.causal) { p.Cband = reinterpret_cast<float*>(take(m.cband)); p.dCband = reinterpret_cast<float*>(take(m.cband)); }
-  __nv_bfloat16* dKt = reinterpret_cast<__nv_bfloat16*>(take(m.dkt));
-  float* theta_part = reinterpret_cast<float*>(take(m.theta_part));
-  float* dw_part = reinterpret_cast<float*>(take(m.dw_part));
-  float* D = reinterpret_cast<float*>(take(up(m.rows * 4)));
-  bf16* dOb = reinterpret_cast<bf16*>(take(up(m.rows * p.d * 2)));
-  if (conv && p.causal) { p.dQ = reinterpret_cast<float*>(take(up(m.rows * p.d * 4))); p.dK = reinterpret_cast<float*>(take(up(m.rows * p.d * 4))); }
+  FMTA_TRY(status_word_of(b.status, stream, &status));
+  if (conv && p.causal) { p.Cband = b.Cband; p.dCband = b.dCband; p.dQ = b.dQ; p.dK = b.dK; }
   p.dV = nullptr;
-  FMTA_TRY(launch_rowdot(dO, O, o_bf16, do_f32 ? dOb : nullptr, D, m.rows, p.d, stream));
-  p.dO = do_f32 ? dOb : reinterpret_cast<const __nv_bfloat16*>(dO);
-  p.Dvec = D;
+  FMTA_TRY(launch_rowdot(dO, O, o_bf16, do_f32 ? b.dOb : nullptr, b.D, m.rows, p.d, stream));
+  p.dO = do_f32 ? b.dOb : reinterpret_cast<const __nv_bfloat16*>(dO);
+  p.Dvec = b.D;
   MixParams q;
   fill(q, p, m, status);
-  q.Cband = p.Cband; q.dCband = p.dCband; q.dW_part = dw_part;
-  q.P8 = reinterpret_cast<bf16*>(take(m.x8)); q.C8 = reinterpret_cast<bf16*>(take(m.x8));
+  q.Cband = p.Cband; q.dCband = p.dCband; q.dW_part = b.dw_part;
+  q.P8 = b.P8; q.C8 = b.C8;
   if (conv) {
-    FMTA_TRY(launch_ktilde(p, Kt, stream, true));
+    FMTA_TRY(launch_ktilde(p, b.Kt, stream, true));
     if (p.causal) FMTA_TRY(launch_band_scores(p, stream));
   }
-  p.dTheta_part = theta_part;
+  p.dTheta_part = b.theta_part;
   for (q.u0 = 0; q.u0 < m.U; q.u0 += m.nU) {
     q.nU = m.U - q.u0 < m.nU ? m.U - q.u0 : m.nU;
-    FMTA_TRY(launch_mix_score(p, q, Kt, true, stream));
+    FMTA_TRY(launch_mix_score(p, q, b.Kt, true, stream));
     if (conv && p.causal) FMTA_TRY(launch_bwd_band_given(p, q.u0 * p.G, q.nU * p.G, stream));
-    if (want & 1) FMTA_TRY(launch_mix_dq(p, q, Kt, stream));
-    if ((want & 2) || conv) FMTA_TRY(launch_mix_dkdv(p, q, dKt, want & 1, stream));      // dTheta comes out of dKt
+    if (want & 1) FMTA_TRY(launch_mix_dq(p, q, b.Kt, stream));
+    if ((want & 2) || conv) FMTA_TRY(launch_mix_dkdv(p, q, b.dKt, want & 1, stream));      // dTheta comes out of dKt
   }
   if (conv) {
-    FMTA_TRY(launch_dk_post(p, dKt, true, theta_part + (size_t)m.theta_band_slots * p.H * p.cq * p.ck, status, stream));
-    if (want & 1) FMTA_TRY(launch_reduce_partials(theta_part, dTheta, m.theta_band_slots + m.theta_post_slots, p.H * p.cq * p.ck, stream));
+    FMTA_TRY(launch_dk_post(p, b.dKt, true, b.theta_part + (size_t)m.theta_band_slots * p.H * p.cq * p.ck, status, stream));
+    if (want & 1) FMTA_TRY(launch_reduce_partials(b.theta_part, dTheta, m.theta_band_slots + m.theta_post_slots, p.H * p.cq * p.ck, stream));
   }
-  if (want & 1) FMTA_TRY(launch_reduce_partials(dw_part, dW, m.dw_slots, p.H * p.G, stream));
+  if (want & 1) FMTA_TRY(launch_reduce_partials(b.dw_part, dW, m.dw_slots, p.H * p.G, stream));
   return cudaSuccess;
 }
 

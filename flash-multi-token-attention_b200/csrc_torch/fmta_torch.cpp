@@ -272,14 +272,14 @@ struct Mix {
   Dims s;
   int G;
   Tensor w, theta;        // fp32 [H/G, G, G]; fp32 [H, cq, ck] or undefined
-  bool tc(bool bwd, size_t* bytes) const {                 // the tensor-core kernels take this problem
+  bool tc(bool bwd, bool causal, size_t* bytes) const {                 // the tensor-core kernels take this problem
     if (exact_only() || (s.d != 64 && s.d != 128) || G > 16 || (theta.defined() && s.cq > 7)) return false;
     // a short sequence without a filter: the 16-row CTAs of the other kernels finish sooner than one 128-row CTA of these (16
     // heads, d = 64, forward + backward on an idle GPU: 12 us per 16 keys there; 190 us at N = 640, 208 at N = 1024 here)
     if (!theta.defined() && G >= 8 && s.N <= 224 && (long)s.B * (s.H / G) * ((s.N + 15) / 16) <= 2 * 148) return false;
     const size_t n8 = ((size_t)s.N + 127) / 128 * 128;     // P and dC of one (batch, group) unit: see fmta_mix_bwd
     if ((size_t)G * (n8 / 8) * (n8 + 16) * 32 > ((size_t)16 << 30)) return false;
-    *bytes = fmta_workspace_bytes(bwd ? FMTA_OP_MIX_BWD : FMTA_OP_MIX_FWD, s.B, s.H, s.N, s.d, s.cq, s.ck, G);
+    *bytes = fmta_mix_workspace_bytes(bwd, s.B, s.H, s.N, s.d, s.cq, s.ck, G, theta.defined(), causal);
     return true;
   }
   size_t exchange(int64_t limit) const {
@@ -319,7 +319,7 @@ void mix_forward_raw(const Mix& m, const Tensor& q, const Tensor& k, const Tenso
   const Dims& s = m.s;
   arm_status(q);
   size_t n = 0;
-  const bool tc = m.tc(false, &n);
+  const bool tc = m.tc(false, causal, &n);
   if (!tc) n = m.exchange(xlimit);
   const Tensor ws = n ? new_bytes(q, n) : Tensor();
   check_status(fmta_fwd(ptr(q), ptr(k), ptr(v), fptr(m.theta), fptr(m.w), ptr(O), fptr(M), fptr(L), fptr(LSE), s.B, s.H, s.N, s.d, s.cq, s.ck, m.G,
@@ -335,7 +335,7 @@ std::vector<Tensor> mix_backward_raw(const Mix& m, const Tensor& q, const Tensor
   const bool conv = m.theta.defined();
   const Tensor dW = want & 1 ? new_f32(q, {s.H / m.G, m.G, m.G}) : Tensor(), dT = conv ? new_f32(q, {s.H, s.cq, s.ck}) : Tensor();
   size_t n = 0;
-  if (m.tc(true, &n)) {
+  if (m.tc(true, causal, &n)) {
     dO = dO.scalar_type() == at::kFloat && dO.is_contiguous() && reinterpret_cast<uintptr_t>(dO.data_ptr()) % 16 == 0 ? dO : bf16c(dO);
     Tensor g[3];
     for (int i = 0; i < 3; ++i)

@@ -63,7 +63,7 @@ extern "C" {
 #define FMTA_OP_BWD_FUSED 6      /* fmta_bwd_fused */
 /* Head mixing on the tensor cores (d = 64 or 128, groups of 2, 4, 8 or 16 heads, c_q <= 7): fmta_fwd with path -1 or 1 and a
  * workspace of FMTA_OP_MIX_FWD; fmta_mix_bwd with FMTA_OP_MIX_BWD.  P (and dC) of a few (batch, group) units at a time:
- * at most 4.5 GiB, or one unit's. */
+ * at most 4.5 GiB, or one unit's.  Of one call: fmta_mix_workspace_bytes. */
 #define FMTA_OP_MIX_FWD 7
 #define FMTA_OP_MIX_BWD 8
 
@@ -332,6 +332,10 @@ int fmta_bwd_dq_dw_static(const void* Q, const void* K, const void* V, const voi
 
 /* Bytes of caller-owned workspace an op needs for the given problem (0 if none). */
 size_t fmta_workspace_bytes(int op, int B, int H, int N, int d, int cq, int ck, int G);
+
+/* FMTA_OP_MIX_FWD (bwd = 0) or FMTA_OP_MIX_BWD for one call whose filter (has_theta) and mask (causal) are known: what that call
+ * lays out, never more than fmta_workspace_bytes, which has to cover all of them. */
+size_t fmta_mix_workspace_bytes(int bwd, int B, int H, int N, int d, int cq, int ck, int G, int has_theta, int causal);
 
 #ifdef __cplusplus
 }

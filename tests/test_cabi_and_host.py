@@ -89,6 +89,26 @@ def test_host_validation_needs_no_gpu():
     assert mix(64, None) == -5 and mix(128, None) == -3 and mix(64, good) == -3
 
 
+def test_mixing_workspace_covers_what_a_call_lays_out():
+    """fmta_workspace_bytes knows neither the mask nor (1 x 1) whether there is a filter: it has to cover every call."""
+    from fmta_b200._lib import lib
+    # without a filter, 16 heads, N = 2048, causal: 64-key chunks, so status word (1 KB, as the base's alignment), maxima,
+    # references and sums of 2 x 32 half chunks, and P
+    rp, n8 = 2048 + 16, 2048
+    laid_out = 2048 + 16 * 2 * 32 * 3 * rp * 4 + 16 * (n8 // 8) * rp * 16
+    assert lib.fmta_workspace_bytes(7, 1, 16, 2048, 64, 1, 1, 16) >= laid_out
+    assert lib.fmta_mix_workspace_bytes(0, 1, 16, 2048, 64, 1, 1, 16, 0, 1) == laid_out
+    for G in (2, 4, 8, 16):
+        for B, H in ((1, G), (2, G), (1, 4 * G), (7, 2 * G)):
+            for d in (64, 128):
+                for N in list(range(1, 4500, 97)) + [2048, 8192]:
+                    for bwd in (0, 1):
+                        for cq, ck, theta in ((1, 1, 0), (1, 1, 1), (6, 11, 1), (7, 7, 1)):
+                            most = lib.fmta_workspace_bytes(7 + bwd, B, H, N, d, cq, ck, G)
+                            for causal in (0, 1):
+                                assert lib.fmta_mix_workspace_bytes(bwd, B, H, N, d, cq, ck, G, theta, causal) <= most, (G, B, H, d, N, bwd, cq, causal)
+
+
 def test_ops_refuse_cpu_tensors():
     import fmta_b200 as F
     Q = torch.zeros(1, 2, 16, 64, dtype=torch.bfloat16)

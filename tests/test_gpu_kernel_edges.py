@@ -117,3 +117,29 @@ def test_mixing_tiles_and_groups(B, H, N, d, G, cq, ck, causal, spread):
     assert rel(o, Or) <= tol
     for got, ref in ((gq, dq), (gk, dk), (gv, dv), (gw, dw)) + (((gt, dth),) if cq else ()):
         assert torch.isfinite(got).all() and rel(got, ref) <= tol
+
+
+@pytest.mark.parametrize("B,H,N,G,causal", [(1, 16, 1600, 16, True), (1, 16, 2048, 16, True), (2, 16, 1500, 16, True), (1, 8, 2100, 8, True)])
+def test_mixing_stays_in_its_workspace(B, H, N, G, causal):
+    """Sizes whose key chunks depend on whether there is a filter: exactly the bytes that the library names, and what lies
+    behind them untouched."""
+    import fmta_b200 as F
+    from fmta_b200._lib import lib, ptr, stream_ptr
+    d, scale = 64, 0.125
+    g = torch.Generator(device="cuda").manual_seed(N)
+    q, k, v = (torch.randn(B, H, N, d, device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+    w = torch.randn(H // G, G, G, device="cuda", generator=g) / math.sqrt(G)
+    n = lib.fmta_mix_workspace_bytes(0, B, H, N, d, 1, 1, G, 0, int(causal))
+    guard = 16 << 20
+    ws = torch.full((n + guard,), 0x5A, dtype=torch.uint8, device="cuda")
+    o = torch.empty(B, H, N, d, device="cuda")
+    st = lib.fmta_fwd(ptr(q), ptr(k), ptr(v), None, ptr(w), ptr(o), None, None, None, B, H, N, d, 1, 1, G, scale, int(causal), 0, -1,
+                      ptr(ws), n, stream_ptr())
+    assert st == 0
+    assert bool((ws[n:] == 0x5A).all())
+    rows = [0, 1, 63, N // 2, N - 2, N - 1]
+    S = torch.einsum("bhid,bhjd->bhij", q[:, :, rows].double(), k.double()) * scale
+    X = torch.einsum("xgy,bxyij->bxgij", w.double(), S.view(B, H // G, G, len(rows), N)).reshape(B, H, len(rows), N)
+    if causal:
+        X = X.masked_fill(torch.arange(N, device="cuda")[None, :] > torch.tensor(rows, device="cuda")[:, None], float("-inf"))
+    assert maxabs(o[:, :, rows], torch.softmax(X, -1) @ v.double()) <= 2e-2
