@@ -6,7 +6,7 @@ namespace fmta {
 
 namespace {
 
-template <int D, int NR, int CKP, bool PAGED>
+template <int D, int NR, int CKP, bool PAGED, bool A32>
 cudaError_t launch_decode_t(const DecodeParams& p, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(p.k_splits * p.n_sub, p.H, p.B); cfg.blockDim = dim3(kDecWarps * 32); cfg.stream = stream;
@@ -23,12 +23,15 @@ cudaError_t launch_decode_t(const DecodeParams& p, cudaStream_t stream) {
     attr[cfg.numAttrs++].val.clusterDim.z = 1;
   }
   cfg.attrs = attr;
-  return cudaLaunchKernelEx(&cfg, decode_kernel<D, NR, CKP, PAGED>, p);
+  return cudaLaunchKernelEx(&cfg, decode_kernel<D, NR, CKP, PAGED, A32>, p);
 }
 
 template <int D, int NR, int CKP>
 cudaError_t launch_decode_p(const DecodeParams& p, cudaStream_t stream) {
-  return p.block_table ? launch_decode_t<D, NR, CKP, true>(p, stream) : launch_decode_t<D, NR, CKP, false>(p, stream);
+  constexpr bool kWide = D >= 64;            // head dim 32 has no 32-byte loads
+  const bool a32 = ((reinterpret_cast<uintptr_t>(p.K) | reinterpret_cast<uintptr_t>(p.V)) & 31) == 0;
+  if (kWide && !a32) return p.block_table ? launch_decode_t<D, NR, CKP, true, !kWide>(p, stream) : launch_decode_t<D, NR, CKP, false, !kWide>(p, stream);
+  return p.block_table ? launch_decode_t<D, NR, CKP, true, true>(p, stream) : launch_decode_t<D, NR, CKP, false, true>(p, stream);
 }
 template <int D, int NR>
 cudaError_t launch_decode_c(const DecodeParams& p, cudaStream_t stream) {

@@ -34,7 +34,9 @@ constexpr int kDecRow = 68;          // ring row stride in floats: even rows 8 b
 constexpr int kDecMaxPages = 2048;   // block-table entries of one sequence kept in shared memory (paged cache)
 
 // 16 or 32 bytes per lane, read once.  The 32-byte form lets the four lanes that share a K row of an MMA fragment fetch a whole
-// 128-byte line with one instruction (with 16 bytes they fetch half of it, and the L2 sees twice the requests).
+// 128-byte line with one instruction (with 16 bytes they fetch half of it, and the L2 sees twice the requests).  It needs K
+// and V on 32-byte boundaries (rows are 128 or 256 bytes, so the bases decide); the callers' contract is 16 bytes, and the
+// launcher takes the instantiations with two 16-byte loads (A32 = false) for bases in between.
 FMTA_DEVINL void ldg_nc_v4(uint32_t* v, const void* p) {
   asm volatile("ld.global.nc.L1::no_allocate.L2::256B.v4.b32 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
@@ -45,10 +47,15 @@ FMTA_DEVINL void ldg_nc_v8(uint32_t* v, const void* p) {
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                : "l"(p));
 }
-template <int W>
+template <int W, bool A32>
 FMTA_DEVINL void ldg_nc(uint32_t* v, const void* p, bool ok) {   // W words, zeros when !ok
   if (ok) {
-    if (W == 8) ldg_nc_v8(v, p); else ldg_nc_v4(v, p);
+    if (W == 8 && A32) {
+      ldg_nc_v8(v, p);
+    } else {
+      ldg_nc_v4(v, p);
+      if (W == 8) ldg_nc_v4(v + 4, reinterpret_cast<const unsigned char*>(p) + 16);
+    }
   } else {
 #pragma unroll
     for (int i = 0; i < W; ++i) v[i] = 0u;
@@ -62,8 +69,8 @@ __host__ __device__ inline int decode_keys_per_split(int Nk, int k_splits) {
 }
 
 // NR: query rows per lane in the conv (2t, 2t + 1 and, from 9 rows on, 8 + those): 2 or 4.  CKP: filter width the taps are padded
-// to with zeros (9: pad_k <= 4, 11: pad_k = 5, 17: any).
-template <int D, int NR, int CKP, bool PAGED>
+// to with zeros (9: pad_k <= 4, 11: pad_k = 5, 17: any).  A32: K and V start on 32-byte boundaries.
+template <int D, int NR, int CKP, bool PAGED, bool A32>
 __global__ void __launch_bounds__(kDecWarps * 32, D == 128 ? 3 : 4) decode_kernel(const DecodeParams p) {
   constexpr int KS = D / 16;               // k-steps of the QK MMA
   constexpr int KW = D >= 64 ? 8 : 4;      // words of a K row per lane and load: 4 lanes cover 128 bytes (64 at d = 32)
@@ -156,14 +163,14 @@ __global__ void __launch_bounds__(kDecWarps * 32, D == 128 ? 3 : 4) decode_kerne
     for (int j = 0; j < 2; ++j) {
       const bool ok = kb >= 0 && 8 * j + g < lim;
 #pragma unroll
-      for (int c = 0; c < KL; ++c) ldg_nc<KW>(&kf[j][c * KW], src + 8 * j * D + c * 8 * KW, ok);
+      for (int c = 0; c < KL; ++c) ldg_nc<KW, A32>(&kf[j][c * KW], src + 8 * j * D + c * 8 * KW, ok);
     }
   };
   auto load_v = [&](int kb, int sb) {                        // keys kb + 8 t + 4 sb + {0..3}: half of the 32-key block at kb
     const int k0 = kb + 8 * t + 4 * sb;
     const bf16* src = tile_base(p.V, kb + 16 * (t >> 1)) + (8 * (t & 1) + 4 * sb) * D + g * 2 * VW;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) ldg_nc<VW>(vf[e], src + e * D, k0 + e < Nk && (D >= 64 || g < 4));
+    for (int e = 0; e < 4; ++e) ldg_nc<VW, A32>(vf[e], src + e * D, k0 + e < Nk && (D >= 64 || g < 4));
   };
   auto scores = [&](int kb) {                                // S of the staged K tile -> ring
 #pragma unroll

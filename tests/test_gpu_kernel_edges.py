@@ -44,6 +44,37 @@ def test_decode_blocks_splits_and_filters(B, H, q_len, Nk, d, cq, ck, k_splits, 
     assert torch.equal(Op[:, :, 0:1], O) and torch.equal(Mp[:, :, 0:1], M) and torch.equal(Lp[:, :, 0:1], L)
 
 
+@pytest.mark.parametrize("off_k,off_v", [(8, 8), (8, 0), (0, 8), (16, 16)])       # elements: 16 bytes are 8
+@pytest.mark.parametrize("d,cq,ck,q_len", [(64, 6, 11, 6), (128, 6, 11, 6), (128, 3, 5, 3), (64, 16, 17, 16), (32, 3, 3, 3)])
+def test_decode_of_caches_on_16_byte_boundaries(d, cq, ck, q_len, off_k, off_v):
+    """A cache or page pool that is a view into a larger buffer: the same bits as from an aligned one."""
+    import fmta_b200 as F
+    B, H, page, pages = 2, 2, 64, 5
+    Nk, scale = page * pages - 7, 1.0 / math.sqrt(d)
+    g = torch.Generator(device="cuda").manual_seed(d + cq)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+
+    def moved(t, off):
+        buf = torch.zeros(t.numel() + 64, dtype=t.dtype, device="cuda")
+        v = buf[off:off + t.numel()].view(t.shape)
+        v.copy_(t)
+        assert v.data_ptr() % 32 == 2 * off % 32
+        return v
+
+    q, k, v = rn(B, H, q_len, d), rn(B, H, Nk, d), rn(B, H, Nk, d)
+    theta = 0.1 * torch.randn(H, cq, ck, device="cuda", generator=g)
+    args = (theta, 2, scale, cq - 1, (ck - 1) // 2)
+    want = F.forward_inference(q, k, v, *args, False)
+    got = F.forward_inference(q, moved(k, off_k), moved(v, off_v), *args, False)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    kp, vp = rn(B * pages, H, page, d), rn(B * pages, H, page, d)
+    table = torch.arange(B * pages, dtype=torch.int32, device="cuda").flip(0).view(B, pages).contiguous()
+    lens = torch.tensor([Nk, Nk - 100], dtype=torch.int32, device="cuda")
+    want = F.forward_inference_paged(q, kp, vp, table, *args, seq_lens=lens)
+    got = F.forward_inference_paged(q, moved(kp, off_k), moved(vp, off_v), table, *args, seq_lens=lens)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 @pytest.mark.parametrize("B,H,N,d,cq,ck,causal", [
     (1, 2, 123, 64, 6, 11, True),      # one row tile of the dQ pair, exactly (128 - 5)
     (1, 2, 247, 64, 6, 11, True),      # two tiles of it and one row
