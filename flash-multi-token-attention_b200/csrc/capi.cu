@@ -163,6 +163,7 @@ size_t fmta_workspace_bytes(int op, int B, int H, int N, int d, int cq, int ck, 
 
 size_t fmta_mix_workspace_bytes(int bwd, int B, int H, int N, int d, int cq, int ck, int G, int has_theta, int causal) {
   if (B < 1 || H < 1 || N < 1 || G < 2 || G > 16 || H % G != 0 || (has_theta && (cq < 1 || ck < 1))) return 0;
+  if (!mix_tc_shape(B, H, N, d, cq, G, has_theta != 0)) return 0;
   return mix_tc_call_bytes(B, H, N, d, cq, ck, G, has_theta != 0, causal != 0, bwd != 0);
 }
 

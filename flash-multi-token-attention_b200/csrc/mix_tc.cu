@@ -31,8 +31,10 @@ MixPlan plan(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool 
   m.U = B * (H / G);
   m.unit = (size_t)G * (m.N8 / 8) * m.RP * 16;
   const size_t per = m.unit * (bwd ? 2 : 1);
-  m.nU = (int)(kMixChunkBytes / per);
-  m.nU = m.nU < 1 ? 1 : (m.nU > m.U ? m.U : m.nU);
+  // grid.y of the launches counts a launch's units or heads: 65535 at most (short sequences of many)
+  const size_t fit = kMixChunkBytes / per, most = (size_t)(65535 / G);
+  m.nU = (int)(fit < 1 ? 1 : fit > most ? most : fit);
+  if (m.nU > m.U) m.nU = m.U;
   // keys per CTA: long chunks keep the row tile's operands and amortise the fixed cost of a CTA; about three CTAs per SM
   // (dead ones above the diagonal not counted) even out the load
   m.kch = 1024;
@@ -101,12 +103,16 @@ size_t bytes_of(const MixPlan& m) { MixBuffers b; return carve(m, nullptr, b); }
 
 }  // namespace
 
+bool mix_tc_shape(int B, int H, int N, int d, int cq, int G, bool conv) {
+  if (G != 2 && G != 4 && G != 8 && G != 16) return false;
+  if ((d != 64 && d != 128) || (conv && cq > 7)) return false;
+  if (conv && (long)B * H > 65535) return false;               // grid.y of the pre-pass and of its adjoint
+  const size_t n8 = (size_t)(N + 127) / 128 * 128;
+  return (size_t)G * (n8 / 8) * (n8 + 16) * 32 <= kMixUnitMax;
+}
+
 bool mix_tc_supported(const TrainParams& p) {
-  if (!p.Wmix || !tensor_maps_available()) return false;
-  if (p.G != 2 && p.G != 4 && p.G != 8 && p.G != 16) return false;
-  if ((p.d != 64 && p.d != 128) || (p.theta && p.cq > 7)) return false;
-  const size_t n8 = (size_t)(p.N + 127) / 128 * 128;
-  return (size_t)p.G * (n8 / 8) * (n8 + 16) * 32 <= kMixUnitMax;
+  return p.Wmix && mix_tc_shape(p.B, p.H, p.N, p.d, p.cq, p.G, p.theta != nullptr) && tensor_maps_available();
 }
 
 // What one call takes.

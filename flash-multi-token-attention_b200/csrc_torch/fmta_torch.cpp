@@ -273,14 +273,12 @@ struct Mix {
   int G;
   Tensor w, theta;        // fp32 [H/G, G, G]; fp32 [H, cq, ck] or undefined
   bool tc(bool bwd, bool causal, size_t* bytes) const {                 // the tensor-core kernels take this problem
-    if (exact_only() || (s.d != 64 && s.d != 128) || G > 16 || (theta.defined() && s.cq > 7)) return false;
+    if (exact_only()) return false;
     // a short sequence without a filter: the 16-row CTAs of the other kernels finish sooner than one 128-row CTA of these (16
     // heads, d = 64, forward + backward on an idle GPU: 12 us per 16 keys there; 190 us at N = 640, 208 at N = 1024 here)
     if (!theta.defined() && G >= 8 && s.N <= 224 && (long)s.B * (s.H / G) * ((s.N + 15) / 16) <= 2 * 148) return false;
-    const size_t n8 = ((size_t)s.N + 127) / 128 * 128;     // P and dC of one (batch, group) unit: see fmta_mix_bwd
-    if ((size_t)G * (n8 / 8) * (n8 + 16) * 32 > ((size_t)16 << 30)) return false;
     *bytes = fmta_mix_workspace_bytes(bwd, s.B, s.H, s.N, s.d, s.cq, s.ck, G, theta.defined(), causal);
-    return true;
+    return *bytes != 0;
   }
   size_t exchange(int64_t limit) const {
     if (!theta.defined()) return 0;

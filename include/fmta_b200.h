@@ -334,7 +334,8 @@ int fmta_bwd_dq_dw_static(const void* Q, const void* K, const void* V, const voi
 size_t fmta_workspace_bytes(int op, int B, int H, int N, int d, int cq, int ck, int G);
 
 /* FMTA_OP_MIX_FWD (bwd = 0) or FMTA_OP_MIX_BWD for one call whose filter (has_theta) and mask (causal) are known: what that call
- * lays out, never more than fmta_workspace_bytes, which has to cover all of them. */
+ * lays out, never more than fmta_workspace_bytes, which has to cover all of them.  0: the tensor-core kernels do not take the
+ * problem. */
 size_t fmta_mix_workspace_bytes(int bwd, int B, int H, int N, int d, int cq, int ck, int G, int has_theta, int causal);
 
 #ifdef __cplusplus

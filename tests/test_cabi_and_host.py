@@ -109,6 +109,17 @@ def test_mixing_workspace_covers_what_a_call_lays_out():
                                 assert lib.fmta_mix_workspace_bytes(bwd, B, H, N, d, cq, ck, G, theta, causal) <= most, (G, B, H, d, N, bwd, cq, causal)
 
 
+def test_mixing_grids_stay_in_range():
+    """grid.y counts heads: a launch takes 65535 of them at most, and what has no loop over launches is left to other kernels."""
+    from fmta_b200._lib import lib
+    one = lib.fmta_mix_workspace_bytes(0, 1, 16, 128, 64, 1, 1, 16, 0, 0)
+    assert one > 0
+    unit = 16 * 16 * (128 + 16) * 16
+    assert lib.fmta_mix_workspace_bytes(0, 8192, 16, 128, 64, 1, 1, 16, 0, 0) < 65536 // 16 * (unit + one)
+    assert lib.fmta_mix_workspace_bytes(0, 32767, 2, 16, 64, 3, 3, 2, 1, 1) > 0
+    assert lib.fmta_mix_workspace_bytes(0, 32768, 2, 16, 64, 3, 3, 2, 1, 1) == 0
+
+
 def test_ops_refuse_cpu_tensors():
     import fmta_b200 as F
     Q = torch.zeros(1, 2, 16, 64, dtype=torch.bfloat16)

@@ -174,3 +174,22 @@ def test_mixing_stays_in_its_workspace(B, H, N, G, causal):
     if causal:
         X = X.masked_fill(torch.arange(N, device="cuda")[None, :] > torch.tensor(rows, device="cuda")[:, None], float("-inf"))
     assert maxabs(o[:, :, rows], torch.softmax(X, -1) @ v.double()) <= 2e-2
+
+
+@pytest.mark.parametrize("G,N,conv", [(16, 16, False), (16, 128, False), (2, 16, True)])
+def test_mixing_more_heads_than_a_grid_dimension(G, N, conv):
+    """65552 heads: forward and backward against float64 at the first and last sequences."""
+    import fmta_b200 as F
+    B, H, d, scale = 65552 // G, G, 64, 0.125
+    g = torch.Generator(device="cuda").manual_seed(N)
+    q, k, v, do = (torch.randn(B, H, N, d, device="cuda", generator=g, dtype=torch.bfloat16) for _ in range(4))
+    w = torch.eye(G, device="cuda")[None] + 0.1 * torch.randn(1, G, G, device="cuda", generator=g)
+    theta = 0.3 * torch.randn(H, 3, 3, device="cuda", generator=g) if conv else None
+    o, l, m, lse = F.conv_headmix_forward(q, k, v, w, theta, scale, True, out_dtype=torch.float32)
+    dq, dk, dv, _, _ = F.conv_headmix_backward(q, k, v, w, o, do, l, m, theta, True, scale, lse=lse)
+    for b in (0, B // 2, B - 1):
+        Q, K, V, dO = (t[b:b + 1].float().cpu() for t in (q, k, v, do))
+        wf, th = w[0].cpu(), theta.cpu() if conv else None
+        ref = (orc.conv_headmix_fwd(Q, K, V, th, wf, scale, True)[0],) + orc.conv_headmix_bwd_autograd(Q, K, V, th, wf, dO, scale, True)[:3]
+        for got, want in zip((o, dq, dk, dv), ref):
+            assert maxabs(got[b:b + 1], want) <= 3e-2
