@@ -173,12 +173,33 @@ def backward(Q, K, V, dO, D, L, conv_kernel, scale, pad_q, pad_k, causal, path=-
 
 class FlashConvAttentionCUDAFunction(torch.autograd.Function):
     """The operator of conv_attention_cuda.py:96-163: same argument list of ``apply``.  Its autograd node is native
-    (csrc_torch/fmta_torch.cpp), so ``apply`` goes there directly."""
+    (csrc_torch/fmta_torch.cpp), so ``apply`` goes there directly; under ``torch.jit.trace``, which would record the native
+    call's allocations and nothing of what fills them, it goes through the node below, which a trace keeps as one operator."""
 
     @staticmethod
     def apply(Q, K, V, conv_kernel, scale, pad_q, pad_k, causal):
+        if torch.jit.is_tracing():
+            return super(FlashConvAttentionCUDAFunction, FlashConvAttentionCUDAFunction).apply(Q, K, V, conv_kernel, scale, pad_q,
+                                                                                               pad_k, causal)
         return _native.conv_attention(Q, K, V, conv_kernel, scale, pad_q, pad_k, bool(causal),
                                       1 << 62 if KEEP_KTILDE else KEEP_KTILDE_BYTES, STREAM_LIMIT_BYTES, PAD_D32)
+
+    @staticmethod
+    def forward(ctx, Q, K, V, conv_kernel, scale, pad_q, pad_k, causal):
+        Qb, Kb, Vb = (t.to(torch.bfloat16).contiguous() for t in (Q, K, V))
+        O, _, _, LSE = forward(Qb, Kb, Vb, conv_kernel, scale, pad_q, pad_k, causal, return_lse=True)
+        ctx.save_for_backward(Qb, Kb, Vb, conv_kernel, LSE, O)
+        ctx.args = (scale, pad_q, pad_k, causal)
+        ctx.in_dtypes = (Q.dtype, K.dtype, V.dtype)
+        return O
+
+    @staticmethod
+    def backward(ctx, dO):
+        Q, K, V, conv_kernel, LSE, O = ctx.saved_tensors
+        dOb = dO.to(torch.bfloat16).contiguous()
+        dQ, dK, dV, dTheta = backward(Q, K, V, dOb, rowdot(dOb, O), LSE, conv_kernel, *ctx.args)
+        tq, tk, tv = ctx.in_dtypes
+        return dQ.to(tq), dK.to(tk), dV.to(tv), dTheta.to(conv_kernel.dtype), None, None, None, None
 
 
 class ConvAttentionCUDA(nn.Module):

@@ -71,13 +71,29 @@ def head_conv_attention_bwd_dkdv(q, k, v, w, o, do, l, m, causal=False, scale=No
 
 
 class HeadConvAttentionFunction(torch.autograd.Function):
-    """Same argument list of ``apply`` as head_conv_attn.py:11-63; the autograd node is native (csrc_torch/fmta_torch.cpp)."""
+    """Same argument list of ``apply`` as head_conv_attn.py:11-63; the autograd node is native (csrc_torch/fmta_torch.cpp),
+    except under ``torch.jit.trace`` (see FlashConvAttentionCUDAFunction)."""
 
     @staticmethod
     def apply(q, k, v, w, causal=False, scale=None):
         if scale is None:
             scale = 1.0 / math.sqrt(q.shape[-1])
+        if torch.jit.is_tracing():
+            return super(HeadConvAttentionFunction, HeadConvAttentionFunction).apply(q, k, v, w, causal, scale)
         return _native.mix_attention(q, k, v, None, w, scale, bool(causal), False, MIX_EXCHANGE_LIMIT_BYTES)
+
+    @staticmethod
+    def forward(ctx, q, k, v, w, causal, scale):
+        o, l, m = head_conv_attention_forward(q, k, v, w, scale=scale, causal=causal)
+        ctx.save_for_backward(q, k, v, w, o, l, m)
+        ctx.causal, ctx.scale = causal, scale
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        q, k, v, w, o, l, m = ctx.saved_tensors
+        dq, dk, dv, dw, _ = conv_headmix_backward(q, k, v, w, o, do, l, m, None, ctx.causal, ctx.scale)
+        return dq.to(q.dtype), dk.to(k.dtype), dv.to(v.dtype), dw.to(w.dtype), None, None
 
 
 class HeadConvAttention(nn.Module):
@@ -103,7 +119,22 @@ class ConvHeadMixFunction(torch.autograd.Function):
 
     @staticmethod
     def apply(q, k, v, conv_kernel, w, causal, scale):
+        if torch.jit.is_tracing():
+            return super(ConvHeadMixFunction, ConvHeadMixFunction).apply(q, k, v, conv_kernel, w, causal, scale)
         return _native.mix_attention(q, k, v, conv_kernel, w, scale, bool(causal), True, MIX_EXCHANGE_LIMIT_BYTES)
+
+    @staticmethod
+    def forward(ctx, q, k, v, conv_kernel, w, causal, scale):
+        o, l, m, lse = conv_headmix_forward(q, k, v, w, conv_kernel, scale, causal, out_dtype=torch.float32)
+        ctx.save_for_backward(q, k, v, conv_kernel, w, o, l, m, lse)
+        ctx.causal, ctx.scale = causal, scale
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        q, k, v, conv_kernel, w, o, l, m, lse = ctx.saved_tensors
+        dq, dk, dv, dw, dth = conv_headmix_backward(q, k, v, w, o, do, l, m, conv_kernel, ctx.causal, ctx.scale, lse=lse)
+        return dq.to(q.dtype), dk.to(k.dtype), dv.to(v.dtype), dth.to(conv_kernel.dtype), dw.to(w.dtype), None, None
 
 
 def conv_headmix_attention(q, k, v, conv_kernel, w, causal=True, scale=None):

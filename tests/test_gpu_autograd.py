@@ -1,0 +1,56 @@
+"""The operators under torch's tracing, transforms, threads and saved-tensor hooks."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(seed, H=4, N=130, d=64):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    q, k, v = (torch.randn(1, H, N, d, device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+    theta = torch.zeros(H, 3, 5, device="cuda")
+    theta[:, 2, 2] = 1.0
+    theta += 0.1 * torch.randn(H, 3, 5, device="cuda", generator=g)
+    w = torch.eye(H, device="cuda") + 0.1 * torch.randn(H, H, device="cuda", generator=g)
+    return q, k, v, theta, w
+
+
+def _ops():
+    import fmta_b200 as F
+    scale = 1.0 / math.sqrt(64)
+    return {
+        "conv": lambda q, k, v, t, w: F.FlashConvAttentionCUDAFunction.apply(q, k, v, t, scale, 2, 2, True),
+        "mix": lambda q, k, v, t, w: F.head_conv_attention(q, k, v, w, True, scale),
+        "conv_mix": lambda q, k, v, t, w: F.conv_headmix_attention(q, k, v, t, w[None], True, scale),
+    }
+
+
+@pytest.mark.parametrize("name", ["conv", "mix", "conv_mix"])
+@pytest.mark.parametrize("grad", [False, True])
+def test_a_trace_computes(name, grad):
+    """A traced operator answers new inputs, and differentiates, as the operator itself does."""
+    op = _ops()[name]
+    first, second = _inputs(0), _inputs(1)
+    for t in first:
+        t.requires_grad_(grad)
+    traced = torch.jit.trace(op, first, check_trace=False)
+    for t in second:
+        t.requires_grad_(grad)
+    got, want = traced(*second), op(*second)
+    assert torch.equal(got, want)
+    if grad:
+        wrt = [t for t, used in zip(second, (1, 1, 1, name != "mix", name != "conv")) if used]
+        do = torch.randn_like(want)
+        for a, b in zip(torch.autograd.grad(got, wrt, do), torch.autograd.grad(want, wrt, do)):
+            assert float((a.float() - b.float()).norm()) <= 4e-3 * float(b.float().norm())     # gradients rounded to bf16 on their own
+
+
+@pytest.mark.parametrize("name", ["conv", "mix", "conv_mix"])
+def test_compiled_around(name):
+    op = _ops()[name]
+    args = _inputs(2)
+    torch._dynamo.reset()
+    f = torch.compile(lambda *a: op(*a) * 2, backend="eager")
+    assert torch.equal(f(*args), op(*args) * 2)
