@@ -46,6 +46,13 @@ void require_on(const Tensor& ref, const Tensor& t, const char* name, at::IntArr
   FMTA_REQUIRE(t.sizes() == shape, name, " must have shape ", shape, " (got ", t.sizes(), ")");
 }
 
+// Where the autograd node is passed by (nothing requires grad), forward-mode tangents would be lost without a word; with the
+// node torch refuses them.
+void refuse_tangents(std::initializer_list<const Tensor*> inputs) {
+  for (const Tensor* t : inputs)
+    FMTA_REQUIRE(!t->defined() || !t->_fw_grad(/*level=*/0).defined(), "forward-mode differentiation of this operator is not implemented");
+}
+
 // The status word of a device is created and registered by the Python module on first use.
 std::atomic<bool> g_armed[64];
 void arm_status(const Tensor& t) {
@@ -253,6 +260,7 @@ Tensor conv_attention(const Tensor& Q, const Tensor& K, const Tensor& V, const T
   c10::cuda::CUDAGuard guard(Q.device());
   if (at::GradMode::is_enabled() && (Q.requires_grad() || K.requires_grad() || V.requires_grad() || theta_.requires_grad()))
     return ConvAttnFn::apply(Q, K, V, theta_, scale, pad_q, pad_k, causal, keep_limit, stream_limit, pad_d32);
+  refuse_tangents({&Q, &K, &V, &theta_});
   at::AutoGradMode no_grad(false);
   const bool pad = wants_pad(Q, theta_, pad_d32);
   Tensor q = bf16c(Q), k = bf16c(K), v = bf16c(V);
@@ -457,6 +465,7 @@ Tensor mix_attention(const Tensor& q, const Tensor& k, const Tensor& v, const st
   c10::cuda::CUDAGuard guard(q.device());
   if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad() || w.requires_grad() || (theta.defined() && theta.requires_grad())))
     return MixFn::apply(q, k, v, theta_, w, scale, causal, out32, xlimit);
+  refuse_tangents({&q, &k, &v, &theta, &w});
   at::AutoGradMode no_grad(false);
   const Mix m = mix_of(q, w, theta);
   const Tensor O = at::empty(q.sizes(), q.options().dtype(out32 ? at::kFloat : mix_out_dtype(q, std::nullopt)));

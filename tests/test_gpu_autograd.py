@@ -54,3 +54,18 @@ def test_compiled_around(name):
     torch._dynamo.reset()
     f = torch.compile(lambda *a: op(*a) * 2, backend="eager")
     assert torch.equal(f(*args), op(*args) * 2)
+
+
+@pytest.mark.parametrize("name", ["conv", "mix", "conv_mix"])
+@pytest.mark.parametrize("which", [0, 2, 3, 4])
+@pytest.mark.parametrize("grad,grad_mode", [(False, True), (False, False), (True, True), (True, False)])
+def test_forward_mode_is_refused(name, which, grad, grad_mode):
+    """No tangent is dropped silently, whether or not the autograd node is passed by."""
+    if (name, which) in (("conv", 4), ("mix", 3)):
+        pytest.skip("not an input of the operator")
+    op = _ops()[name]
+    with torch.autograd.forward_ad.dual_level():
+        args = [t.clone().requires_grad_(grad) for t in _inputs(3)]
+        args[which] = torch.autograd.forward_ad.make_dual(args[which], torch.ones_like(args[which]))
+        with torch.set_grad_enabled(grad_mode), pytest.raises((RuntimeError, NotImplementedError)):
+            op(*args)
