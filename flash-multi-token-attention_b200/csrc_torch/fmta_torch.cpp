@@ -69,6 +69,10 @@ float* fptr(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullpt
 
 Tensor f32(const Tensor& t) { return t.scalar_type() == at::kFloat && t.is_contiguous() ? t : t.to(at::kFloat).contiguous(); }
 Tensor bf16c(const Tensor& t) { return t.scalar_type() == at::kBFloat16 && t.is_contiguous() ? t : t.to(at::kBFloat16).contiguous(); }
+bool on16(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
+// an output that comes back to a backward may be any view of the caller's (its own argument, an unpacked saved tensor); the
+// one-call backwards read it in 16-byte pieces
+Tensor aligned(const Tensor& t) { return on16(t) ? t : t.clone(); }
 Tensor new_f32(const Tensor& like, at::IntArrayRef shape) { return at::empty(shape, like.options().dtype(at::kFloat)); }
 Tensor new_bytes(const Tensor& like, size_t n) { return at::empty({(int64_t)(n < 16 ? 16 : n)}, like.options().dtype(at::kByte)); }
 int dtype_code(at::ScalarType t) { return t == at::kBFloat16 ? FMTA_DTYPE_BF16 : FMTA_DTYPE_F32; }
@@ -227,11 +231,12 @@ struct ConvAttnFn : public torch::autograd::Function<ConvAttnFn> {
     const Tensor theta = f32(theta_);
     const Dims s{(int)q.size(0), (int)q.size(1), (int)q.size(2), (int)q.size(3), (int)theta.size(1), (int)theta.size(2)};
     if (pad) { O = pad64(O); dO = pad64(dO); }
+    O = aligned(O);
     Tensor g[3], dT;
     const int op = conv_backward_op(s, -1, -1, stream_limit);
     if (bwd_tc_shape(s) && !exact_only() && op == FMTA_OP_BWD_TC) {
       arm_status(q);
-      dO = dO.scalar_type() == at::kFloat && dO.is_contiguous() && reinterpret_cast<uintptr_t>(dO.data_ptr()) % 16 == 0 ? dO : bf16c(dO);
+      dO = dO.scalar_type() == at::kFloat && dO.is_contiguous() && on16(dO) ? dO : bf16c(dO);
       const bool g16 = ty[0] == at::kBFloat16 && ty[1] == at::kBFloat16 && ty[2] == at::kBFloat16;
       for (auto& t : g) t = at::empty(q.sizes(), q.options().dtype(g16 ? at::kBFloat16 : at::kFloat));
       dT = new_f32(q, {s.H, s.cq, s.ck});
@@ -342,7 +347,7 @@ std::vector<Tensor> mix_backward_raw(const Mix& m, const Tensor& q, const Tensor
   const Tensor dW = want & 1 ? new_f32(q, {s.H / m.G, m.G, m.G}) : Tensor(), dT = conv ? new_f32(q, {s.H, s.cq, s.ck}) : Tensor();
   size_t n = 0;
   if (m.tc(true, causal, &n)) {
-    dO = dO.scalar_type() == at::kFloat && dO.is_contiguous() && reinterpret_cast<uintptr_t>(dO.data_ptr()) % 16 == 0 ? dO : bf16c(dO);
+    dO = dO.scalar_type() == at::kFloat && dO.is_contiguous() && on16(dO) ? dO : bf16c(dO);
     Tensor g[3];
     for (int i = 0; i < 3; ++i)
       if (conv || (i == 0 ? want & 1 : want & 2)) g[i] = at::empty(q.sizes(), q.options().dtype(g16 ? at::kBFloat16 : at::kFloat));
@@ -410,7 +415,7 @@ std::vector<Tensor> mix_backward(const Tensor& q, const Tensor& k, const Tensor&
   const Mix m = mix_of(q, w, theta);
   require_on(q, l, "l", {m.s.B, m.s.H, m.s.N}); require_on(q, mx, "m", {m.s.B, m.s.H, m.s.N});
   const Tensor lse = lse_ ? f32(*lse_) : at::add(f32(mx), at::log(f32(l)));
-  const Tensor oc = o.scalar_type() == at::kBFloat16 ? o.contiguous() : f32(o);
+  const Tensor oc = aligned(o.scalar_type() == at::kBFloat16 ? o.contiguous() : f32(o));
   auto g = mix_backward_raw(m, bf16c(q), bf16c(k), bf16c(v), bf16c(dO), oc, lse, scale ? *scale : 1.0 / std::sqrt((double)m.s.d), causal, (int)want, false, xlimit);
   if (g[3].defined()) g[3] = g[3].reshape(w.sizes());
   return g;
@@ -441,7 +446,7 @@ struct MixFn : public torch::autograd::Function<MixFn> {
                                   (at::ScalarType)ctx->saved_data["tv"].toInt()};
     c10::cuda::CUDAGuard guard(q.device());
     const Tensor dO = grads[0].defined() ? grads[0] : at::zeros_like(out);
-    const Tensor O = out.scalar_type() == at::kBFloat16 ? out.contiguous() : f32(out);
+    const Tensor O = aligned(out.scalar_type() == at::kBFloat16 ? out.contiguous() : f32(out));
     const bool g16 = ty[0] == at::kBFloat16 && ty[1] == at::kBFloat16 && ty[2] == at::kBFloat16;
     // without a filter each half of the gradients is a set of kernels of its own
     const bool has_theta = ctx->saved_data["has_theta"].toBool();

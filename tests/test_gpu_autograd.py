@@ -69,3 +69,46 @@ def test_forward_mode_is_refused(name, which, grad, grad_mode):
         args[which] = torch.autograd.forward_ad.make_dual(args[which], torch.ones_like(args[which]))
         with torch.set_grad_enabled(grad_mode), pytest.raises((RuntimeError, NotImplementedError)):
             op(*args)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("conv", [False, True])
+def test_backward_of_an_output_on_any_address(dtype, conv):
+    """The output that the caller hands back may be a view that starts anywhere in a buffer."""
+    import fmta_b200 as F
+    q, k, v, theta, w = _inputs(4, N=300)
+    th = theta if conv else None
+    o, l, m, lse = F.conv_headmix_forward(q, k, v, w, th, 0.125, True, out_dtype=dtype)
+    do = torch.randn(q.shape, device="cuda").to(torch.bfloat16)
+    buf = torch.zeros(o.numel() + 8, dtype=dtype, device="cuda")
+    moved = buf[1:1 + o.numel()].view(o.shape)
+    moved.copy_(o)
+    assert moved.data_ptr() % 16 != 0
+    want = F.conv_headmix_backward(q, k, v, w, o, do, l, m, th, True, 0.125)
+    got = F.conv_headmix_backward(q, k, v, w, moved, do, l, m, th, True, 0.125)
+    assert all((a is None and b is None) or torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("name", ["conv", "mix", "conv_mix"])
+def test_saved_tensors_may_come_back_anywhere(name):
+    """Saved-tensor hooks may give the backward copies of what it saved, on other addresses."""
+    op = _ops()[name]
+
+    def unpack(t):
+        if t.dtype == torch.bfloat16:            # operands of the tensor cores: 16-byte boundaries, as everywhere
+            return t.clone()
+        buf = torch.zeros(t.numel() + 4, dtype=t.dtype, device="cuda")
+        buf[1:1 + t.numel()].view(t.shape).copy_(t)
+        return buf[1:1 + t.numel()].view(t.shape)
+
+    grads = []
+    for hooks in (False, True):
+        args = [t.clone().requires_grad_() for t in _inputs(5)]
+        wrt = [t for t, used in zip(args, (1, 1, 1, name != "mix", name != "conv")) if used]
+        if hooks:
+            with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+                o = op(*args)
+        else:
+            o = op(*args)
+        grads.append(torch.autograd.grad(o, wrt, torch.ones_like(o)))
+    assert all(torch.equal(a, b) for a, b in zip(*grads))
