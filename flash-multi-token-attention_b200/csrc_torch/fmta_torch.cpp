@@ -218,7 +218,8 @@ struct ConvAttnFn : public torch::autograd::Function<ConvAttnFn> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     at::AutoGradMode no_grad(false);
     const auto saved = ctx->get_saved_variables();
-    const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &theta_ = saved[3], &LSE = saved[4], &kt = saved[6];
+    const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &theta_ = saved[3], &LSE = saved[4];
+    const Tensor kt = exact_only() ? Tensor() : saved[6];     // (the exact kernels, chosen since the forward, do not use it)
     Tensor O = saved[5], dO = grads[0];
     const double scale = ctx->saved_data["s"].toDouble();
     const int64_t flags = ctx->saved_data["f"].toInt();

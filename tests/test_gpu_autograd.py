@@ -112,3 +112,24 @@ def test_saved_tensors_may_come_back_anywhere(name):
             o = op(*args)
         grads.append(torch.autograd.grad(o, wrt, torch.ones_like(o)))
     assert all(torch.equal(a, b) for a, b in zip(*grads))
+
+
+def test_exact_kernels_chosen_between_forward_and_backward():
+    """The process-wide choice of kernels holds for a backward whose forward ran before it."""
+    import fmta_b200 as F
+    from fmta_b200._lib import lib
+    q, k, v, theta, _ = _inputs(6)
+    scale, do = 0.125, torch.randn(q.shape, device="cuda")
+    args = [t.clone().requires_grad_() for t in (q, k, v, theta)]
+    o = F.FlashConvAttentionCUDAFunction.apply(*args, scale, 2, 2, True)
+    old = lib.fmta_set_path(0)
+    try:
+        got = torch.autograd.grad(o, args, do)
+    finally:
+        lib.fmta_set_path(old)
+    from fmta_b200 import conv_attn
+    O, M, L, LSE = conv_attn.forward(q, k, v, theta, scale, 2, 2, True, return_lse=True)
+    assert torch.equal(O, o)
+    dob = do.to(torch.bfloat16)
+    want = conv_attn.backward(q, k, v, dob, conv_attn.rowdot(dob, O), LSE, theta, scale, 2, 2, True, path=0)
+    assert all(torch.equal(a, b.to(a.dtype)) for a, b in zip(got, want))
