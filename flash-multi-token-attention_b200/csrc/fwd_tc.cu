@@ -510,14 +510,29 @@ EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// bf16 tensor viewed as [outer][rows][D] (D contiguous); box = {box_x, box_rows, 1}
+// cuTensorMapEncodeTiled wants a current context, which a thread gets with its first runtime call that needs one: a thread
+// whose first call of this library comes to a kernel without a pre-pass has none yet, and the driver crashes there.
+bool context_current() {
+  typedef CUresult (*GetCurrentFn)(CUcontext*);
+  static const GetCurrentFn fn = [] {
+    void* ptr = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPoint("cuCtxGetCurrent", &ptr, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess
+               ? reinterpret_cast<GetCurrentFn>(ptr) : nullptr;
+  }();
+  CUcontext ctx = nullptr;
+  if (fn && fn(&ctx) == CUDA_SUCCESS && ctx) return true;
+  int dev = -1;
+  return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
+}
 }  // namespace
 
 bool tensor_maps_available() { return get_encode_fn() != nullptr; }
 
+// bf16 tensor viewed as [outer][rows][D] (D contiguous); box = {box_x, box_rows, box_outer}
 bool make_tensor_map_bf16(CUtensorMap* map, const void* base, int D, int rows, size_t outer, int box_x, int box_rows, bool sw128, int box_outer = 1) {
   EncodeTiledFn fn = get_encode_fn();
-  if (!fn) return false;
+  if (!fn || !context_current()) return false;
   cuuint64_t dims[3] = {(cuuint64_t)D, (cuuint64_t)rows, (cuuint64_t)outer};
   cuuint64_t strides[2] = {(cuuint64_t)D * 2, (cuuint64_t)rows * D * 2};
   cuuint32_t box[3] = {(cuuint32_t)box_x, (cuuint32_t)box_rows, (cuuint32_t)box_outer};
@@ -530,7 +545,7 @@ bool make_tensor_map_bf16(CUtensorMap* map, const void* base, int D, int rows, s
 // fp32 tensor viewed as [outer][rows][D] (D contiguous); box = {box_x, box_rows, 1}; box_x * 4 <= 128 with the swizzle
 bool make_tensor_map_f32(CUtensorMap* map, const void* base, int D, int rows, size_t outer, int box_x, int box_rows, bool sw128) {
   EncodeTiledFn fn = get_encode_fn();
-  if (!fn) return false;
+  if (!fn || !context_current()) return false;
   cuuint64_t dims[3] = {(cuuint64_t)D, (cuuint64_t)rows, (cuuint64_t)outer};
   cuuint64_t strides[2] = {(cuuint64_t)D * 4, (cuuint64_t)rows * D * 4};
   cuuint32_t box[3] = {(cuuint32_t)box_x, (cuuint32_t)box_rows, 1};

@@ -1,5 +1,6 @@
 """The operators under torch's tracing, transforms, threads and saved-tensor hooks."""
 import math
+import threading
 
 import pytest
 import torch
@@ -133,3 +134,26 @@ def test_exact_kernels_chosen_between_forward_and_backward():
     dob = do.to(torch.bfloat16)
     want = conv_attn.backward(q, k, v, dob, conv_attn.rowdot(dob, O), LSE, theta, scale, 2, 2, True, path=0)
     assert all(torch.equal(a, b.to(a.dtype)) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("name", ["mix", "conv", "conv_mix", "conv_kept_keys"])
+def test_first_call_of_a_thread(name):
+    """A thread whose first use of the GPU is this call (its memory comes from the allocator's cache)."""
+    import fmta_b200 as F
+    from fmta_b200 import conv_attn
+    q, k, v, theta, w = _inputs(8)
+    kt = conv_attn.ktilde_buffer(q, theta)
+    ops = dict(_ops(), conv_kept_keys=lambda q, k, v, t, w: conv_attn.forward(q, k, v, t, 0.125, 2, 2, True, ktilde=kt)[0])
+
+    def call(out):
+        with torch.no_grad():
+            out.append(ops[name](q, k, v, theta, w))
+
+    want, got = [], []
+    call(want)
+    call(want)
+    torch.cuda.synchronize()
+    worker = threading.Thread(target=call, args=(got,))
+    worker.start()
+    worker.join()
+    assert len(got) == 1 and torch.equal(got[0], want[0])
