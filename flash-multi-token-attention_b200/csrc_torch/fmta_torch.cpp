@@ -278,6 +278,7 @@ Tensor conv_attention(const Tensor& Q, const Tensor& K, const Tensor& V, const T
 
 // ---------------------------------------------------------------- head mixing
 [[noreturn]] void not_implemented(const std::string& what) {
+  pybind11::gil_scoped_acquire gil;
   PyErr_SetString(PyExc_NotImplementedError, what.c_str());
   throw pybind11::error_already_set();
 }
@@ -545,15 +546,18 @@ void kv_append_paged(const Tensor& Kp, const Tensor& Vp, const Tensor& table, co
 
 }  // namespace
 
+// A launch waits for room in the GPU's queue and an allocation for the driver: other threads of the interpreter run meanwhile
+using nogil = pybind11::call_guard<pybind11::gil_scoped_release>;
+
 PYBIND11_MODULE(_native, m) {
-  m.def("conv_forward", &conv_forward);
-  m.def("conv_backward", &conv_backward);
-  m.def("conv_attention", &conv_attention);
-  m.def("rowdot", &rowdot);
-  m.def("mix_forward", &mix_forward);
-  m.def("mix_backward", &mix_backward);
-  m.def("mix_attention", &mix_attention);
-  m.def("decode", &decode);
-  m.def("decode_paged", &decode_paged);
-  m.def("kv_append_paged", &kv_append_paged);
+  m.def("conv_forward", &conv_forward, nogil());
+  m.def("conv_backward", &conv_backward, nogil());
+  m.def("conv_attention", &conv_attention, nogil());
+  m.def("rowdot", &rowdot, nogil());
+  m.def("mix_forward", &mix_forward, nogil());
+  m.def("mix_backward", &mix_backward, nogil());
+  m.def("mix_attention", &mix_attention, nogil());
+  m.def("decode", &decode, nogil());
+  m.def("decode_paged", &decode_paged, nogil());
+  m.def("kv_append_paged", &kv_append_paged, nogil());
 }

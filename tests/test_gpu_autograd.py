@@ -1,6 +1,7 @@
 """The operators under torch's tracing, transforms, threads and saved-tensor hooks."""
 import math
 import threading
+import time
 
 import pytest
 import torch
@@ -157,3 +158,38 @@ def test_first_call_of_a_thread(name):
     worker.start()
     worker.join()
     assert len(got) == 1 and torch.equal(got[0], want[0])
+
+
+@pytest.mark.parametrize("name", ["conv", "mix", "decode"])
+def test_other_threads_run_while_a_launch_waits(name):
+    """A call that waits for room in the GPU's launch queue does not hold the interpreter."""
+    import fmta_b200 as F
+    q, k, v, theta, w = _inputs(7)
+    ops = dict(_ops(), decode=lambda q, k, v, t, w: F.forward_inference(q[:, :, :3].contiguous(), k, v, t, 1, 0.1, 2, 2, False))
+
+    def call():
+        with torch.no_grad():
+            ops[name](q, k, v, theta, w)
+
+    call()
+    torch.cuda.synchronize()
+    took = []
+
+    def fill():
+        t0 = time.perf_counter()
+        for _ in range(2500):
+            call()
+        took.append(time.perf_counter() - t0)
+
+    torch.cuda._sleep(3_000_000_000)            # about 1.6 s on the GPU: everything behind it queues up
+    worker = threading.Thread(target=fill)
+    worker.start()
+    gap, last = 0.0, time.perf_counter()
+    while worker.is_alive():
+        time.sleep(0.001)
+        now = time.perf_counter()
+        gap, last = max(gap, now - last), now
+    worker.join()
+    torch.cuda.synchronize()
+    assert took[0] > 1.0                        # the queue did fill
+    assert gap < 0.3
