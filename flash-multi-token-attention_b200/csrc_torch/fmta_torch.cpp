@@ -383,6 +383,7 @@ std::vector<Tensor> mix_backward_raw(const Mix& m, const Tensor& q, const Tensor
 }
 
 at::ScalarType mix_out_dtype(const Tensor& q, const std::optional<at::ScalarType>& out) {
+  FMTA_REQUIRE(!out || *out == at::kFloat || *out == at::kBFloat16, "out_dtype must be float32 or bfloat16");   // what the kernels write
   if (out) return *out;
   return q.scalar_type() == at::kFloat || q.scalar_type() == at::kBFloat16 ? q.scalar_type() : at::kFloat;
 }

@@ -142,3 +142,11 @@ def test_32_heads_limits_are_rejected_loudly():
         F.conv_headmix_forward(q, q, q, torch.eye(32, device="cuda"), th, 1.0, True)
     o, l, m = F.head_conv_attention_forward(q, q, q, torch.eye(32, device="cuda"))
     assert torch.isfinite(o.float()).all()
+
+
+def test_output_types_the_kernels_do_not_write_are_refused():
+    import fmta_b200 as F
+    q = torch.zeros(1, 4, 16, 64, device="cuda", dtype=torch.bfloat16)
+    for dt in (torch.float16, torch.float64, torch.int32):
+        with pytest.raises(RuntimeError):
+            F.conv_headmix_forward(q, q, q, torch.eye(4, device="cuda"), out_dtype=dt)
