@@ -54,9 +54,13 @@ def _pad64(t):
 # (c_q times the size of K for as long as the graph lives; about 2 % of a step at B=4, H=16, N=4096, d=64):
 # `ktilde_buffer` + the ``ktilde`` argument of `forward` / `backward`, or FMTA_KEEP_KTILDE=1 for the autograd Function.
 # The Function keeps it by itself up to KEEP_KTILDE_BYTES: there the pre-pass is 2 to 5 % of the step (19 MB: 172 -> 164 us),
-# and a layer holds no more than that much longer.
-KEEP_KTILDE = os.environ.get("FMTA_KEEP_KTILDE", "0") != "0"
+# and a layer holds no more than that much longer.  FMTA_KEEP_KTILDE=0 (KEEP_KTILDE False): never.
+KEEP_KTILDE = {"": None, "0": False}.get(os.environ.get("FMTA_KEEP_KTILDE", ""), True)     # None: up to KEEP_KTILDE_BYTES
 KEEP_KTILDE_BYTES = 64 << 20
+
+
+def _keep_limit():
+    return KEEP_KTILDE_BYTES if KEEP_KTILDE is None else (1 << 62 if KEEP_KTILDE else 0)
 
 
 def ktilde_buffer(Q, conv_kernel):
@@ -182,7 +186,7 @@ class FlashConvAttentionCUDAFunction(torch.autograd.Function):
             return super(FlashConvAttentionCUDAFunction, FlashConvAttentionCUDAFunction).apply(Q, K, V, conv_kernel, scale, pad_q,
                                                                                                pad_k, causal)
         return _native.conv_attention(Q, K, V, conv_kernel, scale, pad_q, pad_k, bool(causal),
-                                      1 << 62 if KEEP_KTILDE else KEEP_KTILDE_BYTES, STREAM_LIMIT_BYTES, PAD_D32)
+                                      _keep_limit(), STREAM_LIMIT_BYTES, PAD_D32)
 
     @staticmethod
     def forward(ctx, Q, K, V, conv_kernel, scale, pad_q, pad_k, causal):

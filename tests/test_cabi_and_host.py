@@ -141,6 +141,16 @@ def test_module_state_dict_names():
     assert list(h.state_dict().keys()) == ["head_conv_weights"] and h.head_conv_weights.dtype == torch.float16
 
 
+@pytest.mark.parametrize("value,limit", [(None, 64 << 20), ("0", 0), ("1", 1 << 62)])
+def test_kept_stacked_keys_follow_the_environment(value, limit):
+    env = {k: v for k, v in os.environ.items() if k != "FMTA_KEEP_KTILDE"}
+    if value is not None:
+        env["FMTA_KEEP_KTILDE"] = value
+    code = "import sys; sys.path.insert(0, %r); from fmta_b200 import conv_attn; print(conv_attn._keep_limit())" % os.path.join(
+        ROOT, "flash-multi-token-attention_b200")
+    assert int(subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=120).stdout) == limit
+
+
 def test_unit_partition_covers_everything():
     from fmta_b200 import sharding as sh
     for n in (1, 7, 16, 64, 1024):

@@ -193,3 +193,14 @@ def test_other_threads_run_while_a_launch_waits(name):
     torch.cuda.synchronize()
     assert took[0] > 1.0                        # the queue did fill
     assert gap < 0.3
+
+
+@pytest.mark.parametrize("keep,kept", [(False, 0), (None, 1), (True, 1)])
+def test_stacked_keys_are_kept_as_asked(monkeypatch, keep, kept):
+    from fmta_b200 import conv_attn
+    monkeypatch.setattr(conv_attn, "KEEP_KTILDE", keep)
+    q, k, v, theta, w = _inputs(9)
+    seen = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (seen.append(t.dim()), t)[1], lambda t: t):
+        _ops()["conv"](q.requires_grad_(), k, v, theta, w)
+    assert seen.count(5) == kept                # [B, H, c_q, N, d]
