@@ -123,6 +123,19 @@ int fmta_selftest_expire_next(int kernel_id) {
 
 static size_t up1k(size_t x) { return (x + 1023) / 1024 * 1024; }
 
+// fmta_bwd_fused: FMTA_OP_BWD_TC, then D, the adjoint kernel's counters, the bf16 rounding of an fp32 dO (do_f32), and the band
+// kernel's fp32 part of dQ, dK, dV where the gradients' own buffers cannot hold it (parts: bf16 gradients, causal)
+static size_t fused_bytes(int B, int H, int N, int d, int cq, int ck, bool do_f32, bool parts) {
+  const size_t rows = (size_t)B * H * N;
+  return up1k(fmta_workspace_bytes(FMTA_OP_BWD_TC, B, H, N, d, cq, ck, 1)) + up1k(rows * 4) + up1k((size_t)H * 4) +
+         (do_f32 ? up1k(rows * d * 2) : 0) + (parts ? 3 * up1k(rows * d * 4) : 0);
+}
+
+size_t fmta_bwd_fused_workspace_bytes(int B, int H, int N, int d, int cq, int ck, int do_dtype, int grad_dtype, int causal) {
+  if (B < 1 || H < 1 || N < 1 || cq < 1 || ck < 1) return 0;
+  return fused_bytes(B, H, N, d, cq, ck, do_dtype == FMTA_DTYPE_F32, grad_dtype == FMTA_DTYPE_BF16 && causal);
+}
+
 size_t fmta_workspace_bytes(int op, int B, int H, int N, int d, int cq, int ck, int G) {
   (void)d;
   if (op == FMTA_OP_BWD_DQ) {
@@ -142,11 +155,7 @@ size_t fmta_workspace_bytes(int op, int B, int H, int N, int d, int cq, int ck, 
     return part + (op == FMTA_OP_BWD_TC_STREAM && d == 64 ? bwd_tc_stream_workspace_bytes(B, H, N, d, cq)
                                                           : bwd_tc_workspace_bytes(B, H, N, d, cq));
   }
-  if (op == FMTA_OP_BWD_FUSED) {
-    // FMTA_OP_BWD_TC, then D, the bf16 dO, the adjoint kernel's counters and the band kernel's fp32 part of dQ, dK, dV
-    const size_t rows = (size_t)B * H * N;
-    return up1k(fmta_workspace_bytes(FMTA_OP_BWD_TC, B, H, N, d, cq, ck, G)) + up1k(rows * 4) + up1k(rows * d * 2) + up1k((size_t)H * 4) + 3 * up1k(rows * d * 4);
-  }
+  if (op == FMTA_OP_BWD_FUSED) return fused_bytes(B, H, N, d, cq, ck, true, true);
   if (op == FMTA_OP_MIX_FWD || op == FMTA_OP_MIX_BWD) return mix_tc_workspace_bytes(B, H, N, d, cq, ck, G, op == FMTA_OP_MIX_BWD);
   if (op == FMTA_OP_MIX_EXCHANGE) {
     // optional scratch of the conv + mix cluster kernels: two sets (alternate tiles) of two fp32 tiles per CTA
@@ -425,18 +434,19 @@ int fmta_bwd_fused(const void* Q, const void* K, const void* V, const void* dO, 
   q.theta = theta; q.d = d; q.cq = cq; q.ck = ck;
   if (!bwd_tc_supported(q)) return FMTA_ERR_UNSUPPORTED;
   const size_t base = up1k(fmta_workspace_bytes(FMTA_OP_BWD_TC, B, H, N, d, cq, ck, 1));
-  if (!workspace || workspace_bytes < fmta_workspace_bytes(FMTA_OP_BWD_FUSED, B, H, N, d, cq, ck, 1)) return FMTA_ERR_WORKSPACE;
+  const bool g16 = grad_dtype == FMTA_DTYPE_BF16, d32 = do_dtype == FMTA_DTYPE_F32, parts = g16 && causal;
+  if (!workspace || workspace_bytes < fused_bytes(B, H, N, d, cq, ck, d32, parts)) return FMTA_ERR_WORKSPACE;
   if (!aligned16(workspace)) return FMTA_ERR_ALIGN;
   const size_t rows = (size_t)B * H * N;
   unsigned char* w = reinterpret_cast<unsigned char*>(workspace) + base;
-  float* D = reinterpret_cast<float*>(w); w += up1k(rows * 4);
-  __nv_bfloat16* dOb = reinterpret_cast<__nv_bfloat16*>(w); w += up1k(rows * d * 2);
-  unsigned* count = reinterpret_cast<unsigned*>(w); w += up1k((size_t)H * 4);
-  float* part[3];
-  for (int i = 0; i < 3; ++i) { part[i] = reinterpret_cast<float*>(w); w += up1k(rows * d * 4); }
+  auto take = [&](size_t n) { unsigned char* r = w; w += up1k(n); return r; };
+  float* D = reinterpret_cast<float*>(take(rows * 4));
+  unsigned* count = reinterpret_cast<unsigned*>(take((size_t)H * 4));
+  __nv_bfloat16* dOb = d32 ? reinterpret_cast<__nv_bfloat16*>(take(rows * d * 2)) : nullptr;
+  // without a causal mask there is no band part: nothing is read from or written to these
   void* outs[3] = {dQ, dK, dV};
-  const bool g16 = grad_dtype == FMTA_DTYPE_BF16, d32 = do_dtype == FMTA_DTYPE_F32;
-  if (!g16) for (int i = 0; i < 3; ++i) part[i] = reinterpret_cast<float*>(outs[i]);
+  float* part[3];
+  for (int i = 0; i < 3; ++i) part[i] = parts ? reinterpret_cast<float*>(take(rows * d * 4)) : reinterpret_cast<float*>(outs[i]);
   if (int s = check_cuda(launch_rowdot(dO, O, o_dtype == FMTA_DTYPE_BF16, d32 ? dOb : nullptr, D, rows, d, (cudaStream_t)stream, count, H))) return s;
   return bwd_impl(Q, K, V, d32 ? dOb : dO, D, LSE, theta, nullptr, part[0], part[1], part[2], dTheta, nullptr, B, H, N, d, cq,
                   ck, 1, scale, causal, 1, workspace, base, stream, ktilde, 0, 0, g16 ? outs : nullptr, count);

@@ -241,7 +241,7 @@ struct ConvAttnFn : public torch::autograd::Function<ConvAttnFn> {
       const bool g16 = ty[0] == at::kBFloat16 && ty[1] == at::kBFloat16 && ty[2] == at::kBFloat16;
       for (auto& t : g) t = at::empty(q.sizes(), q.options().dtype(g16 ? at::kBFloat16 : at::kFloat));
       dT = new_f32(q, {s.H, s.cq, s.ck});
-      const size_t n = fmta_workspace_bytes(FMTA_OP_BWD_FUSED, s.B, s.H, s.N, s.d, s.cq, s.ck, 1);
+      const size_t n = fmta_bwd_fused_workspace_bytes(s.B, s.H, s.N, s.d, s.cq, s.ck, dtype_code(dO.scalar_type()), g16 ? FMTA_DTYPE_BF16 : FMTA_DTYPE_F32, causal);
       const Tensor ws = new_bytes(q, n);
       check_status(fmta_bwd_fused(ptr(q), ptr(k), ptr(v), ptr(dO), dtype_code(dO.scalar_type()), ptr(O), FMTA_DTYPE_F32, fptr(LSE), fptr(theta),
                                   ptr(g[0]), ptr(g[1]), ptr(g[2]), g16 ? FMTA_DTYPE_BF16 : FMTA_DTYPE_F32, fptr(dT), s.B, s.H, s.N, s.d, s.cq,

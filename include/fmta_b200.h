@@ -208,7 +208,8 @@ int fmta_bwd_with_ktilde(const void* Q, const void* K, const void* V, const void
  * `FlashConvAttentionCUDAFunction.backward` (conv_attn/conv_attention_cuda.py:132-163) as a whole.
  *   dO, O: do_dtype / o_dtype (FMTA_DTYPE_F32 or FMTA_DTYPE_BF16)     dQ, dK, dV: grad_dtype
  *   ktilde: NULL, or the operand fmta_fwd_keep_ktilde left for these K, theta and scale
- * Tensor-core shapes only (those of fmta_bwd with path = 1); workspace: FMTA_OP_BWD_FUSED.
+ * Tensor-core shapes only (those of fmta_bwd with path = 1); workspace: FMTA_OP_BWD_FUSED, of
+ * one call fmta_bwd_fused_workspace_bytes.
  */
 int fmta_bwd_fused(const void* Q, const void* K, const void* V, const void* dO, int do_dtype, const void* O, int o_dtype,
                    const float* LSE, const float* theta, void* dQ, void* dK, void* dV, int grad_dtype, float* dTheta,
@@ -332,6 +333,9 @@ int fmta_bwd_dq_dw_static(const void* Q, const void* K, const void* V, const voi
 
 /* Bytes of caller-owned workspace an op needs for the given problem (0 if none). */
 size_t fmta_workspace_bytes(int op, int B, int H, int N, int d, int cq, int ck, int G);
+
+/* FMTA_OP_BWD_FUSED for one call whose types and mask are known: what that call takes, never more than fmta_workspace_bytes. */
+size_t fmta_bwd_fused_workspace_bytes(int B, int H, int N, int d, int cq, int ck, int do_dtype, int grad_dtype, int causal);
 
 /* FMTA_OP_MIX_FWD (bwd = 0) or FMTA_OP_MIX_BWD for one call whose filter (has_theta) and mask (causal) are known: what that call
  * lays out, never more than fmta_workspace_bytes, which has to cover all of them.  0: the tensor-core kernels do not take the

@@ -109,6 +109,20 @@ def test_mixing_workspace_covers_what_a_call_lays_out():
                                 assert lib.fmta_mix_workspace_bytes(bwd, B, H, N, d, cq, ck, G, theta, causal) <= most, (G, B, H, d, N, bwd, cq, causal)
 
 
+def test_fused_backward_takes_what_its_types_need():
+    from fmta_b200._lib import lib
+    up = lambda n: (n + 1023) // 1024 * 1024
+    for B, H, N, d, cq, ck in ((1, 4, 256, 64, 3, 5), (2, 3, 333, 128, 6, 11), (1, 1, 1, 64, 7, 7)):
+        rows = B * H * N
+        most = lib.fmta_workspace_bytes(6, B, H, N, d, cq, ck, 1)
+        need = lambda do, g, causal: lib.fmta_bwd_fused_workspace_bytes(B, H, N, d, cq, ck, do, g, causal)
+        assert need(0, 1, 1) == most                                           # fp32 dO, bf16 gradients, causal
+        assert need(1, 1, 1) == most - up(rows * d * 2)
+        for do in (0, 1):                       # fp32 gradients, or no band: the gradients' own buffers hold what there is
+            assert need(do, 0, 1) == need(do, 0, 0) == need(do, 1, 0) == need(do, 1, 1) - 3 * up(rows * d * 4)
+        assert need(1, 0, 0) > lib.fmta_workspace_bytes(3, B, H, N, d, cq, ck, 1)
+
+
 def test_mixing_grids_stay_in_range():
     """grid.y counts heads: a launch takes 65535 of them at most, and what has no loop over launches is left to other kernels."""
     from fmta_b200._lib import lib

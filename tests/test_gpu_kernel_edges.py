@@ -193,3 +193,30 @@ def test_mixing_more_heads_than_a_grid_dimension(G, N, conv):
         ref = (orc.conv_headmix_fwd(Q, K, V, th, wf, scale, True)[0],) + orc.conv_headmix_bwd_autograd(Q, K, V, th, wf, dO, scale, True)[:3]
         for got, want in zip((o, dq, dk, dv), ref):
             assert maxabs(got[b:b + 1], want) <= 3e-2
+
+
+@pytest.mark.parametrize("do_bf16", [0, 1])
+@pytest.mark.parametrize("grad_bf16", [0, 1])
+@pytest.mark.parametrize("causal", [0, 1])
+@pytest.mark.parametrize("d", [64, 128])
+def test_fused_backward_stays_in_its_workspace(do_bf16, grad_bf16, causal, d):
+    """Exactly the bytes that the library names for the call, what lies behind them untouched, against the separate calls."""
+    import fmta_b200 as F
+    from fmta_b200._lib import lib, ptr, stream_ptr
+    B, H, N, cq, ck, scale = 2, 3, 301, 5, 9, 0.125
+    g = torch.Generator(device="cuda").manual_seed(d)
+    q, k, v, do = (torch.randn(B, H, N, d, device="cuda", generator=g).to(torch.bfloat16) for _ in range(4))
+    theta = 0.1 * torch.randn(H, cq, ck, device="cuda", generator=g)
+    O, M, L, LSE = F.forward(q, k, v, theta, scale, cq - 1, (ck - 1) // 2, bool(causal), return_lse=True)
+    want = F.backward(q, k, v, do, F.rowdot(do, O), LSE, theta, scale, cq - 1, (ck - 1) // 2, bool(causal))
+    dt = torch.bfloat16 if grad_bf16 else torch.float32
+    grads = [torch.empty(B, H, N, d, dtype=dt, device="cuda") for _ in range(3)]
+    dth = torch.empty(H, cq, ck, device="cuda")
+    n = lib.fmta_bwd_fused_workspace_bytes(B, H, N, d, cq, ck, do_bf16, grad_bf16, causal)
+    ws = torch.full((n + (4 << 20),), 0x5A, dtype=torch.uint8, device="cuda")
+    dO = do if do_bf16 else do.float()
+    st = lib.fmta_bwd_fused(ptr(q), ptr(k), ptr(v), ptr(dO), do_bf16, ptr(O), 0, ptr(LSE), ptr(theta), *(ptr(t) for t in grads), grad_bf16,
+                            ptr(dth), B, H, N, d, cq, ck, scale, causal, ptr(ws), n, None, stream_ptr())
+    assert st == 0 and bool((ws[n:] == 0x5A).all())
+    for got, ref in zip(grads + [dth], want):
+        assert torch.equal(got, ref.to(got.dtype))
