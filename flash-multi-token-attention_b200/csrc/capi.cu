@@ -170,10 +170,10 @@ size_t fmta_workspace_bytes(int op, int B, int H, int N, int d, int cq, int ck, 
   return 0;
 }
 
-size_t fmta_mix_workspace_bytes(int bwd, int B, int H, int N, int d, int cq, int ck, int G, int has_theta, int causal) {
+size_t fmta_mix_workspace_bytes(int bwd, int B, int H, int N, int d, int cq, int ck, int G, int has_theta, int causal, size_t limit) {
   if (B < 1 || H < 1 || N < 1 || G < 2 || G > 16 || H % G != 0 || (has_theta && (cq < 1 || ck < 1))) return 0;
   if (!mix_tc_shape(B, H, N, d, cq, G, has_theta != 0)) return 0;
-  return mix_tc_call_bytes(B, H, N, d, cq, ck, G, has_theta != 0, causal != 0, bwd != 0);
+  return mix_tc_call_bytes(B, H, N, d, cq, ck, G, has_theta != 0, causal != 0, bwd != 0, limit);
 }
 
 // A window [lo, hi) of sequence positions: starts on a multiple of 256 (the rows of one CTA of the forward
@@ -206,7 +206,7 @@ static int fwd_impl(const void* Q, const void* K, const void* V, const float* th
   if (wmix && G == 1) return FMTA_ERR_UNSUPPORTED;
   if (path != 0 && path != 1 && path != -1) return FMTA_ERR_SHAPE;
   if (path != 0 && g_path != 0 && row_hi == 0 && mix_tc_supported(p) && workspace && aligned16(workspace) &&
-      workspace_bytes >= mix_tc_call_bytes(B, H, N, d, p.cq, p.ck, p.G, theta != nullptr, causal, false))
+      mix_tc_call_bytes(B, H, N, d, p.cq, p.ck, p.G, theta != nullptr, causal, false, workspace_bytes) != 0)
     return check_cuda(launch_mix_fwd(p, workspace, workspace_bytes, (cudaStream_t)stream));
   bool use_tc = (path != 0) && fwd_tc_supported(p);
   if (path == 1 && !use_tc) return FMTA_ERR_UNSUPPORTED;
@@ -467,7 +467,7 @@ int fmta_mix_bwd(const void* Q, const void* K, const void* V, const void* dO, in
   for (const void* x : {O, (const void*)dQ, (const void*)dK, (const void*)dV, (const void*)workspace})
     if (!aligned16(x)) return FMTA_ERR_ALIGN;
   if (!mix_tc_supported(p)) return FMTA_ERR_UNSUPPORTED;
-  if (!workspace || workspace_bytes < mix_tc_call_bytes(B, H, N, d, p.cq, p.ck, G, theta != nullptr, causal, true)) return FMTA_ERR_WORKSPACE;
+  if (!workspace || mix_tc_call_bytes(B, H, N, d, p.cq, p.ck, G, theta != nullptr, causal, true, workspace_bytes) == 0) return FMTA_ERR_WORKSPACE;
   p.dQo = dQ; p.dKo = dK; p.dVo = dV; p.grad_bf16 = grad_dtype == FMTA_DTYPE_BF16;
   return check_cuda(launch_mix_bwd(p, dO, do_dtype == FMTA_DTYPE_F32, O, o_dtype == FMTA_DTYPE_BF16, dTheta, dW, want, workspace,
                                    workspace_bytes, (cudaStream_t)stream));

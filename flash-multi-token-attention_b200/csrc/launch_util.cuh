@@ -123,7 +123,7 @@ cudaError_t launch_dk_post(const TrainParams& p, __nv_bfloat16* dKt, bool with_l
 bool mix_tc_shape(int B, int H, int N, int d, int cq, int G, bool conv);
 bool mix_tc_supported(const TrainParams& p);
 size_t mix_tc_workspace_bytes(int B, int H, int N, int d, int cq, int ck, int G, bool bwd);
-size_t mix_tc_call_bytes(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool causal, bool bwd);
+size_t mix_tc_call_bytes(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool causal, bool bwd, size_t limit);
 cudaError_t launch_mix_fwd(const TrainParams& p, void* workspace, size_t workspace_bytes, cudaStream_t stream);
 cudaError_t launch_mix_bwd(const TrainParams& p, const void* dO, bool do_f32, const void* O, bool o_bf16, float* dTheta, float* dW, int want,
                            void* workspace, size_t workspace_bytes, cudaStream_t stream);

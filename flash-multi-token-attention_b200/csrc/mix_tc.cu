@@ -24,7 +24,8 @@ struct MixPlan {
   int theta_band_slots, theta_post_slots, dw_slots;
 };
 
-MixPlan plan(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool causal, bool bwd) {
+// max_units: (batch, group) units per launch, at most
+MixPlan plan_units(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool causal, bool bwd, size_t max_units) {
   MixPlan m = {};
   m.d = d; m.conv = conv; m.causal = causal; m.bwd = bwd;
   m.nRT = (N + 127) / 128; m.N8 = m.nRT * 128; m.RP = m.N8 + 16;
@@ -32,7 +33,7 @@ MixPlan plan(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool 
   m.unit = (size_t)G * (m.N8 / 8) * m.RP * 16;
   const size_t per = m.unit * (bwd ? 2 : 1);
   // grid.y of the launches counts a launch's units or heads: 65535 at most (short sequences of many)
-  const size_t fit = kMixChunkBytes / per, most = (size_t)(65535 / G);
+  const size_t fit = kMixChunkBytes / per, most = max_units < (size_t)(65535 / G) ? max_units : (size_t)(65535 / G);
   m.nU = (int)(fit < 1 ? 1 : fit > most ? most : fit);
   if (m.nU > m.U) m.nU = m.U;
   // keys per CTA: long chunks keep the row tile's operands and amortise the fixed cost of a CTA; about three CTAs per SM
@@ -101,6 +102,18 @@ size_t carve(const MixPlan& m, void* base, MixBuffers& b) {
 
 size_t bytes_of(const MixPlan& m) { MixBuffers b; return carve(m, nullptr, b); }
 
+// The plan of a call whose workspace is `limit` bytes: as many units per launch as fit (nU = 0: not even one).
+MixPlan plan(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool causal, bool bwd, size_t limit) {
+  MixPlan m = plan_units(B, H, N, d, cq, ck, G, conv, causal, bwd, ~(size_t)0);
+  while (bytes_of(m) > limit) {
+    // (the statistics of a smaller launch may take more per unit: one by one from what P and dC alone allow)
+    const size_t fit = limit / (m.unit * (bwd ? 2 : 1)), most = fit < (size_t)m.nU - 1 ? fit : m.nU - 1;
+    if (most == 0) { m.nU = 0; break; }
+    m = plan_units(B, H, N, d, cq, ck, G, conv, causal, bwd, most);
+  }
+  return m;
+}
+
 }  // namespace
 
 bool mix_tc_shape(int B, int H, int N, int d, int cq, int G, bool conv) {
@@ -115,9 +128,10 @@ bool mix_tc_supported(const TrainParams& p) {
   return p.Wmix && mix_tc_shape(p.B, p.H, p.N, p.d, p.cq, p.G, p.theta != nullptr) && tensor_maps_available();
 }
 
-// What one call takes.
-size_t mix_tc_call_bytes(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool causal, bool bwd) {
-  return bytes_of(plan(B, H, N, d, conv ? cq : 1, conv ? ck : 1, G, conv, causal, bwd));
+// What one call takes, no more than `limit` (0: it cannot do with that).
+size_t mix_tc_call_bytes(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool causal, bool bwd, size_t limit) {
+  const MixPlan m = plan(B, H, N, d, conv ? cq : 1, conv ? ck : 1, G, conv, causal, bwd, limit);
+  return m.nU ? bytes_of(m) : 0;
 }
 
 // Neither the causal flag nor, for a 1 x 1 filter, the presence of a filter is an argument of fmta_workspace_bytes: the most
@@ -127,7 +141,7 @@ size_t mix_tc_workspace_bytes(int B, int H, int N, int d, int cq, int ck, int G,
   size_t most = 0;
   for (int causal = 0; causal < 2; ++causal)
     for (int conv = cq * ck > 1; conv < 2; ++conv) {
-      const size_t n = bytes_of(plan(B, H, N, d, cq, ck, G, conv, causal, bwd));
+      const size_t n = bytes_of(plan(B, H, N, d, cq, ck, G, conv, causal, bwd, ~(size_t)0));
       if (n > most) most = n;
     }
   return most;
@@ -146,9 +160,9 @@ static void fill(MixParams& q, const TrainParams& p, const MixPlan& m, int* stat
 
 cudaError_t launch_mix_fwd(const TrainParams& p_, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   TrainParams p = p_;
-  const MixPlan m = plan(p.B, p.H, p.N, p.d, p.cq, p.ck, p.G, p.theta != nullptr, p.causal, false);
+  const MixPlan m = plan(p.B, p.H, p.N, p.d, p.cq, p.ck, p.G, p.theta != nullptr, p.causal, false, workspace_bytes);
   MixBuffers b;
-  if (carve(m, workspace, b) > workspace_bytes) return cudaErrorInvalidValue;
+  if (m.nU == 0 || carve(m, workspace, b) > workspace_bytes) return cudaErrorInvalidValue;
   int* status = nullptr;
   FMTA_TRY(status_word_of(b.status, stream, &status));
   MixParams q;
@@ -172,9 +186,9 @@ cudaError_t launch_mix_bwd(const TrainParams& p_, const void* dO, bool do_f32, c
                            void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   TrainParams p = p_;
   const bool conv = p.theta != nullptr;
-  const MixPlan m = plan(p.B, p.H, p.N, p.d, p.cq, p.ck, p.G, conv, p.causal, true);
+  const MixPlan m = plan(p.B, p.H, p.N, p.d, p.cq, p.ck, p.G, conv, p.causal, true, workspace_bytes);
   MixBuffers b;
-  if (carve(m, workspace, b) > workspace_bytes) return cudaErrorInvalidValue;
+  if (m.nU == 0 || carve(m, workspace, b) > workspace_bytes) return cudaErrorInvalidValue;
   int* status = nullptr;
   FMTA_TRY(status_word_of(b.status, stream, &status));
   if (conv && p.causal) { p.Cband = b.Cband; p.dCband = b.dCband; p.dQ = b.dQ; p.dK = b.dK; }

@@ -74,6 +74,7 @@ bool on16(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 
 // one-call backwards read it in 16-byte pieces
 Tensor aligned(const Tensor& t) { return on16(t) ? t : t.clone(); }
 Tensor new_f32(const Tensor& like, at::IntArrayRef shape) { return at::empty(shape, like.options().dtype(at::kFloat)); }
+size_t bytes_of(const Tensor& t) { return t.defined() ? (size_t)t.numel() : 0; }      // of a byte tensor
 Tensor new_bytes(const Tensor& like, size_t n) { return at::empty({(int64_t)(n < 16 ? 16 : n)}, like.options().dtype(at::kByte)); }
 int dtype_code(at::ScalarType t) { return t == at::kBFloat16 ? FMTA_DTYPE_BF16 : FMTA_DTYPE_F32; }
 bool exact_only() { return fmta_set_path(99) == 0; }
@@ -283,22 +284,42 @@ Tensor conv_attention(const Tensor& Q, const Tensor& K, const Tensor& V, const T
   throw pybind11::error_already_set();
 }
 
+using MixLimits = std::pair<int64_t, int64_t>;   // bytes, at most: of the exchange scratch, of the tensor-core kernels' workspace
+
 struct Mix {
   Dims s;
   int G;
   Tensor w, theta;        // fp32 [H/G, G, G]; fp32 [H, cq, ck] or undefined
-  bool tc(bool bwd, bool causal, size_t* bytes) const {                 // the tensor-core kernels take this problem
-    if (exact_only()) return false;
+  // Bytes of the tensor-core kernels' workspace, `limit` at most; 0: the other kernels take this call
+  size_t tc_bytes(bool bwd, bool causal, int64_t limit) const {
+    if (exact_only()) return 0;
     // a short sequence without a filter: the 16-row CTAs of the other kernels finish sooner than one 128-row CTA of these (16
     // heads, d = 64, forward + backward on an idle GPU: 12 us per 16 keys there; 190 us at N = 640, 208 at N = 1024 here)
-    if (!theta.defined() && G >= 8 && s.N <= 224 && (long)s.B * (s.H / G) * ((s.N + 15) / 16) <= 2 * 148) return false;
-    *bytes = fmta_mix_workspace_bytes(bwd, s.B, s.H, s.N, s.d, s.cq, s.ck, G, theta.defined(), causal);
-    return *bytes != 0;
+    if (!theta.defined() && G >= 8 && s.N <= 224 && (long)s.B * (s.H / G) * ((s.N + 15) / 16) <= 2 * 148) return 0;
+    return fmta_mix_workspace_bytes(bwd, s.B, s.H, s.N, s.d, s.cq, s.ck, G, theta.defined(), causal, (size_t)limit);
   }
-  size_t exchange(int64_t limit) const {
-    if (!theta.defined()) return 0;
-    const size_t n = fmta_workspace_bytes(FMTA_OP_MIX_EXCHANGE, s.B, s.H, s.N, s.d, s.cq, s.ck, G);
-    return n <= (size_t)limit ? n : 0;
+  // That workspace, or a smaller one (fewer units at a time) where the GPU has no room for it; undefined: for none.  Call it
+  // when the outputs are there.
+  Tensor tc_workspace(const Tensor& like, bool bwd, bool causal, size_t n) const {
+    for (; n; n = tc_bytes(bwd, causal, (int64_t)(n / 2))) {
+      try {
+        return new_bytes(like, n);
+      } catch (const c10::OutOfMemoryError&) {
+      }
+    }
+    return {};
+  }
+  // The optional exchange scratch of a mix behind a filter, behind `base` bytes (rounded up to 256): up to the caller's limit
+  // and where the GPU has the room.
+  Tensor exchange_workspace(const Tensor& like, size_t base, int64_t limit) const {
+    const size_t x = theta.defined() ? fmta_workspace_bytes(FMTA_OP_MIX_EXCHANGE, s.B, s.H, s.N, s.d, s.cq, s.ck, G) : 0;
+    if (x && x <= (size_t)limit) {
+      try {
+        return new_bytes(like, (base + 255) / 256 * 256 + x);
+      } catch (const c10::OutOfMemoryError&) {
+      }
+    }
+    return base ? new_bytes(like, base) : Tensor();
   }
 };
 
@@ -328,52 +349,49 @@ Mix mix_of(const Tensor& q, const Tensor& w, const Tensor& theta_) {
 
 // O (preallocated, fp32 or bf16), L, M, LSE
 void mix_forward_raw(const Mix& m, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& O, const Tensor& M, const Tensor& L,
-                     const Tensor& LSE, double scale, bool causal, int64_t xlimit) {
+                     const Tensor& LSE, double scale, bool causal, const MixLimits& limits) {
   const Dims& s = m.s;
   arm_status(q);
-  size_t n = 0;
-  const bool tc = m.tc(false, causal, &n);
-  if (!tc) n = m.exchange(xlimit);
-  const Tensor ws = n ? new_bytes(q, n) : Tensor();
+  Tensor ws = m.tc_workspace(q, false, causal, m.tc_bytes(false, causal, limits.second));
+  const bool tc = ws.defined();
+  if (!tc) ws = m.exchange_workspace(q, 0, limits.first);
   check_status(fmta_fwd(ptr(q), ptr(k), ptr(v), fptr(m.theta), fptr(m.w), ptr(O), fptr(M), fptr(L), fptr(LSE), s.B, s.H, s.N, s.d, s.cq, s.ck, m.G,
-                        (float)scale, causal, dtype_code(O.scalar_type()), tc ? -1 : 0, ptr(ws), n, stream_of(q)),
+                        (float)scale, causal, dtype_code(O.scalar_type()), tc ? -1 : 0, ptr(ws), bytes_of(ws), stream_of(q)),
                "fmta_fwd(head mix)");
 }
 
 // {dQ, dK, dV, dW [H/G,G,G], dTheta}: gradients in grad_dtype on the tensor-core kernels, else fp32; want: 1 dQ (dW, dTheta), 2 dK and dV
 std::vector<Tensor> mix_backward_raw(const Mix& m, const Tensor& q, const Tensor& k, const Tensor& v, Tensor dO, const Tensor& O, const Tensor& LSE,
-                                     double scale, bool causal, int want, bool g16, int64_t xlimit) {
+                                     double scale, bool causal, int want, bool g16, const MixLimits& limits) {
   const Dims& s = m.s;
   arm_status(q);
   const bool conv = m.theta.defined();
   const Tensor dW = want & 1 ? new_f32(q, {s.H / m.G, m.G, m.G}) : Tensor(), dT = conv ? new_f32(q, {s.H, s.cq, s.ck}) : Tensor();
-  size_t n = 0;
-  if (m.tc(true, causal, &n)) {
+  if (const size_t n = m.tc_bytes(true, causal, limits.second)) {
     dO = dO.scalar_type() == at::kFloat && dO.is_contiguous() && on16(dO) ? dO : bf16c(dO);
     Tensor g[3];
     for (int i = 0; i < 3; ++i)
       if (conv || (i == 0 ? want & 1 : want & 2)) g[i] = at::empty(q.sizes(), q.options().dtype(g16 ? at::kBFloat16 : at::kFloat));
     const Tensor dWt = dW.defined() ? dW : (conv ? new_f32(q, {s.H / m.G, m.G, m.G}) : Tensor());
-    const Tensor ws = new_bytes(q, n);
-    check_status(fmta_mix_bwd(ptr(q), ptr(k), ptr(v), ptr(dO), dtype_code(dO.scalar_type()), ptr(O), dtype_code(O.scalar_type()), fptr(LSE), fptr(m.theta),
-                              fptr(m.w), ptr(g[0]), ptr(g[1]), ptr(g[2]), g16 ? FMTA_DTYPE_BF16 : FMTA_DTYPE_F32, fptr(dT), fptr(dWt), s.B, s.H, s.N, s.d,
-                              s.cq, s.ck, m.G, (float)scale, causal, ptr(ws), n, stream_of(q)),
-                 "fmta_mix_bwd");
-    return {g[0], g[1], g[2], dW, dT};
+    if (const Tensor ws = m.tc_workspace(q, true, causal, n); ws.defined()) {
+      check_status(fmta_mix_bwd(ptr(q), ptr(k), ptr(v), ptr(dO), dtype_code(dO.scalar_type()), ptr(O), dtype_code(O.scalar_type()), fptr(LSE), fptr(m.theta),
+                                fptr(m.w), ptr(g[0]), ptr(g[1]), ptr(g[2]), g16 ? FMTA_DTYPE_BF16 : FMTA_DTYPE_F32, fptr(dT), fptr(dWt), s.B, s.H, s.N, s.d,
+                                s.cq, s.ck, m.G, (float)scale, causal, ptr(ws), bytes_of(ws), stream_of(q)),
+                   "fmta_mix_bwd");
+      return {g[0], g[1], g[2], dW, dT};
+    }
   }
   dO = bf16c(dO);
   const Tensor D = rowdot(dO, O);
-  n = fmta_workspace_bytes(FMTA_OP_BWD_DQ, s.B, s.H, s.N, s.d, s.cq, s.ck, m.G);
-  if (const size_t x = m.exchange(xlimit)) n = (n + 255) / 256 * 256 + x;
-  const Tensor ws = new_bytes(q, n);
   const Tensor dQ = want & 1 ? new_f32(q, q.sizes()) : Tensor(), dK = want & 2 ? new_f32(q, q.sizes()) : Tensor(), dV = want & 2 ? new_f32(q, q.sizes()) : Tensor();
+  const Tensor ws = m.exchange_workspace(q, std::max<size_t>(fmta_workspace_bytes(FMTA_OP_BWD_DQ, s.B, s.H, s.N, s.d, s.cq, s.ck, m.G), 16), limits.first);
   if (want == 3)
     check_status(fmta_bwd(ptr(q), ptr(k), ptr(v), ptr(dO), fptr(D), fptr(LSE), fptr(m.theta), fptr(m.w), fptr(dQ), fptr(dK), fptr(dV), fptr(dT), fptr(dW),
-                          s.B, s.H, s.N, s.d, s.cq, s.ck, m.G, (float)scale, causal, 0, ptr(ws), n, stream_of(q)),
+                          s.B, s.H, s.N, s.d, s.cq, s.ck, m.G, (float)scale, causal, 0, ptr(ws), bytes_of(ws), stream_of(q)),
                  "fmta_bwd(head mix)");
   else if (want == 1)
     check_status(fmta_bwd_dq_dw(ptr(q), ptr(k), ptr(v), ptr(dO), fptr(D), fptr(LSE), fptr(m.theta), fptr(m.w), fptr(dQ), fptr(dT), fptr(dW), s.B, s.H, s.N,
-                                s.d, s.cq, s.ck, m.G, (float)scale, causal, ptr(ws), n, stream_of(q)),
+                                s.d, s.cq, s.ck, m.G, (float)scale, causal, ptr(ws), bytes_of(ws), stream_of(q)),
                  "fmta_bwd_dq_dw(head mix)");
   else
     check_status(fmta_bwd_dkdv(ptr(q), ptr(k), ptr(v), ptr(dO), fptr(D), fptr(LSE), fptr(m.theta), fptr(m.w), fptr(dK), fptr(dV), s.B, s.H, s.N, s.d, s.cq,
@@ -395,7 +413,7 @@ void mix_check(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& 
 }
 
 std::tuple<Tensor, Tensor, Tensor, Tensor> mix_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& w, const std::optional<Tensor>& theta_,
-                                                      double scale, bool causal, const std::optional<at::ScalarType>& out, int64_t xlimit) {
+                                                      double scale, bool causal, const std::optional<at::ScalarType>& out, const MixLimits& limits) {
   const Tensor theta = theta_ ? *theta_ : Tensor();
   mix_check(q, k, v, w, theta);
   at::AutoGradMode no_grad(false);
@@ -403,13 +421,13 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> mix_forward(const Tensor& q, const Te
   const Mix m = mix_of(q, w, theta);
   const Tensor O = at::empty(q.sizes(), q.options().dtype(mix_out_dtype(q, out)));
   const Tensor M = new_f32(q, {m.s.B, m.s.H, m.s.N}), L = at::empty_like(M), LSE = at::empty_like(M);
-  mix_forward_raw(m, bf16c(q), bf16c(k), bf16c(v), O, M, L, LSE, scale, causal, xlimit);
+  mix_forward_raw(m, bf16c(q), bf16c(k), bf16c(v), O, M, L, LSE, scale, causal, limits);
   return {out ? O : O.to(q.scalar_type()), L, M, LSE};
 }
 
 std::vector<Tensor> mix_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& o, const Tensor& dO, const Tensor& l,
                                  const Tensor& mx, const std::optional<Tensor>& theta_, bool causal, const std::optional<double>& scale,
-                                 const std::optional<Tensor>& lse_, int64_t want, int64_t xlimit) {
+                                 const std::optional<Tensor>& lse_, int64_t want, const MixLimits& limits) {
   const Tensor theta = theta_ ? *theta_ : Tensor();
   mix_check(q, k, v, w, theta);
   require_on(q, dO, "do", q.sizes()); require_on(q, o, "o", q.sizes());
@@ -419,7 +437,7 @@ std::vector<Tensor> mix_backward(const Tensor& q, const Tensor& k, const Tensor&
   require_on(q, l, "l", {m.s.B, m.s.H, m.s.N}); require_on(q, mx, "m", {m.s.B, m.s.H, m.s.N});
   const Tensor lse = lse_ ? f32(*lse_) : at::add(f32(mx), at::log(f32(l)));
   const Tensor oc = aligned(o.scalar_type() == at::kBFloat16 ? o.contiguous() : f32(o));
-  auto g = mix_backward_raw(m, bf16c(q), bf16c(k), bf16c(v), bf16c(dO), oc, lse, scale ? *scale : 1.0 / std::sqrt((double)m.s.d), causal, (int)want, false, xlimit);
+  auto g = mix_backward_raw(m, bf16c(q), bf16c(k), bf16c(v), bf16c(dO), oc, lse, scale ? *scale : 1.0 / std::sqrt((double)m.s.d), causal, (int)want, false, limits);
   if (g[3].defined()) g[3] = g[3].reshape(w.sizes());
   return g;
 }
@@ -427,16 +445,16 @@ std::vector<Tensor> mix_backward(const Tensor& q, const Tensor& k, const Tensor&
 struct MixFn : public torch::autograd::Function<MixFn> {
   // no theta: mix only.  out32: fp32 output whatever q's dtype (the filter + mix operator)
   static Tensor forward(AutogradContext* ctx, const Tensor& Q, const Tensor& K, const Tensor& V, const std::optional<Tensor>& theta_o, const Tensor& w,
-                        double scale, bool causal, bool out32, int64_t xlimit) {
+                        double scale, bool causal, bool out32, const MixLimits& limits) {
     const Tensor theta_ = theta_o ? *theta_o : Tensor();
     const Mix m = mix_of(Q, w, theta_);
     const Tensor q = bf16c(Q), k = bf16c(K), v = bf16c(V);
     const Tensor O = at::empty(q.sizes(), q.options().dtype(out32 ? at::kFloat : mix_out_dtype(Q, std::nullopt)));
     const Tensor LSE = new_f32(q, {m.s.B, m.s.H, m.s.N});
-    mix_forward_raw(m, q, k, v, O, Tensor(), Tensor(), LSE, scale, causal, xlimit);
+    mix_forward_raw(m, q, k, v, O, Tensor(), Tensor(), LSE, scale, causal, limits);
     const Tensor out = out32 ? O : O.to(Q.scalar_type());
     ctx->save_for_backward({q, k, v, theta_, w, out, LSE});
-    ctx->saved_data["scale"] = scale; ctx->saved_data["causal"] = causal; ctx->saved_data["xlimit"] = xlimit;
+    ctx->saved_data["scale"] = scale; ctx->saved_data["causal"] = causal; ctx->saved_data["limit0"] = limits.first; ctx->saved_data["limit1"] = limits.second;
     ctx->saved_data["tq"] = (int64_t)Q.scalar_type(); ctx->saved_data["tk"] = (int64_t)K.scalar_type(); ctx->saved_data["tv"] = (int64_t)V.scalar_type();
     ctx->saved_data["has_theta"] = theta_.defined();
     return out;
@@ -458,7 +476,7 @@ struct MixFn : public torch::autograd::Function<MixFn> {
     if (!has_theta) want = (ctx->needs_input_grad(base) || ctx->needs_input_grad(iw) ? 1 : 0) | (ctx->needs_input_grad(1) || ctx->needs_input_grad(2) ? 2 : 0);
     if (want == 0) return variable_list(9);
     auto g = mix_backward_raw(mix_of(q, w, theta), q, k, v, dO, O, LSE, ctx->saved_data["scale"].toDouble(), ctx->saved_data["causal"].toBool(), want, g16,
-                              ctx->saved_data["xlimit"].toInt());
+                              {ctx->saved_data["limit0"].toInt(), ctx->saved_data["limit1"].toInt()});
     for (int i = 0; i < 3; ++i) if (g[i].defined()) g[i] = g[i].to(ty[i]);
     const Tensor dT = has_theta ? g[4].to(theta.scalar_type()) : Tensor();
     const Tensor dW = g[3].defined() ? g[3].reshape(w.sizes()).to(w.scalar_type()) : Tensor();
@@ -467,17 +485,17 @@ struct MixFn : public torch::autograd::Function<MixFn> {
 };
 
 Tensor mix_attention(const Tensor& q, const Tensor& k, const Tensor& v, const std::optional<Tensor>& theta_, const Tensor& w, double scale, bool causal,
-                     bool out32, int64_t xlimit) {
+                     bool out32, const MixLimits& limits) {
   const Tensor theta = theta_ ? *theta_ : Tensor();
   mix_check(q, k, v, w, theta);
   c10::cuda::CUDAGuard guard(q.device());
   if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad() || w.requires_grad() || (theta.defined() && theta.requires_grad())))
-    return MixFn::apply(q, k, v, theta_, w, scale, causal, out32, xlimit);
+    return MixFn::apply(q, k, v, theta_, w, scale, causal, out32, limits);
   refuse_tangents({&q, &k, &v, &theta, &w});
   at::AutoGradMode no_grad(false);
   const Mix m = mix_of(q, w, theta);
   const Tensor O = at::empty(q.sizes(), q.options().dtype(out32 ? at::kFloat : mix_out_dtype(q, std::nullopt)));
-  mix_forward_raw(m, bf16c(q), bf16c(k), bf16c(v), O, Tensor(), Tensor(), Tensor(), scale, causal, xlimit);
+  mix_forward_raw(m, bf16c(q), bf16c(k), bf16c(v), O, Tensor(), Tensor(), Tensor(), scale, causal, limits);
   return out32 ? O : O.to(q.scalar_type());
 }
 

@@ -18,15 +18,23 @@ import torch.nn as nn
 from . import _native
 
 
-# A mix that follows a key-query conv exchanges the heads' score tiles between the CTAs of a cluster; with this
-# optional scratch (two fp32 tiles per CTA) the exchange goes through global memory, which is faster.  Above the
-# limit the calls run without it.
-MIX_EXCHANGE_LIMIT_BYTES = int(float(os.environ.get("FMTA_MIX_EXCHANGE_LIMIT_GB", "4")) * (1 << 30))
+# What a head mix may take for itself.  On the tensor cores that is the scores' operands P and dC (4.5 GiB of them, or one
+# group's, at a time) and, with a filter, the stacked keys; the kernels for the rest exchange the heads' score tiles through a
+# global scratch (up to 4 GiB) instead of the cluster's shared memory.  FMTA_MIX_EXCHANGE_LIMIT_GB (here: this switch, in bytes)
+# bounds either: fewer groups at a time, then the kernels without such buffers.  So does what the GPU has left.
+_LIMIT_GB = os.environ.get("FMTA_MIX_EXCHANGE_LIMIT_GB")
+MIX_EXCHANGE_LIMIT_BYTES = None if _LIMIT_GB is None else int(float(_LIMIT_GB) * (1 << 30))
+
+
+def _limits():
+    if MIX_EXCHANGE_LIMIT_BYTES is None:
+        return 4 << 30, (1 << 63) - 1
+    return MIX_EXCHANGE_LIMIT_BYTES, MIX_EXCHANGE_LIMIT_BYTES
 
 
 def conv_headmix_forward(q, k, v, w, conv_kernel=None, scale=1.0, causal=False, out_dtype=None):
     """(o, l, m, lse): o in ``out_dtype`` (default: dtype of q), l = sum exp, m = max, fp32 [B,H,N]."""
-    return _native.mix_forward(q, k, v, w, conv_kernel, scale, bool(causal), out_dtype, MIX_EXCHANGE_LIMIT_BYTES)
+    return _native.mix_forward(q, k, v, w, conv_kernel, scale, bool(causal), out_dtype, _limits())
 
 
 def head_conv_attention_forward(q, k, v, w, scale=1.0, causal=False):
@@ -36,7 +44,7 @@ def head_conv_attention_forward(q, k, v, w, scale=1.0, causal=False):
 
 
 def _backward(q, k, v, w, o, do, l, m, conv_kernel, causal, scale, lse, want):
-    return _native.mix_backward(q, k, v, w, o, do, l, m, conv_kernel, bool(causal), scale, lse, want, MIX_EXCHANGE_LIMIT_BYTES)
+    return _native.mix_backward(q, k, v, w, o, do, l, m, conv_kernel, bool(causal), scale, lse, want, _limits())
 
 
 def conv_headmix_bwd_dq_dw(q, k, v, w, o, do, l, m, conv_kernel=None, causal=False, scale=None):
@@ -80,7 +88,7 @@ class HeadConvAttentionFunction(torch.autograd.Function):
             scale = 1.0 / math.sqrt(q.shape[-1])
         if torch.jit.is_tracing():
             return super(HeadConvAttentionFunction, HeadConvAttentionFunction).apply(q, k, v, w, causal, scale)
-        return _native.mix_attention(q, k, v, None, w, scale, bool(causal), False, MIX_EXCHANGE_LIMIT_BYTES)
+        return _native.mix_attention(q, k, v, None, w, scale, bool(causal), False, _limits())
 
     @staticmethod
     def forward(ctx, q, k, v, w, causal, scale):
@@ -121,7 +129,7 @@ class ConvHeadMixFunction(torch.autograd.Function):
     def apply(q, k, v, conv_kernel, w, causal, scale):
         if torch.jit.is_tracing():
             return super(ConvHeadMixFunction, ConvHeadMixFunction).apply(q, k, v, conv_kernel, w, causal, scale)
-        return _native.mix_attention(q, k, v, conv_kernel, w, scale, bool(causal), True, MIX_EXCHANGE_LIMIT_BYTES)
+        return _native.mix_attention(q, k, v, conv_kernel, w, scale, bool(causal), True, _limits())
 
     @staticmethod
     def forward(ctx, q, k, v, conv_kernel, w, causal, scale):

@@ -63,7 +63,7 @@ extern "C" {
 #define FMTA_OP_BWD_FUSED 6      /* fmta_bwd_fused */
 /* Head mixing on the tensor cores (d = 64 or 128, groups of 2, 4, 8 or 16 heads, c_q <= 7): fmta_fwd with path -1 or 1 and a
  * workspace of FMTA_OP_MIX_FWD; fmta_mix_bwd with FMTA_OP_MIX_BWD.  P (and dC) of a few (batch, group) units at a time:
- * at most 4.5 GiB, or one unit's.  Of one call: fmta_mix_workspace_bytes. */
+ * at most 4.5 GiB, or one unit's.  Of one call, and with less: fmta_mix_workspace_bytes. */
 #define FMTA_OP_MIX_FWD 7
 #define FMTA_OP_MIX_BWD 8
 
@@ -338,9 +338,10 @@ size_t fmta_workspace_bytes(int op, int B, int H, int N, int d, int cq, int ck, 
 size_t fmta_bwd_fused_workspace_bytes(int B, int H, int N, int d, int cq, int ck, int do_dtype, int grad_dtype, int causal);
 
 /* FMTA_OP_MIX_FWD (bwd = 0) or FMTA_OP_MIX_BWD for one call whose filter (has_theta) and mask (causal) are known: what that call
- * lays out, never more than fmta_workspace_bytes, which has to cover all of them.  0: the tensor-core kernels do not take the
- * problem. */
-size_t fmta_mix_workspace_bytes(int bwd, int B, int H, int N, int d, int cq, int ck, int G, int has_theta, int causal);
+ * lays out, never more than fmta_workspace_bytes, which has to cover all of them, nor than `limit` ((size_t)-1: none) -- with
+ * less of it the call takes fewer (batch, group) units at a time.  0: the tensor-core kernels do not take the problem, or not
+ * with that little. */
+size_t fmta_mix_workspace_bytes(int bwd, int B, int H, int N, int d, int cq, int ck, int G, int has_theta, int causal, size_t limit);
 
 #ifdef __cplusplus
 }

@@ -13,6 +13,9 @@ import torch
 from helpers import ROOT
 
 
+ANY = 2 ** 64 - 1        # no limit
+
+
 def _declared_symbols():
     txt = open(os.path.join(ROOT, "include", "fmta_b200.h")).read()
     return sorted(set(re.findall(r"\b(fmta_[a-z_A-Z0-9]+)\s*\(", txt)))
@@ -97,7 +100,7 @@ def test_mixing_workspace_covers_what_a_call_lays_out():
     rp, n8 = 2048 + 16, 2048
     laid_out = 2048 + 16 * 2 * 32 * 3 * rp * 4 + 16 * (n8 // 8) * rp * 16
     assert lib.fmta_workspace_bytes(7, 1, 16, 2048, 64, 1, 1, 16) >= laid_out
-    assert lib.fmta_mix_workspace_bytes(0, 1, 16, 2048, 64, 1, 1, 16, 0, 1) == laid_out
+    assert lib.fmta_mix_workspace_bytes(0, 1, 16, 2048, 64, 1, 1, 16, 0, 1, ANY) == laid_out
     for G in (2, 4, 8, 16):
         for B, H in ((1, G), (2, G), (1, 4 * G), (7, 2 * G)):
             for d in (64, 128):
@@ -106,7 +109,7 @@ def test_mixing_workspace_covers_what_a_call_lays_out():
                         for cq, ck, theta in ((1, 1, 0), (1, 1, 1), (6, 11, 1), (7, 7, 1)):
                             most = lib.fmta_workspace_bytes(7 + bwd, B, H, N, d, cq, ck, G)
                             for causal in (0, 1):
-                                assert lib.fmta_mix_workspace_bytes(bwd, B, H, N, d, cq, ck, G, theta, causal) <= most, (G, B, H, d, N, bwd, cq, causal)
+                                assert lib.fmta_mix_workspace_bytes(bwd, B, H, N, d, cq, ck, G, theta, causal, ANY) <= most, (G, B, H, d, N, bwd, cq, causal)
 
 
 def test_fused_backward_takes_what_its_types_need():
@@ -123,15 +126,34 @@ def test_fused_backward_takes_what_its_types_need():
         assert need(1, 0, 0) > lib.fmta_workspace_bytes(3, B, H, N, d, cq, ck, 1)
 
 
+def test_mixing_workspace_follows_a_limit():
+    """Under a limit a call takes fewer units at a time, as many as fit, and the same call with what was named takes just that."""
+    from fmta_b200._lib import lib
+    for bwd, B, H, N, d, cq, ck, G, theta in ((0, 2, 32, 2048, 64, 1, 1, 4, 0), (1, 3, 16, 1001, 128, 6, 11, 8, 1), (1, 5, 16, 300, 64, 1, 1, 16, 0)):
+        for causal in (0, 1):
+            need = lambda limit: lib.fmta_mix_workspace_bytes(bwd, B, H, N, d, cq, ck, G, theta, causal, limit)
+            full, sizes = need(ANY), set()
+            assert need(full) == full and need(0) == 0
+            for k in range(1, 200):
+                n = need(full * k // 200)
+                assert n <= full * k // 200
+                if n:
+                    sizes.add(n)
+                    assert need(n) == n
+            assert len(sizes) > 1 and max(sizes) <= full
+            # one unit is the least
+            assert need(min(sizes) - 1) == 0 or need(min(sizes) - 1) < min(sizes)
+
+
 def test_mixing_grids_stay_in_range():
     """grid.y counts heads: a launch takes 65535 of them at most, and what has no loop over launches is left to other kernels."""
     from fmta_b200._lib import lib
-    one = lib.fmta_mix_workspace_bytes(0, 1, 16, 128, 64, 1, 1, 16, 0, 0)
+    one = lib.fmta_mix_workspace_bytes(0, 1, 16, 128, 64, 1, 1, 16, 0, 0, ANY)
     assert one > 0
     unit = 16 * 16 * (128 + 16) * 16
-    assert lib.fmta_mix_workspace_bytes(0, 8192, 16, 128, 64, 1, 1, 16, 0, 0) < 65536 // 16 * (unit + one)
-    assert lib.fmta_mix_workspace_bytes(0, 32767, 2, 16, 64, 3, 3, 2, 1, 1) > 0
-    assert lib.fmta_mix_workspace_bytes(0, 32768, 2, 16, 64, 3, 3, 2, 1, 1) == 0
+    assert lib.fmta_mix_workspace_bytes(0, 8192, 16, 128, 64, 1, 1, 16, 0, 0, ANY) < 65536 // 16 * (unit + one)
+    assert lib.fmta_mix_workspace_bytes(0, 32767, 2, 16, 64, 3, 3, 2, 1, 1, ANY) > 0
+    assert lib.fmta_mix_workspace_bytes(0, 32768, 2, 16, 64, 3, 3, 2, 1, 1, ANY) == 0
 
 
 def test_ops_refuse_cpu_tensors():

@@ -160,7 +160,7 @@ def test_mixing_stays_in_its_workspace(B, H, N, G, causal):
     g = torch.Generator(device="cuda").manual_seed(N)
     q, k, v = (torch.randn(B, H, N, d, device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
     w = torch.randn(H // G, G, G, device="cuda", generator=g) / math.sqrt(G)
-    n = lib.fmta_mix_workspace_bytes(0, B, H, N, d, 1, 1, G, 0, int(causal))
+    n = lib.fmta_mix_workspace_bytes(0, B, H, N, d, 1, 1, G, 0, int(causal), 2 ** 64 - 1)
     guard = 16 << 20
     ws = torch.full((n + guard,), 0x5A, dtype=torch.uint8, device="cuda")
     o = torch.empty(B, H, N, d, device="cuda")
@@ -220,3 +220,49 @@ def test_fused_backward_stays_in_its_workspace(do_bf16, grad_bf16, causal, d):
     assert st == 0 and bool((ws[n:] == 0x5A).all())
     for got, ref in zip(grads + [dth], want):
         assert torch.equal(got, ref.to(got.dtype))
+
+
+@pytest.mark.parametrize("B,H,G,N,cq,ck", [(4, 16, 16, 1000, 0, 0), (2, 16, 4, 1001, 3, 5), (1, 16, 16, 1500, 0, 0)])
+def test_mixing_with_little_memory(monkeypatch, B, H, G, N, cq, ck):
+    """Under the switch's limit, or with little of the GPU's memory left, a mix takes fewer groups at a time and in the end the
+    kernels without such buffers: the results stay within rounding."""
+    import fmta_b200 as F
+    from fmta_b200 import head_conv
+    from fmta_b200._lib import lib
+    d, scale = 64, 0.125
+    g = torch.Generator(device="cuda").manual_seed(N)
+    q, k, v, do = (torch.randn(B, H, N, d, device="cuda", generator=g).to(torch.bfloat16) for _ in range(4))
+    w = torch.eye(G, device="cuda").repeat(H // G, 1, 1) + 0.1 * torch.randn(H // G, G, G, device="cuda", generator=g)
+    theta = 0.3 * torch.randn(H, cq, ck, device="cuda", generator=g) if cq else None
+
+    def step():
+        o, l, m, lse = F.conv_headmix_forward(q, k, v, w, theta, scale, True, out_dtype=torch.float32)
+        return (o, lse) + tuple(t for t in F.conv_headmix_backward(q, k, v, w, o, do, l, m, theta, True, scale, lse=lse) if t is not None)
+
+    def check(got):
+        for a, b in zip(got, want):
+            assert torch.isfinite(a).all() and float((a - b).norm()) <= 1e-2 * float(b.norm())
+
+    want = step()
+    need = [lib.fmta_mix_workspace_bytes(b, B, H, N, d, max(cq, 1), max(ck, 1), G, int(cq > 0), 1, 2 ** 64 - 1) for b in (0, 1)]
+    for limit in (max(need), need[1] // 2, need[1] // 4, need[0] // 3, 0):
+        monkeypatch.setattr(head_conv, "MIX_EXCHANGE_LIMIT_BYTES", limit)
+        torch.cuda.empty_cache()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        got = step()
+        results = sum(t.numel() * t.element_size() for t in got) + 6 * q.numel() * 4
+        assert torch.cuda.max_memory_allocated() - before <= limit + results + (8 << 20)
+        check(got)
+        del got
+    monkeypatch.setattr(head_conv, "MIX_EXCHANGE_LIMIT_BYTES", None)
+    total = torch.cuda.get_device_properties(0).total_memory
+    for left in (need[1] * 3 // 4, need[1] // 2, 64 << 20):      # (the allocator takes 20 MB at a time)
+        torch.cuda.empty_cache()
+        try:
+            torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + 7 * q.numel() * 4 + left) / total)
+            got = step()
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+        check(got)
+        del got
