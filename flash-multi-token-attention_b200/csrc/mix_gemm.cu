@@ -253,7 +253,7 @@ mix_dq_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ C
         for (int t = 0; t < NT; ++t) {
           // a tile past its last block (or past the last row tile) gets an earlier valid block's data
           const int rt = min(NT * q + t, p.nRT - 1), kk = min(kb, max(nkb_t[t], 1) - 1);
-          if (CONV) tc::tma_load_3d(smem + (st * NT + t) * Cfg::A_BYTES, &tmC, &a_full[st], kk * BC, rt * BM, lh);
+          if (CONV) tc::tma_load_3d(smem + (st * NT + t) * Cfg::A_BYTES, &tmC, &a_full[st], kk * BC, rt * BM, lh * 2);
           else tc::tma_load_3d(smem + (st * NT + t) * Cfg::A_BYTES, &tmC, &a_full[st], 0, rt * (BM / 8), lh * (p.N8 / 8) + kk * (BC / 8));
         }
         *s_aissued = kb + 1;
@@ -338,11 +338,13 @@ mix_dq_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ C
 }
 
 // ==========================================================================================
+template <bool CONV>
 struct MixDkvCfg {
-  static constexpr int BK = 128, BR = 64, HALO = 8, QR = BR + HALO, NSTG = 4;
-  static constexpr int X_BYTES = BK * BR * 2;                 // P or dC: [BK / 8][BR][16 B]
-  static constexpr int sgP = 0, sgC = X_BYTES, sgdO = 2 * X_BYTES, sgQ = sgdO + BR * 128;
-  static constexpr int STAGE = sgQ + QR * 128;                // 50176 bytes
+  static constexpr int BK = 128, BR = 64, HALO = 8, QR = BR + HALO, NSTG = CONV ? 3 : 4;
+  static constexpr int X_BYTES = BK * BR * 2;                 // P or dC: [BK / 8][BR][16 B]; dC with a filter: two slabs of 64 keys
+  static constexpr int sgP = 0, sgC = X_BYTES, sgCl = 2 * X_BYTES;        // P, dC, its low half (with a filter)
+  static constexpr int sgdO = (CONV ? 3 : 2) * X_BYTES, sgQ = sgdO + BR * 128;
+  static constexpr int STAGE = sgQ + QR * 128;                // 50176 bytes, 66560 with a filter
   static constexpr int KT_BYTES = BK * 128;                   // one dKt tile on its way out
   static constexpr int oBar = NSTG * STAGE;
   static constexpr int kSmemBytes = oBar + 256 + 1024;
@@ -351,10 +353,10 @@ struct MixDkvCfg {
 };
 
 template <bool CONV>
-__global__ void __launch_bounds__(MixDkvCfg::kThreads, 1)
+__global__ void __launch_bounds__(MixDkvCfg<CONV>::kThreads, 1)
 mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO, const __grid_constant__ CUtensorMap tmdKt,
                 const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmC, const MixParams p, int cq, int d, MixGradOut dV, MixGradOut dK, int early) {
-  using Cfg = MixDkvCfg;
+  using Cfg = MixDkvCfg<CONV>;
   constexpr int BK = Cfg::BK, BR = Cfg::BR, HALO = Cfg::HALO, NSTG = Cfg::NSTG;
   constexpr int W_TMA = Cfg::kEpWarps, W_A0 = Cfg::kEpWarps + 1;
   extern __shared__ unsigned char smem_raw[];
@@ -398,13 +400,14 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const int st = it % NSTG, ph = (it / NSTG) & 1, i0 = (qb_begin + it) * BR;
         if (!tc::mbar_wait(&empty[st], ph ^ 1, s_abort)) break;
         unsigned char* sg = smem + st * Cfg::STAGE;
-        tc::mbar_expect_tx(&full[st], Cfg::STAGE);
+        tc::mbar_expect_tx(&full[st], CONV && !p.dc_lo ? Cfg::STAGE - Cfg::X_BYTES : Cfg::STAGE);
         tc::tma_load_3d(sg + Cfg::sgdO, &tmdO, &full[st], col0, i0, bh);
         tc::tma_load_3d(sg + Cfg::sgQ, &tmQ, &full[st], col0, i0 - HALO, bh);
         tc::tma_load_3d(sg + Cfg::sgP, &tmP, &full[st], 0, i0 / 8, (lh * p.N8 + j0) / 8);
-        if (CONV) {                                            // two slabs of 64 keys
-          tc::tma_load_3d(sg + Cfg::sgC, &tmC, &full[st], j0, i0, lh);
-          tc::tma_load_3d(sg + Cfg::sgC + BR * 128, &tmC, &full[st], j0 + 64, i0, lh);
+        if (CONV) {                                            // two slabs of 64 keys, hi and lo
+          for (int hl = 0; hl < (p.dc_lo ? 2 : 1); ++hl)
+            for (int sl = 0; sl < 2; ++sl)
+              tc::tma_load_3d(sg + (hl ? Cfg::sgCl : Cfg::sgC) + sl * (BR * 128), &tmC, &full[st], j0 + 64 * sl, i0, lh * 2 + hl);
         } else {
           tc::tma_load_3d(sg + Cfg::sgC, &tmC, &full[st], 0, i0 / 8, (lh * p.N8 + j0) / 8);
         }
@@ -445,6 +448,11 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tc::mma_ss2pe(dacc, ca_lo, ca_hi, bl, qb_hi, idg, it != 0);
 #pragma unroll
         for (int k = 1; k < BR / 16; ++k) tc::mma_ss2e<1>(dacc, ca_lo + k * c_step, ca_hi, bl + (uint32_t)(k * (2048 / 16)), qb_hi, idg);
+        if (CONV && p.dc_lo) {
+          const uint32_t cl_lo = ca_lo + (uint32_t)((Cfg::sgCl - Cfg::sgC) >> 4);
+#pragma unroll
+          for (int k = 0; k < BR / 16; ++k) tc::mma_ss2e<1>(dacc, cl_lo + k * c_step, ca_hi, bl + (uint32_t)(k * (2048 / 16)), qb_hi, idg);
+        }
       }
       tc::mma_commit_e(&empty[st]);
     }
@@ -525,9 +533,9 @@ bool make_x8_map(CUtensorMap* map, const bf16* base, const MixParams& mp, int ro
   return make_tensor_map_bf16(map, base, 64, mp.RP / 8, (size_t)mp.nU * mp.G * (mp.N8 / 8), 64, rows / 8, false, keys / 8);
 }
 
-// dC with a filter: row-major, rows x 64 keys in a 128-byte-swizzled tile.
+// dC with a filter: row-major, rows x 64 keys in a 128-byte-swizzled tile; the (hi, lo) halves of a head one after the other.
 bool make_dc_map(CUtensorMap* map, const MixParams& mp, int rows) {
-  return make_tensor_map_bf16(map, mp.C8, mp.N8, mp.RP, (size_t)mp.nU * mp.G, 64, rows, true);
+  return make_tensor_map_bf16(map, mp.C8, mp.N8, mp.RP, (size_t)mp.nU * mp.G * 2, 64, rows, true);
 }
 
 template <int D>
@@ -570,7 +578,7 @@ cudaError_t launch_mix_dq(const TrainParams& p, const MixParams& mp, const __nv_
 #undef FMTA_MIX_DQ
 }
 cudaError_t launch_mix_dkdv(const TrainParams& p, const MixParams& mp, __nv_bfloat16* dKt, bool early, cudaStream_t stream) {
-  using Cfg = MixDkvCfg;
+  using Cfg = MixDkvCfg<true>;                    // (the tiles are the same without a filter)
   const size_t BH = (size_t)p.B * p.H;
   const bool conv = p.theta != nullptr;
   const int cq = conv ? p.cq : 1;
@@ -580,10 +588,11 @@ cudaError_t launch_mix_dkdv(const TrainParams& p, const MixParams& mp, __nv_bflo
   if (!make_tensor_map_bf16(&tmdO, p.dO, p.d, p.N, BH, 64, Cfg::BR, true)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmdKt, conv ? dKt : p.Q, p.d, p.N, conv ? BH * cq * 2 : BH, 64, Cfg::BK, true)) return cudaErrorInvalidValue;
   auto kern = conv ? mix_dkdv_kernel<true> : mix_dkdv_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+  const int smem = conv ? MixDkvCfg<true>::kSmemBytes : MixDkvCfg<false>::kSmemBytes;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   const MixGradOut dV = {p.dVo, nullptr, p.grad_bf16, 1.f}, dK = {conv ? nullptr : p.dKo, nullptr, p.grad_bf16, p.scale};
-  return launch_pdl(kern, dim3(mp.N8 / 128 * (p.d / 64), mp.nU * mp.G), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmQ, tmdO,
+  return launch_pdl(kern, dim3(mp.N8 / 128 * (p.d / 64), mp.nU * mp.G), dim3(Cfg::kThreads), (size_t)smem, stream, tmQ, tmdO,
                     tmdKt, tmP, tmC, mp, cq, p.d, dV, dK, (int)early);
 }
 

@@ -346,13 +346,24 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if constexpr (KT == 8) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
       else *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
     };
-    auto store_dc = [&](size_t lh, int key, const uint32_t (&w)[KP]) {
+    auto store_dc = [&](size_t lh, int key, const float (&v)[KT]) {
+      uint32_t w[KP];
+#pragma unroll
+      for (int k = 0; k < KP; ++k) w[k] = pack_bf16(v[2 * k], v[2 * k + 1]);
       if constexpr (!CONV) {
         store8(p.C8, lh, key, w);
       } else {
-        bf16* dst = p.C8 + (lh * p.RP + gi) * p.N8 + key;
-        if constexpr (KT == 8) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
-        else *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+        auto put = [&](bf16* dst) {
+          if constexpr (KT == 8) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+          else *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
+        };
+        bf16* dst = p.C8 + (lh * 2 * p.RP + gi) * p.N8 + key;
+        put(dst);
+        if (p.dc_lo) {
+#pragma unroll
+          for (int k = 0; k < KP; ++k) w[k] = pack_bf16(v[2 * k] - __uint_as_float(w[k] << 16), v[2 * k + 1] - __uint_as_float(w[k] & 0xffff0000u));
+          put(dst + (size_t)p.RP * p.N8);
+        }
       }
     };
 
@@ -540,10 +551,7 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                   if (e >= 0 && e < band) { cb[e] = v[k]; v[k] = 0.f; }
                 }
               }
-              uint32_t w[KP];
-#pragma unroll
-              for (int k = 0; k < KP; ++k) w[k] = pack_bf16(v[2 * k], v[2 * k + 1]);
-              store_dc(lh0 + x0 + c, j, w);
+              store_dc(lh0 + x0 + c, j, v);
             }
           }
           // ---- dW[g][x] += sum dC'_g S_x ----
@@ -636,7 +644,7 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         for (int i = tid; i < G * nch * 16; i += 256) {
           const int g = i / (nch * 16), rem = i - g * nch * 16;
           const int row = p.nRT * BM + (rem & 15), ch = rem >> 4;
-          bf16* dst = CONV ? p.C8 + ((lh0 + g) * p.RP + row) * p.N8 + k_lo + 8 * ch : p.C8 + (((lh0 + g) * kc8 + (k_lo >> 3) + ch) * p.RP + row) * 8;
+          bf16* dst = CONV ? p.C8 + ((lh0 + g) * 2 * p.RP + row) * p.N8 + k_lo + 8 * ch : p.C8 + (((lh0 + g) * kc8 + (k_lo >> 3) + ch) * p.RP + row) * 8;
           *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
         }
       }

@@ -11,6 +11,7 @@ inline size_t up(size_t x) { return (x + 1023) / 1024 * 1024; }
 
 // P (and dC) of one (batch, group) unit takes 2 (4) bytes per entry of the N x N score matrices of its G heads, so a launch
 // handles as many units as fit kMixChunkBytes: enough CTAs for the GPU, and a workspace that does not grow with the batch.
+// (The low half of dC, 2 bytes more with a filter, is not counted.)
 // A unit above kMixUnitMax is left to the kernels that need no such buffers.
 constexpr size_t kMixChunkBytes = (size_t)4500 << 20, kMixUnitMax = (size_t)16 << 30;
 
@@ -19,7 +20,7 @@ struct MixPlan {
   bool conv, causal, bwd;
   int nRT, N8, RP, U, nU, nKC, kch;
   size_t unit;            // bytes of one operand tensor (P or dC) of a unit
-  size_t kt, cband, dkt, theta_part, dw_part, stat, x8;      // bytes of the workspace's parts (0: absent)
+  size_t kt, cband, dkt, theta_part, dw_part, stat, p8, c8;  // bytes of the workspace's parts (0: absent)
   size_t rows;
   int theta_band_slots, theta_post_slots, dw_slots;
 };
@@ -62,7 +63,8 @@ MixPlan plan_units(int B, int H, int N, int d, int cq, int ck, int G, bool conv,
   } else {
     m.stat = (size_t)m.nU * G * 2 * m.nKC * 3 * m.RP * 4;
   }
-  m.x8 = (size_t)m.nU * m.unit;
+  m.p8 = (size_t)m.nU * m.unit;
+  if (bwd) m.c8 = m.p8 * (conv ? 2 : 1);          // with a filter (hi, lo)
   return m;
 }
 
@@ -95,8 +97,8 @@ size_t carve(const MixPlan& m, void* base, MixBuffers& b) {
     if (m.conv && m.causal) { take(b.dQ, m.rows * m.d * 4); take(b.dK, m.rows * m.d * 4); }
   }
   take(b.stat, m.stat);
-  take(b.P8, m.x8);
-  if (m.bwd) take(b.C8, m.x8);
+  take(b.P8, m.p8);
+  take(b.C8, m.c8);
   return off + 1024;
 }
 
@@ -107,7 +109,7 @@ MixPlan plan(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool 
   MixPlan m = plan_units(B, H, N, d, cq, ck, G, conv, causal, bwd, ~(size_t)0);
   while (bytes_of(m) > limit) {
     // (the statistics of a smaller launch may take more per unit: one by one from what P and dC alone allow)
-    const size_t fit = limit / (m.unit * (bwd ? 2 : 1)), most = fit < (size_t)m.nU - 1 ? fit : m.nU - 1;
+    const size_t fit = limit / ((m.p8 + m.c8) / m.nU), most = fit < (size_t)m.nU - 1 ? fit : m.nU - 1;
     if (most == 0) { m.nU = 0; break; }
     m = plan_units(B, H, N, d, cq, ck, G, conv, causal, bwd, most);
   }
@@ -199,7 +201,7 @@ cudaError_t launch_mix_bwd(const TrainParams& p_, const void* dO, bool do_f32, c
   MixParams q;
   fill(q, p, m, status);
   q.Cband = p.Cband; q.dCband = p.dCband; q.dW_part = b.dw_part;
-  q.P8 = b.P8; q.C8 = b.C8;
+  q.P8 = b.P8; q.C8 = b.C8; q.dc_lo = conv && (want & 1);
   if (conv) {
     FMTA_TRY(launch_ktilde(p, b.Kt, stream, true));
     if (p.causal) FMTA_TRY(launch_band_scores(p, stream));

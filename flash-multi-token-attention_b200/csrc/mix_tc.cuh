@@ -14,7 +14,9 @@
 // of the score kernel owns a row, so its 16-byte stores of 8 keys are contiguous across a warp; and every consumer gets an
 // MMA operand with one tiled copy of 128-byte pieces: no-swizzle core matrices, K-major for O = P V and dQ (a row shift is
 // 16 bytes), MN-major for dV = P^T dO and dKt = dC^T Q.  With a filter dC is row-major instead: dQ reads it at c_q row shifts,
-// which move whole rows of a swizzled tile.
+// which move whole rows of a swizzled tile.  And it is a (hi, lo) pair there: dTheta is a sum of dC S over every score entry
+// whose terms cancel, and one bf16 rounding of dC costs it five times its error (3.2e-4 of it with 32-bit dC, 1.6e-3 with hi
+// alone, 3.2e-4 with the pair; N 1001 to 2048).  dKt takes both, dQ, which is rounded at the same size anyway, hi.
 #pragma once
 #include <cuda.h>
 
@@ -33,12 +35,13 @@ struct MixParams {
   const float* Cband;     // causal with a filter: [B*H, N, band] scores of the band after the filter, natural units (else nullptr)
   float* dCband;          // backward: the gradient of those
   bf16* P8;               // [heads of the launch][N8 / 8][RP][8]
-  bf16* C8;               // backward: dC, the same; with a filter row-major, [heads of the launch][RP][N8]
+  bf16* C8;               // backward: dC, the same; with a filter row-major, [heads of the launch][hi, lo][RP][N8]
   float* ref;             // forward: [heads of the launch][N8 / 16][RP] log2 reference of 16 keys of P
   float* stat;            // forward: [heads of the launch][2 nKC][3][RP]: row max, reference, sum, per key chunk and half
   float* dW_part;         // backward: [slots][H/G][G*G], slot = (b * nRT + row tile) * nKC + key chunk
   int* status;
   int B, H, N, G, cq, ck, causal;
+  int dc_lo;              // with a filter: the low halves of dC are wanted (dTheta is)
   int u0, nU;             // (batch, group) units of this launch: u0 .. u0 + nU - 1
   int nRT, nKC, kch;      // row tiles of 128, key chunks of kch keys
   int RP, N8;

@@ -63,7 +63,7 @@ extern "C" {
 #define FMTA_OP_BWD_FUSED 6      /* fmta_bwd_fused */
 /* Head mixing on the tensor cores (d = 64 or 128, groups of 2, 4, 8 or 16 heads, c_q <= 7): fmta_fwd with path -1 or 1 and a
  * workspace of FMTA_OP_MIX_FWD; fmta_mix_bwd with FMTA_OP_MIX_BWD.  P (and dC) of a few (batch, group) units at a time:
- * at most 4.5 GiB, or one unit's.  Of one call, and with less: fmta_mix_workspace_bytes. */
+ * at most 4.5 GiB, or one unit's (with a filter, half as much again for the low half of dC).  Of one call, and with less: fmta_mix_workspace_bytes. */
 #define FMTA_OP_MIX_FWD 7
 #define FMTA_OP_MIX_BWD 8
 

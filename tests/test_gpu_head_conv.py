@@ -150,3 +150,22 @@ def test_output_types_the_kernels_do_not_write_are_refused():
     for dt in (torch.float16, torch.float64, torch.int32):
         with pytest.raises(RuntimeError):
             F.conv_headmix_forward(q, q, q, torch.eye(4, device="cuda"), out_dtype=dt)
+
+
+@pytest.mark.parametrize("B,H,N,d,G,cq,ck,causal", [(1, 4, 700, 64, 4, 6, 11, True), (2, 4, 513, 128, 2, 3, 5, False), (1, 8, 400, 64, 8, 7, 7, True)])
+def test_filter_gradient_of_conv_mix_keeps_its_precision(B, H, N, d, G, cq, ck, causal):
+    """dTheta against float64, in the 2-norm.  O, whose rounding to bf16 probabilities enters through D, leaves 3e-4 to 8e-4 of
+    it (kernels with 32-bit score gradients; least at the longest); one bf16 rounding of the score gradients makes 1.5e-3 to 2.2e-3."""
+    import fmta_b200 as F
+    Q, K, V, dO, _ = orc.make_inputs(B, H, N, d, cq, ck, seed=N, dtype=torch.bfloat16)
+    g = torch.Generator().manual_seed(N)
+    wg = torch.eye(G).repeat(H // G, 1, 1) + 0.02 * torch.randn(H // G, G, G, generator=g)
+    theta = 0.02 * torch.randn(H, cq, ck, generator=g)
+    theta[:, cq - 1, ck // 2] += 1.0
+    scale = 1.0 / math.sqrt(d)
+    dev = lambda t: t.cuda().double()
+    dth = orc.conv_headmix_bwd_autograd(dev(Q), dev(K), dev(V), dev(theta), dev(orc.block_diag_mix(wg)), dev(dO), scale, causal)[3]
+    q, k, v, do = (t.cuda().to(torch.bfloat16) for t in (Q, K, V, dO))
+    o, l, m, lse = F.conv_headmix_forward(q, k, v, wg.cuda(), theta.cuda(), scale, causal, out_dtype=torch.float32)
+    got = F.conv_headmix_backward(q, k, v, wg.cuda(), o, do, l, m, theta.cuda(), causal, scale, lse=lse)[4]
+    assert float((got.double() - dth).norm()) <= 1.1e-3 * float(dth.norm())
