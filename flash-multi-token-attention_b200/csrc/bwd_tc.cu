@@ -970,6 +970,7 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
           ok = ok && tc::mbar_wait(&bars[a == 0 ? 0 : 1], 0, s_abort);
         }
         uint32_t ah[2][4], al[2][4];
+        if (dK == nullptr) continue;                         // only dTheta is wanted
         ldsm_x4(ah[0], sT + 2 * a * T_ELEMS + t_off);
         ldsm_x4(ah[1], sT + 2 * a * T_ELEMS + t_off + 16);
         if (kThetaLo) {
@@ -998,7 +999,7 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     }
   }
   pdl_wait();      // for the band kernel's part of dK (and what 'this kernel has completed' has to imply)
-  {
+  if (dK != nullptr) {
     const int g = lane >> 2, t4 = lane & 3;
 #pragma unroll
     for (int m = 0; m < 2; ++m)

@@ -460,7 +460,7 @@ int fmta_mix_bwd(const void* Q, const void* K, const void* V, const void* dO, in
   if (int s = fill_bwd(p, Q, K, V, dO, /* D is made here */ LSE, LSE, theta, wmix, B, H, N, d, cq, ck, G, scale, causal)) return s;
   if (!O || !wmix) return FMTA_ERR_NULL;
   const int want = (dQ ? 1 : 0) | (dK ? 2 : 0);
-  if (!want || (!dK) != (!dV) || (theta && want != 3)) return FMTA_ERR_NULL;
+  if (!want || (!dK) != (!dV)) return FMTA_ERR_NULL;
   if (dQ && (!dW || (theta && !dTheta))) return FMTA_ERR_NULL;
   for (int t : {do_dtype, o_dtype, grad_dtype})
     if (t != FMTA_DTYPE_F32 && t != FMTA_DTYPE_BF16) return FMTA_ERR_UNSUPPORTED;

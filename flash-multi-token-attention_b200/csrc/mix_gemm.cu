@@ -373,6 +373,7 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int nh = d / 64, lh = blockIdx.y, kt = blockIdx.x / nh, col0 = (blockIdx.x % nh) * 64;
   const int u = p.u0 + lh / p.G, HG = p.H / p.G, b = u / HG, bh = b * p.H + (u - b * HG) * p.G + lh % p.G;
   const int N = p.N, pq = cq - 1, j0 = kt * BK;
+  const bool with_dv = dV.out != nullptr;                     // (with a filter dKt may be wanted alone, for dTheta)
   const int nQB = (N + BR - 1) / BR, qb_begin = p.causal ? min(nQB, j0 / BR) : 0, nblk = nQB - qb_begin;
 
   if (tid == 0) {
@@ -400,12 +401,14 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const int st = it % NSTG, ph = (it / NSTG) & 1, i0 = (qb_begin + it) * BR;
         if (!tc::mbar_wait(&empty[st], ph ^ 1, s_abort)) break;
         unsigned char* sg = smem + st * Cfg::STAGE;
-        tc::mbar_expect_tx(&full[st], CONV && !p.dc_lo ? Cfg::STAGE - Cfg::X_BYTES : Cfg::STAGE);
-        tc::tma_load_3d(sg + Cfg::sgdO, &tmdO, &full[st], col0, i0, bh);
+        tc::mbar_expect_tx(&full[st], Cfg::STAGE - (with_dv ? 0 : Cfg::X_BYTES + BR * 128));
+        if (with_dv) {
+          tc::tma_load_3d(sg + Cfg::sgdO, &tmdO, &full[st], col0, i0, bh);
+          tc::tma_load_3d(sg + Cfg::sgP, &tmP, &full[st], 0, i0 / 8, (lh * p.N8 + j0) / 8);
+        }
         tc::tma_load_3d(sg + Cfg::sgQ, &tmQ, &full[st], col0, i0 - HALO, bh);
-        tc::tma_load_3d(sg + Cfg::sgP, &tmP, &full[st], 0, i0 / 8, (lh * p.N8 + j0) / 8);
         if (CONV) {                                            // two slabs of 64 keys, hi and lo
-          for (int hl = 0; hl < (p.dc_lo ? 2 : 1); ++hl)
+          for (int hl = 0; hl < 2; ++hl)
             for (int sl = 0; sl < 2; ++sl)
               tc::tma_load_3d(sg + (hl ? Cfg::sgCl : Cfg::sgC) + sl * (BR * 128), &tmC, &full[st], j0 + 64 * sl, i0, lh * 2 + hl);
         } else {
@@ -436,7 +439,7 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       ok = tc::mbar_wait_warp(&full[st], ph, s_abort);
       if (!ok) break;
       tc::tc_fence_after();
-      if (ai == 0) {
+      if (ai == 0 && with_dv) {
         tc::mma_ss2pe(tmem, pa_lo, pa_hi, ob_lo, ob_hi, idescV, it != 0);
 #pragma unroll
         for (int k = 1; k < BR / 16; ++k) tc::mma_ss2e<1>(tmem, pa_lo + (uint32_t)(k * 16), pa_hi, ob_lo + (uint32_t)(k * (2048 / 16)), ob_hi, idescV);
@@ -448,7 +451,7 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         tc::mma_ss2pe(dacc, ca_lo, ca_hi, bl, qb_hi, idg, it != 0);
 #pragma unroll
         for (int k = 1; k < BR / 16; ++k) tc::mma_ss2e<1>(dacc, ca_lo + k * c_step, ca_hi, bl + (uint32_t)(k * (2048 / 16)), qb_hi, idg);
-        if (CONV && p.dc_lo) {
+        if (CONV) {
           const uint32_t cl_lo = ca_lo + (uint32_t)((Cfg::sgCl - Cfg::sgC) >> 4);
 #pragma unroll
           for (int k = 0; k < BR / 16; ++k) tc::mma_ss2e<1>(dacc, cl_lo + k * c_step, ca_hi, bl + (uint32_t)(k * (2048 / 16)), qb_hi, idg);
@@ -469,7 +472,7 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     // dKt leaves as (hi, lo) bf16 pairs (its adjoint takes bf16 operands; one rounding would be one more than dS K has): the hi
     // tiles of all taps go through the stages (read by no MMA any more), then the lo tiles
     for (int hl = 0; hl < (dK.out == nullptr ? 2 : 1); ++hl) {
-    for (int ch = cg + (hl ? 2 : 0); ch < 2 * (1 + cq); ch += NCG) {
+    for (int ch = cg + (hl || !with_dv ? 2 : 0); ch < 2 * (1 + cq); ch += NCG) {
       const int acc = ch >> 1, half = ch & 1;
       float o[32];
       if (have) {

@@ -359,11 +359,9 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         };
         bf16* dst = p.C8 + (lh * 2 * p.RP + gi) * p.N8 + key;
         put(dst);
-        if (p.dc_lo) {
 #pragma unroll
-          for (int k = 0; k < KP; ++k) w[k] = pack_bf16(v[2 * k] - __uint_as_float(w[k] << 16), v[2 * k + 1] - __uint_as_float(w[k] & 0xffff0000u));
-          put(dst + (size_t)p.RP * p.N8);
-        }
+        for (int k = 0; k < KP; ++k) w[k] = pack_bf16(v[2 * k] - __uint_as_float(w[k] << 16), v[2 * k + 1] - __uint_as_float(w[k] & 0xffff0000u));
+        put(dst + (size_t)p.RP * p.N8);
       }
     };
 

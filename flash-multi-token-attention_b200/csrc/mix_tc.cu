@@ -183,7 +183,7 @@ cudaError_t launch_mix_fwd(const TrainParams& p_, void* workspace, size_t worksp
   return cudaSuccess;
 }
 
-// dO / O in do_f32 / o_bf16; want: 1 = dQ (and dTheta, dW), 2 = dK, dV, 3 = all
+// dO / O in do_f32 / o_bf16; want: 1 = dQ, dTheta and dW, 2 = dK and dV, 3 = all
 cudaError_t launch_mix_bwd(const TrainParams& p_, const void* dO, bool do_f32, const void* O, bool o_bf16, float* dTheta, float* dW, int want,
                            void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   TrainParams p = p_;
@@ -201,7 +201,7 @@ cudaError_t launch_mix_bwd(const TrainParams& p_, const void* dO, bool do_f32, c
   MixParams q;
   fill(q, p, m, status);
   q.Cband = p.Cband; q.dCband = p.dCband; q.dW_part = b.dw_part;
-  q.P8 = b.P8; q.C8 = b.C8; q.dc_lo = conv && (want & 1);
+  q.P8 = b.P8; q.C8 = b.C8;
   if (conv) {
     FMTA_TRY(launch_ktilde(p, b.Kt, stream, true));
     if (p.causal) FMTA_TRY(launch_band_scores(p, stream));
@@ -212,7 +212,7 @@ cudaError_t launch_mix_bwd(const TrainParams& p_, const void* dO, bool do_f32, c
     FMTA_TRY(launch_mix_score(p, q, b.Kt, true, stream));
     if (conv && p.causal) FMTA_TRY(launch_bwd_band_given(p, q.u0 * p.G, q.nU * p.G, stream));
     if (want & 1) FMTA_TRY(launch_mix_dq(p, q, b.Kt, stream));
-    if ((want & 2) || conv) FMTA_TRY(launch_mix_dkdv(p, q, b.dKt, want & 1, stream));      // dTheta comes out of dKt
+    if ((want & 2) || conv) FMTA_TRY(launch_mix_dkdv(p, q, b.dKt, want & 1, stream));      // dTheta comes out of dKt (no dV: p.dVo is null)
   }
   if (conv) {
     FMTA_TRY(launch_dk_post(p, b.dKt, true, b.theta_part + (size_t)m.theta_band_slots * p.H * p.cq * p.ck, status, stream));

@@ -41,7 +41,6 @@ struct MixParams {
   float* dW_part;         // backward: [slots][H/G][G*G], slot = (b * nRT + row tile) * nKC + key chunk
   int* status;
   int B, H, N, G, cq, ck, causal;
-  int dc_lo;              // with a filter: the low halves of dC are wanted (dTheta is)
   int u0, nU;             // (batch, group) units of this launch: u0 .. u0 + nU - 1
   int nRT, nKC, kch;      // row tiles of 128, key chunks of kch keys
   int RP, N8;

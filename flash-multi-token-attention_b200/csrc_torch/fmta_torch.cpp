@@ -366,16 +366,15 @@ std::vector<Tensor> mix_backward_raw(const Mix& m, const Tensor& q, const Tensor
   const Dims& s = m.s;
   arm_status(q);
   const bool conv = m.theta.defined();
-  const Tensor dW = want & 1 ? new_f32(q, {s.H / m.G, m.G, m.G}) : Tensor(), dT = conv ? new_f32(q, {s.H, s.cq, s.ck}) : Tensor();
+  const Tensor dW = want & 1 ? new_f32(q, {s.H / m.G, m.G, m.G}) : Tensor(), dT = conv && (want & 1) ? new_f32(q, {s.H, s.cq, s.ck}) : Tensor();
   if (const size_t n = m.tc_bytes(true, causal, limits.second)) {
     dO = dO.scalar_type() == at::kFloat && dO.is_contiguous() && on16(dO) ? dO : bf16c(dO);
     Tensor g[3];
     for (int i = 0; i < 3; ++i)
-      if (conv || (i == 0 ? want & 1 : want & 2)) g[i] = at::empty(q.sizes(), q.options().dtype(g16 ? at::kBFloat16 : at::kFloat));
-    const Tensor dWt = dW.defined() ? dW : (conv ? new_f32(q, {s.H / m.G, m.G, m.G}) : Tensor());
+      if (i == 0 ? want & 1 : want & 2) g[i] = at::empty(q.sizes(), q.options().dtype(g16 ? at::kBFloat16 : at::kFloat));
     if (const Tensor ws = m.tc_workspace(q, true, causal, n); ws.defined()) {
       check_status(fmta_mix_bwd(ptr(q), ptr(k), ptr(v), ptr(dO), dtype_code(dO.scalar_type()), ptr(O), dtype_code(O.scalar_type()), fptr(LSE), fptr(m.theta),
-                                fptr(m.w), ptr(g[0]), ptr(g[1]), ptr(g[2]), g16 ? FMTA_DTYPE_BF16 : FMTA_DTYPE_F32, fptr(dT), fptr(dWt), s.B, s.H, s.N, s.d,
+                                fptr(m.w), ptr(g[0]), ptr(g[1]), ptr(g[2]), g16 ? FMTA_DTYPE_BF16 : FMTA_DTYPE_F32, fptr(dT), fptr(dW), s.B, s.H, s.N, s.d,
                                 s.cq, s.ck, m.G, (float)scale, causal, ptr(ws), bytes_of(ws), stream_of(q)),
                    "fmta_mix_bwd");
       return {g[0], g[1], g[2], dW, dT};

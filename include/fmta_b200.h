@@ -221,7 +221,7 @@ int fmta_bwd_fused(const void* Q, const void* K, const void* V, const void* dO, 
  * fmta_bwd_prep_D and fmta_bwd with wmix compute, on the tensor-core kernels.  Replaces the host functions
  * `head_conv_attention_bwd_dq_dw` / `_bwd_dkdv` (head_conv_attn/bwd_dq_dw.py:373, bwd_dk_dv.py:407).
  *   dO, O: do_dtype / o_dtype     dQ, dK, dV: grad_dtype     dTheta fp32 (NULL without theta)   dW fp32 [H/G,G,G]
- * Without theta either dQ (and dW) or dK and dV may be NULL.  Shapes and workspace: FMTA_OP_MIX_BWD.
+ * Either dQ (and dW, dTheta) or dK and dV may be NULL: that half of the work is left out.  Shapes and workspace: FMTA_OP_MIX_BWD.
  */
 int fmta_mix_bwd(const void* Q, const void* K, const void* V, const void* dO, int do_dtype, const void* O, int o_dtype,
                  const float* LSE, const float* theta, const float* wmix, void* dQ, void* dK, void* dV, int grad_dtype,

@@ -169,3 +169,25 @@ def test_filter_gradient_of_conv_mix_keeps_its_precision(B, H, N, d, G, cq, ck, 
     o, l, m, lse = F.conv_headmix_forward(q, k, v, wg.cuda(), theta.cuda(), scale, causal, out_dtype=torch.float32)
     got = F.conv_headmix_backward(q, k, v, wg.cuda(), o, do, l, m, theta.cuda(), causal, scale, lse=lse)[4]
     assert float((got.double() - dth).norm()) <= 1.1e-3 * float(dth.norm())
+
+
+@pytest.mark.parametrize("B,H,N,d,G,cq,ck,causal", [(1, 4, 300, 64, 4, 6, 11, True), (1, 4, 257, 128, 2, 3, 5, False), (1, 8, 130, 64, 8, 7, 7, True)])
+def test_halves_of_the_backward_are_halves(B, H, N, d, G, cq, ck, causal):
+    """The calls for half of the gradients give the whole backward's bits and launch only what that half needs."""
+    import fmta_b200 as F
+    from torch.profiler import ProfilerActivity, profile
+    Q, K, V, dO, theta = orc.make_inputs(B, H, N, d, cq, ck, seed=N, dtype=torch.bfloat16)
+    q, k, v, do = (t.cuda().to(torch.bfloat16) for t in (Q, K, V, dO))
+    w, th, scale = torch.eye(G, device="cuda").repeat(H // G, 1, 1) + 0.05, theta.cuda(), 1.0 / math.sqrt(d)
+    o, l, m, lse = F.conv_headmix_forward(q, k, v, w, th, scale, causal, out_dtype=torch.float32)
+    args = (q, k, v, w, o, do, l, m, th, causal, scale)
+    dq, dk, dv, dw, dth = F.conv_headmix_backward(*args)
+    kernels = []
+    for half, want in ((F.conv_headmix_bwd_dq_dw, (dq, dw, dth)), (F.conv_headmix_bwd_dkdv, (dk, dv))):
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            got = half(*args)
+            torch.cuda.synchronize()
+        kernels.append(" ".join(e.key for e in prof.key_averages()))
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    assert "mix_dq_kernel" in kernels[0] and "reduce_partials" in kernels[0]
+    assert "mix_dkdv_kernel" in kernels[1] and "mix_dq_kernel" not in kernels[1] and "reduce_partials" not in kernels[1]
