@@ -126,6 +126,27 @@ bool mix_tc_shape(int B, int H, int N, int d, int cq, int G, bool conv) {
   return (size_t)G * (n8 / 8) * (n8 + 16) * 32 <= kMixUnitMax;
 }
 
+// Short sequences finish sooner on the kernels that keep a group's scores on chip (headmix_dense.cu without a filter, the cluster
+// kernels with one), each direction by itself.  Measured in CUDA graphs, those / these, us, causal:
+//   no filter, forward : theirs grow with N whatever the number of groups, up to these kernels' first 200 rows or so: 16 heads,
+//     d = 64: 39 / 65 at N 224, 64 / 68 at 384, 74 / 69 at 448 (1 group); 125 / 133 and 202 / 197 at 384 and 512 (16 groups);
+//     16 heads, d = 128: 61 / 75, 84 / 77 at 224, 320; 8 heads, d = 64: 25 / 29, 33 / 29 at 192, 256; 2 heads, d = 128: 15 / 17, 20 / 17
+//   no filter, backward: 16 heads, d = 64: 101 / 100 at N 160; d = 128: 101 / 133, 144 / 135 at 64, 96; 2 heads: 20 / 20, 26 / 21
+//   filter: theirs take a step per 64 rows, and another round once their CTAs do not fit the GPU at once (clusters of 8 or 16
+//     leave SMs idle: 112 CTAs).  theta (6,11), 8 heads, d = 128, N 128: forward 27 / 89, backward 151 / 170; N 192: 39 / 91 and
+//     222 / 176; theta (3,3), 4 heads, d = 64, N 64: 12 / 27 and 51 / 57; N 128: 21 / 27 and 92 / 62
+bool mix_tc_pays(int B, int H, int N, int d, int cq, int G, bool conv, bool bwd) {
+  const int g = G >= 16 ? 3 : G >= 8 ? 2 : G >= 4 ? 1 : 0;
+  if (!conv) {
+    constexpr int kRows[2][2][4] = {{{224, 192, 224, 352}, {160, 128, 160, 224}}, {{64, 64, 80, 160}, {32, 32, 40, 80}}};   // [bwd][d = 128][group]
+    return N > kRows[bwd][d == 128][g];
+  }
+  constexpr int kSteps[2][2][2][4] = {{{{2, 2, 3, 6}, {2, 3, 4, 7}}, {{3, 3, 5, 8}, {3, 4, 6, 10}}},          // [bwd][c_q > 4][d = 128][group]
+                                      {{{1, 1, 1, 3}, {0, 1, 1, 2}}, {{1, 1, 2, 4}, {1, 1, 2, 3}}}};
+  const long steps = (N + 63) / 64, fit = G >= 8 ? 112 : 148, rounds = ((long)B * H * steps + fit - 1) / fit;
+  return steps * rounds > kSteps[bwd][cq > 4][d == 128][g];
+}
+
 bool mix_tc_supported(const TrainParams& p) {
   return p.Wmix && mix_tc_shape(p.B, p.H, p.N, p.d, p.cq, p.G, p.theta != nullptr) && tensor_maps_available();
 }

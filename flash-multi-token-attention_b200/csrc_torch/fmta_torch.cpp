@@ -292,10 +292,6 @@ struct Mix {
   Tensor w, theta;        // fp32 [H/G, G, G]; fp32 [H, cq, ck] or undefined
   // Bytes of the tensor-core kernels' workspace, `limit` at most; 0: the other kernels take this call
   size_t tc_bytes(bool bwd, bool causal, int64_t limit) const {
-    if (exact_only()) return 0;
-    // a short sequence without a filter: the 16-row CTAs of the other kernels finish sooner than one 128-row CTA of these (16
-    // heads, d = 64, forward + backward on an idle GPU: 12 us per 16 keys there; 190 us at N = 640, 208 at N = 1024 here)
-    if (!theta.defined() && G >= 8 && s.N <= 224 && (long)s.B * (s.H / G) * ((s.N + 15) / 16) <= 2 * 148) return 0;
     return fmta_mix_workspace_bytes(bwd, s.B, s.H, s.N, s.d, s.cq, s.ck, G, theta.defined(), causal, (size_t)limit);
   }
   // That workspace, or a smaller one (fewer units at a time) where the GPU has no room for it; undefined: for none.  Call it

@@ -340,7 +340,7 @@ size_t fmta_bwd_fused_workspace_bytes(int B, int H, int N, int d, int cq, int ck
 /* FMTA_OP_MIX_FWD (bwd = 0) or FMTA_OP_MIX_BWD for one call whose filter (has_theta) and mask (causal) are known: what that call
  * lays out, never more than fmta_workspace_bytes, which has to cover all of them, nor than `limit` ((size_t)-1: none) -- with
  * less of it the call takes fewer (batch, group) units at a time.  0: the tensor-core kernels do not take the problem, or not
- * with that little. */
+ * with that little, or (unless fmta_set_path(1)) the other kernels finish it sooner: short sequences. */
 size_t fmta_mix_workspace_bytes(int bwd, int B, int H, int N, int d, int cq, int ck, int G, int has_theta, int causal, size_t limit);
 
 #ifdef __cplusplus

@@ -148,12 +148,35 @@ def test_mixing_workspace_follows_a_limit():
 def test_mixing_grids_stay_in_range():
     """grid.y counts heads: a launch takes 65535 of them at most, and what has no loop over launches is left to other kernels."""
     from fmta_b200._lib import lib
-    one = lib.fmta_mix_workspace_bytes(0, 1, 16, 128, 64, 1, 1, 16, 0, 0, ANY)
-    assert one > 0
-    unit = 16 * 16 * (128 + 16) * 16
-    assert lib.fmta_mix_workspace_bytes(0, 8192, 16, 128, 64, 1, 1, 16, 0, 0, ANY) < 65536 // 16 * (unit + one)
-    assert lib.fmta_mix_workspace_bytes(0, 32767, 2, 16, 64, 3, 3, 2, 1, 1, ANY) > 0
-    assert lib.fmta_mix_workspace_bytes(0, 32768, 2, 16, 64, 3, 3, 2, 1, 1, ANY) == 0
+    old = lib.fmta_set_path(1)                   # (whatever the sequences' length)
+    try:
+        need = lambda B, H, N, G, theta: lib.fmta_mix_workspace_bytes(0, B, H, N, 64, 3 if theta else 1, 3 if theta else 1, G, theta, 1, ANY)
+        unit = 16 * 16 * (128 + 16) * 16
+        assert need(4095, 16, 128, 16, 0) > 4095 * unit and need(8192, 16, 128, 16, 0) == need(4095, 16, 128, 16, 0)
+        assert need(32767, 2, 16, 2, 1) > 0 and need(32768, 2, 16, 2, 1) == 0
+    finally:
+        lib.fmta_set_path(old)
+
+
+def test_short_mixes_go_to_the_kernels_that_finish_sooner():
+    """The rule of a mix's default path, for each direction, and the process-wide switch over it."""
+    from fmta_b200._lib import lib
+    on_tc = lambda bwd, B, H, N, d, cq, G: lib.fmta_mix_workspace_bytes(bwd, B, H, N, d, max(cq, 1), max(cq, 1), G, int(cq > 0), 1, ANY) > 0
+    # without a filter: by length alone
+    assert not on_tc(0, 1, 16, 352, 64, 0, 16) and on_tc(0, 1, 16, 353, 64, 0, 16)
+    assert not on_tc(1, 64, 16, 160, 64, 0, 16) and on_tc(1, 1, 16, 161, 64, 0, 16)
+    assert not on_tc(0, 1, 8, 160, 128, 0, 8) and on_tc(1, 1, 8, 160, 128, 0, 8)
+    # with one: steps of 64 rows, rounds of CTAs
+    assert not on_tc(0, 1, 8, 384, 128, 6 + 1, 8) and on_tc(0, 1, 8, 385, 128, 7, 8)
+    assert not on_tc(1, 1, 4, 64, 64, 3, 4) and on_tc(1, 1, 4, 65, 64, 3, 4)
+    assert not on_tc(0, 18, 4, 128, 64, 3, 4) and on_tc(0, 19, 4, 128, 64, 3, 4)
+    old = lib.fmta_set_path(1)
+    try:
+        assert on_tc(0, 1, 16, 1, 64, 0, 16) and on_tc(1, 1, 4, 1, 64, 3, 4)
+        lib.fmta_set_path(0)
+        assert not on_tc(0, 1, 16, 4096, 64, 0, 16)
+    finally:
+        lib.fmta_set_path(old)
 
 
 def test_ops_refuse_cpu_tensors():

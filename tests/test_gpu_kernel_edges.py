@@ -150,6 +150,22 @@ def test_mixing_tiles_and_groups(B, H, N, d, G, cq, ck, causal, spread):
         assert torch.isfinite(got).all() and rel(got, ref) <= tol
 
 
+@pytest.mark.parametrize("B,H,N,d,G,cq,ck,causal", [
+    (1, 4, 127, 64, 2, 3, 5, True), (1, 4, 130, 128, 4, 6, 11, True), (1, 8, 65, 64, 8, 5, 5, False), (2, 2, 193, 64, 2, 7, 7, True),
+    (1, 16, 231, 64, 16, 0, 0, True), (1, 8, 300, 128, 8, 0, 0, False), (1, 16, 65, 64, 16, 3, 3, True),
+    (1, 4, 20, 64, 4, 3, 3, True), (1, 2, 40, 128, 2, 0, 0, False), (1, 16, 129, 128, 16, 0, 0, True),
+])
+@pytest.mark.parametrize("spread", [1.0, 12.0])
+def test_mixing_tiles_and_groups_on_the_tensor_cores(request, B, H, N, d, G, cq, ck, causal, spread):
+    """The same where short sequences would go to the kernels that finish them sooner.  (Not below 20 keys: one key's score
+    gradients vanish, and of two keys' under a sharp softmax the roundings, 2^-9 of P and of dC each, are most of what is left:
+    relative to the gradient they have no bound.)"""
+    from fmta_b200._lib import lib
+    request.addfinalizer(lambda old=lib.fmta_set_path(1): lib.fmta_set_path(old))
+    assert lib.fmta_mix_workspace_bytes(1, B, H, N, d, max(cq, 1), max(ck, 1), G, int(cq > 0), int(causal), 2 ** 64 - 1) > 0
+    test_mixing_tiles_and_groups(B, H, N, d, G, cq, ck, causal, spread)
+
+
 @pytest.mark.parametrize("B,H,N,G,causal", [(1, 16, 1600, 16, True), (1, 16, 2048, 16, True), (2, 16, 1500, 16, True), (1, 8, 2100, 8, True)])
 def test_mixing_stays_in_its_workspace(B, H, N, G, causal):
     """Sizes whose key chunks depend on whether there is a filter: exactly the bytes that the library names, and what lies
@@ -176,11 +192,13 @@ def test_mixing_stays_in_its_workspace(B, H, N, G, causal):
     assert maxabs(o[:, :, rows], torch.softmax(X, -1) @ v.double()) <= 2e-2
 
 
-@pytest.mark.parametrize("G,N,conv", [(16, 16, False), (16, 128, False), (2, 16, True)])
-def test_mixing_more_heads_than_a_grid_dimension(G, N, conv):
+@pytest.mark.parametrize("G,N,conv,tensor_cores", [(16, 16, False, False), (16, 16, False, True), (16, 128, False, True), (2, 16, True, False)])
+def test_mixing_more_heads_than_a_grid_dimension(request, G, N, conv, tensor_cores):
     """65552 heads: forward and backward against float64 at the first and last sequences."""
     import fmta_b200 as F
+    from fmta_b200._lib import lib
     B, H, d, scale = 65552 // G, G, 64, 0.125
+    request.addfinalizer(lambda old=lib.fmta_set_path(1 if tensor_cores else -1): lib.fmta_set_path(old))
     g = torch.Generator(device="cuda").manual_seed(N)
     q, k, v, do = (torch.randn(B, H, N, d, device="cuda", generator=g, dtype=torch.bfloat16) for _ in range(4))
     w = torch.eye(G, device="cuda")[None] + 0.1 * torch.randn(1, G, G, device="cuda", generator=g)
