@@ -81,7 +81,7 @@ bool exact_only() { return fmta_set_path(99) == 0; }
 
 // ---------------------------------------------------------------- conv attention
 struct Dims { int B, H, N, d, cq, ck; };
-Dims conv_dims(const Tensor& Q, const Tensor& theta, int64_t pad_q, int64_t pad_k) {
+Dims conv_dims(const Tensor& Q, const Tensor& theta, double pad_q, double pad_k) {
   FMTA_REQUIRE(Q.dim() == 4, "Q must have shape [batch, heads, seq, d_head]");
   Dims s{(int)Q.size(0), (int)Q.size(1), (int)Q.size(2), (int)Q.size(3), 0, 0};
   FMTA_REQUIRE(theta.dim() == 3 && theta.size(0) == s.H, "conv_kernel must have shape [heads, kx, ky]");
@@ -108,7 +108,7 @@ void conv_forward_raw(const Tensor& Q, const Tensor& K, const Tensor& V, const T
 }
 
 std::tuple<Tensor, Tensor, Tensor, Tensor> conv_forward(const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& theta_, double scale,
-                                                       int64_t pad_q, int64_t pad_k, bool causal, bool out_bf16, bool want_lse,
+                                                       double pad_q, double pad_k, bool causal, bool out_bf16, bool want_lse,
                                                        int64_t path, const std::optional<Tensor>& kt) {
   require_cuda_bf16(Q, "Q"); require_cuda_bf16(K, "K"); require_cuda_bf16(V, "V");
   const Dims s = conv_dims(Q, theta_, pad_q, pad_k);
@@ -163,7 +163,7 @@ int conv_backward_op(const Dims& s, int path, int stream, int64_t stream_limit) 
 }
 
 std::tuple<Tensor, Tensor, Tensor, Tensor> conv_backward(const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& dO, const Tensor& D,
-                                                        const Tensor& L, const Tensor& theta_, double scale, int64_t pad_q, int64_t pad_k,
+                                                        const Tensor& L, const Tensor& theta_, double scale, double pad_q, double pad_k,
                                                         bool causal, int64_t path, int64_t stream, int64_t stream_limit,
                                                         const std::optional<Tensor>& kt) {
   require_cuda_bf16(Q, "Q"); require_cuda_bf16(K, "K"); require_cuda_bf16(V, "V"); require_cuda_bf16(dO, "dO");
@@ -194,8 +194,8 @@ Tensor conv_run(const ConvOp& op, const Tensor& Q, const Tensor& K, const Tensor
 }
 
 struct ConvAttnFn : public torch::autograd::Function<ConvAttnFn> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& theta_, double scale, int64_t pad_q,
-                        int64_t pad_k, bool causal, int64_t keep_limit, int64_t stream_limit, bool pad_d32) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& theta_, double scale, double pad_q,
+                        double pad_k, bool causal, int64_t keep_limit, int64_t stream_limit, bool pad_d32) {
     const bool pad = wants_pad(Q, theta_, pad_d32);
     Tensor q = bf16c(Q), k = bf16c(K), v = bf16c(V);
     const Tensor theta = f32(theta_);
@@ -258,7 +258,7 @@ struct ConvAttnFn : public torch::autograd::Function<ConvAttnFn> {
   }
 };
 
-Tensor conv_attention(const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& theta_, double scale, int64_t pad_q, int64_t pad_k,
+Tensor conv_attention(const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& theta_, double scale, double pad_q, double pad_k,
                       bool causal, int64_t keep_limit, int64_t stream_limit, bool pad_d32) {
   FMTA_REQUIRE(Q.is_cuda(), "Q must be a CUDA tensor");
   conv_dims(Q, theta_, pad_q, pad_k);
@@ -495,6 +495,12 @@ Tensor mix_attention(const Tensor& q, const Tensor& k, const Tensor& v, const st
 }
 
 // ---------------------------------------------------------------- decode
+// The filter's address goes to a kernel that reads H of them
+void check_filter(const Tensor& Q, const Tensor& theta) {
+  require_on(Q, theta, "conv_kernel");
+  FMTA_REQUIRE(theta.dim() == 3 && theta.size(0) >= Q.size(1), "conv_kernel must have shape [heads, kx, ky]");
+}
+
 struct Splits { Tensor O, M, L; };
 Splits split_outputs(const Tensor& Q, int64_t B, int64_t H, int64_t ks, int64_t d) {   // carved out of one allocation
   const int64_t n = B * H * ks;
@@ -504,13 +510,15 @@ Splits split_outputs(const Tensor& Q, int64_t B, int64_t H, int64_t ks, int64_t 
 }
 
 std::tuple<Tensor, Tensor, Tensor> decode(const Tensor& Q, const Tensor& K, const Tensor& V, const Tensor& theta_, int64_t ks, double scale,
-                                          int64_t pad_q, int64_t pad_k, bool offset_causal, bool merged_only) {
+                                          double pad_q, double pad_k, bool offset_causal, bool merged_only) {
   at::AutoGradMode no_grad(false);
   require_cuda_bf16(Q, "Q"); require_cuda_bf16(K, "K"); require_cuda_bf16(V, "V");
   FMTA_REQUIRE(Q.dim() == 4 && K.dim() == 4, "Q and K/V must be [batch, heads, seq, d_head]");
   const int64_t B = Q.size(0), H = Q.size(1), q_len = Q.size(2), d = Q.size(3);
   FMTA_REQUIRE(q_len >= 1 && q_len <= 16, "Q sequence length must be between 1 and 16 for inference");
   FMTA_REQUIRE(K.size(0) == B && K.size(1) == H && K.size(3) == d && V.sizes() == K.sizes(), "K/V must be [batch, heads, seq_len, d_head] matching Q");
+  require_on(Q, K, "K"); require_on(Q, V, "V");
+  check_filter(Q, theta_);
   const int64_t Nk = K.size(2), cq = theta_.size(1), ck = theta_.size(2);
   FMTA_REQUIRE(pad_q == cq - 1 && pad_k == (ck - 1) / 2, "pad_q/pad_k must be (kx-1, (ky-1)//2)");
   FMTA_REQUIRE(ks > 0, "k_splits must be positive");
@@ -526,8 +534,8 @@ std::tuple<Tensor, Tensor, Tensor> decode(const Tensor& Q, const Tensor& K, cons
 }
 
 std::tuple<Tensor, Tensor, Tensor> decode_paged(const Tensor& Q, const Tensor& Kp, const Tensor& Vp, const Tensor& table, const Tensor& theta_,
-                                                int64_t ks, double scale, int64_t pad_q, int64_t pad_k, const std::optional<Tensor>& lens,
-                                                const std::optional<int64_t>& max_len, bool offset_causal) {
+                                                int64_t ks, double scale, double pad_q, double pad_k, const std::optional<Tensor>& lens,
+                                                const std::optional<double>& max_len, bool offset_causal) {
   at::AutoGradMode no_grad(false);
   require_cuda_bf16(Q, "Q"); require_cuda_bf16(Kp, "K_pool"); require_cuda_bf16(Vp, "V_pool");
   FMTA_REQUIRE(Q.dim() == 4, "Q must be [batch, heads, seq, d_head]");
@@ -537,22 +545,32 @@ std::tuple<Tensor, Tensor, Tensor> decode_paged(const Tensor& Q, const Tensor& K
   FMTA_REQUIRE(table.scalar_type() == at::kInt && table.is_cuda() && table.is_contiguous() && table.dim() == 2 && table.size(0) == B,
                "block_table must be a contiguous CUDA int32 tensor [batch, max_pages]");
   FMTA_REQUIRE(!lens || (lens->scalar_type() == at::kInt && lens->is_cuda() && lens->numel() == B), "seq_lens must be a CUDA int32 tensor [batch]");
+  require_on(Q, Kp, "K_pool"); require_on(Q, Vp, "V_pool"); require_on(Q, table, "block_table");
+  if (lens) require_on(Q, *lens, "seq_lens");
+  check_filter(Q, theta_);
   const int64_t page = Kp.size(2), max_pages = table.size(1), cq = theta_.size(1), ck = theta_.size(2);
-  const int64_t Nk = max_len ? *max_len : max_pages * page;
+  const int64_t Nk = max_len ? (int64_t)*max_len : max_pages * page;
   FMTA_REQUIRE(pad_q == cq - 1 && pad_k == (ck - 1) / 2, "pad_q/pad_k must be (kx-1, (ky-1)//2)");
   c10::cuda::CUDAGuard guard(Q.device());
-  const Tensor theta = f32(theta_);
+  const Tensor theta = f32(theta_), len = lens ? lens->contiguous() : Tensor();
   Splits o = split_outputs(Q, B, H, ks, d);
-  check_status(fmta_decode_paged(ptr(Q), ptr(Kp), ptr(Vp), table.data_ptr<int>(), lens ? lens->data_ptr<int>() : nullptr, fptr(theta), fptr(o.O),
+  check_status(fmta_decode_paged(ptr(Q), ptr(Kp), ptr(Vp), table.data_ptr<int>(), len.defined() ? len.data_ptr<int>() : nullptr, fptr(theta), fptr(o.O),
                                  fptr(o.M), fptr(o.L), B, H, q_len, Nk, d, cq, ck, ks, (float)scale, page, max_pages, offset_causal, stream_of(Q)),
                "fmta_decode_paged");
   return {o.O, o.M, o.L};
 }
 
-void kv_append_paged(const Tensor& Kp, const Tensor& Vp, const Tensor& table, const Tensor& lens, const Tensor& Kn, const Tensor& Vn) {
+void kv_append_paged(const Tensor& Kp, const Tensor& Vp, const Tensor& table, const Tensor& lens_, const Tensor& Kn, const Tensor& Vn) {
   require_cuda_bf16(Kp, "K_pool"); require_cuda_bf16(Vp, "V_pool"); require_cuda_bf16(Kn, "K_new"); require_cuda_bf16(Vn, "V_new");
-  FMTA_REQUIRE(Kn.dim() == 4, "K_new must be [batch, heads, n_new, d_head]");
+  FMTA_REQUIRE(Kn.dim() == 4 && Vn.sizes() == Kn.sizes(), "K_new and V_new must be [batch, heads, n_new, d_head]");
+  FMTA_REQUIRE(Kp.dim() == 4 && Kp.size(1) == Kn.size(1) && Kp.size(3) == Kn.size(3) && Vp.sizes() == Kp.sizes(),
+               "K_pool/V_pool must be [n_pages, heads, page_size, d_head] matching K_new");
+  FMTA_REQUIRE(table.scalar_type() == at::kInt && table.is_contiguous() && table.dim() == 2 && table.size(0) >= Kn.size(0),
+               "block_table must be a contiguous CUDA int32 tensor [batch, max_pages]");
+  FMTA_REQUIRE(lens_.scalar_type() == at::kInt && lens_.numel() >= Kn.size(0), "seq_lens must be a CUDA int32 tensor [batch]");
+  for (const Tensor* t : {&Vp, &Kn, &Vn, &table, &lens_}) require_on(Kp, *t, "V_pool, K_new, V_new, block_table and seq_lens");
   c10::cuda::CUDAGuard guard(Kp.device());
+  const Tensor lens = lens_.contiguous();
   check_status(fmta_kv_append_paged(ptr(Kp), ptr(Vp), table.data_ptr<int>(), lens.data_ptr<int>(), ptr(Kn), ptr(Vn), Kn.size(0), Kn.size(1),
                                     Kn.size(2), Kn.size(3), Kp.size(2), table.size(1), stream_of(Kp)),
                "fmta_kv_append_paged");

@@ -208,3 +208,46 @@ def test_paged_lengths_beyond_the_table_are_clamped_not_followed():
     F.kv_append_paged(Kp, Vp, table, wild, Knew, Knew)
     torch.cuda.synchronize()
     assert torch.equal(Kp, Kp0) and torch.equal(Vp, Vp0)
+
+
+def _paged_args(B=2, H=2, d=64, page=64, pages=3):
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g).to(torch.bfloat16)
+    return dict(q=rn(B, H, 3, d), kp=rn(B * pages, H, page, d), vp=rn(B * pages, H, page, d), th=0.1 * torch.randn(H, 3, 5, device="cuda", generator=g),
+                table=torch.arange(B * pages, dtype=torch.int32, device="cuda").view(B, pages).contiguous(),
+                lens=torch.tensor([100, 150], dtype=torch.int32, device="cuda"), kn=rn(B, H, 2, d), vn=rn(B, H, 2, d))
+
+
+def test_numbers_and_lengths_are_taken_as_they_come():
+    """Paddings and the longest length as any number, lengths in any layout: as the Python argument checks took them."""
+    import fmta_b200 as F
+    a = _paged_args()
+    run = lambda pq, pk, lens, longest: F.forward_inference_paged(a["q"], a["kp"], a["vp"], a["table"], a["th"], 2, 0.125, pq, pk, seq_lens=lens,
+                                                                  max_seq_len=longest, offset_causal=True)
+    want = run(2, 2, a["lens"], 192)
+    strided = torch.stack([a["lens"], a["lens"]], 1)[:, 0]
+    assert not strided.is_contiguous()
+    for got in (run(2.0, (5 - 1) / 2, a["lens"], 192.0), run(2, 2, strided, 192)):
+        assert all(torch.equal(x, y) for x, y in zip(got, want))
+    q = torch.randn(1, 2, 70, 64, device="cuda").to(torch.bfloat16)
+    assert torch.equal(F.forward(q, q, q, a["th"], 0.125, 2.0, (5 - 1) / 2, True)[0], F.forward(q, q, q, a["th"], 0.125, 2, 2, True)[0])
+
+
+@pytest.mark.parametrize("bad", [dict(th="cpu"), dict(th=(1, 3, 5)), dict(table="cpu"), dict(lens="cpu"), dict(lens=torch.int64), dict(kn="cpu"),
+                                 dict(kn=(2, 3, 2, 64)), dict(kn=(2, 2, 2, 128)), dict(vn=(2, 2, 1, 64)), dict(table=(1, 3))])
+def test_addresses_that_no_kernel_may_follow_are_refused(bad):
+    """Host tensors and shapes that would lead a kernel out of a buffer end in an error on the host."""
+    import fmta_b200 as F
+    a = _paged_args()
+    (name, how), = bad.items()
+    t = a[name]
+    a[name] = t.cpu() if how == "cpu" else t.to(how) if isinstance(how, torch.dtype) else torch.zeros(how, dtype=t.dtype, device="cuda")
+    if name in ("th", "table", "lens"):
+        with pytest.raises(RuntimeError):
+            F.forward_inference_paged(a["q"], a["kp"], a["vp"], a["table"], a["th"], 2, 0.125, 2, 2, seq_lens=a["lens"])
+    if name == "th":
+        with pytest.raises(RuntimeError):
+            F.forward_inference(a["q"], a["kp"][:2].contiguous(), a["vp"][:2].contiguous(), a["th"], 2, 0.125, 2, 2, False)
+    else:
+        with pytest.raises(RuntimeError):
+            F.kv_append_paged(a["kp"], a["vp"], a["table"], a["lens"], a["kn"], a["vn"])
