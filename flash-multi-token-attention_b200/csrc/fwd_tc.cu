@@ -51,10 +51,10 @@ __global__ void __launch_bounds__(256) ktilde_kernel(const bf16* __restrict__ K,
   constexpr int RPB = 256 / CPR;      // rows per block
   __shared__ float sTh[20];
   const int bh = blockIdx.y, h = bh % H, a = blockIdx.z;
-  if (threadIdx.x < ck) sTh[threadIdx.x] = theta[((size_t)h * cq + a) * ck + threadIdx.x] * scale;   // scale carries log2(e)
   pdl_trigger();
+  pdl_wait();      // before any read: the kernel in front may have written K or the filter (an optimizer, a cast)
+  if (threadIdx.x < ck) sTh[threadIdx.x] = theta[((size_t)h * cq + a) * ck + threadIdx.x] * scale;   // scale carries log2(e)
   __syncthreads();
-  pdl_wait();      // nothing before this line touches global memory that a kernel of this library writes or reads back
   const int j = blockIdx.x * RPB + threadIdx.x / CPR, c = threadIdx.x % CPR;
   if (j >= N) return;
   const int pk = (ck - 1) / 2;
@@ -92,12 +92,9 @@ __global__ void __launch_bounds__(256) ktilde_window_kernel(const bf16* __restri
   constexpr int CPR = D / 8, RUNS = 256 / CPR, PK = (CK - 1) / 2, WIN = RR + CK - 1;
   __shared__ float sTh[16 * CK];
   const int bh = blockIdx.y, h = bh % H;
-  for (int i = threadIdx.x; i < cq * CK; i += 256) sTh[i] = theta[(size_t)h * cq * CK + i] * scale;
   pdl_trigger();
-  __syncthreads();
-  pdl_wait();      // nothing before this line touches global memory that a kernel of this library writes or reads back
+  pdl_wait();      // before any read: the kernel in front may have written K or the filter (an optimizer, a cast)
   const int j0 = (blockIdx.x * RUNS + threadIdx.x / CPR) * RR, c = threadIdx.x % CPR;
-  if (j0 >= N) return;
   const bf16* Kb = K + (size_t)bh * N * D + c * 8;
   uint4 win[WIN];
 #pragma unroll
@@ -105,6 +102,9 @@ __global__ void __launch_bounds__(256) ktilde_window_kernel(const bf16* __restri
     const int jj = j0 + r - PK;
     win[r] = (jj >= 0 && jj < N) ? *reinterpret_cast<const uint4*>(Kb + (size_t)jj * D) : make_uint4(0u, 0u, 0u, 0u);
   }
+  for (int i = threadIdx.x; i < cq * CK; i += 256) sTh[i] = theta[(size_t)h * cq * CK + i] * scale;
+  __syncthreads();
+  if (j0 >= N) return;
   for (int a = 0; a < cq; ++a) {
     float w[CK];
 #pragma unroll

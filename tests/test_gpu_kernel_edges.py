@@ -284,3 +284,25 @@ def test_mixing_with_little_memory(monkeypatch, B, H, G, N, cq, ck):
             torch.cuda.set_per_process_memory_fraction(1.0)
         check(got)
         del got
+
+
+@pytest.mark.parametrize("ck", [5, 13])           # both forms of the pre-pass
+def test_a_filter_written_just_before_is_the_one_read(ck):
+    """The first kernel of a call starts under the tail of whatever ran before it: what that wrote, the filter among it, is
+    read only behind the wait for it."""
+    import fmta_b200 as F
+    B, H, N, d, cq = 4, 16, 128, 64, 5
+    g = torch.Generator(device="cuda").manual_seed(ck)
+    q, k, v = (torch.randn(B, H, N, d, device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+    filters = 0.1 * torch.randn(40, H, cq, ck, device="cuda", generator=g)
+    want = []
+    for f in filters:
+        torch.cuda.synchronize()
+        want.append(F.forward(q, k, v, f, 0.125, cq - 1, (ck - 1) // 2, True)[0])
+    theta, pad = torch.empty_like(filters[0]), torch.empty(32 << 20, device="cuda")
+    got = []
+    for f in filters:
+        pad.zero_()                               # the GPU lags behind: the calls queue up without gaps
+        theta.copy_(f)
+        got.append(F.forward(q, k, v, theta, 0.125, cq - 1, (ck - 1) // 2, True)[0])
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
