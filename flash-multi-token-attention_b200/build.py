@@ -6,7 +6,7 @@ Every translation unit under csrc/ is compiled with
 ``-gencode arch=compute_100a,code=sm_100a -lineinfo`` (cross-compiles without a GPU) and
 linked into ``fmta_b200/libfmta_b200.so`` next to the Python layer, so the library
 travels with the source tree; ``csrc_torch/`` (the operators' host side, C++ against torch) becomes ``fmta_b200/_native.so``.  A unit is rebuilt when it or any header is newer than its
-object file.
+object file, the host side also when torch, the interpreter or the command has changed.
 """
 import argparse
 import concurrent.futures as cf
@@ -82,8 +82,6 @@ def _build_host_layer(force=False, verbose=False):
     import torch
     src = os.path.join(HERE, "csrc_torch", "fmta_torch.cpp")
     hdr = os.path.join(HERE, "..", "include", "fmta_b200.h")
-    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) > max(os.path.getmtime(src), os.path.getmtime(hdr)):
-        return NATIVE
     tdir = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     inc = [os.path.join(tdir, "include"), os.path.join(tdir, "include", "torch", "csrc", "api", "include"),
@@ -94,11 +92,18 @@ def _build_host_layer(force=False, verbose=False):
         cmd += ["-isystem", i]
     cmd += ["-L" + os.path.join(tdir, "lib"), "-L" + os.path.dirname(LIB), "-l:libfmta_b200.so", "-lc10", "-lc10_cuda", "-ltorch",
             "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    # it is bound to the torch (and the interpreter) that it was compiled against
+    stamp, key = os.path.join(OBJ, "_native.stamp"), "\n".join([torch.__version__, sys.version] + cmd)
+    built = open(stamp).read() if os.path.exists(stamp) else None
+    if not force and built == key and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) > max(os.path.getmtime(src), os.path.getmtime(hdr)):
+        return NATIVE
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("host layer failed:\n%s" % (r.stdout + r.stderr)[-4000:])
     if verbose:
         print(r.stdout + r.stderr)
+    with open(stamp, "w") as f:
+        f.write(key)
     return NATIVE
 
 

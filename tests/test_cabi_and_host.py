@@ -210,6 +210,27 @@ def test_kept_stacked_keys_follow_the_environment(value, limit):
     assert int(subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=120).stdout) == limit
 
 
+def test_host_layer_is_rebuilt_for_another_torch(tmp_path, monkeypatch):
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("fmta_b200_build", os.path.join(ROOT, "flash-multi-token-attention_b200", "build.py"))
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    runs = []
+
+    def compiler(cmd, **kw):
+        runs.append(cmd)
+        (tmp_path / "_native.so").write_text("x")
+        return subprocess.CompletedProcess(cmd, 0, "", "")
+
+    monkeypatch.setattr(mod, "OBJ", str(tmp_path))
+    monkeypatch.setattr(mod, "NATIVE", str(tmp_path / "_native.so"))
+    monkeypatch.setattr(mod.subprocess, "run", compiler)
+    for version, builds in ((torch.__version__, 1), (torch.__version__, 1), ("9.9", 2), ("9.9", 2), (torch.__version__, 3)):
+        monkeypatch.setattr(torch, "__version__", version)
+        mod._build_host_layer()
+        assert len(runs) == builds
+
+
 def test_unit_partition_covers_everything():
     from fmta_b200 import sharding as sh
     for n in (1, 7, 16, 64, 1024):
