@@ -13,7 +13,7 @@
 // MMA only when the one before it is under way, so what one issuer does between two tiles (190 cycles) leaves it idle unless
 // the other has MMAs waiting.
 // Measured (B200, c_q 6, causal, N 4096; single CTAs before): d = 128, B 8, H 32: 7.8 -> 5.1 ms; d = 64, B 4, H 16: 831 ->
-// 793 us; d = 64, N 1024, 8 heads, c_q 7: 63 -> 33 us.  Two row tiles per CTA (d = 64, S and dP taking turns in one set of
+// 800 us; d = 64, N 1024, 8 heads, c_q 7: 63 -> 33 us.  Two row tiles per CTA (d = 64, S and dP taking turns in one set of
 // columns) move half the key tiles but took 864 us.  Bound by shared-memory operand reads: 5 KB per 43-cycle dQ MMA at d = 64.
 // Every mbarrier wait is bounded; on expiry the status word is set and the pair drains and leaves.  No TMA multicast.
 #include <cuda.h>
@@ -168,13 +168,13 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const uint32_t s_lo = r_lo - (uint32_t)(Cfg::oRing >> 4);        // descriptor of shared-memory offset 0
       bool ok = true;
       auto wait = [&](uint64_t* bar, int n) {                          // completion n of the barrier
-        ok = tc::mbar_wait_cluster_warp(bar, n & 1, s_abort);
+        ok = tc::mbar_wait_warp(bar, n & 1, s_abort);
         tc::tc_fence_after();
       };
       if (role == 1) {
         const uint32_t q_lo = s_lo + (uint32_t)((Cfg::oQ + (HALO - pq) * 128) >> 4), o_lo = s_lo + (uint32_t)(Cfg::oO >> 4);
         tc::PairRing<NSS> ring(full, empty, s_abort);
-        ok = tc::mbar_wait_cluster_warp(q_full, 0, s_abort);
+        ok = tc::mbar_wait_warp(q_full, 0, s_abort);
         for (int kb = 0; kb < nkb && ok; ++kb) {
           if (kb > 0) wait(s_free, kb - 1);                              // S(kb-1) has been taken
           for (int a = 0; a < cq && ok; ++a) {

@@ -6,8 +6,8 @@
 //     dQ[i'] = ln2 * sum_a sum_j dC[i' + pad_q - a, j] Kt_a[j]
 //     dKt_a  = dC^T Q^(a)  (gradient w.r.t. Kt_a / (scale*log2e) ... i.e. before the pre-pass scaling)     dV = P^T dO
 // and dK / dTheta follow from dKt_a by the adjoint of the pre-pass (dk_post_mma_kernel).
-// The band entries are handled by bwd_band_kernel (bwd_band.cu), which adds its part to the same
-// outputs afterwards.
+// The band entries are handled by bwd_band_kernel (bwd_band.cu), which runs first and leaves its part in fp32; these kernels
+// add it in their epilogues.
 //
 //   bwd_dq_tc_kernel (bwd_dq_tc.cu): dQ on CTA pairs.
 //   bwd_dq_stream_kernel : dQ for the calls that stream P and dC to the dK/dV kernel (bwd_stream.cu): it also leaves
@@ -24,7 +24,7 @@
 //                        lanes (rows of the dV / dKt accumulators).  Q is staged once per block as a
 //                        swizzled tile; its row-shifted views are start-address offsets as above.
 // Head dim 64 here; head dim 128 in bwd_tc128.cu.
-// Every mbarrier wait is bounded; no TMA multicast, no cluster, cta_group::1 only.
+// Every mbarrier wait is bounded; no TMA multicast.  The kernels of this file use no cluster (cta_group::1).
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -422,7 +422,8 @@ struct DkvCfg {
   static_assert(D == 64, "the dK/dV tensor-core kernel is instantiated for d = 64");
   static constexpr int BK = 128;               // keys per CTA (= TMEM lanes)
   static constexpr int BR = 64;                // query rows per block
-  static constexpr int HALO = 8;               // rows of Q staged above the block (pad_q <= 5)
+  static constexpr int HALO = 8;               // rows of Q staged above the block (pad_q <= 6)
+  static_assert(CQMAX - 1 <= HALO, "the taps' row shifts stay in the staged rows");
   static constexpr int QR = BR + HALO;         // 72 rows of Q per stage
   static constexpr int MAXCQ = CQMAX;          // resident Kt tiles; at most 7 accumulators of 64 columns + 64 scratch = 512
   static constexpr int NSTG = (CQMAX <= 6) ? 4 : 3;   // query-block stages in flight (a seventh resident tile leaves room for three)
@@ -468,10 +469,10 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint64_t* empty = bars + NSTG;         // [NSTG]
   uint64_t* kv_full = bars + 2 * NSTG;
   uint64_t* st_full = kv_full + 1;       // S^T in X
-  uint64_t* xs_free = st_full + 1;       // S^T taken into registers (256 arrivals): X free for the next dP^T
+  uint64_t* xs_free = st_full + 1;       // S^T taken into registers (every element-wise thread): X free for the next dP^T
   uint64_t* dpt_full = xs_free + 1;      // dP^T in X
-  uint64_t* xd_free = dpt_full + 1;      // dP^T taken into registers (256 arrivals): X free for S^T
-  uint64_t* pdc_full = xd_free + 1;      // P^T and dC^T (bf16) written to shared memory (256 arrivals)
+  uint64_t* xd_free = dpt_full + 1;      // dP^T taken into registers (every element-wise thread): X free for S^T
+  uint64_t* pdc_full = xd_free + 1;      // P^T and dC^T (bf16) written to shared memory (every element-wise thread)
   uint64_t* pdc_free = pdc_full + 1;     // the dV / dKt MMAs that read them have completed
   uint64_t* all_done = pdc_free + 1;
   uint64_t* never_bar = all_done + 1;    // nothing arrives here (expiry self-test)
@@ -867,10 +868,6 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 //       of shared memory and the products land in the accumulator already summed per (a, b).
 // The rows are staged by TMA (two mbarrier batches, bounded waits); every CTA builds its Toeplitz tiles from the filter.
 // One CTA per (64 keys, batch*head); dTheta leaves as one partial per CTA.
-#ifndef FMTA_DKPOST_THETA_LO
-#define FMTA_DKPOST_THETA_LO 1
-#endif
-constexpr bool kThetaLo = FMTA_DKPOST_THETA_LO != 0;
 struct DkPostCfg {
   static constexpr int D = 64, NT = 256;
   static constexpr int KEYS = 64, HALO = 8, ROWS = KEYS + 2 * HALO;   // c_k <= 17
@@ -973,10 +970,8 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         if (dK == nullptr) continue;                         // only dTheta is wanted
         ldsm_x4(ah[0], sT + 2 * a * T_ELEMS + t_off);
         ldsm_x4(ah[1], sT + 2 * a * T_ELEMS + t_off + 16);
-        if (kThetaLo) {
-          ldsm_x4(al[0], sT + (2 * a + 1) * T_ELEMS + t_off);
-          ldsm_x4(al[1], sT + (2 * a + 1) * T_ELEMS + t_off + 16);
-        }
+        ldsm_x4(al[0], sT + (2 * a + 1) * T_ELEMS + t_off);
+        ldsm_x4(al[1], sT + (2 * a + 1) * T_ELEMS + t_off + 16);
 #pragma unroll
         for (int sh = 0; sh < 3 * HL; ++sh) {
           const int st = sh % 3;
@@ -988,10 +983,8 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
             if (m >= 0 && m < 2) {
               mma_bf16(acc[m][0], ah[ks], bfr[0], bfr[1]);
               mma_bf16(acc[m][1], ah[ks], bfr[2], bfr[3]);
-              if (kThetaLo) {
-                mma_bf16(acc[m][0], al[ks], bfr[0], bfr[1]);
-                mma_bf16(acc[m][1], al[ks], bfr[2], bfr[3]);
-              }
+              mma_bf16(acc[m][0], al[ks], bfr[0], bfr[1]);
+              mma_bf16(acc[m][1], al[ks], bfr[2], bfr[3]);
             }
           }
         }

@@ -332,7 +332,7 @@ int fmta_bwd_dkdv(const void* Q, const void* K, const void* V, const void* dO, c
 // A head's last CTA of the adjoint kernel adds the dTheta partials itself where the step is bound by the host's launches (no
 // more CTAs than SMs) and they are few; with more of either the fences and the serial sum cost the GPU more (2-15 us) than
 // the reduction's own launch.
-constexpr int kFoldSlots = 32, kFoldCtas = 148;
+constexpr int kFoldSlots = 32, kFoldCtas = kSMs;
 
 static int bwd_impl(const void* Q, const void* K, const void* V, const void* dO, const float* D,
                     const float* LSE, const float* theta, const float* wmix, float* dQ, float* dK, float* dV,

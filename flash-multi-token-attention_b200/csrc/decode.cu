@@ -54,10 +54,10 @@ cudaError_t launch_decode(const DecodeParams& p_, cudaStream_t stream) {
   const long ctas = (long)p.B * p.H * p.k_splits;
   const int kps = decode_keys_per_split(p.Nk, p.k_splits);
   p.n_sub = 1;
-  while (p.n_sub < 8 && ctas * p.n_sub < 2 * 148 && kps / (2 * p.n_sub) >= 256) p.n_sub *= 2;
+  while (p.n_sub < 8 && ctas * p.n_sub < 2 * kSMs && kps / (2 * p.n_sub) >= 256) p.n_sub *= 2;
   // One split needs no merge of splits; up to eight CTAs per (batch, head) on a GPU that is not full merge in their
   // cluster, which saves the second launch (a full GPU keeps the free placement of single CTAs).
-  p.fused = p.k_splits == 1 || (p.k_splits * p.n_sub <= 8 && ctas * p.n_sub <= 2 * 148);
+  p.fused = p.k_splits == 1 || (p.k_splits * p.n_sub <= 8 && ctas * p.n_sub <= 2 * kSMs);
   cudaError_t e;
   {
     ScopedKernelTimer timer_(kKernDecode, stream);

@@ -1,6 +1,6 @@
 // Decode (fwd_inference) kernel: last-query-row conv attention over a KV cache, split-K.
 //
-// Memory-bound: K and V are each read once from HBM with 16-byte loads straight into registers (no shared-memory
+// Memory-bound: K and V are each read once from HBM with 32-byte loads (16 at d = 32) straight into registers (no shared-memory
 // staging, no block-level barrier in the key loop).  Every warp owns a contiguous key range of its split and keeps its own
 // online-softmax state; a step is 32 keys:
 //   S_a[j] = scale * q_a . k_j for the <= 16 most recent query rows                                   (mma.sync)

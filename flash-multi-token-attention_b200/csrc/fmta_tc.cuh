@@ -302,21 +302,6 @@ FMTA_DEVINL void mbar_arrive_cluster(uint32_t cluster_bar) {
 FMTA_DEVINL void st_cluster_u32(uint32_t cluster_dst, uint32_t v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_dst), "r"(v) : "memory");
 }
-// bounded wait whose arrivals may come from the other CTA
-FMTA_DEVINL bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t limit = kSpinLimit) {
-  for (uint32_t i = 0; i < limit; ++i) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    if (ok) return true;
-    if ((i & 1023u) == 1023u && *abort_flag) return false;
-  }
-  *abort_flag = 1;
-  return false;
-}
-FMTA_DEVINL bool mbar_wait_cluster_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, abort_flag));
-}
 // One look at a barrier, no waiting.
 FMTA_DEVINL uint32_t mbar_test(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -336,7 +321,7 @@ struct PairRing {
   bool ready = false;
   FMTA_DEVINL PairRing(uint64_t* f, uint64_t* e, volatile int* a) : full(f), empty(e), abort_flag(a) {}
   FMTA_DEVINL bool take() {
-    if (!ready && !mbar_wait_cluster_warp(&full[slot], ph, abort_flag)) return false;
+    if (!ready && !mbar_wait_warp(&full[slot], ph, abort_flag)) return false;
     tc_fence_after();
     nslot = slot + 1 == NSLOT ? 0 : slot + 1;
     nph = nslot == 0 ? ph ^ 1 : ph;

@@ -244,6 +244,9 @@ template <int D, bool SCORES>
 static cudaError_t launch_fwd_band_t(const TrainParams& p, cudaStream_t stream) {
   using Cfg = FwdBandCfg<D>;
   dim3 grid((win_hi(p) - win_lo(p) + Cfg::R - 1) / Cfg::R, p.H, p.B);
+  // Shapes known at compile time: the square filters of the reference (3, 5, 7), (3,5) and (6,11) of the benchmark's
+  // configurations and (5,9), a wide one between them.  Any other shape runs the form that reads it at run time; B 4, H 16, N 2000,
+  // d = 64, us: (5,9) 44, at run time (5,7) 57, (5,11) 68.
   if (p.cq == 6 && p.ck == 11)
     return launch_kernel<TrainParams>(fwd_band_kernel<D, 6, 11, SCORES>, grid, dim3(Cfg::NT), Cfg::kSmemBytes, stream, -1, p);
   if (p.cq == 7 && p.ck == 7)

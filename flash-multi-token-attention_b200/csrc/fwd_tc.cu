@@ -154,7 +154,7 @@ struct TcParams {
 // 6 KB per CTA, which leaves room for the copies that fill the ring, and every key tile crosses from L2 once for 256 rows.
 //   d = 64 : 256 tensor-memory columns and 113 KB, so two pairs share two SMs: one's softmax under the other's MMAs;
 //   d = 128: S is double-buffered instead (2 x 128 + 64 + 128 columns).
-// Measured (B200, c_q 6, causal, N 4096, single CTAs with two row tiles before): d = 64, B 4, H 16: 415 -> 387 us; d = 128,
+// Measured (B200, c_q 6, causal, N 4096, single CTAs with two row tiles before): d = 64, B 4, H 16: 415 -> 370 us; d = 128,
 // B 8, H 32: 4.33 -> 3.7 ms (1040 TFLOP/s); one sequence of N 1000, 8 heads, d = 128: 80 -> 45 us with the pre-pass and the
 // band kernel.  What bounds it is the supply of key tiles (31 bytes per cycle and SM at the tensor core's rate) and power.
 template <int D>
@@ -290,12 +290,12 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       const uint32_t a_hi = (uint32_t)(dQ0 >> 32), a_lo0 = (uint32_t)dQ0;
       const uint32_t k_hi = (uint32_t)(dK0 >> 32), v_hi = (uint32_t)(dV0 >> 32), b_lo0 = (uint32_t)dK0;
       tc::PairRing<NSLOT> ring(full, empty, s_abort);
-      bool ok = tc::mbar_wait_cluster_warp(q_full, 0, s_abort);
+      bool ok = tc::mbar_wait_warp(q_full, 0, s_abort);
       auto issue_S = [&](int kb) {
         const int buf = kb % NS;
         const uint32_t dS = tmem + Cfg::colS + buf * BC;
         if (kb >= NS) {      // the softmax threads have taken block kb - NS out of this buffer
-          ok = tc::mbar_wait_cluster_warp(&s_free[buf], (kb / NS - 1) & 1, s_abort);
+          ok = tc::mbar_wait_warp(&s_free[buf], (kb / NS - 1) & 1, s_abort);
           if (!ok) return;
           tc::tc_fence_after();
         }
@@ -312,7 +312,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         tc::mma_commit_pair(&s_full[buf]);
       };
       auto issue_PV = [&](int kb) {
-        ok = tc::mbar_wait_cluster_warp(p_full, kb & 1, s_abort);
+        ok = tc::mbar_wait_warp(p_full, kb & 1, s_abort);
         if (!ok) return;
 #pragma unroll
         for (int v = 0; v < Cfg::VT; ++v) {

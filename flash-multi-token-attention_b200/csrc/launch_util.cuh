@@ -8,6 +8,8 @@
 
 namespace fmta {
 
+constexpr int kSMs = 148;      // of a B200: what the rules that fill the GPU count with
+
 // FMTA_NO_PDL=1 in the environment launches every kernel with plain stream order (read once per process).
 inline bool pdl_enabled() {
   static const bool on = [] { const char* e = getenv("FMTA_NO_PDL"); return !(e && e[0] == '1'); }();

@@ -1,9 +1,10 @@
 // The per-head products behind the mixed scores (mix_score.cu), as GEMM pipelines on tcgen05: P and dC come from global memory
-// in the X8 layout (mix_tc.cuh), so there is no element-wise phase in the loops.
+// in the X8 layout or row-major (mix_tc.cuh), so there is no element-wise phase in the loops.
 //   mix_pv_kernel   : O = P V.  CTA = 128 rows of a head; P is relative to one reference per row and key chunk, so the
 //                     accumulator is taken out of tensor memory and rescaled once per chunk.  Writes O, M, L, LSE.
-//   mix_dq_kernel   : dQ[i'] = sum_a dC[i' + pad_q - a] Kt_a.  CTA = two tiles of 128 rows that share every key tile; the row
-//                     shift is 16 bytes per row of the no-swizzle dC operand (136 rows are staged).
+//   mix_dq_kernel   : dQ[i'] = sum_a dC[i' + pad_q - a] Kt_a.  CTA = two tiles of 128 rows that share every key tile (136 rows
+//                     of dC are staged).  With a filter dC is a 128-byte-swizzled row-major tile whose shifted views start 128
+//                     bytes per row further; without one there is a single tap, and dC is a no-swizzle operand.
 //   mix_dkdv_kernel : dV = P^T dO, dKt_a = dC^T Q^(a).  CTA = 128 keys x 64 columns of the head dim (two CTAs at d = 128);
 //                     P and dC are read MN-major, so nothing is transposed.
 // All are bound by the stream of P / dC (2 bytes per score entry and tensor) or by the MMAs at c_q = 6.
@@ -574,7 +575,7 @@ cudaError_t launch_mix_pv(const TrainParams& p, const MixParams& mp, cudaStream_
 }
 cudaError_t launch_mix_dq(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, cudaStream_t stream) {
   // two row tiles per CTA share the key tiles; with fewer than two such CTAs per SM one tile per CTA fills the GPU better
-  const bool one = (long)((mp.nRT + 1) / 2) * mp.nU * mp.G < 2 * 148;
+  const bool one = (long)((mp.nRT + 1) / 2) * mp.nU * mp.G < 2 * kSMs;
 #define FMTA_MIX_DQ(DD, C) (one ? launch_dq_t<DD, 1, C>(p, mp, Kt, stream) : launch_dq_t<DD, 2, C>(p, mp, Kt, stream))
   if (p.theta) return p.d == 64 ? FMTA_MIX_DQ(64, true) : FMTA_MIX_DQ(128, true);
   return p.d == 64 ? FMTA_MIX_DQ(64, false) : FMTA_MIX_DQ(128, false);

@@ -41,9 +41,9 @@ MixPlan plan_units(int B, int H, int N, int d, int cq, int ck, int G, bool conv,
   // (dead ones above the diagonal not counted) even out the load
   m.kch = 1024;
   auto live = [&]() { return (long)m.nRT * ((m.N8 + m.kch - 1) / m.kch) * m.nU / (causal ? 2 : 1); };
-  while (m.kch > 128 && live() < 3 * 148) m.kch /= 2;
+  while (m.kch > 128 && live() < 3 * kSMs) m.kch /= 2;
   // a GPU that is not full: half as long CTAs (a block is at most 64 keys there; with a filter a CTA's fixed cost is larger)
-  if (live() < (conv ? 74 : 148) && G >= (conv ? 4 : 8)) m.kch = 64;
+  if (live() < (conv ? kSMs / 2 : kSMs) && G >= (conv ? 4 : 8)) m.kch = 64;
   m.nKC = (m.N8 + m.kch - 1) / m.kch;
   m.rows = (size_t)B * H * N;
   const int band = (cq - 1) + (ck - 1) / 2;
@@ -143,7 +143,7 @@ bool mix_tc_pays(int B, int H, int N, int d, int cq, int G, bool conv, bool bwd)
   }
   constexpr int kSteps[2][2][2][4] = {{{{2, 2, 3, 6}, {2, 3, 4, 7}}, {{3, 3, 5, 8}, {3, 4, 6, 10}}},          // [bwd][c_q > 4][d = 128][group]
                                       {{{1, 1, 1, 3}, {0, 1, 1, 2}}, {{1, 1, 2, 4}, {1, 1, 2, 3}}}};
-  const long steps = (N + 63) / 64, fit = G >= 8 ? 112 : 148, rounds = ((long)B * H * steps + fit - 1) / fit;
+  const long steps = (N + 63) / 64, fit = G >= 8 ? 112 : kSMs, rounds = ((long)B * H * steps + fit - 1) / fit;
   return steps * rounds > kSteps[bwd][cq > 4][d == 128][g];
 }
 

@@ -36,7 +36,6 @@ struct MixParams {
   float* dCband;          // backward: the gradient of those
   bf16* P8;               // [heads of the launch][N8 / 8][RP][8]
   bf16* C8;               // backward: dC, the same; with a filter row-major, [heads of the launch][hi, lo][RP][N8]
-  float* ref;             // forward: [heads of the launch][N8 / 16][RP] log2 reference of 16 keys of P
   float* stat;            // forward: [heads of the launch][2 nKC][3][RP]: row max, reference, sum, per key chunk and half
   float* dW_part;         // backward: [slots][H/G][G*G], slot = (b * nRT + row tile) * nKC + key chunk
   int* status;
@@ -53,14 +52,10 @@ template <int NC>
 FMTA_DEVINL void tmem_ld_nowait(uint32_t taddr, float* v) {
   if constexpr (NC == 4) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(taddr) : "memory");
-  } else if constexpr (NC == 8) {
+  } else {
+    static_assert(NC == 8, "");
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "r"(taddr) : "memory");
-  } else {
-    static_assert(NC == 16, "");
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]),
-                   "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]) : "r"(taddr) : "memory");
   }
 }
 
