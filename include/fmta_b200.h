@@ -76,8 +76,8 @@ const char* fmta_strerror(int status);
 /*
  * Process-wide kernel selection for the entry points that have no `path` argument:
  * -1 = library default, 0 = exact tile kernels only, 1 = tensor-core kernels off the causal band
- * plus exact kernels on it.  Returns the previous value.
- */
+ * plus exact kernels on it.  Returns the previous value.  A head mix: -1 leaves short sequences
+ * to the kernels that finish them sooner, 0 keeps it off the tensor cores, 1 takes them whatever the length. */
 int fmta_set_path(int path);
 
 /*
