@@ -278,6 +278,7 @@ __global__ void __launch_bounds__(kDecWarps * 32, D == 128 ? 3 : 4) decode_kerne
     for (int u = 0; u < 2; ++u) {
       float v = o[w][2 * u] + o[w][2 * u + 1];
       v += __shfl_down_sync(0xffffffffu, v, 1);
+      if (v != v) v = o[w][2 * u];                           // an infinite V times a zero or negative rest of p: hi alone has its sign
       if (t == 0 && (D >= 64 || g < 4)) sMergeO[warp][g * 2 * VW + 2 * w + u] = v;
     }
   {

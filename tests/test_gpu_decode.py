@@ -251,3 +251,20 @@ def test_addresses_that_no_kernel_may_follow_are_refused(bad):
     else:
         with pytest.raises(RuntimeError):
             F.kv_append_paged(a["kp"], a["vp"], a["table"], a["lens"], a["kn"], a["vn"])
+
+
+@pytest.mark.parametrize("d,k_splits", [(64, 1), (128, 4), (32, 3)])
+def test_infinite_values(d, k_splits):
+    """An infinite entry of V is an infinite output of its column, as a product with a positive probability is; no other column sees it."""
+    import fmta_b200 as F
+    g = torch.Generator(device="cuda").manual_seed(d)
+    q, k, v = (torch.randn(1, 2, n, d, device="cuda", generator=g).to(torch.bfloat16) for n in (3, 500, 500))
+    theta = 0.1 * torch.randn(2, 3, 5, device="cuda", generator=g)
+    want = F.fwd_conv_attn_inference(q, k, v, theta, k_splits, 0.125, 2, 2, False)[0]
+    v[:, :, 77, 3], v[:, :, 401, 5] = float("inf"), float("-inf")
+    v[:, :, 100, 9], v[:, :, 300, 9], v[:, :, 20, 11] = float("inf"), float("-inf"), float("nan")
+    got = F.fwd_conv_attn_inference(q, k, v, theta, k_splits, 0.125, 2, 2, False)[0]
+    assert (got[..., 3] == float("inf")).all() and (got[..., 5] == float("-inf")).all()
+    assert got[..., 9].isnan().all() and got[..., 11].isnan().all()
+    rest = [c for c in range(d) if c not in (3, 5, 9, 11)]
+    assert torch.equal(got[..., rest], want[..., rest])
