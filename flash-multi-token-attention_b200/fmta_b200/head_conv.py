@@ -3,10 +3,10 @@
 ``bwd_dq_dw.py:373``, ``bwd_dk_dv.py:407``), plus the composed "key-query conv then grouped
 head mix" operator of the head-mixing training configuration.
 
-Groups of 2 to 16 heads at head dim 64 or 128 run on the tensor-core kernels (csrc/mix_tc.cuh).  What those
-do not take: 32 heads (without a conv, up to head dim 64) and head dim 32 run on kernels that keep all heads of
-a group in one CTA; a conv with more than seven query taps on kernels that keep one head per CTA of a cluster
-and exchange score tiles.  A dense [H,H] matrix is the single-group case G = H; grouped
+Groups of 2 to 16 heads at head dim 64 or 128 run on the tensor-core kernels (csrc/mix_tc.cuh).  Short
+sequences, which the others finish sooner, and what those do not take -- 32 heads (without a conv, up to head dim 64), head
+dim 32, little memory -- run on kernels that keep all heads of a group in one CTA or, behind a conv (there also more than seven
+query taps), one head per CTA of a cluster, exchanging score tiles.  A dense [H,H] matrix is the single-group case G = H; grouped
 mixing takes ``w`` as [H/G, G, G].
 """
 import math
