@@ -173,7 +173,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       };
       if (role == 1) {
         const uint32_t q_lo = s_lo + (uint32_t)((Cfg::oQ + (HALO - pq) * 128) >> 4), o_lo = s_lo + (uint32_t)(Cfg::oO >> 4);
-        tc::PairRing<NSS> ring(full, empty, s_abort);
+        tc::TileRing<NSS> ring(full, empty, s_abort);
         ok = tc::mbar_wait_warp(q_full, 0, s_abort);
         for (int kb = 0; kb < nkb && ok; ++kb) {
           if (kb > 0) wait(s_free, kb - 1);                              // S(kb-1) has been taken
@@ -198,7 +198,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
       } else {
         const uint32_t c_lo = s_lo + (uint32_t)(Cfg::oC >> 4), rd_lo = r_lo + (uint32_t)(NSS * (Cfg::TILE_BYTES >> 4));
-        tc::PairRing<NSLOT - NSS> ring(full + NSS, empty + NSS, s_abort);
+        tc::TileRing<NSLOT - NSS> ring(full + NSS, empty + NSS, s_abort);
         for (int kb = 0; kb < nkb && ok; ++kb) {
           wait(dc_full, kb);
           for (int a = 0; a < cq && ok; ++a) {

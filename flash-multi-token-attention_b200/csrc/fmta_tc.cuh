@@ -312,14 +312,15 @@ FMTA_DEVINL uint32_t mbar_test(uint64_t* bar, uint32_t parity) {
 // The issuer's end of a ring of tiles.  The tensor core takes an MMA only when the one before it is under way, so whatever
 // the issuer does between two tiles leaves it idle: a wait that is over already still costs 200 cycles.  take() therefore
 // looks at the NEXT tile's barrier before the MMAs of this one are issued and give() picks the answer up behind them.
-template <int NSLOT>
-struct PairRing {
+// G = 2: of a CTA pair (the slots are released in both CTAs).
+template <int NSLOT, int G = 2>
+struct TileRing {
   uint64_t *full, *empty;
   volatile int* abort_flag;
   int slot = 0, ph = 0, nslot = 0, nph = 0;
   uint32_t seen = 0;
   bool ready = false;
-  FMTA_DEVINL PairRing(uint64_t* f, uint64_t* e, volatile int* a) : full(f), empty(e), abort_flag(a) {}
+  FMTA_DEVINL TileRing(uint64_t* f, uint64_t* e, volatile int* a) : full(f), empty(e), abort_flag(a) {}
   FMTA_DEVINL bool take() {
     if (!ready && !mbar_wait_warp(&full[slot], ph, abort_flag)) return false;
     tc_fence_after();
@@ -352,9 +353,9 @@ FMTA_DEVINL void mma_commit_pair(uint64_t* bar) {
       ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 
-template <int NSLOT>
-FMTA_DEVINL void PairRing<NSLOT>::give() {
-  mma_commit_pair(&empty[slot]);
+template <int NSLOT, int G>
+FMTA_DEVINL void TileRing<NSLOT, G>::give() {
+  if constexpr (G == 2) mma_commit_pair(&empty[slot]); else mma_commit_e(&empty[slot]);
   slot = nslot; ph = nph;
   ready = __all_sync(0xffffffffu, seen);
 }

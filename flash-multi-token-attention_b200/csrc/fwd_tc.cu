@@ -289,7 +289,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       const uint64_t dV0 = D == 64 ? tc::make_sdesc(smem_u32(sRing), 16, 512, tc::kLayoutSW64) : dK0;
       const uint32_t a_hi = (uint32_t)(dQ0 >> 32), a_lo0 = (uint32_t)dQ0;
       const uint32_t k_hi = (uint32_t)(dK0 >> 32), v_hi = (uint32_t)(dV0 >> 32), b_lo0 = (uint32_t)dK0;
-      tc::PairRing<NSLOT> ring(full, empty, s_abort);
+      tc::TileRing<NSLOT> ring(full, empty, s_abort);
       bool ok = tc::mbar_wait_warp(q_full, 0, s_abort);
       auto issue_S = [&](int kb) {
         const int buf = kb % NS;

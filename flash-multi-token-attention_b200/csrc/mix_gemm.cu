@@ -1,10 +1,9 @@
 // The per-head products behind the mixed scores (mix_score.cu), as GEMM pipelines on tcgen05: P and dC come from global memory
-// in the X8 layout or row-major (mix_tc.cuh), so there is no element-wise phase in the loops.
+// in the X8 layout (mix_tc.cuh), so there is no element-wise phase in the loops.
 //   mix_pv_kernel   : O = P V.  CTA = 128 rows of a head; P is relative to one reference per row and key chunk, so the
 //                     accumulator is taken out of tensor memory and rescaled once per chunk.  Writes O, M, L, LSE.
 //   mix_dq_kernel   : dQ[i'] = sum_a dC[i' + pad_q - a] Kt_a.  CTA = two tiles of 128 rows that share every key tile (136 rows
-//                     of dC are staged).  With a filter dC is a 128-byte-swizzled row-major tile whose shifted views start 128
-//                     bytes per row further; without one there is a single tap, and dC is a no-swizzle operand.
+//                     of dC are staged; views shifted by a tap's rows start 16 bytes per row further).
 //   mix_dkdv_kernel : dV = P^T dO, dKt_a = dC^T Q^(a).  CTA = 128 keys x 64 columns of the head dim (two CTAs at d = 128);
 //                     P and dC are read MN-major, so nothing is transposed.
 // All are bound by the stream of P / dC (2 bytes per score entry and tensor) or by the MMAs at c_q = 6.
@@ -254,8 +253,7 @@ mix_dq_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ C
         for (int t = 0; t < NT; ++t) {
           // a tile past its last block (or past the last row tile) gets an earlier valid block's data
           const int rt = min(NT * q + t, p.nRT - 1), kk = min(kb, max(nkb_t[t], 1) - 1);
-          if (CONV) tc::tma_load_3d(smem + (st * NT + t) * Cfg::A_BYTES, &tmC, &a_full[st], kk * BC, rt * BM, lh * 2);
-          else tc::tma_load_3d(smem + (st * NT + t) * Cfg::A_BYTES, &tmC, &a_full[st], 0, rt * (BM / 8), lh * (p.N8 / 8) + kk * (BC / 8));
+          tc::tma_load_3d(smem + (st * NT + t) * Cfg::A_BYTES, &tmC, &a_full[st], 0, rt * (BM / 8), lh * (CONV ? 2 : 1) * (p.N8 / 8) + kk * (BC / 8));
         }
         *s_aissued = kb + 1;
         for (int a = 0; a < nB; ++a, ++id) {
@@ -271,8 +269,8 @@ mix_dq_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ C
   } else if (warp > NT * 4) {
     const int t = warp - (NT * 4 + 1);
     constexpr uint32_t idesc = tc::make_idesc(BM, D, 0, 1);
-    const uint64_t dA = CONV ? tc::make_sdesc(smem_u32(smem), 16, 1024, tc::kLayoutSW128) : tc::make_sdesc(smem_u32(smem), AR * 16, 128, tc::kLayoutNone);
-    constexpr uint32_t row_step = CONV ? 8 : 1, k_step = CONV ? 2 : 2 * AR;     // 16-byte units per row and per 16 keys
+    const uint64_t dA = tc::make_sdesc(smem_u32(smem), AR * 16, 128, tc::kLayoutNone);
+    constexpr uint32_t k_step = 2 * AR;                       // 16-byte units per 16 keys; one per row
     const uint64_t dB = tc::make_sdesc(smem_u32(smem) + Cfg::oB, SL > 1 ? Cfg::SLAB : 16, 1024, tc::kLayoutSW128);
     const uint32_t a_hi = (uint32_t)(dA >> 32), a0 = (uint32_t)dA, b_hi = (uint32_t)(dB >> 32), b0 = (uint32_t)dB;
     const uint32_t dst = tmem + t * D;
@@ -283,8 +281,8 @@ mix_dq_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ C
       const int st = kb % NA;
       ok = tc::mbar_wait_warp(&a_full[st], (kb / NA) & 1, s_abort);
       if (!ok) break;
-      uint32_t al = a0 + (uint32_t)((st * NT + t) * (Cfg::A_BYTES >> 4) + pq * row_step);        // dC rows i' + pad_q - a
-      for (int a = 0; a < ntap && ok; ++a, al -= row_step) {
+      uint32_t al = a0 + (uint32_t)((st * NT + t) * (Cfg::A_BYTES >> 4) + pq);        // dC rows i' + pad_q - a
+      for (int a = 0; a < ntap && ok; ++a, --al) {
 #pragma unroll
         for (int hl = 0; hl < nhl; ++hl) {
           ok = tc::mbar_wait_warp(&full[s], ph, s_abort);
@@ -408,13 +406,8 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           tc::tma_load_3d(sg + Cfg::sgP, &tmP, &full[st], 0, i0 / 8, (lh * p.N8 + j0) / 8);
         }
         tc::tma_load_3d(sg + Cfg::sgQ, &tmQ, &full[st], col0, i0 - HALO, bh);
-        if (CONV) {                                            // two slabs of 64 keys, hi and lo
-          for (int hl = 0; hl < 2; ++hl)
-            for (int sl = 0; sl < 2; ++sl)
-              tc::tma_load_3d(sg + (hl ? Cfg::sgCl : Cfg::sgC) + sl * (BR * 128), &tmC, &full[st], j0 + 64 * sl, i0, lh * 2 + hl);
-        } else {
-          tc::tma_load_3d(sg + Cfg::sgC, &tmC, &full[st], 0, i0 / 8, (lh * p.N8 + j0) / 8);
-        }
+        for (int hl = 0; hl < (CONV ? 2 : 1); ++hl)
+          tc::tma_load_3d(sg + (hl ? Cfg::sgCl : Cfg::sgC), &tmC, &full[st], 0, i0 / 8, (lh * (CONV ? 2 : 1) + hl) * (p.N8 / 8) + j0 / 8);
         *s_issued = it + 1;
       }
     }
@@ -431,8 +424,7 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint32_t sg = smem_u32(smem + st * Cfg::STAGE);
       // P / dC: M = keys in chunks of 8, BR * 16 bytes apart; K = rows, 16 bytes apart
       const uint64_t dPa = tc::make_sdesc(sg + Cfg::sgP, 128, BR * 16, tc::kLayoutNone);
-      const uint64_t dCa = CONV ? tc::make_sdesc(sg + Cfg::sgC, BR * 128, 1024, tc::kLayoutSW128) : tc::make_sdesc(sg + Cfg::sgC, 128, BR * 16, tc::kLayoutNone);
-      constexpr uint32_t c_step = CONV ? 2048 / 16 : 16;       // 16 rows
+      const uint64_t dCa = tc::make_sdesc(sg + Cfg::sgC, 128, BR * 16, tc::kLayoutNone);
       const uint64_t dOb = tc::make_sdesc(sg + Cfg::sgdO, 16, 1024, tc::kLayoutSW128);
       const uint64_t dQb = tc::make_sdesc(sg + Cfg::sgQ + (HALO - pq) * 128, 128, 1024, tc::kLayoutSW128);
       const uint32_t pa_hi = (uint32_t)(dPa >> 32), pa_lo = (uint32_t)dPa, ca_hi = (uint32_t)(dCa >> 32), ca_lo = (uint32_t)dCa;
@@ -451,11 +443,11 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const uint32_t bl = qb_lo + (uint32_t)(2 * gi * (128 >> 4));
         tc::mma_ss2pe(dacc, ca_lo, ca_hi, bl, qb_hi, idg, it != 0);
 #pragma unroll
-        for (int k = 1; k < BR / 16; ++k) tc::mma_ss2e<1>(dacc, ca_lo + k * c_step, ca_hi, bl + (uint32_t)(k * (2048 / 16)), qb_hi, idg);
+        for (int k = 1; k < BR / 16; ++k) tc::mma_ss2e<1>(dacc, ca_lo + k * 16, ca_hi, bl + (uint32_t)(k * (2048 / 16)), qb_hi, idg);
         if (CONV) {
           const uint32_t cl_lo = ca_lo + (uint32_t)((Cfg::sgCl - Cfg::sgC) >> 4);
 #pragma unroll
-          for (int k = 0; k < BR / 16; ++k) tc::mma_ss2e<1>(dacc, cl_lo + k * c_step, ca_hi, bl + (uint32_t)(k * (2048 / 16)), qb_hi, idg);
+          for (int k = 0; k < BR / 16; ++k) tc::mma_ss2e<1>(dacc, cl_lo + k * 16, ca_hi, bl + (uint32_t)(k * (2048 / 16)), qb_hi, idg);
         }
       }
       tc::mma_commit_e(&empty[st]);
@@ -533,13 +525,9 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 namespace {
 // An X8 tensor as rows of 128 bytes (8 query rows x 8 keys): box = `rows` query rows x `keys` keys, landing as [keys / 8][rows][16 B]
 // with one copy (as bulk copies of one key chunk each, 1 to 2 KB, the copy engine's cost per copy was what bound these kernels).
-bool make_x8_map(CUtensorMap* map, const bf16* base, const MixParams& mp, int rows, int keys) {
-  return make_tensor_map_bf16(map, base, 64, mp.RP / 8, (size_t)mp.nU * mp.G * (mp.N8 / 8), 64, rows / 8, false, keys / 8);
-}
-
-// dC with a filter: row-major, rows x 64 keys in a 128-byte-swizzled tile; the (hi, lo) halves of a head one after the other.
-bool make_dc_map(CUtensorMap* map, const MixParams& mp, int rows) {
-  return make_tensor_map_bf16(map, mp.C8, mp.N8, mp.RP, (size_t)mp.nU * mp.G * 2, 64, rows, true);
+// parts: 2 for the (hi, lo) pair of a head one after the other
+bool make_x8_map(CUtensorMap* map, const bf16* base, const MixParams& mp, int rows, int keys, int parts = 1) {
+  return make_tensor_map_bf16(map, base, 64, mp.RP / 8, (size_t)mp.nU * mp.G * parts * (mp.N8 / 8), 64, rows / 8, false, keys / 8);
 }
 
 template <int D>
@@ -559,7 +547,7 @@ cudaError_t launch_dq_t(const TrainParams& p, const MixParams& mp, const __nv_bf
   const size_t BH = (size_t)p.B * p.H;
   constexpr bool conv = CONV;
   alignas(64) CUtensorMap tmC, tmB;
-  if (!(CONV ? make_dc_map(&tmC, mp, Cfg::AR) : make_x8_map(&tmC, mp.C8, mp, Cfg::AR, Cfg::BC))) return cudaErrorInvalidValue;
+  if (!make_x8_map(&tmC, mp.C8, mp, Cfg::AR, Cfg::BC, conv ? 2 : 1)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmB, conv ? Kt : p.K, D, p.N, conv ? BH * p.cq * 2 : BH, 64, Cfg::BC, true)) return cudaErrorInvalidValue;
   auto kern = mix_dq_kernel<D, NT_, CONV>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
@@ -587,7 +575,7 @@ cudaError_t launch_mix_dkdv(const TrainParams& p, const MixParams& mp, __nv_bflo
   const bool conv = p.theta != nullptr;
   const int cq = conv ? p.cq : 1;
   alignas(64) CUtensorMap tmQ, tmdO, tmdKt, tmP, tmC;
-  if (!make_x8_map(&tmP, mp.P8, mp, Cfg::BR, Cfg::BK) || !(conv ? make_dc_map(&tmC, mp, Cfg::BR) : make_x8_map(&tmC, mp.C8, mp, Cfg::BR, Cfg::BK))) return cudaErrorInvalidValue;
+  if (!make_x8_map(&tmP, mp.P8, mp, Cfg::BR, Cfg::BK) || !make_x8_map(&tmC, mp.C8, mp, Cfg::BR, Cfg::BK, conv ? 2 : 1)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmQ, p.Q, p.d, p.N, BH, 64, Cfg::QR, true)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmdO, p.dO, p.d, p.N, BH, 64, Cfg::BR, true)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmdKt, conv ? dKt : p.Q, p.d, p.N, conv ? BH * cq * 2 : BH, 64, Cfg::BK, true)) return cudaErrorInvalidValue;

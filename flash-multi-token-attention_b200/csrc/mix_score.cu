@@ -11,6 +11,12 @@
 // with one the stacked score MMAs (2 c_q d / 16 per tile).  With a filter the stacked key operand is a bf16 pair (hi, lo), so
 // that the logits keep 16 mantissa bits as the unstacked products followed by an fp32 filter did.
 //
+// With a filter and two waves of CTAs a cluster of two works on 256 rows with cta_group::2 MMAs, each CTA staging its own queries
+// and half of the keys: the stacked keys (384 KB per CTA and block of 64 keys at G 4, c_q 6, d = 128; 768 KB before) and the
+// shared memory that the MMAs read are what bounds it.  B 2, H 32, N 8192, d = 128, groups of 4: forward 9.6 ms with single CTAs,
+// 6.6 with pairs, 5.6 with (hi, lo) in one MMA; backward 16.5, then 13.5 with dC in X8, 11.4 with half of the heads' scores taken
+// at the start of a block, 10.0 with (hi, lo) in one MMA and all of them taken (a block: 40.5 k cycles in series before).
+//
 // Without a filter neither Q nor dO of 16 heads fits shared memory, so their tiles stream through the ring once per block
 // beside K and V (18 bytes per score entry from L2); with a filter Q stays resident where it fits and the stacked keys stream.
 #include <cuda.h>
@@ -20,21 +26,36 @@
 
 namespace fmta {
 
-template <int G, int D, bool CONV, bool BWD>
+// MODE 0: one CTA per 128 rows; 1: a pair of CTAs per 256 rows (cta_group::2); 2: a pair whose MMAs take high and low keys together
+template <int G, int D, bool CONV, bool BWD, int MODE>
 struct MixCfg {
   static constexpr int BM = 128, SL = D / 64, HALO = 8, QR = BM + HALO;
+  // HL: a tap's low keys lie behind its high ones as 2 KB columns of ONE MMA (rank 0 stages the high, rank 1 the low ones), whose
+  // two halves the element-wise warps add up when they take the scores.  An MMA of KB = 64 columns reads 8 KB of queries for 32
+  // cycles of arithmetic; so it reads them once for both.
+  static constexpr bool HL = MODE == 2;
   // keys per block: S and dP (backward) or two buffers of S (forward with a filter, where the MMAs are the bound) take 256
   // columns each; otherwise one buffer of up to 512
   static constexpr int KB = (BWD || (CONV && G <= 8)) ? 256 / G : (512 / G < 128 ? 512 / G : 128);
-  static constexpr int NBUF = BWD ? 1 : 512 / (G * KB);
+  static constexpr int NBUF = BWD || HL ? 1 : 512 / (G * KB);
+  static constexpr int SN = HL ? 2 * KB : KB;                  // columns of a head's scores
   static constexpr int KT = G >= 8 ? 4 : 8;                    // keys per thread and pass
-  static constexpr int GC = G < 4 ? G : 4;                     // output heads per register pass
+  static constexpr int GC = HL || G < 4 ? 2 : 4;                     // output heads per register pass
   static constexpr int NPASS = KB / 2 / KT;
-  static constexpr bool RES = CONV && G * SL * QR * 128 <= 100 * 1024;   // Q resident; else (with a filter) two stages of one head's Q
+  static constexpr bool PAIR = MODE > 0;
+  static_assert(!PAIR || (CONV && KB >= 32), "pairs: with a filter, N = KB a multiple of 32");
+  static constexpr bool RES = CONV && G * SL * QR * 128 <= (PAIR && !BWD ? 140 : 100) * 1024;   // Q resident; else (with a filter) two stages of one head's Q
   static constexpr int Q_HEAD = SL * QR * 128;
   static constexpr int SLOT = BM * 128;                        // ring slot: one A slab tile, or B slab tiles
-  static constexpr int TB = KB * 128, TPS = 16384 / TB;        // B slab tile (KB keys x 64 columns), tiles per slot
+  static constexpr int KC = PAIR ? KB / 2 : KB;                // keys of a block that this CTA stages
+  static constexpr int TB = (HL ? KB : KC) * 128, TPS = 16384 / TB;        // stacked slab tile (KC keys x 64 columns; HL: KB), tiles per slot
+  static constexpr int TBP = KC * 128;                         // slab tile of K or V
   static constexpr bool DW_MMA = BWD && G == 16;               // dW by mma.sync from transposed bf16 pairs; else in registers
+  // heads whose scores go to registers when a block begins, so that the next block's score MMAs run on those heads' columns
+  // under this block's arithmetic: with HL all (128 registers), else backward the first half
+  static constexpr int colP = HL ? 0 : 256;                    // backward: dP; HL: over the scores of the first half of the heads
+  static constexpr int SH = HL ? G : BWD && G <= 4 ? G / 2 : 0;
+  static constexpr bool STASH = SH > 0;
   static constexpr int oQ = 0;
   static constexpr int oW = oQ + (CONV ? (RES ? G : 2) * Q_HEAD : 0);
   static constexpr int W_BYTES = G * G * 4;
@@ -46,23 +67,25 @@ struct MixCfg {
   static constexpr int NSLOT_ = (226 * 1024 - oRing) / SLOT;
   static constexpr int NSLOT = NSLOT_ > 20 ? 20 : NSLOT_;
   // a slot is held until the last tile that uses it: B tiles of several heads in one slot, with an A slot for each
-  static constexpr int TPP = TPS < NSLOT - 2 ? TPS : NSLOT - 2;
+  static constexpr int TPP = SLOT / TBP < NSLOT - 2 ? SLOT / TBP : NSLOT - 2;
   static constexpr int kSmemBytes = oRing + NSLOT * SLOT + 1024;
   // 8 element-wise warps with 216 registers, a warpgroup with 72 for the TMA and the MMA warp: 256 * 216 + 128 * 72 = 384 * 168,
   // the registers the block is launched with
-  static constexpr int kThreads = 384, kRegsEw = 216, kRegsOther = 72;
+  static constexpr int kThreads = 384, kRegsEw = 224, kRegsOther = 56;
   static_assert(NSLOT >= 4, "ring");
   static_assert(kSmemBytes <= 227 * 1024, "shared memory");
   static_assert(SLOT % 1024 == 0 && TB % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
 };
 
-template <int G, int D, bool CONV, bool BWD>
-__global__ void __launch_bounds__(384, 1)
+template <int G, int D, bool CONV, bool BWD, int MODE>
+__global__ void __cluster_dims__(MODE > 0 ? 2 : 1, 1, 1) __launch_bounds__(384, 1)
 mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmdO, const __grid_constant__ CUtensorMap tmV, const MixParams p) {
-  using Cfg = MixCfg<G, D, CONV, BWD>;
+  using Cfg = MixCfg<G, D, CONV, BWD, MODE>;
   constexpr int BM = Cfg::BM, SL = Cfg::SL, HALO = Cfg::HALO, KB = Cfg::KB, KT = Cfg::KT, GC = Cfg::GC, NPASS = Cfg::NPASS;
-  constexpr int SLOT = Cfg::SLOT, NSLOT = Cfg::NSLOT, TB = Cfg::TB, TPS = Cfg::TPS, TPP = Cfg::TPP, NBUF = Cfg::NBUF;
+  constexpr int SLOT = Cfg::SLOT, NSLOT = Cfg::NSLOT, TB = Cfg::TB, TBP = Cfg::TBP, TPS = Cfg::TPS, TPP = Cfg::TPP, NBUF = Cfg::NBUF;
+  constexpr bool PAIR = Cfg::PAIR, HL = Cfg::HL, HLB = HL && BWD;
+  constexpr int CPG = PAIR ? 2 : 1;                          // CTAs that issue together
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* sQ = smem + Cfg::oQ;
@@ -72,12 +95,13 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   float* sR0 = reinterpret_cast<float*>(smem + Cfg::oRow);                      // [G][128]: LSE (log2) / ref
   float* sR1 = sR0 + G * BM;                                                    // [G][128]: D / exchange
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::oBar);
+  // of a pair, the barriers that the MMA warp waits on (full, q_full, s_free, d_free) are rank 0's; commits arrive in both
   uint64_t* full = bars;                 // [NSLOT]
   uint64_t* empty = full + NSLOT;        // [NSLOT]
   uint64_t* q_full = empty + NSLOT;      // [2] resident Q, or the two stages
   uint64_t* q_empty = q_full + 2;        // [2]
   uint64_t* s_full = q_empty + 2;        // [2]
-  uint64_t* s_free = s_full + 2;         // [2]
+  uint64_t* s_free = s_full + 2;         // [2] the buffers, or (STASH) the first and the second half of the heads
   uint64_t* d_full = s_free + 2;
   uint64_t* d_free = d_full + 1;
   uint64_t* x_bar = d_free + 1;          // the element-wise warps meet (bounded, unlike a named barrier)
@@ -87,30 +111,43 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   volatile int* s_issued = s_abort + 1;
   volatile int* s_qissued = s_abort + 3;
   volatile int* s_redo = s_abort + 2;    // forward: a logit left the range of P around the row's reference
-  static_assert((2 * NSLOT + 12) * 8 + 16 <= 512, "barrier block");
+  volatile int* s_peer_redo = s_abort + 4;   // ... in the other CTA of the pair
+  static_assert((2 * NSLOT + 12) * 8 + 24 <= 512, "barrier block");
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int N = p.N, cq = CONV ? p.cq : 1, pq = cq - 1, pk = CONV ? (p.ck - 1) / 2 : 0;
   const int band = CONV && p.causal ? pq + pk : 0;
-  // row tiles from the last (most keys) on; the key chunks of a row tile side by side
-  const int kc = blockIdx.x % p.nKC, rt = p.nRT - 1 - blockIdx.x / p.nKC, ul = blockIdx.y;
+  const uint32_t rank = PAIR ? tc::cluster_rank() : 0u;
+  // row tiles (of a pair: two) from the last (most keys) on; the key chunks of a row tile side by side.  An odd row tile is
+  // left over at the front, where a causal mask leaves the fewest keys: rank 0 has no rows there (rt = -1)
+  const int bx = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
+  const int kc = bx % p.nKC, rt = p.nRT - CPG * (1 + bx / p.nKC) + (int)rank, ul = blockIdx.y;
   const int u = p.u0 + ul, HG = p.H / G, b = u / HG, grp = u - b * HG;
   const int bh0 = b * p.H + grp * G;                         // first head of the group
   const int R0 = rt * BM;
   const int k_lo = kc * p.kch;
-  const int k_hi = min(min(k_lo + p.kch, p.N8), p.causal ? R0 + BM : p.N8);     // multiples of 128
-  const int nblk = k_hi > k_lo ? (k_hi - k_lo) / KB : 0;
+  const int k_hi = min(min(k_lo + p.kch, p.N8), p.causal ? R0 + BM : p.N8);     // multiples of 128 (or a chunk of 64)
+  const int my_nblk = k_hi > k_lo && rt >= 0 ? (k_hi - k_lo) / KB : 0;          // blocks with keys of this CTA's rows
+  int nblk = my_nblk;                                                           // ... of the pair's
+  if constexpr (PAIR) {
+    const int kp = min(min(k_lo + p.kch, p.N8), p.causal ? R0 + (int)(2 - rank) * BM : p.N8);
+    nblk = kp > k_lo ? (kp - k_lo) / KB : 0;
+  }
 
   if (tid == 0) {
     for (int i = 0; i < NSLOT; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 1); }
-    tc::mbar_init(d_full, 1); tc::mbar_init(d_free, 8); tc::mbar_init(x_bar, 8); tc::mbar_init(mma_drain, 1);
-    for (int i = 0; i < 2; ++i) { tc::mbar_init(&q_full[i], 1); tc::mbar_init(&q_empty[i], 1); tc::mbar_init(&s_full[i], 1); tc::mbar_init(&s_free[i], 8); }
-    *s_abort = 0; *s_issued = 0; *s_redo = 0; *s_qissued = 0;
+    tc::mbar_init(d_full, 1); tc::mbar_init(d_free, 8 * CPG); tc::mbar_init(x_bar, 8); tc::mbar_init(mma_drain, 1);
+    for (int i = 0; i < 2; ++i) { tc::mbar_init(&q_full[i], 1); tc::mbar_init(&q_empty[i], 1); tc::mbar_init(&s_full[i], 1); tc::mbar_init(&s_free[i], 8 * CPG); }
+    *s_abort = 0; *s_issued = 0; *s_redo = 0; *s_qissued = 0; *s_peer_redo = 0;
     tc::mbar_fence_init();
   }
   if (warp == 9) {
-    tc::tmem_alloc(s_tmem, 512);
-    tc::tmem_relinquish();
+    if constexpr (PAIR) {
+      tc::tmem_alloc_pair(s_tmem, 512);
+    } else {
+      tc::tmem_alloc(s_tmem, 512);
+      tc::tmem_relinquish();
+    }
   }
   tc::tc_fence_before();
   pdl_wait();
@@ -124,25 +161,34 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   for (int i = tid; i < G * BM; i += Cfg::kThreads) {
     const int g = i / BM, r = R0 + i % BM;
     if (BWD) {
-      sR0[i] = r < N ? p.LSE[(size_t)(bh0 + g) * N + r] * kLog2e : 0.f;
-      sR1[i] = r < N ? p.Dvec[(size_t)(bh0 + g) * N + r] : 0.f;
+      sR0[i] = r >= 0 && r < N ? p.LSE[(size_t)(bh0 + g) * N + r] * kLog2e : 0.f;
+      sR1[i] = r >= 0 && r < N ? p.Dvec[(size_t)(bh0 + g) * N + r] : 0.f;
     } else {
       sR0[i] = -INFINITY;
     }
   }
-  __syncthreads();
+  if constexpr (PAIR) tc::cluster_sync_all(); else __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = *s_tmem;
   int ring = 0, ring_ph = 0, qring = 0, meets = 0;    // ring positions (warps 8 and 9) and meetings of the element-wise warps, over all attempts
+  bool ready = false;                                 // (warp 9) the ring's next slot was seen full
 
   // forward: a second attempt only when a logit exceeds its row's reference (the maximum of the first keys) by 2^100
   const int attempts = nblk > 0 ? (BWD ? 1 : 2) : 0;
-  auto attempt_done = [&]() -> bool {                        // every warp, after each attempt
+  auto attempt_done = [&]() -> bool {                        // every warp, after each attempt; the same in both CTAs of a pair
     __syncwarp();
     tc::tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) {
+      if (tid == 0) {
+        if (*s_abort) tc::st_cluster_u32(tc::cluster_addr((const void*)s_abort, rank ^ 1), 1);
+        if (!BWD && *s_redo) tc::st_cluster_u32(tc::cluster_addr((const void*)s_peer_redo, rank ^ 1), 1);
+      }
+      __syncwarp();
+      tc::cluster_sync_all();
+    }
     tc::tc_fence_after();
-    return BWD || !*s_redo || *s_abort;
+    return BWD || !(*s_redo || *s_peer_redo) || *s_abort;
   };
   if (warp >= 8) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::kRegsOther));
   if (warp == 8) {
@@ -153,36 +199,41 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       auto slot_of = [&](uint32_t bytes) -> int {            // waits for the slot, arms its barrier
         const int slot = ring % NSLOT, ph = (ring / NSLOT) & 1;
         if (!tc::mbar_wait(&empty[slot], ph ^ 1, s_abort)) { ok = false; return slot; }
-        tc::mbar_expect_tx(&full[slot], bytes);
+        if (rank == 0) tc::mbar_expect_tx(&full[slot], CPG * bytes);
         ++ring;
         *s_issued = ring;
         return slot;
       };
+      auto load = [&](unsigned char* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
+        if constexpr (PAIR) tc::tma_load_3d_pair(dst, map, tc::cluster_addr(bar, 0), x, y, z);
+        else tc::tma_load_3d(dst, map, bar, x, y, z);
+      };
       if (Cfg::RES && attempt == 0) {
-        tc::mbar_expect_tx(q_full, G * SL * Cfg::QR * 128);
-        for (int i = 0; i < G * SL; ++i) tc::tma_load_3d(sQ + i * (Cfg::QR * 128), &tmQ, q_full, (i % SL) * 64, R0 - HALO, bh0 + i / SL);
+        if (rank == 0) tc::mbar_expect_tx(q_full, CPG * (G * SL * Cfg::QR * 128));
+        for (int i = 0; i < G * SL; ++i) load(sQ + i * (Cfg::QR * 128), &tmQ, q_full, (i % SL) * 64, R0 - HALO, bh0 + i / SL);
       }
       // the B tiles of one head pair up in slots; A and B in the order the MMA warp takes them
       auto plain = [&](const CUtensorMap* ta, const CUtensorMap* tb, int key) {
         for (int i = 0; i < G * SL && ok; ++i) {
           if (i % TPP == 0) {
-            const int n = min(TPP, G * SL - i), s = slot_of(n * TB);
+            const int n = min(TPP, G * SL - i), s = slot_of(n * TBP);
             if (!ok) return;
-            for (int j = 0; j < n; ++j) tc::tma_load_3d(sRing + s * SLOT + j * TB, tb, &full[s], ((i + j) % SL) * 64, key, bh0 + (i + j) / SL);
+            for (int j = 0; j < n; ++j) load(sRing + s * SLOT + j * TBP, tb, &full[s], ((i + j) % SL) * 64, key, bh0 + (i + j) / SL);
           }
           const int s = slot_of(BM * 128);
           if (!ok) return;
-          tc::tma_load_3d(sRing + s * SLOT, ta, &full[s], (i % SL) * 64, R0, bh0 + i / SL);
+          load(sRing + s * SLOT, ta, &full[s], (i % SL) * 64, R0, bh0 + i / SL);
         }
       };
       auto stacked = [&](int key) {
-        const int nt = cq * 2 * SL;                          // (tap, hi / lo, slab) tiles of a head
-        for (int g = 0; g < G && ok; ++g) {
+        const int nt = cq * (HL ? 1 : 2) * SL;               // (tap, hi / lo, slab) tiles of a head; HL: of this CTA's part
+        for (int gi = 0; gi < G && ok; ++gi) {
+          const int g = HLB ? (gi + G / 2) % G : gi;         // in the order of the MMA warp
           if (!Cfg::RES) {
             const int st = qring & 1;
             if (!tc::mbar_wait(&q_empty[st], ((qring >> 1) & 1) ^ 1, s_abort)) { ok = false; return; }
-            tc::mbar_expect_tx(&q_full[st], Cfg::Q_HEAD);
-            for (int sl = 0; sl < SL; ++sl) tc::tma_load_3d(sQ + st * Cfg::Q_HEAD + sl * (Cfg::QR * 128), &tmQ, &q_full[st], sl * 64, R0 - HALO, bh0 + g);
+            if (rank == 0) tc::mbar_expect_tx(&q_full[st], CPG * Cfg::Q_HEAD);
+            for (int sl = 0; sl < SL; ++sl) load(sQ + st * Cfg::Q_HEAD + sl * (Cfg::QR * 128), &tmQ, &q_full[st], sl * 64, R0 - HALO, bh0 + g);
             ++qring;
             *s_qissued = qring;
           }
@@ -190,14 +241,20 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const int n = min(TPS, nt - i), s = slot_of(n * TB);
             if (!ok) return;
             for (int j = 0; j < n; ++j)
-              tc::tma_load_3d(sRing + s * SLOT + j * TB, &tmB, &full[s], ((i + j) % SL) * 64, key, (bh0 + g) * cq * 2 + (i + j) / SL);
+              load(sRing + s * SLOT + j * TB, &tmB, &full[s], ((i + j) % SL) * 64, key, (bh0 + g) * cq * 2 + (HL ? 2 * ((i + j) / SL) + (int)rank : (i + j) / SL));
           }
         }
       };
       for (int kb = 0; kb < nblk && ok; ++kb) {
-        const int key = k_lo + kb * KB;
-        if constexpr (CONV) stacked(key); else plain(&tmQ, &tmB, key);
+        const int key = k_lo + kb * KB + (int)rank * Cfg::KC;
+        if constexpr (CONV) stacked(HL ? k_lo + kb * KB : key); else plain(&tmQ, &tmB, key);
         if constexpr (BWD) { if (ok) plain(&tmdO, &tmV, key); }
+      }
+      // of a pair: the last arrivals on this CTA's `empty` barriers have landed before it leaves
+      if constexpr (PAIR) {
+        for (int id = max(0, ring - NSLOT); id < ring && ok; ++id) ok = tc::mbar_wait(&empty[id % NSLOT], (id / NSLOT) & 1, s_abort);
+        if (!Cfg::RES)
+          for (int id = max(0, qring - 2); id < qring && ok; ++id) ok = tc::mbar_wait(&q_empty[id & 1], (id >> 1) & 1, s_abort);
       }
     }
     if (attempt_done()) break;
@@ -205,38 +262,47 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   } else if (warp == 9) {
     // ===================== MMA issuer: all lanes run the loop; one elected lane issues =====================
     for (int attempt = 0; attempt < attempts; ++attempt) {
-    constexpr uint32_t idesc = tc::make_idesc(BM, KB, 0, 0);
+    if (rank == 0) {
+    constexpr uint32_t idesc = tc::make_idesc(CPG * BM, Cfg::SN, 0, 0), idescP = tc::make_idesc(CPG * BM, KB, 0, 0);
     const uint64_t d0 = tc::make_sdesc(smem_u32(sRing), 16, 1024, tc::kLayoutSW128);
     const uint32_t hi = (uint32_t)(d0 >> 32), lo0 = (uint32_t)d0;
     const uint32_t q_lo = (uint32_t)tc::make_sdesc(smem_u32(sQ), 16, 1024, tc::kLayoutSW128);
     bool ok = true;
+    // a wait that is over already costs 200 cycles, in which the tensor core runs dry: take() looks at the next slot before
+    // the MMAs of this one are issued, picked() takes the answer up behind them
+    uint32_t seen = 0;
     auto take = [&]() -> int {
       const int slot = ring;
-      if (!tc::mbar_wait_warp(&full[slot], ring_ph, s_abort)) { ok = false; return slot; }
+      if (!ready && !tc::mbar_wait_warp(&full[slot], ring_ph, s_abort)) { ok = false; return slot; }
       tc::tc_fence_after();
       if (++ring == NSLOT) { ring = 0; ring_ph ^= 1; }
+      seen = tc::mbar_test(&full[ring], ring_ph);
       return slot;
     };
-    auto mma4 = [&](uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t acc) {
-      tc::mma_ss2pe(d, a_lo, hi, b_lo, hi, idesc, acc);
-#pragma unroll
-      for (int k = 1; k < 4; ++k) tc::mma_ss2e<1>(d, a_lo + 2 * k, hi, b_lo + 2 * k, hi, idesc);
-    };
-    auto plain = [&](uint32_t dst) {
+    auto picked = [&]() { ready = __all_sync(0xffffffffu, seen); };
+    auto commit = [&](uint64_t* bar) { if constexpr (PAIR) tc::mma_commit_pair(bar); else tc::mma_commit_e(bar); };
+    auto wait = [&](uint64_t* bar, int parity) { ok = tc::mbar_wait_warp(bar, parity & 1, s_abort); tc::tc_fence_after(); };
+    auto plain = [&](uint32_t dst, int n) {                  // n: blocks of scores issued before (0 for dP)
       int bs = 0;
       for (int i = 0; i < G * SL && ok; ++i) {
-        if (i % TPP == 0) bs = take();
+        if (Cfg::STASH && i == G / 2 * SL && n > 0) { wait(&s_free[1], n - 1); if (!ok) return; }
+        if (i % TPP == 0) { bs = take(); picked(); }
         if (!ok) return;
         const int s = take();
         if (!ok) return;
-        mma4(dst + (i / SL) * KB, lo0 + (uint32_t)(s * (SLOT >> 4)), lo0 + (uint32_t)(bs * (SLOT >> 4) + (i % TPP) * (TB >> 4)), i % SL != 0);
-        tc::mma_commit_e(&empty[s]);
-        if (i % TPP == TPP - 1 || i == G * SL - 1) tc::mma_commit_e(&empty[bs]);
+        tc::mma4_ss<CPG>(dst + (i / SL) * KB, lo0 + (uint32_t)(s * (SLOT >> 4)), hi, 2,
+                         lo0 + (uint32_t)(bs * (SLOT >> 4) + (i % TPP) * (TBP >> 4)), hi, 2, idescP, i % SL != 0);
+        commit(&empty[s]);
+        if (i % TPP == TPP - 1 || i == G * SL - 1) commit(&empty[bs]);
+        picked();
       }
     };
-    auto stacked = [&](uint32_t dst) {
-      const int nt = cq * 2 * SL;
-      for (int g = 0; g < G && ok; ++g) {
+    auto stacked = [&](uint32_t dst, int n) {
+      const int nt = cq * (HL ? 1 : 2) * SL;
+      for (int gi = 0; gi < G && ok; ++gi) {
+        const int g = HLB ? (gi + G / 2) % G : gi;
+        // the second half of the heads to be written: their scores have been taken, or (HLB) dP has, which lies over them
+        if (Cfg::STASH && gi == G / 2 && n > 0) { wait(HLB ? d_free : &s_free[1], n - 1); if (!ok) return; }
         const int st = qring & 1;
         if (!Cfg::RES) {
           ok = tc::mbar_wait_warp(&q_full[st], (qring >> 1) & 1, s_abort);
@@ -251,29 +317,33 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
           for (int j = 0; j < TPS; ++j)
             if (i + j < nt) {
-              const int a = (i + j) / (2 * SL), sl = (i + j) % SL;
-              mma4(dst + g * KB, aq + (uint32_t)(sl * (Cfg::QR * 8) + a * 8), bl + (uint32_t)(j * (TB >> 4)), i + j != 0);
+              const int a = (i + j) / ((HL ? 1 : 2) * SL), sl = (i + j) % SL;
+              tc::mma4_ss<CPG>(dst + g * Cfg::SN, aq + (uint32_t)(sl * (Cfg::QR * 8) + a * 8), hi, 2, bl + (uint32_t)(j * (TB >> 4)), hi, 2,
+                               idesc, i + j != 0);
             }
-          tc::mma_commit_e(&empty[s]);
+          commit(&empty[s]);
+          picked();
         }
-        if (!Cfg::RES) tc::mma_commit_e(&q_empty[st]);
+        if (!Cfg::RES) commit(&q_empty[st]);
       }
     };
     if (Cfg::RES && attempt == 0) ok = tc::mbar_wait_warp(q_full, 0, s_abort);
     for (int kb = 0; kb < nblk && ok; ++kb) {
       const int it = attempt * nblk + kb;                    // uses of the buffers over both attempts
       const int bf = it % NBUF, ub = it / NBUF;
-      if (ub > 0) { ok = tc::mbar_wait_warp(&s_free[bf], (ub - 1) & 1, s_abort); tc::tc_fence_after(); }
+      if (ub > 0) wait(&s_free[HLB ? 1 : bf], ub - 1);
       if (!ok) break;
-      if constexpr (CONV) stacked(tmem + bf * (G * KB)); else plain(tmem + bf * (G * KB));
+      if constexpr (CONV) stacked(tmem + bf * (G * KB), it); else plain(tmem + bf * (G * KB), it);
       if (!ok) break;
-      tc::mma_commit_e(&s_full[bf]);
+      commit(&s_full[bf]);
       if constexpr (BWD) {
-        if (kb > 0) { ok = tc::mbar_wait_warp(d_free, (kb - 1) & 1, s_abort); tc::tc_fence_after(); }
+        if (HLB) wait(&s_free[0], kb);                       // dP goes over the scores of the first heads
+        else if (kb > 0) wait(d_free, kb - 1);
         if (!ok) break;
-        plain(tmem + 256);
-        if (ok) tc::mma_commit_e(d_full);
+        plain(tmem + Cfg::colP, 0);
+        if (ok) commit(d_full);
       }
+    }
     }
     if (attempt_done()) break;
     }
@@ -292,6 +362,17 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const size_t kc8 = p.N8 / 8;
     bool ok = true;
     constexpr int KP = KT / 2;
+    const uint32_t r_sfree = PAIR ? tc::cluster_addr(s_free, 0) : 0u, r_dfree = PAIR ? tc::cluster_addr(d_free, 0) : 0u;
+    auto free_s = [&](int bf) {                              // this warp has taken the scores of buffer bf
+      tc::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) { if constexpr (PAIR) tc::mbar_arrive_cluster(r_sfree + 8 * bf); else tc::mbar_arrive(&s_free[bf]); }
+    };
+    auto free_d = [&]() {
+      tc::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) { if constexpr (PAIR) tc::mbar_arrive_cluster(r_dfree); else tc::mbar_arrive(d_free); }
+    };
     auto meet = [&]() {                                      // false: a wait ran out somewhere
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(x_bar);
@@ -301,11 +382,22 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     };
     // S of this thread's keys of a pass, all heads, as key pairs; with a filter and a causal mask the entries of the band
     // come from the band kernel (the stacked product does not hold there)
-    auto load_s = [&](uint64_t (&s)[G][KP], uint32_t base, int j0) {
+    constexpr int SH = Cfg::SH;                              // heads whose scores were taken when the block began
+    constexpr bool ROT = SH > 0 && !HL;                      // st starts with this pass's; HL: the passes are unrolled
+    uint64_t st[SH > 0 ? NPASS * SH * KP : 1];
+    auto load_s = [&](uint64_t (&s)[G][KP], uint32_t base, int ps, int j0) {
       float v[G][KT];
 #pragma unroll
-      for (int g = 0; g < G; ++g) tmem_ld_nowait<KT>(base + g * KB, v[g]);
-      tc::tmem_wait_ld();
+      for (int g = SH; g < G; ++g) tmem_ld_nowait<KT>(base + g * KB + ps * KT, v[g]);
+#pragma unroll
+      for (int g = 0; g < SH; ++g)
+#pragma unroll
+        for (int k = 0; k < KP; ++k) f2_unpack(st[((ROT ? 0 : ps) * SH + g) * KP + k], v[g][2 * k], v[g][2 * k + 1]);
+      if constexpr (ROT) {
+#pragma unroll
+        for (int i = 0; i < (NPASS - 1) * SH * KP; ++i) st[i] = st[i + SH * KP];
+      }
+      if (SH < G) tc::tmem_wait_ld();
       if (CONV && band > 0 && gi < N && j0 + KT - 1 > gi - band && j0 <= gi) {
 #pragma unroll
         for (int g = 0; g < G; ++g) {
@@ -350,21 +442,35 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       uint32_t w[KP];
 #pragma unroll
       for (int k = 0; k < KP; ++k) w[k] = pack_bf16(v[2 * k], v[2 * k + 1]);
-      if constexpr (!CONV) {
-        store8(p.C8, lh, key, w);
-      } else {
-        auto put = [&](bf16* dst) {
-          if constexpr (KT == 8) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
-          else *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
-        };
-        bf16* dst = p.C8 + (lh * 2 * p.RP + gi) * p.N8 + key;
-        put(dst);
+      store8(p.C8, CONV ? 2 * lh : lh, key, w);
+      if constexpr (CONV) {
 #pragma unroll
         for (int k = 0; k < KP; ++k) w[k] = pack_bf16(v[2 * k] - __uint_as_float(w[k] << 16), v[2 * k + 1] - __uint_as_float(w[k] & 0xffff0000u));
-        put(dst + (size_t)p.RP * p.N8);
+        store8(p.C8, 2 * lh + 1, key, w);
       }
     };
 
+    auto take_all = [&]() {                                  // HL: the scores of a block, high + low
+      constexpr int NC = KB / 2 < 32 ? KB / 2 : 32;
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+#pragma unroll
+        for (int c = 0; c < KB / 2; c += NC) {
+          float hi[NC], lo[NC];
+          tmem_ld_nowait<NC>(tS0 + g * Cfg::SN + c, hi);
+          tmem_ld_nowait<NC>(tS0 + g * Cfg::SN + KB + c, lo);
+          tc::tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < NC; i += 2) {
+            const int k = c + i;
+            st[((k / KT) * G + g) * KP + (k % KT) / 2] = f2_pack(hi[i] + lo[i], hi[i + 1] + lo[i + 1]);
+          }
+        }
+        if (g == G / 2 - 1) free_s(0);
+      }
+      free_s(1);
+    };
+    constexpr int UN = HL ? NPASS : 1;                       // st is indexed by the pass
     if constexpr (!BWD) {
       float mt[G], l[G];
 #pragma unroll
@@ -372,11 +478,12 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // row maximum of this thread's valid keys of a block -> ref (both halves of a row agree on one value)
       auto init_ref = [&](uint32_t base, int j0) {
         const bool whole = k_lo + KB <= N && (!p.causal || j0 - hf * (KB / 2) + KB - 1 <= R0);   // every key valid for every row
-#pragma unroll 1
-        for (int ps = 0; ps < (whole ? 1 : NPASS); ++ps) {
+#pragma unroll UN
+        for (int ps = 0; ps < NPASS; ++ps) {
+          if (ps > 0 && whole) break;
           const int j = j0 + ps * KT;
           uint64_t s[G][KP];
-          load_s(s, base + ps * KT, j);
+          load_s(s, base, ps, j);
 #pragma unroll
           for (int g0 = 0; g0 < G; g0 += GC) {
             uint64_t acc[GC][KP];
@@ -411,22 +518,20 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const int it = attempt * nblk + kb, bf = it % NBUF;
         ok = __all_sync(0xffffffffu, tc::mbar_wait(&s_full[bf], (it / NBUF) & 1, s_abort));
         if (!ok) break;
+        if (PAIR && kb >= my_nblk) { free_s(0); free_s(1); continue; }   // keys of the other CTA's rows only
         tc::tc_fence_after();
+        if constexpr (HL) take_all();
         const uint32_t base = tS0 + bf * (G * KB);
         const int j0 = k_lo + kb * KB + hf * (KB / 2);
         // rows whose first valid key is not in block 0 exist only on the diagonal
         if (attempt == 0 && (kb == 0 || (p.causal && k_lo + kb * KB + KB - 1 > R0))) ok = init_ref(base, j0);
         if (!ok) break;
-#pragma unroll 1
+#pragma unroll UN
         for (int ps = 0; ps < NPASS; ++ps) {
           const int j = j0 + ps * KT;
           uint64_t s[G][KP];
-          load_s(s, base + ps * KT, j);
-          if (ps == NPASS - 1) {
-            tc::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&s_free[bf]);
-          }
+          load_s(s, base, ps, j);
+          if (!HL && ps == NPASS - 1) free_s(bf);
           const bool mask = !__all_sync(0xffffffffu, j + KT - 1 <= jlim);
 #pragma unroll
           for (int g0 = 0; g0 < G; g0 += GC) {
@@ -461,7 +566,7 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
         }
       }
-      if (ok) {
+      if (ok && my_nblk > 0) {
         const size_t ns = 2 * (size_t)p.nKC;
 #pragma unroll
         for (int g = 0; g < G; ++g) {
@@ -482,31 +587,54 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
     } else {
       // ---- backward ----
-      constexpr bool DWM = Cfg::DW_MMA;
+      constexpr bool DWM = Cfg::DW_MMA, DW2 = Cfg::STASH;      // dW in two partial sums (even and odd keys), for packed FMAs
       float dw[DWM ? 8 : G * G];
+      uint64_t dw2[DW2 ? G * G : 1];
 #pragma unroll
       for (int i = 0; i < (DWM ? 8 : G * G); ++i) dw[i] = 0.f;
+#pragma unroll
+      for (int i = 0; i < (DW2 ? G * G : 1); ++i) dw2[i] = 0ull;
       for (int kb = 0; kb < nblk; ++kb) {
-        ok = __all_sync(0xffffffffu, tc::mbar_wait(s_full, kb & 1, s_abort) && tc::mbar_wait(d_full, kb & 1, s_abort));
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(s_full, kb & 1, s_abort));
         if (!ok) break;
         tc::tc_fence_after();
+        const bool skip = PAIR && kb >= my_nblk;             // keys of the other CTA's rows only
+        if constexpr (HL) {
+          if (!skip) take_all();
+          else { free_s(0); free_s(1); }
+        } else if constexpr (SH > 0) {
+          if (!skip) {
+            float t[SH][KB / 2];
+#pragma unroll
+            for (int g = 0; g < SH; ++g)
+#pragma unroll
+              for (int c = 0; c < KB / 2; c += 32) tc::tmem_ld32_nowait(tS0 + g * KB + c, reinterpret_cast<float (&)[32]>(t[g][c]));
+            tc::tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < NPASS * SH * KP; ++i) {
+              const int c = (i / (SH * KP)) * KT + 2 * (i % KP);
+              st[i] = f2_pack(t[(i / KP) % SH][c], t[(i / KP) % SH][c + 1]);
+            }
+          }
+          free_s(0);
+        }
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(d_full, kb & 1, s_abort));
+        if (!ok) break;
+        if (skip) { if (!HL) free_s(SH > 0 ? 1 : 0); free_d(); continue; }
+        tc::tc_fence_after();
         const int j0 = k_lo + kb * KB + hf * (KB / 2);
-#pragma unroll 1
+#pragma unroll UN
         for (int ps = 0; ps < NPASS; ++ps) {
           const int j = j0 + ps * KT;
           uint64_t s[G][KP], dc[G][KP];
-          load_s(s, tS0 + ps * KT, j);
-          if (ps == NPASS - 1) {                             // the scores are in registers: the next block's MMAs may start
-            tc::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(s_free);
-          }
+          load_s(s, tS0, ps, j);
+          if (!HL && ps == NPASS - 1) free_s(SH > 0 ? 1 : 0);       // the scores are in registers: the next block's MMAs may start
           const bool mask = !__all_sync(0xffffffffu, j + KT - 1 <= jlim);
 #pragma unroll
           for (int g0 = 0; g0 < G; g0 += GC) {
             float dp[GC][KT];
 #pragma unroll
-            for (int c = 0; c < GC; ++c) tmem_ld_nowait<KT>(tS0 + 256 + (g0 + c) * KB + ps * KT, dp[c]);
+            for (int c = 0; c < GC; ++c) tmem_ld_nowait<KT>(tS0 + Cfg::colP + (g0 + c) * KB + ps * KT, dp[c]);
             uint64_t acc[GC][KP];
             mix(acc, s, sWf, g0);
             tc::tmem_wait_ld();
@@ -526,11 +654,7 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
               store8(p.P8, lh0 + g0 + c, j, w);
             }
           }
-          if (ps == NPASS - 1) {
-            tc::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(d_free);
-          }
+          if (ps == NPASS - 1) free_d();
           // ---- dC_x = sum_g W[g,x] dC'_g ----
 #pragma unroll
           for (int x0 = 0; x0 < G; x0 += GC) {
@@ -554,7 +678,14 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
           // ---- dW[g][x] += sum dC'_g S_x ----
           // masked entries have dC' = 0; S is finite there
-          if constexpr (!DWM) {
+          if constexpr (DW2) {
+#pragma unroll
+            for (int g = 0; g < G; ++g)
+#pragma unroll
+              for (int x = 0; x < G; ++x)
+#pragma unroll
+                for (int k = 0; k < KP; ++k) dw2[g * G + x] = f2_fma(dc[g][k], s[x][k], dw2[g * G + x]);
+          } else if constexpr (!DWM) {
 #pragma unroll
             for (int g = 0; g < G; ++g)
 #pragma unroll
@@ -621,6 +752,14 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
       }
       // ---- dW partial of the CTA ----
+      if constexpr (DW2) {
+#pragma unroll
+        for (int i = 0; i < G * G; ++i) {
+          float a, bb;
+          f2_unpack(dw2[i], a, bb);
+          dw[i] = a + bb;
+        }
+      }
       __syncwarp();
       float* red = reinterpret_cast<float*>(smem + Cfg::oDW) + warp * (G * G);
       if constexpr (DWM) {
@@ -637,13 +776,12 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
       }
       // the rows past the padded tile that a shifted dC operand of the last row tile reads
-      if (rt == p.nRT - 1 && ok) {
+      if (rt == p.nRT - 1 && ok) {                           // (nblk > 0 here)
         const int nch = (k_hi - k_lo) / 8;
         for (int i = tid; i < G * nch * 16; i += 256) {
           const int g = i / (nch * 16), rem = i - g * nch * 16;
           const int row = p.nRT * BM + (rem & 15), ch = rem >> 4;
-          bf16* dst = CONV ? p.C8 + ((lh0 + g) * 2 * p.RP + row) * p.N8 + k_lo + 8 * ch : p.C8 + (((lh0 + g) * kc8 + (k_lo >> 3) + ch) * p.RP + row) * 8;
-          *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(p.C8 + (((CONV ? 2 * (lh0 + g) : lh0 + g) * kc8 + (k_lo >> 3) + ch) * p.RP + row) * 8) = make_uint4(0u, 0u, 0u, 0u);
         }
       }
     }
@@ -652,12 +790,12 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
   __syncthreads();
 
-  if constexpr (BWD) {
+  if (BWD && rt >= 0) {
     const int slot = (b * p.nRT + rt) * p.nKC + kc;
     float* out = p.dW_part + ((size_t)slot * HG + grp) * (G * G);
     for (int i = tid; i < G * G; i += Cfg::kThreads) {
       float t = 0.f;
-      if (nblk > 0)
+      if (nblk > 0)                                          // (of a pair, with no key of this CTA's rows: zeros)
         for (int w = 0; w < 8; ++w) t += reinterpret_cast<const float*>(smem + Cfg::oDW + w * (Cfg::DW_MMA ? 4096 : G * G * 4))[i];
       out[i] = t * p.cw;
     }
@@ -665,39 +803,62 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (*s_abort) {
     if (tid == 0) atomicExch(p.status, 1);
     // nothing of this CTA may still be in flight when its shared and tensor memory are given up
-    if (warp == 9) tc::mma_commit_e(mma_drain);
-    if (tid == 256) {
+    if (warp == 9 && rank == 0) { if constexpr (PAIR) tc::mma_commit_pair(mma_drain); else tc::mma_commit_e(mma_drain); }
+    if (tid == 256 && rank == 0) {
       volatile int never = 0;
-      if (Cfg::RES && nblk > 0) tc::mbar_wait(q_full, 0, &never);
+      constexpr uint32_t kDrain = PAIR ? 1u << 14 : tc::kSpinLimit;      // of a pair, the other CTA may not have issued its share
+      if (Cfg::RES && nblk > 0) tc::mbar_wait(q_full, 0, &never, kDrain);
       const int issued = *s_issued, qi = *s_qissued;
-      for (int id = max(0, qi - 2); id < qi; ++id) tc::mbar_wait(&q_full[id & 1], (id >> 1) & 1, &never);
-      for (int id = max(0, issued - NSLOT); id < issued; ++id) tc::mbar_wait(&full[id % NSLOT], (id / NSLOT) & 1, &never);
+      for (int id = max(0, qi - 2); id < qi; ++id) tc::mbar_wait(&q_full[id & 1], (id >> 1) & 1, &never, kDrain);
+      for (int id = max(0, issued - NSLOT); id < issued; ++id) tc::mbar_wait(&full[id % NSLOT], (id / NSLOT) & 1, &never, kDrain);
     }
     if (tid == 256) { volatile int never = 0; tc::mbar_wait(mma_drain, 0, &never); }
-    __syncthreads();
+    if constexpr (PAIR) tc::cluster_sync_all(); else __syncthreads();
   }
+  if constexpr (PAIR) tc::cluster_sync_all();
   if (warp == 9) {
     tc::tc_fence_after();
-    tc::tmem_dealloc(tmem, 512);
+    if constexpr (PAIR) tc::tmem_dealloc_pair(tmem, 512); else tc::tmem_dealloc(tmem, 512);
   }
 }
 
 // ------------------------------------------------------------------------------------------
 namespace {
 
-template <int G, int D, bool CONV, bool BWD>
-cudaError_t launch_score_t(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, cudaStream_t stream) {
-  using Cfg = MixCfg<G, D, CONV, BWD>;
+template <int G, int D, bool CONV, bool BWD, int MODE>
+cudaError_t launch_score_m(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, cudaStream_t stream) {
+  using Cfg = MixCfg<G, D, CONV, BWD, MODE>;
   const size_t BH = (size_t)p.B * p.H;
   alignas(64) CUtensorMap tmQ, tmB, tmdO, tmV;
   if (!make_tensor_map_bf16(&tmQ, p.Q, D, p.N, BH, 64, CONV ? Cfg::QR : Cfg::BM, true)) return cudaErrorInvalidValue;
-  if (!make_tensor_map_bf16(&tmB, CONV ? Kt : p.K, D, p.N, CONV ? BH * p.cq * 2 : BH, 64, Cfg::KB, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmB, CONV ? Kt : p.K, D, p.N, CONV ? BH * p.cq * 2 : BH, 64, Cfg::HL ? Cfg::KB : Cfg::KC, true)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmdO, BWD ? p.dO : p.Q, D, p.N, BH, 64, Cfg::BM, true)) return cudaErrorInvalidValue;
-  if (!make_tensor_map_bf16(&tmV, p.V, D, p.N, BH, 64, Cfg::KB, true)) return cudaErrorInvalidValue;
-  auto kern = mix_score_kernel<G, D, CONV, BWD>;
+  if (!make_tensor_map_bf16(&tmV, p.V, D, p.N, BH, 64, Cfg::KC, true)) return cudaErrorInvalidValue;
+  auto kern = mix_score_kernel<G, D, CONV, BWD, MODE>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
-  return launch_pdl(kern, dim3(mp.nRT * mp.nKC, mp.nU), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmQ, tmB, tmdO, tmV, mp);
+  const int rows = MODE > 0 ? (mp.nRT + 1) / 2 * 2 : mp.nRT;
+  return launch_pdl(kern, dim3(rows * mp.nKC, mp.nU), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmQ, tmB, tmdO, tmV, mp);
+}
+
+template <int G, int D, bool CONV, bool BWD>
+cudaError_t launch_score_t(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, cudaStream_t stream) {
+  if constexpr (CONV && G <= 8) {
+    // Pairs from two waves of CTAs on (those above the diagonal not counted); below, they double the grain of the work:
+    // N 1001, 8 heads in groups of 4, d = 64 (144 CTAs): forward 82 us with single CTAs, 93 with pairs
+    const long live = (long)mp.nRT * mp.nKC * mp.nU / (p.causal ? 2 : 1);
+    if (live >= 2 * kSMs) {
+      // (hi, lo) together where the MMAs are the bound, from five slab tiles per head on: N 4096, d = 64, groups of 8, theta
+      // (5,9): forward 1088 -> 985 us; groups of 4, theta (3,5): 575 us, 607 with them together, as taking all scores is work of
+      // its own.  Groups of 2 are bound by the tensor core either way; the backward of 8 has no registers left for the scores.
+      constexpr bool has_hl = BWD ? G == 4 : G >= 4;
+      if constexpr (has_hl) {
+        if (p.cq * (D / 64) >= 5) return launch_score_m<G, D, CONV, BWD, 2>(p, mp, Kt, stream);
+      }
+      return launch_score_m<G, D, CONV, BWD, 1>(p, mp, Kt, stream);
+    }
+  }
+  return launch_score_m<G, D, CONV, BWD, 0>(p, mp, Kt, stream);
 }
 
 template <int G, int D>

@@ -13,8 +13,9 @@
 // Operand tensors P / dC: "X8" = [head][key chunk of 8][row][8 keys], rows padded to X8 rows = roundup(N, 128) + 16.  A thread
 // of the score kernel owns a row, so its 16-byte stores of 8 keys are contiguous across a warp; and every consumer gets an
 // MMA operand with one tiled copy of 128-byte pieces: no-swizzle core matrices, K-major for O = P V and dQ (a row shift is
-// 16 bytes), MN-major for dV = P^T dO and dKt = dC^T Q.  With a filter dC is row-major instead: dQ reads it at c_q row shifts,
-// which move whole rows of a swizzled tile.  And it is a (hi, lo) pair there: dTheta is a sum of dC S over every score entry
+// 16 bytes), MN-major for dV = P^T dO and dKt = dC^T Q.  (dC as rows of N keys, for dQ's row shifts, made each of those stores
+// 32 half sectors: 16.5 -> 13.5 ms of score kernel at B 2, H 32, N 8192, d = 128 in groups of 4; dQ does not mind.)  With a
+// filter dC is a (hi, lo) pair: dTheta is a sum of dC S over every score entry
 // whose terms cancel, and one bf16 rounding of dC costs it five times its error (3.2e-4 of it with 32-bit dC, 1.6e-3 with hi
 // alone, 3.2e-4 with the pair; N 1001 to 2048).  dKt takes both, dQ, which is rounded at the same size anyway, hi.
 #pragma once
@@ -35,7 +36,7 @@ struct MixParams {
   const float* Cband;     // causal with a filter: [B*H, N, band] scores of the band after the filter, natural units (else nullptr)
   float* dCband;          // backward: the gradient of those
   bf16* P8;               // [heads of the launch][N8 / 8][RP][8]
-  bf16* C8;               // backward: dC, the same; with a filter row-major, [heads of the launch][hi, lo][RP][N8]
+  bf16* C8;               // backward: dC, the same; with a filter [heads of the launch][hi, lo] of it
   float* stat;            // forward: [heads of the launch][2 nKC][3][RP]: row max, reference, sum, per key chunk and half
   float* dW_part;         // backward: [slots][H/G][G*G], slot = (b * nRT + row tile) * nKC + key chunk
   int* status;
@@ -52,6 +53,15 @@ template <int NC>
 FMTA_DEVINL void tmem_ld_nowait(uint32_t taddr, float* v) {
   if constexpr (NC == 4) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(taddr) : "memory");
+  } else if constexpr (NC == 32) {
+    tc::tmem_ld32_nowait(taddr, *reinterpret_cast<float (*)[32]>(v));
+  } else if constexpr (NC == 16) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
+          "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+        : "r"(taddr)
+        : "memory");
   } else {
     static_assert(NC == 8, "");
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"

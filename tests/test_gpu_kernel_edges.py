@@ -166,6 +166,19 @@ def test_mixing_tiles_and_groups_on_the_tensor_cores(request, B, H, N, d, G, cq,
     test_mixing_tiles_and_groups(B, H, N, d, G, cq, ck, causal, spread)
 
 
+@pytest.mark.parametrize("B,H,N,d,G,cq,ck,causal", [
+    (33, 4, 300, 64, 4, 5, 5, False),      # (hi, lo) keys in one product; three row tiles: a pair with a tile of no rows
+    (5, 32, 385, 64, 4, 6, 11, True),      # the same behind a causal mask; one row past the third tile
+    (66, 4, 260, 64, 4, 3, 5, True),       # pairs with few taps: high and low keys one after the other
+    (33, 2, 300, 128, 2, 3, 3, False),
+    (33, 8, 290, 64, 8, 5, 3, False),      # groups of 8: (hi, lo) together in the forward only
+])
+@pytest.mark.parametrize("spread", [1.0, 12.0])
+def test_mixing_behind_a_filter_on_cta_pairs(B, H, N, d, G, cq, ck, causal, spread):
+    """Two waves of CTAs and more: the score kernel works on pairs of row tiles."""
+    test_mixing_tiles_and_groups(B, H, N, d, G, cq, ck, causal, spread)
+
+
 @pytest.mark.parametrize("B,H,N,G,causal", [(1, 16, 1600, 16, True), (1, 16, 2048, 16, True), (2, 16, 1500, 16, True), (1, 8, 2100, 8, True)])
 def test_mixing_stays_in_its_workspace(B, H, N, G, causal):
     """Sizes whose key chunks depend on whether there is a filter: exactly the bytes that the library names, and what lies
