@@ -8,16 +8,18 @@
 //
 //   bwd_dkdv_tc128_kernel : CTA = 64 keys, loops 128-row query blocks.  The accumulators are kept TRANSPOSED, with the head
 //                           dim on the lanes: dV^T[d, key] += dO^T P and dKt_a^T[d, key] += Q^(a)T dC are
-//                           M = 128 MMAs whose A operand is the staged dO / Q tile read MN-major (for Q
-//                           with the tap's row shift as a start-address offset of 128 bytes per row into
-//                           the 128-byte-swizzled tile) and whose B operand is the
-//                           bf16 P / dC tile exactly as the element-wise warps write it (one row per
-//                           thread).  dV^T + 6 dKt^T take 448 columns; S and dP share the last 64
+//                           M = 128 MMAs whose A operand is the staged dO / Q tile read MN-major and whose B
+//                           operand is the bf16 P / dC tile as the element-wise warps write it (one row per
+//                           thread), dC with the tap's row shift as a start-address offset of 128 bytes per row
+//                           into a 128-byte-swizzled tile: three taps are one MMA of 192 columns (blocks walked
+//                           from the last one down; with the shift on Q, 64 columns each: 9.4 ms, now 7.9, at
+//                           B 8, H 32, N 4096).  dV^T + 6 dKt^T take 448 columns; S and dP share the last 64
 //                           (S(0) dP(0) | S(1) dP(1) | ...).  Scores and dP are computed once per entry.
 //   Four of the stacked key tiles stay resident; the others and V come again for every block through a ring of three 8 KB
 //   slabs, interleaved with the resident ones.  That is 48 KB per 128 x 64 block more from L2, and makes room for a second
 //   Q tile, so that S of the next block runs under the dKt MMAs of this one: with everything resident and one Q tile the
-//   block's load, S, element-wise part and dKt were one chain (tensor core 35 % busy, B 8, H 32, N 4096: 10.4 ms; now 9.4).
+//   block's load, S, element-wise part and dKt were one chain (tensor core 35 % busy, B 8, H 32, N 4096: 10.4 ms, then 9.4).
+//   Bound by the shared-memory port: S (M = 128, N = 64) reads 6 KB for 32 cycles of arithmetic.
 // Every mbarrier wait is bounded; no TMA multicast, no cluster, cta_group::1 only.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -48,10 +50,10 @@ struct Dkv128Cfg {
   static constexpr int oQ = oSt + NST * SLAB_BYTES;             // two buffers of two slabs
   static constexpr int odO = oQ + 4 * Q_SLAB;                   // two slabs
   static constexpr int oP = odO + 2 * DO_SLAB;                  // P  : [BK/8][BR][16 B]  (MN-major B operand)
-  static constexpr int oDC = oP + (BK / 8) * BR * 16;           // dC : same layout
-  static constexpr int oBar = oDC + (BK / 8) * BR * 16;
+  static constexpr int oDC = oP + (BK / 8) * BR * 16;           // dC : [136 rows][128 B], 128-byte swizzle
+  static constexpr int oBar = oDC + QR * 128;
   static constexpr int kSmemBytes = oBar + 512 + 1024;
-  static_assert(odO % 1024 == 0 && oSt % 1024 == 0 && oQ % 1024 == 0 && Q_SLAB % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
+  static_assert(odO % 1024 == 0 && oDC % 1024 == 0 && oSt % 1024 == 0 && oQ % 1024 == 0 && Q_SLAB % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
   static_assert(kSmemBytes <= 227 * 1024, "dK/dV kernel (d = 128): shared memory budget");
   static constexpr int kTmemCols = 512;        // dV^T at 0, dKt_a^T at 64 (1 + a), scratch X (S / dP) at 448
   static constexpr int colX = 448;
@@ -105,7 +107,10 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   j0 += p.key_base;
   const int bh = b * p.H + h;
   const int nQB = (N + BR - 1) / BR;
-  const int qb_begin = p.causal ? min(nQB, (j0 + band) / BR) : 0;
+  // The blocks are walked from the last one down, as a block's dKt^T takes the first pad_q rows of dC of the block behind it.
+  // No block in front of the last one walked misses its own: the first pad_q rows there are not owned (j0 + band is the first
+  // owned row), or there is nothing in front of it.
+  const int qb_begin = p.causal ? min(nQB, (j0 + pk) / BR) : 0;
   const int nblk = nQB - qb_begin;
 
   if (tid == 0) {
@@ -142,7 +147,7 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       auto load_q = [&](int it) {
         uint64_t* bar = &q_full[it & 1];
         unsigned char* dst = sQ + (it & 1) * (2 * Cfg::Q_SLAB);
-        const int i0 = (qb_begin + it) * BR;
+        const int i0 = (nQB - 1 - it) * BR;
         tc::mbar_expect_tx(bar, QR * D * 2);
         tc::tma_load_3d(dst, &tmQ, bar, 0, i0 - HALO, bh);
         tc::tma_load_3d(dst + Cfg::Q_SLAB, &tmQ, bar, 64, i0 - HALO, bh);
@@ -155,7 +160,7 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         tc::tma_load_3d(sKt + a * Cfg::KT_BYTES + Cfg::SLAB_BYTES, &tmKt, kt_full, 64, j0, bh * cq + a);
       }
       for (int it = 0; it < nblk; ++it) {
-        const int i0 = (qb_begin + it) * BR;
+        const int i0 = (nQB - 1 - it) * BR;
         if (it > 0 && !tc::mbar_wait(do_free, (it - 1) & 1, s_abort)) break;                     // dP and dV of block it-1
         tc::mbar_expect_tx(do_full, 2 * Cfg::DO_SLAB);
         tc::tma_load_3d(sdO, &tmdO, do_full, 0, i0, bh);
@@ -243,27 +248,28 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
     }
   } else if (role > 0) {
-    // ===================== MMA issuers A0 / A1: dV^T += dO^T P ; dKt_a^T += Q^(a)T dC =====================
+    // ===================== MMA issuers A0 / A1: dV^T += dO^T P ; dKt_a^T += Q^T dC^(a) =====================
+    // The tap's row shift is on dC, whose rows are the contraction: dKt_a[j] = sum_i q_i dC[i + s, j], s = pad_q - a.  Three taps
+    // then share their A operand: three 64-key atoms of B that start one row (128 bytes) apart are one MMA of 192 columns.
+    // With the shift on Q each tap was an MMA of its own, whose 4 KB of Q take as long to read as 64 columns to multiply.
     const int ai = role - 1;
     if (nblk > 0) {   // all lanes run the loop; one elected lane issues
       constexpr uint32_t idescA = tc::make_idesc(D, BK, 1, 1);     // 128 (head dim) x 64 (keys), both operands MN-major
-      // A0 takes dV^T and the first half of the taps, A1 the rest
-      const int ntap = p.ntap, accb = p.with_dv ? 1 : 0;
-      const int t_half = ntap / 2;
-      const int t_begin = ai == 0 ? 0 : t_half, t_end = ai == 0 ? t_half : ntap;
+      // A0 takes dV^T and the first half of the shifts, A1 the rest (c_q <= 6: at most three)
+      const int accb = p.with_dv ? 1 : 0;
+      const int s_begin = ai == 0 ? 0 : cq / 2, ns = ai == 0 ? cq / 2 : cq - cq / 2;
+      const uint32_t idescK = tc::make_idesc(D, BK * ns, 1, 1);
       // dO read MN-major (M = head dim across the two slabs, K = rows): 16 rows = 2048 bytes per step
       const uint64_t dOm = tc::make_sdesc(smem_u32(sdO), Cfg::DO_SLAB, 1024, tc::kLayoutSW128);
-      // Q read MN-major (M = head dim across the two slabs, K = rows, shifted by the tap through the start address)
-      const uint64_t dQm = tc::make_sdesc(smem_u32(sQ) + (HALO - pq) * 128, Cfg::Q_SLAB, 1024, tc::kLayoutSW128);
-      // P / dC: N = keys in 8-key chunks BR * 16 bytes apart, K = rows 16 bytes apart
+      // Q read MN-major (M = head dim across the two slabs, K = rows)
+      const uint64_t dQm = tc::make_sdesc(smem_u32(sQ) + HALO * 128, Cfg::Q_SLAB, 1024, tc::kLayoutSW128);
+      // dC: N = 64 keys per shift, one row apart, K = rows
+      const uint64_t dCb = tc::make_sdesc(smem_u32(smem + Cfg::oDC) + s_begin * 128, 128, 1024, tc::kLayoutSW128);
+      // P: N = keys in 8-key chunks BR * 16 bytes apart, K = rows 16 bytes apart
       const uint64_t dPb = tc::make_sdesc(smem_u32(smem + Cfg::oP), 128, BR * 16, tc::kLayoutNone);
       const uint32_t om_hi = (uint32_t)(dOm >> 32), om_lo = (uint32_t)dOm;
       const uint32_t qm_hi = (uint32_t)(dQm >> 32), qm_lo0 = (uint32_t)dQm;
-      const uint32_t pb_hi = (uint32_t)(dPb >> 32), pb_lo = (uint32_t)dPb, cb_lo = pb_lo + (uint32_t)((Cfg::oDC - Cfg::oP) >> 4);
-      auto mma8 = [&](uint32_t dst, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t acc) {       // 128 rows
-        tc::mma4_ss(dst, a_lo, a_hi, 2048 / 16, b_lo, pb_hi, 16, idescA, acc);
-        tc::mma4_ss(dst, a_lo + 4 * (2048 / 16), a_hi, 2048 / 16, b_lo + 4 * 16, pb_hi, 16, idescA, 1);
-      };
+      const uint32_t pb_hi = (uint32_t)(dPb >> 32), pb_lo = (uint32_t)dPb, cb_hi = (uint32_t)(dCb >> 32), cb_lo = (uint32_t)dCb;
       bool ok = true;
       for (int it = 0; it < nblk && ok; ++it) {
         const uint32_t acc_on = it != 0;
@@ -271,7 +277,10 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           ok = tc::mbar_wait_warp(do_full, it & 1, s_abort) && tc::mbar_wait_warp(p_full, it & 1, s_abort);
           if (!ok) break;
           tc::tc_fence_after();
-          if (p.with_dv) mma8(tmem, om_lo, om_hi, pb_lo, acc_on);
+          if (p.with_dv) {
+            tc::mma4_ss(tmem, om_lo, om_hi, 2048 / 16, pb_lo, pb_hi, 16, idescA, acc_on);
+            tc::mma4_ss(tmem, om_lo + 4 * (2048 / 16), om_hi, 2048 / 16, pb_lo + 4 * 16, pb_hi, 16, idescA, 1);
+          }
           tc::mma_commit_e(do_free);
           tc::mma_commit_e(p_free);
         }
@@ -282,8 +291,11 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         // A1's taps go behind S of the next block, which would otherwise share the tensor core with all of them from its
         // first MMA on and end with nothing left to run while it is taken out of X
         if (ai == 1 && it + 1 < nblk && !tc::mbar_wait_warp(s_full, (it + 1) & 1, s_abort)) { ok = false; break; }
-        for (int i = t_begin; i < t_end; ++i)
-          mma8(tmem + 64 * (accb + i), qm_lo + (uint32_t)(i * (128 >> 4)), qm_hi, cb_lo, acc_on);        // K (row) shift = +128 B per row
+        if (ns > 0) {
+          const uint32_t dst = tmem + 64 * (accb + s_begin);
+          tc::mma4_ss(dst, qm_lo, qm_hi, 2048 / 16, cb_lo, cb_hi, 2048 / 16, idescK, acc_on);
+          tc::mma4_ss(dst, qm_lo + 4 * (2048 / 16), qm_hi, 2048 / 16, cb_lo + 4 * (2048 / 16), cb_hi, 2048 / 16, idescK, 1);
+        }
         tc::mma_commit_e(&q_free[it & 1]);
         tc::mma_commit_e(dc_free);
       }
@@ -299,17 +311,20 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     bool ok = true;
     // every thread fetches the statistics of its own row (LSE in log2 units, D), one block ahead
     float lse2 = 0.f, dvec = 0.f;
+    uint32_t above[CW / 2];                             // dC of this row of the block before, which lies behind this one
+#pragma unroll
+    for (int c = 0; c < CW / 2; ++c) above[c] = 0u;
     if (nblk > 0) {
-      const int gi = qb_begin * BR + row;
+      const int gi = (nQB - 1) * BR + row;
       if (gi < N) { lse2 = p.LSE[(size_t)bh * N + gi] * kLog2e; dvec = p.Dvec[(size_t)bh * N + gi]; }
     }
     for (int it = 0; it < nblk && ok; ++it) {
-      const int i0 = (qb_begin + it) * BR;
+      const int i0 = (nQB - 1 - it) * BR;
       const int gi = i0 + row;
       float lse2_next = 0.f, dvec_next = 0.f;
-      if (it + 1 < nblk && gi + BR < N) {
-        lse2_next = p.LSE[(size_t)bh * N + gi + BR] * kLog2e;
-        dvec_next = p.Dvec[(size_t)bh * N + gi + BR];
+      if (it + 1 < nblk) {                              // (every row of a block but the last is a row of the sequence)
+        lse2_next = p.LSE[(size_t)bh * N + gi - BR] * kLog2e;
+        dvec_next = p.Dvec[(size_t)bh * N + gi - BR];
       }
       ok = __all_sync(0xffffffffu, (p.selftest_expire && it == 0) ? tc::mbar_wait(never_bar, 0, s_abort, tc::kSelfTestSpinLimit)
                                                                   : tc::mbar_wait(s_full, it & 1, s_abort));
@@ -337,7 +352,7 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (!ok) break;
       }
       unsigned char* pt = smem + Cfg::oP + row * 16;
-      unsigned char* dc = smem + Cfg::oDC + row * 16;
+      unsigned char* dc = smem + Cfg::oDC + row * 128;
 #pragma unroll
       for (int q4 = 0; q4 < CW / 8; ++q4)            // 8 keys (16 bytes) per chunk
         *reinterpret_cast<uint4*>(pt + ((CW / 8) * cg + q4) * (BR * 16)) = make_uint4(pp[4 * q4], pp[4 * q4 + 1], pp[4 * q4 + 2], pp[4 * q4 + 3]);
@@ -358,7 +373,15 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
 #pragma unroll
       for (int q4 = 0; q4 < CW / 8; ++q4)
-        *reinterpret_cast<uint4*>(dc + ((CW / 8) * cg + q4) * (BR * 16)) = make_uint4(pp[4 * q4], pp[4 * q4 + 1], pp[4 * q4 + 2], pp[4 * q4 + 3]);
+        *reinterpret_cast<uint4*>(dc + ((((CW / 8) * cg + q4) ^ (row & 7)) << 4)) = make_uint4(pp[4 * q4], pp[4 * q4 + 1], pp[4 * q4 + 2], pp[4 * q4 + 3]);
+      if (row < HALO) {
+#pragma unroll
+        for (int q4 = 0; q4 < CW / 8; ++q4)
+          *reinterpret_cast<uint4*>(dc + BR * 128 + ((((CW / 8) * cg + q4) ^ (row & 7)) << 4)) =
+              make_uint4(above[4 * q4], above[4 * q4 + 1], above[4 * q4 + 2], above[4 * q4 + 3]);
+      }
+#pragma unroll
+      for (int c = 0; c < CW / 2; ++c) above[c] = pp[c];
       tc::fence_proxy_async_smem();
       tc::mbar_arrive(dc_full);
       lse2 = lse2_next; dvec = dvec_next;
@@ -399,7 +422,7 @@ bwd_dkdv_tc128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
       } else {
         // dKt_a leaves as bf16 [key][d]: neighbouring lanes pair up so that every lane stores one 4-byte word
-        const int tap = acc - (p.with_dv ? 1 : 0);
+        const int tap = cq - 1 - (acc - (p.with_dv ? 1 : 0));      // accumulators in the order of the shifts
         bf16* dst = p.dKt + (((size_t)bh * cq + tap) * N + key0) * D + (dcol & ~1);
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {

@@ -107,6 +107,16 @@ def test_training_tiles_and_taps(B, H, N, d, cq, ck, causal, fp32_inputs):
                   "edges B%d H%d N%d d%d theta(%d,%d) causal=%d fp32=%d" % (B, H, N, d, cq, ck, causal, fp32_inputs))
 
 
+@pytest.mark.parametrize("B,H,N,d,cq,ck,causal", [
+    (1, 2, 389, 128, 6, 3, False),         # every block's first rows feed the block in front; five rows past the third
+    (1, 1, 261, 128, 2, 5, False),         # one shift per issuer
+    (2, 1, 321, 128, 5, 1, True),          # no key padding: the mask is as near to the block's end as it gets
+    (1, 1, 131, 128, 6, 11, False),        # three rows behind a block's end, fewer than the shifts reach
+])
+def test_row_shifts_across_query_blocks(B, H, N, d, cq, ck, causal):
+    test_training_tiles_and_taps(B, H, N, d, cq, ck, causal, True)
+
+
 @pytest.mark.parametrize("B,H,N,d,G,cq,ck,causal", [
     (1, 4, 127, 64, 2, 3, 5, True),        # groups of 2; one key short of a block
     (1, 4, 130, 128, 4, 6, 11, True),      # two keys past one
