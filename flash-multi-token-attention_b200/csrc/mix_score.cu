@@ -77,6 +77,13 @@ struct MixCfg {
   static_assert(SLOT % 1024 == 0 && TB % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
 };
 
+// Key chunks with keys of row tile `top` or before (kch is a power of two).  Only these get a CTA: one without keys kept its SM for
+// 5 us of setting up, and at B 2, H 8, N 1001 (groups of 4) 112 of 256 were such: the last of the others began 11 us late.
+__host__ __device__ inline int score_chunks(const MixParams& p, int top) {
+  const int n = p.causal ? ((top + 1) * 128 + p.kch - 1) / p.kch : p.nKC;
+  return n < p.nKC ? n : p.nKC;
+}
+
 template <int G, int D, bool CONV, bool BWD, int MODE>
 __global__ void __cluster_dims__(MODE > 0 ? 2 : 1, 1, 1) __launch_bounds__(384, 1)
 mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmB,
@@ -120,8 +127,9 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const uint32_t rank = PAIR ? tc::cluster_rank() : 0u;
   // row tiles (of a pair: two) from the last (most keys) on; the key chunks of a row tile side by side.  An odd row tile is
   // left over at the front, where a causal mask leaves the fewest keys: rank 0 has no rows there (rt = -1)
-  const int bx = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
-  const int kc = bx % p.nKC, rt = p.nRT - CPG * (1 + bx / p.nKC) + (int)rank, ul = blockIdx.y;
+  int top = p.nRT - 1, kc = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, nkc = score_chunks(p, top);
+  while (kc >= nkc) { kc -= nkc; top -= CPG; nkc = score_chunks(p, top); }
+  const int rt = top - (CPG - 1) + (int)rank, ul = blockIdx.y;
   const int u = p.u0 + ul, HG = p.H / G, b = u / HG, grp = u - b * HG;
   const int bh0 = b * p.H + grp * G;                         // first head of the group
   const int R0 = rt * BM;
@@ -399,14 +407,23 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
       if (SH < G) tc::tmem_wait_ld();
       if (CONV && band > 0 && gi < N && j0 + KT - 1 > gi - band && j0 <= gi) {
+        // loads without a branch for each, several heads at a time: one after the other their latencies were half of the time of
+        // the blocks on the diagonal (backward, groups of 4: 24 us against 13 off it), and small problems end with such a block
+        constexpr int GB = G < 4 ? G : 4;
 #pragma unroll
-        for (int g = 0; g < G; ++g) {
-          const float* cb = p.Cband + ((size_t)(bh0 + g) * N + gi) * band;
+        for (int g0 = 0; g0 < G; g0 += GB) {
+          float t[GB][KT];
 #pragma unroll
-          for (int k = 0; k < KT; ++k) {
-            const int e = gi - (j0 + k);
-            if (e >= 0 && e < band) v[g][k] = cb[e] * kLog2e;
-          }
+          for (int g = 0; g < GB; ++g)
+#pragma unroll
+            for (int k = 0; k < KT; ++k) t[g][k] = __ldg(p.Cband + ((size_t)(bh0 + g0 + g) * N + gi) * band + min(max(gi - (j0 + k), 0), band - 1));
+#pragma unroll
+          for (int g = 0; g < GB; ++g)
+#pragma unroll
+            for (int k = 0; k < KT; ++k) {
+              const int e = gi - (j0 + k);
+              v[g0 + g][k] = e >= 0 && e < band ? t[g][k] * kLog2e : v[g0 + g][k];
+            }
         }
       }
 #pragma unroll
@@ -793,6 +810,9 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (BWD && rt >= 0) {
     const int slot = (b * p.nRT + rt) * p.nKC + kc;
     float* out = p.dW_part + ((size_t)slot * HG + grp) * (G * G);
+    if (kc == nkc - 1)                                       // the slots of the chunks that no CTA has
+      for (int i = tid; i < (p.nKC - nkc) * G * G; i += Cfg::kThreads)
+        p.dW_part[((size_t)(slot + 1 + i / (G * G)) * HG + grp) * (G * G) + i % (G * G)] = 0.f;
     for (int i = tid; i < G * G; i += Cfg::kThreads) {
       float t = 0.f;
       if (nblk > 0)                                          // (of a pair, with no key of this CTA's rows: zeros)
@@ -837,8 +857,9 @@ cudaError_t launch_score_m(const TrainParams& p, const MixParams& mp, const __nv
   auto kern = mix_score_kernel<G, D, CONV, BWD, MODE>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
-  const int rows = MODE > 0 ? (mp.nRT + 1) / 2 * 2 : mp.nRT;
-  return launch_pdl(kern, dim3(rows * mp.nKC, mp.nU), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmQ, tmB, tmdO, tmV, mp);
+  int ctas = 0;
+  for (int top = mp.nRT - 1; top >= 0; top -= MODE > 0 ? 2 : 1) ctas += (MODE > 0 ? 2 : 1) * score_chunks(mp, top);
+  return launch_pdl(kern, dim3(ctas, mp.nU), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmQ, tmB, tmdO, tmV, mp);
 }
 
 template <int G, int D, bool CONV, bool BWD>
