@@ -85,20 +85,16 @@ mix_pv_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ C
     const uint64_t dA = tc::make_sdesc(smem_u32(smem), BM * 16, 128, tc::kLayoutNone);
     const uint64_t dB = tc::make_sdesc(smem_u32(smem) + Cfg::P_BYTES, SL > 1 ? Cfg::V_SLAB : 16, 1024, tc::kLayoutSW128);
     const uint32_t a_hi = (uint32_t)(dA >> 32), a0 = (uint32_t)dA, b_hi = (uint32_t)(dB >> 32), b0 = (uint32_t)dB;
+    tc::TileRing<NSTG, 1> ring(full, empty, s_abort);
     bool ok = true;
     for (int ch = 0; ch < nch && ok; ++ch) {
       const int bf = ch & 1;
       if (ch > 1) { ok = tc::mbar_wait_warp(&o_free[bf], ((ch >> 1) - 1) & 1, s_abort); tc::tc_fence_after(); }
       for (int kb = ch * bpc; kb < min(nblk, (ch + 1) * bpc) && ok; ++kb) {
-        const int st = kb % NSTG, ph = (kb / NSTG) & 1;
-        ok = tc::mbar_wait_warp(&full[st], ph, s_abort);
-        if (!ok) break;
-        tc::tc_fence_after();
-        const uint32_t a = a0 + (uint32_t)(st * (Cfg::STAGE >> 4)), bb = b0 + (uint32_t)(st * (Cfg::STAGE >> 4));
-        tc::mma_ss2pe(tmem + bf * D, a, a_hi, bb, b_hi, idesc, kb != ch * bpc);
-#pragma unroll
-        for (int k = 1; k < BC / 16; ++k) tc::mma_ss2e<1>(tmem + bf * D, a + (uint32_t)(2 * k * BM), a_hi, bb + (uint32_t)(k * (2048 / 16)), b_hi, idesc);
-        tc::mma_commit_e(&empty[st]);
+        if (!(ok = ring.take())) break;
+        const uint32_t a = a0 + (uint32_t)(ring.slot * (Cfg::STAGE >> 4)), bb = b0 + (uint32_t)(ring.slot * (Cfg::STAGE >> 4));
+        tc::mma4_ss(tmem + bf * D, a, a_hi, 2 * BM, bb, b_hi, 2048 / 16, idesc, kb != ch * bpc);
+        ring.give();
       }
       if (ok) tc::mma_commit_e(&o_full[bf]);
     }
@@ -275,7 +271,7 @@ mix_dq_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ C
     const uint32_t a_hi = (uint32_t)(dA >> 32), a0 = (uint32_t)dA, b_hi = (uint32_t)(dB >> 32), b0 = (uint32_t)dB;
     const uint32_t dst = tmem + t * D;
     bool ok = true;
-    int s = 0, ph = 0;                                        // key-tile ring position
+    tc::TileRing<NB, 1> ring(full, empty, s_abort);           // key tiles
     for (int kb = 0; kb < nkb && ok; ++kb) {
       const bool active = kb < nkb_t[t];
       const int st = kb % NA;
@@ -285,17 +281,9 @@ mix_dq_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ C
       for (int a = 0; a < ntap && ok; ++a, --al) {
 #pragma unroll
         for (int hl = 0; hl < nhl; ++hl) {
-          ok = tc::mbar_wait_warp(&full[s], ph, s_abort);
-          if (!ok) break;
-          if (active) {
-            tc::tc_fence_after();
-            const uint32_t bl = b0 + (uint32_t)(s * (Cfg::B_BYTES >> 4));
-            tc::mma_ss2pe(dst, al, a_hi, bl, b_hi, idesc, (kb | a | hl) != 0);
-#pragma unroll
-            for (int k = 1; k < BC / 16; ++k) tc::mma_ss2e<1>(dst, al + k * k_step, a_hi, bl + (uint32_t)(k * (2048 / 16)), b_hi, idesc);
-          }
-          tc::mma_commit_e(&empty[s]);
-          if (++s == NB) { s = 0; ph ^= 1; }
+          if (!(ok = ring.take())) break;
+          if (active) tc::mma4_ss(dst, al, a_hi, k_step, b0 + (uint32_t)(ring.slot * (Cfg::B_BYTES >> 4)), b_hi, 2048 / 16, idesc, (kb | a | hl) != 0);
+          ring.give();
         }
       }
       if (ok) tc::mma_commit_e(&a_empty[st]);
@@ -418,10 +406,11 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     constexpr uint32_t idescK2 = tc::make_idesc(BK, 128, 1, 1);      // two adjacent taps (see bwd_stream.cu)
     const int pairs = cq / 2, ngrp = pairs + (cq & 1), g_half = ngrp / 2;
     const int g_begin = ai == 0 ? 0 : g_half, g_end = ai == 0 ? g_half : ngrp;
+    tc::TileRing<NSTG, 1> ring(full, empty, s_abort);
     bool ok = true;
     for (int it = 0; it < nblk && ok; ++it) {
-      const int st = it % NSTG, ph = (it / NSTG) & 1;
-      const uint32_t sg = smem_u32(smem + st * Cfg::STAGE);
+      if (!(ok = ring.take())) break;
+      const uint32_t sg = smem_u32(smem + ring.slot * Cfg::STAGE);
       // P / dC: M = keys in chunks of 8, BR * 16 bytes apart; K = rows, 16 bytes apart
       const uint64_t dPa = tc::make_sdesc(sg + Cfg::sgP, 128, BR * 16, tc::kLayoutNone);
       const uint64_t dCa = tc::make_sdesc(sg + Cfg::sgC, 128, BR * 16, tc::kLayoutNone);
@@ -429,28 +418,17 @@ mix_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint64_t dQb = tc::make_sdesc(sg + Cfg::sgQ + (HALO - pq) * 128, 128, 1024, tc::kLayoutSW128);
       const uint32_t pa_hi = (uint32_t)(dPa >> 32), pa_lo = (uint32_t)dPa, ca_hi = (uint32_t)(dCa >> 32), ca_lo = (uint32_t)dCa;
       const uint32_t ob_hi = (uint32_t)(dOb >> 32), ob_lo = (uint32_t)dOb, qb_hi = (uint32_t)(dQb >> 32), qb_lo = (uint32_t)dQb;
-      ok = tc::mbar_wait_warp(&full[st], ph, s_abort);
-      if (!ok) break;
-      tc::tc_fence_after();
       if (ai == 0 && with_dv) {
-        tc::mma_ss2pe(tmem, pa_lo, pa_hi, ob_lo, ob_hi, idescV, it != 0);
-#pragma unroll
-        for (int k = 1; k < BR / 16; ++k) tc::mma_ss2e<1>(tmem, pa_lo + (uint32_t)(k * 16), pa_hi, ob_lo + (uint32_t)(k * (2048 / 16)), ob_hi, idescV);
+        tc::mma4_ss(tmem, pa_lo, pa_hi, 16, ob_lo, ob_hi, 2048 / 16, idescV, it != 0);
       }
       for (int gi = g_begin; gi < g_end; ++gi) {
         const bool pair = gi < pairs;
         const uint32_t dacc = tmem + 64 * (1 + 2 * gi), idg = pair ? idescK2 : idescV;
         const uint32_t bl = qb_lo + (uint32_t)(2 * gi * (128 >> 4));
-        tc::mma_ss2pe(dacc, ca_lo, ca_hi, bl, qb_hi, idg, it != 0);
-#pragma unroll
-        for (int k = 1; k < BR / 16; ++k) tc::mma_ss2e<1>(dacc, ca_lo + k * 16, ca_hi, bl + (uint32_t)(k * (2048 / 16)), qb_hi, idg);
-        if (CONV) {
-          const uint32_t cl_lo = ca_lo + (uint32_t)((Cfg::sgCl - Cfg::sgC) >> 4);
-#pragma unroll
-          for (int k = 0; k < BR / 16; ++k) tc::mma_ss2e<1>(dacc, cl_lo + k * 16, ca_hi, bl + (uint32_t)(k * (2048 / 16)), qb_hi, idg);
-        }
+        tc::mma4_ss(dacc, ca_lo, ca_hi, 16, bl, qb_hi, 2048 / 16, idg, it != 0);
+        if (CONV) tc::mma4_ss(dacc, ca_lo + (uint32_t)((Cfg::sgCl - Cfg::sgC) >> 4), ca_hi, 16, bl, qb_hi, 2048 / 16, idg, 1);
       }
-      tc::mma_commit_e(&empty[st]);
+      ring.give();
     }
     if (ok) tc::mma_commit_e(all_done);
   } else {
