@@ -2,8 +2,9 @@
 // in the X8 layout (mix_tc.cuh), so there is no element-wise phase in the loops.
 //   mix_pv_kernel   : O = P V.  CTA = 128 rows of a head; P is relative to one reference per row and key chunk, so the
 //                     accumulator is taken out of tensor memory and rescaled once per chunk.  Writes O, M, L, LSE.
-//   mix_dq_kernel   : dQ[i'] = sum_a dC[i' + pad_q - a] Kt_a.  CTA = two tiles of 128 rows that share every key tile (136 rows
-//                     of dC are staged; views shifted by a tap's rows start 16 bytes per row further).
+//   mix_dq_kernel   : dQ = dC K, without a filter.  CTA = one or two tiles of 128 rows that share every key tile.
+//   pair_mix_dq_kernel : dQ[i'] = sum_a dC[i' + pad_q - a] Kt_a, on CTA pairs (136 rows of dC are staged; views shifted by a tap's
+//                     rows start 16 bytes per row further).
 //   mix_dkdv_kernel : dV = P^T dO, dKt_a = dC^T Q^(a).  CTA = 128 keys x 64 columns of the head dim (two CTAs at d = 128);
 //                     P and dC are read MN-major, so nothing is transposed.
 // All are bound by the stream of P / dC (2 bytes per score entry and tensor) or by the MMAs at c_q = 6.
@@ -163,14 +164,12 @@ mix_pv_kernel(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ C
 }
 
 // ==========================================================================================
-template <int D, int NT_, bool CONV>
+template <int D, int NT_>
 struct MixDqCfg {
   static constexpr int BM = 128, AR = BM + 8, BC = 64, SL = D / 64, NT = NT_;
   static constexpr int A_BYTES = AR * 128;                    // one dC tile: 136 rows x 64 keys
   static constexpr int SLAB = BC * 128, B_BYTES = SL * SLAB;  // one key tile: 64 x D
-  // dC stages (all tiles), held for the key tiles of their block, and key tiles in flight: with a filter a block has 2 c_q key
-  // tiles, without one a single one
-  static constexpr int NA = CONV ? 2 : (NT == 2 ? 3 : 6);
+  static constexpr int NA = NT == 2 ? 3 : 6;                  // dC stages (all tiles), and key tiles in flight
   static constexpr int NB_ = (225 * 1024 - NA * NT * A_BYTES) / B_BYTES, NB = NB_ > 16 ? 16 : NB_;
   static constexpr int oB = NA * NT * A_BYTES;
   static constexpr int oBar = oB + NB * B_BYTES;
@@ -186,11 +185,11 @@ struct MixGradOut {
   float mul;
 };
 
-template <int D, int NT_, bool CONV>
-__global__ void __launch_bounds__(MixDqCfg<D, NT_, CONV>::kThreads, 1)
-mix_dq_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmB, const MixParams p, int ntap, MixGradOut out) {
-  constexpr int nhl = CONV ? 2 : 1;      // key tiles per tap: a (hi, lo) pair with a filter
-  using Cfg = MixDqCfg<D, NT_, CONV>;
+// without a filter: one key tile per block
+template <int D, int NT_>
+__global__ void __launch_bounds__(MixDqCfg<D, NT_>::kThreads, 1)
+mix_dq_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmB, const MixParams p, MixGradOut out) {
+  using Cfg = MixDqCfg<D, NT_>;
   constexpr int BM = Cfg::BM, AR = Cfg::AR, BC = Cfg::BC, SL = Cfg::SL, NT = Cfg::NT, NA = Cfg::NA, NB = Cfg::NB;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -208,14 +207,13 @@ mix_dq_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ C
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int lh = blockIdx.y, nQ = (p.nRT + NT - 1) / NT, q = nQ - 1 - blockIdx.x;
   const int u = p.u0 + lh / p.G, HG = p.H / p.G, b = u / HG, bh = b * p.H + (u - b * HG) * p.G + lh % p.G;
-  const int N = p.N, pq = ntap - 1;
+  const int N = p.N;
   int nkb_t[NT];
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
     const int rt = NT * q + t;
     nkb_t[t] = rt >= p.nRT ? 0 : (p.causal ? min(rt * BM + BM, p.N8) : p.N8) / BC;
   }
-  const int nB = ntap * nhl;             // key tiles per block
   const int nkb = max(nkb_t[0], nkb_t[NT - 1]);
 
   if (tid == 0) {
@@ -249,44 +247,36 @@ mix_dq_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ C
         for (int t = 0; t < NT; ++t) {
           // a tile past its last block (or past the last row tile) gets an earlier valid block's data
           const int rt = min(NT * q + t, p.nRT - 1), kk = min(kb, max(nkb_t[t], 1) - 1);
-          tc::tma_load_3d(smem + (st * NT + t) * Cfg::A_BYTES, &tmC, &a_full[st], 0, rt * (BM / 8), lh * (CONV ? 2 : 1) * (p.N8 / 8) + kk * (BC / 8));
+          tc::tma_load_3d(smem + (st * NT + t) * Cfg::A_BYTES, &tmC, &a_full[st], 0, rt * (BM / 8), lh * (p.N8 / 8) + kk * (BC / 8));
         }
         *s_aissued = kb + 1;
-        for (int a = 0; a < nB; ++a, ++id) {
-          const int s = id % NB;
-          ok = tc::mbar_wait(&empty[s], ((id / NB) & 1) ^ 1, s_abort);
-          if (!ok) break;
-          tc::mbar_expect_tx(&full[s], Cfg::B_BYTES);
-          for (int sl = 0; sl < SL; ++sl) tc::tma_load_3d(smem + Cfg::oB + s * Cfg::B_BYTES + sl * Cfg::SLAB, &tmB, &full[s], sl * 64, kb * BC, bh * nB + a);
-          *s_issued = id + 1;
-        }
+        const int s = id % NB;
+        ok = tc::mbar_wait(&empty[s], ((id / NB) & 1) ^ 1, s_abort);
+        if (!ok) break;
+        tc::mbar_expect_tx(&full[s], Cfg::B_BYTES);
+        for (int sl = 0; sl < SL; ++sl) tc::tma_load_3d(smem + Cfg::oB + s * Cfg::B_BYTES + sl * Cfg::SLAB, &tmB, &full[s], sl * 64, kb * BC, bh);
+        *s_issued = ++id;
       }
     }
   } else if (warp > NT * 4) {
     const int t = warp - (NT * 4 + 1);
     constexpr uint32_t idesc = tc::make_idesc(BM, D, 0, 1);
     const uint64_t dA = tc::make_sdesc(smem_u32(smem), AR * 16, 128, tc::kLayoutNone);
-    constexpr uint32_t k_step = 2 * AR;                       // 16-byte units per 16 keys; one per row
+    constexpr uint32_t k_step = 2 * AR;                       // 16-byte units per 16 keys
     const uint64_t dB = tc::make_sdesc(smem_u32(smem) + Cfg::oB, SL > 1 ? Cfg::SLAB : 16, 1024, tc::kLayoutSW128);
     const uint32_t a_hi = (uint32_t)(dA >> 32), a0 = (uint32_t)dA, b_hi = (uint32_t)(dB >> 32), b0 = (uint32_t)dB;
     const uint32_t dst = tmem + t * D;
     bool ok = true;
     tc::TileRing<NB, 1> ring(full, empty, s_abort);           // key tiles
     for (int kb = 0; kb < nkb && ok; ++kb) {
-      const bool active = kb < nkb_t[t];
       const int st = kb % NA;
       ok = tc::mbar_wait_warp(&a_full[st], (kb / NA) & 1, s_abort);
-      if (!ok) break;
-      uint32_t al = a0 + (uint32_t)((st * NT + t) * (Cfg::A_BYTES >> 4) + pq);        // dC rows i' + pad_q - a
-      for (int a = 0; a < ntap && ok; ++a, --al) {
-#pragma unroll
-        for (int hl = 0; hl < nhl; ++hl) {
-          if (!(ok = ring.take())) break;
-          if (active) tc::mma4_ss(dst, al, a_hi, k_step, b0 + (uint32_t)(ring.slot * (Cfg::B_BYTES >> 4)), b_hi, 2048 / 16, idesc, (kb | a | hl) != 0);
-          ring.give();
-        }
-      }
-      if (ok) tc::mma_commit_e(&a_empty[st]);
+      if (!ok || !(ok = ring.take())) break;
+      if (kb < nkb_t[t])
+        tc::mma4_ss(dst, a0 + (uint32_t)((st * NT + t) * (Cfg::A_BYTES >> 4)), a_hi, k_step, b0 + (uint32_t)(ring.slot * (Cfg::B_BYTES >> 4)), b_hi,
+                    2048 / 16, idesc, kb != 0);
+      ring.give();
+      tc::mma_commit_e(&a_empty[st]);
     }
     if (ok) tc::mma_commit_e(&done[t]);
   } else {
@@ -321,6 +311,159 @@ mix_dq_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ C
   if (warp == NT * 4 + 1) {
     tc::tc_fence_after();
     tc::tmem_dealloc(tmem, NT * D);
+  }
+}
+
+// ==========================================================================================
+// With a filter: dQ[i'] = sum_a dC[i' + pad_q - a] (Kt_a hi + lo).  A pair of CTAs works on two row tiles (cta_group::2), each staging its
+// own 136 rows of dC and half of the COLUMNS of every key tile: 12 key tiles per block of keys at c_q 6 are the traffic that
+// bounds this (24 bytes per cycle and SM from L2; one CTA per tile, N 1001, 16 heads, d = 64: 42 us).  An odd row tile is left
+// over at the front: rank 0 has no rows there.  Its dC, like that of keys past a tile's causal limit, is fetched from outside the
+// tensor and so zero.
+template <int D>
+struct MixDqPairCfg {
+  static constexpr int BM = 128, AR = BM + 8, BC = 64;
+  static constexpr int A_BYTES = AR * 128;                    // one dC tile: 136 rows x 64 keys
+  static constexpr int BT = BC * D, SLOT = 2 * BT;            // half a key tile: 64 keys x D / 2 columns; a tap's high and low one
+  // d = 64: two CTAs per SM
+  static constexpr int NA = D == 64 ? 2 : 3, NB = ((D == 64 ? 110 : 225) * 1024 - NA * A_BYTES) / SLOT;
+  static constexpr int oB = (NA * A_BYTES + 1023) / 1024 * 1024;
+  static constexpr int oBar = oB + NB * SLOT;
+  static constexpr int kSmemBytes = oBar + 512 + 1024;
+  static constexpr int kThreads = 192;
+  static_assert((D == 64 ? 2 : 1) * (kSmemBytes + 1024) <= 228 * 1024 && NB >= 4 && NB <= 24, "shared memory");
+};
+
+template <int D>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, D == 64 ? 2 : 1)
+pair_mix_dq_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmB, const MixParams p, int ntap, MixGradOut out) {
+  using Cfg = MixDqPairCfg<D>;
+  constexpr int BM = Cfg::BM, AR = Cfg::AR, BC = Cfg::BC, NA = Cfg::NA, NB = Cfg::NB;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::oBar);
+  // full and a_full: rank 0's; commits arrive in both CTAs
+  uint64_t* a_full = bars;               // [NA]
+  uint64_t* a_empty = a_full + NA;
+  uint64_t* full = a_empty + NA;         // [NB]
+  uint64_t* empty = full + NB;
+  uint64_t* done = empty + NB;
+  uint64_t* mma_drain = done + 1;
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(mma_drain + 1);
+  volatile int* s_abort = reinterpret_cast<volatile int*>(s_tmem + 1);
+  volatile int* s_issued = s_abort + 1;  // key tiles and dC stages the producer has issued
+  volatile int* s_aissued = s_abort + 2;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = tc::cluster_rank();
+  const int lh = blockIdx.y, top = p.nRT - 1 - 2 * (int)(blockIdx.x >> 1), rt = top - 1 + (int)rank;
+  const int u = p.u0 + lh / p.G, HG = p.H / p.G, b = u / HG, bh = b * p.H + (u - b * HG) * p.G + lh % p.G;
+  const int N = p.N, pq = ntap - 1;
+  auto blocks = [&](int t) { return t < 0 ? 0 : (p.causal ? min((t + 1) * BM, p.N8) : p.N8) / BC; };
+  const int my_nkb = blocks(rt), nkb = blocks(top);
+
+  if (tid == 0) {
+    for (int i = 0; i < NA; ++i) { tc::mbar_init(&a_full[i], 1); tc::mbar_init(&a_empty[i], 1); }
+    for (int i = 0; i < NB; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 1); }
+    tc::mbar_init(done, 1); tc::mbar_init(mma_drain, 1);
+    *s_abort = 0; *s_issued = 0; *s_aissued = 0;
+    tc::mbar_fence_init();
+  }
+  if (warp == 5) tc::tmem_alloc_pair(s_tmem, D);
+  tc::tc_fence_before();
+  tc::cluster_sync_all();
+  pdl_wait();
+  pdl_trigger();
+  tc::tc_fence_after();
+  const uint32_t tmem = *s_tmem;
+
+  if (warp == 4) {
+    if (lane == 0) {
+      int id = 0;
+      bool ok = true;
+      for (int kb = 0; kb < nkb && ok; ++kb) {
+        const int st = kb % NA;
+        ok = tc::mbar_wait(&a_empty[st], ((kb / NA) & 1) ^ 1, s_abort);
+        if (!ok) break;
+        if (rank == 0) tc::mbar_expect_tx(&a_full[st], 2 * Cfg::A_BYTES);
+        tc::tma_load_3d_pair(smem + st * Cfg::A_BYTES, &tmC, tc::cluster_addr(&a_full[st], 0), 0, kb < my_nkb ? rt * (BM / 8) : p.RP / 8,
+                             lh * 2 * (p.N8 / 8) + kb * (BC / 8));
+        *s_aissued = kb + 1;
+        for (int a = 0; a < ntap; ++a, ++id) {
+          const int s = id % NB;
+          ok = tc::mbar_wait(&empty[s], ((id / NB) & 1) ^ 1, s_abort);
+          if (!ok) break;
+          if (rank == 0) tc::mbar_expect_tx(&full[s], 2 * Cfg::SLOT);
+          for (int hl = 0; hl < 2; ++hl)
+            tc::tma_load_3d_pair(smem + Cfg::oB + s * Cfg::SLOT + hl * Cfg::BT, &tmB, tc::cluster_addr(&full[s], 0), (int)rank * (D / 2), kb * BC,
+                                 (bh * ntap + a) * 2 + hl);
+          *s_issued = id + 1;
+        }
+      }
+      // the last arrivals on this CTA's barriers have landed before it leaves
+      for (int i = max(0, id - NB); i < id && ok; ++i) ok = tc::mbar_wait(&empty[i % NB], (i / NB) & 1, s_abort);
+      for (int kb = max(0, nkb - NA); kb < nkb && ok; ++kb) ok = tc::mbar_wait(&a_empty[kb % NA], (kb / NA) & 1, s_abort);
+    }
+  } else if (warp == 5) {
+    if (rank == 0) {
+      constexpr uint32_t idesc = tc::make_idesc(2 * BM, D, 0, 1);
+      const uint64_t dA = tc::make_sdesc(smem_u32(smem), AR * 16, 128, tc::kLayoutNone);
+      const uint64_t dB = D == 64 ? tc::make_sdesc(smem_u32(smem) + Cfg::oB, 16, 512, tc::kLayoutSW64)
+                                  : tc::make_sdesc(smem_u32(smem) + Cfg::oB, 16, 1024, tc::kLayoutSW128);
+      const uint32_t a_hi = (uint32_t)(dA >> 32), a0 = (uint32_t)dA, b_hi = (uint32_t)(dB >> 32), b0 = (uint32_t)dB;
+      constexpr uint32_t k_step = 2 * AR, b_step = 16 * D / 16;     // 16-byte units per 16 keys
+      tc::TileRing<NB> ring(full, empty, s_abort);
+      bool ok = true;
+      for (int kb = 0; kb < nkb && ok; ++kb) {
+        const int st = kb % NA;
+        ok = tc::mbar_wait_warp(&a_full[st], (kb / NA) & 1, s_abort);
+        if (!ok) break;
+        uint32_t al = a0 + (uint32_t)(st * (Cfg::A_BYTES >> 4) + pq);      // dC rows i' + pad_q - a: 16 bytes per row
+        for (int a = 0; a < ntap; ++a, --al) {
+          if (!(ok = ring.take())) break;
+          const uint32_t bl = b0 + (uint32_t)(ring.slot * (Cfg::SLOT >> 4));
+          tc::mma4_ss<2>(tmem, al, a_hi, k_step, bl, b_hi, b_step, idesc, (kb | a) != 0);
+          tc::mma4_ss<2>(tmem, al, a_hi, k_step, bl + (Cfg::BT >> 4), b_hi, b_step, idesc, 1);
+          ring.give();
+        }
+        if (ok) tc::mma_commit_pair(&a_empty[st]);
+      }
+      if (ok) tc::mma_commit_pair(done);
+    }
+  } else {
+    const int gi = rt * BM + tid;
+    const uint32_t tQ = tmem + ((uint32_t)(warp * 32) << 16);
+    const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(done, 0, s_abort));
+    tc::tc_fence_after();
+#pragma unroll
+    for (int c = 0; c < D / 32; ++c) {
+      float o[32];
+      if (ok && my_nkb > 0) {
+        tc::tmem_ld32(tQ + c * 32, o);
+        if (gi < N) store_grad32(out.out, out.bf16_out, out.add, ((size_t)bh * N + gi) * D + c * 32, o, out.mul);
+      }
+    }
+  }
+  __syncwarp();
+  if (tid == 0 && *s_abort) tc::st_cluster_u32(tc::cluster_addr((const void*)s_abort, rank ^ 1), 1);
+  __syncwarp();
+  tc::tc_fence_before();
+  tc::cluster_sync_all();
+  if (*s_abort) {        // of either CTA
+    if (tid == 0) atomicExch(p.status, 1);
+    if (rank == 0 && warp == 5) tc::mma_commit_pair(mma_drain);
+    if (rank == 0 && tid == 128) {
+      volatile int never = 0;
+      constexpr uint32_t kDrain = 1u << 14;
+      const int issued = *s_issued, ai = *s_aissued;
+      for (int id = max(0, issued - NB); id < issued; ++id) tc::mbar_wait(&full[id % NB], (id / NB) & 1, &never, kDrain);
+      for (int kb = max(0, ai - NA); kb < ai; ++kb) tc::mbar_wait(&a_full[kb % NA], (kb / NA) & 1, &never, kDrain);
+    }
+    if (tid == 128) { volatile int never = 0; tc::mbar_wait(mma_drain, 0, &never); }
+    tc::cluster_sync_all();
+  }
+  if (warp == 5) {
+    tc::tc_fence_after();
+    tc::tmem_dealloc_pair(tmem, D);
   }
 }
 
@@ -519,20 +662,29 @@ cudaError_t launch_pv_t(const TrainParams& p, const MixParams& mp, cudaStream_t 
   if (e != cudaSuccess) return e;
   return launch_pdl(kern, dim3(mp.nRT, mp.nU * mp.G), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmP, tmV, mp, p.O, p.o_bf16, p.M, p.L, p.LSEout);
 }
-template <int D, int NT_, bool CONV>
-cudaError_t launch_dq_t(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, cudaStream_t stream) {
-  using Cfg = MixDqCfg<D, NT_, CONV>;
-  const size_t BH = (size_t)p.B * p.H;
-  constexpr bool conv = CONV;
+template <int D, int NT_>
+cudaError_t launch_dq_t(const TrainParams& p, const MixParams& mp, cudaStream_t stream) {
+  using Cfg = MixDqCfg<D, NT_>;
   alignas(64) CUtensorMap tmC, tmB;
-  if (!make_x8_map(&tmC, mp.C8, mp, Cfg::AR, Cfg::BC, conv ? 2 : 1)) return cudaErrorInvalidValue;
-  if (!make_tensor_map_bf16(&tmB, conv ? Kt : p.K, D, p.N, conv ? BH * p.cq * 2 : BH, 64, Cfg::BC, true)) return cudaErrorInvalidValue;
-  auto kern = mix_dq_kernel<D, NT_, CONV>;
+  if (!make_x8_map(&tmC, mp.C8, mp, Cfg::AR, Cfg::BC)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmB, p.K, D, p.N, (size_t)p.B * p.H, 64, Cfg::BC, true)) return cudaErrorInvalidValue;
+  auto kern = mix_dq_kernel<D, NT_>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
-  const MixGradOut out = {p.dQo, conv && p.causal ? p.dQ : nullptr, p.grad_bf16, conv ? kLn2 : p.scale};
-  return launch_pdl(kern, dim3((mp.nRT + NT_ - 1) / NT_, mp.nU * mp.G), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmC, tmB, mp, conv ? p.cq : 1,
-                    out);
+  const MixGradOut out = {p.dQo, nullptr, p.grad_bf16, p.scale};
+  return launch_pdl(kern, dim3((mp.nRT + NT_ - 1) / NT_, mp.nU * mp.G), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmC, tmB, mp, out);
+}
+template <int D>
+cudaError_t launch_dq_pair_t(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, cudaStream_t stream) {
+  using Cfg = MixDqPairCfg<D>;
+  alignas(64) CUtensorMap tmC, tmB;
+  if (!make_x8_map(&tmC, mp.C8, mp, Cfg::AR, Cfg::BC, 2)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmB, Kt, D, p.N, (size_t)p.B * p.H * p.cq * 2, D / 2, Cfg::BC, true)) return cudaErrorInvalidValue;
+  auto kern = pair_mix_dq_kernel<D>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+  if (e != cudaSuccess) return e;
+  const MixGradOut out = {p.dQo, p.causal ? p.dQ : nullptr, p.grad_bf16, kLn2};
+  return launch_pdl(kern, dim3((mp.nRT + 1) / 2 * 2, mp.nU * mp.G), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmC, tmB, mp, p.cq, out);
 }
 }  // namespace
 
@@ -540,12 +692,11 @@ cudaError_t launch_mix_pv(const TrainParams& p, const MixParams& mp, cudaStream_
   return p.d == 64 ? launch_pv_t<64>(p, mp, stream) : launch_pv_t<128>(p, mp, stream);
 }
 cudaError_t launch_mix_dq(const TrainParams& p, const MixParams& mp, const __nv_bfloat16* Kt, cudaStream_t stream) {
+  if (p.theta) return p.d == 64 ? launch_dq_pair_t<64>(p, mp, Kt, stream) : launch_dq_pair_t<128>(p, mp, Kt, stream);
   // two row tiles per CTA share the key tiles; with fewer than two such CTAs per SM one tile per CTA fills the GPU better
   const bool one = (long)((mp.nRT + 1) / 2) * mp.nU * mp.G < 2 * kSMs;
-#define FMTA_MIX_DQ(DD, C) (one ? launch_dq_t<DD, 1, C>(p, mp, Kt, stream) : launch_dq_t<DD, 2, C>(p, mp, Kt, stream))
-  if (p.theta) return p.d == 64 ? FMTA_MIX_DQ(64, true) : FMTA_MIX_DQ(128, true);
-  return p.d == 64 ? FMTA_MIX_DQ(64, false) : FMTA_MIX_DQ(128, false);
-#undef FMTA_MIX_DQ
+  if (p.d == 64) return one ? launch_dq_t<64, 1>(p, mp, stream) : launch_dq_t<64, 2>(p, mp, stream);
+  return one ? launch_dq_t<128, 1>(p, mp, stream) : launch_dq_t<128, 2>(p, mp, stream);
 }
 cudaError_t launch_mix_dkdv(const TrainParams& p, const MixParams& mp, __nv_bfloat16* dKt, bool early, cudaStream_t stream) {
   using Cfg = MixDkvCfg<true>;                    // (the tiles are the same without a filter)
