@@ -867,10 +867,12 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 //       contraction steps are 16 consecutive columns, so every fragment row is 16 contiguous bytes
 //       of shared memory and the products land in the accumulator already summed per (a, b).
 // The rows are staged by TMA (two mbarrier batches, bounded waits); every CTA builds its Toeplitz tiles from the filter.
-// One CTA per (64 keys, batch*head); dTheta leaves as one partial per CTA.
+// One CTA per (64 keys, batch*head), or 32 keys where dKt comes as (hi, lo) pairs: their 13 tiles of 64 keys leave room for one CTA
+// per SM, whose fetch and arithmetic take turns (16 heads, N 1001, d = 64: 22.3 us, now 19.5; 64 heads, N 8192, d = 128: 1345 us, now 1194).  dTheta leaves as one partial per CTA.
+template <bool LO>
 struct DkPostCfg {
   static constexpr int D = 64, NT = 256;
-  static constexpr int KEYS = 64, HALO = 8, ROWS = KEYS + 2 * HALO;   // c_k <= 17
+  static constexpr int KEYS = LO ? 32 : 64, HALO = 8, ROWS = KEYS + 2 * HALO;   // c_k <= 17
   // A staged tile is [ROWS][128 B] as TMA writes it with the 128-byte swizzle: the 16-byte chunk c of
   // a row sits at chunk c ^ (address bits 7..9).  Consecutive tiles start 128 bytes further along that
   // pattern, so that the same row of the c_q tap tiles (one dTheta fragment) covers all banks.
@@ -879,19 +881,20 @@ struct DkPostCfg {
   static constexpr int T_LD = 40, T_ELEMS = 16 * T_LD;        // one 16 x 32 Toeplitz tile (bf16), rows 80 bytes apart
   static constexpr int RED_LD = 7 * 24;              // floats per warp in the dTheta reduction buffer
   __host__ __device__ static constexpr int t_bytes(int cq) { return 2 * cq * T_ELEMS * 2; }
-  static constexpr int smem_bytes(int cq, bool lo) {           // alignment slack + key rows + c_q tap tiles + max(Toeplitz tiles, reduction buffer) + barriers
-    return 1024 + (cq * (lo ? 2 : 1) + 1) * TILE_STRIDE + (t_bytes(cq) > 8 * RED_LD * 4 ? t_bytes(cq) : 8 * RED_LD * 4) + 64;
+  static constexpr int smem_bytes(int cq) {           // alignment slack + key rows + c_q tap tiles + max(Toeplitz tiles, reduction buffer) + barriers
+    return 1024 + (cq * (LO ? 2 : 1) + 1) * TILE_STRIDE + (t_bytes(cq) > 8 * RED_LD * 4 ? t_bytes(cq) : 8 * RED_LD * 4) + 64;
   }
 };
 
 // LO: dKt_a is a (hi, lo) pair of tiles; the lo tiles follow the hi tiles in shared memory.  FOLD: see ThetaFold (an
 // instantiation of its own, because its registers cost the others their third CTA per SM)
 template <bool LO, bool FOLD>
-__global__ void __launch_bounds__(DkPostCfg::NT, LO ? 1 : 2)
+__global__ void __launch_bounds__(DkPostCfg<LO>::NT, 2)
 dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmX,
                    const float* __restrict__ theta, void* dK, const float* dKadd, int out_bf16, float* __restrict__ dTheta_part, int* status,
                    int H, int N, int cq, int ck, float scale, int n_jblocks, int dfull, int j_base, const ThetaFold fold) {
-  using Cfg = DkPostCfg;
+  using Cfg = DkPostCfg<LO>;
+  constexpr int MT = Cfg::KEYS / 32;                         // 16-key tiles per warp
   constexpr int D = Cfg::D, NT = Cfg::NT, KEYS = Cfg::KEYS, HALO = Cfg::HALO;
   constexpr int T_LD = Cfg::T_LD, T_ELEMS = Cfg::T_ELEMS, RED_LD = Cfg::RED_LD;
   extern __shared__ unsigned char smem_raw[];
@@ -952,14 +955,14 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   __syncthreads();
   bool ok = true;
 
-  // ---- dK: warp = (32 keys, 16 columns).  Its two 16-key tiles share the middle one of their three
-  // 16-row steps through X_a, and the Toeplitz fragments are the same for every tile ----
+  // ---- dK: warp = (16 MT keys, 16 columns).  With two 16-key tiles they share the middle one of their three
+  // 16-row steps through X_a; the Toeplitz fragments are the same for every tile ----
   const int cgp = warp & 3, kh = warp >> 2;
-  float acc[2][2][4] = {};
+  float acc[MT][2][4] = {};
   {
     const int l8 = lane & 7, q = lane >> 3;
     const int t_off = (l8 + (q & 1) * 8) * T_LD + (q >> 1) * 8;
-    const int x_row = 32 * kh + l8 + (q & 1) * 8, x_chunk = 2 * cgp + (q >> 1);
+    const int x_row = 16 * MT * kh + l8 + (q & 1) * 8, x_chunk = 2 * cgp + (q >> 1);
 #pragma unroll
     for (int a = 0; a < 7; ++a) {
       if (a < cq) {
@@ -973,14 +976,14 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         ldsm_x4(al[0], sT + (2 * a + 1) * T_ELEMS + t_off);
         ldsm_x4(al[1], sT + (2 * a + 1) * T_ELEMS + t_off + 16);
 #pragma unroll
-        for (int sh = 0; sh < 3 * HL; ++sh) {
-          const int st = sh % 3;
+        for (int sh = 0; sh < (MT + 1) * HL; ++sh) {
+          const int st = sh % (MT + 1);
           uint32_t bfr[4];
-          ldsm_x4_t(bfr, at(a + 1 + (sh / 3) * cq, x_row + 16 * st, x_chunk));
+          ldsm_x4_t(bfr, at(a + 1 + (sh / (MT + 1)) * cq, x_row + 16 * st, x_chunk));
 #pragma unroll
           for (int ks = 0; ks < 2; ++ks) {
             const int m = st - ks;                           // the tile whose step ks these rows are
-            if (m >= 0 && m < 2) {
+            if (m >= 0 && m < MT) {
               mma_bf16(acc[m][0], ah[ks], bfr[0], bfr[1]);
               mma_bf16(acc[m][1], ah[ks], bfr[2], bfr[3]);
               mma_bf16(acc[m][0], al[ks], bfr[0], bfr[1]);
@@ -995,12 +998,12 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   if (dK != nullptr) {
     const int g = lane >> 2, t4 = lane & 3;
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
+    for (int m = 0; m < MT; ++m)
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
-          const int key = J0 + 32 * kh + 16 * m + g + 8 * hh;
+          const int key = J0 + 16 * MT * kh + 16 * m + g + 8 * hh;
           if (key < N) {
             const size_t at_ = ((size_t)bh * N + key) * dfull + col0 + 16 * cgp + 8 * j + 2 * t4;
             float2 v = make_float2(acc[m][j][2 * hh], acc[m][j][2 * hh + 1]);
@@ -1011,7 +1014,7 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         }
   }
 
-  // ---- dTheta^T (filter columns x taps): warp = 8 keys, two 32-column contraction steps each ----
+  // ---- dTheta^T (filter columns x taps): warp = 4 MT keys, two 32-column contraction steps each ----
   float th[2][4][4] = {};                                    // [16 filter columns][four independent accumulation chains]
   {
     const int l8 = lane & 7, q = lane >> 3;
@@ -1020,8 +1023,8 @@ dk_post_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     const int bt = 1 + (l8 < cq ? l8 : 0);                   // B fragment row = tap (past c_q: tap 0); four 8-column slabs
     const bool wide = ck > 16;
 #pragma unroll 4
-    for (int kk = 0; kk < 8; ++kk) {
-      const int row = HALO + 8 * warp + kk;                  // shared-memory row of this key
+    for (int kk = 0; kk < 4 * MT; ++kk) {
+      const int row = HALO + 4 * MT * warp + kk;             // shared-memory row of this key
 #pragma unroll
       for (int ch_ = 0; ch_ < D / 8 * HL; ch_ += 4) {
         const int c0 = ch_ % (D / 8);
@@ -1252,28 +1255,35 @@ cudaError_t launch_bwd_dkdv_tc(const TrainParams& p, void* workspace, float* dTh
 }
 
 // The adjoint of the pre-pass over the call's window: dK (plus the band's part, causal) and the dTheta partials.
-cudaError_t launch_dk_post(const TrainParams& p, __nv_bfloat16* dKt, bool with_lo, float* dTheta_part_tc, int* status, cudaStream_t stream) {
+template <bool LO, bool FOLD>
+static cudaError_t launch_dk_post_t(const TrainParams& p, __nv_bfloat16* dKt, float* dTheta_part_tc, int* status, cudaStream_t stream) {
+  using Cfg = DkPostCfg<LO>;
   const int D = p.d;
   const size_t BH = (size_t)p.B * p.H;
   const int j_base = win_lo(p);
-  const int njb = (win_hi(p) - j_base + DkPostCfg::KEYS - 1) / DkPostCfg::KEYS;
-  dim3 g2(njb, (unsigned)BH, D / DkPostCfg::D);      // one CTA per 64 keys and 64 columns of the head dim
-  const int smem = DkPostCfg::smem_bytes(p.cq, with_lo);
-  auto kern = with_lo ? dk_post_mma_kernel<true, false> : p.fold.count ? dk_post_mma_kernel<false, true> : dk_post_mma_kernel<false, false>;
+  const int njb = (win_hi(p) - j_base + Cfg::KEYS - 1) / Cfg::KEYS;
+  dim3 g2(njb, (unsigned)BH, D / Cfg::D);            // one CTA per KEYS keys and 64 columns of the head dim
+  const int smem = Cfg::smem_bytes(p.cq);
+  auto kern = dk_post_mma_kernel<LO, FOLD>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   alignas(64) CUtensorMap tmK, tmX;
-  if (!make_tensor_map_bf16(&tmK, p.K, D, p.N, BH, 64, DkPostCfg::ROWS, true)) return cudaErrorInvalidValue;
-  if (!make_tensor_map_bf16(&tmX, dKt, D, p.N, BH * p.cq * (with_lo ? 2 : 1), 64, DkPostCfg::ROWS, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmK, p.K, D, p.N, BH, 64, Cfg::ROWS, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmX, dKt, D, p.N, BH * p.cq * (LO ? 2 : 1), 64, Cfg::ROWS, true)) return cudaErrorInvalidValue;
   // (the maps span the full head dim; each CTA fetches its 64-column slab)
   ScopedKernelTimer timer2_(kKernDkPost, stream);
-  return launch_pdl(kern, g2, dim3(DkPostCfg::NT), (size_t)smem, stream, tmK, tmX, p.theta, p.dKo, p.causal ? p.dK : (const float*)nullptr, p.grad_bf16, dTheta_part_tc, status, p.H, p.N, p.cq,
+  return launch_pdl(kern, g2, dim3(Cfg::NT), (size_t)smem, stream, tmK, tmX, p.theta, p.dKo, p.causal ? p.dK : (const float*)nullptr, p.grad_bf16, dTheta_part_tc, status, p.H, p.N, p.cq,
                     p.ck, p.scale, njb, D, j_base, p.fold);
+}
+cudaError_t launch_dk_post(const TrainParams& p, __nv_bfloat16* dKt, bool with_lo, float* dTheta_part_tc, int* status, cudaStream_t stream) {
+  if (with_lo) return launch_dk_post_t<true, false>(p, dKt, dTheta_part_tc, status, stream);
+  return p.fold.count ? launch_dk_post_t<false, true>(p, dKt, dTheta_part_tc, status, stream) : launch_dk_post_t<false, false>(p, dKt, dTheta_part_tc, status, stream);
 }
 
 // slots of dTheta partials written by the dKt adjoint kernel: one per CTA
-int bwd_tc_theta_slots(int B, int N, int d) {
-  return B * (d > DkPostCfg::D ? d / DkPostCfg::D : 1) * ((N + DkPostCfg::KEYS - 1) / DkPostCfg::KEYS);
+int bwd_tc_theta_slots(int B, int N, int d, bool with_lo) {
+  const int keys = with_lo ? DkPostCfg<true>::KEYS : DkPostCfg<false>::KEYS;
+  return B * (d > 64 ? d / 64 : 1) * ((N + keys - 1) / keys);
 }
 
 
