@@ -208,8 +208,11 @@ static int fwd_impl(const void* Q, const void* K, const void* V, const float* th
   if (path != 0 && path != 1 && path != -1) return FMTA_ERR_SHAPE;
   if (path != 0 && g_path != 0 && row_hi == 0 && mix_tc_supported(p) && workspace &&
       (path == 1 || g_path == 1 || mix_tc_pays(B, H, N, d, p.cq, p.G, theta != nullptr, false)) && aligned16(workspace) &&
-      mix_tc_call_bytes(B, H, N, d, p.cq, p.ck, p.G, theta != nullptr, causal, false, workspace_bytes) != 0)
+      mix_tc_call_bytes(B, H, N, d, p.cq, p.ck, p.G, theta != nullptr, causal, false, workspace_bytes) != 0) {
+    p.Kt_ext = reinterpret_cast<__nv_bfloat16*>(ktilde);
     return check_cuda(launch_mix_fwd(p, workspace, workspace_bytes, (cudaStream_t)stream));
+  }
+  if (ktilde && p.Wmix) return FMTA_ERR_UNSUPPORTED;     // the other mixing kernels make no stacked keys
   bool use_tc = (path != 0) && fwd_tc_supported(p);
   if (path == 1 && !use_tc) return FMTA_ERR_UNSUPPORTED;
   if (use_tc) {
@@ -454,11 +457,34 @@ int fmta_bwd_fused(const void* Q, const void* K, const void* V, const void* dO, 
                   ck, 1, scale, causal, 1, workspace, base, stream, ktilde, 0, 0, g16 ? outs : nullptr, count);
 }
 
+size_t fmta_mix_kept_bytes(int B, int H, int N, int d, int cq, int ck, int causal) {
+  if (B < 1 || H < 1 || N < 1 || d < 1 || cq < 1 || ck < 1) return 0;
+  return mix_tc_kept_bytes(B, H, N, d, cq, ck, causal != 0);
+}
+
+int fmta_mix_fwd_keep(const void* Q, const void* K, const void* V, const float* theta, const float* wmix, void* O, float* M, float* L,
+                      float* LSE, int B, int H, int N, int d, int cq, int ck, int G, float scale, int causal, int o_dtype,
+                      void* workspace, size_t workspace_bytes, void* kept, void* stream) {
+  if (!kept || !theta || !wmix) return FMTA_ERR_NULL;
+  if (G < 2) return FMTA_ERR_UNSUPPORTED;
+  return fwd_impl(Q, K, V, theta, wmix, O, M, L, LSE, B, H, N, d, cq, ck, G, scale, causal, o_dtype, -1, workspace, workspace_bytes, stream, kept);
+}
+
 int fmta_mix_bwd(const void* Q, const void* K, const void* V, const void* dO, int do_dtype, const void* O, int o_dtype,
                  const float* LSE, const float* theta, const float* wmix, void* dQ, void* dK, void* dV, int grad_dtype,
                  float* dTheta, float* dW, int B, int H, int N, int d, int cq, int ck, int G, float scale, int causal,
                  void* workspace, size_t workspace_bytes, void* stream) {
+  return fmta_mix_bwd_kept(Q, K, V, dO, do_dtype, O, o_dtype, LSE, theta, wmix, dQ, dK, dV, grad_dtype, dTheta, dW, B, H, N, d, cq, ck, G, scale,
+                           causal, workspace, workspace_bytes, nullptr, stream);
+}
+
+int fmta_mix_bwd_kept(const void* Q, const void* K, const void* V, const void* dO, int do_dtype, const void* O, int o_dtype,
+                      const float* LSE, const float* theta, const float* wmix, void* dQ, void* dK, void* dV, int grad_dtype,
+                      float* dTheta, float* dW, int B, int H, int N, int d, int cq, int ck, int G, float scale, int causal,
+                      void* workspace, size_t workspace_bytes, const void* kept, void* stream) {
   TrainParams p = {};
+  if (kept && !theta) return FMTA_ERR_NULL;
+  if (kept && !aligned16(kept)) return FMTA_ERR_ALIGN;
   if (int s = fill_bwd(p, Q, K, V, dO, /* D is made here */ LSE, LSE, theta, wmix, B, H, N, d, cq, ck, G, scale, causal)) return s;
   if (!O || !wmix) return FMTA_ERR_NULL;
   const int want = (dQ ? 1 : 0) | (dK ? 2 : 0);
@@ -471,6 +497,8 @@ int fmta_mix_bwd(const void* Q, const void* K, const void* V, const void* dO, in
   if (!mix_tc_supported(p)) return FMTA_ERR_UNSUPPORTED;
   if (!workspace || mix_tc_call_bytes(B, H, N, d, p.cq, p.ck, G, theta != nullptr, causal, true, workspace_bytes) == 0) return FMTA_ERR_WORKSPACE;
   p.dQo = dQ; p.dKo = dK; p.dVo = dV; p.grad_bf16 = grad_dtype == FMTA_DTYPE_BF16;
+  p.Kt_ext = reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(kept));
+  p.kt_valid = kept != nullptr;
   return check_cuda(launch_mix_bwd(p, dO, do_dtype == FMTA_DTYPE_F32, O, o_dtype == FMTA_DTYPE_BF16, dTheta, dW, want, workspace,
                                    workspace_bytes, (cudaStream_t)stream));
 }

@@ -126,6 +126,7 @@ bool mix_tc_shape(int B, int H, int N, int d, int cq, int G, bool conv);
 bool mix_tc_pays(int B, int H, int N, int d, int cq, int G, bool conv, bool bwd);      // ... sooner than the kernels it replaces
 bool mix_tc_supported(const TrainParams& p);
 size_t mix_tc_workspace_bytes(int B, int H, int N, int d, int cq, int ck, int G, bool bwd);
+size_t mix_tc_kept_bytes(int B, int H, int N, int d, int cq, int ck, bool causal);
 size_t mix_tc_call_bytes(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool causal, bool bwd, size_t limit);
 cudaError_t launch_mix_fwd(const TrainParams& p, void* workspace, size_t workspace_bytes, cudaStream_t stream);
 cudaError_t launch_mix_bwd(const TrainParams& p, const void* dO, bool do_f32, const void* O, bool o_bf16, float* dTheta, float* dW, int want,

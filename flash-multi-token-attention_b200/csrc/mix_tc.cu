@@ -151,6 +151,18 @@ bool mix_tc_supported(const TrainParams& p) {
   return p.Wmix && mix_tc_shape(p.B, p.H, p.N, p.d, p.cq, p.G, p.theta != nullptr) && tensor_maps_available();
 }
 
+// What a forward leaves for its backward (p.Kt_ext): the stacked keys, then the band's scores.
+static size_t kept_at(size_t rows, int d, int cq) { return up(rows * cq * 2 * d * 2); }
+size_t mix_tc_kept_bytes(int B, int H, int N, int d, int cq, int ck, bool causal) {
+  const size_t rows = (size_t)B * H * N, band = (cq - 1) + (ck - 1) / 2;
+  return kept_at(rows, d, cq) + (causal ? rows * (band > 0 ? band : 1) * 4 : 0);
+}
+static void use_kept(const TrainParams& p, const MixPlan& m, MixBuffers& b) {
+  if (!p.Kt_ext) return;
+  b.Kt = p.Kt_ext;
+  if (m.cband) b.Cband = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(p.Kt_ext) + kept_at(m.rows, p.d, p.cq));
+}
+
 // What one call takes, no more than `limit` (0: it cannot do with that).
 size_t mix_tc_call_bytes(int B, int H, int N, int d, int cq, int ck, int G, bool conv, bool causal, bool bwd, size_t limit) {
   const MixPlan m = plan(B, H, N, d, conv ? cq : 1, conv ? ck : 1, G, conv, causal, bwd, limit);
@@ -186,6 +198,7 @@ cudaError_t launch_mix_fwd(const TrainParams& p_, void* workspace, size_t worksp
   const MixPlan m = plan(p.B, p.H, p.N, p.d, p.cq, p.ck, p.G, p.theta != nullptr, p.causal, false, workspace_bytes);
   MixBuffers b;
   if (m.nU == 0 || carve(m, workspace, b) > workspace_bytes) return cudaErrorInvalidValue;
+  use_kept(p, m, b);
   int* status = nullptr;
   FMTA_TRY(status_word_of(b.status, stream, &status));
   MixParams q;
@@ -212,6 +225,7 @@ cudaError_t launch_mix_bwd(const TrainParams& p_, const void* dO, bool do_f32, c
   const MixPlan m = plan(p.B, p.H, p.N, p.d, p.cq, p.ck, p.G, conv, p.causal, true, workspace_bytes);
   MixBuffers b;
   if (m.nU == 0 || carve(m, workspace, b) > workspace_bytes) return cudaErrorInvalidValue;
+  use_kept(p, m, b);
   int* status = nullptr;
   FMTA_TRY(status_word_of(b.status, stream, &status));
   if (conv && p.causal) { p.Cband = b.Cband; p.dCband = b.dCband; p.dQ = b.dQ; p.dK = b.dK; }
@@ -223,7 +237,7 @@ cudaError_t launch_mix_bwd(const TrainParams& p_, const void* dO, bool do_f32, c
   fill(q, p, m, status);
   q.Cband = p.Cband; q.dCband = p.dCband; q.dW_part = b.dw_part;
   q.P8 = b.P8; q.C8 = b.C8;
-  if (conv) {
+  if (conv && !p.kt_valid) {
     FMTA_TRY(launch_ktilde(p, b.Kt, stream, true));
     if (p.causal) FMTA_TRY(launch_band_scores(p, stream));
   }

@@ -345,12 +345,27 @@ Mix mix_of(const Tensor& q, const Tensor& w, const Tensor& theta_) {
 
 // O (preallocated, fp32 or bf16), L, M, LSE
 void mix_forward_raw(const Mix& m, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& O, const Tensor& M, const Tensor& L,
-                     const Tensor& LSE, double scale, bool causal, const MixLimits& limits) {
+                     const Tensor& LSE, double scale, bool causal, const MixLimits& limits, int64_t keep_limit = 0, Tensor* kept = nullptr) {
   const Dims& s = m.s;
   arm_status(q);
   Tensor ws = m.tc_workspace(q, false, causal, m.tc_bytes(false, causal, limits.second));
   const bool tc = ws.defined();
   if (!tc) ws = m.exchange_workspace(q, 0, limits.first);
+  // The stacked keys and the band's scores for the backward (where it runs on the same kernels): two launches less.  Up to
+  // keep_limit bytes, within the caller's limit on what a mix takes and where the GPU has the room.
+  const size_t n = tc && kept && m.theta.defined() ? fmta_mix_kept_bytes(s.B, s.H, s.N, s.d, s.cq, s.ck, causal) : 0;
+  if (n && (int64_t)n <= keep_limit && (int64_t)(n + bytes_of(ws)) <= limits.second && m.tc_bytes(true, causal, limits.second)) {
+    try {
+      *kept = new_bytes(q, n);
+    } catch (const c10::OutOfMemoryError&) {
+    }
+  }
+  if (kept && kept->defined()) {
+    check_status(fmta_mix_fwd_keep(ptr(q), ptr(k), ptr(v), fptr(m.theta), fptr(m.w), ptr(O), fptr(M), fptr(L), fptr(LSE), s.B, s.H, s.N, s.d, s.cq,
+                                   s.ck, m.G, (float)scale, causal, dtype_code(O.scalar_type()), ptr(ws), bytes_of(ws), ptr(*kept), stream_of(q)),
+                 "fmta_mix_fwd_keep");
+    return;
+  }
   check_status(fmta_fwd(ptr(q), ptr(k), ptr(v), fptr(m.theta), fptr(m.w), ptr(O), fptr(M), fptr(L), fptr(LSE), s.B, s.H, s.N, s.d, s.cq, s.ck, m.G,
                         (float)scale, causal, dtype_code(O.scalar_type()), tc ? -1 : 0, ptr(ws), bytes_of(ws), stream_of(q)),
                "fmta_fwd(head mix)");
@@ -358,7 +373,7 @@ void mix_forward_raw(const Mix& m, const Tensor& q, const Tensor& k, const Tenso
 
 // {dQ, dK, dV, dW [H/G,G,G], dTheta}: gradients in grad_dtype on the tensor-core kernels, else fp32; want: 1 dQ (dW, dTheta), 2 dK and dV
 std::vector<Tensor> mix_backward_raw(const Mix& m, const Tensor& q, const Tensor& k, const Tensor& v, Tensor dO, const Tensor& O, const Tensor& LSE,
-                                     double scale, bool causal, int want, bool g16, const MixLimits& limits) {
+                                     double scale, bool causal, int want, bool g16, const MixLimits& limits, const Tensor& kept = {}) {
   const Dims& s = m.s;
   arm_status(q);
   const bool conv = m.theta.defined();
@@ -369,9 +384,9 @@ std::vector<Tensor> mix_backward_raw(const Mix& m, const Tensor& q, const Tensor
     for (int i = 0; i < 3; ++i)
       if (i == 0 ? want & 1 : want & 2) g[i] = at::empty(q.sizes(), q.options().dtype(g16 ? at::kBFloat16 : at::kFloat));
     if (const Tensor ws = m.tc_workspace(q, true, causal, n); ws.defined()) {
-      check_status(fmta_mix_bwd(ptr(q), ptr(k), ptr(v), ptr(dO), dtype_code(dO.scalar_type()), ptr(O), dtype_code(O.scalar_type()), fptr(LSE), fptr(m.theta),
+      check_status(fmta_mix_bwd_kept(ptr(q), ptr(k), ptr(v), ptr(dO), dtype_code(dO.scalar_type()), ptr(O), dtype_code(O.scalar_type()), fptr(LSE), fptr(m.theta),
                                 fptr(m.w), ptr(g[0]), ptr(g[1]), ptr(g[2]), g16 ? FMTA_DTYPE_BF16 : FMTA_DTYPE_F32, fptr(dT), fptr(dW), s.B, s.H, s.N, s.d,
-                                s.cq, s.ck, m.G, (float)scale, causal, ptr(ws), bytes_of(ws), stream_of(q)),
+                                s.cq, s.ck, m.G, (float)scale, causal, ptr(ws), bytes_of(ws), kept.defined() ? ptr(kept) : nullptr, stream_of(q)),
                    "fmta_mix_bwd");
       return {g[0], g[1], g[2], dW, dT};
     }
@@ -440,15 +455,16 @@ std::vector<Tensor> mix_backward(const Tensor& q, const Tensor& k, const Tensor&
 struct MixFn : public torch::autograd::Function<MixFn> {
   // no theta: mix only.  out32: fp32 output whatever q's dtype (the filter + mix operator)
   static Tensor forward(AutogradContext* ctx, const Tensor& Q, const Tensor& K, const Tensor& V, const std::optional<Tensor>& theta_o, const Tensor& w,
-                        double scale, bool causal, bool out32, const MixLimits& limits) {
+                        double scale, bool causal, bool out32, const MixLimits& limits, int64_t keep_limit) {
     const Tensor theta_ = theta_o ? *theta_o : Tensor();
     const Mix m = mix_of(Q, w, theta_);
     const Tensor q = bf16c(Q), k = bf16c(K), v = bf16c(V);
     const Tensor O = at::empty(q.sizes(), q.options().dtype(out32 ? at::kFloat : mix_out_dtype(Q, std::nullopt)));
     const Tensor LSE = new_f32(q, {m.s.B, m.s.H, m.s.N});
-    mix_forward_raw(m, q, k, v, O, Tensor(), Tensor(), LSE, scale, causal, limits);
+    Tensor kept;
+    mix_forward_raw(m, q, k, v, O, Tensor(), Tensor(), LSE, scale, causal, limits, keep_limit, &kept);
     const Tensor out = out32 ? O : O.to(Q.scalar_type());
-    ctx->save_for_backward({q, k, v, theta_, w, out, LSE});
+    ctx->save_for_backward({q, k, v, theta_, w, out, LSE, kept});
     ctx->saved_data["scale"] = scale; ctx->saved_data["causal"] = causal; ctx->saved_data["limit0"] = limits.first; ctx->saved_data["limit1"] = limits.second;
     ctx->saved_data["tq"] = (int64_t)Q.scalar_type(); ctx->saved_data["tk"] = (int64_t)K.scalar_type(); ctx->saved_data["tv"] = (int64_t)V.scalar_type();
     ctx->saved_data["has_theta"] = theta_.defined();
@@ -469,23 +485,24 @@ struct MixFn : public torch::autograd::Function<MixFn> {
     const int base = 0, iw = has_theta ? 4 : 3;
     int want = 3;
     if (!has_theta) want = (ctx->needs_input_grad(base) || ctx->needs_input_grad(iw) ? 1 : 0) | (ctx->needs_input_grad(1) || ctx->needs_input_grad(2) ? 2 : 0);
-    if (want == 0) return variable_list(9);
+    if (want == 0) return variable_list(10);
+    const Tensor kept = saved[7].defined() ? aligned(saved[7].contiguous()) : Tensor();       // (a saved-tensor hook may have moved it)
     auto g = mix_backward_raw(mix_of(q, w, theta), q, k, v, dO, O, LSE, ctx->saved_data["scale"].toDouble(), ctx->saved_data["causal"].toBool(), want, g16,
-                              {ctx->saved_data["limit0"].toInt(), ctx->saved_data["limit1"].toInt()});
+                              {ctx->saved_data["limit0"].toInt(), ctx->saved_data["limit1"].toInt()}, kept);
     for (int i = 0; i < 3; ++i) if (g[i].defined()) g[i] = g[i].to(ty[i]);
     const Tensor dT = has_theta ? g[4].to(theta.scalar_type()) : Tensor();
     const Tensor dW = g[3].defined() ? g[3].reshape(w.sizes()).to(w.scalar_type()) : Tensor();
-    return {g[0], g[1], g[2], dT, dW, Tensor(), Tensor(), Tensor(), Tensor()};
+    return {g[0], g[1], g[2], dT, dW, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
 
 Tensor mix_attention(const Tensor& q, const Tensor& k, const Tensor& v, const std::optional<Tensor>& theta_, const Tensor& w, double scale, bool causal,
-                     bool out32, const MixLimits& limits) {
+                     bool out32, const MixLimits& limits, int64_t keep_limit) {
   const Tensor theta = theta_ ? *theta_ : Tensor();
   mix_check(q, k, v, w, theta);
   c10::cuda::CUDAGuard guard(q.device());
   if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad() || w.requires_grad() || (theta.defined() && theta.requires_grad())))
-    return MixFn::apply(q, k, v, theta_, w, scale, causal, out32, limits);
+    return MixFn::apply(q, k, v, theta_, w, scale, causal, out32, limits, keep_limit);
   refuse_tangents({&q, &k, &v, &theta, &w});
   at::AutoGradMode no_grad(false);
   const Mix m = mix_of(q, w, theta);

@@ -99,7 +99,14 @@ lib.fmta_bwd_fused_workspace_bytes.argtypes = [_i] * 9
 lib.fmta_mix_workspace_bytes.restype = _sz
 lib.fmta_mix_workspace_bytes.argtypes = [_i] * 10 + [_sz]
 
-EXPORTS = ["fmta_mix_bwd", "fmta_mix_workspace_bytes", "fmta_bwd_fused_workspace_bytes", "fmta_bwd_fused", "fmta_set_status_word", "fmta_selftest_expire_next", "fmta_version", "fmta_strerror", "fmta_last_cuda_error", "fmta_workspace_bytes", "fmta_fwd",
+lib.fmta_mix_kept_bytes.restype = _sz
+lib.fmta_mix_kept_bytes.argtypes = [_i] * 7
+lib.fmta_mix_fwd_keep.restype = _i
+lib.fmta_mix_fwd_keep.argtypes = [_vp, _vp, _vp, _fp, _fp, _vp, _fp, _fp, _fp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _vp, _sz, _vp, _vp]
+lib.fmta_mix_bwd_kept.restype = _i
+lib.fmta_mix_bwd_kept.argtypes = lib.fmta_mix_bwd.argtypes[:-1] + [_vp, _vp]
+
+EXPORTS = ["fmta_mix_kept_bytes", "fmta_mix_fwd_keep", "fmta_mix_bwd_kept", "fmta_mix_bwd", "fmta_mix_workspace_bytes", "fmta_bwd_fused_workspace_bytes", "fmta_bwd_fused", "fmta_set_status_word", "fmta_selftest_expire_next", "fmta_version", "fmta_strerror", "fmta_last_cuda_error", "fmta_workspace_bytes", "fmta_fwd",
            "fmta_bwd_prep_D", "fmta_bwd", "fmta_fwd_keep_ktilde", "fmta_bwd_with_ktilde", "fmta_fwd_window", "fmta_bwd_window", "fmta_stacked_keys", "fmta_set_path", "fmta_profile_kernel", "fmta_bwd_dq_dw", "fmta_bwd_dq_dw_static", "fmta_bwd_dkdv", "fmta_decode", "fmta_decode_offset_causal", "fmta_decode_paged", "fmta_kv_append_paged"]
 
 

@@ -16,6 +16,7 @@ import torch
 import torch.nn as nn
 
 from . import _native
+from .conv_attn import _keep_limit
 
 
 # What a head mix may take for itself.  On the tensor cores that is the scores' operands P and dC (4.5 GiB of them, or one
@@ -88,7 +89,7 @@ class HeadConvAttentionFunction(torch.autograd.Function):
             scale = 1.0 / math.sqrt(q.shape[-1])
         if torch.jit.is_tracing():
             return super(HeadConvAttentionFunction, HeadConvAttentionFunction).apply(q, k, v, w, causal, scale)
-        return _native.mix_attention(q, k, v, None, w, scale, bool(causal), False, _limits())
+        return _native.mix_attention(q, k, v, None, w, scale, bool(causal), False, _limits(), 0)
 
     @staticmethod
     def forward(ctx, q, k, v, w, causal, scale):
@@ -129,7 +130,7 @@ class ConvHeadMixFunction(torch.autograd.Function):
     def apply(q, k, v, conv_kernel, w, causal, scale):
         if torch.jit.is_tracing():
             return super(ConvHeadMixFunction, ConvHeadMixFunction).apply(q, k, v, conv_kernel, w, causal, scale)
-        return _native.mix_attention(q, k, v, conv_kernel, w, scale, bool(causal), True, _limits())
+        return _native.mix_attention(q, k, v, conv_kernel, w, scale, bool(causal), True, _limits(), _keep_limit())
 
     @staticmethod
     def forward(ctx, q, k, v, conv_kernel, w, causal, scale):

@@ -229,6 +229,21 @@ int fmta_mix_bwd(const void* Q, const void* K, const void* V, const void* dO, in
                  void* workspace, size_t workspace_bytes, void* stream);
 
 /*
+ * The forward of a filter + mix and its backward need the same stacked keys ((hi, lo) pairs) and, behind a causal mask, the same
+ * scores of the filter's band.  fmta_mix_fwd_keep is fmta_fwd on the tensor-core kernels (fmta_mix_workspace_bytes says whether
+ * they take the call) and leaves both in `kept` (fmta_mix_kept_bytes, 16-byte aligned); fmta_mix_bwd_kept is fmta_mix_bwd of the
+ * same K, theta, scale and mask, which takes them from there.  Same bits as without.
+ */
+size_t fmta_mix_kept_bytes(int B, int H, int N, int d, int cq, int ck, int causal);
+int fmta_mix_fwd_keep(const void* Q, const void* K, const void* V, const float* theta, const float* wmix, void* O, float* M, float* L,
+                      float* LSE, int B, int H, int N, int d, int cq, int ck, int G, float scale, int causal, int o_dtype,
+                      void* workspace, size_t workspace_bytes, void* kept, void* stream);
+int fmta_mix_bwd_kept(const void* Q, const void* K, const void* V, const void* dO, int do_dtype, const void* O, int o_dtype,
+                      const float* LSE, const float* theta, const float* wmix, void* dQ, void* dK, void* dV, int grad_dtype,
+                      float* dTheta, float* dW, int B, int H, int N, int d, int cq, int ck, int G, float scale, int causal,
+                      void* workspace, size_t workspace_bytes, const void* kept, void* stream);
+
+/*
  * One window of sequence positions of a forward / backward (no counterpart in the reference, which has no
  * sequence parallelism): the building block of context-parallel training and prefill, where every GPU holds the
  * whole Q, K, V (dO, D, LSE) of its (batch, head) pairs -- gathered over NVLink -- and computes one or two

@@ -191,3 +191,25 @@ def test_halves_of_the_backward_are_halves(B, H, N, d, G, cq, ck, causal):
         assert all(torch.equal(a, b) for a, b in zip(got, want))
     assert "mix_dq_kernel" in kernels[0] and "reduce_partials" in kernels[0]
     assert "mix_dkdv_kernel" in kernels[1] and "mix_dq_kernel" not in kernels[1] and "reduce_partials" not in kernels[1]
+
+
+@pytest.mark.parametrize("B,H,N,d,G,cq,ck,causal", [(1, 4, 300, 64, 4, 6, 11, True), (2, 4, 257, 128, 2, 3, 5, False)])
+def test_backward_from_kept_keys_is_the_backward(monkeypatch, B, H, N, d, G, cq, ck, causal):
+    """The autograd node keeps the stacked keys and the band's scores of its forward; without them the bits are the same."""
+    import fmta_b200 as F
+    from fmta_b200 import head_conv
+    Q, K, V, dO, theta = orc.make_inputs(B, H, N, d, cq, ck, seed=N, dtype=torch.bfloat16)
+    w0 = torch.eye(G).repeat(H // G, 1, 1) + 0.05
+    res = []
+    for limit, hook in ((1 << 40, None), (0, None), (1 << 40, lambda t: torch.cat([t.flatten()[:1], t.flatten()])[1:].view(t.shape))):
+        monkeypatch.setattr(head_conv, "_keep_limit", lambda: limit)
+        q, k, v = (t.cuda().to(torch.bfloat16).requires_grad_() for t in (Q, K, V))
+        w, th = w0.cuda().requires_grad_(), theta.cuda().requires_grad_()
+        if hook is None:
+            o = F.conv_headmix_attention(q, k, v, th, w, causal, 1.0 / math.sqrt(d))
+        else:      # saved bytes come back at another address
+            with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: hook(t) if t.dtype == torch.uint8 else t):
+                o = F.conv_headmix_attention(q, k, v, th, w, causal, 1.0 / math.sqrt(d))
+        res.append((o.detach(),) + torch.autograd.grad(o, (q, k, v, th, w), dO.cuda().to(o.dtype)))
+    for other in res[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(res[0], other))
