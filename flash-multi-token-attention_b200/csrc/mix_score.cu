@@ -18,7 +18,7 @@
 // at the start of a block, 10.0 with (hi, lo) in one MMA and all of them taken (a block: 40.5 k cycles in series before).
 //
 // Without a filter neither Q nor dO of 16 heads fits shared memory, so their tiles stream through the ring once per block
-// beside K and V (18 bytes per score entry from L2); with a filter Q stays resident where it fits and the stacked keys stream.
+// beside K and V (18 bytes per score entry from L2; 10 where a pair of CTAs has 64 rows each); with a filter Q stays resident where it fits and the stacked keys stream.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -26,27 +26,35 @@
 
 namespace fmta {
 
-// MODE 0: one CTA per 128 rows; 1: a pair of CTAs per 256 rows (cta_group::2); 2: a pair whose MMAs take high and low keys together
+// MODE 0: one CTA per 128 rows; 1: a pair of CTAs per 256 rows (cta_group::2); 2: a pair whose MMAs take high and low keys together;
+// 3: a pair per 128 rows, 64 each
 template <int G, int D, bool CONV, bool BWD, int MODE>
 struct MixCfg {
   static constexpr int BM = 128, SL = D / 64, HALO = 8, QR = BM + HALO;
+  // HALF: an MMA of 128 rows over a pair leaves a CTA's 64 rows on the lanes twice: the first half of the keys on lanes 0..63, the
+  // second on 64..127.  So the same columns hold twice as many keys of half as many rows, whose tiles, streamed for every block, are
+  // half as large: 10 bytes per entry instead of 18.
+  static constexpr bool HALF = MODE == 3;
+  static constexpr int RC = HALF ? 64 : BM, RTS = MODE == 1 || MODE == 2 ? 2 : 1;      // rows per CTA, row tiles per CTA or pair
   // HL: a tap's low keys lie behind its high ones as 2 KB columns of ONE MMA (rank 0 stages the high, rank 1 the low ones), whose
   // two halves the element-wise warps add up when they take the scores.  An MMA of KB = 64 columns reads 8 KB of queries for 32
   // cycles of arithmetic; so it reads them once for both.
   static constexpr bool HL = MODE == 2;
   // keys per block: S and dP (backward) or two buffers of S (forward with a filter, where the MMAs are the bound) take 256
   // columns each; otherwise one buffer of up to 512
-  static constexpr int KB = (BWD || (CONV && G <= 8)) ? 256 / G : (512 / G < 128 ? 512 / G : 128);
+  static constexpr int KB = (HALF ? 2 : 1) * ((BWD || (CONV && G <= 8)) ? 256 / G : (512 / G < 128 ? 512 / G : 128));
   static constexpr int NBUF = BWD || HL ? 1 : 512 / (G * KB);
-  static constexpr int SN = HL ? 2 * KB : KB;                  // columns of a head's scores
+  static constexpr int CB = HALF ? KB / 2 : KB;                // keys of a block on a lane
+  static constexpr int SN = HL ? 2 * KB : CB;                  // columns of a head's scores
   static constexpr int KT = G >= 8 ? 4 : 8;                    // keys per thread and pass
   static constexpr int GC = HL || G < 4 ? 2 : 4;                     // output heads per register pass
-  static constexpr int NPASS = KB / 2 / KT;
+  static constexpr int NPASS = CB / 2 / KT;
   static constexpr bool PAIR = MODE > 0;
-  static_assert(!PAIR || (CONV && KB >= 32), "pairs: with a filter, N = KB a multiple of 32");
+  static_assert(!PAIR || (CONV != HALF && KB >= 32), "pairs: N = KB a multiple of 32");
+  static_assert(!HALF || BWD, "the forward's rows have two threads");
   static constexpr bool RES = CONV && G * SL * QR * 128 <= (PAIR && !BWD ? 140 : 100) * 1024;   // Q resident; else (with a filter) two stages of one head's Q
   static constexpr int Q_HEAD = SL * QR * 128;
-  static constexpr int SLOT = BM * 128;                        // ring slot: one A slab tile, or B slab tiles
+  static constexpr int SLOT = RC * 128;                        // ring slot: one A slab tile, or B slab tiles
   static constexpr int KC = PAIR ? KB / 2 : KB;                // keys of a block that this CTA stages
   static constexpr int TB = (HL ? KB : KC) * 128, TPS = 16384 / TB;        // stacked slab tile (KC keys x 64 columns; HL: KB), tiles per slot
   static constexpr int TBP = KC * 128;                         // slab tile of K or V
@@ -65,7 +73,7 @@ struct MixCfg {
   static constexpr int oBar = oDW + DW_BYTES;
   static constexpr int oRing = (oBar + 512 + 1023) / 1024 * 1024;
   static constexpr int NSLOT_ = (226 * 1024 - oRing) / SLOT;
-  static constexpr int NSLOT = NSLOT_ > 20 ? 20 : NSLOT_;
+  static constexpr int NSLOT = NSLOT_ > 24 ? 24 : NSLOT_;
   // a slot is held until the last tile that uses it: B tiles of several heads in one slot, with an A slot for each
   static constexpr int TPP = SLOT / TBP < NSLOT - 2 ? SLOT / TBP : NSLOT - 2;
   static constexpr int kSmemBytes = oRing + NSLOT * SLOT + 1024;
@@ -76,6 +84,12 @@ struct MixCfg {
   static_assert(kSmemBytes <= 227 * 1024, "shared memory");
   static_assert(SLOT % 1024 == 0 && TB % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
 };
+
+FMTA_DEVINL float ld_cluster_f32(uint32_t cluster_src) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_src) : "memory");
+  return v;
+}
 
 // Key chunks with keys of row tile `top` or before (kch is a power of two).  Only these get a CTA: one without keys kept its SM for
 // 5 us of setting up, and at B 2, H 8, N 1001 (groups of 4) 112 of 256 were such: the last of the others began 11 us late.
@@ -89,7 +103,7 @@ __global__ void __cluster_dims__(MODE > 0 ? 2 : 1, 1, 1) __launch_bounds__(384, 
 mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmdO, const __grid_constant__ CUtensorMap tmV, const MixParams p) {
   using Cfg = MixCfg<G, D, CONV, BWD, MODE>;
-  constexpr int BM = Cfg::BM, SL = Cfg::SL, HALO = Cfg::HALO, KB = Cfg::KB, KT = Cfg::KT, GC = Cfg::GC, NPASS = Cfg::NPASS;
+  constexpr int BM = Cfg::BM, RC = Cfg::RC, CB = Cfg::CB, SL = Cfg::SL, HALO = Cfg::HALO, KB = Cfg::KB, KT = Cfg::KT, GC = Cfg::GC, NPASS = Cfg::NPASS;
   constexpr int SLOT = Cfg::SLOT, NSLOT = Cfg::NSLOT, TB = Cfg::TB, TBP = Cfg::TBP, TPS = Cfg::TPS, TPP = Cfg::TPP, NBUF = Cfg::NBUF;
   constexpr bool PAIR = Cfg::PAIR, HL = Cfg::HL, HLB = HL && BWD;
   constexpr int CPG = PAIR ? 2 : 1;                          // CTAs that issue together
@@ -128,16 +142,16 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   // row tiles (of a pair: two) from the last (most keys) on; the key chunks of a row tile side by side.  An odd row tile is
   // left over at the front, where a causal mask leaves the fewest keys: rank 0 has no rows there (rt = -1)
   int top = p.nRT - 1, kc = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, nkc = score_chunks(p, top);
-  while (kc >= nkc) { kc -= nkc; top -= CPG; nkc = score_chunks(p, top); }
-  const int rt = top - (CPG - 1) + (int)rank, ul = blockIdx.y;
+  while (kc >= nkc) { kc -= nkc; top -= Cfg::RTS; nkc = score_chunks(p, top); }
+  const int rt = Cfg::RTS == 2 ? top - 1 + (int)rank : top, ul = blockIdx.y;
   const int u = p.u0 + ul, HG = p.H / G, b = u / HG, grp = u - b * HG;
   const int bh0 = b * p.H + grp * G;                         // first head of the group
-  const int R0 = rt * BM;
+  const int R0 = rt * BM + (Cfg::HALF ? (int)rank * RC : 0);               // first row of this CTA
   const int k_lo = kc * p.kch;
-  const int k_hi = min(min(k_lo + p.kch, p.N8), p.causal ? R0 + BM : p.N8);     // multiples of 128 (or a chunk of 64)
+  const int k_hi = min(min(k_lo + p.kch, p.N8), p.causal ? rt * BM + BM : p.N8);     // multiples of 128 (or a chunk of 64)
   const int my_nblk = k_hi > k_lo && rt >= 0 ? (k_hi - k_lo) / KB : 0;          // blocks with keys of this CTA's rows
   int nblk = my_nblk;                                                           // ... of the pair's
-  if constexpr (PAIR) {
+  if constexpr (Cfg::RTS == 2) {
     const int kp = min(min(k_lo + p.kch, p.N8), p.causal ? R0 + (int)(2 - rank) * BM : p.N8);
     nblk = kp > k_lo ? (kp - k_lo) / KB : 0;
   }
@@ -228,7 +242,7 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             if (!ok) return;
             for (int j = 0; j < n; ++j) load(sRing + s * SLOT + j * TBP, tb, &full[s], ((i + j) % SL) * 64, key, bh0 + (i + j) / SL);
           }
-          const int s = slot_of(BM * 128);
+          const int s = slot_of(RC * 128);
           if (!ok) return;
           load(sRing + s * SLOT, ta, &full[s], (i % SL) * 64, R0, bh0 + i / SL);
         }
@@ -271,7 +285,7 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // ===================== MMA issuer: all lanes run the loop; one elected lane issues =====================
     for (int attempt = 0; attempt < attempts; ++attempt) {
     if (rank == 0) {
-    constexpr uint32_t idesc = tc::make_idesc(CPG * BM, Cfg::SN, 0, 0), idescP = tc::make_idesc(CPG * BM, KB, 0, 0);
+    constexpr uint32_t idesc = tc::make_idesc(CPG * RC, HL ? 2 * KB : KB, 0, 0), idescP = tc::make_idesc(CPG * RC, KB, 0, 0);
     const uint64_t d0 = tc::make_sdesc(smem_u32(sRing), 16, 1024, tc::kLayoutSW128);
     const uint32_t hi = (uint32_t)(d0 >> 32), lo0 = (uint32_t)d0;
     const uint32_t q_lo = (uint32_t)tc::make_sdesc(smem_u32(sQ), 16, 1024, tc::kLayoutSW128);
@@ -298,7 +312,7 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         if (!ok) return;
         const int s = take();
         if (!ok) return;
-        tc::mma4_ss<CPG>(dst + (i / SL) * KB, lo0 + (uint32_t)(s * (SLOT >> 4)), hi, 2,
+        tc::mma4_ss<CPG>(dst + (i / SL) * CB, lo0 + (uint32_t)(s * (SLOT >> 4)), hi, 2,
                          lo0 + (uint32_t)(bs * (SLOT >> 4) + (i % TPP) * (TBP >> 4)), hi, 2, idescP, i % SL != 0);
         commit(&empty[s]);
         if (i % TPP == TPP - 1 || i == G * SL - 1) commit(&empty[bs]);
@@ -341,7 +355,7 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const int bf = it % NBUF, ub = it / NBUF;
       if (ub > 0) wait(&s_free[HLB ? 1 : bf], ub - 1);
       if (!ok) break;
-      if constexpr (CONV) stacked(tmem + bf * (G * KB), it); else plain(tmem + bf * (G * KB), it);
+      if constexpr (CONV) stacked(tmem + bf * (G * KB), it); else plain(tmem + bf * (G * CB), it);
       if (!ok) break;
       commit(&s_full[bf]);
       if constexpr (BWD) {
@@ -363,8 +377,9 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::kRegsEw));
     for (int attempt = 0; attempt < attempts; ++attempt) {
     const int qtr = warp & 3, hf = warp >> 2;
-    const int r = qtr * 32 + lane, gi = R0 + r;              // row of the tile = TMEM lane; query index
-    const uint32_t tS0 = tmem + ((uint32_t)(qtr * 32) << 16) + hf * (KB / 2);
+    const int r = (Cfg::HALF ? qtr & 1 : qtr) * 32 + lane, gi = R0 + r;        // row of the tile = TMEM lane (HALF: mod 64); query index
+    const int key0 = (Cfg::HALF ? (qtr >> 1) * CB : 0) + hf * (CB / 2);        // this thread's first key of a block
+    const uint32_t tS0 = tmem + ((uint32_t)(qtr * 32) << 16) + hf * (CB / 2);
     const int jlim = gi < N ? (p.causal ? min(gi, N - 1) : N - 1) : -1;        // last key of this row
     const size_t lh0 = (size_t)ul * G;
     const size_t kc8 = p.N8 / 8;
@@ -396,7 +411,7 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     auto load_s = [&](uint64_t (&s)[G][KP], uint32_t base, int ps, int j0) {
       float v[G][KT];
 #pragma unroll
-      for (int g = SH; g < G; ++g) tmem_ld_nowait<KT>(base + g * KB + ps * KT, v[g]);
+      for (int g = SH; g < G; ++g) tmem_ld_nowait<KT>(base + g * CB + ps * KT, v[g]);
 #pragma unroll
       for (int g = 0; g < SH; ++g)
 #pragma unroll
@@ -539,7 +554,7 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         tc::tc_fence_after();
         if constexpr (HL) take_all();
         const uint32_t base = tS0 + bf * (G * KB);
-        const int j0 = k_lo + kb * KB + hf * (KB / 2);
+        const int j0 = k_lo + kb * KB + key0;
         // rows whose first valid key is not in block 0 exist only on the diagonal
         if (attempt == 0 && (kb == 0 || (p.causal && k_lo + kb * KB + KB - 1 > R0))) ok = init_ref(base, j0);
         if (!ok) break;
@@ -639,7 +654,7 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         if (!ok) break;
         if (skip) { if (!HL) free_s(SH > 0 ? 1 : 0); free_d(); continue; }
         tc::tc_fence_after();
-        const int j0 = k_lo + kb * KB + hf * (KB / 2);
+        const int j0 = k_lo + kb * KB + key0;
         uint64_t s[G][KP];
         // a pass's scores are fetched when dW of the one before is made, ahead of its dC: the last one's columns are released, and
         // the next block's MMAs begin, that much earlier (16 heads: 27 k cycles of arithmetic and 9 k of waiting per block before)
@@ -657,7 +672,7 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           for (int g0 = 0; g0 < G; g0 += GC) {
             float dp[GC][KT];
 #pragma unroll
-            for (int c = 0; c < GC; ++c) tmem_ld_nowait<KT>(tS0 + Cfg::colP + (g0 + c) * KB + ps * KT, dp[c]);
+            for (int c = 0; c < GC; ++c) tmem_ld_nowait<KT>(tS0 + Cfg::colP + (g0 + c) * CB + ps * KT, dp[c]);
             uint64_t acc[GC][KP];
             mix(acc, s, sWf, g0);
             tc::tmem_wait_ld();
@@ -814,7 +829,7 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
   __syncthreads();
 
-  if (BWD && rt >= 0) {
+  if (BWD && rt >= 0 && !(Cfg::HALF && rank != 0)) {
     const int slot = (b * p.nRT + rt) * p.nKC + kc;
     float* out = p.dW_part + ((size_t)slot * HG + grp) * (G * G);
     if (kc == nkc - 1)                                       // the slots of the chunks that no CTA has
@@ -824,6 +839,11 @@ mix_score_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       float t = 0.f;
       if (nblk > 0)                                          // (of a pair, with no key of this CTA's rows: zeros)
         for (int w = 0; w < 8; ++w) t += reinterpret_cast<const float*>(smem + Cfg::oDW + w * (Cfg::DW_MMA ? 4096 : G * G * 4))[i];
+      if constexpr (Cfg::HALF) {                             // the other CTA of the row tile
+        if (nblk > 0)
+          for (int w = 0; w < 8; ++w)
+            t += ld_cluster_f32(tc::cluster_addr(reinterpret_cast<const float*>(smem + Cfg::oDW + w * (Cfg::DW_MMA ? 4096 : G * G * 4)) + i, 1));
+      }
       out[i] = t * p.cw;
     }
   }
@@ -857,15 +877,15 @@ cudaError_t launch_score_m(const TrainParams& p, const MixParams& mp, const __nv
   using Cfg = MixCfg<G, D, CONV, BWD, MODE>;
   const size_t BH = (size_t)p.B * p.H;
   alignas(64) CUtensorMap tmQ, tmB, tmdO, tmV;
-  if (!make_tensor_map_bf16(&tmQ, p.Q, D, p.N, BH, 64, CONV ? Cfg::QR : Cfg::BM, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmQ, p.Q, D, p.N, BH, 64, CONV ? Cfg::QR : Cfg::RC, true)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmB, CONV ? Kt : p.K, D, p.N, CONV ? BH * p.cq * 2 : BH, 64, Cfg::HL ? Cfg::KB : Cfg::KC, true)) return cudaErrorInvalidValue;
-  if (!make_tensor_map_bf16(&tmdO, BWD ? p.dO : p.Q, D, p.N, BH, 64, Cfg::BM, true)) return cudaErrorInvalidValue;
+  if (!make_tensor_map_bf16(&tmdO, BWD ? p.dO : p.Q, D, p.N, BH, 64, Cfg::RC, true)) return cudaErrorInvalidValue;
   if (!make_tensor_map_bf16(&tmV, p.V, D, p.N, BH, 64, Cfg::KC, true)) return cudaErrorInvalidValue;
   auto kern = mix_score_kernel<G, D, CONV, BWD, MODE>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
   int ctas = 0;
-  for (int top = mp.nRT - 1; top >= 0; top -= MODE > 0 ? 2 : 1) ctas += (MODE > 0 ? 2 : 1) * score_chunks(mp, top);
+  for (int top = mp.nRT - 1; top >= 0; top -= Cfg::RTS) ctas += (MODE > 0 ? 2 : 1) * score_chunks(mp, top);
   return launch_pdl(kern, dim3(ctas, mp.nU), dim3(Cfg::kThreads), (size_t)Cfg::kSmemBytes, stream, tmQ, tmB, tmdO, tmV, mp);
 }
 
@@ -885,6 +905,13 @@ cudaError_t launch_score_t(const TrainParams& p, const MixParams& mp, const __nv
       }
       return launch_score_m<G, D, CONV, BWD, 1>(p, mp, Kt, stream);
     }
+  }
+  if constexpr (!CONV && BWD && G == 16) {
+    // Pairs of 64 rows each: at head dim 128, where the streamed tiles are twice as large (N 4096, 2 groups: 2334 -> 2203 us of
+    // backward), and while single CTAs do not fill the GPU (1 group, d = 64: N 300 140 -> 107 us, N 1000 148 -> 123).  Else the
+    // pairs' shorter CTAs cost more than they give (2 groups, N 2048: 325 us of this kernel, 345 with pairs).
+    const long live = (long)mp.nRT * mp.nKC * mp.nU / (p.causal ? 2 : 1);
+    if (D == 128 || live < kSMs) return launch_score_m<G, D, CONV, BWD, 3>(p, mp, Kt, stream);
   }
   return launch_score_m<G, D, CONV, BWD, 0>(p, mp, Kt, stream);
 }

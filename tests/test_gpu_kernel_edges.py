@@ -189,6 +189,12 @@ def test_mixing_behind_a_filter_on_cta_pairs(B, H, N, d, G, cq, ck, causal, spre
     test_mixing_tiles_and_groups(B, H, N, d, G, cq, ck, causal, spread)
 
 
+@pytest.mark.parametrize("B,H,N,d,causal", [(1, 16, 200, 64, False), (1, 16, 260, 128, False), (2, 32, 321, 128, True), (3, 16, 449, 64, True)])
+def test_mixing_of_16_heads_on_half_tiles(request, B, H, N, d, causal):
+    """The backward without a filter on pairs of CTAs with 64 rows each: a tile that rank 0 alone has rows of, several groups."""
+    test_mixing_tiles_and_groups_on_the_tensor_cores(request, B, H, N, d, 16, 0, 0, causal, 1.0)
+
+
 @pytest.mark.parametrize("B,H,N,G,causal", [(1, 16, 1600, 16, True), (1, 16, 2048, 16, True), (2, 16, 1500, 16, True), (1, 8, 2100, 8, True)])
 def test_mixing_stays_in_its_workspace(B, H, N, G, causal):
     """Sizes whose key chunks depend on whether there is a filter: exactly the bytes that the library names, and what lies
